@@ -9,6 +9,10 @@
 
 using bf16 = __nv_bfloat16;
 
+// seq_gemm_fp32.cu
+int pg_gemm_fp32(const float* x, long long ldx, long long bsx, const float* w, long long ldw, long long bsw, float* out, long long ldo, long long bso,
+                 const float* bias, int accumulate, float scale, int T, int F, int K, int batch, cudaStream_t st);
+
 #define PG_ST(s) reinterpret_cast<cudaStream_t>(s)
 #define PG_RET()                                                   \
   do {                                                             \
@@ -50,8 +54,8 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
-// out[t, f] = sum_k x[t, k] * w[f, k]: 64 x 64 output tile per CTA, 16-wide k steps through shared memory, a 4 x 4
-// register tile per thread, plain fp32 FMAs in k order (no reduced-precision tensor mode, no split accumulation).
+// bf16 operands of shapes the TMA kernels cannot take (fp32 operands: seq_gemm_fp32.cu).  out[t, f] = sum_k x[t, k] * w[f, k]: 64 x 64
+// output tile per CTA, 16-wide k steps through shared memory, a 4 x 4 register tile per thread, plain fp32 FMAs in k order.
 // ---------------------------------------------------------------------------------------------------------------------
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(256) gemm_simt_kernel(const TI* __restrict__ x, long long ldx, const TI* __restrict__ w, long long ldw,
@@ -268,8 +272,8 @@ extern "C" int pg_gemm_simt(const void* x, long long ldx, const void* w, long lo
   if (grid.y > 65535) return PG_ERR_ARG;
   cudaStream_t st = PG_ST(stream);
   if (in_f32 && out_f32)
-    gemm_simt_kernel<float, float><<<grid, 256, 0, st>>>(static_cast<const float*>(x), ldx, static_cast<const float*>(w), ldw, static_cast<float*>(out), ldo, tokens, features, K);
-  else if (!in_f32 && out_f32)
+    return pg_gemm_fp32(static_cast<const float*>(x), ldx, 0, static_cast<const float*>(w), ldw, 0, static_cast<float*>(out), ldo, 0, nullptr, 0, 1.0f, tokens, features, K, 1, st);
+  if (!in_f32 && out_f32)
     gemm_simt_kernel<bf16, float><<<grid, 256, 0, st>>>(static_cast<const bf16*>(x), ldx, static_cast<const bf16*>(w), ldw, static_cast<float*>(out), ldo, tokens, features, K);
   else if (!in_f32 && !out_f32)
     gemm_simt_kernel<bf16, bf16><<<grid, 256, 0, st>>>(static_cast<const bf16*>(x), ldx, static_cast<const bf16*>(w), ldw, static_cast<bf16*>(out), ldo, tokens, features, K);
@@ -285,8 +289,8 @@ extern "C" int pg_gemm_simt_bias(const void* x, long long ldx, const void* w, lo
   if (grid.y > 65535) return PG_ERR_ARG;
   cudaStream_t st = PG_ST(stream);
   if (in_f32 && out_f32)
-    gemm_simt_kernel<float, float><<<grid, 256, 0, st>>>(static_cast<const float*>(x), ldx, static_cast<const float*>(w), ldw, static_cast<float*>(out), ldo, tokens, features, K, 0, 0, 0, bias, accumulate, scale);
-  else if (!in_f32 && out_f32)
+    return pg_gemm_fp32(static_cast<const float*>(x), ldx, 0, static_cast<const float*>(w), ldw, 0, static_cast<float*>(out), ldo, 0, bias, accumulate, scale, tokens, features, K, 1, st);
+  if (!in_f32 && out_f32)
     gemm_simt_kernel<bf16, float><<<grid, 256, 0, st>>>(static_cast<const bf16*>(x), ldx, static_cast<const bf16*>(w), ldw, static_cast<float*>(out), ldo, tokens, features, K, 0, 0, 0, bias, accumulate, scale);
   else if (!in_f32 && !out_f32)
     gemm_simt_kernel<bf16, bf16><<<grid, 256, 0, st>>>(static_cast<const bf16*>(x), ldx, static_cast<const bf16*>(w), ldw, static_cast<bf16*>(out), ldo, tokens, features, K, 0, 0, 0, bias, accumulate, scale);
@@ -303,8 +307,9 @@ extern "C" int pg_gemm_simt_batched(const void* x, long long ldx, long long batc
   if (grid.y > 65535) return PG_ERR_ARG;
   cudaStream_t st = PG_ST(stream);
   if (in_f32 && out_f32)
-    gemm_simt_kernel<float, float><<<grid, 256, 0, st>>>(static_cast<const float*>(x), ldx, static_cast<const float*>(w), ldw, static_cast<float*>(out), ldo, tokens, features, K, batch_x, batch_w, batch_out);
-  else if (!in_f32 && out_f32)
+    return pg_gemm_fp32(static_cast<const float*>(x), ldx, batch_x, static_cast<const float*>(w), ldw, batch_w, static_cast<float*>(out), ldo, batch_out, nullptr, 0, 1.0f, tokens,
+                        features, K, batch, st);
+  if (!in_f32 && out_f32)
     gemm_simt_kernel<bf16, float><<<grid, 256, 0, st>>>(static_cast<const bf16*>(x), ldx, static_cast<const bf16*>(w), ldw, static_cast<float*>(out), ldo, tokens, features, K, batch_x, batch_w, batch_out);
   else if (!in_f32 && !out_f32)
     gemm_simt_kernel<bf16, bf16><<<grid, 256, 0, st>>>(static_cast<const bf16*>(x), ldx, static_cast<const bf16*>(w), ldw, static_cast<bf16*>(out), ldo, tokens, features, K, batch_x, batch_w, batch_out);
