@@ -1,0 +1,31 @@
+// The tcgen05 product for a moderate number of tokens (gemm_cluster.cu): what gemm_tcgen05.cu needs to choose and launch it.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace pg {
+
+struct ClusterGemmArgs {
+  int tokens, features, K;
+  int mode, act;
+  float scale, glu_alpha;
+  void* out;
+  long long ldo;
+  const float* bias;
+  const float* resid;
+  long long ldr;
+  const int* out_row_map;
+  int resid_mod;
+  // set by the launcher
+  int tile_tokens, split, stages, smem_tiles;
+};
+
+// tokens per tile, CTAs that share K, and the estimated clocks of the launch
+struct ClusterGemmPlan {
+  int tile_tokens, split;
+  float clocks;
+};
+
+ClusterGemmPlan plan_cluster_gemm(int tokens, int features, int K);
+int launch_cluster_gemm(const ClusterGemmPlan& plan, const void* x, long long ldx, const void* w, long long ldw, ClusterGemmArgs a, cudaStream_t st);
+
+}  // namespace pg

@@ -16,6 +16,8 @@
 #include <cmath>
 
 #include "common.cuh"
+#include "gemm_act.cuh"
+#include "gemm_cluster.h"
 #include "paligemma_b200.h"
 #include "tmap.cuh"
 
@@ -127,26 +129,6 @@ PG_DEVINL TileInfo decode_tile(int tile, int m_blocks, int n_blocks, int total_k
   t.kb0 = split * kb_per;
   t.kb1 = min(total_kb, t.kb0 + kb_per);
   return t;
-}
-
-// activation of the bf16 epilogue (GemmArgs::act_gelu): 1 = gelu(tanh), 2 = relu(x)^2, 6 = gelu(erf)
-PG_DEVINL float epilogue_act(float x, int act) {
-  if (act == 2) { const float r = fmaxf(x, 0.f); return r * r; }
-  if (act == 6) return pg::gelu_erf(x);
-  return gelu_tanh_fast(x);
-}
-
-// gated unit of the GEGLU epilogue (GemmArgs::act_gelu in that mode): 0 / 1 gelu_tanh(g) * u; 3 silu(g) * u; 5 relu(g) * u;
-// 4 clamped: g' = min(g, c), u' = clamp(u, -c, c), g' * sigmoid(alpha * g') * (u' + 1) with c = GemmArgs::scale
-PG_DEVINL float glu_act(float g, float u, int kind, float limit, float alpha) {
-  if (kind == 3) return g / (1.0f + __expf(-g)) * u;
-  if (kind == 4) {
-    g = fminf(g, limit);
-    u = fminf(fmaxf(u, -limit), limit);
-    return g / (1.0f + __expf(-alpha * g)) * (u + 1.0f);
-  }
-  if (kind == 5) return fmaxf(g, 0.f) * u;
-  return gelu_tanh_fast(g) * u;
 }
 
 PG_DEVINL void named_bar_sync(int id, int nthreads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory"); }
@@ -1165,6 +1147,20 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& 
              ? PG_OK : PG_ERR_CUDA;
 }
 
+// Whether a token-major product takes the form of gemm_cluster.cu: up to 1408 tokens, but for plain epilogues that give the CTA-pair kernel one and
+// a half waves of 256 x 256 tiles.  Measured on both sides of the lines (us, this file's kernels / gemm_cluster.cu; N x K weights): 3456 x 1152
+// 263 tokens 14.4 / 8.2, 1024 17.0 / 10.8, 2048 20.2 / 22.2; 2048 x 2048 with residual 263 15.2 / 10.1, 1300 28.5 / 18.2; 2048 x 16384 with residual
+// 263 41 / 28, 1300 163 / 86, 2048 113 / 120; 32768 x 2048 gate || up 263 91 / 40, 1300 223 / 172; 5120 x 2048 1024 (80 pair tiles) 27.9 / 22.0, 1536
+// (120) 29.0 / 30.3; 8192 x 2048 706 (96) 28.6 / 23.4, 1024 (128) 29.3 / 31.5; 3072 x 768 1300 10.4 / 9.1, 1536 10.7 / 11.5.
+static bool cluster_form(const GemmArgs& a, long long ldr) {
+  auto aligned = [](const void* p, int n) { return (reinterpret_cast<uintptr_t>(p) & (n - 1)) == 0; };
+  // vectors of four: outputs, bias and residual rows
+  if (a.features % 4 != 0 || a.ldo % 4 != 0 || !aligned(a.out, 16) || !aligned(a.bias, 16)) return false;
+  if (a.resid != nullptr && (ldr % 4 != 0 || !aligned(a.resid, 16))) return false;
+  const int pair_tiles = ((a.tokens + 2 * BM - 1) / (2 * BM)) * ((a.features + 255) / 256);
+  return a.tokens <= 1408 && (a.mode == PG_EPI_GEGLU || pair_tiles < 3 * (num_sms() / 2) / 2);
+}
+
 }  // namespace pg
 
 using namespace pg;
@@ -1262,6 +1258,12 @@ extern "C" int pg_gemm_bf16_fused(const void* x, long long ldx, const void* w, l
       default: return launch<128, true>(ta, tb, a, tiles, st);
     }
   } else {
+    if (cluster_form(a, ldr)) {
+      ClusterGemmArgs c = {};
+      c.tokens = tokens; c.features = features; c.K = K; c.mode = mode; c.act = act_gelu; c.scale = scale; c.glu_alpha = a.glu_alpha;
+      c.out = out; c.ldo = ldo; c.bias = bias; c.resid = mode == PG_EPI_F32 ? resid : nullptr; c.ldr = ldr; c.out_row_map = a.out_row_map; c.resid_mod = a.resid_mod;
+      return launch_cluster_gemm(plan_cluster_gemm(tokens, features, K), x, ldx, w, ldw, c, st);
+    }
     // largest N tile that still gives the persistent grid ~a wave of CTAs (small token counts: latency path)
     const int m_blocks = (tokens + BM - 1) / BM;
     auto ntiles = [&](int bn) { return m_blocks * ((features + bn - 1) / bn) * split_k; };

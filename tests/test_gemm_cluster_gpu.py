@@ -1,0 +1,90 @@
+"""Products of a moderate number of tokens (gemm_cluster.cu, chosen by pg_gemm_bf16 for token-major calls) against 64-bit products.
+
+Bound per element: bf16 products are exact in fp32, the tensor core adds them with at most one unit in the last place per addition, so the sum is
+within K 2^-23 sum_k |x w|; an fp32 result adds four roundings, a bf16 result 2^-8 of itself, gelu / silu in their fast forms 2^-10 of the operands."""
+import pytest
+import torch
+
+from paligemma_multimodal_system_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+def _operands(T, F, K, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn(T, K, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(F, K, device="cuda", generator=g) * K ** -0.5).bfloat16()
+    b = torch.randn(F, device="cuda", generator=g)
+    xd, wd = x.double(), w.double()
+    return x, w, b, xd @ wd.T, K * 2.0 ** -23 * (xd.abs() @ wd.abs().T)
+
+
+def _check(got, want, bound):
+    assert got.isfinite().all()
+    assert ((got.double() - want).abs() <= bound).all()
+
+
+# token counts around the 16-, 32-, 128-, 256- and 384-token edges; feature and K tails; one to eight CTAs that share K
+@pytest.mark.parametrize("T", [1, 15, 16, 129, 255, 256, 257, 263, 384, 385, 770, 1408])
+@pytest.mark.parametrize("F,K", [(4, 8), (100, 64), (1152, 1152), (132, 72), (2048, 4304), (640, 520)])
+def test_fp32_bias_residual(T, F, K):
+    x, w, b, acc, bound = _operands(T, F, K, T + F)
+    h = torch.randn(T, F, device="cuda")
+    want = (acc + b.double()) * 0.5 + h.double()
+    out = _lib.gemm(x, w, h.clone(), mode=_lib.EPI_F32, bias=b, resid=h, scale=0.5, swap=0)
+    _check(out, want, bound + 2.0 ** -22 * (want.abs() + h.double().abs() + b.double().abs()))
+    more = _lib.gemm(x, w, h.clone(), mode=_lib.EPI_ATOMIC_F32, bias=b, scale=0.5, swap=0, split_k=3)
+    _check(more, want, bound + 2.0 ** -22 * (want.abs() + h.double().abs() + b.double().abs()))
+    assert torch.equal(out, _lib.gemm(x, w, h.clone(), mode=_lib.EPI_F32, bias=b, resid=h, scale=0.5, swap=0))
+
+
+@pytest.mark.parametrize("T", [130, 257, 300, 900])
+@pytest.mark.parametrize("act,f", [(0, lambda z: z), (1, lambda z: torch.nn.functional.gelu(z, approximate="tanh")), (2, lambda z: z.clamp(min=0) ** 2), (6, torch.nn.functional.gelu)])
+def test_bf16_activations(T, act, f):
+    x, w, b, acc, bound = _operands(T, 516, 696, T + act)
+    z = acc + b.double()
+    out = torch.full((T, 520), float("nan"), device="cuda", dtype=torch.bfloat16)
+    _lib.gemm(x, w, out[:, :516], mode=_lib.EPI_BF16, bias=b, act_gelu=act, swap=0)
+    slope = 1.2 if act != 2 else 2 * z.abs() + 1
+    _check(out[:, :516], f(z), bound * slope + 2.0 ** -8 * f(z).abs() + (2.0 ** -10 * z.abs() if act == 1 else 0) + 1e-6)
+    assert out[:, 516:].isnan().all()
+
+
+@pytest.mark.parametrize("T", [16, 200, 263, 1024])
+@pytest.mark.parametrize("kind", [_lib.GLU_GELU, _lib.GLU_SILU, _lib.GLU_CLAMPED, _lib.GLU_RELU])
+def test_gated_units(T, kind):
+    F, K = 384, 1032
+    x, w, b, acc, bound = _operands(T, F, K, T * 3 + kind)
+    z, e = (acc + b.double()).view(T, F // 128, 2, 64), bound.view(T, F // 128, 2, 64)
+    g, u = z[:, :, 0], z[:, :, 1]
+    limit, alpha = 1.5, 1.7
+    if kind == _lib.GLU_GELU:
+        want = torch.nn.functional.gelu(g, approximate="tanh") * u
+    elif kind == _lib.GLU_SILU:
+        want = g * torch.sigmoid(g) * u
+    elif kind == _lib.GLU_RELU:
+        want = g.clamp(min=0) * u
+    else:
+        gc, uc = g.clamp(max=limit), u.clamp(-limit, limit)
+        want = gc * torch.sigmoid(alpha * gc) * (uc + 1)
+    out = torch.empty(T, F // 2, device="cuda", dtype=torch.bfloat16)
+    _lib.gemm(x, w, out, mode=_lib.EPI_GEGLU, bias=b, act_gelu=kind, scale=limit if kind == _lib.GLU_CLAMPED else 1.0, glu_alpha=alpha, swap=0)
+    bound = 2 * (e[:, :, 0] * (u.abs() + 2) + e[:, :, 1] * (g.abs() + 2)) + 2.0 ** -8 * want.abs() + 2.0 ** -10 * (g * u).abs() + 2.0 ** -20 * (g.abs() + 1) * (u.abs() + 1)
+    _check(out, want.reshape(T, -1), bound.reshape(T, -1))
+
+
+@pytest.mark.parametrize("T", [140, 512])
+def test_row_map_and_table(T):
+    F, K, N = 256, 640, 70
+    x, w, b, acc, bound = _operands(T, F, K, T)
+    rows = torch.randperm(T + 9, device="cuda")[:T].to(torch.int32)
+    out = torch.full((T + 9, F), float("nan"), device="cuda")
+    _lib.gemm(x, w, out, mode=_lib.EPI_F32, bias=b, scale=0.25, swap=0, out_row_map=rows)
+    want = (acc + b.double()) * 0.25
+    _check(out[rows.long()], want, bound + 2.0 ** -22 * (want.abs() + b.double().abs()))
+    assert int(out.isnan().all(1).sum()) == 9
+    table = torch.randn(N, F, device="cuda")
+    out = torch.empty(T, F, device="cuda")
+    _lib.gemm(x, w, out, mode=_lib.EPI_F32, bias=b, resid=table, resid_row_mod=N, swap=0)
+    want = acc + b.double() + table.double()[torch.arange(T, device="cuda") % N]
+    _check(out, want, bound + 2.0 ** -21 * (want.abs() + 4))
