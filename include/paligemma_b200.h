@@ -101,6 +101,47 @@ int pg_gemm_bf16_fused(const void* x, long long ldx, const void* w, long long ld
                        const float* bias, const float* resid, long long ldr, int tokens, int features, int K, int mode,
                        int act_gelu, float scale, int swap, int split_k, const PgGemmFusion* fusion, void* stream);
 
+/* h[t,f] += (sum_k x[t,k] w[f,k] + bias[f]) * scale (h fp32): a projection that ends in the residual stream.  Few output tiles: K is split over CTAs. */
+int pg_gemm_residual(const void* x, long long ldx, const void* w, long long ldw, float* h, long long ldh, const float* bias, int tokens, int features,
+                     int K, float scale, void* stream);
+
+/* The encoder layers of the vision tower (modeling_siglip.py:216-263): seven launches each, issued by one call.  Weights as the entry points above take
+ * them (matrices bf16, dense rows; q | k | v projections fused), x fp32 [images * patches, D] in place; hn, att bf16 [., D], qkv bf16 [., 3 D],
+ * mid bf16 [., F] are scratch. */
+typedef struct {
+  const float *ln1_w, *ln1_b;
+  const void* qkv_w;
+  const float* qkv_b;
+  const void* out_w;
+  const float *out_b, *ln2_w, *ln2_b;
+  const void* fc1_w;
+  const float* fc1_b;
+  const void* fc2_w;
+  const float* fc2_b;
+} PgSiglipLayer;
+int pg_siglip_layers(const PgSiglipLayer* layers, int count, float* x, void* hn, void* qkv, void* att, void* mid, int images, int patches, int D, int F,
+                     int heads, float eps, void* stream);
+
+/* The decoder layers of a prompt pass (modeling_gemma.py:385-418): h fp32 [B * S, D] in place.  fused: RoPE and KV append in the q/k/v projection's
+ * epilogue (q, k, v unused), else bf16 scratch q [B*S, Hq*dh], k, v [B*S, Hkv*dh].  k_pages / v_pages: pages of layer 0 (NULL: no cache), those of
+ * layer i layer_bytes * i further on.  lens: int32 [B] prompt lengths of a ragged batch, or NULL. */
+typedef struct {
+  const float *ln1, *ln2;
+  const void *qkv_w, *o_w, *gu_w, *down_w;
+} PgGemmaLayer;
+typedef struct {
+  float* h;
+  void *hn, *qkv, *q, *k, *v, *att, *mid;
+  const int* pos;
+  const float* inv_freq;
+  void *k_pages, *v_pages;
+  long long layer_bytes;
+  const int *page_table, *slot_base, *lens;
+  int B, S, D, F, Hq, Hkv, dh, page, max_pages, fused;
+  float eps;
+} PgGemmaPrefill;
+int pg_gemma_prefill_layers(const PgGemmaLayer* layers, int count, const PgGemmaPrefill* args, void* stream);
+
 /*
  * Prefill q/k/v projection with RoPE and the KV-cache append in the GEMM epilogue (modeling_gemma.py:274-302 + KVCache.update
  * :18-57): qkv_out[t, :] = bf16 of [rope(q heads) | rope(k heads) | v heads] of x[t, :] @ w^T, w = [q_proj; k_proj; v_proj]

@@ -13,7 +13,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("PG_LIB_PATH") or os.path.join(_HERE, "libpaligemma_b200.so")  # PG_LIB_PATH: A/B builds (profiling)
 
 EPI_BF16, EPI_F32, EPI_ATOMIC_F32, EPI_GEGLU = 0, 1, 2, 3
-ABI_VERSION = 6  # pg_abi_version() of the library these signatures describe
+ABI_VERSION = 7  # pg_abi_version() of the library these signatures describe
 
 _ERRORS = {-1: "PG_ERR_ARG", -2: "PG_ERR_CUDA", -3: "PG_ERR_DRIVER", -4: "PG_ERR_TMAP", -5: "PG_ERR_ARCH"}
 
@@ -40,6 +40,9 @@ SIGNATURES = {
     "pg_debug_set_topp_bracket": [i32],
     "pg_gemm_bf16": [p, i64, p, i64, p, i64, p, p, i64, i32, i32, i32, i32, i32, f32, i32, i32, p],
     "pg_gemm_bf16_fused": [p, i64, p, i64, p, i64, p, p, i64, i32, i32, i32, i32, i32, f32, i32, i32, p, p],
+    "pg_gemm_residual": [p, i64, p, i64, p, i64, p, i32, i32, i32, f32, p],
+    "pg_siglip_layers": [p, i32, p, p, p, p, p, i32, i32, i32, i32, i32, f32, p],
+    "pg_gemma_prefill_layers": [p, i32, p, p],
     "pg_gemm_qkv_rope": [p, i64, p, i64, p, i64, i32, i32, i32, i32, i32, p, p, p, p, p, p, i32, i32, i32, p],
     "pg_pack_gate_up": [p, p, p, i32, i32, p],
     "pg_cast_f32_bf16": [p, p, i64, p],
@@ -154,6 +157,28 @@ class GemmFusion(C.Structure):
     ]
 
 
+class SiglipLayer(C.Structure):
+    """Mirror of PgSiglipLayer."""
+    _fields_ = [(n, p) for n in ("ln1_w", "ln1_b", "qkv_w", "qkv_b", "out_w", "out_b", "ln2_w", "ln2_b", "fc1_w", "fc1_b", "fc2_w", "fc2_b")]
+
+
+class GemmaLayer(C.Structure):
+    """Mirror of PgGemmaLayer."""
+    _fields_ = [(n, p) for n in ("ln1", "ln2", "qkv_w", "o_w", "gu_w", "down_w")]
+
+
+class GemmaPrefill(C.Structure):
+    """Mirror of PgGemmaPrefill."""
+    _fields_ = ([(n, p) for n in ("h", "hn", "qkv", "q", "k", "v", "att", "mid", "pos", "inv_freq", "k_pages", "v_pages")] + [("layer_bytes", i64)]
+                + [(n, p) for n in ("page_table", "slot_base", "lens")]
+                + [(n, i32) for n in ("B", "S", "D", "F", "Hq", "Hkv", "dh", "page", "max_pages", "fused")] + [("eps", f32)])
+
+
+def layer_array(kind, layers):
+    """ctypes array of `kind` from the packed tensors of every layer (dicts with the struct's field names; they must outlive the array)."""
+    return (kind * len(layers))(*[kind(*[l[n].data_ptr() for n, _ in kind._fields_]) for l in layers])
+
+
 _lib = None
 
 
@@ -187,7 +212,10 @@ def check(rc, what):
 
 
 def stream():
-    return torch.cuda.current_stream().cuda_stream
+    """Raw handle of the current stream (torch.cuda.current_stream() builds a stream object: 3.2 us of the 9 .. 13 us a launch costs from here)."""
+    if not torch.cuda.is_initialized():
+        torch.cuda.init()
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def ptr(t):
@@ -283,22 +311,9 @@ def gemm_residual(x, w, h, bias=None, scale=1.0):
     """h += (x @ w.T + bias) * scale: the residual-stream GEMMs (out_proj / fc2 / o_proj / down_proj).  With enough output tiles
     the epilogue adds the fp32 residual in place; with few tiles (small token counts: latency path, decode) the K
     dimension is split over CTAs and the partials are red.add-ed into h so that the whole GPU streams the weights."""
-    T, K = x.shape
-    F = w.shape[0]
-    swap = 1 if T <= 128 else 0
-    kb = (K + 63) // 64
-    if swap:
-        tiles = (F + 127) // 128
-    else:
-        tiles = ((T + 127) // 128) * ((F + 255) // 256)
-        if kb < 128:
-            # few-token prefill (latency path), short/medium K: count 128x64 tiles -- the kernel narrows its N tile before
-            # the host splits K, because every split costs a full fp32 red.add pass over the output tile (measured at
-            # T = 256: fc2 14 splits x 256 columns 34 us -> 4 splits x 64 columns 15.6 us; o_proj 6 splits 25.6 -> 1 split
-            # 15.4 us).  Long reductions (down_proj, K = 16384) keep wide tiles + splits: 64-column tiles re-read the
-            # activation tile from L2 too often.
-            tiles = ((T + 127) // 128) * ((F + 63) // 64)
-    if tiles >= 96 or kb < 8 or T > 512:  # (large-batch prefill keeps the deterministic, atomics-free epilogue)
-        return gemm(x, w, h, mode=EPI_F32, bias=bias, resid=h, swap=swap, scale=scale)
-    split = max(1, min(kb // 4, (2 * 148 if swap else 148) // tiles))
-    return gemm(x, w, h, mode=EPI_ATOMIC_F32, bias=bias, swap=swap, split_k=split, scale=scale)
+    assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.is_cuda and w.is_cuda and x.stride(1) == 1 and w.stride(1) == 1
+    assert h.dtype == torch.float32 and h.stride(-1) == 1 and x.shape[1] == w.shape[1] and h.shape == (x.shape[0], w.shape[0])
+    assert bias is None or (bias.dtype == torch.float32 and bias.is_contiguous())
+    check(lib().pg_gemm_residual(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), h.data_ptr(), h.stride(0), ptr(bias), x.shape[0], w.shape[0], x.shape[1],
+                                 float(scale), stream()), "pg_gemm_residual")
+    return h

@@ -1,0 +1,91 @@
+// Whole runs of layers issued by one call: the launches of a SigLIP encoder or of a Gemma prompt pass are the same few per layer, and issuing each
+// from Python costs 9 .. 13 us (argument checks, tensor metadata, the foreign call) where the launch itself costs 3 and the kernels of one
+// image take 4 .. 10.  No kernels here.
+#include <cmath>
+
+#include "common.cuh"
+#include "paligemma_b200.h"
+
+extern "C" int pg_gemm_residual(const void* x, long long ldx, const void* w, long long ldw, float* h, long long ldh, const float* bias, int tokens,
+                                int features, int K, float scale, void* stream) {
+  if (tokens <= 0 || features <= 0 || K <= 0) return PG_ERR_ARG;
+  const int swap = tokens <= 128 ? 1 : 0, kb = (K + 63) / 64;
+  int tiles;
+  if (swap) {
+    tiles = (features + 127) / 128;
+  } else if (kb < 128) {
+    // short and medium K: count 128 x 64 tiles -- the kernel narrows its N tile before K is split, because every split costs a full
+    // fp32 red.add pass over the output tile
+    tiles = ((tokens + 127) / 128) * ((features + 63) / 64);
+  } else {
+    tiles = ((tokens + 127) / 128) * ((features + 255) / 256);
+  }
+  if (tiles >= 96 || kb < 8 || tokens > 512)
+    return pg_gemm_bf16(x, ldx, w, ldw, h, ldh, bias, h, ldh, tokens, features, K, PG_EPI_F32, 0, scale, swap, 1, stream);
+  int split = (swap ? 2 * 148 : 148) / tiles;
+  if (split > kb / 4) split = kb / 4;
+  return pg_gemm_bf16(x, ldx, w, ldw, h, ldh, bias, nullptr, 0, tokens, features, K, PG_EPI_ATOMIC_F32, 0, scale, swap, split < 1 ? 1 : split, stream);
+}
+
+#define PG_TRY(call)                  \
+  do {                                \
+    const int rc_ = (call);           \
+    if (rc_ != PG_OK) return rc_;     \
+  } while (0)
+
+extern "C" int pg_siglip_layers(const PgSiglipLayer* layers, int count, float* x, void* hn, void* qkv, void* att, void* mid, int images, int patches,
+                                int D, int F, int heads, float eps, void* stream) {
+  if (layers == nullptr || count < 0 || images <= 0 || patches <= 0 || heads <= 0 || D <= 0 || D % heads != 0) return PG_ERR_ARG;
+  const int M = images * patches, dh = D / heads;
+  const long long N = patches, D3 = 3LL * D;
+  const char* q = static_cast<const char*>(qkv);
+  for (int i = 0; i < count; ++i) {
+    const PgSiglipLayer& l = layers[i];
+    PG_TRY(pg_layernorm(x, l.ln1_w, l.ln1_b, hn, nullptr, M, D, eps, stream));
+    PG_TRY(pg_gemm_bf16(hn, D, l.qkv_w, D, qkv, D3, l.qkv_b, nullptr, 0, M, 3 * D, D, PG_EPI_BF16, 0, 1.f, 0, 1, stream));
+    PG_TRY(pg_attention_prefill(q, q + 2LL * D, q + 4LL * D, att, images, heads, patches, patches, dh, 1, N * D3, D3, 0, dh, N * D3, D3, dh, N * D, D, 0,
+                                dh, static_cast<float>(1.0 / std::sqrt(static_cast<double>(dh))), stream));
+    PG_TRY(pg_gemm_residual(att, D, l.out_w, D, x, D, l.out_b, M, D, D, 1.f, stream));
+    PG_TRY(pg_layernorm(x, l.ln2_w, l.ln2_b, hn, nullptr, M, D, eps, stream));
+    PG_TRY(pg_gemm_bf16(hn, D, l.fc1_w, D, mid, F, l.fc1_b, nullptr, 0, M, F, D, PG_EPI_BF16, 1, 1.f, 0, 1, stream));
+    PG_TRY(pg_gemm_residual(mid, F, l.fc2_w, F, x, D, l.fc2_b, M, D, F, 1.f, stream));
+  }
+  return PG_OK;
+}
+
+extern "C" int pg_gemma_prefill_layers(const PgGemmaLayer* layers, int count, const PgGemmaPrefill* a, void* stream) {
+  if (layers == nullptr || a == nullptr || count < 0 || a->B <= 0 || a->S <= 0 || a->Hkv <= 0 || a->Hq % a->Hkv != 0) return PG_ERR_ARG;
+  const int T = a->B * a->S, D = a->D, F = a->F, Hq = a->Hq, Hkv = a->Hkv, dh = a->dh, G = Hq / Hkv, swap = T > 128 ? 0 : 1;
+  const long long W = (Hq + 2LL * Hkv) * dh, S = a->S, qs = a->fused ? W : (long long)Hq * dh, kvs = a->fused ? W : (long long)Hkv * dh, os = (long long)Hq * dh;
+  const char* qkv = static_cast<const char*>(a->qkv);
+  const void* q = a->fused ? qkv : a->q;
+  const void* k = a->fused ? qkv + 2LL * Hq * dh : a->k;
+  const void* v = a->fused ? qkv + 2LL * (Hq + Hkv) * dh : a->v;
+  const float scale = static_cast<float>(1.0 / std::sqrt(static_cast<double>(dh)));
+  for (int i = 0; i < count; ++i) {
+    const PgGemmaLayer& l = layers[i];
+    void* kp = a->k_pages == nullptr ? nullptr : static_cast<char*>(a->k_pages) + i * a->layer_bytes;
+    void* vp = a->v_pages == nullptr ? nullptr : static_cast<char*>(a->v_pages) + i * a->layer_bytes;
+    PG_TRY(pg_rmsnorm(a->h, l.ln1, a->hn, T, D, a->eps, stream));
+    if (a->fused) {
+      PG_TRY(pg_gemm_qkv_rope(a->hn, D, l.qkv_w, D, a->qkv, W, T, D, Hq, Hkv, dh, a->pos, a->inv_freq, kp, vp, a->page_table, a->slot_base, a->S, a->page,
+                              a->max_pages, stream));
+    } else {
+      PG_TRY(pg_gemm_bf16(a->hn, D, l.qkv_w, D, a->qkv, W, nullptr, nullptr, 0, T, static_cast<int>(W), D, PG_EPI_BF16, 0, 1.f, swap, 1, stream));
+      PG_TRY(pg_rope_kv_append(a->qkv, 0, a->pos, a->q, a->k, a->v, kp, vp, a->page_table, a->slot_base, a->B, a->S, Hq, Hkv, dh, a->page, a->max_pages,
+                               a->inv_freq, stream));
+    }
+    // the G query heads of a k/v head are consecutive rows of one attention problem
+    if (a->lens == nullptr)
+      PG_TRY(pg_attention_prefill(q, k, v, a->att, a->B, Hkv, a->S * G, a->S, dh, G, S * qs, qs, dh, (long long)G * dh, S * kvs, kvs, dh, S * os, os, dh,
+                                  (long long)G * dh, scale, stream));
+    else
+      PG_TRY(pg_attention_prefill_varlen(q, k, v, a->att, a->lens, a->B, Hkv, a->S * G, a->S, dh, G, S * qs, qs, dh, (long long)G * dh, S * kvs, kvs, dh, S * os,
+                                         os, dh, (long long)G * dh, scale, stream));
+    PG_TRY(pg_gemm_residual(a->att, os, l.o_w, os, a->h, D, nullptr, T, D, static_cast<int>(os), 1.f, stream));
+    PG_TRY(pg_rmsnorm(a->h, l.ln2, a->hn, T, D, a->eps, stream));
+    PG_TRY(pg_gemm_bf16(a->hn, D, l.gu_w, D, a->mid, F, nullptr, nullptr, 0, T, 2 * F, D, PG_EPI_GEGLU, 0, 1.f, swap, 1, stream));
+    PG_TRY(pg_gemm_residual(a->mid, F, l.down_w, F, a->h, D, nullptr, T, D, F, 1.f, stream));
+  }
+  return PG_OK;
+}

@@ -8,6 +8,7 @@ Compute path per layer (all through the C ABI of include/paligemma_b200.h):
             residual stream, and split-KV attention over the paged bf16 cache.
 The residual stream is fp32 (as in the reference); GEMM operands are bf16.
 """
+import ctypes as C
 import math
 import os
 from typing import List, Optional, Tuple
@@ -263,6 +264,7 @@ class GemmaForCausalLM(nn.Module):
                 qkv_w=torch.cat([_bf16(a.q_proj.weight), _bf16(a.k_proj.weight), _bf16(a.v_proj.weight)], 0).contiguous(),
                 o_w=_bf16(a.o_proj.weight), gu_w=gu, down_w=_bf16(l.mlp.down_proj.weight)))
             del gate, up
+        pk["array"] = _lib.layer_array(_lib.GemmaLayer, pk["layers"])
         torch.cuda.synchronize()
         self._packed = pk
         return pk
@@ -301,52 +303,24 @@ class GemmaForCausalLM(nn.Module):
         qkv = torch.empty(T, W, device=dev, dtype=torch.bfloat16)
         att = torch.empty(T, Hq * dh, device=dev, dtype=torch.bfloat16)
         mid = torch.empty(T, F, device=dev, dtype=torch.bfloat16)
-        G = Hq // Hkv
-        scale = 1.0 / math.sqrt(dh)
         # RoPE + KV append in the q/k/v projection's epilogue (one head per 128 x dh output tile) once that grid fills the GPU;
         # few-token prefills (latency path) keep narrower GEMM tiles and the separate RoPE / append launch
         fused = self.fused_qkv_rope
         if fused is None:
             fused = dh in (64, 256) and ((T + 127) // 128) * (Hq + 2 * Hkv) >= 96
-        if fused:
-            # q, k, v are column slices of `qkv` (token pitch W): the attention's tensor maps take the strides
-            q, k, v = qkv, qkv[:, Hq * dh:], qkv[:, (Hq + Hkv) * dh:]
-            q_ts = kv_ts = W
-        else:
+        # fused: q, k, v are column slices of `qkv` (token pitch W), the attention's tensor maps take the strides
+        q = k = v = None
+        if not fused:
             q = torch.empty(T, Hq * dh, device=dev, dtype=torch.bfloat16)
             k = torch.empty(T, Hkv * dh, device=dev, dtype=torch.bfloat16)
             v = torch.empty(T, Hkv * dh, device=dev, dtype=torch.bfloat16)
-            q_ts, kv_ts = Hq * dh, Hkv * dh
-        for li, lw in enumerate(pk["layers"]):
-            _lib.rmsnorm(h, lw["ln1"], hn)
-            kp = kv_cache.k_pages[li].data_ptr() if have_cache else 0
-            vp = kv_cache.v_pages[li].data_ptr() if have_cache else 0
-            pt = page_table.data_ptr() if have_cache else 0
-            sb = slot_base.data_ptr() if have_cache else 0
-            mp = page_table.shape[1] if have_cache else 0
-            if fused:
-                _lib.check(L.pg_gemm_qkv_rope(hn.data_ptr(), D, lw["qkv_w"].data_ptr(), D, qkv.data_ptr(), W, T, D, Hq, Hkv, dh,
-                                              pos.data_ptr(), pk["inv_freq"].data_ptr(), kp, vp, pt, sb, S, PAGE, mp, st),
-                           "pg_gemm_qkv_rope")
-            else:
-                _lib.gemm(hn, lw["qkv_w"], qkv, mode=_lib.EPI_BF16, swap=0 if T > 128 else 1)
-                _lib.check(L.pg_rope_kv_append(qkv.data_ptr(), 0, pos.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), kp, vp, pt, sb,
-                                               B, S, Hq, Hkv, dh, PAGE, mp, pk["inv_freq"].data_ptr(), st), "pg_rope_kv_append")
-            # MQA/GQA: the G query heads of a KV head are consecutive rows of one attention problem (no repeat_kv)
-            if lens is None:
-                _lib.check(L.pg_attention_prefill(
-                    q.data_ptr(), k.data_ptr(), v.data_ptr(), att.data_ptr(), B, Hkv, S * G, S, dh, G,
-                    S * q_ts, q_ts, dh, G * dh, S * kv_ts, kv_ts, dh,
-                    S * Hq * dh, Hq * dh, dh, G * dh, scale, st), "pg_attention_prefill")
-            else:
-                _lib.check(L.pg_attention_prefill_varlen(
-                    q.data_ptr(), k.data_ptr(), v.data_ptr(), att.data_ptr(), lens.data_ptr(), B, Hkv, S * G, S, dh, G,
-                    S * q_ts, q_ts, dh, G * dh, S * kv_ts, kv_ts, dh,
-                    S * Hq * dh, Hq * dh, dh, G * dh, scale, st), "pg_attention_prefill_varlen")
-            _lib.gemm_residual(att, lw["o_w"], h)
-            _lib.rmsnorm(h, lw["ln2"], hn)
-            _lib.gemm(hn, lw["gu_w"], mid, mode=_lib.EPI_GEGLU, swap=0 if T > 128 else 1)
-            _lib.gemm_residual(mid, lw["down_w"], h)
+        assert h.dtype == torch.float32 and h.is_contiguous() and h.numel() == T * D
+        kp = kv_cache.k_pages if have_cache else None
+        args = _lib.GemmaPrefill(h.data_ptr(), hn.data_ptr(), qkv.data_ptr(), _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), att.data_ptr(), mid.data_ptr(), pos.data_ptr(),
+                                 pk["inv_freq"].data_ptr(), _lib.ptr(kp), _lib.ptr(kv_cache.v_pages) if have_cache else 0,
+                                 kp.stride(0) * kp.element_size() if have_cache else 0, _lib.ptr(page_table), slot_base.data_ptr() if have_cache else 0,
+                                 _lib.ptr(lens), B, S, D, F, Hq, Hkv, dh, PAGE, page_table.shape[1] if have_cache else 0, int(fused), 1e-6)
+        _lib.check(L.pg_gemma_prefill_layers(C.addressof(pk["array"]), len(pk["layers"]), C.addressof(args), st), "pg_gemma_prefill_layers")
         if have_cache and page_rows is None:
             kv_cache._set_len(S, c.num_hidden_layers)
         if last_only:

@@ -10,6 +10,8 @@ packs the parameters once (bf16, fused QKV) and runs
 
 through the C ABI (include/paligemma_b200.h).  The residual stream stays fp32 as in the reference.
 """
+import ctypes as C
+
 import torch
 import torch.nn as nn
 
@@ -139,6 +141,7 @@ class SiglipVisionModel(nn.Module):
                 ln2_w=_f32(l.layer_norm2.weight), ln2_b=_f32(l.layer_norm2.bias),
                 fc1_w=_bf16(l.mlp.fc1.weight), fc1_b=_f32(l.mlp.fc1.bias),
                 fc2_w=_bf16(l.mlp.fc2.weight), fc2_b=_f32(l.mlp.fc2.bias)))
+        pk["array"] = _lib.layer_array(_lib.SiglipLayer, pk["layers"])
         self._packed = pk
         return pk
 
@@ -152,16 +155,15 @@ class SiglipVisionModel(nn.Module):
         L = _lib.lib()
         st = _lib.stream()
         px = pixel_values.to(device="cuda", dtype=torch.float32).contiguous()
-        B, C, H, W = px.shape
-        if C != c.num_channels or H != c.image_size or W != c.image_size:
+        B, channels, H, W = px.shape
+        if channels != c.num_channels or H != c.image_size or W != c.image_size:
             raise ValueError(f"pixel_values must be [B,{c.num_channels},{c.image_size},{c.image_size}], got {tuple(px.shape)}")
         P, Dv, Fv, Hh = c.patch_size, c.hidden_size, c.intermediate_size, c.num_attention_heads
-        dh = Dv // Hh
         N = (H // P) * (W // P)
         M = B * N
         dev = px.device
         patches = torch.empty(M, pk["Kp"], device=dev, dtype=torch.bfloat16)
-        _lib.check(L.pg_im2col(px.data_ptr(), patches.data_ptr(), B, C, H, W, P, pk["Kp"], st), "pg_im2col")
+        _lib.check(L.pg_im2col(px.data_ptr(), patches.data_ptr(), B, channels, H, W, P, pk["Kp"], st), "pg_im2col")
         x = torch.empty(M, Dv, device=dev, dtype=torch.float32)
         # conv-as-GEMM with bias and the position embeddings (row n of the table for token b*N + n) in one epilogue
         _lib.gemm(patches, pk["patch_w"], x, mode=_lib.EPI_F32, bias=pk["patch_b"], resid=pk["pos"], resid_row_mod=N, swap=0)
@@ -169,17 +171,8 @@ class SiglipVisionModel(nn.Module):
         qkv = torch.empty(M, 3 * Dv, device=dev, dtype=torch.bfloat16)
         att = torch.empty(M, Dv, device=dev, dtype=torch.bfloat16)
         mid = torch.empty(M, Fv, device=dev, dtype=torch.bfloat16)
-        scale = 1.0 / (dh ** 0.5)
-        for lw in pk["layers"]:
-            _lib.layernorm(x, lw["ln1_w"], lw["ln1_b"], c.layer_norm_eps, out_bf16=h)
-            _lib.gemm(h, lw["qkv_w"], qkv, mode=_lib.EPI_BF16, bias=lw["qkv_b"], swap=0)
-            _lib.check(L.pg_attention_prefill(
-                qkv.data_ptr(), qkv.data_ptr() + 2 * Dv, qkv.data_ptr() + 4 * Dv, att.data_ptr(), B, Hh, N, N, dh, 1,
-                N * 3 * Dv, 3 * Dv, 0, dh, N * 3 * Dv, 3 * Dv, dh, N * Dv, Dv, 0, dh, scale, st), "pg_attention_prefill")
-            _lib.gemm_residual(att, lw["out_w"], x, bias=lw["out_b"])
-            _lib.layernorm(x, lw["ln2_w"], lw["ln2_b"], c.layer_norm_eps, out_bf16=h)
-            _lib.gemm(h, lw["fc1_w"], mid, mode=_lib.EPI_BF16, bias=lw["fc1_b"], act_gelu=True, swap=0)
-            _lib.gemm_residual(mid, lw["fc2_w"], x, bias=lw["fc2_b"])
+        _lib.check(L.pg_siglip_layers(C.addressof(pk["array"]), len(pk["layers"]), x.data_ptr(), h.data_ptr(), qkv.data_ptr(), att.data_ptr(), mid.data_ptr(), B, N,
+                                      Dv, Fv, Hh, float(c.layer_norm_eps), st), "pg_siglip_layers")
         if out_bf16:
             _lib.layernorm(x, pk["post_w"], pk["post_b"], c.layer_norm_eps, out_bf16=h)
             return h
