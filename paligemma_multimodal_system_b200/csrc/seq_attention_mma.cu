@@ -11,6 +11,13 @@
 // mma.sync.m16n8k16 fragments: S accumulators of two adjacent 8-key blocks are, element for element, the A operand of one
 // 16-key step of P V, so P never leaves the registers.  (tcgen05 would want P in shared or tensor memory as bf16; three
 // passes from there cost the round trips this kernel avoids.)
+//
+// What bounds it: instruction issue (ncu: 47 % of the slots, 16 warps per SM by registers) beside a tensor pipe at half its mma.sync rate.  So what
+// is not arithmetic is kept out of the key loop: one page lookup per tile, a tile ahead, with constant row steps (a division and a lookup per
+// 16-byte chunk cost as much as the softmax); K fragments by ldmatrix; masks only on the tiles that have an edge; one FMA and one ex2 per score when
+// there is no cap or penalty; the exact split of P by byte permutation; products ordered so that neighbours go to different accumulators; the
+// longest rows first.  8 prompts of 1024 tokens, 32 heads x 64 over 8 k/v heads: 524 -> 245 us (softcap 629 -> 309); 2 portions of 333 tokens behind 1400,
+// 32 heads x 96 / 64: 295 -> 132 us.
 #include "common.cuh"
 #include "paligemma_b200.h"
 
@@ -19,9 +26,9 @@ using bf16 = __nv_bfloat16;
 namespace {
 
 __device__ __forceinline__ void mma16816(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
 // four 8 x 8 bf16 matrices from shared memory, transposed: key-major value rows -> the k-pairs an m16n8k16 B fragment wants
@@ -36,26 +43,41 @@ __device__ __forceinline__ void cp_async16(bf16* smem_dst, const bf16* gmem_src)
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(a), "l"(gmem_src) : "memory");
 }
 
+// 2^x by the hardware approximation (results below 2^-126 become 0, 2^-inf = 0)
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 // tanh to fp32 accuracy without the library's slow path: odd series below 0.1 (next term 17 x^7 / 315 < 6e-10), else
 // 1 - 2 / (exp(2|x|) + 1), whose absolute error of ~1e-7 is relative there as well
 __device__ __forceinline__ float tanh32(float x) {
   const float ax = fabsf(x), x2 = x * x;
   const float small = x * fmaf(x2, fmaf(x2, 0.13333333f, -0.33333334f), 1.0f);
-  const float big = copysignf(1.0f - __fdividef(2.0f, exp2f(ax * 2.885390082f) + 1.0f), x);
+  const float big = copysignf(1.0f - __fdividef(2.0f, ex2(ax * 2.885390082f) + 1.0f), x);
   return ax < 0.1f ? small : big;
 }
 
-// p = hi + mid + lo with bf16 terms (round to nearest each time; the remainders are exact in fp32)
+// four 8 x 8 bf16 matrices: key-major key rows -> the B fragments of S = Q K^T
+__device__ __forceinline__ void ldmatrix_x4(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, const bf16* p) {
+  const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p));
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(a));
+}
+
+template <int N>
+struct Int { static constexpr int value = N; };
+
+// p = hi + mid + lo exactly: the upper halves of p, of the remainder and of the remainder's remainder (8 + 8 + 8 mantissa bits, truncated, so
+// packing is a byte permutation and nothing is converted)
 __device__ __forceinline__ void split3(float p, float q, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  const __nv_bfloat162 h = __floats2bfloat162_rn(p, q);
-  const float2 hf = __bfloat1622float2(h);
-  const float rp = p - hf.x, rq = q - hf.y;
-  const __nv_bfloat162 m = __floats2bfloat162_rn(rp, rq);
-  const float2 mf = __bfloat1622float2(m);
-  const __nv_bfloat162 l = __floats2bfloat162_rn(rp - mf.x, rq - mf.y);
-  hi = *reinterpret_cast<const uint32_t*>(&h);
-  mid = *reinterpret_cast<const uint32_t*>(&m);
-  lo = *reinterpret_cast<const uint32_t*>(&l);
+  const uint32_t up = __float_as_uint(p), uq = __float_as_uint(q);
+  hi = __byte_perm(up, uq, 0x7632);
+  const float rp = p - __uint_as_float(up & 0xffff0000u), rq = q - __uint_as_float(uq & 0xffff0000u);
+  const uint32_t vp = __float_as_uint(rp), vq = __float_as_uint(rq);
+  mid = __byte_perm(vp, vq, 0x7632);
+  const float sp = rp - __uint_as_float(vp & 0xffff0000u), sq = rq - __uint_as_float(vq & 0xffff0000u);
+  lo = __byte_perm(__float_as_uint(sp), __float_as_uint(sq), 0x7632);
 }
 
 template <int DIM, int VDIM, bool LOGI>
@@ -71,7 +93,7 @@ __global__ void __launch_bounds__(128, (DIM + VDIM <= 128) ? 4 : 2) attn_ragged_
   const int n = entry_n[e], ctx = entry_ctx[e], row0 = entry_row0[e];
   if (skip_single && n == 1) return;
   const int rows = n * gsz;
-  const int r0 = blockIdx.x * 64;
+  const int r0 = (gridDim.x - 1 - blockIdx.x) * 64;  // the longest rows start first
   if (r0 >= rows) return;
   extern __shared__ __align__(16) unsigned char smraw[];
   bf16* Qs = reinterpret_cast<bf16*>(smraw);  // [64][QP]
@@ -125,29 +147,47 @@ __global__ void __launch_bounds__(128, (DIM + VDIM <= 128) ? 4 : 2) attn_ragged_
   const long long krow = (long long)G * DIM, vrow = (long long)G * VDIM;
   // K / V tiles go through two buffers: the next tile is in flight (cp.async) while this one is multiplied; rows past the last
   // key any row of the CTA sees are zero (a masked probability times a stale value must stay zero)
-  auto fetch = [&](int k0, int buf) {
-    bf16* Kd = Kb + buf * 64 * QP;
-    bf16* Vd = Vb + buf * 64 * VLD;
-    for (int id = threadIdx.x; id < 64 * (DIM / 8); id += 128) {
-      const int r = id / (DIM / 8), cc = id % (DIM / 8), j = k0 + r;
-      bf16* d = Kd + r * QP + cc * 8;
-      if (j <= kmax) cp_async16(d, k_pages + ((long long)pt[j / page] * page + j % page) * krow + (long long)g * DIM + cc * 8);
-      else *reinterpret_cast<uint4*>(d) = make_uint4(0, 0, 0, 0);
+  // (a tile starts on a multiple of 64: pages of 64 rows are tiles; page_at is read a tile ahead)
+  const bool page_is_tile = page == 64;
+  auto page_at = [&](int k0) { return page_is_tile && k0 <= kmax ? pt[k0 >> 6] : 0; };
+  auto rows_of = [&](auto width, bf16* d, const bf16* pages, long long row, int head0, int k0, int at) {
+    constexpr int CPR = decltype(width)::value / 8, PITCH = decltype(width)::value + 8;  // 16-byte chunks per row
+    if (128 % CPR == 0 && page_is_tile && k0 + 63 <= kmax) {
+      constexpr int RPP = 128 % CPR == 0 ? 128 / CPR : 1;
+      const int r = threadIdx.x / CPR, cc = (threadIdx.x % CPR) * 8;
+      const bf16* src = pages + ((long long)at * 64 + r) * row + head0 + cc;
+      bf16* dst = d + r * PITCH + cc;
+#pragma unroll
+      for (int i = 0; i < 64 / RPP; ++i, src += RPP * row) cp_async16(dst + i * RPP * PITCH, src);
+      return;
     }
-    for (int id = threadIdx.x; id < 64 * (VDIM / 8); id += 128) {
-      const int r = id / (VDIM / 8), cc = id % (VDIM / 8), j = k0 + r;
-      bf16* d = Vd + r * VLD + cc * 8;
-      if (j <= kmax) cp_async16(d, v_pages + ((long long)pt[j / page] * page + j % page) * vrow + (long long)g * VDIM + cc * 8);
-      else *reinterpret_cast<uint4*>(d) = make_uint4(0, 0, 0, 0);
+#pragma unroll 2
+    for (int id = threadIdx.x; id < 64 * CPR; id += 128) {
+      const int r = id / CPR, cc = id % CPR, j = k0 + r;
+      bf16* dst = d + r * PITCH + cc * 8;
+      if (j > kmax) *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
+      else if (page_is_tile) cp_async16(dst, pages + ((long long)at * 64 + r) * row + head0 + cc * 8);
+      else cp_async16(dst, pages + ((long long)pt[j / page] * page + j % page) * row + head0 + cc * 8);
     }
+  };
+  auto fetch = [&](int k0, int at, int buf) {
+    rows_of(Int<DIM>{}, Kb + buf * 64 * QP, k_pages, krow, g * DIM, k0, at);
+    rows_of(Int<VDIM>{}, Vb + buf * 64 * VLD, v_pages, vrow, g * VDIM, k0, at);
   };
   const int lm_key = (lane & 7) + ((lane >> 3) & 1) * 8, lm_col = (lane >> 4) * 8;  // this lane's row of a 16-key x 16-column block
   int cur = 0;
   const int k_first = next_tile(-64);
-  fetch(k_first, 0);
+  fetch(k_first, page_at(k_first), 0);
+  int at_next = page_at(next_tile(k_first));
   asm volatile("cp.async.commit_group;" ::: "memory");
+  // rows of the warp that see every key of a tile need no mask; scores with nothing but a positive scale keep their maximum in units of Q K^T
+  const int warp_first = ctx + (r0 + warp * 16) / gsz;
+  const bool warp_full = r0 + warp * 16 + 16 <= rows;
+  const bool plain = !(softcap > 0.f) && !dist && sx.head_scale == nullptr && scale > 0.f;
+  const float c_plain = scale * 1.4426950408889634f;
   for (int k0 = k_first; k0 <= kmax; k0 = next_tile(k0), cur ^= 1) {
-    if (next_tile(k0) <= kmax) fetch(next_tile(k0), cur ^ 1);  // that buffer was released by the barrier at the end of the last iteration
+    if (next_tile(k0) <= kmax) fetch(next_tile(k0), at_next, cur ^ 1);  // that buffer was released by the barrier at the end of the last iteration
+    at_next = page_at(next_tile(next_tile(k0)));
     asm volatile("cp.async.commit_group;" ::: "memory");
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncthreads();
@@ -156,15 +196,18 @@ __global__ void __launch_bounds__(128, (DIM + VDIM <= 128) ? 4 : 2) attn_ragged_
     if (k0 <= wlim && !(k0 >= keep && k0 + 64 <= warp_lo)) {  // else: no row of this warp sees a key of the tile
     float sacc[8][4];
 #pragma unroll
-    for (int nb = 0; nb < 8; ++nb) {
-      sacc[nb][0] = sacc[nb][1] = sacc[nb][2] = sacc[nb][3] = 0.f;
+    for (int nb = 0; nb < 8; ++nb) sacc[nb][0] = sacc[nb][1] = sacc[nb][2] = sacc[nb][3] = 0.f;
+    // one 16-wide step of the dot products at a time: eight independent accumulators in flight
 #pragma unroll
-      for (int ks = 0; ks < KS; ++ks) {
-        const uint32_t b0 = *reinterpret_cast<const uint32_t*>(Ks + (nb * 8 + gq) * QP + ks * 16 + 2 * tq);
-        const uint32_t b1 = *reinterpret_cast<const uint32_t*>(Ks + (nb * 8 + gq) * QP + ks * 16 + 8 + 2 * tq);
+    for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+      for (int nb = 0; nb < 8; nb += 2) {
+        uint32_t b0, b1, b2, b3;
+        ldmatrix_x4(b0, b1, b2, b3, Ks + (nb * 8 + (lane & 7) + ((lane >> 4) & 1) * 8) * QP + ks * 16 + ((lane >> 3) & 1) * 8);
         mma16816(sacc[nb], qa[ks], b0, b1);
+        mma16816(sacc[nb + 1], qa[ks], b2, b3);
       }
-    }
+    const bool unmasked = warp_full && k0 + 63 <= warp_first && (wlim - k0 < window || k0 + 64 <= keep);
     if constexpr (LOGI) {
       // every visible key's weight is the logistic function of its biased score: no maximum, no sum
 #pragma unroll
@@ -179,32 +222,74 @@ __global__ void __launch_bounds__(128, (DIM + VDIM <= 128) ? 4 : 2) attn_ragged_
     } else {
     // scores -> probabilities (fp32), running max / sum per row; the four lanes of a quad share a row
     float mx_l = -INFINITY, mx_h = -INFINITY;
+    if (plain) {
+      if (!unmasked) {
 #pragma unroll
-    for (int nb = 0; nb < 8; ++nb)
+        for (int nb = 0; nb < 8; ++nb)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        float sc = sacc[nb][c] * ((c & 2) ? sc_h : sc_l);
-        if (softcap > 0.f) sc = softcap * tanh32(sc * inv_cap);
-        const int key = k0 + nb * 8 + 2 * tq + (c & 1);
-        const int away = ((c & 2) ? lim_h : lim_l) - key;
-        const bool vis = away >= 0 && (away < window || key < keep);
-        if (dist && vis) sc -= ((c & 2) ? da_h : da_l) * log1pf(((c & 2) ? db_h : db_l) * (float)away);
-        sc *= 1.4426950408889634f;  // base-2 exponentials below
-        sc = vis ? sc : -INFINITY;
-        sacc[nb][c] = sc;
-        if (c & 2) mx_h = fmaxf(mx_h, sc); else mx_l = fmaxf(mx_l, sc);
+          for (int c = 0; c < 4; ++c) {
+            const int key = k0 + nb * 8 + 2 * tq + (c & 1), away = ((c & 2) ? lim_h : lim_l) - key;
+            if (!(away >= 0 && (away < window || key < keep))) sacc[nb][c] = -INFINITY;
+          }
       }
+#pragma unroll
+      for (int nb = 0; nb < 8; ++nb) {
+        mx_l = fmaxf(mx_l, fmaxf(sacc[nb][0], sacc[nb][1]));
+        mx_h = fmaxf(mx_h, fmaxf(sacc[nb][2], sacc[nb][3]));
+      }
+      mx_l *= c_plain;
+      mx_h *= c_plain;
+    } else {
+      if (softcap > 0.f) {
+        const float in_l = sc_l * inv_cap, in_h = sc_h * inv_cap;
+#pragma unroll
+        for (int nb = 0; nb < 8; ++nb)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) sacc[nb][c] = softcap * tanh32(sacc[nb][c] * ((c & 2) ? in_h : in_l));
+      } else {
+#pragma unroll
+        for (int nb = 0; nb < 8; ++nb)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) sacc[nb][c] *= (c & 2) ? sc_h : sc_l;
+      }
+      if (dist) {
+#pragma unroll
+        for (int nb = 0; nb < 8; ++nb)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const int away = ((c & 2) ? lim_h : lim_l) - (k0 + nb * 8 + 2 * tq + (c & 1));
+            if (away >= 0) sacc[nb][c] -= ((c & 2) ? da_h : da_l) * log1pf(((c & 2) ? db_h : db_l) * (float)away);
+          }
+      }
+      if (!unmasked) {
+#pragma unroll
+        for (int nb = 0; nb < 8; ++nb)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const int key = k0 + nb * 8 + 2 * tq + (c & 1), away = ((c & 2) ? lim_h : lim_l) - key;
+            if (!(away >= 0 && (away < window || key < keep))) sacc[nb][c] = -INFINITY;
+          }
+      }
+#pragma unroll
+      for (int nb = 0; nb < 8; ++nb) {
+        mx_l = fmaxf(mx_l, fmaxf(sacc[nb][0], sacc[nb][1]));
+        mx_h = fmaxf(mx_h, fmaxf(sacc[nb][2], sacc[nb][3]));
+      }
+      mx_l *= 1.4426950408889634f;  // base-2 exponentials below
+      mx_h *= 1.4426950408889634f;
+    }
     mx_l = fmaxf(mx_l, __shfl_xor_sync(0xffffffffu, mx_l, 1)); mx_l = fmaxf(mx_l, __shfl_xor_sync(0xffffffffu, mx_l, 2));
     mx_h = fmaxf(mx_h, __shfl_xor_sync(0xffffffffu, mx_h, 1)); mx_h = fmaxf(mx_h, __shfl_xor_sync(0xffffffffu, mx_h, 2));
     const float mn_l = fmaxf(m_l, mx_l), mn_h = fmaxf(m_h, mx_h);
     const float ml_safe = mn_l > -INFINITY ? mn_l : 0.f, mh_safe = mn_h > -INFINITY ? mn_h : 0.f;  // rows that see no key yet
-    const float corr_l = exp2f(m_l - ml_safe), corr_h = exp2f(m_h - mh_safe);
+    const float corr_l = ex2(m_l - ml_safe), corr_h = ex2(m_h - mh_safe);
     float sum_l = 0.f, sum_h = 0.f;
+    const float cs = plain ? c_plain : 1.4426950408889634f;
 #pragma unroll
     for (int nb = 0; nb < 8; ++nb)
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        const float p = exp2f(sacc[nb][c] - ((c & 2) ? mh_safe : ml_safe));  // exp2(-inf) = 0 for masked keys
+        const float p = ex2(fmaf(sacc[nb][c], cs, (c & 2) ? -mh_safe : -ml_safe));  // 2^-inf = 0 for masked keys
         sacc[nb][c] = p;
         if (c & 2) sum_h += p; else sum_l += p;
       }
@@ -225,16 +310,23 @@ __global__ void __launch_bounds__(128, (DIM + VDIM <= 128) ? 4 : 2) attn_ragged_
       split3(sacc[2 * kk + 1][0], sacc[2 * kk + 1][1], a1[2], a2[2], a3[2]);
       split3(sacc[2 * kk + 1][2], sacc[2 * kk + 1][3], a1[3], a2[3], a3[3]);
       const bf16* vbase = Vs + (kk * 16 + lm_key) * VLD + lm_col;
+      // four value blocks at a time, term after term: neighbouring products go to different accumulators
 #pragma unroll
-      for (int np = 0; np < NV / 2; ++np) {
-        uint32_t b0, b1, b2, b3;
-        ldmatrix_x4_trans(b0, b1, b2, b3, vbase + np * 16);
-        mma16816(oacc[2 * np], a1, b0, b1);
-        mma16816(oacc[2 * np], a2, b0, b1);
-        mma16816(oacc[2 * np], a3, b0, b1);
-        mma16816(oacc[2 * np + 1], a1, b2, b3);
-        mma16816(oacc[2 * np + 1], a2, b2, b3);
-        mma16816(oacc[2 * np + 1], a3, b2, b3);
+      for (int n0 = 0; n0 < NV / 2; n0 += 2) {
+        constexpr int NB = 2;
+        uint32_t vb[NB][4];
+#pragma unroll
+        for (int np = 0; np < NB; ++np)
+          if (n0 + np < NV / 2) ldmatrix_x4_trans(vb[np][0], vb[np][1], vb[np][2], vb[np][3], vbase + (n0 + np) * 16);
+#pragma unroll
+        for (int term = 0; term < 3; ++term)
+#pragma unroll
+          for (int np = 0; np < NB; ++np)
+            if (n0 + np < NV / 2) {
+              const uint32_t* a = term == 0 ? a1 : term == 1 ? a2 : a3;
+              mma16816(oacc[2 * (n0 + np)], a, vb[np][0], vb[np][1]);
+              mma16816(oacc[2 * (n0 + np) + 1], a, vb[np][2], vb[np][3]);
+            }
       }
     }
     }
