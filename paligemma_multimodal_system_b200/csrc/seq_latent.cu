@@ -12,6 +12,8 @@
 //                       [plain | rotated] and value rows in dense scratch "pages"
 //
 // Norm statistics and angles are fp32 / double; the stored rows have the activation type.
+#include <initializer_list>
+
 #include "common.cuh"
 #include "paligemma_b200.h"
 
@@ -34,6 +36,11 @@ template <>
 __device__ __forceinline__ float ldv<bf16>(const bf16* p, long long i) { return __bfloat162float(p[i]); }
 __device__ __forceinline__ void stv(float* p, long long i, float v) { p[i] = v; }
 __device__ __forceinline__ void stv(bf16* p, long long i, float v) { p[i] = __float2bfloat16_rn(v); }
+
+template <typename TA, bool VEC>
+struct Piece { using type = uint4; };
+template <typename TA>
+struct Piece<TA, false> { using type = TA; };
 
 __device__ __forceinline__ float block_sum128(float v, float* red) {
 #pragma unroll
@@ -119,43 +126,65 @@ __global__ void rotate_heads_kernel(const TA* __restrict__ src, long long ld_src
   }
 }
 
+// The two copies below move whole rows.  A warp takes a row at a time; rows whose parts are multiples of 16 bytes go in 16-byte pieces (VEC).  The grid
+// has a CTA for every kRowsPerCta rows of the longest entry: one per row made tens of thousands of empty CTAs in a step of a few portions beside
+// many single tokens (2 portions of 1733 rows + 40 singles, rank 256, 32 heads: gather,
+// up projection and pack together 122 us, now 37).
+constexpr int kRowsPerCta = 16;
+
 // dense row r of entry e (r < ctx + n) <- cached latent row of position r: the first `rank` columns to lat [rows, rank]
-template <typename TA>
-__global__ void latent_gather_kernel(const TA* __restrict__ pages, const int* __restrict__ page_table, int max_pages, int page,
-                                     const int* __restrict__ dense_row0, const int* __restrict__ entry_n, const int* __restrict__ entry_ctx,
-                                     TA* __restrict__ lat, int rank, int width) {
+template <typename TA, bool VEC>
+__global__ void __launch_bounds__(256) latent_gather_kernel(const TA* __restrict__ pages, const int* __restrict__ page_table, int max_pages, int page,
+                                                            const int* __restrict__ dense_row0, const int* __restrict__ entry_n,
+                                                            const int* __restrict__ entry_ctx, TA* __restrict__ lat, int rank, int width) {
+  constexpr int E = VEC ? 16 / sizeof(TA) : 1;  // elements of a piece
+  using P = typename Piece<TA, VEC>::type;
   const int e = blockIdx.y;
   if (entry_n[e] == 1) return;  // single-token entries are served by the absorbed form: they own no dense rows
-  const int len = entry_ctx[e] + entry_n[e];
-  for (int j = blockIdx.x; j < len; j += gridDim.x) {
-    const TA* src = pages + ((long long)page_table[(long long)e * max_pages + j / page] * page + j % page) * width;
-    TA* dst = lat + (long long)(dense_row0[e] + j) * rank;
-    for (int d = threadIdx.x; d < rank; d += blockDim.x) dst[d] = src[d];
+  const int len = entry_ctx[e] + entry_n[e], lane = threadIdx.x & 31, nw = gridDim.x * 8;
+  for (int j = blockIdx.x * 8 + (threadIdx.x >> 5); j < len; j += nw) {
+    const P* src = reinterpret_cast<const P*>(pages + ((long long)page_table[(long long)e * max_pages + j / page] * page + j % page) * width);
+    P* dst = reinterpret_cast<P*>(lat + (long long)(dense_row0[e] + j) * rank);
+#pragma unroll 4
+    for (int d = lane; d < rank / E; d += 32) dst[d] = src[d];
   }
 }
 
 // per dense row: k[row, h, :] = [up[row, h * dim ..] | rotated part of the cached row], v[row, h, :] = up[row, H * dim + h * vdim ..]
-template <typename TA>
-__global__ void latent_pack_kv_kernel(const TA* __restrict__ up, long long ld_up, const TA* __restrict__ pages, const int* __restrict__ page_table,
-                                      int max_pages, int page, const int* __restrict__ dense_row0, const int* __restrict__ entry_n,
-                                      const int* __restrict__ entry_ctx, TA* __restrict__ k_out, TA* __restrict__ v_out, int H, int dim, int rot,
-                                      int vdim, int rank) {
+template <typename TA, bool VEC>
+__global__ void __launch_bounds__(256) latent_pack_kv_kernel(const TA* __restrict__ up, long long ld_up, const TA* __restrict__ pages,
+                                                             const int* __restrict__ page_table, int max_pages, int page, const int* __restrict__ dense_row0,
+                                                             const int* __restrict__ entry_n, const int* __restrict__ entry_ctx, TA* __restrict__ k_out,
+                                                             TA* __restrict__ v_out, int H, int dim, int rot, int vdim, int rank) {
+  constexpr int E = VEC ? 16 / sizeof(TA) : 1;
+  using P = typename Piece<TA, VEC>::type;
   const int e = blockIdx.y;
   if (entry_n[e] == 1) return;
-  const int len = entry_ctx[e] + entry_n[e];
-  const int kd = dim + rot;
-  for (int j = blockIdx.x; j < len; j += gridDim.x) {
+  const int len = entry_ctx[e] + entry_n[e], lane = threadIdx.x & 31, nw = gridDim.x * 8;
+  const int kd = (dim + rot) / E, plain = dim / E;
+  for (int j = blockIdx.x * 8 + (threadIdx.x >> 5); j < len; j += nw) {
     const long long row = dense_row0[e] + j;
-    const TA* src = pages + ((long long)page_table[(long long)e * max_pages + j / page] * page + j % page) * (long long)(rank + rot) + rank;
-    const TA* u = up + row * ld_up;
-    TA* ko = k_out + row * (long long)H * kd;
-    TA* vo = v_out + row * (long long)H * vdim;
-    for (int i = threadIdx.x; i < H * kd; i += blockDim.x) {
-      const int h = i / kd, d = i % kd;
-      ko[i] = d < dim ? u[(long long)h * dim + d] : src[d - dim];
+    const P* src = reinterpret_cast<const P*>(pages + ((long long)page_table[(long long)e * max_pages + j / page] * page + j % page) * (long long)(rank + rot) + rank);
+    const P* u = reinterpret_cast<const P*>(up + row * ld_up);
+    P* ko = reinterpret_cast<P*>(k_out + row * (long long)H * (dim + rot));
+    P* vo = reinterpret_cast<P*>(v_out + row * (long long)H * vdim);
+#pragma unroll 4
+    for (int i = lane; i < H * kd; i += 32) {
+      const int h = i / kd, d = i - h * kd;
+      ko[i] = d < plain ? u[h * plain + d] : src[d - plain];
     }
-    for (int i = threadIdx.x; i < H * vdim; i += blockDim.x) vo[i] = u[(long long)H * dim + i];
+#pragma unroll 4
+    for (int i = lane; i < H * vdim / E; i += 32) vo[i] = u[H * plain + i];
   }
+}
+
+// whether every size (elements) and address is a whole number of 16-byte pieces
+bool whole_pieces(int elem, std::initializer_list<long long> sizes, std::initializer_list<const void*> ptrs) {
+  for (long long n : sizes)
+    if (n * elem % 16 != 0) return false;
+  for (const void* p : ptrs)
+    if (reinterpret_cast<uintptr_t>(p) & 15) return false;
+  return true;
 }
 
 }  // namespace
@@ -192,13 +221,15 @@ extern "C" int pg_rotate_heads(const void* src, long long ld_src, long long head
 extern "C" int pg_latent_gather(const void* pages, const int* page_table, int max_pages, int page, const int* dense_row0, const int* entry_n,
                                 const int* entry_ctx, void* lat, int entries, int max_len, int rank, int width, int act_f32, void* stream) {
   if (entries <= 0 || entries > 65535 || max_len <= 0 || rank <= 0 || width < rank || page <= 0) return PG_ERR_ARG;
-  dim3 grid(max_len < 4096 ? max_len : 4096, entries);
-  if (act_f32)
-    latent_gather_kernel<float><<<grid, 128, 0, PG_ST(stream)>>>(static_cast<const float*>(pages), page_table, max_pages, page, dense_row0, entry_n,
-                                                                entry_ctx, static_cast<float*>(lat), rank, width);
-  else
-    latent_gather_kernel<bf16><<<grid, 128, 0, PG_ST(stream)>>>(static_cast<const bf16*>(pages), page_table, max_pages, page, dense_row0, entry_n,
-                                                               entry_ctx, static_cast<bf16*>(lat), rank, width);
+  const dim3 grid((max_len + kRowsPerCta - 1) / kRowsPerCta < 4096 ? (max_len + kRowsPerCta - 1) / kRowsPerCta : 4096, entries);
+  const bool vec = whole_pieces(act_f32 ? 4 : 2, {rank, width}, {pages, lat});
+  auto go = [&](auto kernel, auto t) {
+    using TA = decltype(t);
+    kernel<<<grid, 256, 0, PG_ST(stream)>>>(static_cast<const TA*>(pages), page_table, max_pages, page, dense_row0, entry_n, entry_ctx, static_cast<TA*>(lat),
+                                            rank, width);
+  };
+  if (act_f32) vec ? go(latent_gather_kernel<float, true>, float()) : go(latent_gather_kernel<float, false>, float());
+  else vec ? go(latent_gather_kernel<bf16, true>, bf16()) : go(latent_gather_kernel<bf16, false>, bf16());
   PG_RET();
 }
 
@@ -206,14 +237,14 @@ extern "C" int pg_latent_pack_kv(const void* up, long long ld_up, const void* pa
                                  const int* dense_row0, const int* entry_n, const int* entry_ctx, void* k_out, void* v_out, int entries, int max_len,
                                  int H, int dim, int rot, int vdim, int rank, int act_f32, void* stream) {
   if (entries <= 0 || entries > 65535 || max_len <= 0 || H <= 0 || dim <= 0 || rot < 0 || vdim <= 0 || rank <= 0 || page <= 0) return PG_ERR_ARG;
-  dim3 grid(max_len < 4096 ? max_len : 4096, entries);
-  if (act_f32)
-    latent_pack_kv_kernel<float><<<grid, 256, 0, PG_ST(stream)>>>(static_cast<const float*>(up), ld_up, static_cast<const float*>(pages), page_table,
-                                                                 max_pages, page, dense_row0, entry_n, entry_ctx, static_cast<float*>(k_out),
-                                                                 static_cast<float*>(v_out), H, dim, rot, vdim, rank);
-  else
-    latent_pack_kv_kernel<bf16><<<grid, 256, 0, PG_ST(stream)>>>(static_cast<const bf16*>(up), ld_up, static_cast<const bf16*>(pages), page_table,
-                                                                max_pages, page, dense_row0, entry_n, entry_ctx, static_cast<bf16*>(k_out),
-                                                                static_cast<bf16*>(v_out), H, dim, rot, vdim, rank);
+  const dim3 grid((max_len + kRowsPerCta - 1) / kRowsPerCta < 4096 ? (max_len + kRowsPerCta - 1) / kRowsPerCta : 4096, entries);
+  const bool vec = whole_pieces(act_f32 ? 4 : 2, {dim, rot, vdim, rank, ld_up}, {up, pages, k_out, v_out});
+  auto go = [&](auto kernel, auto t) {
+    using TA = decltype(t);
+    kernel<<<grid, 256, 0, PG_ST(stream)>>>(static_cast<const TA*>(up), ld_up, static_cast<const TA*>(pages), page_table, max_pages, page, dense_row0, entry_n,
+                                            entry_ctx, static_cast<TA*>(k_out), static_cast<TA*>(v_out), H, dim, rot, vdim, rank);
+  };
+  if (act_f32) vec ? go(latent_pack_kv_kernel<float, true>, float()) : go(latent_pack_kv_kernel<float, false>, float());
+  else vec ? go(latent_pack_kv_kernel<bf16, true>, bf16()) : go(latent_pack_kv_kernel<bf16, false>, bf16());
   PG_RET();
 }

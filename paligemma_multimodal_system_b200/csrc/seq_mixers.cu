@@ -139,6 +139,139 @@ __global__ void __launch_bounds__(128) attn_prepare_kernel(const TA* __restrict_
   }
 }
 
+// The same for heads of whole 16-byte groups (8 elements a lane, so dim / 8 lanes -- a power of two -- hold a head and its norm stays inside them): the
+// row is read once, in 16-byte pieces, all of them under way together.  A CTA takes TOK tokens, so that the double-precision angles -- a chain of ~60
+// dependent operations that only dim / 2 threads had work in -- run on all of its threads.  What bounds it: prompts, HBM (8192 rows of 32 + 8 + 8 heads x 64,
+// 100 MB: 65 -> 28 us, with norms 101 -> 37); a decode step, the latency of its loads (48 rows: 7.9 -> 3.5 us, with norms 12.8 -> 4.5).
+template <typename TA>
+__device__ __forceinline__ void ld8(float (&v)[8], const TA* p);
+template <>
+__device__ __forceinline__ void ld8<float>(float (&v)[8], const float* p) {
+  const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+template <>
+__device__ __forceinline__ void ld8<bf16>(float (&v)[8], const bf16* p) {
+  const uint4 u = *reinterpret_cast<const uint4*>(p);
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) { v[2 * i] = __uint_as_float(w[i] << 16); v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
+}
+__device__ __forceinline__ void st8(float* p, const float (&v)[8]) {
+  reinterpret_cast<float4*>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
+  reinterpret_cast<float4*>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
+}
+__device__ __forceinline__ void st8(bf16* p, const float (&v)[8]) {
+  *reinterpret_cast<uint4*>(p) = make_uint4(pg::pack_bf16(v[0], v[1]), pg::pack_bf16(v[2], v[3]), pg::pack_bf16(v[4], v[5]), pg::pack_bf16(v[6], v[7]));
+}
+
+template <typename TA, int TOK>
+__global__ void __launch_bounds__(128) attn_prepare_vec_kernel(const TA* __restrict__ qkv, long long ld, const int* __restrict__ pos,
+                                                               const int* __restrict__ row_entry, const int* __restrict__ page_table, int max_pages,
+                                                               int page, const double* __restrict__ freq, const float* __restrict__ qn,
+                                                               const float* __restrict__ kn, TA* __restrict__ q_out, TA* __restrict__ k_pages,
+                                                               TA* __restrict__ v_pages, int rows, int H, int G, int dim, int vdim, int rot, float eps,
+                                                               int norm_qk, int norm_v, int v_from_k, float rot_gain, const TA* __restrict__ v_other,
+                                                               long long ldvo, float v_mix) {
+  extern __shared__ float cs[];  // [TOK][cos rot/2 | sin rot/2]
+  __shared__ float part[2][TOK][4];
+  const int t0 = blockIdx.x * TOK, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nq = H * dim / 8, nk = k_pages != nullptr ? G * dim / 8 : 0, nv = k_pages != nullptr ? G * vdim / 8 : 0, half = rot / 2;
+  long long pg_row[TOK];
+#pragma unroll
+  for (int k = 0; k < TOK; ++k) {
+    const int t = min(t0 + k, rows - 1), p = pos[t];
+    pg_row[k] = nk > 0 ? (long long)page_table[(long long)row_entry[t] * max_pages + p / page] * page + p % page : 0;
+  }
+  for (int i = threadIdx.x; i < TOK * half; i += 128) {
+    const int k = i / half, j = i - k * half;
+    double s, c;
+    sincos((double)pos[min(t0 + k, rows - 1)] * freq[j], &s, &c);
+    cs[k * rot + j] = rot_gain * (float)c;
+    cs[k * rot + half + j] = rot_gain * (float)s;
+  }
+  if (norm_qk == 2) {  // one root mean square for all of q, one for all of k
+#pragma unroll
+    for (int k = 0; k < TOK; ++k) {
+      const TA* row = qkv + (long long)min(t0 + k, rows - 1) * ld;
+      float sq = 0.f, sk = 0.f;
+      for (int c = threadIdx.x; c < nq + nk; c += 128) {
+        float v[8], s = 0.f;
+        ld8<TA>(v, row + 8LL * c);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s = fmaf(v[i], v[i], s);
+        if (c < nq) sq += s; else sk += s;
+      }
+      sq = wsum(sq);
+      sk = wsum(sk);
+      if (lane == 0) { part[0][k][warp] = sq; part[1][k][warp] = sk; }
+    }
+  }
+  __syncthreads();
+  const int total = nq + nk + nv;
+#pragma unroll 2
+  for (int c = threadIdx.x; c < (total + 31) / 32 * 32; c += 128) {  // whole warps: the norms shuffle
+    const bool in = c < total, is_q = c < nq, is_k = !is_q && c < nq + nk;
+    const int cc = is_q ? c : is_k ? c - nq : c - nq - nk, lph = (is_q || is_k ? dim : vdim) / 8;  // lanes of the head
+    const int d0 = (cc & (lph - 1)) * 8;
+    const long long off = is_q || is_k ? 8LL * c : v_from_k ? 8LL * (c - nk) : 8LL * c;
+    const float* w = is_q ? qn : kn;  // NULL: a norm without a weight
+    if (w != nullptr) w += norm_qk == 2 ? 8LL * cc : d0;
+    float x[TOK][8];
+#pragma unroll
+    for (int k = 0; k < TOK; ++k)
+      if (in) ld8<TA>(x[k], qkv + (long long)min(t0 + k, rows - 1) * ld + off);
+#pragma unroll
+    for (int k = 0; k < TOK; ++k) {
+      float inv = 1.0f;
+      if ((is_q || is_k) && norm_qk == 2) {
+        const float* ps = part[is_q ? 0 : 1][k];
+        inv = 1.0f / sqrtf((ps[0] + ps[1] + ps[2] + ps[3]) / (float)(8 * (is_q ? nq : nk)) + eps);
+      } else if (norm_qk == 1 || norm_v) {  // (uniform: every lane takes part in the shuffles, the others' sums are not used)
+        float s = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s = in ? fmaf(x[k][i], x[k][i], s) : 0.f;
+        for (int o = 1; o < 32; o <<= 1) {
+          const float u = __shfl_xor_sync(0xffffffffu, s, o);
+          if (o < lph) s += u;
+        }
+        if ((is_q || is_k) ? norm_qk == 1 : norm_v) inv = 1.0f / sqrtf(s / (float)(8 * lph) + eps);
+      }
+      const int t = t0 + k;
+      if (!in || t >= rows) continue;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[k][i] *= inv;
+      if (is_q || is_k) {
+        if (w != nullptr) {
+          float ww[8];
+          ld8<float>(ww, w);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) x[k][i] *= ww[i];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int pair = d0 / 2 + i;
+          if (pair < half) {
+            const float c0 = cs[k * rot + pair], s0 = cs[k * rot + half + pair], a = x[k][2 * i], b = x[k][2 * i + 1];
+            x[k][2 * i] = a * c0 - b * s0;
+            x[k][2 * i + 1] = b * c0 + a * s0;
+          }
+        }
+        if (is_q) st8(q_out + (long long)t * H * dim + 8LL * cc, x[k]);
+        else st8(k_pages + pg_row[k] * ((long long)G * dim) + 8LL * cc, x[k]);
+      } else {
+        if (v_other != nullptr) {
+          float o[8];
+          ld8<TA>(o, v_other + (long long)t * ldvo + 8LL * cc);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) x[k][i] = (1.0f - v_mix) * x[k][i] + v_mix * o[i];
+        }
+        st8(v_pages + pg_row[k] * ((long long)G * vdim) + 8LL * cc, x[k]);
+      }
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------------------------------------------------
 // Causal attention of an entry's new rows over its paged keys / values.  CTA = 32 query rows (token x query head of one
 // k/v head) of one entry; 8 warps x 4 rows.  Keys pass in tiles of 32 through shared memory (fp32); per tile lane j scores
@@ -893,6 +1026,23 @@ extern "C" int pg_attn_prepare(const void* qkv, long long ld, const int* pos, co
   if (v_from_k && vdim != dim) return PG_ERR_ARG;
   if (norm_qk < 0 || norm_qk > 2 || (v_other != nullptr && k_pages == nullptr)) return PG_ERR_ARG;
   if ((k_pages == nullptr) != (v_pages == nullptr)) return PG_ERR_ARG;
+  // heads of 8, 16, .. 256 elements on 16-byte boundaries take the vector form (a norm per value head wants its lanes inside a warp as well)
+  auto lanes = [](int n) { return n % 8 == 0 && n / 8 <= 32 && (n / 8 & (n / 8 - 1)) == 0; };
+  const uintptr_t ptrs = reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(k_pages) |
+                         reinterpret_cast<uintptr_t>(v_pages) | reinterpret_cast<uintptr_t>(q_norm) | reinterpret_cast<uintptr_t>(k_norm) |
+                         reinterpret_cast<uintptr_t>(v_other);
+  if (lanes(dim) && lanes(vdim) && (vdim == dim || !norm_v) && ld % 8 == 0 && ld_v_other % 8 == 0 && (ptrs & 15) == 0) {
+    auto go = [&](auto kernel, auto t, int tok) {
+      using TA = decltype(t);
+      kernel<<<(rows + tok - 1) / tok, 128, (size_t)(tok * rot_dims + 2) * sizeof(float), PG_ST(stream)>>>(
+          static_cast<const TA*>(qkv), ld, pos, row_entry, page_table, max_pages, page, freq, q_norm, k_norm, static_cast<TA*>(q_out), static_cast<TA*>(k_pages),
+          static_cast<TA*>(v_pages), rows, H, G, dim, vdim, rot_dims, eps, norm_qk, norm_v, v_from_k, rot_gain, static_cast<const TA*>(v_other), ld_v_other, v_mix);
+    };
+    // four tokens a CTA once that still fills the SMs
+    if (act_f32) rows >= 4 * 4 * pg::num_sms() ? go(attn_prepare_vec_kernel<float, 4>, float(), 4) : go(attn_prepare_vec_kernel<float, 1>, float(), 1);
+    else rows >= 4 * 4 * pg::num_sms() ? go(attn_prepare_vec_kernel<bf16, 4>, bf16(), 4) : go(attn_prepare_vec_kernel<bf16, 1>, bf16(), 1);
+    PG_RET();
+  }
   const size_t smem = (size_t)(rot_dims + 2) * sizeof(float);
   if (act_f32)
     attn_prepare_kernel<float><<<rows, 128, smem, PG_ST(stream)>>>(static_cast<const float*>(qkv), ld, pos, row_entry, page_table, max_pages, page, freq,
