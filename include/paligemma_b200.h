@@ -105,6 +105,9 @@ int pg_gemm_bf16_fused(const void* x, long long ldx, const void* w, long long ld
 int pg_gemm_residual(const void* x, long long ldx, const void* w, long long ldw, float* h, long long ldh, const float* bias, int tokens, int features,
                      int K, float scale, void* stream);
 
+/* out[t,f] = sum_k x[t,k] w[f,k] in fp32 rows; few tokens and few output tiles: K is shared out over the GPU. */
+int pg_linear_f32(const void* x, long long ldx, const void* w, long long ldw, float* out, long long ldo, int tokens, int features, int K, void* stream);
+
 /* The encoder layers of the vision tower (modeling_siglip.py:216-263): seven launches each, issued by one call.  Weights as the entry points above take
  * them (matrices bf16, dense rows; q | k | v projections fused), x fp32 [images * patches, D] in place; hn, att bf16 [., D], qkv bf16 [., 3 D],
  * mid bf16 [., F] are scratch. */

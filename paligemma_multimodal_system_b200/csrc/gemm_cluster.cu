@@ -302,7 +302,7 @@ ClusterGemmPlan plan_cluster_gemm(int tokens, int features, int K) {
   const int dev = current_device();
   Known& slot = known[(tokens * 31u + features * 7u + K) / 8u % 64u];
   if (slot.tokens == tokens && slot.features == features && slot.K == K && slot.dev == dev) return slot.plan;
-  ClusterGemmPlan best{0, 0, 0.f};
+  ClusterGemmPlan best{0, 0, 0, 0.f};
   const int f_tiles = (features + kFeat - 1) / kFeat, total_kb = (K + kKb - 1) / kKb;
   for (int nt = (tokens + 383) / 384; nt <= (tokens + 383) / 384 + 7; ++nt) {
     int tile = (tokens + nt - 1) / nt;
@@ -314,7 +314,7 @@ ClusterGemmPlan plan_cluster_gemm(int tokens, int features, int K) {
       const int at_once = S == 1 ? num_sms() : clusters_at_once(S), waves = (f_tiles * nt + at_once - 1) / at_once;
       // clocks: launch, dependency wait and first bytes; an SM takes in 64 bytes a clock; the exchange writes and reads its tile
       const float cost = waves * (4000.f + per * (256.f + 2.f * tile) + (S > 1 ? 1500.f + 16.f * tile : 10.f * tile));
-      if (best.split == 0 || cost < best.clocks) best = ClusterGemmPlan{tile, S, cost};
+      if (best.split == 0 || cost < best.clocks) best = ClusterGemmPlan{tile, S, waves, cost};
     }
   }
   slot = Known{dev, tokens, features, K, best};

@@ -19,9 +19,9 @@ struct ClusterGemmArgs {
   int tile_tokens, split, stages, smem_tiles;
 };
 
-// tokens per tile, CTAs that share K, and the estimated clocks of the launch
+// tokens per tile, CTAs that share K, waves of the grid, and the estimated clocks of the launch
 struct ClusterGemmPlan {
-  int tile_tokens, split;
+  int tile_tokens, split, waves;
   float clocks;
 };
 

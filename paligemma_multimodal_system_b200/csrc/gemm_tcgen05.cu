@@ -1152,11 +1152,17 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& 
 // 263 tokens 14.4 / 8.2, 1024 17.0 / 10.8, 2048 20.2 / 22.2; 2048 x 2048 with residual 263 15.2 / 10.1, 1300 28.5 / 18.2; 2048 x 16384 with residual
 // 263 41 / 28, 1300 163 / 86, 2048 113 / 120; 32768 x 2048 gate || up 263 91 / 40, 1300 223 / 172; 5120 x 2048 1024 (80 pair tiles) 27.9 / 22.0, 1536
 // (120) 29.0 / 30.3; 8192 x 2048 706 (96) 28.6 / 23.4, 1024 (128) 29.3 / 31.5; 3072 x 768 1300 10.4 / 9.1, 1536 10.7 / 11.5.
-static bool cluster_form(const GemmArgs& a, long long ldr) {
+//
+// Decode-sized calls (up to 128 tokens): where its grid is one wave, but for long K with up to 64 tokens, which the two-CTAs-per-SM stream of this file's
+// swap kernels reads faster.  Not for split-K accumulation into a residual stream: in a chain of decode launches under the L2 prefetch stream of
+// modeling_gemma.py the clusters wait for whole GPCs (one request of 24 tokens 28.5 -> 29.5 ms, 64 requests 132 -> 138).  5 tokens: 8192 x 2048 13.4 / 9.3, 2048 x 2048 7.1 / 5.6 (without the zeroed accumulator), 16384 x 2048 gate || up
+// 15.1 / 13.1, 2048 x 8192 10.7 / 10.9, 2048 x 16384 15.0 / 16.6, two waves: 32000 x 2048 22 / 36; 128 tokens: 2048 x 8192 18.0 / 14.0.
+static bool cluster_form(const GemmArgs& a, long long ldr, int swap) {
   auto aligned = [](const void* p, int n) { return (reinterpret_cast<uintptr_t>(p) & (n - 1)) == 0; };
   // vectors of four: outputs, bias and residual rows
   if (a.features % 4 != 0 || a.ldo % 4 != 0 || !aligned(a.out, 16) || !aligned(a.bias, 16)) return false;
   if (a.resid != nullptr && (ldr % 4 != 0 || !aligned(a.resid, 16))) return false;
+  if (swap) return a.mode != PG_EPI_ATOMIC_F32 && a.stats == nullptr && a.zero_buf == nullptr && (a.K <= 4096 || a.tokens > 64) && plan_cluster_gemm(a.tokens, a.features, a.K).waves == 1;
   const int pair_tiles = ((a.tokens + 2 * BM - 1) / (2 * BM)) * ((a.features + 255) / 256);
   return a.tokens <= 1408 && (a.mode == PG_EPI_GEGLU || pair_tiles < 3 * (num_sms() / 2) / 2);
 }
@@ -1164,6 +1170,13 @@ static bool cluster_form(const GemmArgs& a, long long ldr) {
 }  // namespace pg
 
 using namespace pg;
+
+// Whether a decode-sized fp32 product adds up K by itself (gemm_cluster.cu), without split-K partials.
+bool pg_gemm_sums_once(int tokens, int features, int K, const void* out, long long ldo) {
+  GemmArgs a = {};
+  a.tokens = tokens; a.features = features; a.K = K; a.mode = PG_EPI_F32; a.out = const_cast<void*>(out); a.ldo = ldo;
+  return cluster_form(a, 0, 1);
+}
 
 extern "C" int pg_gemm_bf16(const void* x, long long ldx, const void* w, long long ldw, void* out, long long ldo,
                             const float* bias, const float* resid, long long ldr, int tokens, int features, int K,
@@ -1241,6 +1254,12 @@ extern "C" int pg_gemm_bf16_fused(const void* x, long long ldx, const void* w, l
                      (resid == nullptr || ((ldr % 4) == 0 && (reinterpret_cast<uintptr_t>(resid) & 15) == 0))) ? 1 : 0;
   a.trace = g_gemm_trace ? g_gemm_trace + 8 * (g_gemm_trace_idx++ % 64) : nullptr;
 
+  if (cluster_form(a, ldr, swap)) {
+    ClusterGemmArgs c = {};
+    c.tokens = tokens; c.features = features; c.K = K; c.mode = mode; c.act = act_gelu; c.scale = scale; c.glu_alpha = a.glu_alpha;
+    c.out = out; c.ldo = ldo; c.bias = bias; c.resid = mode == PG_EPI_F32 ? resid : nullptr; c.ldr = ldr; c.out_row_map = a.out_row_map; c.resid_mod = a.resid_mod;
+    return launch_cluster_gemm(plan_cluster_gemm(tokens, features, K), x, ldx, w, ldw, c, st);
+  }
   CUtensorMap ta, tb;
   int rc;
   if (swap) {
@@ -1258,12 +1277,6 @@ extern "C" int pg_gemm_bf16_fused(const void* x, long long ldx, const void* w, l
       default: return launch<128, true>(ta, tb, a, tiles, st);
     }
   } else {
-    if (cluster_form(a, ldr)) {
-      ClusterGemmArgs c = {};
-      c.tokens = tokens; c.features = features; c.K = K; c.mode = mode; c.act = act_gelu; c.scale = scale; c.glu_alpha = a.glu_alpha;
-      c.out = out; c.ldo = ldo; c.bias = bias; c.resid = mode == PG_EPI_F32 ? resid : nullptr; c.ldr = ldr; c.out_row_map = a.out_row_map; c.resid_mod = a.resid_mod;
-      return launch_cluster_gemm(plan_cluster_gemm(tokens, features, K), x, ldx, w, ldw, c, st);
-    }
     // largest N tile that still gives the persistent grid ~a wave of CTAs (small token counts: latency path)
     const int m_blocks = (tokens + BM - 1) / BM;
     auto ntiles = [&](int bn) { return m_blocks * ((features + bn - 1) / bn) * split_k; };

@@ -6,6 +6,8 @@
 #include "common.cuh"
 #include "paligemma_b200.h"
 
+bool pg_gemm_sums_once(int tokens, int features, int K, const void* out, long long ldo);  // gemm_tcgen05.cu
+
 extern "C" int pg_gemm_residual(const void* x, long long ldx, const void* w, long long ldw, float* h, long long ldh, const float* bias, int tokens,
                                 int features, int K, float scale, void* stream) {
   if (tokens <= 0 || features <= 0 || K <= 0) return PG_ERR_ARG;
@@ -25,6 +27,19 @@ extern "C" int pg_gemm_residual(const void* x, long long ldx, const void* w, lon
   int split = (swap ? 2 * 148 : 148) / tiles;
   if (split > kb / 4) split = kb / 4;
   return pg_gemm_bf16(x, ldx, w, ldw, h, ldh, bias, nullptr, 0, tokens, features, K, PG_EPI_ATOMIC_F32, 0, scale, swap, split < 1 ? 1 : split, stream);
+}
+
+extern "C" int pg_linear_f32(const void* x, long long ldx, const void* w, long long ldw, float* out, long long ldo, int tokens, int features, int K,
+                             void* stream) {
+  if (tokens <= 0 || features <= 0 || K <= 0 || out == nullptr) return PG_ERR_ARG;
+  const int tiles = (features + 127) / 128, kb = (K + 63) / 64, swap = tokens <= 128 ? 1 : 0;
+  int split = 2 * pg::num_sms() / tiles;
+  if (split > kb / 4) split = kb / 4;
+  if (!swap || split <= 1 || pg_gemm_sums_once(tokens, features, K, out, ldo))
+    return pg_gemm_bf16(x, ldx, w, ldw, out, ldo, nullptr, nullptr, 0, tokens, features, K, PG_EPI_F32, 0, 1.f, swap, 1, stream);
+  // few tiles of a long K: split-K partials are red.add-ed into the zeroed output
+  if (cudaMemset2DAsync(out, ldo * sizeof(float), 0, features * sizeof(float), tokens, reinterpret_cast<cudaStream_t>(stream)) != cudaSuccess) return PG_ERR_CUDA;
+  return pg_gemm_bf16(x, ldx, w, ldw, out, ldo, nullptr, nullptr, 0, tokens, features, K, PG_EPI_ATOMIC_F32, 0, 1.f, swap, split, stream);
 }
 
 #define PG_TRY(call)                  \

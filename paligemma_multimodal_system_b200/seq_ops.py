@@ -157,14 +157,10 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: int = ACT_N
         assert act == ACT_NONE or out.dtype == torch.bfloat16
         if act != ACT_NONE:
             return _lib.gemm(x, w, out, mode=_lib.EPI_BF16, act_gelu=act, swap=1 if T <= 128 else 0, bias=bias)
-        if T <= 128 and out.dtype == torch.float32 and bias is None:
-            # few rows, few 128-feature tiles (output and down projections): split K over CTAs so that the whole GPU streams the
-            # weights; the fp32 partials are red.add-ed into the zeroed output (as the framework's other decode GEMMs do)
-            tiles, kb = (F + 127) // 128, (K + 63) // 64
-            split = max(1, min(kb // 4, (2 * _lib.num_sms()) // tiles))
-            if split > 1:
-                out.zero_()
-                return _lib.gemm(x, w, out, mode=_lib.EPI_ATOMIC_F32, swap=1, split_k=split)
+        if out.dtype == torch.float32 and bias is None:
+            _lib.check(_lib.lib().pg_linear_f32(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), T, F, K, _lib.stream()),
+                       "pg_linear_f32")
+            return out
         return _lib.gemm(x, w, out, mode=_lib.EPI_F32 if out.dtype == torch.float32 else _lib.EPI_BF16, swap=1 if T <= 128 else 0, bias=bias)
     if x.dtype == torch.float32 and out.dtype != torch.float32:
         raise ValueError("fp32 operands produce fp32 outputs")
