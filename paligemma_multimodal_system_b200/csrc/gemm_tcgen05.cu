@@ -150,7 +150,7 @@ PG_DEVINL void swap_tile_epilogue(const GemmArgs& args, uint32_t taddr, int fr, 
   const char* res = (MODE == PG_EPI_F32 && args.resid != nullptr)
                         ? reinterpret_cast<const char*>(args.resid + static_cast<long long>(j_base + col_begin) * args.ldr + fr) : nullptr;
   const long long rstep = args.ldr * 4;
-  const int act = MODE == PG_EPI_BF16 ? args.act_gelu : 0;  // 1: gelu(tanh), 2: relu squared
+  const int act = MODE == PG_EPI_BF16 ? args.act_gelu : 0;  // 1: gelu(tanh), 2: relu squared, 6: gelu(erf)
 #pragma unroll 1
   for (int c0 = col_begin; c0 < BN; c0 += 16) {
     if (c0 >= nvalid) break;  // warp-uniform
@@ -394,7 +394,7 @@ PG_DEVINL void rowmajor_tile_epilogue(const GemmArgs& args, uint32_t taddr, int 
   const bool row_ok = tok < args.tokens;
   const float scale = args.scale;
   const bool has_bias = args.bias != nullptr && first_split;
-  const int act = MODE == PG_EPI_BF16 ? args.act_gelu : 0;  // 1: gelu(tanh), 2: relu squared
+  const int act = MODE == PG_EPI_BF16 ? args.act_gelu : 0;  // 1: gelu(tanh), 2: relu squared, 6: gelu(erf)
   __nv_bfloat16* out_bf = reinterpret_cast<__nv_bfloat16*>(args.out) + static_cast<long long>(tok) * args.ldo;
   const int orow = (MODE == PG_EPI_F32 && args.out_row_map != nullptr && tok < args.tokens) ? __ldg(args.out_row_map + tok) : tok;
   float* out_f = reinterpret_cast<float*>(args.out) + static_cast<long long>(orow) * args.ldo;
@@ -444,8 +444,10 @@ PG_DEVINL void rowmajor_tile_epilogue(const GemmArgs& args, uint32_t taddr, int 
         }
         if (MODE == PG_EPI_BF16) {
           if (act) {
+            with_act(act, [&](auto a) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = epilogue_act(v[i], act);
+              for (int i = 0; i < 16; ++i) v[i] = epilogue_act(v[i], decltype(a)::value);
+            });
           }
           if (collective) {
 #pragma unroll
@@ -590,7 +592,6 @@ PG_DEVINL void geglu_swap_epilogue_group(const GemmArgs& args, uint32_t taddr, f
   __nv_bfloat16* out_bf = reinterpret_cast<__nv_bfloat16*>(args.out);
   const bool is_gate = q < 2;
   const int r = (q * 32 + lane) & 63;
-  const int kind = args.act_gelu;
   const float glim = args.scale, galpha = args.glu_alpha;
   // bias of this thread's packed weight row (rows of a 128-row tile: [64 gate | 64 up]); it travels with the exchanged value
   const float bias_me = args.bias != nullptr ? __ldg(args.bias + m_blk * 128 + q * 32 + lane) : 0.f;
@@ -615,17 +616,19 @@ PG_DEVINL void geglu_swap_epilogue_group(const GemmArgs& args, uint32_t taddr, f
       if constexpr (LDN == 16) tmem_ld16(taddr + keep0 + c0, v); else tmem_ld8(taddr + keep0 + c0, v);
       tmem_ld_wait();
     }
+    with_glu(args.act_gelu, [&](auto kind) {
 #pragma unroll
-    for (int i = 0; i < LDN; i += 2) {
-      float res[2];
+      for (int i = 0; i < LDN; i += 2) {
+        float res[2];
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        float mine = __uint_as_float(v[i + e]) + bias_me;
-        float other = xrecv[r * HB + ((c0 + i + e) ^ (r & (HB - 1) & 31))];
-        res[e] = is_gate ? glu_act(mine, other, kind, glim, galpha) : glu_act(other, mine, kind, glim, galpha);
+        for (int e = 0; e < 2; ++e) {
+          const float mine = __uint_as_float(v[i + e]) + bias_me;
+          const float other = xrecv[r * HB + ((c0 + i + e) ^ (r & (HB - 1) & 31))];
+          res[e] = glu_act(is_gate ? mine : other, is_gate ? other : mine, decltype(kind)::value, glim, galpha);
+        }
+        pk[(c0 + i) / 2] = pack_bf16(res[0], res[1]);
       }
-      pk[(c0 + i) / 2] = pack_bf16(res[0], res[1]);
-    }
+    });
   }
   named_bar_sync(bar, 128);  // every exchange value has been consumed: the area is reused for the transposed tile
   __nv_bfloat16* out_s = reinterpret_cast<__nv_bfloat16*>(xg);  // [CG tokens][64 features]
@@ -681,37 +684,48 @@ PG_DEVINL void token_major_epilogue(const GemmArgs& args, uint32_t taddr, int m_
     // columns: [g0..g63 | u0..u63] per 128-column block; out feature = n_blk*BN/2 + blk*64 + c.  The 64 bf16
     // results of a block (one 128-byte row per token) leave through the warp transposition tile as full lines.
     const bool al = ((reinterpret_cast<uintptr_t>(args.out) & 15) == 0) && ((args.ldo % 8) == 0);
+    {
 #pragma unroll 1
-    for (int blk = ((EPI8 && BN >= 256) ? half : 0); blk < ((EPI8 && BN >= 256) ? half + 1 : (half == 0 ? BN / 128 : 0)); ++blk) {
-      const int f0 = n_blk * (BN / 2) + blk * 64;
-      if (f0 >= args.features / 2) break;  // warp-uniform (features % 128 == 0)
-      uint32_t pk[32];
+      for (int blk = ((EPI8 && BN >= 256) ? half : 0); blk < ((EPI8 && BN >= 256) ? half + 1 : (half == 0 ? BN / 128 : 0)); ++blk) {
+        const int f0 = n_blk * (BN / 2) + blk * 64;
+        if (f0 >= args.features / 2) break;  // warp-uniform (features % 128 == 0)
+        uint32_t pk[32];
 #pragma unroll
-      for (int c0 = 0; c0 < 64; c0 += 16) {
-        uint32_t g[16], u[16];
-        tmem_ld16(taddr + blk * 128 + c0, g);
-        tmem_ld16(taddr + blk * 128 + 64 + c0, u);
-        tmem_ld_wait();
-        const float* bg = args.bias != nullptr ? args.bias + n_blk * BN + blk * 128 + c0 : nullptr;  // packed order: [64 gate | 64 up]
+        for (int c0 = 0; c0 < 64; c0 += 32) {
+          // 32 pairs requested together: one wait for the accumulator per half block
+          uint32_t g[2][16], u[2][16];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          float g0 = __uint_as_float(g[2 * i]), g1 = __uint_as_float(g[2 * i + 1]), u0 = __uint_as_float(u[2 * i]), u1 = __uint_as_float(u[2 * i + 1]);
-          if (bg != nullptr) {
-            g0 += __ldg(bg + 2 * i); g1 += __ldg(bg + 2 * i + 1);
-            u0 += __ldg(bg + 64 + 2 * i); u1 += __ldg(bg + 64 + 2 * i + 1);
+          for (int h = 0; h < 2; ++h) {
+            tmem_ld16(taddr + blk * 128 + c0 + 16 * h, g[h]);
+            tmem_ld16(taddr + blk * 128 + 64 + c0 + 16 * h, u[h]);
           }
-          float a = glu_act(g0, u0, args.act_gelu, args.scale, args.glu_alpha);
-          float b = glu_act(g1, u1, args.act_gelu, args.scale, args.glu_alpha);
-          pk[(c0 / 2 + i) & 31] = pack_bf16(a, b);
-        }
-      }
-      if (al) {
-        warp_store_rows_128B(wstage, lane, pk, reinterpret_cast<char*>(out_bf + static_cast<long long>(m_blk * BM + q * 32) * args.ldo + f0),
-                             args.ldo * 2, rows_valid, true);
-      } else if (row_ok) {
-        __nv_bfloat16* dst = out_bf + static_cast<long long>(tok) * args.ldo + f0;
+          tmem_ld_wait();
+          const float* bg = args.bias != nullptr ? args.bias + n_blk * BN + blk * 128 + c0 : nullptr;  // packed order: [64 gate | 64 up]
+          if (bg != nullptr) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) *reinterpret_cast<uint32_t*>(dst + 2 * i) = pk[i];
+            for (int i = 0; i < 32; ++i) {
+              g[i / 16][i % 16] = __float_as_uint(__uint_as_float(g[i / 16][i % 16]) + __ldg(bg + i));
+              u[i / 16][i % 16] = __float_as_uint(__uint_as_float(u[i / 16][i % 16]) + __ldg(bg + 64 + i));
+            }
+          }
+          with_glu(args.act_gelu, [&](auto kind) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              const float a = glu_act(__uint_as_float(g[i / 8][2 * i % 16]), __uint_as_float(u[i / 8][2 * i % 16]), decltype(kind)::value, args.scale, args.glu_alpha);
+              const float b = glu_act(__uint_as_float(g[i / 8][2 * i % 16 + 1]), __uint_as_float(u[i / 8][2 * i % 16 + 1]), decltype(kind)::value, args.scale,
+                                      args.glu_alpha);
+              pk[(c0 / 2 + i) & 31] = pack_bf16(a, b);
+            }
+          });
+        }
+        if (al) {
+          warp_store_rows_128B(wstage, lane, pk, reinterpret_cast<char*>(out_bf + static_cast<long long>(m_blk * BM + q * 32) * args.ldo + f0),
+                               args.ldo * 2, rows_valid, true);
+        } else if (row_ok) {
+          __nv_bfloat16* dst = out_bf + static_cast<long long>(tok) * args.ldo + f0;
+#pragma unroll
+          for (int i = 0; i < 32; ++i) *reinterpret_cast<uint32_t*>(dst + 2 * i) = pk[i];
+        }
       }
     }
   } else if (mode == PG_EPI_BF16) {
@@ -1147,11 +1161,12 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& 
              ? PG_OK : PG_ERR_CUDA;
 }
 
-// Whether a token-major product takes the form of gemm_cluster.cu: up to 1408 tokens, but for plain epilogues that give the CTA-pair kernel one and
-// a half waves of 256 x 256 tiles.  Measured on both sides of the lines (us, this file's kernels / gemm_cluster.cu; N x K weights): 3456 x 1152
-// 263 tokens 14.4 / 8.2, 1024 17.0 / 10.8, 2048 20.2 / 22.2; 2048 x 2048 with residual 263 15.2 / 10.1, 1300 28.5 / 18.2; 2048 x 16384 with residual
-// 263 41 / 28, 1300 163 / 86, 2048 113 / 120; 32768 x 2048 gate || up 263 91 / 40, 1300 223 / 172; 5120 x 2048 1024 (80 pair tiles) 27.9 / 22.0, 1536
-// (120) 29.0 / 30.3; 8192 x 2048 706 (96) 28.6 / 23.4, 1024 (128) 29.3 / 31.5; 3072 x 768 1300 10.4 / 9.1, 1536 10.7 / 11.5.
+// Whether a token-major product takes the form of gemm_cluster.cu: up to 1408 tokens, where the CTA-pair kernel has no tile for every pair of SMs or
+// the estimate of its waves (740 clocks a 64-deep step, fitted to the times below) is the longer one.  Measured on both sides of the lines (us, this
+// file's kernels / gemm_cluster.cu; N x K weights): 3456 x 1152 263 tokens 14.4 / 8.2, 1024 17.0 / 10.8, 2048 20.2 / 22.2; 2048 x 2048 with residual
+// 263 15.2 / 10.1, 1300 28.5 / 18.2; 2048 x 16384 with residual 263 41 / 28, 1300 163 / 86, 2048 113 / 120; 3072 x 768 1300 10.4 / 9.1, 1536
+// 10.7 / 11.5; pair tiles: 32768 x 2048 gate || up 263 54 / 39, 400 56 / 64, 1024 101 / 133; 16384 x 2048 263 29 / 20, 400 29.7 / 29.7, 706 42 / 46;
+// 5120 x 2048 1024 27.9 / 22.0, 1536 29.0 / 30.3; 8192 x 2048 706 28.6 / 23.4, 1024 29.3 / 31.5.
 //
 // Decode-sized calls (up to 128 tokens): where its grid is one wave, but for long K with up to 64 tokens, which the two-CTAs-per-SM stream of this file's
 // swap kernels reads faster.  Not for split-K accumulation into a residual stream: in a chain of decode launches under the L2 prefetch stream of
@@ -1163,8 +1178,12 @@ static bool cluster_form(const GemmArgs& a, long long ldr, int swap) {
   if (a.features % 4 != 0 || a.ldo % 4 != 0 || !aligned(a.out, 16) || !aligned(a.bias, 16)) return false;
   if (a.resid != nullptr && (ldr % 4 != 0 || !aligned(a.resid, 16))) return false;
   if (swap) return a.mode != PG_EPI_ATOMIC_F32 && a.stats == nullptr && a.zero_buf == nullptr && (a.K <= 4096 || a.tokens > 64) && plan_cluster_gemm(a.tokens, a.features, a.K).waves == 1;
-  const int pair_tiles = ((a.tokens + 2 * BM - 1) / (2 * BM)) * ((a.features + 255) / 256);
-  return a.tokens <= 1408 && (a.mode == PG_EPI_GEGLU || pair_tiles < 3 * (num_sms() / 2) / 2);
+  if (a.tokens > 1408) return false;
+  const int pairs = num_sms() / 2, pair_tiles = ((a.tokens + 2 * BM - 1) / (2 * BM)) * ((a.features + 255) / 256);
+  if (pair_tiles < pairs || (a.mode == PG_EPI_BF16 && a.act_gelu)) return true;
+  const ClusterGemmPlan plan = plan_cluster_gemm(a.tokens, a.features, a.K);
+  // (CTAs of a second wave start one by one, against the estimate of whole waves: 12 % more)
+  return plan.clocks * (plan.waves > 1 ? 1.12f : 1.f) < (pair_tiles + pairs - 1) / pairs * ((a.K + BK - 1) / BK * 740.f + 1500.f) + 5000.f;
 }
 
 }  // namespace pg
@@ -1291,7 +1310,7 @@ extern "C" int pg_gemm_bf16_fused(const void* x, long long ldx, const void* w, l
     if ((rc = make_tmap_2d(&ta, x, tokens, K, ldx, BM)) != PG_OK) return rc;
     // many tokens: a PAIR of CTAs per 256 x 256 tile (cta_group::2), each staging half of the weight tile
     const int pair_tiles = ((tokens + 2 * BM - 1) / (2 * BM)) * ((features + 255) / 256);
-    // (measured per call site, profiles/r02h_gemm_pair_ab.txt: +2..16 % everywhere but the gelu epilogue of fc1, -3 %)
+    // (against one CTA per tile: +2 .. 16 % per call site but for the gelu epilogue of fc1: 4 vision layers on 8 x 1024 patches 1862 -> 1893 us)
     if (g_pair_mode != 0 && BN == 256 && split_k == 1 && pair_tiles >= g_pair_min_tiles && !(mode == PG_EPI_BF16 && act_gelu)) {
       if (band_rows > 0) a.n_fast = 2 + (static_cast<int>(band_rows) / (2 * BM) > 0 ? static_cast<int>(band_rows) / (2 * BM) : 1);
       if ((rc = make_tmap_2d(&tb, w, features, K, ldw, PAIR_BN / 2)) != PG_OK) return rc;
