@@ -657,6 +657,12 @@ int pg_moe_gemm(const void* x, long long ldx, const int* sorted_pair, int src_di
  * every expert as one contiguous run of rows, for per-expert dense products. */
 int pg_moe_gather_rows(const void* x, long long ldx, const int* sorted_pair, const int* total_rows, int top, void* xg, long long ldg,
                        int max_rows, int D, int act_f32, void* stream);
+/* Both products of every chosen expert over few rows: xg (bf16 scratch [pairs, D]) = the plan's rows of x, mid = act(xg W_up^T) (bf16 scratch [pairs, F]),
+ * eo (fp32 [pairs, D]) = mid W_down^T, rows in the plan's order.  w_up [n_real, F, D] (act 3: [n_real, 2 F, D], rows alternate gate / up), w_down
+ * [n_real, D, F], dense; act 0, 2, 3 or 6.  total_rows: the number of rows on the device (the last word of the plan's offsets). */
+int pg_moe_products(const void* x, long long ldx, const int* sorted_pair, const int* total_rows, int top, void* xg, const void* w_up, const void* w_down, void* mid,
+                    float* eo, const int* plan, int max_tiles, int pairs, int n_real, int D, int F, int act, void* stream);
+
 /* Per-expert dense products over the gathered runs: expert e owns the next counts_host[e] rows (host array, n_real entries);
  * mid[rows, F] = act(xg W_up[e]^T) in bf16, eo[rows, D] = mid W_down[e]^T in fp32, both through pg_gemm_bf16.  bf16 only;
  * D, F and the pitches multiples of 8.  act: 2 relu(x)^2, 6 gelu (erf form); 3: w_up holds [n_real, 2F, D] with gate and up rows in blocks of 64

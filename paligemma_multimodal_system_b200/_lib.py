@@ -98,6 +98,7 @@ SIGNATURES = {
     "pg_moe_plan": [p, p, p, p, p, p, p, i32, i32, i32, p],
     "pg_moe_gemm": [p, i64, p, i32, p, i64, i64, p, i64, p, i32, i32, i32, i32, i32, i32, i64, i64, p],
     "pg_moe_gather_rows": [p, i64, p, p, i32, p, i64, i32, i32, i32, p],
+    "pg_moe_products": [p, i64, p, p, i32, p, p, p, p, p, p, i32, i32, i32, i32, i32, i32, p],
     "pg_moe_dense_runs": [p, i64, p, p, p, i64, p, i64, p, i32, i32, i32, i32, p],
     "pg_moe_combine": [p, i64, p, p, p, p, i64, p, i64, p, i32, i32, i32, i32, p, i64, i32, p],
     "pg_gemm_simt_bias": [p, i64, p, i64, p, i64, p, i32, f32, i32, i32, i32, i32, i32, p],

@@ -52,15 +52,25 @@ PG_DEVINL float4 gather4(uint32_t addr, int S) {
   return v;
 }
 
-template <bool SPLIT>
-__global__ void __launch_bounds__(kThreads, 1) gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmapW, const __grid_constant__ CUtensorMap tmapX,
+// GROUPED: a CTA takes a tile of a device-side plan (one expert's rows); everything it reads may come from the kernel before, the plan included.
+template <bool SPLIT, bool GROUPED = false>
+__global__ void __launch_bounds__(kThreads, GROUPED ? 2 : 1) gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmapW, const __grid_constant__ CUtensorMap tmapX,
                                                                    const ClusterGemmArgs args) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t smem_base = smem_u32(smem_raw);
   if ((smem_base & 1023u) != 0) __trap();
   constexpr int kU = SPLIT ? 2 : 4;  // tokens a thread finishes together
   const int S = SPLIT ? args.split : 1, rank = SPLIT ? static_cast<int>(cluster_ctarank()) : 0;
-  const int f0 = (blockIdx.x / S) * kFeat, t0 = blockIdx.y * args.tile_tokens;
+  const int f0 = (blockIdx.x / S) * kFeat;
+  int t0 = blockIdx.y * args.tile_tokens, w0 = f0, t_end = args.tokens;  // first token and weight row of the tile, end of its tokens
+  if (GROUPED) {
+    griddep_wait();
+    if (static_cast<int>(blockIdx.y) >= args.plan[0]) return;
+    const int* tile = args.plan + 4 + 3 * blockIdx.y;
+    w0 += tile[0] * args.features;
+    t0 = tile[1];
+    t_end = t0 + tile[2];
+  }
   const int stages = args.stages, stage_bytes = kATile + args.tile_tokens * 128;
   const int total_kb = (args.K + kKb - 1) / kKb, per = (total_kb + S - 1) / S;
   const int kb0 = rank * per, nkb = min(total_kb, kb0 + per) - kb0;  // (host: no empty rank)
@@ -97,9 +107,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_cluster_kernel(const __grid_
       const int pre = min(stages, nkb);
       for (int s = 0; s < pre; ++s) {  // weights do not depend on the kernel before: requested ahead of the dependency wait
         mbar_expect_tx(full_bar(s), stage_bytes);
-        tma_load_2d(smem_base + s * stage_bytes, &tmapW, full_bar(s), (kb0 + s) * kKb, f0, kEvictNormal);
+        tma_load_2d(smem_base + s * stage_bytes, &tmapW, full_bar(s), (kb0 + s) * kKb, w0, kEvictNormal);
       }
-      griddep_wait();
+      if (!GROUPED) griddep_wait();
       griddep_launch_dependents();
       int stage = 0;
       uint32_t phase = 0;
@@ -108,7 +118,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_cluster_kernel(const __grid_
         if (kb >= pre) {
           mbar_wait(empty_bar(stage), phase ^ 1);
           mbar_expect_tx(full_bar(stage), stage_bytes);
-          tma_load_2d(sa, &tmapW, full_bar(stage), (kb0 + kb) * kKb, f0, kEvictNormal);
+          tma_load_2d(sa, &tmapW, full_bar(stage), (kb0 + kb) * kKb, w0, kEvictNormal);
         }
         for (int c = 0; c < chunks; ++c)
           tma_load_2d(sa + kATile + c * chunk * 128, &tmapX, full_bar(stage), (kb0 + kb) * kKb, t0 + c * chunk, kEvictLast);
@@ -143,7 +153,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_cluster_kernel(const __grid_
     mbar_wait(done_bar, 0);
     tc_fence_after();
     const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
-    const int valid = min(args.tile_tokens, args.tokens - t0);
+    const int valid = min(args.tile_tokens, t_end - t0);
     for (int c = half * 16; c < valid; c += 32) {
       uint32_t r[16];
       tmem_ld16(taddr + c, r);
@@ -160,10 +170,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_cluster_kernel(const __grid_
     tmem_dealloc(tmem_base, cols);
   }
   if (warp >= 2) {
-    griddep_wait();  // residual and output may belong to kernels before
+    if (!GROUPED) griddep_wait();  // residual and output may belong to kernels before
     const int et = threadIdx.x - 64;
     const int share = (args.tile_tokens + S - 1) / S, lo = rank * share;
-    const int hi = min(min(args.tile_tokens, lo + share), args.tokens - t0);
+    const int hi = min(min(args.tile_tokens, lo + share), t_end - t0);
     const float scale = args.scale;
     if (args.mode == PG_EPI_GEGLU) {
       // rows of a weight tile: [64 gate | 64 up]; half a warp takes the 64 outputs of one token
@@ -224,7 +234,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_cluster_kernel(const __grid_
             for (int j = 0; j < kU; ++j) {
               if (t + 8 * j >= hi) break;
               v[j].x = fmaf(v[j].x, scale, b.x); v[j].y = fmaf(v[j].y, scale, b.y); v[j].z = fmaf(v[j].z, scale, b.z); v[j].w = fmaf(v[j].w, scale, b.w);
-              if (args.mode == PG_EPI_BF16) {
+              if (GROUPED && decltype(act)::value == 3) {  // neighbouring features are a gate and its up value
+                *reinterpret_cast<uint32_t*>(static_cast<__nv_bfloat16*>(args.out) + static_cast<long long>(t0 + t + 8 * j) * args.ldo + f / 2) =
+                    pack_bf16(v[j].x / (1.0f + expf(-v[j].x)) * v[j].y, v[j].z / (1.0f + expf(-v[j].z)) * v[j].w);
+              } else if (args.mode == PG_EPI_BF16) {
                 if (decltype(act)::value) {
                   v[j].x = epilogue_act(v[j].x, decltype(act)::value); v[j].y = epilogue_act(v[j].y, decltype(act)::value);
                   v[j].z = epilogue_act(v[j].z, decltype(act)::value); v[j].w = epilogue_act(v[j].w, decltype(act)::value);
@@ -237,7 +250,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_cluster_kernel(const __grid_
             }
           }
         };
-        with_act(args.mode == PG_EPI_BF16 ? args.act : 0, rows);
+        if (GROUPED && args.act == 3) rows(ActConst<3>{});
+        else with_act(args.mode == PG_EPI_BF16 ? args.act : 0, rows);
       }
     }
   }
@@ -249,7 +263,8 @@ bool configure() {
   const int dev = current_device();
   if (!configured[dev]) {
     if (cudaFuncSetAttribute(gemm_cluster_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax + 256) != cudaSuccess ||
-        cudaFuncSetAttribute(gemm_cluster_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax + 256) != cudaSuccess) {
+        cudaFuncSetAttribute(gemm_cluster_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax + 256) != cudaSuccess ||
+        cudaFuncSetAttribute(gemm_cluster_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax + 256) != cudaSuccess) {
       cudaGetLastError();  // do not leave a sticky error behind
       return false;
     }
@@ -340,6 +355,28 @@ int launch_cluster_gemm(const ClusterGemmPlan& plan, const void* x, long long ld
   cfg.numAttrs = pg_pdl_enabled() ? 2 : 1;
   pg_count_launch(1);
   return cudaLaunchKernelEx(&cfg, a.split > 1 ? gemm_cluster_kernel<true> : gemm_cluster_kernel<false>, tw, tx, a) == cudaSuccess ? PG_OK : PG_ERR_CUDA;
+}
+
+int launch_grouped_gemm(const void* x, int rows, int K, const void* w, int experts, int F, void* out, bool out_f32, int act, const int* plan, int max_tiles,
+                        int most_rows, cudaStream_t st) {
+  if (!configure() || max_tiles <= 0 || max_tiles > 65535) return PG_ERR_CUDA;
+  ClusterGemmArgs a = {};
+  a.tokens = rows; a.features = F; a.K = K; a.mode = out_f32 ? PG_EPI_F32 : PG_EPI_BF16; a.act = act; a.scale = 1.f; a.out = out; a.plan = plan;
+  a.ldo = act == 3 ? F / 2 : F;
+  a.split = 1;
+  a.tile_tokens = most_rows >= 64 ? 64 : (most_rows + 15) / 16 * 16;  // (an expert has no more rows than the step has tokens)
+  // two CTAs per SM: tiles are short and their number is known to the device only
+  const int stage = kATile + a.tile_tokens * 128, per = (K + kKb - 1) / kKb;
+  a.stages = 104 * 1024 / stage < 8 ? 104 * 1024 / stage : 8;
+  if (a.stages > per) a.stages = per < 2 ? 2 : per;
+  const int exchange = a.tile_tokens * kFeat * 4, tiles = a.stages * stage > exchange ? a.stages * stage : exchange;
+  a.smem_tiles = (tiles + 1023) / 1024 * 1024;
+  CUtensorMap tw, tx;
+  int rc;
+  if ((rc = make_tmap_2d(&tw, w, static_cast<long long>(experts) * F, K, K, kFeat)) != PG_OK) return rc;
+  if ((rc = make_tmap_2d(&tx, x, rows, K, K, a.tile_tokens)) != PG_OK) return rc;
+  return launch_kernel(gemm_cluster_kernel<false, true>, dim3((F + kFeat - 1) / kFeat, max_tiles), dim3(kThreads), a.smem_tiles + 256, st, tw, tx, a) == cudaSuccess
+             ? PG_OK : PG_ERR_CUDA;
 }
 
 }  // namespace pg

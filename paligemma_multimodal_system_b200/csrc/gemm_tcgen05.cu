@@ -1178,6 +1178,7 @@ static bool cluster_form(const GemmArgs& a, long long ldr, int swap) {
   if (a.features % 4 != 0 || a.ldo % 4 != 0 || !aligned(a.out, 16) || !aligned(a.bias, 16)) return false;
   if (a.resid != nullptr && (ldr % 4 != 0 || !aligned(a.resid, 16))) return false;
   if (swap) return a.mode != PG_EPI_ATOMIC_F32 && a.stats == nullptr && a.zero_buf == nullptr && (a.K <= 4096 || a.tokens > 64) && plan_cluster_gemm(a.tokens, a.features, a.K).waves == 1;
+  if (a.K <= 128 && a.tokens <= 4096) return true;  // (all epilogue: 2048 x 64 3750 tokens 14.6 / 9.3, 8192 25.9 / 28.0; K 256 15.9 / 16.9)
   if (a.tokens > 1408) return false;
   const int pairs = num_sms() / 2, pair_tiles = ((a.tokens + 2 * BM - 1) / (2 * BM)) * ((a.features + 255) / 256);
   if (pair_tiles < pairs || (a.mode == PG_EPI_BF16 && a.act_gelu)) return true;

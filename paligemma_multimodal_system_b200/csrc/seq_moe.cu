@@ -14,6 +14,7 @@
 //
 // Router arithmetic, weights and the combine are fp32.
 #include "common.cuh"
+#include "gemm_cluster.h"
 #include "paligemma_b200.h"
 
 using bf16 = __nv_bfloat16;
@@ -600,6 +601,24 @@ extern "C" int pg_moe_gather_rows(const void* x, long long ldx, const int* sorte
   else
     moe_gather_rows_kernel<bf16><<<grid, 128, 0, PG_ST(stream)>>>(static_cast<const bf16*>(x), ldx, sorted_pair, total_rows, top, static_cast<bf16*>(xg), ldg, D);
   PG_RET();
+}
+
+// Few rows per expert (decode and mixed steps): the rows gathered into runs, then one grouped tcgen05 product each for the up and the down projections,
+// whose CTAs walk the device-side plan.  What bounds them is the weights of the chosen experts (HBM) and the 64 bytes a clock an SM takes in from L2; the
+// mma.sync kernel above, which gathers on the way, is bound by its fragment reads.  top 4 of 14 experts 2048 x 1024 (117 MB = 18 us): 300
+// tokens 102 -> 42 us, 64 tokens 61 -> 32, one token 48 -> 22.
+extern "C" int pg_moe_products(const void* x, long long ldx, const int* sorted_pair, const int* total_rows, int top, void* xg, const void* w_up, const void* w_down,
+                               void* mid, float* eo, const int* plan, int max_tiles, int pairs, int n_real, int D, int F, int act, void* stream) {
+  if (pairs <= 0 || n_real <= 0 || top <= 0 || D <= 0 || F <= 0 || D % 8 != 0 || F % 8 != 0 || (act != 0 && act != 2 && act != 3 && act != 6)) return PG_ERR_ARG;
+  if ((reinterpret_cast<uintptr_t>(xg) | reinterpret_cast<uintptr_t>(w_up) | reinterpret_cast<uintptr_t>(w_down) | reinterpret_cast<uintptr_t>(mid) |
+       reinterpret_cast<uintptr_t>(eo)) & 15)
+    return PG_ERR_ARG;
+  int rc = pg_moe_gather_rows(x, ldx, sorted_pair, total_rows, top, xg, D, pairs, D, 0, stream);
+  if (rc != PG_OK) return rc;
+  cudaStream_t st = PG_ST(stream);
+  const int most = (pairs + top - 1) / top;  // rows of one expert at most: a token chooses it once
+  if ((rc = pg::launch_grouped_gemm(xg, pairs, D, w_up, n_real, act == 3 ? 2 * F : F, mid, false, act, plan, max_tiles, most, st)) != PG_OK) return rc;
+  return pg::launch_grouped_gemm(mid, pairs, F, w_down, n_real, D, eo, true, 0, plan, max_tiles, most, st);
 }
 
 // Every expert's run of gathered rows through two dense tensor-core products (tcgen05 kernels of pg_gemm_bf16), issued from

@@ -670,6 +670,9 @@ class RoutedFeedForward:
                                                     eo.data_ptr(), eo.stride(0), C.addressof(per), self.n_real, self.D, self.F, self.act, _lib.stream()),
                        "pg_moe_dense_runs")
             return eo
+        if not prec.f32 and self.D % 8 == 0 and self.F % 8 == 0 and plan.max_tiles <= 65535:
+            return seq_ops.moe_products(h, plan, self.w_up, self.w_down, prec.empty(plan.pairs, self.D), prec.empty(plan.pairs, self.F),
+                                        torch.empty(plan.pairs, self.D, device="cuda", dtype=torch.float32), self.act)
         mid = seq_ops.moe_gemm(h, plan, self.w_up, prec.empty(plan.pairs, self.F), gather=True, act=self.act)
         return seq_ops.moe_gemm(mid, plan, self.w_down, torch.empty(plan.pairs, self.D, device="cuda", dtype=torch.float32), gather=False)
 

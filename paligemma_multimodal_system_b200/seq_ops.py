@@ -571,6 +571,18 @@ def moe_gemm(x, plan: MoePlan, w, out, gather, act=0):
     return out
 
 
+def moe_products(x, plan: MoePlan, w_up, w_down, xg, mid, eo, act):
+    """eo[row] = act(x[token of row] @ w_up[expert(row)].T) @ w_down[expert(row)].T over the plan's rows (bf16; eo fp32); xg, mid: scratch."""
+    n_real, D, F = w_down.shape
+    assert x.dtype == w_up.dtype == w_down.dtype == xg.dtype == mid.dtype == torch.bfloat16 and eo.dtype == torch.float32 and x.stride(1) == 1
+    assert all(t.is_contiguous() for t in (w_up, w_down, xg, mid, eo)) and x.shape[1] == D and w_up.shape == (n_real, 2 * F if act == ACT_SILU_GLU else F, D)
+    assert xg.shape == (plan.pairs, D) and mid.shape == (plan.pairs, F) and eo.shape == (plan.pairs, D)
+    _lib.check(_lib.lib().pg_moe_products(x.data_ptr(), x.stride(0), plan.sorted_pair.data_ptr(), plan.offsets.data_ptr() + 4 * n_real, plan.top, xg.data_ptr(),
+                                          w_up.data_ptr(), w_down.data_ptr(), mid.data_ptr(), eo.data_ptr(), plan.plan.data_ptr(), plan.max_tiles, plan.pairs,
+                                          n_real, D, F, int(act), _lib.stream()), "pg_moe_products")
+    return eo
+
+
 def moe_gather_rows(x, plan: MoePlan, out):
     """out[row] = x[token of sorted pair `row`]: every expert's tokens as one contiguous run of rows."""
     assert x.dtype == out.dtype and x.stride(1) == 1 and out.stride(1) == 1 and out.shape[0] >= plan.pairs

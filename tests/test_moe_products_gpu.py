@@ -1,0 +1,46 @@
+"""pg_moe_products (grouped tcgen05 products over the routing plan) against 64-bit products of the same rows.
+
+Bounds: the activations between the products are bf16 (2^-8 of the value that is rounded; the silu / relu^2 slope carries the sum's error), sums are fp32."""
+import pytest
+import torch
+
+from paligemma_multimodal_system_b200 import seq_ops
+
+pytestmark = pytest.mark.gpu
+
+ACTS = {seq_ops.ACT_NONE: lambda z: z, seq_ops.ACT_RELU2: lambda z: z.clamp(min=0) ** 2, seq_ops.ACT_GELU_ERF: torch.nn.functional.gelu}
+
+
+@pytest.mark.parametrize("T,top,n", [(1, 1, 1), (1, 4, 9), (5, 2, 3), (16, 4, 6), (17, 3, 40), (64, 2, 2), (65, 1, 3), (300, 4, 14), (700, 2, 5)])
+@pytest.mark.parametrize("D,F", [(64, 8), (136, 200), (2048, 1024), (72, 520)])
+@pytest.mark.parametrize("act", [seq_ops.ACT_NONE, seq_ops.ACT_RELU2, seq_ops.ACT_GELU_ERF, seq_ops.ACT_SILU_GLU])
+def test_against_64_bits(T, top, n, D, F, act):
+    g = torch.Generator(device="cuda").manual_seed(T * 31 + D + act)
+    ids = torch.stack([torch.randperm(n + 1, generator=g, device="cuda")[:top] for _ in range(T)]).to(torch.int32)  # id n: an identity output, no row
+    counts = torch.bincount(ids[ids < n].long(), minlength=n).to(torch.int32)
+    plan = seq_ops.MoePlan(ids.contiguous(), counts, n)
+    glu = act == seq_ops.ACT_SILU_GLU
+    x = torch.randn(T, D, generator=g, device="cuda").bfloat16()
+    up = (torch.randn(n, 2 * F if glu else F, D, generator=g, device="cuda") * D ** -0.5).bfloat16()
+    down = (torch.randn(n, D, F, generator=g, device="cuda") * F ** -0.5).bfloat16()
+    xg, mid = torch.empty(plan.pairs, D, device="cuda", dtype=torch.bfloat16), torch.empty(plan.pairs, F, device="cuda", dtype=torch.bfloat16)
+    eo = torch.full((plan.pairs, D), float("nan"), device="cuda")
+    seq_ops.moe_products(x, plan, up, down, xg, mid, eo, act)
+    for t in range(T):
+        for k in range(top):
+            e, row = int(ids[t, k]), int(plan.pair_row[t * top + k])
+            if e >= n:
+                assert row == -1
+                continue
+            if t % 7 and T > 64:
+                continue
+            z = up[e].double() @ x[t].double()
+            if glu:
+                want = z[0::2] * torch.sigmoid(z[0::2]) * z[1::2]
+                slope = z.abs().view(-1, 2).amax(1) + 1
+            else:
+                want, slope = ACTS[act](z), 2 * z.abs() + 2
+            err = 2.0 ** -8 * want.abs() + 2.0 ** -18 * slope ** 2
+            assert ((mid[row].double() - want).abs() <= err).all()
+            got = down[e].double() @ mid[row].double()
+            assert ((eo[row].double() - got).abs() <= 2.0 ** -20 * (down[e].double().abs() @ mid[row].double().abs()) + 1e-30).all()
