@@ -224,10 +224,7 @@ __global__ void __launch_bounds__(128) attn_prepare_vec_kernel(const TA* __restr
 #pragma unroll
     for (int k = 0; k < TOK; ++k) {
       float inv = 1.0f;
-      if ((is_q || is_k) && norm_qk == 2) {
-        const float* ps = part[is_q ? 0 : 1][k];
-        inv = 1.0f / sqrtf((ps[0] + ps[1] + ps[2] + ps[3]) / (float)(8 * (is_q ? nq : nk)) + eps);
-      } else if (norm_qk == 1 || norm_v) {  // (uniform: every lane takes part in the shuffles, the others' sums are not used)
+      if (norm_qk == 1 || norm_v) {  // (uniform: every lane takes part in the shuffles, whatever it holds; sums that are not wanted are not used)
         float s = 0.f;
 #pragma unroll
         for (int i = 0; i < 8; ++i) s = in ? fmaf(x[k][i], x[k][i], s) : 0.f;
@@ -236,6 +233,10 @@ __global__ void __launch_bounds__(128) attn_prepare_vec_kernel(const TA* __restr
           if (o < lph) s += u;
         }
         if ((is_q || is_k) ? norm_qk == 1 : norm_v) inv = 1.0f / sqrtf(s / (float)(8 * lph) + eps);
+      }
+      if ((is_q || is_k) && norm_qk == 2) {
+        const float* ps = part[is_q ? 0 : 1][k];
+        inv = 1.0f / sqrtf((ps[0] + ps[1] + ps[2] + ps[3]) / (float)(8 * (is_q ? nq : nk)) + eps);
       }
       const int t = t0 + k;
       if (!in || t >= rows) continue;

@@ -18,9 +18,10 @@ def _batch(entries):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("entries", [[(1, 70)] * 5, [(130, 0), (1, 3), (77, 60)], [(2500, 0)]])
-@pytest.mark.parametrize("H,G,dim,vdim,rot", [(4, 2, 64, 64, 64), (6, 3, 16, 8, 6), (2, 1, 256, 32, 0), (8, 8, 32, 128, 10)])
-@pytest.mark.parametrize("norm_qk,norm_v,form", [(False, False, ""), (True, True, ""), (True, False, "keys"), (seq_ops.NORM_PROJECTION, False, "blend"), (True, False, "queries")])
+@pytest.mark.parametrize("entries", [[(1, 70)] * 5, [(130, 0), (1, 3), (77, 60)], [(2500, 0)], [(2501, 0)], [(2400, 3), (103, 0)]])
+@pytest.mark.parametrize("H,G,dim,vdim,rot", [(4, 2, 64, 64, 64), (6, 3, 16, 8, 6), (2, 1, 256, 32, 0), (8, 8, 32, 128, 10), (8, 1, 64, 64, 16)])
+@pytest.mark.parametrize("norm_qk,norm_v,form", [(False, False, ""), (True, True, ""), (True, False, "keys"), (seq_ops.NORM_PROJECTION, False, "blend"), (seq_ops.NORM_PROJECTION, True, ""),
+                                              (True, False, "queries")])
 def test_attn_prepare(dtype, entries, H, G, dim, vdim, rot, norm_qk, norm_v, form):
     if norm_v or form == "keys":
         vdim = dim
