@@ -364,7 +364,7 @@ int launch_grouped_gemm(const void* x, int rows, int K, const void* w, int exper
   a.tokens = rows; a.features = F; a.K = K; a.mode = out_f32 ? PG_EPI_F32 : PG_EPI_BF16; a.act = act; a.scale = 1.f; a.out = out; a.plan = plan;
   a.ldo = act == 3 ? F / 2 : F;
   a.split = 1;
-  a.tile_tokens = most_rows >= 64 ? 64 : (most_rows + 15) / 16 * 16;  // (an expert has no more rows than the step has tokens)
+  a.tile_tokens = most_rows >= 64 ? 64 : (most_rows + 15) / 16 * 16;  // (the plan's tiles hold up to 64 rows)
   // two CTAs per SM: tiles are short and their number is known to the device only
   const int stage = kATile + a.tile_tokens * 128, per = (K + kKb - 1) / kKb;
   a.stages = 104 * 1024 / stage < 8 ? 104 * 1024 / stage : 8;

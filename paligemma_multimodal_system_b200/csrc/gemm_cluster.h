@@ -29,7 +29,8 @@ struct ClusterGemmPlan {
 ClusterGemmPlan plan_cluster_gemm(int tokens, int features, int K);
 int launch_cluster_gemm(const ClusterGemmPlan& plan, const void* x, long long ldx, const void* w, long long ldw, ClusterGemmArgs a, cudaStream_t st);
 
-// One product per expert over its run of rows: out[r, :] = act(x[r, :] W_e^T) for the rows of every tile of `plan` (at most `max_tiles`, 64 rows each).
+// One product per expert over its run of rows: out[r, :] = act(x[r, :] W_e^T) for the rows of every tile of `plan` (at most `max_tiles`, 64 rows each, and
+// `most_rows` of them where that is fewer).
 // w: [experts * F, K] dense; act 3: rows alternate gate / up, out has F / 2 columns; out bf16, or fp32 without activation.
 int launch_grouped_gemm(const void* x, int rows, int K, const void* w, int experts, int F, void* out, bool out_f32, int act, const int* plan, int max_tiles,
                         int most_rows, cudaStream_t st);

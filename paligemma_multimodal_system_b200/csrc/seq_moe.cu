@@ -616,7 +616,7 @@ extern "C" int pg_moe_products(const void* x, long long ldx, const int* sorted_p
   int rc = pg_moe_gather_rows(x, ldx, sorted_pair, total_rows, top, xg, D, pairs, D, 0, stream);
   if (rc != PG_OK) return rc;
   cudaStream_t st = PG_ST(stream);
-  const int most = (pairs + top - 1) / top;  // rows of one expert at most: a token chooses it once
+  const int most = pairs;  // rows of one tile at most: a token may choose one expert several times (its choice scores are NaN, or the ids come from elsewhere)
   if ((rc = pg::launch_grouped_gemm(xg, pairs, D, w_up, n_real, act == 3 ? 2 * F : F, mid, false, act, plan, max_tiles, most, st)) != PG_OK) return rc;
   return pg::launch_grouped_gemm(mid, pairs, F, w_down, n_real, D, eo, true, 0, plan, max_tiles, most, st);
 }

@@ -44,3 +44,29 @@ def test_against_64_bits(T, top, n, D, F, act):
             assert ((mid[row].double() - want).abs() <= err).all()
             got = down[e].double() @ mid[row].double()
             assert ((eo[row].double() - got).abs() <= 2.0 ** -20 * (down[e].double().abs() @ mid[row].double().abs()) + 1e-30).all()
+
+
+@pytest.mark.parametrize("T,top,n", [(16, 4, 2), (32, 3, 2), (48, 4, 2)])
+def test_one_token_may_choose_an_expert_again(T, top, n):
+    """A token whose router scores are NaN takes expert 0 every time: that expert then owns more rows than the step has tokens, and the other tokens' rows are
+    what they are without it."""
+    D, F = 64, 72
+    logits = torch.randn(T, max(n, top), device="cuda")
+    logits[0] = float("nan")
+    ids, _, counts = seq_ops.moe_route(logits, None, n, top, 1, 1, 1.0)
+    plan = seq_ops.MoePlan(ids, counts, n)
+    assert int(counts.max()) > T
+    x = torch.randn(T, D, device="cuda").bfloat16()
+    up, down = torch.randn(n, F, D, device="cuda").bfloat16(), torch.randn(n, D, F, device="cuda").bfloat16()
+    xg, mid = torch.empty(plan.pairs, D, device="cuda", dtype=torch.bfloat16), torch.empty(plan.pairs, F, device="cuda", dtype=torch.bfloat16)
+    eo = torch.full((plan.pairs, D), float("nan"), device="cuda")
+    seq_ops.moe_products(x, plan, up, down, xg, mid, eo, seq_ops.ACT_NONE)
+    for t in range(T):
+        for k in range(top):
+            e, row = int(ids[t, k]), int(plan.pair_row[t * top + k])
+            if e >= n:
+                continue
+            z = up[e].double() @ x[t].double()
+            assert ((mid[row].double() - z).abs() <= 2.0 ** -8 * z.abs() + 2.0 ** -18 * (up[e].double().abs() @ x[t].double().abs())).all()
+            got = down[e].double() @ mid[row].double()
+            assert ((eo[row].double() - got).abs() <= 2.0 ** -20 * (down[e].double().abs() @ mid[row].double().abs()) + 1e-30).all()
