@@ -2,6 +2,8 @@
 
 Bound per element: bf16 products are exact in fp32, the tensor core adds them with at most one unit in the last place per addition, so the sum is
 within K 2^-23 sum_k |x w|; an fp32 result adds four roundings, a bf16 result 2^-8 of itself, gelu / silu in their fast forms 2^-10 of the operands."""
+import json
+
 import pytest
 import torch
 
@@ -88,3 +90,20 @@ def test_row_map_and_table(T):
     _lib.gemm(x, w, out, mode=_lib.EPI_F32, bias=b, resid=table, resid_row_mod=N, swap=0)
     want = acc + b.double() + table.double()[torch.arange(T, device="cuda") % N]
     _check(out, want, bound + 2.0 ** -21 * (want.abs() + 4))
+
+
+@pytest.mark.parametrize("T,F,K", [(16, 256, 512), (40, 640, 2048), (300, 512, 1024), (129, 1152, 4304)])
+def test_clustered_ctas_have_an_sm_to_themselves(T, F, K, tmp_path):
+    """A CTA that shares K with others holds tensor memory while it waits for them, so no second one may fit beside it: its launch asks for more than half of
+    an SM's 228 KB of shared memory (1 KB a CTA belongs to the system)."""
+    x, w, b, acc, bound = _operands(T, F, K, 1)
+    out = torch.empty(T, F, device="cuda")
+    _lib.gemm(x, w, out, mode=_lib.EPI_F32, swap=0)
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        _lib.gemm(x, w, out, mode=_lib.EPI_F32, swap=0)
+        torch.cuda.synchronize()
+    prof.export_chrome_trace(str(tmp_path / "trace.json"))
+    launches = [e["args"] for e in json.load(open(tmp_path / "trace.json"))["traceEvents"] if "gemm_cluster_kernel<true" in e.get("name", "")]
+    assert launches and all(2 * (a["shared memory"] + 1024) > 228 * 1024 for a in launches)
+    _check(out, acc, bound + 2.0 ** -22 * acc.abs())
