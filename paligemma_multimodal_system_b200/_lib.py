@@ -176,9 +176,23 @@ class GemmaPrefill(C.Structure):
                 + [(n, i32) for n in ("B", "S", "D", "F", "Hq", "Hkv", "dh", "page", "max_pages", "fused")] + [("eps", f32)])
 
 
-def layer_array(kind, layers):
-    """ctypes array of `kind` from the packed tensors of every layer (dicts with the struct's field names; they must outlive the array)."""
-    return (kind * len(layers))(*[kind(*[l[n].data_ptr() for n, _ in kind._fields_]) for l in layers])
+class _LayerArray:
+    """A ctypes array of weight addresses.  They are good for the tensors of one model in one process: a deep copy or a pickle has None in its place."""
+    __slots__ = ("array",)
+
+    def __init__(self, array):
+        self.array = array
+
+    def __reduce__(self):
+        return type(None), ()
+
+
+def layer_array(kind, packed):
+    """Array of `kind` over packed["layers"] (dicts of tensors with the struct's field names), built on first use and kept beside them."""
+    holder = packed.get("array")
+    if holder is None:
+        holder = packed["array"] = _LayerArray((kind * len(packed["layers"]))(*[kind(*[l[n].data_ptr() for n, _ in kind._fields_]) for l in packed["layers"]]))
+    return holder.array
 
 
 _lib = None

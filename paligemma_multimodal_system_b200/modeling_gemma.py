@@ -264,7 +264,6 @@ class GemmaForCausalLM(nn.Module):
                 qkv_w=torch.cat([_bf16(a.q_proj.weight), _bf16(a.k_proj.weight), _bf16(a.v_proj.weight)], 0).contiguous(),
                 o_w=_bf16(a.o_proj.weight), gu_w=gu, down_w=_bf16(l.mlp.down_proj.weight)))
             del gate, up
-        pk["array"] = _lib.layer_array(_lib.GemmaLayer, pk["layers"])
         torch.cuda.synchronize()
         self._packed = pk
         return pk
@@ -320,7 +319,7 @@ class GemmaForCausalLM(nn.Module):
                                  pk["inv_freq"].data_ptr(), _lib.ptr(kp), _lib.ptr(kv_cache.v_pages) if have_cache else 0,
                                  kp.stride(0) * kp.element_size() if have_cache else 0, _lib.ptr(page_table), slot_base.data_ptr() if have_cache else 0,
                                  _lib.ptr(lens), B, S, D, F, Hq, Hkv, dh, PAGE, page_table.shape[1] if have_cache else 0, int(fused), 1e-6)
-        _lib.check(L.pg_gemma_prefill_layers(C.addressof(pk["array"]), len(pk["layers"]), C.addressof(args), st), "pg_gemma_prefill_layers")
+        _lib.check(L.pg_gemma_prefill_layers(_lib.layer_array(_lib.GemmaLayer, pk), len(pk["layers"]), C.addressof(args), st), "pg_gemma_prefill_layers")
         if have_cache and page_rows is None:
             kv_cache._set_len(S, c.num_hidden_layers)
         if last_only:

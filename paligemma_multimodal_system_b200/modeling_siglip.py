@@ -10,8 +10,6 @@ packs the parameters once (bf16, fused QKV) and runs
 
 through the C ABI (include/paligemma_b200.h).  The residual stream stays fp32 as in the reference.
 """
-import ctypes as C
-
 import torch
 import torch.nn as nn
 
@@ -141,7 +139,6 @@ class SiglipVisionModel(nn.Module):
                 ln2_w=_f32(l.layer_norm2.weight), ln2_b=_f32(l.layer_norm2.bias),
                 fc1_w=_bf16(l.mlp.fc1.weight), fc1_b=_f32(l.mlp.fc1.bias),
                 fc2_w=_bf16(l.mlp.fc2.weight), fc2_b=_f32(l.mlp.fc2.bias)))
-        pk["array"] = _lib.layer_array(_lib.SiglipLayer, pk["layers"])
         self._packed = pk
         return pk
 
@@ -171,7 +168,7 @@ class SiglipVisionModel(nn.Module):
         qkv = torch.empty(M, 3 * Dv, device=dev, dtype=torch.bfloat16)
         att = torch.empty(M, Dv, device=dev, dtype=torch.bfloat16)
         mid = torch.empty(M, Fv, device=dev, dtype=torch.bfloat16)
-        _lib.check(L.pg_siglip_layers(C.addressof(pk["array"]), len(pk["layers"]), x.data_ptr(), h.data_ptr(), qkv.data_ptr(), att.data_ptr(), mid.data_ptr(), B, N,
+        _lib.check(L.pg_siglip_layers(_lib.layer_array(_lib.SiglipLayer, pk), len(pk["layers"]), x.data_ptr(), h.data_ptr(), qkv.data_ptr(), att.data_ptr(), mid.data_ptr(), B, N,
                                       Dv, Fv, Hh, float(c.layer_norm_eps), st), "pg_siglip_layers")
         if out_bf16:
             _lib.layernorm(x, pk["post_w"], pk["post_b"], c.layer_norm_eps, out_bf16=h)

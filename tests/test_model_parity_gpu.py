@@ -298,3 +298,23 @@ def test_decode_l2_prefetch_branch_changes_nothing(late, monkeypatch):
             outs.append((toks.clone(), toks2.clone(), logits.clone()))
     for o in outs[1:]:
         assert torch.equal(outs[0][0], o[0]) and torch.equal(outs[0][1], o[1]) and torch.equal(outs[0][2], o[2])
+
+
+def test_a_model_that_has_run_can_be_copied_and_saved(tmp_path):
+    """A packed model survives a deep copy and a pickle, and neither reads the first one's weights."""
+    import copy
+    sd = make_state_dict(TINY_CONFIG, "R1", seed=11)
+    inp = {k: v.cuda() for k, v in make_inputs(TINY_CONFIG, batch=2, prompt_len=6, seed=7).items()}
+    model = build_model(TINY_CONFIG, sd)
+
+    def logits(m):
+        return m(input_ids=inp["input_ids"], pixel_values=inp["pixel_values"], attention_mask=inp["attention_mask"], kv_cache=None)["logits"]
+
+    want = logits(model)
+    torch.save(model, tmp_path / "model.pt")
+    copies = [copy.deepcopy(model), torch.load(tmp_path / "model.pt", weights_only=False)]
+    for part in (model.vision_tower, model.language_model):
+        for layer in part._packed["layers"]:
+            for t in layer.values():
+                t.fill_(float("nan"))
+    assert all(torch.equal(logits(m), want) for m in copies)
