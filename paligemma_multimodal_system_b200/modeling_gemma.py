@@ -287,8 +287,9 @@ class GemmaForCausalLM(nn.Module):
         have_cache = kv_cache is not None
         page_table = None
         if have_cache and page_rows is not None:
-            if kv_cache._geom is None or page_rows.shape[1] * PAGE < S or page_rows.shape[0] != B:
-                raise ValueError("prefill through page_rows needs an allocated KVCache and rows that hold the padded prompt")
+            # (the layers' pages are reached from the first layer's: a cache of fewer layers must not come that far)
+            if kv_cache._geom is None or page_rows.shape[1] * PAGE < S or page_rows.shape[0] != B or kv_cache.k_pages.shape[0] < len(pk["layers"]):
+                raise ValueError("prefill through page_rows needs an allocated KVCache of the model's layers and rows that hold the padded prompt")
             page_table = page_rows.to(torch.int32).contiguous()
             slot_base = torch.zeros(B, device=dev, dtype=torch.int32)
         elif have_cache:
