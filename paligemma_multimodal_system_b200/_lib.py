@@ -327,8 +327,9 @@ def gemm_residual(x, w, h, bias=None, scale=1.0):
     """h += (x @ w.T + bias) * scale: the residual-stream GEMMs (out_proj / fc2 / o_proj / down_proj).  With enough output tiles
     the epilogue adds the fp32 residual in place; with few tiles (small token counts: latency path, decode) the K
     dimension is split over CTAs and the partials are red.add-ed into h so that the whole GPU streams the weights."""
-    assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.is_cuda and w.is_cuda and x.stride(1) == 1 and w.stride(1) == 1
-    assert h.dtype == torch.float32 and h.stride(-1) == 1 and x.shape[1] == w.shape[1] and h.shape == (x.shape[0], w.shape[0])
+    assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.is_cuda and w.is_cuda
+    assert x.dim() == 2 and w.dim() == 2 and x.stride(1) == 1 and w.stride(1) == 1 and x.shape[1] == w.shape[1]
+    assert h.dtype == torch.float32 and h.stride(-1) == 1 and h.shape[0] >= x.shape[0] and h.shape[-1] >= w.shape[0]  # (h may hold more rows and columns)
     assert bias is None or (bias.dtype == torch.float32 and bias.is_contiguous())
     check(lib().pg_gemm_residual(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), h.data_ptr(), h.stride(0), ptr(bias), x.shape[0], w.shape[0], x.shape[1],
                                  float(scale), stream()), "pg_gemm_residual")

@@ -107,3 +107,17 @@ def test_clustered_ctas_have_an_sm_to_themselves(T, F, K, tmp_path):
     launches = [e["args"] for e in json.load(open(tmp_path / "trace.json"))["traceEvents"] if "gemm_cluster_kernel<true" in e.get("name", "")]
     assert launches and all(2 * (a["shared memory"] + 1024) > 228 * 1024 for a in launches)
     _check(out, acc, bound + 2.0 ** -22 * acc.abs())
+
+
+@pytest.mark.parametrize("T", [5, 100, 263, 700])
+def test_residual_buffers_may_be_larger(T):
+    """gemm_residual adds to the first rows and columns of the stream it is given."""
+    x, w, b, acc, bound = _operands(T, 256, 640, T)
+    h = torch.randn(T + 3, 260, device="cuda")
+    was = h.clone()
+    _lib.gemm_residual(x, w, h, bias=b, scale=0.5)
+    want = was[:T, :256].double() + (acc + b.double()) * 0.5
+    _check(h[:T, :256], want, bound + 2.0 ** -21 * (want.abs() + was[:T, :256].double().abs() + b.double().abs()))
+    assert torch.equal(h[T:], was[T:]) and torch.equal(h[:, 256:], was[:, 256:])
+    with pytest.raises(AssertionError):
+        _lib.gemm_residual(x, w, h[:T - 1], bias=b)
