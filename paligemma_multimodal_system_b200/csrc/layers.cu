@@ -37,8 +37,12 @@ extern "C" int pg_linear_f32(const void* x, long long ldx, const void* w, long l
   if (split > kb / 4) split = kb / 4;
   if (!swap || split <= 1 || pg_gemm_sums_once(tokens, features, K, out, ldo))
     return pg_gemm_bf16(x, ldx, w, ldw, out, ldo, nullptr, nullptr, 0, tokens, features, K, PG_EPI_F32, 0, 1.f, swap, 1, stream);
-  // few tiles of a long K: split-K partials are red.add-ed into the zeroed output
-  if (cudaMemset2DAsync(out, ldo * sizeof(float), 0, features * sizeof(float), tokens, reinterpret_cast<cudaStream_t>(stream)) != cudaSuccess) return PG_ERR_CUDA;
+  // few tiles of a long K: split-K partials are red.add-ed into the zeroed output (one row has no pitch: any ldo goes with it)
+  const size_t row = features * sizeof(float);
+  if (cudaMemset2DAsync(out, tokens == 1 ? row : ldo * sizeof(float), 0, row, tokens, reinterpret_cast<cudaStream_t>(stream)) != cudaSuccess) {
+    cudaGetLastError();  // do not leave a sticky error behind
+    return PG_ERR_CUDA;
+  }
   return pg_gemm_bf16(x, ldx, w, ldw, out, ldo, nullptr, nullptr, 0, tokens, features, K, PG_EPI_ATOMIC_F32, 0, 1.f, swap, split, stream);
 }
 

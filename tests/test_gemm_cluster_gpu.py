@@ -7,7 +7,7 @@ import json
 import pytest
 import torch
 
-from paligemma_multimodal_system_b200 import _lib
+from paligemma_multimodal_system_b200 import _lib, seq_ops
 
 pytestmark = pytest.mark.gpu
 
@@ -121,3 +121,14 @@ def test_residual_buffers_may_be_larger(T):
     assert torch.equal(h[T:], was[T:]) and torch.equal(h[:, 256:], was[:, 256:])
     with pytest.raises(AssertionError):
         _lib.gemm_residual(x, w, h[:T - 1], bias=b)
+
+
+@pytest.mark.parametrize("F,K", [(64, 4104), (256, 8192), (512, 1024)])
+def test_one_row_of_any_pitch(F, K):
+    """The one row of a one-token product may come with any row pitch (a view of a column, an expanded row), also where its sums are split."""
+    x, w, b, acc, bound = _operands(1, F, K, F)
+    for pitch in (0, 8, F, 2 * F):
+        out = torch.full((2 * F,), float("nan"), device="cuda")
+        seq_ops.linear(x, w, out.as_strided((1, F), (pitch, 1)))
+        _check(out[:F].view(1, F), acc, bound + 2.0 ** -22 * acc.abs())
+        assert out[F:].isnan().all()
