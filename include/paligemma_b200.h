@@ -59,7 +59,7 @@ int pg_debug_set_attn_trace(long long* device_buffer); /* same for pg_attention_
  * Replaces every nn.Linear on the path: modeling_siglip.py:59-62,71-75,156,177-185; modeling_paligemma.py:57,64;
  * modeling_gemma.py:205-218,255-259,274-278,356,484,523; and nn.Conv2d (modeling_siglip.py:258-263) after pg_im2col.
  *   swap:   0 = tokens on the UMMA M axis (prefill), 1 = features on the M axis (decode, tokens <= 128), -1 = auto
- *   split_k: >1 only with PG_EPI_ATOMIC_F32 (a hint: token-major calls of up to 1408 tokens choose their own split and add each sum once)
+ *   split_k: >1 only with PG_EPI_ATOMIC_F32
  */
 int pg_gemm_bf16(const void* x, long long ldx, const void* w, long long ldw, void* out, long long ldo,
                  const float* bias, const float* resid, long long ldr, int tokens, int features, int K, int mode,
@@ -101,7 +101,8 @@ int pg_gemm_bf16_fused(const void* x, long long ldx, const void* w, long long ld
                        const float* bias, const float* resid, long long ldr, int tokens, int features, int K, int mode,
                        int act_gelu, float scale, int swap, int split_k, const PgGemmFusion* fusion, void* stream);
 
-/* h[t,f] += (sum_k x[t,k] w[f,k] + bias[f]) * scale (h fp32): a projection that ends in the residual stream.  Few output tiles: K is split over CTAs. */
+/* h[t,f] += (sum_k x[t,k] w[f,k] + bias[f]) * scale (h fp32): a projection that ends in the residual stream.  Few output tiles: K is split over CTAs.  h belongs to
+ * this call until it is done (for sums that several streams add into: PG_EPI_ATOMIC_F32). */
 int pg_gemm_residual(const void* x, long long ldx, const void* w, long long ldw, float* h, long long ldh, const float* bias, int tokens, int features,
                      int K, float scale, void* stream);
 

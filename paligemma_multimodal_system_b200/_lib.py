@@ -324,9 +324,9 @@ def rmsnorm(x, w, out_bf16, eps=1e-6):
 
 
 def gemm_residual(x, w, h, bias=None, scale=1.0):
-    """h += (x @ w.T + bias) * scale: the residual-stream GEMMs (out_proj / fc2 / o_proj / down_proj).  With enough output tiles
-    the epilogue adds the fp32 residual in place; with few tiles (small token counts: latency path, decode) the K
-    dimension is split over CTAs and the partials are red.add-ed into h so that the whole GPU streams the weights."""
+    """h += (x @ w.T + bias) * scale: the residual-stream GEMMs (out_proj / fc2 / o_proj / down_proj).  Prompts: every sum is added up by one tile (or one cluster,
+    which shares out K) and the epilogue adds the fp32 residual in place.  Up to 128 tokens with few output tiles: the K dimension is split over CTAs and the
+    partials are red.add-ed into h so that the whole GPU streams the weights.  h belongs to this call until it is done."""
     assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.is_cuda and w.is_cuda
     assert x.dim() == 2 and w.dim() == 2 and x.stride(1) == 1 and w.stride(1) == 1 and x.shape[1] == w.shape[1]
     assert h.dtype == torch.float32 and h.stride(-1) == 1 and h.shape[0] >= x.shape[0] and h.shape[-1] >= w.shape[0]  # (h may hold more rows and columns)

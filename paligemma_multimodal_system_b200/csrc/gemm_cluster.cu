@@ -227,10 +227,8 @@ __global__ void __launch_bounds__(kThreads, GROUPED ? 2 : 1) gemm_cluster_kernel
               h[j] = make_float4(0.f, 0.f, 0.f, 0.f);
               if (args.mode != PG_EPI_BF16) {
                 o[j] = static_cast<float*>(args.out) + (args.out_row_map != nullptr ? static_cast<long long>(__ldg(args.out_row_map + tok)) : tok) * args.ldo + f;
-                const float* res = args.mode == PG_EPI_ATOMIC_F32 ? o[j]
-                                   : args.resid != nullptr        ? args.resid + (args.resid_mod > 0 ? tok % args.resid_mod : tok) * args.ldr + f
-                                                                  : nullptr;
-                if (res != nullptr) h[j] = *reinterpret_cast<const float4*>(res);
+                if (args.resid != nullptr)
+                  h[j] = *reinterpret_cast<const float4*>(args.resid + (args.resid_mod > 0 ? tok % args.resid_mod : tok) * args.ldr + f);
               }
             }
 #pragma unroll

@@ -1169,15 +1169,18 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& 
 // 5120 x 2048 1024 27.9 / 22.0, 1536 29.0 / 30.3; 8192 x 2048 706 28.6 / 23.4, 1024 29.3 / 31.5.
 //
 // Decode-sized calls (up to 128 tokens): where its grid is one wave, but for long K with up to 64 tokens, which the two-CTAs-per-SM stream of this file's
-// swap kernels reads faster.  Not for split-K accumulation into a residual stream: in a chain of decode launches under the L2 prefetch stream of
-// modeling_gemma.py the clusters wait for whole GPCs (one request of 24 tokens 28.5 -> 29.5 ms, 64 requests 132 -> 138).  5 tokens: 8192 x 2048 13.4 / 9.3, 2048 x 2048 7.1 / 5.6 (without the zeroed accumulator), 16384 x 2048 gate || up
+// swap kernels reads faster.  5 tokens: 8192 x 2048 13.4 / 9.3, 2048 x 2048 7.1 / 5.6 (without the zeroed accumulator), 16384 x 2048 gate || up
 // 15.1 / 13.1, 2048 x 8192 10.7 / 10.9, 2048 x 16384 15.0 / 16.6, two waves: 32000 x 2048 22 / 36; 128 tokens: 2048 x 8192 18.0 / 14.0.
+//
+// Never for PG_EPI_ATOMIC_F32: calls that share an output, on several streams or as several splits, need the red.add of this file's kernels.  (pg_gemm_residual
+// chooses: an owned residual stream of a prompt takes PG_EPI_F32; that of a decode step stays with the split, because under the L2 prefetch stream of
+// modeling_gemma.py clusters wait for whole GPCs: one request of 24 tokens 28.5 -> 29.5 ms, 64 requests 132 -> 138.)
 static bool cluster_form(const GemmArgs& a, long long ldr, int swap) {
   auto aligned = [](const void* p, int n) { return (reinterpret_cast<uintptr_t>(p) & (n - 1)) == 0; };
   // vectors of four: outputs, bias and residual rows
   if (a.features % 4 != 0 || a.ldo % 4 != 0 || !aligned(a.out, 16) || !aligned(a.bias, 16)) return false;
-  if (a.resid != nullptr && (ldr % 4 != 0 || !aligned(a.resid, 16))) return false;
-  if (swap) return a.mode != PG_EPI_ATOMIC_F32 && a.stats == nullptr && a.zero_buf == nullptr && (a.K <= 4096 || a.tokens > 64) && plan_cluster_gemm(a.tokens, a.features, a.K).waves == 1;
+  if (a.mode == PG_EPI_ATOMIC_F32 || (a.resid != nullptr && (ldr % 4 != 0 || !aligned(a.resid, 16)))) return false;
+  if (swap) return a.stats == nullptr && a.zero_buf == nullptr && (a.K <= 4096 || a.tokens > 64) && plan_cluster_gemm(a.tokens, a.features, a.K).waves == 1;
   if (a.K <= 128 && a.tokens <= 4096) return true;  // (all epilogue: 2048 x 64 3750 tokens 14.6 / 9.3, 8192 25.9 / 28.0; K 256 15.9 / 16.9)
   if (a.tokens > 1408) return false;
   const int pairs = num_sms() / 2, pair_tiles = ((a.tokens + 2 * BM - 1) / (2 * BM)) * ((a.features + 255) / 256);
@@ -1191,11 +1194,11 @@ static bool cluster_form(const GemmArgs& a, long long ldr, int swap) {
 
 using namespace pg;
 
-// Whether a decode-sized fp32 product adds up K by itself (gemm_cluster.cu), without split-K partials.
-bool pg_gemm_sums_once(int tokens, int features, int K, const void* out, long long ldo) {
+// Whether a product with fp32 rows adds up K by itself (gemm_cluster.cu), without split-K partials.
+bool pg_gemm_sums_once(int tokens, int features, int K, const void* out, long long ldo, const float* bias, int swap) {
   GemmArgs a = {};
-  a.tokens = tokens; a.features = features; a.K = K; a.mode = PG_EPI_F32; a.out = const_cast<void*>(out); a.ldo = ldo;
-  return cluster_form(a, 0, 1);
+  a.tokens = tokens; a.features = features; a.K = K; a.mode = PG_EPI_F32; a.out = const_cast<void*>(out); a.ldo = ldo; a.bias = bias;
+  return cluster_form(a, 0, swap);
 }
 
 extern "C" int pg_gemm_bf16(const void* x, long long ldx, const void* w, long long ldw, void* out, long long ldo,

@@ -6,12 +6,15 @@
 #include "common.cuh"
 #include "paligemma_b200.h"
 
-bool pg_gemm_sums_once(int tokens, int features, int K, const void* out, long long ldo);  // gemm_tcgen05.cu
+bool pg_gemm_sums_once(int tokens, int features, int K, const void* out, long long ldo, const float* bias, int swap);  // gemm_tcgen05.cu
 
 extern "C" int pg_gemm_residual(const void* x, long long ldx, const void* w, long long ldw, float* h, long long ldh, const float* bias, int tokens,
                                 int features, int K, float scale, void* stream) {
   if (tokens <= 0 || features <= 0 || K <= 0) return PG_ERR_ARG;
-  const int swap = tokens <= 128 ? 1 : 0, kb = (K + 63) / 64;
+  const int swap = tokens <= 128 ? 1 : 0, kb = (K + 63) / 64, sms = pg::num_sms();
+  if (!swap && pg_gemm_sums_once(tokens, features, K, h, ldh, bias, 0))
+    return pg_gemm_bf16(x, ldx, w, ldw, h, ldh, bias, h, ldh, tokens, features, K, PG_EPI_F32, 0, scale, 0, 1, stream);
+  // what is left: decode steps, many tokens, and rows off a 16-byte boundary
   int tiles;
   if (swap) {
     tiles = (features + 127) / 128;
@@ -24,7 +27,7 @@ extern "C" int pg_gemm_residual(const void* x, long long ldx, const void* w, lon
   }
   if (tiles >= 96 || kb < 8 || tokens > 512)
     return pg_gemm_bf16(x, ldx, w, ldw, h, ldh, bias, h, ldh, tokens, features, K, PG_EPI_F32, 0, scale, swap, 1, stream);
-  int split = (swap ? 2 * 148 : 148) / tiles;
+  int split = (swap ? 2 * sms : sms) / tiles;
   if (split > kb / 4) split = kb / 4;
   return pg_gemm_bf16(x, ldx, w, ldw, h, ldh, bias, nullptr, 0, tokens, features, K, PG_EPI_ATOMIC_F32, 0, scale, swap, split < 1 ? 1 : split, stream);
 }
@@ -35,7 +38,7 @@ extern "C" int pg_linear_f32(const void* x, long long ldx, const void* w, long l
   const int tiles = (features + 127) / 128, kb = (K + 63) / 64, swap = tokens <= 128 ? 1 : 0;
   int split = 2 * pg::num_sms() / tiles;
   if (split > kb / 4) split = kb / 4;
-  if (!swap || split <= 1 || pg_gemm_sums_once(tokens, features, K, out, ldo))
+  if (!swap || split <= 1 || pg_gemm_sums_once(tokens, features, K, out, ldo, nullptr, swap))
     return pg_gemm_bf16(x, ldx, w, ldw, out, ldo, nullptr, nullptr, 0, tokens, features, K, PG_EPI_F32, 0, 1.f, swap, 1, stream);
   // few tiles of a long K: split-K partials are red.add-ed into the zeroed output (one row has no pitch: any ldo goes with it)
   const size_t row = features * sizeof(float);

@@ -132,3 +132,17 @@ def test_one_row_of_any_pitch(F, K):
         seq_ops.linear(x, w, out.as_strided((1, F), (pitch, 1)))
         _check(out[:F].view(1, F), acc, bound + 2.0 ** -22 * acc.abs())
         assert out[F:].isnan().all()
+
+
+@pytest.mark.parametrize("T,F,K,split", [(200, 256, 512, 1), (300, 512, 1024, 4), (1400, 260, 640, 3)])
+def test_atomic_accumulation_from_several_streams(T, F, K, split):
+    """PG_EPI_ATOMIC_F32 outputs may be shared: sums of small whole numbers are exact in any order, so none may be lost."""
+    xs, ws = (torch.randint(-2, 3, (8, n, K), device="cuda").bfloat16() for n in (T, F))
+    out = torch.zeros(T, F, device="cuda")
+    streams = [torch.cuda.Stream() for _ in range(4)]
+    torch.cuda.synchronize()
+    for i in range(8):
+        with torch.cuda.stream(streams[i % 4]):
+            _lib.gemm(xs[i], ws[i], out, mode=_lib.EPI_ATOMIC_F32, swap=0, split_k=split)
+    torch.cuda.synchronize()
+    assert torch.equal(out.double(), torch.einsum("itk,ifk->tf", xs.double(), ws.double()))
