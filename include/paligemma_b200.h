@@ -40,7 +40,8 @@ long long pg_launch_count(void);
 /* Programmatic dependent launch for the decode-step kernels (default on): the next kernel's prologue and weight
  * prefetch overlap the running kernel; every such kernel executes griddepcontrol.wait before dependent accesses. */
 int pg_set_pdl(int on);
-/* Profiling aid: when non-NULL, CTA 0 of launch i writes 6 clock64 stamps to buffer[8*(i%64) ..] (device). */
+/* The GEMM switches below (trace, pair, bn) speak of the persistent kernels: while one is set, no product (pair, bn: no token-major product) takes the clustered form.
+ * Profiling aid: when non-NULL, CTA 0 of launch i writes 6 clock64 stamps to buffer[8*(i%64) ..] (device). */
 int pg_debug_set_gemm_trace(long long* device_buffer);
 int pg_debug_set_rmsnorm_early_trigger(int on); /* A/B runs: the decode RMSNorm triggers its dependents before / after its own dependency wait */
 int pg_debug_set_gemm_pair(int mode, int min_tiles); /* A/B runs: mode bit 0 = CTA-pair (cta_group::2) prefill GEMM allowed, bit 1 = banded tile raster OFF, bits 2-3 = epilogue warps of the pair kernel (1 = eight, 2 = four, 0 = automatic) (default mode 1); min_tiles > 0 sets the pair kernel's tile-count threshold */

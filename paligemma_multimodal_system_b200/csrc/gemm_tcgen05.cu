@@ -1128,7 +1128,8 @@ extern "C" int pg_debug_set_gemm_trace(long long* p) { g_gemm_trace = p; g_gemm_
 static int g_epi8_mode = 0;  // tuning: 1 = eight epilogue warps for every pair GEMM, 2 = four, 0 = by K
 static int g_band_mode = 1;        // 0: never use the banded raster (A/B runs)
 static int g_pair_mode = 1;        // 0: never use the CTA-pair kernel (A/B runs)
-static int g_pair_min_tiles = 74;  // at least one 256 x 256 tile per pair of SMs
+constexpr int kPairMinTiles = 74;  // at least one 256 x 256 tile per pair of SMs
+static int g_pair_min_tiles = kPairMinTiles;
 extern "C" int pg_debug_set_gemm_pair(int mode, int min_tiles) {
   g_pair_mode = mode & 1;
   g_epi8_mode = (mode >> 2) & 3;
@@ -1177,6 +1178,9 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& 
 // modeling_gemma.py clusters wait for whole GPCs: one request of 24 tokens 28.5 -> 29.5 ms, 64 requests 132 -> 138.)
 static bool cluster_form(const GemmArgs& a, long long ldr, int swap) {
   auto aligned = [](const void* p, int n) { return (reinterpret_cast<uintptr_t>(p) & (n - 1)) == 0; };
+  // a tuning or profiling switch that is set speaks of this file's kernels
+  if (g_gemm_trace != nullptr) return false;
+  if (!swap && (g_force_bn != 0 || g_pair_mode != 1 || g_epi8_mode != 0 || g_band_mode != 1 || g_pair_min_tiles != kPairMinTiles)) return false;
   // vectors of four: outputs, bias and residual rows
   if (a.features % 4 != 0 || a.ldo % 4 != 0 || !aligned(a.out, 16) || !aligned(a.bias, 16)) return false;
   if (a.mode == PG_EPI_ATOMIC_F32 || (a.resid != nullptr && (ldr % 4 != 0 || !aligned(a.resid, 16)))) return false;

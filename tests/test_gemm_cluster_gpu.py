@@ -146,3 +146,44 @@ def test_atomic_accumulation_from_several_streams(T, F, K, split):
             _lib.gemm(xs[i], ws[i], out, mode=_lib.EPI_ATOMIC_F32, swap=0, split_k=split)
     torch.cuda.synchronize()
     assert torch.equal(out.double(), torch.einsum("itk,ifk->tf", xs.double(), ws.double()))
+
+
+def _kernels(call):
+    call()
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    return " ".join(e.key for e in prof.key_averages())
+
+
+def test_tuning_switches_reach_the_persistent_kernels():
+    L = _lib.lib()
+    x, w, b, acc, bound = _operands(300, 512, 640, 2)
+    out = torch.empty(300, 512, device="cuda", dtype=torch.bfloat16)
+    few = torch.empty(5, 512, device="cuda", dtype=torch.bfloat16)
+    prompt = lambda: _lib.gemm(x, w, out, mode=_lib.EPI_BF16, swap=0)
+    assert "gemm_cluster_kernel" in _kernels(prompt)
+    try:
+        for bn in (64, 128, 256):
+            assert L.pg_debug_set_gemm_bn(bn) == 0 and f"gemm_tcgen05_kernel<{bn}" in _kernels(prompt)
+            _check(out, acc, bound + 2.0 ** -8 * acc.abs())
+        L.pg_debug_set_gemm_bn(0)
+        L.pg_debug_set_gemm_pair(0, 0)  # one CTA per tile only
+        assert "gemm_tcgen05_kernel" in _kernels(prompt)
+        L.pg_debug_set_gemm_pair(1, 1)  # pairs from one tile on
+        assert L.pg_debug_set_gemm_bn(256) == 0 and "gemm_pair_kernel" in _kernels(prompt)
+        _check(out, acc, bound + 2.0 ** -8 * acc.abs())
+        L.pg_debug_set_gemm_bn(0)
+        L.pg_debug_set_gemm_pair(1, 74)
+        stamps = torch.zeros(64 * 8, device="cuda", dtype=torch.int64)
+        L.pg_debug_set_gemm_trace(stamps.data_ptr())
+        prompt()
+        _lib.gemm(x[:5], w, few, mode=_lib.EPI_BF16, swap=1)
+        torch.cuda.synchronize()
+        assert (stamps.view(64, 8)[:2, 0] > 0).all()
+    finally:
+        L.pg_debug_set_gemm_bn(0)
+        L.pg_debug_set_gemm_pair(1, 74)
+        L.pg_debug_set_gemm_trace(0)
+    assert "gemm_cluster_kernel" in _kernels(prompt)
