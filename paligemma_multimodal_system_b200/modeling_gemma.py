@@ -20,6 +20,7 @@ from . import _lib
 from .modeling_siglip import _ParamsOnly, _bf16, _f32
 
 PAGE = 64  # tokens per KV page (= the decode attention key tile)
+NORM_EPS = 1e-6  # of every RMSNorm: the reference's layers never pass config.rms_norm_eps on (modeling_gemma.py:158,379,381,448)
 MAX_DECODE_BATCH = 128  # rows of one decode step (the batch sits on the UMMA N axis of the weight-streaming GEMMs)
 
 
@@ -156,7 +157,7 @@ class GemmaConfig:
 
 
 class GemmaRMSNorm(_ParamsOnly):
-    def __init__(self, dim: int, eps: float = 1e-6, **fk):
+    def __init__(self, dim: int, eps: float = NORM_EPS, **fk):
         super().__init__()
         self.dim, self.eps = dim, eps
         self.weight = nn.Parameter(torch.zeros(dim, **fk))
@@ -319,7 +320,7 @@ class GemmaForCausalLM(nn.Module):
         args = _lib.GemmaPrefill(h.data_ptr(), hn.data_ptr(), qkv.data_ptr(), _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), att.data_ptr(), mid.data_ptr(), pos.data_ptr(),
                                  pk["inv_freq"].data_ptr(), _lib.ptr(kp), _lib.ptr(kv_cache.v_pages) if have_cache else 0,
                                  kp.stride(0) * kp.element_size() if have_cache else 0, _lib.ptr(page_table), slot_base.data_ptr() if have_cache else 0,
-                                 _lib.ptr(lens), B, S, D, F, Hq, Hkv, dh, PAGE, page_table.shape[1] if have_cache else 0, int(fused), 1e-6)
+                                 _lib.ptr(lens), B, S, D, F, Hq, Hkv, dh, PAGE, page_table.shape[1] if have_cache else 0, int(fused), NORM_EPS)
         _lib.check(L.pg_gemma_prefill_layers(_lib.layer_array(_lib.GemmaLayer, pk), len(pk["layers"]), C.addressof(args), st), "pg_gemma_prefill_layers")
         if have_cache and page_rows is None:
             kv_cache._set_len(S, c.num_hidden_layers)
@@ -329,11 +330,11 @@ class GemmaForCausalLM(nn.Module):
             else:
                 last = h.view(B, S, D)[torch.arange(B, device=dev), lens.long() - 1].contiguous()
             ln = torch.empty(B, D, device=dev, dtype=torch.bfloat16)
-            _lib.rmsnorm(last, pk["norm_w"], ln)
+            _lib.rmsnorm(last, pk["norm_w"], ln, eps=NORM_EPS)
             logits = torch.empty(B, V, device=dev, dtype=torch.float32)
             _lib.gemm(ln, pk["head_w"], logits, mode=_lib.EPI_F32, bias=pk["head_b"], swap=1 if B <= 128 else 0)
             return logits.view(B, 1, V)
-        _lib.rmsnorm(h, pk["norm_w"], hn)
+        _lib.rmsnorm(h, pk["norm_w"], hn, eps=NORM_EPS)
         logits = torch.empty(T, V, device=dev, dtype=torch.float32)
         _lib.gemm(hn, pk["head_w"], logits, mode=_lib.EPI_F32, bias=pk["head_b"], swap=0 if T > 128 else 1)
         return logits.view(B, S, V)
@@ -397,7 +398,6 @@ class GemmaForCausalLM(nn.Module):
         pos, kvl = kv_cache.counters[0], kv_cache.counters[2]
         max_pages = kv_cache.page_table.shape[1]
         scale = 1.0 / math.sqrt(dh)
-        eps = c.rms_norm_eps if c.rms_norm_eps is not None else 1e-6
         W = (Hq + 2 * Hkv) * dh
         sms = _lib.num_sms()
         sp_qkv = _pick_split((W + 127) // 128, D // 64, sms)
@@ -425,7 +425,7 @@ class GemmaForCausalLM(nn.Module):
             _lib.check(L.pg_prefetch_l2(lw["gu_w"].data_ptr(), pf_bytes, pf_ctas, 0, side.cuda_stream), "pg_prefetch_l2")
 
         for li, lw in enumerate(pk["layers"]):
-            _lib.rmsnorm(h, lw["ln1"], hn, eps=eps)
+            _lib.rmsnorm(h, lw["ln1"], hn, eps=NORM_EPS)
             _lib.gemm(hn, lw["qkv_w"], qkv, mode=_lib.EPI_ATOMIC_F32, swap=1, split_k=sp_qkv)
             if side is not None and not pf_late:
                 prefetch(lw)
@@ -436,12 +436,12 @@ class GemmaForCausalLM(nn.Module):
             if side is not None and pf_late:
                 prefetch(lw)
             _lib.gemm_fused(att, lw["o_w"], h, mode=_lib.EPI_ATOMIC_F32, split_k=sp_o, zero_buf=qkv)
-            _lib.rmsnorm(h, lw["ln2"], hn, eps=eps)
+            _lib.rmsnorm(h, lw["ln2"], hn, eps=NORM_EPS)
             _lib.gemm(hn, lw["gu_w"], mid, mode=_lib.EPI_GEGLU, swap=1)
             _lib.gemm(mid, lw["down_w"], h, mode=_lib.EPI_ATOMIC_F32, swap=1, split_k=sp_down)
         if side is not None:
             cur.wait_stream(side)  # join (the last prefetch finished a layer ago)
-        _lib.rmsnorm(h, pk["norm_w"], hn, eps=eps)
+        _lib.rmsnorm(h, pk["norm_w"], hn, eps=NORM_EPS)
         _lib.gemm_fused(hn, pk["head_w"], bufs["logits"], mode=_lib.EPI_F32, bias=pk["head_b"], stats=bufs["stats"],
                         inv_temperature=inv_temperature)
         return bufs["logits"]
