@@ -23,7 +23,7 @@
 // S_{j+1} is computed while the softmax of tile j runs, and P_j V_j runs while the softmax of tile j+1 runs.
 // Zero padding comes from TMA: columns beyond dh (72 -> 80) and key / query rows beyond the sequence are out-of-bounds
 // box elements and arrive as zeros; padded keys are masked to -inf before the softmax.
-// Timelines of one CTA (clock64 stamps, Params::trace): profiles/tools/attn_prefill_trace.py, profiles/r02h_attn_prefill_trace_*.txt.
+// Timelines of one CTA: clock64 stamps through Params::trace.
 #include "common.cuh"
 #include "paligemma_b200.h"
 #include "tmap.cuh"
@@ -44,7 +44,7 @@ struct Params {
   float sl2;  // softmax scale * log2(e)
   const int* key_lens;  // optional [B]: problem b only attends to its first key_lens[b] keys (ragged prompts); else nullptr
   int stagger;          // QT = 2 (tuning): clock cycles the softmax group of query tile 1 idles after its first S tile is ready
-  long long* trace;     // optional clock64 stamps of CTA (0,0,0): [role][tile][event], see profiles/tools/attn_prefill_trace.py
+  long long* trace;     // optional clock64 stamps of CTA (0,0,0): [role][tile][event]
 };
 
 template <int DH, int QT>
@@ -257,9 +257,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   } else if (warp == 1) {
     // ============================== MMA issuer ================================
     // All 32 lanes run the loop and ONE elected lane issues: with uniform control flow the compiler keeps the descriptors
-    // and TMEM addresses in uniform registers.  (Under `if (lane == 0)` every tcgen05.mma paid an ELECT + R2UR.BROADCAST
-    // chain per operand, ~115 clk per instruction: the issuer, not the softmax or the tensor pipe, paced the kernel --
-    // profiles/r02h_attn_prefill_trace_before.txt.)
+    // and TMEM addresses uniform over the warp.  (Under `if (lane == 0)` every tcgen05.mma took ~115 clk to issue: the issuer, not the
+    // softmax or the tensor pipe, paced the kernel.)
     auto issue_s = [&](int j) {  // S_j = Q K_j^T of every query tile into its S buffer j % 2
       const int ks = j % KST, sb = j & 1;
       mbar_wait(k_full(ks), (j / KST) & 1);
@@ -414,7 +413,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       // Three separate passes over the thread's HB scores (exponent arguments, then the MUFU exponentials back to back, then
       // pack + store): interleaved chunk by chunk, each exp2 -> pack -> store chain exposed the ~40 clk MUFU latency with two
       // or three exponentials in flight (900 clk per 64 scores for a warp ALONE on its sub-partition's MUFU pipe, which
-      // could do them in 512 -- profiles/r02h_attn_prefill_trace_qt2.txt).
+      // could do them in 512).
 #pragma unroll
       for (int i = 0; i < HB; ++i) s[i] = fmaf(s[i], p.sl2, -m_new);
       // (an earlier variant with floorf / float->int range reduction was 40 % SLOWER: those conversions run on the XU pipe
@@ -582,7 +581,7 @@ int pg_attention_prefill_tc(const void* q, const void* k, const void* v, void* o
   }
   // query tiles per CTA (dh <= 128).  Two tiles share every K / V tile and give each SM sub-partition two INDEPENDENT softmax
   // warps (one per query tile) instead of two halves of one row in lock step: with the S and P V issuers split into two
-  // warps, 4096 keys run at 1.02 ms vs 1.21 ms for the one-tile variant (profiles/r02h_attn72_variants.txt).
+  // warps, 4096 keys run at 1.02 ms vs 1.21 ms for the one-tile variant.
   const int qt = dh > 128 ? 1 : (g_force_qt ? g_force_qt : (rows > 128 ? 2 : 1));
   const int BN = (dh > 128 || qt == 2) ? 64 : 128;
   {

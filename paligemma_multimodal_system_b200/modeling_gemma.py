@@ -409,7 +409,7 @@ class GemmaForCausalLM(nn.Module):
             sp_qkv = sp_o = sp_down = 1
         # L2 weight prefetch on a forked branch (pg_prefetch_l2): while the attention block of a layer (q/k/v, attention, o_proj,
         # norm: ~17 us of kernel-boundary latency with the HBM pins idle) runs, the bulk-copy engines of a few SMs pull the
-        # head of the layer's gate||up weights into L2.  Measured per layer (profiles/r02g_decode_l2_prefetch_sweep.txt):
+        # head of the layer's gate||up weights into L2.  Measured per layer:
         # 64 x 324 keys 61.6 -> 58.9 us, 1 x 324 51.9 -> 48.5, 32 x 1092 63.9 -> 61.2, 8 x 4164 63.6 -> 63.1.  The stream
         # must not queue ahead of the loads on the critical path: it is forked AFTER the q/k/v launch (64 MB, 32 SMs) when
         # the KV pages of a layer are small, and after the attention launch (48 MB, 64 SMs) when attention itself streams

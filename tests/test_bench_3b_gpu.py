@@ -9,7 +9,7 @@
 Tolerance (north_star: bf16 tolerance stated in the test): last-position logits cosine >= 0.9999 and max-abs <= 1 % of the
 oracle logit absmax in R1; cosine >= 0.999 and <= 3 % in the diffuse regime R2; greedy tokens identical to the oracle's
 whenever its top-2 margin exceeds 4x the measured error (all 32 steps in R1).  Every measured figure is also written to
-gpurun_out/parity_r02.json (copied to profiles/parity_r02.json, which bench.py attaches to its line as `parity`)."""
+build/parity_r02.json (copied to profiles/parity_r02.json, which bench.py attaches to its line as `parity`)."""
 import json
 import os
 
@@ -24,7 +24,7 @@ from oracle import paligemma_oracle as O  # noqa: E402
 from paligemma_multimodal_system_b200.random_init import make_inputs, make_state_dict, paligemma_3b_config  # noqa: E402
 
 
-OUT = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "gpurun_out", "parity_r02.json")
+OUT = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "build", "parity_r02.json")
 
 
 def _record(name, payload):
