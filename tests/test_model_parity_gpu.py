@@ -320,19 +320,20 @@ def test_a_model_that_has_run_can_be_copied_and_saved(tmp_path):
     assert all(torch.equal(logits(m), want) for m in copies)
 
 
-def test_prompt_and_decode_share_one_norm_epsilon():
-    """The reference's norms take 1e-6 whatever the config says: a decoded token sees the same norms as the prompt."""
+def test_no_pass_takes_the_norm_epsilon_of_the_config():
+    """The reference's norms take 1e-6 whatever the config says, in the prompt pass and in decode steps alike."""
     import copy
     from paligemma_multimodal_system_b200.modeling_gemma import KVCache
-    config = copy.deepcopy(TINY_CONFIG)
-    config["text_config"]["rms_norm_eps"] = 1.0
     sd = make_state_dict(TINY_CONFIG, "R1", seed=11)
-    lm = build_model(config, sd).language_model
-    S, D = 9, config["text_config"]["hidden_size"]
+    S, D = 9, TINY_CONFIG["text_config"]["hidden_size"]
     e = torch.randn(2, S + 1, D, generator=torch.Generator().manual_seed(3)) * 0.02
     pos = torch.arange(S + 1).expand(2, -1)
-    whole = lm(input_embeds=e, position_ids=pos)["logits"]
-    kv = KVCache()
-    lm(input_embeds=e[:, :S], position_ids=pos[:, :S], kv_cache=kv)
-    step = lm(input_embeds=e[:, S:], position_ids=pos[:, S:], kv_cache=kv)["logits"]
-    _check(step[:, -1], whole[:, -1], "R2", "decode after a prompt")  # (two bf16 paths against each other; another epsilon changes the logits several times over)
+    logits = []
+    for eps in (1e-6, 1.0):
+        config = copy.deepcopy(TINY_CONFIG)
+        config["text_config"]["rms_norm_eps"] = eps
+        lm, kv = build_model(config, sd).language_model, KVCache()
+        prompt = lm(input_embeds=e[:, :S], position_ids=pos[:, :S], kv_cache=kv)["logits"]
+        logits.append((prompt, lm(input_embeds=e[:, S:], position_ids=pos[:, S:], kv_cache=kv)["logits"]))
+    _check(logits[1][0], logits[0][0], "R1", "prompt")
+    _check(logits[1][1], logits[0][1], "R1", "decode step")
