@@ -70,3 +70,35 @@ def test_one_token_may_choose_an_expert_again(T, top, n):
             assert ((mid[row].double() - z).abs() <= 2.0 ** -8 * z.abs() + 2.0 ** -18 * (up[e].double().abs() @ x[t].double().abs())).all()
             got = down[e].double() @ mid[row].double()
             assert ((eo[row].double() - got).abs() <= 2.0 ** -20 * (down[e].double().abs() @ mid[row].double().abs()) + 1e-30).all()
+
+
+@pytest.mark.parametrize("T,top,n", [(3, 2, 2), (70, 3, 4)])
+def test_rows_next_to_a_tile_stay_out(T, top, n):
+    """Scratch rows that no expert owns hold anything, an infinity in one token's row and a NaN in one expert's weights stay with their rows."""
+    D, F = 72, 136
+    ids = torch.stack([torch.randperm(n + 1, device="cuda")[:top] for _ in range(T)]).to(torch.int32).contiguous()  # id n: no row
+    ids[0, 0], ids[0, 1:] = n, torch.arange(top - 1, device="cuda")
+    counts = torch.bincount(ids[ids < n].long(), minlength=n).to(torch.int32)
+    plan = seq_ops.MoePlan(ids, counts, n)
+    x = torch.randn(T, D, device="cuda").bfloat16()
+    up, down = (torch.randn(n, F, D, device="cuda") * D ** -0.5).bfloat16(), (torch.randn(n, D, F, device="cuda") * F ** -0.5).bfloat16()
+    x[1, 5], down[n - 1, D - 1, 3] = float("inf"), float("nan")
+    b = dict(device="cuda", dtype=torch.bfloat16)
+    xg, mid = torch.full((plan.pairs, D), float("nan"), **b), torch.full((plan.pairs, F), float("nan"), **b)
+    eo = torch.zeros(plan.pairs, D, device="cuda")
+    seq_ops.moe_products(x, plan, up, down, xg, mid, eo, seq_ops.ACT_RELU2)
+    owned = 0
+    for t in range(T):
+        for k in range(top):
+            e, row = int(ids[t, k]), int(plan.pair_row[t * top + k])
+            if e >= n:
+                continue
+            owned += 1
+            last = D - 1 if e == n - 1 else D
+            if t != 1:
+                assert eo[row, :last].isfinite().all() and mid[row].isfinite().all()
+                got = down[e, :last].double() @ mid[row].double()
+                assert ((eo[row, :last].double() - got).abs() <= 2.0 ** -20 * (down[e, :last].double().abs() @ mid[row].double().abs()) + 1e-30).all()
+            if e == n - 1:
+                assert eo[row, D - 1].isnan()
+    assert owned < plan.pairs and not eo[owned:].any()
