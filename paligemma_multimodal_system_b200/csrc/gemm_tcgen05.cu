@@ -1162,12 +1162,17 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& 
              ? PG_OK : PG_ERR_CUDA;
 }
 
-// Whether a token-major product takes the form of gemm_cluster.cu: up to 1408 tokens, where the CTA-pair kernel has no tile for every pair of SMs or
-// the estimate of its waves (740 clocks a 64-deep step, fitted to the times below) is the longer one.  Measured on both sides of the lines (us, this
-// file's kernels / gemm_cluster.cu; N x K weights): 3456 x 1152 263 tokens 14.4 / 8.2, 1024 17.0 / 10.8, 2048 20.2 / 22.2; 2048 x 2048 with residual
-// 263 15.2 / 10.1, 1300 28.5 / 18.2; 2048 x 16384 with residual 263 41 / 28, 1300 163 / 86, 2048 113 / 120; 3072 x 768 1300 10.4 / 9.1, 1536
-// 10.7 / 11.5; pair tiles: 32768 x 2048 gate || up 263 54 / 39, 400 56 / 64, 1024 101 / 133; 16384 x 2048 263 29 / 20, 400 29.7 / 29.7, 706 42 / 46;
-// 5120 x 2048 1024 27.9 / 22.0, 1536 29.0 / 30.3; 8192 x 2048 706 28.6 / 23.4, 1024 29.3 / 31.5.
+// Whether a product takes the form of gemm_cluster.cu.  Prompts: up to 1408 tokens, where its estimate (plan_cluster_gemm) is below that of this file's kernel for the
+// call.  The estimates were fitted to 1900 products timed in turn on both sides (256 .. 32768 features, K 16 .. 16384, 200 .. 4096 tokens); where
+// the clustered form is chosen no one of them is more than 3 % slower by it.  us, this file's kernels / gemm_cluster.cu, N x K weights:
+//   K <= 128: all epilogue, and the clustered one is spread over more CTAs.  2048 x 64, 3750 tokens, fp32 rows 14.4 / 9.9; above 1408 tokens not for few features (256,
+//     4096 tokens 6.5 / 9.7; 512, fp32 rows 9.0 / 9.6) nor for many waves of bf16 rows (8192, 4096 tokens 32.0 / 36.2).
+//   activations (bf16 rows): this file's one-CTA kernel (640 clocks a 64-deep step, 4500 a tile).  8192 x 2048, 640 tokens 36.4 / 23.0; 16384 x 2048, 1408 tokens 84.6 / 99.2.
+//   fewer than 74 pair tiles: 3456 x 1152, 263 tokens 14.4 / 8.2; 2048 x 16384 with residual, 1300 tokens 163 / 86; but plain bf16 rows of a short K that would be shared
+//     by three and more (512 x 512, 1200 tokens 6.6 / 7.3; 1152 x 1152, 769 tokens 10.0 / 10.8; 400 tokens 9.4 / 8.2).
+//   else the pair kernel (740 clocks a step, 1500 a tile).  A second wave of CTAs starts one by one, not as a whole, and fp32 rows with their residual are moved after
+//     the products of a tile and not beside them: 12 % more, bf16 rows 20, fp32 rows 30.  8192 x 2048: bf16 640 tokens 27.8 / 21.0, 1200 tokens 38.4 / 40.5; residual 640
+//     tokens 34.6 / 26.9, 1200 tokens 48.7 / 56.1; 16384 x 2048 residual 1025 tokens 78.1 / 96.0; gate || up 32768 x 2048 263 tokens 54 / 39, 1024 tokens 101 / 133.
 //
 // Decode-sized calls (up to 128 tokens): where its grid is one wave, but for long K with up to 64 tokens, which the two-CTAs-per-SM stream of this file's
 // swap kernels reads faster.  5 tokens: 8192 x 2048 13.4 / 9.3, 2048 x 2048 7.1 / 5.6 (without the zeroed accumulator), 16384 x 2048 gate || up
@@ -1185,13 +1190,20 @@ static bool cluster_form(const GemmArgs& a, long long ldr, int swap) {
   if (a.features % 4 != 0 || a.ldo % 4 != 0 || !aligned(a.out, 16) || !aligned(a.bias, 16)) return false;
   if (a.mode == PG_EPI_ATOMIC_F32 || (a.resid != nullptr && (ldr % 4 != 0 || !aligned(a.resid, 16)))) return false;
   if (swap) return a.stats == nullptr && a.zero_buf == nullptr && (a.K <= 4096 || a.tokens > 64) && plan_cluster_gemm(a.tokens, a.features, a.K).waves == 1;
-  if (a.K <= 128 && a.tokens <= 4096) return true;  // (all epilogue: 2048 x 64 3750 tokens 14.6 / 9.3, 8192 25.9 / 28.0; K 256 15.9 / 16.9)
-  if (a.tokens > 1408) return false;
-  const int pairs = num_sms() / 2, pair_tiles = ((a.tokens + 2 * BM - 1) / (2 * BM)) * ((a.features + 255) / 256);
-  if (pair_tiles < pairs || (a.mode == PG_EPI_BF16 && a.act_gelu)) return true;
+  if (a.tokens > 4096 || (a.tokens > 1408 && a.K > 128)) return false;
   const ClusterGemmPlan plan = plan_cluster_gemm(a.tokens, a.features, a.K);
-  // (CTAs of a second wave start one by one, against the estimate of whole waves: 12 % more)
-  return plan.clocks * (plan.waves > 1 ? 1.12f : 1.f) < (pair_tiles + pairs - 1) / pairs * ((a.K + BK - 1) / BK * 740.f + 1500.f) + 5000.f;
+  const bool f32 = a.mode == PG_EPI_F32, act = a.mode == PG_EPI_BF16 && a.act_gelu, plain = a.mode == PG_EPI_BF16 && !act;
+  if (a.tokens > 1408) return a.features >= (f32 ? 1024 : 512) && plan.waves <= (plain ? 3 : f32 ? 4 : 5);
+  if (a.K <= 128) return true;
+  const int sms = num_sms(), pairs = sms / 2, pair_tiles = ((a.tokens + 2 * BM - 1) / (2 * BM)) * ((a.features + 255) / 256);
+  const float steps = static_cast<float>((a.K + BK - 1) / BK);
+  if (act) {
+    const int tiles = ((a.tokens + BM - 1) / BM) * ((a.features + 255) / 256);
+    return plan.waves == 1 || plan.clocks < (tiles + sms - 1) / sms * (steps * 640.f + 4500.f) + 8000.f;
+  }
+  if (pair_tiles < pairs) return !(plain && plan.split >= 3 && a.K <= 1152 && a.tokens > 512);
+  const float more = plan.waves == 1 ? 1.f : f32 ? 1.3f : plain ? 1.2f : 1.12f;
+  return plan.clocks * more < (pair_tiles + pairs - 1) / pairs * (steps * 740.f + 1500.f) + 5000.f;
 }
 
 }  // namespace pg
