@@ -1210,11 +1210,15 @@ static bool cluster_form(const GemmArgs& a, long long ldr, int swap) {
 
 using namespace pg;
 
-// Whether a product with fp32 rows adds up K by itself (gemm_cluster.cu), without split-K partials.
+// Whether a product with fp32 rows adds up K by itself (gemm_cluster.cu), without split-K partials.  Decode-sized: not where one CTA per tile leaves a third of the SMs
+// or more without weights to stream and there are many of them (us, split / clustered, up to 64 tokens: 12288 x 4096 20.8 / 22.2, 10240 x 2048 12.4 / 12.8;
+// 12288 x 1024 10.4 / 8.8, 16384 x 2048 with 128 tiles 16.6 / 13.6; 128 tokens 12288 x 4096 27.6 / 25.6).
 bool pg_gemm_sums_once(int tokens, int features, int K, const void* out, long long ldo, const float* bias, int swap) {
   GemmArgs a = {};
   a.tokens = tokens; a.features = features; a.K = K; a.mode = PG_EPI_F32; a.out = const_cast<void*>(out); a.ldo = ldo; a.bias = bias;
-  return cluster_form(a, 0, swap);
+  if (!cluster_form(a, 0, swap)) return false;
+  const int tiles = (features + BM - 1) / BM;
+  return !(swap && tokens <= 64 && tiles * 10 < num_sms() * 7 && static_cast<long long>(features) * K >= 20000000 && plan_cluster_gemm(tokens, features, K).split == 1);
 }
 
 extern "C" int pg_gemm_bf16(const void* x, long long ldx, const void* w, long long ldw, void* out, long long ldo,

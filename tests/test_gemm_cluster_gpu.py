@@ -123,7 +123,7 @@ def test_residual_buffers_may_be_larger(T):
         _lib.gemm_residual(x, w, h[:T - 1], bias=b)
 
 
-@pytest.mark.parametrize("F,K", [(64, 4104), (256, 8192), (512, 1024)])
+@pytest.mark.parametrize("F,K", [(64, 4104), (256, 8192), (512, 1024), (12288, 1640)])
 def test_one_row_of_any_pitch(F, K):
     """The one row of a one-token product may come with any row pitch (a view of a column, an expanded row), also where its sums are split."""
     x, w, b, acc, bound = _operands(1, F, K, F)
