@@ -1027,12 +1027,15 @@ extern "C" int pg_attn_prepare(const void* qkv, long long ld, const int* pos, co
   if (v_from_k && vdim != dim) return PG_ERR_ARG;
   if (norm_qk < 0 || norm_qk > 2 || (v_other != nullptr && k_pages == nullptr)) return PG_ERR_ARG;
   if ((k_pages == nullptr) != (v_pages == nullptr)) return PG_ERR_ARG;
-  // heads of 8, 16, .. 256 elements on 16-byte boundaries take the vector form (a norm per value head wants its lanes inside a warp as well)
+  // heads of 8, 16, .. 256 elements on 16-byte boundaries take the vector form (a norm per value head wants its lanes inside a warp as well); but not up to four
+  // short vectors, one for each warp of the element-wise form (us, element-wise / vector: 2 + 1 + 1 heads x 32, fp32, 2200 rows 4.3 / 5.1, 1 + 1 + 1 with norms,
+  // 8192 rows 11.8 / 15.0; 4 + 1 + 1 heads 5.3 / 5.1 and 17.5 / 15.0)
   auto lanes = [](int n) { return n % 8 == 0 && n / 8 <= 32 && (n / 8 & (n / 8 - 1)) == 0; };
   const uintptr_t ptrs = reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(k_pages) |
                          reinterpret_cast<uintptr_t>(v_pages) | reinterpret_cast<uintptr_t>(q_norm) | reinterpret_cast<uintptr_t>(k_norm) |
                          reinterpret_cast<uintptr_t>(v_other);
-  if (lanes(dim) && lanes(vdim) && (vdim == dim || !norm_v) && ld % 8 == 0 && ld_v_other % 8 == 0 && (ptrs & 15) == 0) {
+  const bool few = (k_pages != nullptr ? H + 2 * G : H) <= 4 && dim <= 64 && vdim <= 64;
+  if (!few && lanes(dim) && lanes(vdim) && (vdim == dim || !norm_v) && ld % 8 == 0 && ld_v_other % 8 == 0 && (ptrs & 15) == 0) {
     auto go = [&](auto kernel, auto t, int tok) {
       using TA = decltype(t);
       kernel<<<(rows + tok - 1) / tok, 128, (size_t)(tok * rot_dims + 2) * sizeof(float), PG_ST(stream)>>>(
