@@ -655,6 +655,12 @@ class RoutedFeedForward:
         return ((not self.glu or self.w_up_dense is not None) and not prec.f32 and self.D % 8 == 0 and self.F % 8 == 0 and T * self.top >= self.DENSE_SEGMENT_ROWS * self.n_real
                 and not torch.cuda.is_current_stream_capturing())
 
+    def _gather_pays(self, pairs):
+        """Whether the products over gathered rows (one launch more) beat those that gather on the way: not for the smallest experts.  us, gather on the way / gathered:
+        128 x 64 64 tokens 7.8 / 9.4, one token 7.7 / 7.8; 256 x 128 one token 10.1 / 8.8, 256 pairs 10.5 / 10.6, 1400 pairs 11.3 / 12.0; 512 x 256 2800 pairs 19.8 / 15.2."""
+        size = self.D * self.F
+        return size >= 65536 or (size >= 16384 and pairs < 512)
+
     def expert_products(self, h, plan, counts, prec):
         """fp32 rows [pairs, D] in the plan's sorted order: the expert's output for every (token, real expert) pair."""
         T = h.shape[0]
@@ -670,7 +676,7 @@ class RoutedFeedForward:
                                                     eo.data_ptr(), eo.stride(0), C.addressof(per), self.n_real, self.D, self.F, self.act, _lib.stream()),
                        "pg_moe_dense_runs")
             return eo
-        if not prec.f32 and self.D % 8 == 0 and self.F % 8 == 0 and plan.max_tiles <= 65535:
+        if not prec.f32 and self.D % 8 == 0 and self.F % 8 == 0 and plan.max_tiles <= 65535 and self._gather_pays(plan.pairs):
             return seq_ops.moe_products(h, plan, self.w_up, self.w_down, prec.empty(plan.pairs, self.D), prec.empty(plan.pairs, self.F),
                                         torch.empty(plan.pairs, self.D, device="cuda", dtype=torch.float32), self.act)
         mid = seq_ops.moe_gemm(h, plan, self.w_up, prec.empty(plan.pairs, self.F), gather=True, act=self.act)

@@ -102,3 +102,23 @@ def test_rows_next_to_a_tile_stay_out(T, top, n):
             if e == n - 1:
                 assert eo[row, D - 1].isnan()
     assert owned < plan.pairs and not eo[owned:].any()
+
+
+@pytest.mark.parametrize("D,F,T", [(128, 64, 5), (128, 128, 5), (128, 128, 300), (256, 256, 5), (256, 256, 300)])
+@pytest.mark.parametrize("activation", ["relu2", "silu_glu"])
+def test_both_sides_of_the_line(D, F, T, activation):
+    """Whichever kernels a routed feed-forward takes for its size, its rows are those of the products that gather on the way."""
+    from paligemma_multimodal_system_b200 import mixers
+    prec, n, top = seq_ops.Precision(torch.bfloat16), 4, 2
+    ff = mixers.RoutedFeedForward(D, n, 0, top, 1, 1, 1.0, F, 0, activation=activation, correction=False)
+    ff.load(lambda name, shape: torch.randn(*shape, device="cuda") * shape[-1] ** -0.5, "")
+    ff.pack(prec)
+    ids = torch.stack([torch.randperm(n, device="cuda")[:top] for _ in range(T)]).to(torch.int32).contiguous()
+    counts = torch.bincount(ids.flatten().long(), minlength=n).to(torch.int32)
+    plan = seq_ops.MoePlan(ids, counts, n)
+    h = torch.randn(T, D, device="cuda").bfloat16()
+    eo = ff.expert_products(h, plan, counts, prec)
+    mid = seq_ops.moe_gemm(h, plan, ff.w_up, prec.empty(plan.pairs, F), gather=True, act=ff.act)
+    want = seq_ops.moe_gemm(mid, plan, ff.w_down, torch.empty(plan.pairs, D, device="cuda"), gather=False)
+    # activations that round to neighbouring bf16 values: 2^-8 of each, F of them with weights of about F^-0.5
+    assert (eo - want).abs().max() <= 2.0 ** -7 * mid.float().abs().max()
