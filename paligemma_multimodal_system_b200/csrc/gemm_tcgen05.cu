@@ -1181,11 +1181,17 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& 
 // Never for PG_EPI_ATOMIC_F32: calls that share an output, on several streams or as several splits, need the red.add of this file's kernels.  (pg_gemm_residual
 // chooses: an owned residual stream of a prompt takes PG_EPI_F32; that of a decode step stays with the split, because under the L2 prefetch stream of
 // modeling_gemma.py clusters wait for whole GPCs: one request of 24 tokens 28.5 -> 29.5 ms, 64 requests 132 -> 138.)
-static bool cluster_form(const GemmArgs& a, long long ldr, int swap) {
+//
+// beside: other products run next to this one, on other streams.  A cluster form is planned for the whole GPU and leaves nothing for them; it pays where the product
+// alone is worth that, and for gated rows, whose persistent kernels have no tile below 128 features.  One call of routed experts on four streams (us, this file's kernels /
+// clustered): 64 x (1024 x 512), relu squared, 384 rows each 393 / 605, 128 x (2048 x 512) 256 rows 1007 / 1448, 32 x (2048 x 768) 512 rows (0.8e9) 485 / 509, 875 rows
+// (1.4e9) 671 / 588, 8 x (4096 x 2048) 375 rows 333 / 253; gated 8 x (4096 x 2048) 377 / 298.
+static bool cluster_form(const GemmArgs& a, long long ldr, int swap, bool beside = false) {
   auto aligned = [](const void* p, int n) { return (reinterpret_cast<uintptr_t>(p) & (n - 1)) == 0; };
   // a tuning or profiling switch that is set speaks of this file's kernels
   if (g_gemm_trace != nullptr) return false;
   if (!swap && (g_force_bn != 0 || g_pair_mode != 1 || g_epi8_mode != 0 || g_band_mode != 1 || g_pair_min_tiles != kPairMinTiles)) return false;
+  if (beside && a.mode != PG_EPI_GEGLU && static_cast<double>(a.tokens) * a.features * a.K < 1.2e9) return false;
   // vectors of four: outputs, bias and residual rows
   if (a.features % 4 != 0 || a.ldo % 4 != 0 || !aligned(a.out, 16) || !aligned(a.bias, 16)) return false;
   if (a.mode == PG_EPI_ATOMIC_F32 || (a.resid != nullptr && (ldr % 4 != 0 || !aligned(a.resid, 16)))) return false;
@@ -1221,17 +1227,8 @@ bool pg_gemm_sums_once(int tokens, int features, int K, const void* out, long lo
   return !(swap && tokens <= 64 && tiles * 10 < num_sms() * 7 && static_cast<long long>(features) * K >= 20000000 && plan_cluster_gemm(tokens, features, K).split == 1);
 }
 
-extern "C" int pg_gemm_bf16(const void* x, long long ldx, const void* w, long long ldw, void* out, long long ldo,
-                            const float* bias, const float* resid, long long ldr, int tokens, int features, int K,
-                            int mode, int act_gelu, float scale, int swap, int split_k, void* stream) {
-  return pg_gemm_bf16_fused(x, ldx, w, ldw, out, ldo, bias, resid, ldr, tokens, features, K, mode, act_gelu, scale, swap,
-                            split_k, nullptr, stream);
-}
-
-extern "C" int pg_gemm_bf16_fused(const void* x, long long ldx, const void* w, long long ldw, void* out, long long ldo,
-                                  const float* bias, const float* resid, long long ldr, int tokens, int features, int K,
-                                  int mode, int act_gelu, float scale, int swap, int split_k, const PgGemmFusion* fu,
-                                  void* stream) {
+static int gemm_bf16(const void* x, long long ldx, const void* w, long long ldw, void* out, long long ldo, const float* bias, const float* resid, long long ldr, int tokens,
+                     int features, int K, int mode, int act_gelu, float scale, int swap, int split_k, const PgGemmFusion* fu, bool beside, void* stream) {
   if (tokens <= 0 || features <= 0 || K <= 0) return PG_ERR_ARG;
   if ((K % 8) != 0 || (ldw % 8) != 0) return PG_ERR_ARG;  // TMA: 16 B pitch granularity
   if (reinterpret_cast<uintptr_t>(w) & 15) return PG_ERR_ARG;
@@ -1297,7 +1294,7 @@ extern "C" int pg_gemm_bf16_fused(const void* x, long long ldx, const void* w, l
                      (resid == nullptr || ((ldr % 4) == 0 && (reinterpret_cast<uintptr_t>(resid) & 15) == 0))) ? 1 : 0;
   a.trace = g_gemm_trace ? g_gemm_trace + 8 * (g_gemm_trace_idx++ % 64) : nullptr;
 
-  if (cluster_form(a, ldr, swap)) {
+  if (cluster_form(a, ldr, swap, beside)) {
     ClusterGemmArgs c = {};
     c.tokens = tokens; c.features = features; c.K = K; c.mode = mode; c.act = act_gelu; c.scale = scale; c.glu_alpha = a.glu_alpha;
     c.out = out; c.ldo = ldo; c.bias = bias; c.resid = mode == PG_EPI_F32 ? resid : nullptr; c.ldr = ldr; c.out_row_map = a.out_row_map; c.resid_mod = a.resid_mod;
@@ -1354,6 +1351,25 @@ extern "C" int pg_gemm_bf16_fused(const void* x, long long ldx, const void* w, l
       default: return launch<256, false>(ta, tb, a, tiles, st);
     }
   }
+}
+
+extern "C" int pg_gemm_bf16(const void* x, long long ldx, const void* w, long long ldw, void* out, long long ldo,
+                            const float* bias, const float* resid, long long ldr, int tokens, int features, int K,
+                            int mode, int act_gelu, float scale, int swap, int split_k, void* stream) {
+  return gemm_bf16(x, ldx, w, ldw, out, ldo, bias, resid, ldr, tokens, features, K, mode, act_gelu, scale, swap, split_k, nullptr, false, stream);
+}
+
+extern "C" int pg_gemm_bf16_fused(const void* x, long long ldx, const void* w, long long ldw, void* out, long long ldo,
+                                  const float* bias, const float* resid, long long ldr, int tokens, int features, int K,
+                                  int mode, int act_gelu, float scale, int swap, int split_k, const PgGemmFusion* fu,
+                                  void* stream) {
+  return gemm_bf16(x, ldx, w, ldw, out, ldo, bias, resid, ldr, tokens, features, K, mode, act_gelu, scale, swap, split_k, fu, false, stream);
+}
+
+// One of several products on streams of their own (seq_moe.cu): rows without bias and residual.
+int pg_gemm_beside(const void* x, long long ldx, const void* w, long long ldw, void* out, long long ldo, int tokens, int features, int K, int mode, int act, bool beside,
+                   void* stream) {
+  return gemm_bf16(x, ldx, w, ldw, out, ldo, nullptr, nullptr, 0, tokens, features, K, mode, act, 1.0f, tokens <= 128 ? 1 : 0, 1, nullptr, beside, stream);
 }
 
 extern "C" int pg_gemm_qkv_rope(const void* x, long long ldx, const void* w, long long ldw, void* qkv_out, long long ldo, int tokens,

@@ -19,6 +19,10 @@
 
 using bf16 = __nv_bfloat16;
 
+// gemm_tcgen05.cu
+int pg_gemm_beside(const void* x, long long ldx, const void* w, long long ldw, void* out, long long ldo, int tokens, int features, int K, int mode, int act, bool beside,
+                   void* stream);
+
 #define PG_ST(s) reinterpret_cast<cudaStream_t>(s)
 #define PG_RET()                                                    \
   do {                                                              \
@@ -668,16 +672,15 @@ extern "C" int pg_moe_dense_runs(const void* xg, long long ldx, const void* w_up
       if (cudaStreamWaitEvent(ss->s[i], ss->fork, 0) != cudaSuccess) return PG_ERR_CUDA;
   }
   long long off = 0;
-  int rc = PG_OK, used = 0;
+  int rc = PG_OK, used = 0, runs = 0;
+  for (int e = 0; e < n_real; ++e) runs += counts_host[e] > 0;
+  const bool beside = ss != nullptr && runs > 1;
   for (int e = 0; e < n_real && rc == PG_OK; ++e) {
     const int c = counts_host[e];
     if (c <= 0) continue;
     void* st = ss != nullptr ? static_cast<void*>(ss->s[used++ % kSideStreams]) : stream;
-    const int swap = c <= 128 ? 1 : 0;
-    rc = pg_gemm_bf16(x + off * ldx, ldx, wu + (long long)e * up_rows * D, D, m + off * ldm, ldm, nullptr, nullptr, 0, c, up_rows, D,
-                      glu ? PG_EPI_GEGLU : PG_EPI_BF16, act, 1.0f, swap, 1, st);
-    if (rc == PG_OK)
-      rc = pg_gemm_bf16(m + off * ldm, ldm, wd + (long long)e * D * F, F, eo + off * ldo, ldo, nullptr, nullptr, 0, c, D, F, PG_EPI_F32, 0, 1.0f, swap, 1, st);
+    rc = pg_gemm_beside(x + off * ldx, ldx, wu + (long long)e * up_rows * D, D, m + off * ldm, ldm, c, up_rows, D, glu ? PG_EPI_GEGLU : PG_EPI_BF16, act, beside, st);
+    if (rc == PG_OK) rc = pg_gemm_beside(m + off * ldm, ldm, wd + (long long)e * D * F, F, eo + off * ldo, ldo, c, D, F, PG_EPI_F32, 0, beside, st);
     off += c;
   }
   if (ss != nullptr)  // join even after an error: the caller's stream must not run ahead of work already issued

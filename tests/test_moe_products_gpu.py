@@ -122,3 +122,23 @@ def test_both_sides_of_the_line(D, F, T, activation):
     want = seq_ops.moe_gemm(mid, plan, ff.w_down, torch.empty(plan.pairs, D, device="cuda"), gather=False)
     # activations that round to neighbouring bf16 values: 2^-8 of each, F of them with weights of about F^-0.5
     assert (eo - want).abs().max() <= 2.0 ** -7 * mid.float().abs().max()
+
+
+@pytest.mark.parametrize("D,F,T", [(128, 64, 520), (1024, 512, 900), (2048, 2048, 700)])  # the last: above 1.2e9 multiply-adds a run
+@pytest.mark.parametrize("activation", ["relu2", "silu_glu"])
+def test_dense_runs(D, F, T, activation):
+    """Long runs as dense products side by side, the small ones on the persistent kernels and the large ones clustered: the rows of the products that gather on the way."""
+    from paligemma_multimodal_system_b200 import mixers
+    prec, n = seq_ops.Precision(torch.bfloat16), 2
+    ff = mixers.RoutedFeedForward(D, n, 0, 1, 1, 1, 1.0, F, 0, activation=activation, correction=False)
+    ff.load(lambda name, shape: torch.randn(*shape, device="cuda") * shape[-1] ** -0.5, "")
+    ff.pack(prec)
+    ids = (torch.rand(T, 1, device="cuda") < 0.4).to(torch.int32)
+    counts = torch.bincount(ids.flatten().long(), minlength=n).to(torch.int32)
+    plan = seq_ops.MoePlan(ids, counts, n)
+    h = torch.randn(T, D, device="cuda").bfloat16()
+    assert ff._dense_segments(T, prec)
+    eo = ff.expert_products(h, plan, counts, prec)
+    mid = seq_ops.moe_gemm(h, plan, ff.w_up, prec.empty(plan.pairs, F), gather=True, act=ff.act)
+    want = seq_ops.moe_gemm(mid, plan, ff.w_down, torch.empty(plan.pairs, D, device="cuda"), gather=False)
+    assert (eo - want).abs().max() <= 2.0 ** -7 * mid.float().abs().max()
