@@ -25,7 +25,7 @@ PG_DEVINL float glu_act(float g, float u, int kind, float limit, float alpha) {
 }
 
 // f(ActConst<...>) for the activation of a call: chosen once per run of elements.  A test per element made the epilogue, not the main loop, pace the products with a
-// gated unit or a gelu: gate || up of 16640 tokens, 32768 x 2048: 2296 us (973 TFLOP/s), now 1515 (1474).
+// gated unit or a gelu: gate || up of 16640 tokens, 32768 x 2048: 2296 us (973 TFLOP/s), now 1500 (1489).
 template <int N>
 struct ActConst { static constexpr int value = N; };
 template <typename Fn>

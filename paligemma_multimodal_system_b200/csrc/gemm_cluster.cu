@@ -1,5 +1,6 @@
-// Products of a moderate number of tokens (above the 128 of a decode step, below what fills the GPU with 256-wide token tiles):
-// one image, one prompt, one mixed step of the serving engine.
+// Products of a moderate number of tokens, below what fills the GPU with 256-wide token tiles: one image, one prompt, one mixed step of the serving engine (up to
+// 1408 tokens, with K <= 128 up to 4096), and decode steps of up to 128 tokens whose grid is one wave.  cluster_form in gemm_tcgen05.cu gives the lines and
+// both sides of them.  In its grouped form the same kernel walks the routing plan of the experts.
 //
 //   out[t, f] = epilogue(sum_k X[t, k] W[f, k])       X [tokens, K], W [features, K] bf16, fp32 accumulation
 //

@@ -684,48 +684,46 @@ PG_DEVINL void token_major_epilogue(const GemmArgs& args, uint32_t taddr, int m_
     // columns: [g0..g63 | u0..u63] per 128-column block; out feature = n_blk*BN/2 + blk*64 + c.  The 64 bf16
     // results of a block (one 128-byte row per token) leave through the warp transposition tile as full lines.
     const bool al = ((reinterpret_cast<uintptr_t>(args.out) & 15) == 0) && ((args.ldo % 8) == 0);
-    {
 #pragma unroll 1
-      for (int blk = ((EPI8 && BN >= 256) ? half : 0); blk < ((EPI8 && BN >= 256) ? half + 1 : (half == 0 ? BN / 128 : 0)); ++blk) {
-        const int f0 = n_blk * (BN / 2) + blk * 64;
-        if (f0 >= args.features / 2) break;  // warp-uniform (features % 128 == 0)
-        uint32_t pk[32];
+    for (int blk = ((EPI8 && BN >= 256) ? half : 0); blk < ((EPI8 && BN >= 256) ? half + 1 : (half == 0 ? BN / 128 : 0)); ++blk) {
+      const int f0 = n_blk * (BN / 2) + blk * 64;
+      if (f0 >= args.features / 2) break;  // warp-uniform (features % 128 == 0)
+      uint32_t pk[32];
 #pragma unroll
-        for (int c0 = 0; c0 < 64; c0 += 32) {
-          // 32 pairs requested together: one wait for the accumulator per half block
-          uint32_t g[2][16], u[2][16];
+      for (int c0 = 0; c0 < 64; c0 += 32) {
+        // 32 pairs requested together: one wait for the accumulator per half block
+        uint32_t g[2][16], u[2][16];
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            tmem_ld16(taddr + blk * 128 + c0 + 16 * h, g[h]);
-            tmem_ld16(taddr + blk * 128 + 64 + c0 + 16 * h, u[h]);
-          }
-          tmem_ld_wait();
-          const float* bg = args.bias != nullptr ? args.bias + n_blk * BN + blk * 128 + c0 : nullptr;  // packed order: [64 gate | 64 up]
-          if (bg != nullptr) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              g[i / 16][i % 16] = __float_as_uint(__uint_as_float(g[i / 16][i % 16]) + __ldg(bg + i));
-              u[i / 16][i % 16] = __float_as_uint(__uint_as_float(u[i / 16][i % 16]) + __ldg(bg + 64 + i));
-            }
-          }
-          with_glu(args.act_gelu, [&](auto kind) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const float a = glu_act(__uint_as_float(g[i / 8][2 * i % 16]), __uint_as_float(u[i / 8][2 * i % 16]), decltype(kind)::value, args.scale, args.glu_alpha);
-              const float b = glu_act(__uint_as_float(g[i / 8][2 * i % 16 + 1]), __uint_as_float(u[i / 8][2 * i % 16 + 1]), decltype(kind)::value, args.scale,
-                                      args.glu_alpha);
-              pk[(c0 / 2 + i) & 31] = pack_bf16(a, b);
-            }
-          });
+        for (int h = 0; h < 2; ++h) {
+          tmem_ld16(taddr + blk * 128 + c0 + 16 * h, g[h]);
+          tmem_ld16(taddr + blk * 128 + 64 + c0 + 16 * h, u[h]);
         }
-        if (al) {
-          warp_store_rows_128B(wstage, lane, pk, reinterpret_cast<char*>(out_bf + static_cast<long long>(m_blk * BM + q * 32) * args.ldo + f0),
-                               args.ldo * 2, rows_valid, true);
-        } else if (row_ok) {
-          __nv_bfloat16* dst = out_bf + static_cast<long long>(tok) * args.ldo + f0;
+        tmem_ld_wait();
+        const float* bg = args.bias != nullptr ? args.bias + n_blk * BN + blk * 128 + c0 : nullptr;  // packed order: [64 gate | 64 up]
+        if (bg != nullptr) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) *reinterpret_cast<uint32_t*>(dst + 2 * i) = pk[i];
+          for (int i = 0; i < 32; ++i) {
+            g[i / 16][i % 16] = __float_as_uint(__uint_as_float(g[i / 16][i % 16]) + __ldg(bg + i));
+            u[i / 16][i % 16] = __float_as_uint(__uint_as_float(u[i / 16][i % 16]) + __ldg(bg + 64 + i));
+          }
         }
+        with_glu(args.act_gelu, [&](auto kind) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const float a = glu_act(__uint_as_float(g[i / 8][2 * i % 16]), __uint_as_float(u[i / 8][2 * i % 16]), decltype(kind)::value, args.scale, args.glu_alpha);
+            const float b = glu_act(__uint_as_float(g[i / 8][2 * i % 16 + 1]), __uint_as_float(u[i / 8][2 * i % 16 + 1]), decltype(kind)::value, args.scale,
+                                    args.glu_alpha);
+            pk[(c0 / 2 + i) & 31] = pack_bf16(a, b);
+          }
+        });
+      }
+      if (al) {
+        warp_store_rows_128B(wstage, lane, pk, reinterpret_cast<char*>(out_bf + static_cast<long long>(m_blk * BM + q * 32) * args.ldo + f0),
+                             args.ldo * 2, rows_valid, true);
+      } else if (row_ok) {
+        __nv_bfloat16* dst = out_bf + static_cast<long long>(tok) * args.ldo + f0;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) *reinterpret_cast<uint32_t*>(dst + 2 * i) = pk[i];
       }
     }
   } else if (mode == PG_EPI_BF16) {

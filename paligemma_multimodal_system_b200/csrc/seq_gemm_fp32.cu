@@ -328,8 +328,9 @@ int pg_gemm_fp32(const float* x, long long ldx, long long bsx, const float* w, l
                     ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
   cudaError_t e;
   if (wide && T <= 16) {
-    // four features a warp while the sums leave room for two CTAs per SM; 16384 x 2048 weights: 4 tokens 25 us (5.3 TB/s), 6 tokens 27, 8 tokens 36,
-    // 16 tokens 51; the 32 x 64 tile takes 66 for 17 .. 32 tokens
+    // A warp keeps a pair of sums per feature and token.  Two CTAs of 256 threads on an SM leave a thread 128 registers: four features a warp fit them up to six
+    // tokens (48 registers of sums; 32 bytes spill), two features up to eight; nine and more take four features with one CTA per SM.  16384 x 2048 weights: 4
+    // tokens 25 us (5.3 TB/s), 6 tokens 27, 8 tokens 36, 16 tokens 51; the 32 x 64 tile takes 66 for 17 .. 32 tokens
     e = T <= 4   ? launch_rows<4, 4, 2, 2>(batch, sms, st, p)
         : T <= 6 ? launch_rows<6, 4, 2, 2>(batch, sms, st, p)
         : T <= 8 ? launch_rows<8, 2, 4, 2>(batch, sms, st, p)
