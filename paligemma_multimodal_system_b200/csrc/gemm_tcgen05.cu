@@ -1180,16 +1180,15 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& 
 // chooses: an owned residual stream of a prompt takes PG_EPI_F32; that of a decode step stays with the split, because under the L2 prefetch stream of
 // modeling_gemma.py clusters wait for whole GPCs: one request of 24 tokens 28.5 -> 29.5 ms, 64 requests 132 -> 138.)
 //
-// beside: other products run next to this one, on other streams.  A cluster form is planned for the whole GPU and leaves nothing for them; it pays where the product
-// alone is worth that, and for gated rows, whose persistent kernels have no tile below 128 features.  One call of routed experts on four streams (us, this file's kernels /
-// clustered): 64 x (1024 x 512), relu squared, 384 rows each 393 / 605, 128 x (2048 x 512) 256 rows 1007 / 1448, 32 x (2048 x 768) 512 rows (0.8e9) 485 / 509, 875 rows
-// (1.4e9) 671 / 588, 8 x (4096 x 2048) 375 rows 333 / 253; gated 8 x (4096 x 2048) 377 / 298.
+// beside: other products run next to this one, on other streams.  A clustered product is planned for the whole GPU and leaves nothing for them; it pays where the
+// product alone is worth that.  One call of routed experts on four streams (us, this file's kernels / clustered): 64 x (1024 x 512), relu squared, 384 rows each
+// 393 / 605, 128 x (2048 x 512) 256 rows 1007 / 1448, 32 x (2048 x 768) 512 rows (0.8e9) 485 / 509, 875 rows (1.4e9) 671 / 588, 8 x (4096 x 2048) 375 rows 333 / 253.
 static bool cluster_form(const GemmArgs& a, long long ldr, int swap, bool beside = false) {
   auto aligned = [](const void* p, int n) { return (reinterpret_cast<uintptr_t>(p) & (n - 1)) == 0; };
   // a tuning or profiling switch that is set speaks of this file's kernels
   if (g_gemm_trace != nullptr) return false;
   if (!swap && (g_force_bn != 0 || g_pair_mode != 1 || g_epi8_mode != 0 || g_band_mode != 1 || g_pair_min_tiles != kPairMinTiles)) return false;
-  if (beside && a.mode != PG_EPI_GEGLU && static_cast<double>(a.tokens) * a.features * a.K < 1.2e9) return false;
+  if (beside && static_cast<double>(a.tokens) * a.features * a.K < 1.2e9) return false;
   // vectors of four: outputs, bias and residual rows
   if (a.features % 4 != 0 || a.ldo % 4 != 0 || !aligned(a.out, 16) || !aligned(a.bias, 16)) return false;
   if (a.mode == PG_EPI_ATOMIC_F32 || (a.resid != nullptr && (ldr % 4 != 0 || !aligned(a.resid, 16)))) return false;

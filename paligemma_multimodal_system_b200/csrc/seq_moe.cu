@@ -674,7 +674,9 @@ extern "C" int pg_moe_dense_runs(const void* xg, long long ldx, const void* w_up
   long long off = 0;
   int rc = PG_OK, used = 0, runs = 0;
   for (int e = 0; e < n_real; ++e) runs += counts_host[e] > 0;
-  const bool beside = ss != nullptr && runs > 1;
+  // (gated experts keep both products clustered: the persistent kernels have no gated tile below 128 features; 8 x (4096 x 2048) 377 / 298, 14 x (2048 x 1024) 1170
+  // rows 492 / 387; with few rows each 64 x (1024 x 512) 590 / 688, and clustered up beside persistent down products 721)
+  const bool beside = ss != nullptr && runs > 1 && !glu;
   for (int e = 0; e < n_real && rc == PG_OK; ++e) {
     const int c = counts_host[e];
     if (c <= 0) continue;
