@@ -1162,12 +1162,12 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& 
 
 // Whether a product takes the form of gemm_cluster.cu.  Prompts: up to 1408 tokens, where its estimate (plan_cluster_gemm) is below that of this file's kernel for the
 // call.  The estimates were fitted to 1900 products timed in turn on both sides (256 .. 32768 features, K 16 .. 16384, 200 .. 4096 tokens); where
-// the clustered form is chosen no one of them is more than 3 % slower by it.  us, this file's kernels / gemm_cluster.cu, N x K weights:
+// the clustered form is chosen no one of them is more than 3 % slower by it, but for the last note on few pair tiles.  us, this file's kernels / gemm_cluster.cu, N x K weights:
 //   K <= 128: all epilogue, and the clustered one is spread over more CTAs.  2048 x 64, 3750 tokens, fp32 rows 14.4 / 9.9; above 1408 tokens not for few features (256,
 //     4096 tokens 6.5 / 9.7; 512, fp32 rows 9.0 / 9.6) nor for many waves of bf16 rows (8192, 4096 tokens 32.0 / 36.2).
 //   activations (bf16 rows): this file's one-CTA kernel (640 clocks a 64-deep step, 4500 a tile).  8192 x 2048, 640 tokens 36.4 / 23.0; 16384 x 2048, 1408 tokens 84.6 / 99.2.
-//   fewer than 74 pair tiles: 3456 x 1152, 263 tokens 14.4 / 8.2; 2048 x 16384 with residual, 1300 tokens 163 / 86; but plain bf16 rows of a short K that would be shared
-//     by three and more (512 x 512, 1200 tokens 6.6 / 7.3; 1152 x 1152, 769 tokens 10.0 / 10.8; 400 tokens 9.4 / 8.2).
+//   fewer than 74 pair tiles: 3456 x 1152, 263 tokens 14.4 / 8.2; 2048 x 16384 with residual, 1300 tokens 163 / 86.  (Plain bf16 rows of a short K that three and more share
+//     lose a little: 512 x 512, 1200 tokens 6.6 / 7.3; 1152 x 1152, 769 tokens 10.0 / 10.8, 400 tokens 9.4 / 8.2.)
 //   else the pair kernel (740 clocks a step, 1500 a tile).  A second wave of CTAs starts one by one, not as a whole, and fp32 rows with their residual are moved after
 //     the products of a tile and not beside them: 12 % more, bf16 rows 20, fp32 rows 30.  8192 x 2048: bf16 640 tokens 27.8 / 21.0, 1200 tokens 38.4 / 40.5; residual 640
 //     tokens 34.6 / 26.9, 1200 tokens 48.7 / 56.1; 16384 x 2048 residual 1025 tokens 78.1 / 96.0; gate || up 32768 x 2048 263 tokens 54 / 39, 1024 tokens 101 / 133.
@@ -1204,7 +1204,7 @@ static bool cluster_form(const GemmArgs& a, long long ldr, int swap, bool beside
     const int tiles = ((a.tokens + BM - 1) / BM) * ((a.features + 255) / 256);
     return plan.waves == 1 || plan.clocks < (tiles + sms - 1) / sms * (steps * 640.f + 4500.f) + 8000.f;
   }
-  if (pair_tiles < pairs) return !(plain && plan.split >= 3 && a.K <= 1152 && a.tokens > 512);
+  if (pair_tiles < pairs) return true;
   const float more = plan.waves == 1 ? 1.f : f32 ? 1.3f : plain ? 1.2f : 1.12f;
   return plan.clocks * more < (pair_tiles + pairs - 1) / pairs * (steps * 740.f + 1500.f) + 5000.f;
 }
