@@ -575,7 +575,7 @@ def moe_gemm(x, plan: MoePlan, w, out, gather, act=0):
 def moe_products(x, plan: MoePlan, w_up, w_down, xg, mid, eo, act):
     """eo[row] = act(x[token of row] @ w_up[expert(row)].T) @ w_down[expert(row)].T over the plan's rows (bf16; eo fp32); xg, mid: scratch."""
     n_real, D, F = w_down.shape
-    assert all(t.is_cuda for t in (x, w_up, w_down, xg, mid, eo))
+    assert x.is_cuda and w_up.is_cuda and w_down.is_cuda and xg.is_cuda and mid.is_cuda and eo.is_cuda
     assert x.dtype == w_up.dtype == w_down.dtype == xg.dtype == mid.dtype == torch.bfloat16 and eo.dtype == torch.float32 and x.stride(1) == 1
     assert all(t.is_contiguous() for t in (w_up, w_down, xg, mid, eo)) and x.shape[1] == D and w_up.shape == (n_real, 2 * F if act == ACT_SILU_GLU else F, D)
     assert xg.shape == (plan.pairs, D) and mid.shape == (plan.pairs, F) and eo.shape == (plan.pairs, D)
