@@ -198,10 +198,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   auto stamp = [&](int role, int j, int ev) {
     if (tr_on && j < 32) p.trace[(role * 32 + j) * 8 + ev] = clock64();
   };
-  // ragged batches: keys [key_lens[b], keys) of problem b exist in memory (padding tokens, finite values) but weigh nothing
-  const int n_keys = p.key_lens ? max(1, min(p.keys, __ldg(p.key_lens + b))) : p.keys;
-  const int n_tiles = (n_keys + BN - 1) / BN;
-
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmQ);
     tma_prefetch_desc(&tmK);
@@ -227,6 +223,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_gen;
+  griddep_wait();
+  griddep_launch_dependents();  // (tensor memory is held by now: a product behind this kernel cannot take it first)
+  // ragged batches: keys [key_lens[b], keys) of problem b exist in memory (padding tokens, finite values) but weigh nothing
+  const int n_keys = p.key_lens ? max(1, min(p.keys, __ldg(p.key_lens + b))) : p.keys;
+  const int n_tiles = (n_keys + BN - 1) / BN;
 
   if (warp == 0) {
     // ============================== TMA producer ==============================
@@ -537,9 +538,7 @@ static int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
     configured[dev] = true;
   }
   dim3 grid((p.rows + C::BM * QT - 1) / (C::BM * QT), H, B);
-  attn_prefill_tc_kernel<DH, SW, QT><<<grid, 96 + 128 * SW * QT, C::SMEM, st>>>(tq, tk, tv, p);
-  pg_count_launch(1);
-  return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
+  return launch_kernel(attn_prefill_tc_kernel<DH, SW, QT>, grid, dim3(96 + 128 * SW * QT), C::SMEM, st, tq, tk, tv, p) == cudaSuccess ? PG_OK : PG_ERR_CUDA;
 }
 
 }  // namespace ap

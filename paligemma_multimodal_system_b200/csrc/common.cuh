@@ -142,6 +142,13 @@ PG_DEVINL void prefetch_l2_bulk_hint(const void* ptr, uint32_t bytes, uint64_t h
 // PDL (programmatic dependent launch)
 PG_DEVINL void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 PG_DEVINL void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// First statement of the kernels that are a link of a chain (norms, mixers, routing): lets the next kernel become resident -- a product then requests its
+// first weight tiles, the only thing any kernel here touches ahead of its own wait -- and waits for the kernel before.  Triggering ahead of the wait is safe
+// because every link waits: the next one passes its wait when this kernel has completed, and this one completes after all before it.
+PG_DEVINL void griddep_begin() {
+  griddep_launch_dependents();
+  griddep_wait();
+}
 
 // ---------------------------------------------------------------------------------------------
 // tcgen05 / TMEM
@@ -306,10 +313,10 @@ inline int num_sms() {
   return sms[dev];
 }
 
-// Host-side launch through cudaLaunchKernelEx, optionally as a programmatic dependent launch.  Every kernel launched
-// this way executes griddepcontrol.wait before its first dependent global access.
+// Host-side launch through cudaLaunchKernelEx, as a programmatic dependent launch unless that is switched off (the caller counts it).  Every kernel launched this
+// way executes griddepcontrol.wait before its first dependent global access.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -320,8 +327,14 @@ inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pg_pdl_enabled() ? 1 : 0;
-  pg_count_launch(1);
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+// The same, counted.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+  pg_count_launch(1);
+  return launch_dependent(kernel, grid, block, smem, st, args...);
 }
 
 }  // namespace pg

@@ -35,6 +35,7 @@ PG_DEVINL float block_sum(float v, float* red) {
 __global__ void __launch_bounds__(256) layernorm_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
                                                         const float* __restrict__ beta, bf16* __restrict__ y_bf,
                                                         float* __restrict__ y_f, int D, float eps) {
+  pg::griddep_begin();
   extern __shared__ float row[];  // D floats + 33
   float* red = row + D;
   const long long r = blockIdx.x;
@@ -99,6 +100,7 @@ template <int NV>
 __global__ void __launch_bounds__(256) layernorm_warp_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
                                                              const float* __restrict__ beta, bf16* __restrict__ y_bf,
                                                              float* __restrict__ y_f, int rows, int D, float eps) {
+  pg::griddep_begin();
   const int lane = threadIdx.x & 31;
   const long long r = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (r >= rows) return;
@@ -139,6 +141,7 @@ __global__ void __launch_bounds__(256) layernorm_warp_kernel(const float* __rest
 template <int NV>
 __global__ void __launch_bounds__(256) rmsnorm_warp_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                            bf16* __restrict__ y, int rows, int D, float eps) {
+  pg::griddep_begin();
   const int lane = threadIdx.x & 31;
   const long long r = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (r >= rows) return;
@@ -170,6 +173,7 @@ __global__ void __launch_bounds__(256) rmsnorm_warp_kernel(const float* __restri
 // ---------------------------------------------------------------------------------------------------------
 __global__ void im2col_kernel(const float* __restrict__ px, bf16* __restrict__ out, int C, int H, int W, int P, int Kpad,
                               long long total) {
+  pg::griddep_begin();
   const long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   if (idx >= total) return;
   const int col = static_cast<int>(idx % Kpad);
@@ -218,6 +222,7 @@ __global__ void __launch_bounds__(1024) merge_scan_kernel(const long long* __res
                                                           int* __restrict__ src, int* __restrict__ pos, int* __restrict__ err,
                                                           int* __restrict__ dst_row, int S, int N, long long image_token,
                                                           long long pad_token) {
+  pg::griddep_begin();
   __shared__ int wsum_img[32], wsum_msk[32];
   __shared__ int carry_img, carry_msk;
   const int b = blockIdx.x;
@@ -259,6 +264,7 @@ __global__ void __launch_bounds__(256) merge_gather_kernel(const long long* __re
                                                            const bf16* __restrict__ embed, const float* __restrict__ img,
                                                            float* __restrict__ h, int S, int D, int N, float text_scale,
                                                            float img_scale, int skip_image) {
+  pg::griddep_begin();
   const long long tok = blockIdx.x;
   const int b = static_cast<int>(tok / S);
   const int sidx = src[tok];
@@ -325,6 +331,7 @@ __global__ void __launch_bounds__(128) rope_kv_append_kernel(const void* __restr
                                                              const int* __restrict__ slot_base, int tokens_per_seq, int Hq,
                                                              int Hkv, int dh, int page_size, int max_pages,
                                                              const float* __restrict__ inv_freq) {
+  pg::griddep_begin();
   const long long t = blockIdx.x;
   const int b = static_cast<int>(t / tokens_per_seq);
   const int half = dh / 2;
@@ -450,10 +457,10 @@ extern "C" int pg_layernorm(const float* x, const float* gamma, const float* bet
   const bool al = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(beta) |
                     reinterpret_cast<uintptr_t>(y_bf16) | reinterpret_cast<uintptr_t>(y_f32)) & 15) == 0;
   if (rows >= 1024 && (D % 128) == 0 && D <= 2048 && al) {  // prefill: one warp per row, the row stays in registers
-    layernorm_warp_kernel<16><<<(rows + 7) / 8, 256, 0, PG_ST(stream)>>>(x, gamma, beta, static_cast<bf16*>(y_bf16), y_f32, rows, D, eps);
+    pg::launch_dependent(layernorm_warp_kernel<16>, (rows + 7) / 8, 256, 0, PG_ST(stream), x, gamma, beta, static_cast<bf16*>(y_bf16), y_f32, rows, D, eps);
     PG_RET();
   }
-  layernorm_kernel<<<rows, 256, (D + 33) * sizeof(float), PG_ST(stream)>>>(x, gamma, beta, static_cast<bf16*>(y_bf16), y_f32, D, eps);
+  pg::launch_dependent(layernorm_kernel, rows, 256, (D + 33) * sizeof(float), PG_ST(stream), x, gamma, beta, static_cast<bf16*>(y_bf16), y_f32, D, eps);
   PG_RET();
 }
 
@@ -464,7 +471,7 @@ extern "C" int pg_rmsnorm(const float* x, const float* w, void* y_bf16, int rows
   if (rows <= 0 || D <= 0 || (D % 4) != 0 || D > 8192) return PG_ERR_ARG;
   if (rows >= 1024 && (D % 128) == 0 && D <= 2048 &&
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y_bf16)) & 15) == 0) {
-    rmsnorm_warp_kernel<16><<<(rows + 7) / 8, 256, 0, PG_ST(stream)>>>(x, w, static_cast<bf16*>(y_bf16), rows, D, eps);
+    pg::launch_dependent(rmsnorm_warp_kernel<16>, (rows + 7) / 8, 256, 0, PG_ST(stream), x, w, static_cast<bf16*>(y_bf16), rows, D, eps);
     PG_RET();
   }
   return launch_kernel(rmsnorm_kernel, dim3(rows), dim3(256), (D + 33) * sizeof(float), PG_ST(stream), x, w,
@@ -474,7 +481,7 @@ extern "C" int pg_rmsnorm(const float* x, const float* w, void* y_bf16, int rows
 extern "C" int pg_im2col(const float* pixels, void* patches, int B, int C, int H, int W, int P, int Kpad, void* stream) {
   if (B <= 0 || P <= 0 || H % P || W % P || Kpad < C * P * P || (Kpad % 8)) return PG_ERR_ARG;
   const long long total = static_cast<long long>(B) * (H / P) * (W / P) * Kpad;
-  im2col_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, PG_ST(stream)>>>(pixels, static_cast<bf16*>(patches), C, H, W, P, Kpad, total);
+  pg::launch_dependent(im2col_kernel, static_cast<unsigned>((total + 255) / 256), 256, 0, PG_ST(stream), pixels, static_cast<bf16*>(patches), C, H, W, P, Kpad, total);
   PG_RET();
 }
 
@@ -498,10 +505,10 @@ extern "C" int pg_merge_embeddings(const long long* input_ids, const long long* 
                                    long long image_token, long long pad_token, float text_scale, float img_scale,
                                    void* stream) {
   if (B <= 0 || S <= 0 || D <= 0 || (D % 4)) return PG_ERR_ARG;
-  merge_scan_kernel<<<B, 1024, 0, PG_ST(stream)>>>(input_ids, attn_mask, src_scratch, pos, err_flag, nullptr, S, N, image_token, pad_token);
+  pg::launch_dependent(merge_scan_kernel, B, 1024, 0, PG_ST(stream), input_ids, attn_mask, src_scratch, pos, err_flag, nullptr, S, N, image_token, pad_token);
   if (cudaGetLastError() != cudaSuccess) return PG_ERR_CUDA;
   pg_count_launch(1);
-  merge_gather_kernel<<<B * S, 256, 0, PG_ST(stream)>>>(input_ids, src_scratch, static_cast<const bf16*>(embed), img, h, S, D, N,
+  pg::launch_dependent(merge_gather_kernel, B * S, 256, 0, PG_ST(stream), input_ids, src_scratch, static_cast<const bf16*>(embed), img, h, S, D, N,
                                                         text_scale, img_scale, 0);
   PG_RET();
 }
@@ -509,14 +516,14 @@ extern "C" int pg_merge_embeddings(const long long* input_ids, const long long* 
 extern "C" int pg_merge_scan(const long long* input_ids, const long long* attn_mask, int* pos, int* src_scratch, int* dst_row,
                              int* err_flag, int B, int S, int N, long long image_token, long long pad_token, void* stream) {
   if (B <= 0 || S <= 0 || N < 0 || !input_ids || !attn_mask || !pos || !src_scratch || !err_flag) return PG_ERR_ARG;
-  merge_scan_kernel<<<B, 1024, 0, PG_ST(stream)>>>(input_ids, attn_mask, src_scratch, pos, err_flag, dst_row, S, N, image_token, pad_token);
+  pg::launch_dependent(merge_scan_kernel, B, 1024, 0, PG_ST(stream), input_ids, attn_mask, src_scratch, pos, err_flag, dst_row, S, N, image_token, pad_token);
   PG_RET();
 }
 
 extern "C" int pg_merge_text(const long long* input_ids, const int* src_scratch, const void* embed, float* h, int B, int S, int D,
                              int N, float text_scale, void* stream) {
   if (B <= 0 || S <= 0 || D <= 0 || (D % 4) || !input_ids || !src_scratch || !embed || !h) return PG_ERR_ARG;
-  merge_gather_kernel<<<B * S, 256, 0, PG_ST(stream)>>>(input_ids, src_scratch, static_cast<const bf16*>(embed), nullptr, h, S, D, N,
+  pg::launch_dependent(merge_gather_kernel, B * S, 256, 0, PG_ST(stream), input_ids, src_scratch, static_cast<const bf16*>(embed), nullptr, h, S, D, N,
                                                         text_scale, 0.f, 1);
   PG_RET();
 }
@@ -535,12 +542,12 @@ extern "C" int pg_rope_kv_append(const void* qkv, int qkv_is_f32, const int* pos
   if (B <= 0 || tokens_per_seq <= 0 || (dh % 2)) return PG_ERR_ARG;
   const int T = B * tokens_per_seq;
   if (qkv_is_f32)
-    rope_kv_append_kernel<true><<<T, 128, 0, PG_ST(stream)>>>(qkv, pos, static_cast<bf16*>(q_out), static_cast<bf16*>(k_out),
+    pg::launch_dependent(rope_kv_append_kernel<true>, T, 128, 0, PG_ST(stream), qkv, pos, static_cast<bf16*>(q_out), static_cast<bf16*>(k_out),
                                                              static_cast<bf16*>(v_out), static_cast<bf16*>(k_pages),
                                                              static_cast<bf16*>(v_pages), page_table, slot_base, tokens_per_seq,
                                                              Hq, Hkv, dh, page_size, max_pages, inv_freq);
   else
-    rope_kv_append_kernel<false><<<T, 128, 0, PG_ST(stream)>>>(qkv, pos, static_cast<bf16*>(q_out), static_cast<bf16*>(k_out),
+    pg::launch_dependent(rope_kv_append_kernel<false>, T, 128, 0, PG_ST(stream), qkv, pos, static_cast<bf16*>(q_out), static_cast<bf16*>(k_out),
                                                               static_cast<bf16*>(v_out), static_cast<bf16*>(k_pages),
                                                               static_cast<bf16*>(v_pages), page_table, slot_base, tokens_per_seq,
                                                               Hq, Hkv, dh, page_size, max_pages, inv_freq);

@@ -87,6 +87,7 @@ __global__ void __launch_bounds__(128, (DIM + VDIM <= 128) ? 4 : 2) attn_ragged_
                                                               const int* __restrict__ entry_ctx, const int* __restrict__ page_table, int max_pages,
                                                               int page, int H, int G, float scale, float softcap, int skip_single, int gate_per_head,
                                                               PgAttnScore sx) {
+  pg::griddep_begin();
   constexpr int KS = DIM / 16, NV = VDIM / 8, QP = DIM + 8, VLD = VDIM + 8;
   static_assert(VDIM % 16 == 0, "value blocks are fetched in pairs");
   const int e = blockIdx.z, g = blockIdx.y, gsz = H / G;
@@ -383,6 +384,7 @@ __global__ void __launch_bounds__(128) attn_latent_decode_mma_kernel(const bf16*
                                                                      float* __restrict__ partial, const int* __restrict__ entry_row0,
                                                                      const int* __restrict__ entry_n, const int* __restrict__ entry_ctx,
                                                                      const int* __restrict__ page_table, int max_pages, int page, int H, float scale, int window) {
+  pg::griddep_begin();
   constexpr int VPART = VDIM / VS, KS = DIM / 16, NV = VPART / 8, LD = DIM + 8;
   static_assert(DIM % 16 == 0 && VDIM % VS == 0 && VPART % 16 == 0 && VDIM <= DIM && (KT == 32 || KT == 64), "tile shapes");
   constexpr int NB = KT / 8;  // 8-key blocks per tile
@@ -534,7 +536,7 @@ int launch_latent_kt(const void* q, const void* pages, const void* gate, long lo
   const size_t smem = ((size_t)(16 * warps + 2 * KT) * (DIM + 8)) * sizeof(bf16);
   auto kern = attn_latent_decode_mma_kernel<DIM, VDIM, KT, VS>;
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return PG_ERR_CUDA;
-  kern<<<dim3(nsplit, ((H + 63) / 64) * VS, entries), 32 * warps, smem, st>>>(static_cast<const bf16*>(q), static_cast<const bf16*>(pages), static_cast<const bf16*>(gate),
+  pg::launch_dependent(kern, dim3(nsplit, ((H + 63) / 64) * VS, entries), 32 * warps, smem, st, static_cast<const bf16*>(q), static_cast<const bf16*>(pages), static_cast<const bf16*>(gate),
                                                                       ldg, static_cast<bf16*>(out), partial, row0, n, ctx, pt, max_pages, page, H, scale, window);
   pg_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
@@ -560,7 +562,7 @@ int launch(const void* q, const void* kp, const void* vp, const void* gate, long
   auto kern = sx.logistic ? attn_ragged_mma_kernel<DIM, VDIM, true> : attn_ragged_mma_kernel<DIM, VDIM, false>;
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return PG_ERR_CUDA;
   dim3 grid((max_n * (H / G) + 63) / 64, G, entries);
-  kern<<<grid, 128, smem, st>>>(static_cast<const bf16*>(q), static_cast<const bf16*>(kp), static_cast<const bf16*>(vp), static_cast<const bf16*>(gate), ldg,
+  pg::launch_dependent(kern, grid, 128, smem, st, static_cast<const bf16*>(q), static_cast<const bf16*>(kp), static_cast<const bf16*>(vp), static_cast<const bf16*>(gate), ldg,
                                 static_cast<bf16*>(out), row0, n, ctx, pt, max_pages, page, H, G, scale, softcap, skip_single, gate_per_head, sx);
   pg_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;

@@ -64,6 +64,7 @@ __global__ void __launch_bounds__(256) rmsnorm_conv_kernel(const float* __restri
                                                            const int* __restrict__ entry_row0, const int* __restrict__ entry_n,
                                                            const int* __restrict__ entry_ctx, const int* __restrict__ entry_slot, int D, float eps,
                                                            int by_entry) {
+  pg::griddep_begin();
   __shared__ float red[8];
   __shared__ float inv[2 * MAX_K + 1];
   const int K = cw != nullptr ? taps - 1 : 0;
@@ -183,6 +184,7 @@ __global__ void __launch_bounds__(256) rmsnorm_conv_vec_kernel(const float* __re
                                                                const int* __restrict__ entry_row0, const int* __restrict__ entry_n,
                                                                const int* __restrict__ entry_ctx, const int* __restrict__ entry_slot, int D, float eps,
                                                                int by_entry) {
+  pg::griddep_begin();
   __shared__ float red[8];
   __shared__ float inv[2 * MAX_K + 1];
   const int K = cw != nullptr ? taps - 1 : 0;
@@ -286,6 +288,7 @@ __global__ void __launch_bounds__(256) rmsnorm_conv_rows_kernel(const float* __r
                                                                 const float* __restrict__ cw, int taps, TO* __restrict__ out_h,
                                                                 TO* __restrict__ out_conv, const int* __restrict__ row_entry,
                                                                 const int* __restrict__ entry_row0, int rows, int RC, int D, float eps) {
+  pg::griddep_begin();
   __shared__ float inv[32 + MAX_K];
   __shared__ int into[32];  // rows into their entry
   const int K = taps - 1;
@@ -330,6 +333,7 @@ __global__ void __launch_bounds__(256) rmsnorm_conv_rows_kernel(const float* __r
 template <typename TA>
 __global__ void __launch_bounds__(256) polynorm_kernel(const TA* z, long long ldz, const float* __restrict__ coef, TA* out,
                                                        long long ldo, int F, float eps) {
+  pg::griddep_begin();
   __shared__ float red[8];
   const long long t = blockIdx.x;
   const TA* zr = z + t * ldz;
@@ -373,6 +377,7 @@ __device__ __forceinline__ void st8(bf16* p, const float* v) {
 template <typename TA>
 __global__ void __launch_bounds__(256) polynorm_vec_kernel(const TA* z, long long ldz, const float* __restrict__ coef, TA* out, long long ldo, int F,
                                                            float eps) {
+  pg::griddep_begin();
   __shared__ float red[8];
   const long long t = blockIdx.x;
   const TA* zr = z + t * ldz;
@@ -404,6 +409,7 @@ __global__ void __launch_bounds__(256) polynorm_vec_kernel(const TA* z, long lon
 
 template <typename TA>
 __global__ void sigmoid_gate_mul_kernel(TA* __restrict__ y, long long ldy, const TA* __restrict__ gate, long long ldg, int n, long long total) {
+  pg::griddep_begin();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const long long t = i / n;
     const int c = (int)(i % n);
@@ -431,12 +437,12 @@ extern "C" int pg_rmsnorm_conv(const float* x, const float* w, int w_scalar, con
   if (conv_w != nullptr && taps > 1 && entries > 0 && RC >= 2 && D % 4 == 0 && al16(x) && (w_scalar || al16(w)) && al16(conv_w) && al16(state) && al16(out_h) && al16(out_conv)) {
     const int chunks = (rows + RC - 1) / RC;
     if (out_f32) {
-      rmsnorm_conv_rows_kernel<float><<<chunks, 256, 0, st>>>(x, w, ws, conv_w, taps, static_cast<float*>(out_h), static_cast<float*>(out_conv), row_entry, entry_row0, rows, RC, D, eps);
-      rmsnorm_conv_vec_kernel<float><<<entries, 256, 0, st>>>(x, w, ws, conv_w, taps, state, static_cast<float*>(out_h), static_cast<float*>(out_conv), row_entry,
+      pg::launch_dependent(rmsnorm_conv_rows_kernel<float>, chunks, 256, 0, st, x, w, ws, conv_w, taps, static_cast<float*>(out_h), static_cast<float*>(out_conv), row_entry, entry_row0, rows, RC, D, eps);
+      pg::launch_dependent(rmsnorm_conv_vec_kernel<float>, entries, 256, 0, st, x, w, ws, conv_w, taps, state, static_cast<float*>(out_h), static_cast<float*>(out_conv), row_entry,
                                                               entry_row0, entry_n, entry_ctx, entry_slot, D, eps, 1);
     } else {
-      rmsnorm_conv_rows_kernel<bf16><<<chunks, 256, 0, st>>>(x, w, ws, conv_w, taps, static_cast<bf16*>(out_h), static_cast<bf16*>(out_conv), row_entry, entry_row0, rows, RC, D, eps);
-      rmsnorm_conv_vec_kernel<bf16><<<entries, 256, 0, st>>>(x, w, ws, conv_w, taps, state, static_cast<bf16*>(out_h), static_cast<bf16*>(out_conv), row_entry,
+      pg::launch_dependent(rmsnorm_conv_rows_kernel<bf16>, chunks, 256, 0, st, x, w, ws, conv_w, taps, static_cast<bf16*>(out_h), static_cast<bf16*>(out_conv), row_entry, entry_row0, rows, RC, D, eps);
+      pg::launch_dependent(rmsnorm_conv_vec_kernel<bf16>, entries, 256, 0, st, x, w, ws, conv_w, taps, state, static_cast<bf16*>(out_h), static_cast<bf16*>(out_conv), row_entry,
                                                              entry_row0, entry_n, entry_ctx, entry_slot, D, eps, 1);
     }
     pg_count_launch(1);
@@ -444,7 +450,7 @@ extern "C" int pg_rmsnorm_conv(const float* x, const float* w, int w_scalar, con
   }
   const bool vec = D % 4 == 0 && al16(x) && (w_scalar || al16(w)) && al16(conv_w) && al16(state) && al16(out_h) && al16(out_conv);
 #define PG_RC(KERN, TO, GRID, BY)                                                                                                                     \
-  KERN<TO><<<GRID, 256, 0, st>>>(x, w, ws, conv_w, taps, state, static_cast<TO*>(out_h), static_cast<TO*>(out_conv), row_entry, entry_row0, entry_n, \
+  pg::launch_dependent(KERN<TO>, GRID, 256, 0, st, x, w, ws, conv_w, taps, state, static_cast<TO*>(out_h), static_cast<TO*>(out_conv), row_entry, entry_row0, entry_n, \
                                  entry_ctx, entry_slot, D, eps, BY)
   if (vec) {
     if (out_f32) PG_RC(rmsnorm_conv_vec_kernel, float, rows, 0);
@@ -461,15 +467,15 @@ extern "C" int pg_polynorm(const void* z, long long ldz, const float* coef, void
   if (rows <= 0 || F <= 0 || z == nullptr || coef == nullptr || out == nullptr) return PG_ERR_ARG;
   if (F % 8 == 0 && ldz % 8 == 0 && ldo % 8 == 0 && ((reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
     if (act_f32)
-      polynorm_vec_kernel<float><<<rows, 256, 0, PG_ST(stream)>>>(static_cast<const float*>(z), ldz, coef, static_cast<float*>(out), ldo, F, eps);
+      pg::launch_dependent(polynorm_vec_kernel<float>, rows, 256, 0, PG_ST(stream), static_cast<const float*>(z), ldz, coef, static_cast<float*>(out), ldo, F, eps);
     else
-      polynorm_vec_kernel<bf16><<<rows, 256, 0, PG_ST(stream)>>>(static_cast<const bf16*>(z), ldz, coef, static_cast<bf16*>(out), ldo, F, eps);
+      pg::launch_dependent(polynorm_vec_kernel<bf16>, rows, 256, 0, PG_ST(stream), static_cast<const bf16*>(z), ldz, coef, static_cast<bf16*>(out), ldo, F, eps);
     PG_RET();
   }
   if (act_f32)
-    polynorm_kernel<float><<<rows, 256, 0, PG_ST(stream)>>>(static_cast<const float*>(z), ldz, coef, static_cast<float*>(out), ldo, F, eps);
+    pg::launch_dependent(polynorm_kernel<float>, rows, 256, 0, PG_ST(stream), static_cast<const float*>(z), ldz, coef, static_cast<float*>(out), ldo, F, eps);
   else
-    polynorm_kernel<bf16><<<rows, 256, 0, PG_ST(stream)>>>(static_cast<const bf16*>(z), ldz, coef, static_cast<bf16*>(out), ldo, F, eps);
+    pg::launch_dependent(polynorm_kernel<bf16>, rows, 256, 0, PG_ST(stream), static_cast<const bf16*>(z), ldz, coef, static_cast<bf16*>(out), ldo, F, eps);
   PG_RET();
 }
 
@@ -478,8 +484,8 @@ extern "C" int pg_sigmoid_gate_mul(void* y, long long ldy, const void* gate, lon
   const long long total = (long long)rows * n;
   const int blocks = (int)((total + 255) / 256 < 8 * 148 ? (total + 255) / 256 : 8 * 148);
   if (act_f32)
-    sigmoid_gate_mul_kernel<float><<<blocks, 256, 0, PG_ST(stream)>>>(static_cast<float*>(y), ldy, static_cast<const float*>(gate), ldg, n, total);
+    pg::launch_dependent(sigmoid_gate_mul_kernel<float>, blocks, 256, 0, PG_ST(stream), static_cast<float*>(y), ldy, static_cast<const float*>(gate), ldg, n, total);
   else
-    sigmoid_gate_mul_kernel<bf16><<<blocks, 256, 0, PG_ST(stream)>>>(static_cast<bf16*>(y), ldy, static_cast<const bf16*>(gate), ldg, n, total);
+    pg::launch_dependent(sigmoid_gate_mul_kernel<bf16>, blocks, 256, 0, PG_ST(stream), static_cast<bf16*>(y), ldy, static_cast<const bf16*>(gate), ldg, n, total);
   PG_RET();
 }

@@ -108,6 +108,7 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const TI* __restrict__ x
 template <typename TI>
 __global__ void embed_rows_kernel(const int* __restrict__ tokens, const TI* __restrict__ table, long long ld, int col0, float* __restrict__ out,
                                   TI* __restrict__ out_act, int D, float scale) {
+  pg::griddep_begin();
   const int t = blockIdx.x;
   const long long row = tokens[t];
   for (int d = threadIdx.x; d < D; d += blockDim.x) {
@@ -133,6 +134,7 @@ __device__ __forceinline__ void st_act4(bf16* p, long long i, float4 v) {
 template <typename TO, bool VEC>
 __global__ void __launch_bounds__(256) group_rmsnorm_add_kernel(const float* __restrict__ y, long long ldy, const float* __restrict__ w,
                                                                 float* __restrict__ x, TO* __restrict__ out_act, int D, int groups, float eps) {
+  pg::griddep_begin();
   extern __shared__ float sm[];  // 8 partial sums, then 1 / rms of every group
   float* red = sm;
   float* inv = sm + 8;
@@ -202,6 +204,7 @@ __device__ __forceinline__ float4 ld_act4(const bf16* p, long long i) {
 template <typename TA, bool VEC>
 __global__ void __launch_bounds__(256) rmsnorm_gate_kernel(const float* __restrict__ o, const float* __restrict__ w, const TA* __restrict__ gate,
                                                            long long ldg, TA* __restrict__ out, int D, float eps) {
+  pg::griddep_begin();
   __shared__ float red[32];
   const long long t = blockIdx.x;
   float s = 0.f;
@@ -232,6 +235,7 @@ __global__ void __launch_bounds__(256) rmsnorm_gate_kernel(const float* __restri
 // out[t, f] = gelu_tanh(gu[t, f]) * gu[t, F + f]    (unfused gate || up product: the exact-precision path)
 template <typename TA>
 __global__ void geglu_kernel(const TA* __restrict__ gu, long long ldgu, TA* __restrict__ out, long long ldo, int F, long long total) {
+  pg::griddep_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const long long t = i / F;
@@ -242,6 +246,7 @@ __global__ void geglu_kernel(const TA* __restrict__ gu, long long ldgu, TA* __re
 // x[t, f] <- relu(x[t, f])^2 in place (the unfused activation of the exact-precision path)
 template <typename TA>
 __global__ void relu2_kernel(TA* __restrict__ x, long long ld, int F, long long total) {
+  pg::griddep_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const long long t = i / F;
@@ -254,6 +259,7 @@ __global__ void relu2_kernel(TA* __restrict__ x, long long ld, int F, long long 
 template <typename TA>
 __global__ void side_gate_kernel(const float* __restrict__ z, long long ldz, const int* __restrict__ tokens, const TA* __restrict__ table, long long ldt,
                                  int col0, TA* __restrict__ out, long long ldo, int n, int n_pad, long long total) {
+  pg::griddep_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const long long t = i / n_pad;
@@ -322,9 +328,9 @@ extern "C" int pg_embed_rows(const int* tokens, const void* table, long long ld,
                              int table_f32, void* stream) {
   if (rows <= 0 || D <= 0) return PG_ERR_ARG;
   if (table_f32)
-    embed_rows_kernel<float><<<rows, 128, 0, PG_ST(stream)>>>(tokens, static_cast<const float*>(table), ld, col0, out, static_cast<float*>(out_act), D, scale);
+    pg::launch_dependent(embed_rows_kernel<float>, rows, 128, 0, PG_ST(stream), tokens, static_cast<const float*>(table), ld, col0, out, static_cast<float*>(out_act), D, scale);
   else
-    embed_rows_kernel<bf16><<<rows, 128, 0, PG_ST(stream)>>>(tokens, static_cast<const bf16*>(table), ld, col0, out, static_cast<bf16*>(out_act), D, scale);
+    pg::launch_dependent(embed_rows_kernel<bf16>, rows, 128, 0, PG_ST(stream), tokens, static_cast<const bf16*>(table), ld, col0, out, static_cast<bf16*>(out_act), D, scale);
   PG_RET();
 }
 
@@ -336,11 +342,11 @@ extern "C" int pg_group_rmsnorm_add(const float* y, long long ldy, const float* 
   const bool vec = ((D / groups) % 4 == 0) && (ldy % 4 == 0) &&
                    ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out_act)) & 15) == 0;
   if (out_f32) {
-    if (vec) group_rmsnorm_add_kernel<float, true><<<rows, 256, smem, st>>>(y, ldy, w, x, static_cast<float*>(out_act), D, groups, eps);
-    else group_rmsnorm_add_kernel<float, false><<<rows, 256, smem, st>>>(y, ldy, w, x, static_cast<float*>(out_act), D, groups, eps);
+    if (vec) pg::launch_dependent(group_rmsnorm_add_kernel<float, true>, rows, 256, smem, st, y, ldy, w, x, static_cast<float*>(out_act), D, groups, eps);
+    else pg::launch_dependent(group_rmsnorm_add_kernel<float, false>, rows, 256, smem, st, y, ldy, w, x, static_cast<float*>(out_act), D, groups, eps);
   } else {
-    if (vec) group_rmsnorm_add_kernel<bf16, true><<<rows, 256, smem, st>>>(y, ldy, w, x, static_cast<bf16*>(out_act), D, groups, eps);
-    else group_rmsnorm_add_kernel<bf16, false><<<rows, 256, smem, st>>>(y, ldy, w, x, static_cast<bf16*>(out_act), D, groups, eps);
+    if (vec) pg::launch_dependent(group_rmsnorm_add_kernel<bf16, true>, rows, 256, smem, st, y, ldy, w, x, static_cast<bf16*>(out_act), D, groups, eps);
+    else pg::launch_dependent(group_rmsnorm_add_kernel<bf16, false>, rows, 256, smem, st, y, ldy, w, x, static_cast<bf16*>(out_act), D, groups, eps);
   }
   PG_RET();
 }
@@ -353,11 +359,11 @@ extern "C" int pg_rmsnorm_gate(const float* o, const float* w, const void* gate,
                    ((reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(out)) & act_mask) == 0;
   cudaStream_t st = PG_ST(stream);
   if (act_f32) {
-    if (vec) rmsnorm_gate_kernel<float, true><<<rows, 256, 0, st>>>(o, w, static_cast<const float*>(gate), ldg, static_cast<float*>(out), D, eps);
-    else rmsnorm_gate_kernel<float, false><<<rows, 256, 0, st>>>(o, w, static_cast<const float*>(gate), ldg, static_cast<float*>(out), D, eps);
+    if (vec) pg::launch_dependent(rmsnorm_gate_kernel<float, true>, rows, 256, 0, st, o, w, static_cast<const float*>(gate), ldg, static_cast<float*>(out), D, eps);
+    else pg::launch_dependent(rmsnorm_gate_kernel<float, false>, rows, 256, 0, st, o, w, static_cast<const float*>(gate), ldg, static_cast<float*>(out), D, eps);
   } else {
-    if (vec) rmsnorm_gate_kernel<bf16, true><<<rows, 256, 0, st>>>(o, w, static_cast<const bf16*>(gate), ldg, static_cast<bf16*>(out), D, eps);
-    else rmsnorm_gate_kernel<bf16, false><<<rows, 256, 0, st>>>(o, w, static_cast<const bf16*>(gate), ldg, static_cast<bf16*>(out), D, eps);
+    if (vec) pg::launch_dependent(rmsnorm_gate_kernel<bf16, true>, rows, 256, 0, st, o, w, static_cast<const bf16*>(gate), ldg, static_cast<bf16*>(out), D, eps);
+    else pg::launch_dependent(rmsnorm_gate_kernel<bf16, false>, rows, 256, 0, st, o, w, static_cast<const bf16*>(gate), ldg, static_cast<bf16*>(out), D, eps);
   }
   PG_RET();
 }
@@ -367,9 +373,9 @@ extern "C" int pg_geglu(const void* gu, long long ldgu, void* out, long long ldo
   const long long total = (long long)rows * F;
   const unsigned blocks = (unsigned)((total + 255) / 256);
   if (act_f32)
-    geglu_kernel<float><<<blocks, 256, 0, PG_ST(stream)>>>(static_cast<const float*>(gu), ldgu, static_cast<float*>(out), ldo, F, total);
+    pg::launch_dependent(geglu_kernel<float>, blocks, 256, 0, PG_ST(stream), static_cast<const float*>(gu), ldgu, static_cast<float*>(out), ldo, F, total);
   else
-    geglu_kernel<bf16><<<blocks, 256, 0, PG_ST(stream)>>>(static_cast<const bf16*>(gu), ldgu, static_cast<bf16*>(out), ldo, F, total);
+    pg::launch_dependent(geglu_kernel<bf16>, blocks, 256, 0, PG_ST(stream), static_cast<const bf16*>(gu), ldgu, static_cast<bf16*>(out), ldo, F, total);
   PG_RET();
 }
 
@@ -377,8 +383,8 @@ extern "C" int pg_relu2(void* x, long long ld, int rows, int F, int act_f32, voi
   if (rows <= 0 || F <= 0) return PG_ERR_ARG;
   const long long total = (long long)rows * F;
   const unsigned blocks = (unsigned)((total + 255) / 256);
-  if (act_f32) relu2_kernel<float><<<blocks, 256, 0, PG_ST(stream)>>>(static_cast<float*>(x), ld, F, total);
-  else relu2_kernel<bf16><<<blocks, 256, 0, PG_ST(stream)>>>(static_cast<bf16*>(x), ld, F, total);
+  if (act_f32) pg::launch_dependent(relu2_kernel<float>, blocks, 256, 0, PG_ST(stream), static_cast<float*>(x), ld, F, total);
+  else pg::launch_dependent(relu2_kernel<bf16>, blocks, 256, 0, PG_ST(stream), static_cast<bf16*>(x), ld, F, total);
   PG_RET();
 }
 
@@ -388,10 +394,10 @@ extern "C" int pg_side_gate(const float* z, long long ldz, const int* tokens, co
   const long long total = (long long)rows * n_pad;
   const unsigned blocks = (unsigned)((total + 255) / 256);
   if (act_f32)
-    side_gate_kernel<float><<<blocks, 256, 0, PG_ST(stream)>>>(z, ldz, tokens, static_cast<const float*>(table), ldt, col0,
+    pg::launch_dependent(side_gate_kernel<float>, blocks, 256, 0, PG_ST(stream), z, ldz, tokens, static_cast<const float*>(table), ldt, col0,
                                                               static_cast<float*>(out), ldo, n, n_pad, total);
   else
-    side_gate_kernel<bf16><<<blocks, 256, 0, PG_ST(stream)>>>(z, ldz, tokens, static_cast<const bf16*>(table), ldt, col0,
+    pg::launch_dependent(side_gate_kernel<bf16>, blocks, 256, 0, PG_ST(stream), z, ldz, tokens, static_cast<const bf16*>(table), ldt, col0,
                                                              static_cast<bf16*>(out), ldo, n, n_pad, total);
   PG_RET();
 }

@@ -58,6 +58,7 @@ __global__ void __launch_bounds__(128) latent_prepare_kernel(const TA* __restric
                                                              int page, const double* __restrict__ freq, const float* __restrict__ qn,
                                                              const float* __restrict__ cn, TA* __restrict__ cq_out, TA* __restrict__ pages,
                                                              int q_rank, int rank, int rot, int rot_dims, float eps, float rot_gain) {
+  pg::griddep_begin();
   __shared__ float red[4];
   const long long t = blockIdx.x;
   const TA* row = proj + t * ld;
@@ -100,6 +101,7 @@ template <typename TA>
 __global__ void rotate_heads_kernel(const TA* __restrict__ src, long long ld_src, long long hs_src, TA* __restrict__ dst, long long ld_dst,
                                     long long hs_dst, const int* __restrict__ pos, const double* __restrict__ freq, int H, int n, int rot_dims,
                                     float rot_gain) {
+  pg::griddep_begin();
   extern __shared__ float cs[];  // cos, sin of the row's rot_dims/2 angles
   const long long t = blockIdx.x;
   const int p = pos[t];
@@ -137,6 +139,7 @@ template <typename TA, bool VEC>
 __global__ void __launch_bounds__(256) latent_gather_kernel(const TA* __restrict__ pages, const int* __restrict__ page_table, int max_pages, int page,
                                                             const int* __restrict__ dense_row0, const int* __restrict__ entry_n,
                                                             const int* __restrict__ entry_ctx, TA* __restrict__ lat, int rank, int width) {
+  pg::griddep_begin();
   constexpr int E = VEC ? 16 / sizeof(TA) : 1;  // elements of a piece
   using P = typename Piece<TA, VEC>::type;
   const int e = blockIdx.y;
@@ -156,6 +159,7 @@ __global__ void __launch_bounds__(256) latent_pack_kv_kernel(const TA* __restric
                                                              const int* __restrict__ page_table, int max_pages, int page, const int* __restrict__ dense_row0,
                                                              const int* __restrict__ entry_n, const int* __restrict__ entry_ctx, TA* __restrict__ k_out,
                                                              TA* __restrict__ v_out, int H, int dim, int rot, int vdim, int rank) {
+  pg::griddep_begin();
   constexpr int E = VEC ? 16 / sizeof(TA) : 1;
   using P = typename Piece<TA, VEC>::type;
   const int e = blockIdx.y;
@@ -195,11 +199,11 @@ extern "C" int pg_latent_prepare(const void* proj, long long ld, const int* pos,
   if (rows <= 0 || q_rank < 0 || rank <= 0 || rot < 0 || rot_dims < 0 || rot_dims > rot || (rot_dims & 1) || page <= 0) return PG_ERR_ARG;
   if (pages == nullptr && q_rank == 0) return PG_ERR_ARG;
   if (act_f32)
-    latent_prepare_kernel<float><<<rows, 128, 0, PG_ST(stream)>>>(static_cast<const float*>(proj), ld, pos, row_entry, page_table, max_pages, page, freq,
+    pg::launch_dependent(latent_prepare_kernel<float>, rows, 128, 0, PG_ST(stream), static_cast<const float*>(proj), ld, pos, row_entry, page_table, max_pages, page, freq,
                                                                  q_norm, c_norm, static_cast<float*>(cq_out), static_cast<float*>(pages), q_rank, rank,
                                                                  rot, rot_dims, eps, rot_gain);
   else
-    latent_prepare_kernel<bf16><<<rows, 128, 0, PG_ST(stream)>>>(static_cast<const bf16*>(proj), ld, pos, row_entry, page_table, max_pages, page, freq,
+    pg::launch_dependent(latent_prepare_kernel<bf16>, rows, 128, 0, PG_ST(stream), static_cast<const bf16*>(proj), ld, pos, row_entry, page_table, max_pages, page, freq,
                                                                 q_norm, c_norm, static_cast<bf16*>(cq_out), static_cast<bf16*>(pages), q_rank, rank,
                                                                 rot, rot_dims, eps, rot_gain);
   PG_RET();
@@ -210,10 +214,10 @@ extern "C" int pg_rotate_heads(const void* src, long long ld_src, long long head
   if (rows <= 0 || H <= 0 || n <= 0 || rot_dims < 0 || rot_dims > n || (rot_dims & 1)) return PG_ERR_ARG;
   const size_t smem = (size_t)(rot_dims + 2) * sizeof(float);
   if (act_f32)
-    rotate_heads_kernel<float><<<rows, 128, smem, PG_ST(stream)>>>(static_cast<const float*>(src), ld_src, head_stride_src, static_cast<float*>(dst),
+    pg::launch_dependent(rotate_heads_kernel<float>, rows, 128, smem, PG_ST(stream), static_cast<const float*>(src), ld_src, head_stride_src, static_cast<float*>(dst),
                                                                   ld_dst, head_stride_dst, pos, freq, H, n, rot_dims, rot_gain);
   else
-    rotate_heads_kernel<bf16><<<rows, 128, smem, PG_ST(stream)>>>(static_cast<const bf16*>(src), ld_src, head_stride_src, static_cast<bf16*>(dst), ld_dst,
+    pg::launch_dependent(rotate_heads_kernel<bf16>, rows, 128, smem, PG_ST(stream), static_cast<const bf16*>(src), ld_src, head_stride_src, static_cast<bf16*>(dst), ld_dst,
                                                                  head_stride_dst, pos, freq, H, n, rot_dims, rot_gain);
   PG_RET();
 }
@@ -225,7 +229,7 @@ extern "C" int pg_latent_gather(const void* pages, const int* page_table, int ma
   const bool vec = whole_pieces(act_f32 ? 4 : 2, {rank, width}, {pages, lat});
   auto go = [&](auto kernel, auto t) {
     using TA = decltype(t);
-    kernel<<<grid, 256, 0, PG_ST(stream)>>>(static_cast<const TA*>(pages), page_table, max_pages, page, dense_row0, entry_n, entry_ctx, static_cast<TA*>(lat),
+    pg::launch_dependent(kernel, grid, 256, 0, PG_ST(stream), static_cast<const TA*>(pages), page_table, max_pages, page, dense_row0, entry_n, entry_ctx, static_cast<TA*>(lat),
                                             rank, width);
   };
   if (act_f32) vec ? go(latent_gather_kernel<float, true>, float()) : go(latent_gather_kernel<float, false>, float());
@@ -241,7 +245,7 @@ extern "C" int pg_latent_pack_kv(const void* up, long long ld_up, const void* pa
   const bool vec = whole_pieces(act_f32 ? 4 : 2, {dim, rot, vdim, rank, ld_up}, {up, pages, k_out, v_out});
   auto go = [&](auto kernel, auto t) {
     using TA = decltype(t);
-    kernel<<<grid, 256, 0, PG_ST(stream)>>>(static_cast<const TA*>(up), ld_up, static_cast<const TA*>(pages), page_table, max_pages, page, dense_row0, entry_n,
+    pg::launch_dependent(kernel, grid, 256, 0, PG_ST(stream), static_cast<const TA*>(up), ld_up, static_cast<const TA*>(pages), page_table, max_pages, page, dense_row0, entry_n,
                                             entry_ctx, static_cast<TA*>(k_out), static_cast<TA*>(v_out), H, dim, rot, vdim, rank);
   };
   if (act_f32) vec ? go(latent_pack_kv_kernel<float, true>, float()) : go(latent_pack_kv_kernel<float, false>, float());

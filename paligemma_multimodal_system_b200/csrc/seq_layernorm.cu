@@ -77,6 +77,7 @@ __global__ void __launch_bounds__(256) layernorm_shift_kernel(const float* __res
                                                               float* __restrict__ state, const int* __restrict__ pos,
                                                               const int* __restrict__ row_entry, const int* __restrict__ entry_row0,
                                                               const int* __restrict__ entry_n, const int* __restrict__ entry_slot, int D, float eps) {
+  pg::griddep_begin();
   extern __shared__ float sm[];
   float* cur = sm;          // [D] this row
   float* oth = sm + D;      // [D] the row before / the entry's last row (only with a shift)
@@ -158,6 +159,7 @@ __global__ void __launch_bounds__(256) layernorm_shift_vec_kernel(const float* _
                                                                   float* __restrict__ state, const int* __restrict__ pos,
                                                                   const int* __restrict__ row_entry, const int* __restrict__ entry_row0,
                                                                   const int* __restrict__ entry_n, const int* __restrict__ entry_slot, int D, float eps) {
+  pg::griddep_begin();
   __shared__ float red[2][8];
   const long long t = blockIdx.x;
   int e = 0, first = 0, n = 1, prev_kind = 0;
@@ -277,6 +279,7 @@ __global__ void __launch_bounds__(256) layernorm_shift_rows_kernel(const float* 
                                                                    const int* __restrict__ row_entry, const int* __restrict__ entry_row0,
                                                                    const int* __restrict__ entry_n, const int* __restrict__ entry_slot, int rows, int R, int D,
                                                                    float eps) {
+  pg::griddep_begin();
   __shared__ float red[8];
   const int t0 = blockIdx.x * R, t1 = min(rows, t0 + R);
   if (t0 >= rows) return;
@@ -337,7 +340,7 @@ template <typename TO, int VT>
 int launch_ln_rows(const float* x, const float* w1, const float* b1, const float* shift, const float* w2, const float* b2, void* out1, void* out2, float* state,
                    const int* pos, const int* row_entry, const int* entry_row0, const int* entry_n, const int* entry_slot, int rows, int R, int D, float eps,
                    cudaStream_t st) {
-  layernorm_shift_rows_kernel<TO, VT><<<(rows + R - 1) / R, 256, 0, st>>>(x, w1, b1, shift, w2, b2, static_cast<TO*>(out1), static_cast<TO*>(out2), state, pos,
+  pg::launch_dependent(layernorm_shift_rows_kernel<TO, VT>, (rows + R - 1) / R, 256, 0, st, x, w1, b1, shift, w2, b2, static_cast<TO*>(out1), static_cast<TO*>(out2), state, pos,
                                                                           row_entry, entry_row0, entry_n, entry_slot, rows, R, D, eps);
   pg_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
@@ -347,7 +350,7 @@ template <typename TO, int VT>
 int launch_ln_vec(const float* x, const float* w1, const float* b1, const float* shift, const float* w2, const float* b2, void* out1, void* out2, float* state,
                   const int* pos, const int* row_entry, const int* entry_row0, const int* entry_n, const int* entry_slot, int rows, int D, float eps,
                   cudaStream_t st) {
-  layernorm_shift_vec_kernel<TO, VT><<<rows, 256, 0, st>>>(x, w1, b1, shift, w2, b2, static_cast<TO*>(out1), static_cast<TO*>(out2), state, pos, row_entry,
+  pg::launch_dependent(layernorm_shift_vec_kernel<TO, VT>, rows, 256, 0, st, x, w1, b1, shift, w2, b2, static_cast<TO*>(out1), static_cast<TO*>(out2), state, pos, row_entry,
                                                            entry_row0, entry_n, entry_slot, D, eps);
   pg_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
@@ -357,6 +360,7 @@ int launch_ln_vec(const float* x, const float* w1, const float* b1, const float*
 template <typename TA>
 __global__ void glu_kernel(const TA* __restrict__ gu, long long ldgu, TA* __restrict__ out, long long ldo, int F, long long total, int kind,
                            float limit, float alpha) {
+  pg::griddep_begin();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const long long t = i / F;
     const int f = (int)(i % F);
@@ -389,6 +393,7 @@ __global__ void __launch_bounds__(256) gated_layernorm_add_vec_kernel(const floa
                                                                       const float* __restrict__ gb, const float* __restrict__ w1,
                                                                       const float* __restrict__ b1, float* __restrict__ x, const float* __restrict__ w2,
                                                                       const float* __restrict__ b2, TA* __restrict__ out, int D, float eps) {
+  pg::griddep_begin();
   __shared__ float red[8];
   const long long t = blockIdx.x;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -435,6 +440,7 @@ __global__ void __launch_bounds__(256) gated_layernorm_add_kernel(const float* _
                                                                   const float* __restrict__ gb, const float* __restrict__ w1, const float* __restrict__ b1,
                                                                   float* __restrict__ x, const float* __restrict__ w2, const float* __restrict__ b2,
                                                                   TA* __restrict__ out, int D, float eps) {
+  pg::griddep_begin();
   extern __shared__ float buf[];  // [D]; every thread re-reads what it wrote
   __shared__ float red[8];
   const long long t = blockIdx.x;
@@ -476,7 +482,7 @@ int launch_gated_ln(const float* y, long long ldy, const void* gate, long long l
   auto al = [](const void* p, size_t n) { return (reinterpret_cast<uintptr_t>(p) & (n - 1)) == 0; };
   if (D % 4 == 0 && D <= 8192 && ldy % 4 == 0 && ldg % 4 == 0 && al(y, 16) && al(gate, 4 * sizeof(TG)) && al(gb, 16) && al(w1, 16) && al(b1, 16) && al(x, 16) &&
       al(w2, 16) && al(b2, 16) && al(out, 4 * sizeof(TA))) {
-#define PG_GLN(VT) gated_layernorm_add_vec_kernel<TA, TG, VT><<<rows, 256, 0, st>>>(y, ldy, g, ldg, gb, w1, b1, x, w2, b2, o, D, eps)
+#define PG_GLN(VT) pg::launch_dependent(gated_layernorm_add_vec_kernel<TA, TG, VT>, rows, 256, 0, st, y, ldy, g, ldg, gb, w1, b1, x, w2, b2, o, D, eps)
     if (D <= 1024) PG_GLN(1);
     else if (D <= 2048) PG_GLN(2);
     else if (D <= 4096) PG_GLN(4);
@@ -488,7 +494,7 @@ int launch_gated_ln(const float* y, long long ldy, const void* gate, long long l
   if (smem > 200 * 1024) return PG_ERR_ARG;
   auto kern = gated_layernorm_add_kernel<TA, TG>;
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return PG_ERR_CUDA;
-  kern<<<rows, 256, smem, st>>>(y, ldy, g, ldg, gb, w1, b1, x, w2, b2, o, D, eps);
+  pg::launch_dependent(kern, rows, 256, smem, st, y, ldy, g, ldg, gb, w1, b1, x, w2, b2, o, D, eps);
   PG_RET();
 }
 
@@ -541,12 +547,12 @@ extern "C" int pg_layernorm_shift(const float* x, const float* w1, const float* 
   if (out_f32) {
     auto kern = layernorm_shift_kernel<float>;
     if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return PG_ERR_CUDA;
-    kern<<<rows, 256, smem, st>>>(x, w1, b1, shift, w2, b2, static_cast<float*>(out1), static_cast<float*>(out2), state, pos, row_entry, entry_row0,
+    pg::launch_dependent(kern, rows, 256, smem, st, x, w1, b1, shift, w2, b2, static_cast<float*>(out1), static_cast<float*>(out2), state, pos, row_entry, entry_row0,
                                   entry_n, entry_slot, D, eps);
   } else {
     auto kern = layernorm_shift_kernel<bf16>;
     if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return PG_ERR_CUDA;
-    kern<<<rows, 256, smem, st>>>(x, w1, b1, shift, w2, b2, static_cast<bf16*>(out1), static_cast<bf16*>(out2), state, pos, row_entry, entry_row0,
+    pg::launch_dependent(kern, rows, 256, smem, st, x, w1, b1, shift, w2, b2, static_cast<bf16*>(out1), static_cast<bf16*>(out2), state, pos, row_entry, entry_row0,
                                   entry_n, entry_slot, D, eps);
   }
   PG_RET();
@@ -558,8 +564,8 @@ extern "C" int pg_glu(const void* gu, long long ldgu, void* out, long long ldo, 
   const long long total = (long long)rows * F;
   const int blocks = (int)((total + 255) / 256 < 65535 ? (total + 255) / 256 : 65535);
   if (act_f32)
-    glu_kernel<float><<<blocks, 256, 0, PG_ST(stream)>>>(static_cast<const float*>(gu), ldgu, static_cast<float*>(out), ldo, F, total, kind, limit, alpha);
+    pg::launch_dependent(glu_kernel<float>, blocks, 256, 0, PG_ST(stream), static_cast<const float*>(gu), ldgu, static_cast<float*>(out), ldo, F, total, kind, limit, alpha);
   else
-    glu_kernel<bf16><<<blocks, 256, 0, PG_ST(stream)>>>(static_cast<const bf16*>(gu), ldgu, static_cast<bf16*>(out), ldo, F, total, kind, limit, alpha);
+    pg::launch_dependent(glu_kernel<bf16>, blocks, 256, 0, PG_ST(stream), static_cast<const bf16*>(gu), ldgu, static_cast<bf16*>(out), ldo, F, total, kind, limit, alpha);
   PG_RET();
 }

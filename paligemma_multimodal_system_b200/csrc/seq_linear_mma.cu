@@ -38,6 +38,7 @@ __global__ void __launch_bounds__(128, 2) linear_attn_block_kernel(const bf16* _
                                                                    const int* __restrict__ entry_row0, const int* __restrict__ entry_n,
                                                                    const int* __restrict__ entry_ctx, const int* __restrict__ entry_slot, int H, int dim,
                                                                    int vdim, PgLinearAttnOps ops) {
+  pg::griddep_begin();
   constexpr int LD = DIM + 8, LV = 64 + 8, LP = C + 8, CH = DIM / 8, NI = C * CH / 128, TILE = C * LD, R = C / 16;
   static_assert(C * CH % 128 == 0, "every thread stages the same number of 8-element pieces");
   const int e = blockIdx.z, h = blockIdx.y;
@@ -258,7 +259,7 @@ int launch_blocks(const bf16* qkv, long long ld, float* state, const float* deca
   const size_t smem = (size_t)(6 * C * (DIM + 8) + 3 * C * (C + 8) + 2 * C * 72) * sizeof(bf16) + (C + 1) * sizeof(float);
   auto kern = linear_attn_block_kernel<DIM, C>;
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return PG_ERR_CUDA;
-  kern<<<dim3((vdim + 63) / 64, H, entries), 128, smem, st>>>(qkv, ld, state, decay, out, row0, n, ctx, slot, H, dim, vdim, ops);
+  pg::launch_dependent(kern, dim3((vdim + 63) / 64, H, entries), 128, smem, st, qkv, ld, state, decay, out, row0, n, ctx, slot, H, dim, vdim, ops);
   pg_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
 }

@@ -64,6 +64,7 @@ __global__ void __launch_bounds__(128) attn_prepare_kernel(const TA* __restrict_
                                                            TA* __restrict__ v_pages, int H, int G, int dim, int vdim, int rot, float eps,
                                                            int norm_qk, int norm_v, int v_from_k, float rot_gain,
                                                            const TA* __restrict__ v_other, long long ldvo, float v_mix) {
+  pg::griddep_begin();
   extern __shared__ float cs[];  // cos[rot/2], sin[rot/2]
   const long long t = blockIdx.x;
   const int p = pos[t];
@@ -173,6 +174,7 @@ __global__ void __launch_bounds__(128) attn_prepare_vec_kernel(const TA* __restr
                                                                TA* __restrict__ v_pages, int rows, int H, int G, int dim, int vdim, int rot, float eps,
                                                                int norm_qk, int norm_v, int v_from_k, float rot_gain, const TA* __restrict__ v_other,
                                                                long long ldvo, float v_mix) {
+  pg::griddep_begin();
   extern __shared__ float cs[];  // [TOK][cos rot/2 | sin rot/2]
   __shared__ float part[2][TOK][4];
   const int t0 = blockIdx.x * TOK, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -286,6 +288,7 @@ __global__ void __launch_bounds__(256) attn_ragged_kernel(const TA* __restrict__
                                                           const int* __restrict__ entry_ctx, const int* __restrict__ page_table, int max_pages,
                                                           int page, int H, int G, int dim, int vdim, float scale, float softcap, int skip_single,
                                                           long long krow, long long vrow, int gate_per_head, int alias, PgAttnScore sx) {
+  pg::griddep_begin();
   const int e = blockIdx.z, g = blockIdx.y, gsz = H / G;
   const int n = entry_n[e], ctx = entry_ctx[e], row0 = entry_row0[e];
   if (skip_single && n == 1) return;
@@ -472,6 +475,7 @@ __global__ void __launch_bounds__(256) attn_decode_kernel(const TA* __restrict__
                                                           const int* __restrict__ entry_ctx, const int* __restrict__ page_table, int max_pages,
                                                           int page, int H, int G, int dim, int vdim, float scale, float softcap, long long krow,
                                                           long long vrow, int gate_per_head, PgAttnScore sx) {
+  pg::griddep_begin();
   constexpr int NO = VEC ? 8 * VC : 2 * VC;  // accumulator columns per lane
   const int e = blockIdx.z, g = blockIdx.y, split = blockIdx.x, nsplit = gridDim.x, gsz = H / G;
   if (entry_n[e] != 1) return;
@@ -681,6 +685,7 @@ template <typename TA>
 __global__ void attn_decode_merge_kernel(const float* __restrict__ partial, const TA* __restrict__ gate, long long ldg, TA* __restrict__ out,
                                          const int* __restrict__ entry_row0, const int* __restrict__ entry_n, int H, int vdim, int nsplit,
                                          int gate_per_head, PgAttnScore sx) {
+  pg::griddep_begin();
   const float* sink = sx.logistic ? nullptr : sx.sink;
   const long long ldo = sx.out_ld > 0 ? sx.out_ld : (long long)H * vdim;
   const float oscale = sx.out_scale != 0.f ? sx.out_scale : 1.f;
@@ -734,6 +739,7 @@ __global__ void __launch_bounds__(256) linear_attn_scan_kernel(const TA* __restr
                                                                const int* __restrict__ entry_row0, const int* __restrict__ entry_n,
                                                                const int* __restrict__ entry_ctx, const int* __restrict__ entry_slot, int H,
                                                                int dim, int vdim, int VB, PgLinearAttnOps ops) {
+  pg::griddep_begin();
   const int e = blockIdx.z, h = blockIdx.y, vb = blockIdx.x;
   const int n = entry_n[e], row0 = entry_row0[e];
   if (n < ops.n_min || n > ops.n_max) return;
@@ -815,6 +821,7 @@ __global__ void __launch_bounds__(256, 2) linear_attn_chunked_kernel(const TA* _
                                                                   const int* __restrict__ entry_row0, const int* __restrict__ entry_n,
                                                                   const int* __restrict__ entry_ctx, const int* __restrict__ entry_slot, int H,
                                                                   int dim, int vdim, PgLinearAttnOps ops) {
+  pg::griddep_begin();
   constexpr int C = 32;
   const int e = blockIdx.z, h = blockIdx.y, vb = blockIdx.x;
   const int n = entry_n[e], row0 = entry_row0[e];
@@ -997,6 +1004,7 @@ __global__ void __launch_bounds__(256, 2) linear_attn_chunked_kernel(const TA* _
 // out[t, 0, i] = gain cos(pos[t] freq[i]), out[t, 1, i] = gain sin(.) for i < rot / 2; 1 and 0 for the other pairs
 __global__ void rotary_table_kernel(const int* __restrict__ pos, const double* __restrict__ freq, float* __restrict__ out, int rot, int pairs, float gain,
                                     long long total) {
+  pg::griddep_begin();
   const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (id >= total) return;
   const long long t = id / pairs;
@@ -1015,7 +1023,7 @@ __global__ void rotary_table_kernel(const int* __restrict__ pos, const double* _
 extern "C" int pg_rotary_table(const int* pos, const double* freq, float* out, int rows, int rot_dims, int pairs, float gain, void* stream) {
   if (rows <= 0 || rot_dims < 0 || (rot_dims & 1) || pairs <= 0 || 2 * pairs < rot_dims) return PG_ERR_ARG;
   const long long total = (long long)rows * pairs;
-  rotary_table_kernel<<<(unsigned)((total + 127) / 128), 128, 0, PG_ST(stream)>>>(pos, freq, out, rot_dims, pairs, gain, total);
+  pg::launch_dependent(rotary_table_kernel, (unsigned)((total + 127) / 128), 128, 0, PG_ST(stream), pos, freq, out, rot_dims, pairs, gain, total);
   PG_RET();
 }
 
@@ -1038,7 +1046,7 @@ extern "C" int pg_attn_prepare(const void* qkv, long long ld, const int* pos, co
   if (!few && lanes(dim) && lanes(vdim) && (vdim == dim || !norm_v) && ld % 8 == 0 && ld_v_other % 8 == 0 && (ptrs & 15) == 0) {
     auto go = [&](auto kernel, auto t, int tok) {
       using TA = decltype(t);
-      kernel<<<(rows + tok - 1) / tok, 128, (size_t)(tok * rot_dims + 2) * sizeof(float), PG_ST(stream)>>>(
+      pg::launch_dependent(kernel, (rows + tok - 1) / tok, 128, (size_t)(tok * rot_dims + 2) * sizeof(float), PG_ST(stream), 
           static_cast<const TA*>(qkv), ld, pos, row_entry, page_table, max_pages, page, freq, q_norm, k_norm, static_cast<TA*>(q_out), static_cast<TA*>(k_pages),
           static_cast<TA*>(v_pages), rows, H, G, dim, vdim, rot_dims, eps, norm_qk, norm_v, v_from_k, rot_gain, static_cast<const TA*>(v_other), ld_v_other, v_mix);
     };
@@ -1049,12 +1057,12 @@ extern "C" int pg_attn_prepare(const void* qkv, long long ld, const int* pos, co
   }
   const size_t smem = (size_t)(rot_dims + 2) * sizeof(float);
   if (act_f32)
-    attn_prepare_kernel<float><<<rows, 128, smem, PG_ST(stream)>>>(static_cast<const float*>(qkv), ld, pos, row_entry, page_table, max_pages, page, freq,
+    pg::launch_dependent(attn_prepare_kernel<float>, rows, 128, smem, PG_ST(stream), static_cast<const float*>(qkv), ld, pos, row_entry, page_table, max_pages, page, freq,
                                                                   q_norm, k_norm, static_cast<float*>(q_out), static_cast<float*>(k_pages),
                                                                   static_cast<float*>(v_pages), H, G, dim, vdim, rot_dims, eps, norm_qk, norm_v, v_from_k, rot_gain,
                                                                   static_cast<const float*>(v_other), ld_v_other, v_mix);
   else
-    attn_prepare_kernel<bf16><<<rows, 128, smem, PG_ST(stream)>>>(static_cast<const bf16*>(qkv), ld, pos, row_entry, page_table, max_pages, page, freq,
+    pg::launch_dependent(attn_prepare_kernel<bf16>, rows, 128, smem, PG_ST(stream), static_cast<const bf16*>(qkv), ld, pos, row_entry, page_table, max_pages, page, freq,
                                                                  q_norm, k_norm, static_cast<bf16*>(q_out), static_cast<bf16*>(k_pages),
                                                                  static_cast<bf16*>(v_pages), H, G, dim, vdim, rot_dims, eps, norm_qk, norm_v, v_from_k, rot_gain,
                                                                  static_cast<const bf16*>(v_other), ld_v_other, v_mix);
@@ -1074,7 +1082,7 @@ static int launch_attn_ragged(const void* q, const void* kp, const void* vp, con
   auto kern = sx.logistic ? attn_ragged_kernel<TA, VC, true> : attn_ragged_kernel<TA, VC, false>;
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return PG_ERR_CUDA;
   dim3 grid((max_n * (H / G) + 31) / 32, G, entries);
-  kern<<<grid, 256, smem, st>>>(static_cast<const TA*>(q), static_cast<const TA*>(kp), static_cast<const TA*>(vp), static_cast<const TA*>(gate), ldg,
+  pg::launch_dependent(kern, grid, 256, smem, st, static_cast<const TA*>(q), static_cast<const TA*>(kp), static_cast<const TA*>(vp), static_cast<const TA*>(gate), ldg,
                                 static_cast<TA*>(out), row0, n, ctx, pt, max_pages, page, H, G, dim, vdim, scale, softcap, skip_single, krow, vrow,
                                 gate_per_head, alias, sx);
   PG_RET();
@@ -1119,7 +1127,7 @@ static int launch_scan(const void* qkv, long long ld, float* state, const float*
   const int nchunk = 256 / VB;
   const size_t smem = ((size_t)2 * dim + (size_t)nchunk * VB) * sizeof(float);
   dim3 grid((vdim + VB - 1) / VB, H, entries);
-  linear_attn_scan_kernel<TA, DCMAX><<<grid, 256, smem, st>>>(static_cast<const TA*>(qkv), ld, state, decay, out, row0, n, ctx, slot, H, dim, vdim, VB, ops);
+  pg::launch_dependent(linear_attn_scan_kernel<TA, DCMAX>, grid, 256, smem, st, static_cast<const TA*>(qkv), ld, state, decay, out, row0, n, ctx, slot, H, dim, vdim, VB, ops);
   PG_RET();
 }
 
@@ -1151,7 +1159,7 @@ static int launch_chunked(const void* qkv, long long ld, float* state, const flo
                           const int* slot, int entries, int H, int dim, int vdim, size_t smem, const PgLinearAttnOps& ops, cudaStream_t st) {
   auto kern = linear_attn_chunked_kernel<TA, VEC, VB>;
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return PG_ERR_CUDA;
-  kern<<<dim3((vdim + VB - 1) / VB, H, entries), 256, smem, st>>>(static_cast<const TA*>(qkv), ld, state, decay, out, row0, n, ctx, slot, H, dim, vdim, ops);
+  pg::launch_dependent(kern, dim3((vdim + VB - 1) / VB, H, entries), 256, smem, st, static_cast<const TA*>(qkv), ld, state, decay, out, row0, n, ctx, slot, H, dim, vdim, ops);
   PG_RET();
 }
 
@@ -1202,12 +1210,12 @@ static int launch_attn_decode(const void* q, const void* kp, const void* vp, con
   if (smem > 200 * 1024) return PG_ERR_ARG;
   auto kern = sx.logistic ? attn_decode_kernel<TA, VC, VEC, true> : attn_decode_kernel<TA, VC, VEC, false>;
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return PG_ERR_CUDA;
-  kern<<<dim3(nsplit, G, entries), 256, smem, st>>>(static_cast<const TA*>(q), static_cast<const TA*>(kp), static_cast<const TA*>(vp),
+  pg::launch_dependent(kern, dim3(nsplit, G, entries), 256, smem, st, static_cast<const TA*>(q), static_cast<const TA*>(kp), static_cast<const TA*>(vp),
                                                      static_cast<const TA*>(gate), ldg, static_cast<TA*>(out), partial, row0, n, ctx, pt, max_pages, page,
                                                      H, G, dim, vdim, scale, softcap, krow, vrow, gate_per_head, sx);
   pg_count_launch(1);
   if (nsplit > 1) {
-    attn_decode_merge_kernel<TA><<<dim3(H, entries), merge_threads(vdim), 0, st>>>(partial, static_cast<const TA*>(gate), ldg, static_cast<TA*>(out), row0, n, H, vdim, nsplit,
+    pg::launch_dependent(attn_decode_merge_kernel<TA>, dim3(H, entries), merge_threads(vdim), 0, st, partial, static_cast<const TA*>(gate), ldg, static_cast<TA*>(out), row0, n, H, vdim, nsplit,
                                                                   gate_per_head, sx);
     pg_count_launch(1);
   }
@@ -1220,10 +1228,10 @@ extern "C" int pg_attn_decode_merge(const float* partial, const void* gate, long
   cudaStream_t st = PG_ST(stream);
   const PgAttnScore sx = score != nullptr ? *score : PgAttnScore{};
   if (act_f32)
-    attn_decode_merge_kernel<float><<<dim3(H, entries), merge_threads(vdim), 0, st>>>(partial, static_cast<const float*>(gate), ldg, static_cast<float*>(out), entry_row0, entry_n,
+    pg::launch_dependent(attn_decode_merge_kernel<float>, dim3(H, entries), merge_threads(vdim), 0, st, partial, static_cast<const float*>(gate), ldg, static_cast<float*>(out), entry_row0, entry_n,
                                                                      H, vdim, nsplit, gate_per_head, sx);
   else
-    attn_decode_merge_kernel<bf16><<<dim3(H, entries), merge_threads(vdim), 0, st>>>(partial, static_cast<const bf16*>(gate), ldg, static_cast<bf16*>(out), entry_row0, entry_n, H,
+    pg::launch_dependent(attn_decode_merge_kernel<bf16>, dim3(H, entries), merge_threads(vdim), 0, st, partial, static_cast<const bf16*>(gate), ldg, static_cast<bf16*>(out), entry_row0, entry_n, H,
                                                                     vdim, nsplit, gate_per_head, sx);
   PG_RET();
 }

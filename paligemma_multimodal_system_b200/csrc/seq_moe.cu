@@ -68,6 +68,7 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict_
                                                         int* __restrict__ ids, float* __restrict__ weights, int* __restrict__ counts, int T,
                                                         int n_all, int n_real, int top, int group_count, int group_keep, float scale,
                                                         const float* __restrict__ logit_bias, int flags) {
+  pg::griddep_begin();
   extern __shared__ float sm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int t = blockIdx.x * 4 + warp;
@@ -168,6 +169,7 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict_
 // One warp: 32 experts at a time, prefix sums of their counts and tile numbers by shuffles.
 __global__ void moe_plan_kernel(const int* __restrict__ counts, int* __restrict__ offsets, int* __restrict__ fill, int* __restrict__ plan, int n_real,
                                 int max_tiles) {
+  pg::griddep_begin();
   const int lane = threadIdx.x;
   int off = 0, nt = 0;
   for (int e0 = 0; e0 < n_real; e0 += 32) {
@@ -200,6 +202,7 @@ __global__ void moe_plan_kernel(const int* __restrict__ counts, int* __restrict_
 
 __global__ void moe_scatter_kernel(const int* __restrict__ ids, const int* __restrict__ offsets, int* __restrict__ fill, int* __restrict__ sorted_pair,
                                    int* __restrict__ pair_row, int pairs, int n_real) {
+  pg::griddep_begin();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= pairs) return;
   const int e = ids[p];
@@ -215,6 +218,7 @@ __global__ void __launch_bounds__(256) moe_gemm_kernel(const TI* __restrict__ x,
                                                        const TI* __restrict__ w, long long expert_stride, long long ldw, TO* __restrict__ out,
                                                        long long ldo, const int* __restrict__ plan, int F, int K, int act, long long x_off,
                                                        long long out_off) {
+  pg::griddep_begin();
   const int tile = blockIdx.y;
   if (tile >= plan[0]) return;
   const int e = plan[4 + 3 * tile], r0 = plan[4 + 3 * tile + 1], nr = plan[4 + 3 * tile + 2];
@@ -305,6 +309,7 @@ __global__ void __launch_bounds__(128) moe_gemm_mma_kernel(const bf16* __restric
                                                            const bf16* __restrict__ w, long long expert_stride, long long ldw, TO* __restrict__ out,
                                                            long long ldo, const int* __restrict__ plan, int F, int K, int act, long long x_off,
                                                            long long out_off) {
+  pg::griddep_begin();
   constexpr int KT = MOE_KT, LD = MOE_LD, ST = MOE_STAGES;
   constexpr int NI = BN / 16;  // 8-feature blocks per warp (two warps side by side)
   const int tile = blockIdx.y;
@@ -419,7 +424,7 @@ static int launch_moe_mma(dim3 grid, cudaStream_t st, const void* x, long long l
   const size_t smem = (size_t)MOE_STAGES * (MOE_TILE + BN) * MOE_LD * sizeof(bf16);
   auto kern = moe_gemm_mma_kernel<TO, BN>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return PG_ERR_CUDA;
-  kern<<<grid, 128, smem, st>>>(static_cast<const bf16*>(x), ldx, sorted_pair, src_div, static_cast<const bf16*>(w), expert_stride, ldw, static_cast<TO*>(out), ldo,
+  pg::launch_dependent(kern, grid, 128, smem, st, static_cast<const bf16*>(x), ldx, sorted_pair, src_div, static_cast<const bf16*>(w), expert_stride, ldw, static_cast<TO*>(out), ldo,
                                 plan, F, K, act, x_off, out_off);
   pg_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
@@ -430,6 +435,7 @@ static int launch_moe_mma(dim3 grid, cudaStream_t st, const void* x, long long l
 template <typename TA>
 __global__ void moe_gather_rows_kernel(const TA* __restrict__ x, long long ldx, const int* __restrict__ sorted_pair, const int* __restrict__ total,
                                        int top, TA* __restrict__ xg, long long ldg, int D) {
+  pg::griddep_begin();
   const int n = *total;
   for (int row = blockIdx.x; row < n; row += gridDim.x) {
     const TA* src = x + (long long)(sorted_pair[row] / top) * ldx;
@@ -443,6 +449,7 @@ __global__ void moe_combine_kernel(const float* __restrict__ expert_out, long lo
                                    const float* __restrict__ weights, const TA* __restrict__ h, long long ldh, const float* __restrict__ shared_out,
                                    long long lds, float* __restrict__ y, int D, int top, const float* __restrict__ shared_gate, long long ldsg,
                                    int accumulate) {
+  pg::griddep_begin();
   const long long t = blockIdx.x;
   const float sgate = shared_gate != nullptr ? 1.0f / (1.0f + expf(-shared_gate[t * ldsg])) : 1.0f;
   for (int d = threadIdx.x; d < D; d += blockDim.x) {
@@ -464,6 +471,7 @@ template <typename TA, bool VEC>
 __global__ void __launch_bounds__(256) moe_combine_norm_add_kernel(const float* __restrict__ expert_out, long long ldy, const int* __restrict__ pair_row,
                                                                    const float* __restrict__ weights, const float* __restrict__ norm_w,
                                                                    float* __restrict__ x, TA* __restrict__ out_act, int D, int top, float eps) {
+  pg::griddep_begin();
   extern __shared__ __align__(16) float comb_y[];  // [D]
   __shared__ float red[8];
   const long long t = blockIdx.x;
@@ -527,7 +535,7 @@ extern "C" int pg_moe_combine_norm_add(const float* expert_out, long long ldy, c
   const bool vec = D % 4 == 0 && ldy % 4 == 0 && ((reinterpret_cast<uintptr_t>(expert_out) | reinterpret_cast<uintptr_t>(norm_w) | reinterpret_cast<uintptr_t>(x) |
                                                    reinterpret_cast<uintptr_t>(out_act)) & 15) == 0;
   const size_t smem = (size_t)D * sizeof(float);
-#define PG_CN(TA, VEC) moe_combine_norm_add_kernel<TA, VEC><<<tokens, 256, smem, st>>>(expert_out, ldy, pair_row, weights, norm_w, x, static_cast<TA*>(out_act), D, top, eps)
+#define PG_CN(TA, VEC) pg::launch_dependent(moe_combine_norm_add_kernel<TA, VEC>, tokens, 256, smem, st, expert_out, ldy, pair_row, weights, norm_w, x, static_cast<TA*>(out_act), D, top, eps)
   if (act_f32) { if (vec) PG_CN(float, true); else PG_CN(float, false); }
   else { if (vec) PG_CN(bf16, true); else PG_CN(bf16, false); }
 #undef PG_CN
@@ -543,7 +551,7 @@ extern "C" int pg_moe_route(const float* logits, long long ld, const float* corr
   if (smem > 48 * 1024) return PG_ERR_ARG;
   cudaStream_t st = PG_ST(stream);
   if (n_real > 0 && cudaMemsetAsync(counts, 0, (size_t)n_real * sizeof(int), st) != cudaSuccess) return PG_ERR_CUDA;
-  moe_route_kernel<<<(tokens + 3) / 4, 128, smem, st>>>(logits, ld, correction, ids, weights, counts, tokens, n_all, n_real, top, group_count, group_keep,
+  pg::launch_dependent(moe_route_kernel, (tokens + 3) / 4, 128, smem, st, logits, ld, correction, ids, weights, counts, tokens, n_all, n_real, top, group_count, group_keep,
                                                         scale, logit_bias, flags);
   PG_RET();
 }
@@ -554,9 +562,9 @@ extern "C" int pg_moe_plan(const int* counts, const int* ids, int* offsets, int*
                            int n_real, int max_tiles, void* stream) {
   if (pairs <= 0 || n_real <= 0 || max_tiles <= 0) return PG_ERR_ARG;
   cudaStream_t st = PG_ST(stream);
-  moe_plan_kernel<<<1, 32, 0, st>>>(counts, offsets, fill, plan, n_real, max_tiles);
+  pg::launch_dependent(moe_plan_kernel, 1, 32, 0, st, counts, offsets, fill, plan, n_real, max_tiles);
   pg_count_launch(1);
-  moe_scatter_kernel<<<(pairs + 255) / 256, 256, 0, st>>>(ids, offsets, fill, sorted_pair, pair_row, pairs, n_real);
+  pg::launch_dependent(moe_scatter_kernel, (pairs + 255) / 256, 256, 0, st, ids, offsets, fill, sorted_pair, pair_row, pairs, n_real);
   PG_RET();
 }
 
@@ -580,13 +588,13 @@ extern "C" int pg_moe_gemm(const void* x, long long ldx, const int* sorted_pair,
 #undef PG_MOE_MMA
   }
   if (in_f32 && out_f32)
-    moe_gemm_kernel<float, float><<<grid, 256, 0, st>>>(static_cast<const float*>(x), ldx, sorted_pair, src_div, static_cast<const float*>(w), expert_stride,
+    pg::launch_dependent(moe_gemm_kernel<float, float>, grid, 256, 0, st, static_cast<const float*>(x), ldx, sorted_pair, src_div, static_cast<const float*>(w), expert_stride,
                                                        ldw, static_cast<float*>(out), ldo, plan, F, K, act, x_expert_off, out_expert_off);
   else if (!in_f32 && out_f32)
-    moe_gemm_kernel<bf16, float><<<grid, 256, 0, st>>>(static_cast<const bf16*>(x), ldx, sorted_pair, src_div, static_cast<const bf16*>(w), expert_stride,
+    pg::launch_dependent(moe_gemm_kernel<bf16, float>, grid, 256, 0, st, static_cast<const bf16*>(x), ldx, sorted_pair, src_div, static_cast<const bf16*>(w), expert_stride,
                                                       ldw, static_cast<float*>(out), ldo, plan, F, K, act, x_expert_off, out_expert_off);
   else if (!in_f32 && !out_f32)
-    moe_gemm_kernel<bf16, bf16><<<grid, 256, 0, st>>>(static_cast<const bf16*>(x), ldx, sorted_pair, src_div, static_cast<const bf16*>(w), expert_stride,
+    pg::launch_dependent(moe_gemm_kernel<bf16, bf16>, grid, 256, 0, st, static_cast<const bf16*>(x), ldx, sorted_pair, src_div, static_cast<const bf16*>(w), expert_stride,
                                                      ldw, static_cast<bf16*>(out), ldo, plan, F, K, act, x_expert_off, out_expert_off);
   else
     return PG_ERR_ARG;
@@ -599,11 +607,11 @@ extern "C" int pg_moe_gather_rows(const void* x, long long ldx, const int* sorte
   const int grid = max_rows < 16384 ? max_rows : 16384;
   const int per = act_f32 ? 4 : 8;  // elements of a 16-byte piece
   if (D % per == 0 && ldx % per == 0 && ldg % per == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(xg)) & 15) == 0)
-    moe_gather_rows_kernel<uint4><<<grid, 128, 0, PG_ST(stream)>>>(static_cast<const uint4*>(x), ldx / per, sorted_pair, total_rows, top, static_cast<uint4*>(xg), ldg / per, D / per);
+    pg::launch_dependent(moe_gather_rows_kernel<uint4>, grid, 128, 0, PG_ST(stream), static_cast<const uint4*>(x), ldx / per, sorted_pair, total_rows, top, static_cast<uint4*>(xg), ldg / per, D / per);
   else if (act_f32)
-    moe_gather_rows_kernel<float><<<grid, 128, 0, PG_ST(stream)>>>(static_cast<const float*>(x), ldx, sorted_pair, total_rows, top, static_cast<float*>(xg), ldg, D);
+    pg::launch_dependent(moe_gather_rows_kernel<float>, grid, 128, 0, PG_ST(stream), static_cast<const float*>(x), ldx, sorted_pair, total_rows, top, static_cast<float*>(xg), ldg, D);
   else
-    moe_gather_rows_kernel<bf16><<<grid, 128, 0, PG_ST(stream)>>>(static_cast<const bf16*>(x), ldx, sorted_pair, total_rows, top, static_cast<bf16*>(xg), ldg, D);
+    pg::launch_dependent(moe_gather_rows_kernel<bf16>, grid, 128, 0, PG_ST(stream), static_cast<const bf16*>(x), ldx, sorted_pair, total_rows, top, static_cast<bf16*>(xg), ldg, D);
   PG_RET();
 }
 
@@ -697,8 +705,8 @@ extern "C" int pg_moe_combine(const float* expert_out, long long ldy, const int*
   if (tokens <= 0 || D <= 0 || top <= 0) return PG_ERR_ARG;
   cudaStream_t st = PG_ST(stream);
   if (act_f32)
-    moe_combine_kernel<float><<<tokens, 256, 0, st>>>(expert_out, ldy, pair_row, ids, weights, static_cast<const float*>(h), ldh, shared_out, lds, y, D, top, shared_gate, ldsg, accumulate);
+    pg::launch_dependent(moe_combine_kernel<float>, tokens, 256, 0, st, expert_out, ldy, pair_row, ids, weights, static_cast<const float*>(h), ldh, shared_out, lds, y, D, top, shared_gate, ldsg, accumulate);
   else
-    moe_combine_kernel<bf16><<<tokens, 256, 0, st>>>(expert_out, ldy, pair_row, ids, weights, static_cast<const bf16*>(h), ldh, shared_out, lds, y, D, top, shared_gate, ldsg, accumulate);
+    pg::launch_dependent(moe_combine_kernel<bf16>, tokens, 256, 0, st, expert_out, ldy, pair_row, ids, weights, static_cast<const bf16*>(h), ldh, shared_out, lds, y, D, top, shared_gate, ldsg, accumulate);
   PG_RET();
 }

@@ -104,6 +104,7 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const TA* __restrict__ 
                                                          long long ldo, float* __restrict__ inv, int ldi, PgConvSections sec, int taps, int C,
                                                          const int* __restrict__ entry_row0, const int* __restrict__ entry_n,
                                                          const int* __restrict__ entry_ctx, const int* __restrict__ entry_slot, int chunk) {
+  pg::griddep_begin();
   const int e = blockIdx.z, lane = threadIdx.x & 31;
   const int n = entry_n[e], r0 = blockIdx.y * chunk;
   if (r0 >= n) return;
@@ -230,6 +231,7 @@ __global__ void __launch_bounds__(128) short_conv_vec_kernel(const bf16* __restr
                                                              long long ldo, float* __restrict__ inv, int ldi, PgConvSections sec, int taps, int C,
                                                              const int* __restrict__ entry_row0, const int* __restrict__ entry_n,
                                                              const int* __restrict__ entry_ctx, const int* __restrict__ entry_slot, int chunk) {
+  pg::griddep_begin();
   constexpr int AHEAD = 4, WC = 32 * V;
   using P = typename Packed<V>::T;
   const int e = blockIdx.z, lane = threadIdx.x & 31;
@@ -337,6 +339,7 @@ __global__ void __launch_bounds__(128) short_conv_vec_kernel(const bf16* __restr
 // ---------------------------------------------------------------------------------------------------------------------
 template <typename TA, int VEC, int RP>
 __global__ void __launch_bounds__(256) delta_scan_kernel(PgDeltaArgs a, int n_min, int n_max) {
+  pg::griddep_begin();
   constexpr int VB = 16 * VEC;
   const int e = blockIdx.z, h = blockIdx.y;
   const int n = a.entry_n[e];
@@ -451,6 +454,7 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(PgDeltaArgs a, int n_mi
 // of value columns (norm_state [slots, blocks, H, dim + 1], m last), so that the CTAs of one head share no slot.
 template <typename TA, int VEC, int RP, int KIND>
 __global__ void __launch_bounds__(256) gated_scan_kernel(PgGatedArgs a, int n_min, int n_max) {
+  pg::griddep_begin();
   constexpr int VB = 16 * VEC;
   const int e = blockIdx.z, h = blockIdx.y;
   const int n = a.entry_n[e];
@@ -575,6 +579,7 @@ template <typename TA, int V>
 __global__ void __launch_bounds__(256) group_norm_gate_kernel(const float* __restrict__ o, const float* __restrict__ w, int w_n,
                                                               const TA* __restrict__ gate, long long ldg, int gate_mode, TA* __restrict__ out,
                                                               long long ldo, int D, int groups, float eps, float scale) {
+  pg::griddep_begin();
   __shared__ float red[8];
   const long long t = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gs = D / groups;
@@ -629,6 +634,7 @@ template <typename TA, int NV>
 __global__ void __launch_bounds__(256) group_norm_gate_flat_kernel(const float* __restrict__ o, const float* __restrict__ w, int w_n,
                                                                    const TA* __restrict__ gate, long long ldg, int gate_mode, TA* __restrict__ out,
                                                                    long long ldo, int D, int gs, long long total_groups, float eps, float scale) {
+  pg::griddep_begin();
   const int lanes = gs / (4 * NV), groups = D / gs;
   const long long id = (long long)blockIdx.x * (256 / lanes) + threadIdx.x / lanes;  // (row, group)
   const int l = threadIdx.x & (lanes - 1);
@@ -684,7 +690,7 @@ int launch_conv(const void* x, long long ldx, const float* w, const float* bias,
   int chunk = 32;
   while (chunk > 8 && (long long)groups * entries * ((max_n + chunk - 1) / chunk) < 16LL * pg::num_sms()) chunk /= 2;
   const dim3 grid((groups + 3) / 4, (max_n + chunk - 1) / chunk, entries);
-  short_conv_kernel<TA, V, NK, TAPS><<<grid, 128, 0, st>>>(static_cast<const TA*>(x), ldx, w, bias, state, static_cast<TA*>(out), ldo, inv, ldi, sec, taps, C,
+  pg::launch_dependent(short_conv_kernel<TA, V, NK, TAPS>, grid, 128, 0, st, static_cast<const TA*>(x), ldx, w, bias, state, static_cast<TA*>(out), ldo, inv, ldi, sec, taps, C,
                                                             row0, n, ctx, slot, chunk);
   PG_RET();
 }
@@ -713,7 +719,7 @@ int launch_conv_vec(const void* x, long long ldx, const float* w, const float* b
   int chunk = 64;
   while (chunk > 8 && (long long)warps * entries * ((max_n + chunk - 1) / chunk) < 48LL * pg::num_sms()) chunk /= 2;
   const dim3 grid((warps + 3) / 4, (max_n + chunk - 1) / chunk, entries);
-  short_conv_vec_kernel<TAPS, V><<<grid, 128, 0, st>>>(static_cast<const bf16*>(x), ldx, w, bias, state, static_cast<bf16*>(out), ldo, inv, ldi, sec, taps, C, row0,
+  pg::launch_dependent(short_conv_vec_kernel<TAPS, V>, grid, 128, 0, st, static_cast<const bf16*>(x), ldx, w, bias, state, static_cast<bf16*>(out), ldo, inv, ldi, sec, taps, C, row0,
                                                         n, ctx, slot, chunk);
   PG_RET();
 }
@@ -776,7 +782,7 @@ template <typename TA, int VEC, int RP>
 int launch_delta_scan(const PgDeltaArgs& a, int n_min, int n_max, cudaStream_t st) {
   constexpr int VB = 16 * VEC;
   const size_t smem = ((size_t)6 * a.dim + 64 * VB) * sizeof(float);
-  delta_scan_kernel<TA, VEC, RP><<<dim3((a.vdim + VB - 1) / VB, a.H, a.entries), 256, smem, st>>>(a, n_min, n_max);
+  pg::launch_dependent(delta_scan_kernel<TA, VEC, RP>, dim3((a.vdim + VB - 1) / VB, a.H, a.entries), 256, smem, st, a, n_min, n_max);
   PG_RET();
 }
 
@@ -784,7 +790,7 @@ template <typename TA, int VEC, int RP, int KIND>
 int launch_gated_scan(const PgGatedArgs& a, int n_min, int n_max, cudaStream_t st) {
   constexpr int VB = 16 * VEC;
   const size_t smem = ((size_t)4 * a.dim + 32 * VB + 32) * sizeof(float);
-  gated_scan_kernel<TA, VEC, RP, KIND><<<dim3((a.vdim + VB - 1) / VB, a.H, a.entries), 256, smem, st>>>(a, n_min, n_max);
+  pg::launch_dependent(gated_scan_kernel<TA, VEC, RP, KIND>, dim3((a.vdim + VB - 1) / VB, a.H, a.entries), 256, smem, st, a, n_min, n_max);
   PG_RET();
 }
 
@@ -851,14 +857,14 @@ extern "C" int pg_group_norm_gate(const float* o, const float* w, int w_n, const
       const int lanes = gs / (4 * nv);
       if (lanes * 4 * nv != gs || lanes > 32 || (lanes & (lanes - 1))) continue;
       const unsigned blocks = (unsigned)((total + 256 / lanes - 1) / (256 / lanes));
-#define PG_GF(TA, NV) group_norm_gate_flat_kernel<TA, NV><<<blocks, 256, 0, st>>>(o, w, w_n, static_cast<const TA*>(gate), ldg, gate_mode, static_cast<TA*>(out), ldo, D, gs, total, eps, scale)
+#define PG_GF(TA, NV) pg::launch_dependent(group_norm_gate_flat_kernel<TA, NV>, blocks, 256, 0, st, o, w, w_n, static_cast<const TA*>(gate), ldg, gate_mode, static_cast<TA*>(out), ldo, D, gs, total, eps, scale)
       if (act_f32) { if (nv == 1) PG_GF(float, 1); else if (nv == 2) PG_GF(float, 2); else if (nv == 4) PG_GF(float, 4); else PG_GF(float, 8); }
       else { if (nv == 1) PG_GF(bf16, 1); else if (nv == 2) PG_GF(bf16, 2); else if (nv == 4) PG_GF(bf16, 4); else PG_GF(bf16, 8); }
 #undef PG_GF
       PG_RET();
     }
   }
-#define PG_GN(TA, V) group_norm_gate_kernel<TA, V><<<rows, 256, 0, st>>>(o, w, w_n, static_cast<const TA*>(gate), ldg, gate_mode, static_cast<TA*>(out), ldo, D, groups, eps, scale)
+#define PG_GN(TA, V) pg::launch_dependent(group_norm_gate_kernel<TA, V>, rows, 256, 0, st, o, w, w_n, static_cast<const TA*>(gate), ldg, gate_mode, static_cast<TA*>(out), ldo, D, groups, eps, scale)
   if (act_f32) {
     if (gs >= 128 && fits(4)) PG_GN(float, 4);
     else if (fits(2)) PG_GN(float, 2);

@@ -107,6 +107,7 @@ __device__ __forceinline__ void store_state(const float (&S)[DIM / 8][4], float*
 // ---------------------------------------------------------------------------------------------------------------------
 template <int DIM, int C, int KIND>
 __global__ void __launch_bounds__(128) gated_block_kernel(PgGatedArgs a, int n_min) {
+  pg::griddep_begin();
   constexpr int LD = DIM + 8, LV = 64 + 8, LP = C + 8, TL = C / 32;  // TL: tokens per lane of warp 0
   const int e = blockIdx.z, h = blockIdx.y;
   const int n = a.entry_n[e];
@@ -425,6 +426,7 @@ __device__ __forceinline__ long long block_index(const PgDeltaArgs& a, int e, in
 
 template <int DIMP>
 __global__ void __launch_bounds__(128) delta_blocks_kernel(PgDeltaArgs a, float* __restrict__ decay, uint4* __restrict__ scratch, int n_min) {
+  pg::griddep_begin();
   constexpr int LD = DIMP + 4;
   const int e = blockIdx.z, h = blockIdx.y, blk = blockIdx.x;
   const int n = a.entry_n[e];
@@ -598,6 +600,7 @@ __global__ void __launch_bounds__(128) delta_blocks_kernel(PgDeltaArgs a, float*
 // ---------------------------------------------------------------------------------------------------------------------
 template <int DIM>
 __global__ void __launch_bounds__(128) delta_chain_kernel(PgDeltaArgs a, const uint4* __restrict__ scratch, int n_min) {
+  pg::griddep_begin();
   constexpr int LD = DIM + 8, LV = 72, NI = (DIM + 63) / 64, TILE = 16 * LD;
   const int e = blockIdx.z, h = blockIdx.y;
   const int n = a.entry_n[e];
@@ -777,7 +780,7 @@ int launch_gated(const PgGatedArgs& a, int n_min, cudaStream_t st) {
   auto kern = gated_block_kernel<DIM, C, KIND>;
   const int rc = set_smem(kern, smem);
   if (rc != PG_OK) return rc;
-  kern<<<dim3((a.vdim + 63) / 64, a.H, a.entries), 128, smem, st>>>(a, n_min);
+  pg::launch_dependent(kern, dim3((a.vdim + 63) / 64, a.H, a.entries), 128, smem, st, a, n_min);
   pg_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
 }
@@ -789,13 +792,13 @@ int launch_delta(const PgDeltaArgs& a, float* decay, uint4* scratch, int max_n, 
   auto k1 = delta_blocks_kernel<DP>;
   int rc = set_smem(k1, s1);
   if (rc != PG_OK) return rc;
-  k1<<<dim3((max_n + 15) / 16, a.H, a.entries), 128, s1, st>>>(a, decay, scratch, n_min);
+  pg::launch_dependent(k1, dim3((max_n + 15) / 16, a.H, a.entries), 128, s1, st, a, decay, scratch, n_min);
   pg_count_launch(1);
   const size_t s2 = (size_t)(18 * 16 * (DIM + 8) + 2 * 16 * 72) * sizeof(bf16) + (size_t)2 * DIM * sizeof(float);
   auto k2 = delta_chain_kernel<DIM>;
   rc = set_smem(k2, s2);
   if (rc != PG_OK) return rc;
-  k2<<<dim3((a.vdim + 63) / 64, a.H, a.entries), 128, s2, st>>>(a, scratch, n_min);
+  pg::launch_dependent(k2, dim3((a.vdim + 63) / 64, a.H, a.entries), 128, s2, st, a, scratch, n_min);
   pg_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
 }

@@ -31,6 +31,7 @@ __device__ __forceinline__ void st_t(bf16* p, long long i, float v) { p[i] = __f
 template <typename TI>
 __global__ void embed_streams_kernel(const int* __restrict__ tokens, const TI* __restrict__ table, long long ld, float* __restrict__ xs, int S, int D,
                                      float scale) {
+  pg::griddep_begin();
   const long long t = blockIdx.x;
   const long long row = tokens[t];
   for (int d = threadIdx.x; d < D; d += blockDim.x) {
@@ -76,6 +77,7 @@ __global__ void __launch_bounds__(256) stream_mix_norm_kernel(float* __restrict_
                                                               const float* __restrict__ mix, const float* __restrict__ wr,
                                                               const float* __restrict__ rd, const float* __restrict__ norm_w,
                                                               TO* __restrict__ out_act, int S, int D, float eps) {
+  pg::griddep_begin();
   extern __shared__ __align__(16) float sm[];  // u[D], then 32 partial sums
   float* us = sm;
   float* red = sm + D;
@@ -151,7 +153,7 @@ int launch_stream(float* xs, const float* y, long long ldy, const float* mix, co
                   int rows, int S, int D, float eps, size_t smem, cudaStream_t st) {
   auto kern = stream_mix_norm_kernel<TO, V, SMAX>;
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return PG_ERR_CUDA;
-  kern<<<rows, 256, smem, st>>>(xs, y, ldy, mix, wr, rd, norm_w, static_cast<TO*>(out_act), S, D, eps);
+  pg::launch_dependent(kern, rows, 256, smem, st, xs, y, ldy, mix, wr, rd, norm_w, static_cast<TO*>(out_act), S, D, eps);
   pg_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
 }
@@ -162,9 +164,9 @@ extern "C" int pg_embed_streams(const int* tokens, const void* table, long long 
                                 void* stream) {
   if (rows <= 0 || D <= 0 || S <= 0) return PG_ERR_ARG;
   if (table_f32)
-    embed_streams_kernel<float><<<rows, 128, 0, PG_ST(stream)>>>(tokens, static_cast<const float*>(table), ld, xs, S, D, scale);
+    pg::launch_dependent(embed_streams_kernel<float>, rows, 128, 0, PG_ST(stream), tokens, static_cast<const float*>(table), ld, xs, S, D, scale);
   else
-    embed_streams_kernel<bf16><<<rows, 128, 0, PG_ST(stream)>>>(tokens, static_cast<const bf16*>(table), ld, xs, S, D, scale);
+    pg::launch_dependent(embed_streams_kernel<bf16>, rows, 128, 0, PG_ST(stream), tokens, static_cast<const bf16*>(table), ld, xs, S, D, scale);
   pg_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
 }
