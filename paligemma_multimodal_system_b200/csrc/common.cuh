@@ -142,13 +142,18 @@ PG_DEVINL void prefetch_l2_bulk_hint(const void* ptr, uint32_t bytes, uint64_t h
 // PDL (programmatic dependent launch)
 PG_DEVINL void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 PG_DEVINL void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// First statement of the kernels that are a link of a chain (norms, mixers, routing): lets the next kernel become resident -- a product then requests its
-// first weight tiles, the only thing any kernel here touches ahead of its own wait -- and waits for the kernel before.  Triggering ahead of the wait is safe
-// because every link waits: the next one passes its wait when this kernel has completed, and this one completes after all before it.
+// First statement of the kernels that are a link of a chain (norms, mixers, routing): lets the next kernel become resident and waits for the kernel before.
+// Triggering ahead of the wait is safe because every link waits: the next one passes its wait when this kernel has completed, and this one completes after all
+// before it.  Ahead of its wait a kernel touches only what no kernel of the chain writes: weights, and the descriptors of a ragged step (tokens, positions,
+// entries, page table), which the host copies ahead of the step's first kernel -- a kernel of the chain starts after the one before has started, so after that
+// copy.  L2 prefetches are hints and may cover anything.
+template <bool EARLY = true>
 PG_DEVINL void griddep_begin() {
-  griddep_launch_dependents();
+  if (EARLY) griddep_launch_dependents();
   griddep_wait();
 }
+// EARLY = false: the next kernel comes when this one ends.  Long kernels of the fp32 mode, whose SMs come free one after the other: a product behind them takes nothing
+// in ahead of its wait, and its CTAs would crowd on the first SMs that are free.
 
 // ---------------------------------------------------------------------------------------------
 // tcgen05 / TMEM
@@ -330,7 +335,14 @@ inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 bl
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-// The same, counted.
+// For kernels that run long with few CTAs per SM: behind the whole of the kernel before.  CTAs that become resident while that one still holds most SMs share the few
+// that are free, and stay there (an fp32 product of 24 tokens behind the merge of a decode attention: 16 -> 34 us).
+template <typename... KArgs, typename... Args>
+inline void launch_spread(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+  kernel<<<grid, block, smem, st>>>(static_cast<KArgs>(args)...);
+}
+
+// launch_dependent, counted.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
   pg_count_launch(1);

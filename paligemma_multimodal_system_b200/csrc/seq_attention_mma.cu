@@ -562,7 +562,7 @@ int launch(const void* q, const void* kp, const void* vp, const void* gate, long
   auto kern = sx.logistic ? attn_ragged_mma_kernel<DIM, VDIM, true> : attn_ragged_mma_kernel<DIM, VDIM, false>;
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return PG_ERR_CUDA;
   dim3 grid((max_n * (H / G) + 63) / 64, G, entries);
-  pg::launch_dependent(kern, grid, 128, smem, st, static_cast<const bf16*>(q), static_cast<const bf16*>(kp), static_cast<const bf16*>(vp), static_cast<const bf16*>(gate), ldg,
+  pg::launch_spread(kern, grid, 128, smem, st, static_cast<const bf16*>(q), static_cast<const bf16*>(kp), static_cast<const bf16*>(vp), static_cast<const bf16*>(gate), ldg,
                                 static_cast<bf16*>(out), row0, n, ctx, pt, max_pages, page, H, G, scale, softcap, skip_single, gate_per_head, sx);
   pg_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;

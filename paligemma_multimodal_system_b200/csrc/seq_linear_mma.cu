@@ -259,7 +259,7 @@ int launch_blocks(const bf16* qkv, long long ld, float* state, const float* deca
   const size_t smem = (size_t)(6 * C * (DIM + 8) + 3 * C * (C + 8) + 2 * C * 72) * sizeof(bf16) + (C + 1) * sizeof(float);
   auto kern = linear_attn_block_kernel<DIM, C>;
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return PG_ERR_CUDA;
-  pg::launch_dependent(kern, dim3((vdim + 63) / 64, H, entries), 128, smem, st, qkv, ld, state, decay, out, row0, n, ctx, slot, H, dim, vdim, ops);
+  pg::launch_spread(kern, dim3((vdim + 63) / 64, H, entries), 128, smem, st, qkv, ld, state, decay, out, row0, n, ctx, slot, H, dim, vdim, ops);
   pg_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
 }

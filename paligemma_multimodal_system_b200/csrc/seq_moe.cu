@@ -424,7 +424,7 @@ static int launch_moe_mma(dim3 grid, cudaStream_t st, const void* x, long long l
   const size_t smem = (size_t)MOE_STAGES * (MOE_TILE + BN) * MOE_LD * sizeof(bf16);
   auto kern = moe_gemm_mma_kernel<TO, BN>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return PG_ERR_CUDA;
-  pg::launch_dependent(kern, grid, 128, smem, st, static_cast<const bf16*>(x), ldx, sorted_pair, src_div, static_cast<const bf16*>(w), expert_stride, ldw, static_cast<TO*>(out), ldo,
+  pg::launch_spread(kern, grid, 128, smem, st, static_cast<const bf16*>(x), ldx, sorted_pair, src_div, static_cast<const bf16*>(w), expert_stride, ldw, static_cast<TO*>(out), ldo,
                                 plan, F, K, act, x_off, out_off);
   pg_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
@@ -588,13 +588,13 @@ extern "C" int pg_moe_gemm(const void* x, long long ldx, const int* sorted_pair,
 #undef PG_MOE_MMA
   }
   if (in_f32 && out_f32)
-    pg::launch_dependent(moe_gemm_kernel<float, float>, grid, 256, 0, st, static_cast<const float*>(x), ldx, sorted_pair, src_div, static_cast<const float*>(w), expert_stride,
+    pg::launch_spread(moe_gemm_kernel<float, float>, grid, 256, 0, st, static_cast<const float*>(x), ldx, sorted_pair, src_div, static_cast<const float*>(w), expert_stride,
                                                        ldw, static_cast<float*>(out), ldo, plan, F, K, act, x_expert_off, out_expert_off);
   else if (!in_f32 && out_f32)
-    pg::launch_dependent(moe_gemm_kernel<bf16, float>, grid, 256, 0, st, static_cast<const bf16*>(x), ldx, sorted_pair, src_div, static_cast<const bf16*>(w), expert_stride,
+    pg::launch_spread(moe_gemm_kernel<bf16, float>, grid, 256, 0, st, static_cast<const bf16*>(x), ldx, sorted_pair, src_div, static_cast<const bf16*>(w), expert_stride,
                                                       ldw, static_cast<float*>(out), ldo, plan, F, K, act, x_expert_off, out_expert_off);
   else if (!in_f32 && !out_f32)
-    pg::launch_dependent(moe_gemm_kernel<bf16, bf16>, grid, 256, 0, st, static_cast<const bf16*>(x), ldx, sorted_pair, src_div, static_cast<const bf16*>(w), expert_stride,
+    pg::launch_spread(moe_gemm_kernel<bf16, bf16>, grid, 256, 0, st, static_cast<const bf16*>(x), ldx, sorted_pair, src_div, static_cast<const bf16*>(w), expert_stride,
                                                      ldw, static_cast<bf16*>(out), ldo, plan, F, K, act, x_expert_off, out_expert_off);
   else
     return PG_ERR_ARG;

@@ -780,7 +780,7 @@ int launch_gated(const PgGatedArgs& a, int n_min, cudaStream_t st) {
   auto kern = gated_block_kernel<DIM, C, KIND>;
   const int rc = set_smem(kern, smem);
   if (rc != PG_OK) return rc;
-  pg::launch_dependent(kern, dim3((a.vdim + 63) / 64, a.H, a.entries), 128, smem, st, a, n_min);
+  pg::launch_spread(kern, dim3((a.vdim + 63) / 64, a.H, a.entries), 128, smem, st, a, n_min);
   pg_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
 }
@@ -792,13 +792,13 @@ int launch_delta(const PgDeltaArgs& a, float* decay, uint4* scratch, int max_n, 
   auto k1 = delta_blocks_kernel<DP>;
   int rc = set_smem(k1, s1);
   if (rc != PG_OK) return rc;
-  pg::launch_dependent(k1, dim3((max_n + 15) / 16, a.H, a.entries), 128, s1, st, a, decay, scratch, n_min);
+  pg::launch_spread(k1, dim3((max_n + 15) / 16, a.H, a.entries), 128, s1, st, a, decay, scratch, n_min);
   pg_count_launch(1);
   const size_t s2 = (size_t)(18 * 16 * (DIM + 8) + 2 * 16 * 72) * sizeof(bf16) + (size_t)2 * DIM * sizeof(float);
   auto k2 = delta_chain_kernel<DIM>;
   rc = set_smem(k2, s2);
   if (rc != PG_OK) return rc;
-  pg::launch_dependent(k2, dim3((a.vdim + 63) / 64, a.H, a.entries), 128, s2, st, a, scratch, n_min);
+  pg::launch_spread(k2, dim3((a.vdim + 63) / 64, a.H, a.entries), 128, s2, st, a, scratch, n_min);
   pg_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
 }
