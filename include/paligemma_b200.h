@@ -395,6 +395,11 @@ int pg_geglu(const void* gu, long long ldgu, void* out, long long ldo, int rows,
 /* x[t, f] <- relu(x[t, f])^2 in place (rows x F, pitch ld): the activation when it is not fused into the GEMM epilogue. */
 int pg_relu2(void* x, long long ld, int rows, int F, int act_f32, void* stream);
 
+/* The whole side input of a step of few rows: g = gelu_tanh(gate_w act) * table[token, col0 : col0 + n] in the activation type, y = proj_w g,
+ * x += y / rms(y) * norm_w, out_act (may be NULL, may be act) = x.  gate_w [n_pad, D], proj_w [D, n_pad]; D a multiple of 256 up to 8192, n_pad a multiple of 8
+ * up to 256, every pointer but the table on a 16-byte boundary; anything else returns PG_ERR_ARG and belongs to the separate launches.  act_f32: act is x, out_act is not used. */
+int pg_token_side(const void* act, const void* gate_w, const int* tokens, const void* table, long long ldt, int col0, const void* proj_w, const float* norm_w,
+                  float* x, void* out_act, int rows, int D, int n, int n_pad, float eps, int act_f32, void* stream);
 /* out[t, j] = gelu_tanh(z[t, j]) * table[tokens[t], col0 + j] for j < n, 0 for n <= j < n_pad (per-token side input: a
  * gate projection of the residual, fp32, times the token's own low-dimensional embedding slice). */
 int pg_side_gate(const float* z, long long ldz, const int* tokens, const void* table, long long ldt, int col0, void* out,

@@ -17,6 +17,11 @@
 
 using bf16 = __nv_bfloat16;
 
+// seq_attention_decode.cu
+int pg_attn_decode_vec(const void* q, const void* kp, const void* vp, const void* gate, long long ldg, void* out, float* partial, const int* row0,
+                       const int* n, const int* ctx, const int* pt, int max_pages, int page, int entries, int nsplit, int H, int G, int dim, int vdim,
+                       float scale, float softcap, int act_f32, long long krow, long long vrow, int gate_per_head, const PgAttnScore& sx, cudaStream_t st);
+
 #define PG_ST(s) reinterpret_cast<cudaStream_t>(s)
 #define PG_RET()                                                    \
   do {                                                              \
@@ -174,7 +179,7 @@ __global__ void __launch_bounds__(128) attn_prepare_vec_kernel(const TA* __restr
                                                                TA* __restrict__ v_pages, int rows, int H, int G, int dim, int vdim, int rot, float eps,
                                                                int norm_qk, int norm_v, int v_from_k, float rot_gain, const TA* __restrict__ v_other,
                                                                long long ldvo, float v_mix) {
-  pg::griddep_begin();
+  pg::griddep_launch_dependents();
   extern __shared__ float cs[];  // [TOK][cos rot/2 | sin rot/2]
   __shared__ float part[2][TOK][4];
   const int t0 = blockIdx.x * TOK, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -192,6 +197,7 @@ __global__ void __launch_bounds__(128) attn_prepare_vec_kernel(const TA* __restr
     cs[k * rot + j] = rot_gain * (float)c;
     cs[k * rot + half + j] = rot_gain * (float)s;
   }
+  pg::griddep_wait();  // (positions, pages and frequencies are the host's)
   if (norm_qk == 2) {  // one root mean square for all of q, one for all of k
 #pragma unroll
     for (int k = 0; k < TOK; ++k) {
@@ -288,7 +294,7 @@ __global__ void __launch_bounds__(256) attn_ragged_kernel(const TA* __restrict__
                                                           const int* __restrict__ entry_ctx, const int* __restrict__ page_table, int max_pages,
                                                           int page, int H, int G, int dim, int vdim, float scale, float softcap, int skip_single,
                                                           long long krow, long long vrow, int gate_per_head, int alias, PgAttnScore sx) {
-  pg::griddep_begin();
+  pg::griddep_begin<sizeof(TA) == 2>();
   const int e = blockIdx.z, g = blockIdx.y, gsz = H / G;
   const int n = entry_n[e], ctx = entry_ctx[e], row0 = entry_row0[e];
   if (skip_single && n == 1) return;
@@ -465,18 +471,16 @@ __device__ __forceinline__ void ld8<bf16>(const bf16* p, float* v) {
   }
 }
 
-// VC = ceil(vdim / 64).  VEC: 16-byte loads -- lane l reads key l's row for the scores; for P V the warp reads four keys per
-// instruction (lane = key l / 8 of the four, value columns 8 (l % 8) .. + 8 of every 64) and the four key groups are summed
-// by shuffles at the end.  All loads of a tile are independent, so a tile costs about one memory round trip.
-template <typename TA, int VC, bool VEC, bool LOGI>
+// VC = ceil(vdim / 64).  (Rows of whole 16-byte pieces: seq_attention_decode.cu.)
+template <typename TA, int VC, bool LOGI>
 __global__ void __launch_bounds__(256) attn_decode_kernel(const TA* __restrict__ q, const TA* __restrict__ k_pages, const TA* __restrict__ v_pages,
                                                           const TA* __restrict__ gate, long long ldg, TA* __restrict__ out, float* __restrict__ partial,
                                                           const int* __restrict__ entry_row0, const int* __restrict__ entry_n,
                                                           const int* __restrict__ entry_ctx, const int* __restrict__ page_table, int max_pages,
                                                           int page, int H, int G, int dim, int vdim, float scale, float softcap, long long krow,
                                                           long long vrow, int gate_per_head, PgAttnScore sx) {
-  pg::griddep_begin();
-  constexpr int NO = VEC ? 8 * VC : 2 * VC;  // accumulator columns per lane
+  pg::griddep_begin<sizeof(TA) == 2>();
+  constexpr int NO = 2 * VC;  // accumulator columns per lane
   const int e = blockIdx.z, g = blockIdx.y, split = blockIdx.x, nsplit = gridDim.x, gsz = H / G;
   if (entry_n[e] != 1) return;
   const int ctx = entry_ctx[e];
@@ -489,7 +493,6 @@ __global__ void __launch_bounds__(256) attn_decode_kernel(const TA* __restrict__
   float* Lg = Mg + 32;
   float* Og = Lg + 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int kg = lane >> 3, l8 = lane & 7;
   for (int i = threadIdx.x; i < gsz * dimp; i += 256) {
     const int r = i / dimp, d = i % dimp;
     Qs[i] = d < dim ? ldf(q, t * ((long long)H * dim) + (long long)(g * gsz + r) * dim + d) : 0.f;
@@ -526,26 +529,11 @@ __global__ void __launch_bounds__(256) attn_decode_kernel(const TA* __restrict__
       float s[4] = {0.f, 0.f, 0.f, 0.f};
       if (vis) {
         const TA* kr = k_pages + ((long long)pt[j / page] * page + j % page) * krow + (long long)g * dim;
-        if (VEC) {
-#pragma unroll 4
-          for (int d = 0; d < dim; d += 8) {
-            float kv[8];
-            ld8(kr + d, kv);
+        for (int d = 0; d < dim; ++d) {
+          const float kv = ldf(kr, d);
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-              if (i < nr) {
-                const float4 qa = *reinterpret_cast<const float4*>(Qs + (rb + i) * dimp + d), qb = *reinterpret_cast<const float4*>(Qs + (rb + i) * dimp + d + 4);
-                s[i] = fmaf(qa.x, kv[0], s[i]); s[i] = fmaf(qa.y, kv[1], s[i]); s[i] = fmaf(qa.z, kv[2], s[i]); s[i] = fmaf(qa.w, kv[3], s[i]);
-                s[i] = fmaf(qb.x, kv[4], s[i]); s[i] = fmaf(qb.y, kv[5], s[i]); s[i] = fmaf(qb.z, kv[6], s[i]); s[i] = fmaf(qb.w, kv[7], s[i]);
-              }
-          }
-        } else {
-          for (int d = 0; d < dim; ++d) {
-            const float kv = ldf(kr, d);
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              if (i < nr) s[i] = fmaf(Qs[(rb + i) * dimp + d], kv, s[i]);
-          }
+          for (int i = 0; i < 4; ++i)
+            if (i < nr) s[i] = fmaf(Qs[(rb + i) * dimp + d], kv, s[i]);
         }
       }
       float* pw = Pw + warp * 128;
@@ -570,81 +558,35 @@ __global__ void __launch_bounds__(256) attn_decode_kernel(const TA* __restrict__
         pw[i * 32 + lane] = pr;
       }
       __syncwarp();
-      if (VEC) {
-        // a 32-key tile never straddles a page (the page size is a multiple of 32)
-        const TA* vt = v_pages + ((long long)pt[(it * 32) / page] * page + (it * 32) % page) * vrow + (long long)g * vdim;
+      const int nk = min(32, ctx + 1 - it * 32);
+      for (int jj = 0; jj < nk; ++jj) {
+        const int key = it * 32 + jj;
+        const TA* vr = v_pages + ((long long)pt[key / page] * page + key % page) * vrow + (long long)g * vdim;
+        float vv[2 * VC];
 #pragma unroll
-        for (int jj0 = 0; jj0 < 32; jj0 += 4) {
-          const int jj = jj0 + kg;
-          if (it * 32 + jj <= ctx) {
-            float vv[8 * VC];
-#pragma unroll
-            for (int c = 0; c < VC; ++c) {
-              const int col = 8 * l8 + 64 * c;
-              if (col < vdim) ld8(vt + (long long)jj * vrow + col, vv + 8 * c);
-              else {
-#pragma unroll
-                for (int x = 0; x < 8; ++x) vv[8 * c + x] = 0.f;
-              }
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float pj = pw[i * 32 + jj];
-#pragma unroll
-              for (int c = 0; c < 8 * VC; ++c) o[i][c] = fmaf(pj, vv[c], o[i][c]);
-            }
-          }
+        for (int c = 0; c < VC; ++c) {
+          const int col = 2 * lane + 64 * c;
+          vv[2 * c] = col < vdim ? ldf(vr, col) : 0.f;
+          vv[2 * c + 1] = col + 1 < vdim ? ldf(vr, col + 1) : 0.f;
         }
-      } else {
-        const int nk = min(32, ctx + 1 - it * 32);
-        for (int jj = 0; jj < nk; ++jj) {
-          const int key = it * 32 + jj;
-          const TA* vr = v_pages + ((long long)pt[key / page] * page + key % page) * vrow + (long long)g * vdim;
-          float vv[2 * VC];
 #pragma unroll
-          for (int c = 0; c < VC; ++c) {
-            const int col = 2 * lane + 64 * c;
-            vv[2 * c] = col < vdim ? ldf(vr, col) : 0.f;
-            vv[2 * c + 1] = col + 1 < vdim ? ldf(vr, col + 1) : 0.f;
-          }
+        for (int i = 0; i < 4; ++i) {
+          const float pj = pw[i * 32 + jj];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float pj = pw[i * 32 + jj];
-#pragma unroll
-            for (int c = 0; c < 2 * VC; ++c) o[i][c] = fmaf(pj, vv[c], o[i][c]);
-          }
+          for (int c = 0; c < 2 * VC; ++c) o[i][c] = fmaf(pj, vv[c], o[i][c]);
         }
       }
       __syncwarp();
-    }
-    if (VEC) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int c = 0; c < NO; ++c) {
-          o[i][c] += __shfl_xor_sync(0xffffffffu, o[i][c], 8);
-          o[i][c] += __shfl_xor_sync(0xffffffffu, o[i][c], 16);
-        }
     }
     // merge the 8 warps
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       if (lane == 0) { Mg[warp * 4 + i] = m[i]; Lg[warp * 4 + i] = l[i]; }
-      if (VEC) {
-        if (kg == 0) {
 #pragma unroll
-          for (int c = 0; c < NO; ++c) {
-            const int col = 8 * l8 + 64 * (c / 8) + (c % 8);
-            if (col < vdim) Og[(warp * 4 + i) * vdim + col] = o[i][c];
-          }
-        }
-      } else {
-#pragma unroll
-        for (int c = 0; c < NO; ++c) {
-          const int col = 2 * lane + 64 * (c / 2) + (c % 2);
-          if (col < vdim) Og[(warp * 4 + i) * vdim + col] = o[i][c];
-        }
+      for (int c = 0; c < NO; ++c) {
+        const int col = 2 * lane + 64 * (c / 2) + (c % 2);
+        if (col < vdim) Og[(warp * 4 + i) * vdim + col] = o[i][c];
       }
     }
     __syncthreads();
@@ -685,7 +627,7 @@ template <typename TA>
 __global__ void attn_decode_merge_kernel(const float* __restrict__ partial, const TA* __restrict__ gate, long long ldg, TA* __restrict__ out,
                                          const int* __restrict__ entry_row0, const int* __restrict__ entry_n, int H, int vdim, int nsplit,
                                          int gate_per_head, PgAttnScore sx) {
-  pg::griddep_begin();
+  pg::griddep_begin<sizeof(TA) == 2>();
   const float* sink = sx.logistic ? nullptr : sx.sink;
   const long long ldo = sx.out_ld > 0 ? sx.out_ld : (long long)H * vdim;
   const float oscale = sx.out_scale != 0.f ? sx.out_scale : 1.f;
@@ -807,6 +749,91 @@ __global__ void __launch_bounds__(256) linear_attn_scan_kernel(const TA* __restr
   }
 }
 
+// The same with the state in 16-byte pieces (vdim a multiple of four, dim <= 8 RP): thread = four value columns x every eighth key dimension, CTA = 64 columns of
+// a head.  A step of single tokens moves the state once in and once out and is bound by that (48 requests x 32 heads x 64 x 64, 50 MB: 19.6 -> 13 us): all
+// its pieces are requested at once, beside the token's q, k and v.
+template <typename TA, int RP>
+__global__ void __launch_bounds__(128, RP == 8 ? 7 : 3) linear_attn_scan_vec_kernel(const TA* __restrict__ qkv, long long ld, float* __restrict__ state,
+                                                                   const float* __restrict__ decay, float* __restrict__ out,
+                                                                   const int* __restrict__ entry_row0, const int* __restrict__ entry_n,
+                                                                   const int* __restrict__ entry_ctx, const int* __restrict__ entry_slot, int H,
+                                                                   int dim, int vdim, PgLinearAttnOps ops) {
+  pg::griddep_launch_dependents();
+  __shared__ float qs[8 * RP], ksm[8 * RP];
+  __shared__ __align__(16) float red[8][64];
+  const int e = blockIdx.z, h = blockIdx.y, vb = 64 * blockIdx.x;
+  const int n = entry_n[e], row0 = entry_row0[e], slot = entry_slot[e], ctx = entry_ctx[e];
+  const float a = decay[h];
+  const bool mine = n >= ops.n_min && n <= ops.n_max;
+  const int rg = threadIdx.x >> 4, v = vb + 4 * (threadIdx.x & 15);
+  const bool v_ok = v < vdim;
+  float4* st = reinterpret_cast<float4*>(state + (((long long)slot * H + h) * dim) * vdim + (v_ok ? v : 0));
+  const long long pitch = vdim / 4;
+  // the state, on its way to L2 while the kernels before still run (only a hint: it is read behind the wait)
+  if (mine && ctx != 0 && (threadIdx.x & 7) == 0 && v_ok)
+    for (int d = rg; d < dim; d += 8) asm volatile("prefetch.global.L2 [%0];" ::"l"(st + d * pitch));
+  pg::griddep_wait();
+  if (!mine) return;
+  float4 S[RP];
+#pragma unroll
+  for (int i = 0; i < RP; ++i) {
+    const int d = 8 * i + rg;
+    S[i] = (ctx != 0 && d < dim && v_ok) ? st[d * pitch] : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  const long long qo = (long long)h * dim, ko = (long long)H * dim + (long long)h * dim, vo = 2LL * H * dim + (long long)h * vdim;
+  for (int t = 0; t < n; ++t) {
+    const TA* row = qkv + (long long)(row0 + t) * ld;
+    float vv[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) vv[c] = v_ok ? ldf(row, vo + v + c) : 0.f;
+    if (ops.silu) {
+      for (int d = threadIdx.x; d < dim; d += 128) {
+        qs[d] = silu(ldf(row, qo + d));
+        ksm[d] = silu(ldf(row, ko + d));
+      }
+#pragma unroll
+      for (int c = 0; c < 4; ++c) vv[c] = silu(vv[c]);
+    } else {
+      for (int i = threadIdx.x; 2 * i < dim; i += 128) {
+        const int d = 2 * i;
+        const bool two = d + 1 < dim;
+        float q0 = ldf(row, qo + d), q1 = two ? ldf(row, qo + d + 1) : 0.f, k0 = ldf(row, ko + d), k1 = two ? ldf(row, ko + d + 1) : 0.f;
+        enter_pair(ops, row0 + t, i, 1.0f, q0, q1);
+        enter_pair(ops, row0 + t, i, ops.kscale, k0, k1);
+        qs[d] = q0;
+        ksm[d] = k0;
+        if (two) { qs[d + 1] = q1; ksm[d + 1] = k1; }
+      }
+    }
+    __syncthreads();
+    float4 part = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < RP; ++i) {
+      const int d = 8 * i + rg;
+      if (d < dim) {
+        const float kd = ksm[d], qd = qs[d];
+        S[i].x = fmaf(a, S[i].x, kd * vv[0]); S[i].y = fmaf(a, S[i].y, kd * vv[1]); S[i].z = fmaf(a, S[i].z, kd * vv[2]); S[i].w = fmaf(a, S[i].w, kd * vv[3]);
+        part.x = fmaf(S[i].x, qd, part.x); part.y = fmaf(S[i].y, qd, part.y); part.z = fmaf(S[i].z, qd, part.z); part.w = fmaf(S[i].w, qd, part.w);
+      }
+    }
+    if (t == n - 1) {
+#pragma unroll
+      for (int i = 0; i < RP; ++i) {
+        const int d = 8 * i + rg;
+        if (d < dim && v_ok) st[d * pitch] = S[i];
+      }
+    }
+    *reinterpret_cast<float4*>(&red[rg][4 * (threadIdx.x & 15)]) = part;
+    __syncthreads();
+    if (threadIdx.x < 64 && vb + threadIdx.x < vdim) {
+      float o = 0.f;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) o += red[c][threadIdx.x];
+      out[(long long)(row0 + t) * ((long long)H * vdim) + (long long)h * vdim + vb + threadIdx.x] = o;
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------------------------------------------------
 // The same recurrence advanced 32 tokens at a time.  With a = decay, block rows i, j = 0 .. c-1 and S the state before the block:
 //   o_i = sum_{j <= i} a^(i-j) (q_i . k_j) v_j  +  a^(i+1) S^T q_i        S' = a^c S + sum_j a^(c-1-j) k_j v_j^T
@@ -821,7 +848,7 @@ __global__ void __launch_bounds__(256, 2) linear_attn_chunked_kernel(const TA* _
                                                                   const int* __restrict__ entry_row0, const int* __restrict__ entry_n,
                                                                   const int* __restrict__ entry_ctx, const int* __restrict__ entry_slot, int H,
                                                                   int dim, int vdim, PgLinearAttnOps ops) {
-  pg::griddep_begin();
+  pg::griddep_begin<sizeof(TA) == 2>();
   constexpr int C = 32;
   const int e = blockIdx.z, h = blockIdx.y, vb = blockIdx.x;
   const int n = entry_n[e], row0 = entry_row0[e];
@@ -1082,7 +1109,7 @@ static int launch_attn_ragged(const void* q, const void* kp, const void* vp, con
   auto kern = sx.logistic ? attn_ragged_kernel<TA, VC, true> : attn_ragged_kernel<TA, VC, false>;
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return PG_ERR_CUDA;
   dim3 grid((max_n * (H / G) + 31) / 32, G, entries);
-  pg::launch_dependent(kern, grid, 256, smem, st, static_cast<const TA*>(q), static_cast<const TA*>(kp), static_cast<const TA*>(vp), static_cast<const TA*>(gate), ldg,
+  pg::launch_spread(kern, grid, 256, smem, st, static_cast<const TA*>(q), static_cast<const TA*>(kp), static_cast<const TA*>(vp), static_cast<const TA*>(gate), ldg,
                                 static_cast<TA*>(out), row0, n, ctx, pt, max_pages, page, H, G, dim, vdim, scale, softcap, skip_single, krow, vrow,
                                 gate_per_head, alias, sx);
   PG_RET();
@@ -1138,6 +1165,18 @@ extern "C" int pg_linear_attn_scan(const void* qkv, long long ld, float* state, 
   PgLinearAttnOps ops;
   if (!linear_attn_ops(options, dim, ops)) return PG_ERR_ARG;
   cudaStream_t st = PG_ST(stream);
+  if (vdim % 4 == 0 && dim <= 128 && (reinterpret_cast<uintptr_t>(state) & 15) == 0) {
+#define PG_SCANV(TA, RP)                                                                                                                                     \
+  pg::launch_dependent(linear_attn_scan_vec_kernel<TA, RP>, dim3((vdim + 63) / 64, H, entries), 128, 0, st, static_cast<const TA*>(qkv), ld, state, decay, \
+                       out, entry_row0, entry_n, entry_ctx, entry_slot, H, dim, vdim, ops)
+    if (act_f32) {
+      if (dim <= 64) PG_SCANV(float, 8); else PG_SCANV(float, 16);
+    } else {
+      if (dim <= 64) PG_SCANV(bf16, 8); else PG_SCANV(bf16, 16);
+    }
+#undef PG_SCANV
+    PG_RET();
+  }
   // VB value columns per CTA (a power of two <= 64); the 256 / VB thread groups split the key dimensions
   int VB = 64;
   while (VB > 8 && VB / 2 >= vdim) VB /= 2;
@@ -1159,7 +1198,7 @@ static int launch_chunked(const void* qkv, long long ld, float* state, const flo
                           const int* slot, int entries, int H, int dim, int vdim, size_t smem, const PgLinearAttnOps& ops, cudaStream_t st) {
   auto kern = linear_attn_chunked_kernel<TA, VEC, VB>;
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return PG_ERR_CUDA;
-  pg::launch_dependent(kern, dim3((vdim + VB - 1) / VB, H, entries), 256, smem, st, static_cast<const TA*>(qkv), ld, state, decay, out, row0, n, ctx, slot, H, dim, vdim, ops);
+  pg::launch_spread(kern, dim3((vdim + VB - 1) / VB, H, entries), 256, smem, st, static_cast<const TA*>(qkv), ld, state, decay, out, row0, n, ctx, slot, H, dim, vdim, ops);
   PG_RET();
 }
 
@@ -1200,7 +1239,7 @@ extern "C" int pg_linear_attn_chunked(const void* qkv, long long ld, float* stat
 #undef PG_CHUNK
 }
 
-template <typename TA, int VC, bool VEC>
+template <typename TA, int VC>
 static int launch_attn_decode(const void* q, const void* kp, const void* vp, const void* gate, long long ldg, void* out, float* partial,
                               const int* row0, const int* n, const int* ctx, const int* pt, int max_pages, int page, int entries, int nsplit, int H,
                               int G, int dim, int vdim, float scale, float softcap, long long krow, long long vrow, int gate_per_head,
@@ -1208,7 +1247,7 @@ static int launch_attn_decode(const void* q, const void* kp, const void* vp, con
   const int gsz = H / G, dimp = (dim + 7) & ~7;
   const size_t smem = ((size_t)gsz * dimp + 8 * 128 + 64 + (size_t)32 * vdim) * sizeof(float);
   if (smem > 200 * 1024) return PG_ERR_ARG;
-  auto kern = sx.logistic ? attn_decode_kernel<TA, VC, VEC, true> : attn_decode_kernel<TA, VC, VEC, false>;
+  auto kern = sx.logistic ? attn_decode_kernel<TA, VC, true> : attn_decode_kernel<TA, VC, false>;
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return PG_ERR_CUDA;
   pg::launch_dependent(kern, dim3(nsplit, G, entries), 256, smem, st, static_cast<const TA*>(q), static_cast<const TA*>(kp), static_cast<const TA*>(vp),
                                                      static_cast<const TA*>(gate), ldg, static_cast<TA*>(out), partial, row0, n, ctx, pt, max_pages, page,
@@ -1250,23 +1289,26 @@ extern "C" int pg_attn_decode(const void* q, const void* k_pages, const void* v_
   cudaStream_t st = PG_ST(stream);
   // 16-byte loads need every head's key / value row to start on an 8-element boundary and tiles that stay inside a page
   const bool vec = (dim % 8 == 0) && (vdim % 8 == 0) && (krow % 8 == 0) && (vrow % 8 == 0) && (page % 32 == 0) && vdim <= 128 &&
-                   ((reinterpret_cast<uintptr_t>(k_pages) & 15) == 0) && ((reinterpret_cast<uintptr_t>(v_pages) & 15) == 0);
-#define PG_ATTD(TA, VC, VEC) \
-  return launch_attn_decode<TA, VC, VEC>(q, k_pages, v_pages, gate, ldg, out, partial, entry_row0, entry_n, entry_ctx, page_table, max_pages, page, \
-                                         entries, nsplit, H, G, dim, vdim, scale, softcap, krow, vrow, gate_per_head, sx, st)
-  if (act_f32) {
-    if (vec && vdim <= 64) PG_ATTD(float, 1, true);
-    if (vec) PG_ATTD(float, 2, true);
-    if (vdim <= 64) PG_ATTD(float, 1, false);
-    if (vdim <= 128) PG_ATTD(float, 2, false);
-    if (vdim <= 256) PG_ATTD(float, 4, false);
-    PG_ATTD(float, 8, false);
+                   ((reinterpret_cast<uintptr_t>(k_pages) & 15) == 0) && ((reinterpret_cast<uintptr_t>(v_pages) & 15) == 0) &&
+                   (long long)(H / G) * ((dim + 63) / 64) <= 700;  // (its query rows in shared memory)
+  if (vec) {
+    const int rc = pg_attn_decode_vec(q, k_pages, v_pages, gate, ldg, out, partial, entry_row0, entry_n, entry_ctx, page_table, max_pages, page, entries, nsplit, H, G,
+                                      dim, vdim, scale, softcap, act_f32, krow, vrow, gate_per_head, sx, st);
+    if (rc != PG_OK || nsplit <= 1) return rc;
+    return pg_attn_decode_merge(partial, gate, ldg, out, entry_row0, entry_n, entries, nsplit, H, vdim, gate_per_head, act_f32, score, stream);
   }
-  if (vec && vdim <= 64) PG_ATTD(bf16, 1, true);
-  if (vec) PG_ATTD(bf16, 2, true);
-  if (vdim <= 64) PG_ATTD(bf16, 1, false);
-  if (vdim <= 128) PG_ATTD(bf16, 2, false);
-  if (vdim <= 256) PG_ATTD(bf16, 4, false);
-  PG_ATTD(bf16, 8, false);
+#define PG_ATTD(TA, VC) \
+  return launch_attn_decode<TA, VC>(q, k_pages, v_pages, gate, ldg, out, partial, entry_row0, entry_n, entry_ctx, page_table, max_pages, page, \
+                                    entries, nsplit, H, G, dim, vdim, scale, softcap, krow, vrow, gate_per_head, sx, st)
+  if (act_f32) {
+    if (vdim <= 64) PG_ATTD(float, 1);
+    if (vdim <= 128) PG_ATTD(float, 2);
+    if (vdim <= 256) PG_ATTD(float, 4);
+    PG_ATTD(float, 8);
+  }
+  if (vdim <= 64) PG_ATTD(bf16, 1);
+  if (vdim <= 128) PG_ATTD(bf16, 2);
+  if (vdim <= 256) PG_ATTD(bf16, 4);
+  PG_ATTD(bf16, 8);
 #undef PG_ATTD
 }

@@ -398,6 +398,13 @@ class TokenSideInput:
         seq_ops.side_gate(z, b.tokens, table, self.index * self.n, gz, self.n)
         return seq_ops.linear(gz, self.w_proj, torch.empty(T, self.D, device="cuda", dtype=torch.float32))
 
+    def add(self, h, b, table, prec, norm_w, x, xa, eps):
+        """x += rms-norm(y) * norm_w; xa (None: fp32 models) receives a copy in the activation type.  h is xa, or x itself."""
+        if seq_ops.token_side_fits(h.shape[0], self.D, self.n_pad, h.dtype):
+            seq_ops.token_side(h, self.w_gate, b.tokens, table, self.index * self.n, self.n, self.w_proj, norm_w, x, xa, eps)
+        else:
+            seq_ops.group_rmsnorm_add(self(h, b, table, prec), norm_w, x, xa, 1, eps)
+
 
 class LatentAttention:
     """Attention whose keys and values are linear images of one cached low-rank row per token.

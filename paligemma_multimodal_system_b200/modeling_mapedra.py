@@ -150,12 +150,11 @@ class MapedraForCausalLM:
             self.pack()
         c, prec = self.config, self.prec
         eps, groups = c.norm_eps, c.norm_groups
-        x = seq_ops.embed_rows(b.tokens, self.embed_d, 0, c.width, c.embedding_scale)
-        # the sub-layers read x in the activation type: in fp32 that is x itself, in bf16 a rounded copy each norm kernel leaves
+        # the sub-layers read x in the activation type: in fp32 that is x itself, in bf16 a rounded copy that the embedding and each norm kernel leave
+        xa = None if prec.f32 else prec.empty(b.T, c.width)
+        x = seq_ops.embed_rows(b.tokens, self.embed_d, 0, c.width, c.embedding_scale, out_act=xa)
         if prec.f32:
             xa = x
-        else:
-            xa = x.to(torch.bfloat16)
         for li, blk in enumerate(self.blocks):
             y = blk.mixer(xa, b, store, li, prec)
             seq_ops.group_rmsnorm_add(y, blk.norm1_d, x, None if prec.f32 else xa, groups, eps)
@@ -163,8 +162,7 @@ class MapedraForCausalLM:
                 y = blk.ff(xa, b, prec)
                 seq_ops.group_rmsnorm_add(y, blk.norm2_d, x, None if prec.f32 else xa, groups, eps)
             if blk.side is not None:
-                y = blk.side(xa, b, self.side_embed_d, prec)
-                seq_ops.group_rmsnorm_add(y, blk.side_norm_d, x, None if prec.f32 else xa, 1, eps)
+                blk.side.add(xa, b, self.side_embed_d, prec, blk.side_norm_d, x, None if prec.f32 else xa, eps)
             if trace is not None:
                 trace.append(x.clone())
         if want_rows is None or want_rows.numel() == 0:

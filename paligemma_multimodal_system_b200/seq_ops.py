@@ -304,6 +304,27 @@ def side_gate(z, tokens, table, col0, out, n):
                                        out.stride(0), rows, int(n), n_pad, int(out.dtype == torch.float32), _lib.stream()), "pg_side_gate")
 
 
+def token_side_fits(rows, D, n_pad, dtype):
+    """The line up to which the side input is one launch: every row reads the weights from L2 for itself, so its four CTAs a row have to be one wave (two CTAs per SM
+    in bf16, one in fp32) and a weight row short.  2048 wide, 64 inner values, separate / one launch in us: bf16 1 row 9.3 / 5.9, 48 rows 10.7 / 7.8, 96 rows 12.0 / 14.0;
+    fp32 5 rows 9.7 / 7.3, 48 rows 14.2 / 13.8, 96 rows 14.5 / 20.8; 4096 wide fp32, 1 row 9.7 / 10.8."""
+    f32 = dtype == torch.float32
+    return rows <= (32 if f32 else 64) and D % 256 == 0 and D <= (2048 if f32 else 4096) and n_pad <= 256
+
+
+def token_side(act, w_gate, tokens, table, col0, n, w_proj, norm_w, x, out_act, eps):
+    """x += rms-norm(w_proj (gelu_tanh(w_gate act) * table[token, col0 : col0 + n])) * norm_w in one launch; out_act (bf16 models) receives a copy of x."""
+    rows, D = x.shape
+    n_pad = w_gate.shape[0]
+    assert act.is_contiguous() and act.shape == x.shape and x.is_contiguous() and x.dtype == torch.float32 and x.is_cuda and act.is_cuda
+    assert act.dtype == w_gate.dtype == w_proj.dtype == table.dtype and w_gate.is_contiguous() and w_proj.is_contiguous() and w_proj.shape == (D, n_pad)
+    assert norm_w.dtype == torch.float32 and norm_w.is_contiguous() and norm_w.numel() == D and table.stride(1) == 1 and tokens.numel() == rows
+    assert out_act is None or (out_act.is_contiguous() and out_act.shape == x.shape and out_act.dtype == act.dtype)
+    _lib.check(_lib.lib().pg_token_side(act.data_ptr(), w_gate.data_ptr(), tokens.data_ptr(), table.data_ptr(), table.stride(0), int(col0), w_proj.data_ptr(),
+                                        norm_w.data_ptr(), x.data_ptr(), _lib.ptr(out_act), rows, D, int(n), n_pad, float(eps), int(act.dtype == torch.float32),
+                                        _lib.stream()), "pg_token_side")
+
+
 NORM_PROJECTION = "projection"  # attn_prepare: one norm over all of q, one over all of k
 
 
@@ -409,8 +430,8 @@ def attn_ragged(q, k_pages, v_pages, gate, out, b: StepBatch, H, G, dim, vdim, s
                                               vdim, gph, 0, 0, _lib.stream()), "pg_attn_decode_merge")
     elif singles and not skip_singles:
         tiles = (reach - 1) // 32 + 1
-        # enough CTAs for two waves, but at least two 32-key tiles for every warp of a CTA
-        nsplit = max(1, min(-(-2 * _lib.num_sms() // (G * singles)), tiles // 16, 32))
+        # three CTAs of four warps per SM at once: what one wave holds, and at least two 32-key tiles for every warp
+        nsplit = max(1, min(3 * _lib.num_sms() // (G * singles), tiles // 8, 32))
         partial = torch.empty(b.E * H * nsplit * (vdim + 2), device="cuda", dtype=torch.float32) if nsplit > 1 else None
         _lib.check(L.pg_attn_decode(q.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), _lib.ptr(gate), ldg, out.data_ptr(), _lib.ptr(partial),
                                     b.row0.data_ptr(), b.n.data_ptr(), b.ctx.data_ptr(), b.page_table.data_ptr(), b.max_pages, page, b.E, nsplit,
