@@ -65,6 +65,7 @@ struct GemmArgs {
                   // broadcast over the batch: the position embeddings added to the patch embeddings, modeling_siglip.py:289-298)
   int n_fast;  // tile raster order (decode_tile)
   int f32_coalesced;  // token-major fp32 epilogue through the shared-memory transposition (alignment checked by the host)
+  int bf16_pieces;    // bf16 rows, outputs and bias start on 16-byte boundaries and hold whole 16-byte pieces
   long long* trace;  // optional profiling stamps (clock64) written by CTA 0
   // ---- decode-step chores of the SWAP kernels ----
   float* zero_buf;  // zero-filled after the dependency wait (the split-K accumulator of a LATER kernel of the chain)
@@ -500,6 +501,62 @@ PG_DEVINL void rowmajor_tile_epilogue(const GemmArgs& args, uint32_t taddr, int 
   }
 }
 
+// bf16 (+bias, +activation) epilogue of a token-major tile whose rows are whole 16-byte pieces.  Lane = token row; 32 columns at a time are turned through a warp-private,
+// swizzled 2 KB shared-memory tile (two of them in turn) into rows of 64 bytes, eight rows a store.  The products of K = 1152 are paced by this: slices of 64 columns
+// (the general form above) need more registers than eight epilogue warps have and spilled 300 bytes a thread; a slice at the end of the features is short
+// here, not element by element.  8192 tokens, gelu rows 4304 x 1152: 109 -> 70 us, plain 86 -> 60; gelu 8192 x 2048 216 -> 196.
+PG_DEVINL void rowmajor_tile_epilogue_bf16(const GemmArgs& args, uint32_t taddr, int m0, int n0, uint32_t stage, int q, int lane, int c_begin, int c_end) {
+  const float scale = args.scale;
+  const int row_base = m0 + q * 32, rows_valid = args.tokens - row_base;
+  char* out = reinterpret_cast<char*>(static_cast<__nv_bfloat16*>(args.out) + static_cast<long long>(row_base + (lane >> 2)) * args.ldo + n0) + (lane & 3) * 16;
+  const long long pitch8 = args.ldo * 16;  // bytes from a row to the eighth one after it
+  const uint32_t mine = stage + lane * 64, swz = (lane >> 1) & 3;
+  int buf = 0;
+#pragma unroll 1
+  for (int c0 = c_begin; c0 < c_end; c0 += 32, buf ^= 2048) {
+    const int left = args.features - n0 - c0;  // columns of this slice and behind it (a multiple of 8)
+    if (left <= 0) break;
+    uint32_t r[2][16];
+    tmem_ld16(taddr + c0, r[0]);
+    tmem_ld16(taddr + c0 + 16, r[1]);
+    float4 b[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      b[i] = args.bias != nullptr && 4 * i < left ? __ldg(reinterpret_cast<const float4*>(args.bias + n0 + c0) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    tmem_ld_wait();
+    uint32_t pk[16];
+    with_act(args.act_gelu, [&](auto act) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float bb[4] = {b[i].x, b[i].y, b[i].z, b[i].w};
+        float v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = fmaf(bb[j], scale, __uint_as_float(r[i >> 2][4 * (i & 3) + j]) * scale);
+        if (decltype(act)::value) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) v[j] = epilogue_act(v[j], decltype(act)::value);
+        }
+        pk[2 * i] = pack_bf16(v[0], v[1]);
+        pk[2 * i + 1] = pack_bf16(v[2], v[3]);
+      }
+    });
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(mine + buf + ((p ^ swz) << 4)), "r"(pk[4 * p]), "r"(pk[4 * p + 1]), "r"(pk[4 * p + 2]),
+                   "r"(pk[4 * p + 3]) : "memory");
+    __syncwarp();
+    const bool col_ok = (lane & 3) * 8 < left;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int row = 8 * k + (lane >> 2);
+      uint4 v;
+      asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                   : "r"(stage + buf + row * 64 + (((lane & 3) ^ ((row >> 1) & 3)) << 4)) : "memory");
+      if (col_ok && row < rows_valid) *reinterpret_cast<uint4*>(out + k * pitch8 + c0 * 2) = v;
+    }
+  }
+}
+
 // fp32 (+bias, +fp32 residual) epilogue of a token-major tile with COALESCED global access.  The accumulator comes out
 // of TMEM one row per thread; 32 columns at a time it is transposed through a warp-private, swizzled 4 KB shared-memory
 // tile into the mapping "8 lanes per row, 16 bytes per lane", so that every global load / store instruction of the
@@ -676,11 +733,13 @@ PG_DEVINL void token_major_epilogue(const GemmArgs& args, uint32_t taddr, int m_
   const uint32_t wstage = xch_base + (warp - 2) * 4096;  // this warp's transposition tile
   const int rows_valid = max(0, min(32, args.tokens - (m_blk * BM + q * 32)));
   // column range of this warp: halves of >= 64 columns (BN = 64: the first warp of the pair takes everything)
-  const int cb = !EPI8 ? 0 : (BN >= 128 ? half * (BN / 2) : (half == 0 ? 0 : BN));
-  const int ce = !EPI8 ? BN : (BN >= 128 ? cb + BN / 2 : BN);
+  // (192 columns: 32-column slices in halves, the 64-column slices of the general form two to one)
+  const int mid = BN == 192 && !(mode == PG_EPI_F32 ? args.f32_coalesced : args.bf16_pieces) ? 128 : BN / 2;
+  const int cb = !EPI8 ? 0 : (BN >= 128 ? (half == 0 ? 0 : mid) : (half == 0 ? 0 : BN));
+  const int ce = !EPI8 ? BN : (BN >= 128 ? (half == 0 ? mid : BN) : BN);
   if constexpr (ROPE) {
     qkv_rope_tile_epilogue<BN>(args, taddr, tok, n_blk, wstage, rows_valid, lane, m_blk * BM + q * 32);
-  } else if (mode == PG_EPI_GEGLU) {
+  } else if (BN != 192 && mode == PG_EPI_GEGLU) {  // (host: gated units come in blocks of 128 columns and take no 192-wide tile)
     // columns: [g0..g63 | u0..u63] per 128-column block; out feature = n_blk*BN/2 + blk*64 + c.  The 64 bf16
     // results of a block (one 128-byte row per token) leave through the warp transposition tile as full lines.
     const bool al = ((reinterpret_cast<uintptr_t>(args.out) & 15) == 0) && ((args.ldo % 8) == 0);
@@ -727,7 +786,8 @@ PG_DEVINL void token_major_epilogue(const GemmArgs& args, uint32_t taddr, int m_
       }
     }
   } else if (mode == PG_EPI_BF16) {
-    rowmajor_tile_epilogue<BN, PG_EPI_BF16>(args, taddr, tok, n_blk * BN, first_split, wstage, rows_valid, lane, cb, ce);
+    if (args.bf16_pieces) rowmajor_tile_epilogue_bf16(args, taddr, m_blk * BM, n_blk * BN, wstage, q, lane, cb, ce);
+    else rowmajor_tile_epilogue<BN, PG_EPI_BF16>(args, taddr, tok, n_blk * BN, first_split, wstage, rows_valid, lane, cb, ce);
   } else if (mode == PG_EPI_F32) {
     // (measured: pulling the NEXT tile's residual rows into L2 from here does not help: o_proj 926 -> 824 TFLOP/s)
     if (args.f32_coalesced)
@@ -853,7 +913,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_cons
     __syncwarp();  // the whole warp reaches the CTA-wide barrier below together (bar.sync counts warps, not lanes)
   } else if (warp == 1) {
     // =================================== MMA issuer =====================================
-    if (lane == 0) {
+    // (all lanes run the loop and one elected lane issues: see gemm_pair_kernel)
+    {
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -869,13 +930,16 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_cons
           const uint32_t sa = smem_base + stage * STAGE_BYTES;
           const uint64_t adesc = make_sdesc_k_sw128(sa);
           const uint64_t bdesc = make_sdesc_k_sw128(sa + A_TILE_BYTES);
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            // advance 16 elements (32 B) along K inside the 128B swizzle row: +2 in the (addr>>4) field
-            umma_f16(d_tmem, adesc + 2 * k, bdesc + 2 * k, IDESC, (kb > t.kb0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < BK / 16; ++k) {
+              // advance 16 elements (32 B) along K inside the 128B swizzle row: +2 in the (addr>>4) field
+              umma_f16(d_tmem, adesc + 2 * k, bdesc + 2 * k, IDESC, (kb > t.kb0 || k > 0) ? 1u : 0u);
+            }
+            umma_commit(empty_bar(stage));  // frees the smem slot once these MMAs have read it
+            if (kb == t.kb1 - 1) umma_commit(tfull_bar(acc));
           }
-          umma_commit(empty_bar(stage));  // frees the smem slot once these MMAs have read it
-          if (kb == t.kb1 - 1) umma_commit(tfull_bar(acc));
+          __syncwarp();
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         if (++acc == ACC_STAGES) { acc = 0; acc_phase ^= 1; }
@@ -967,15 +1031,15 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_cons
 //   tfull[a]  (both CTAs)  : the leader's tcgen05.commit after the last k-block of a tile, multicast
 //   tempty[a] (leader)     : 2 x NEPI arrivals, the epilogue warps of both CTAs
 // ------------------------------------------------------------------------------------------------------------
-constexpr int PAIR_BN = 256;
-constexpr int PAIR_STAGE_BYTES = A_TILE_BYTES + (PAIR_BN / 2) * BK * 2;  // 32 KB
-constexpr int PAIR_STAGES = (232448 - 256 - 8 * 4096) / PAIR_STAGE_BYTES;  // 6
-constexpr int PAIR_SMEM = PAIR_STAGES * PAIR_STAGE_BYTES + 8 * 4096 + 256;
+// 192-column tiles (28 KB a stage, 192-column accumulators): where 256-column tiles leave most of a wave or of the last feature tile empty.
+__host__ __device__ constexpr int pair_stage_bytes(int BN) { return A_TILE_BYTES + (BN / 2) * BK * 2; }                   // 32 / 28 KB
+__host__ __device__ constexpr int pair_stages(int BN) { return (232448 - 256 - 8 * 4096) / pair_stage_bytes(BN); }        // 6 / 6
+__host__ __device__ constexpr int pair_smem(int BN) { return pair_stages(BN) * pair_stage_bytes(BN) + 8 * 4096 + 256; }
 
-template <bool EPI8, bool ROPE>
+template <int BN, bool EPI8, bool ROPE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(EPI8 ? 320 : NUM_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB, const GemmArgs args) {
-  constexpr int BN = PAIR_BN, STAGES = PAIR_STAGES, STAGE_BYTES = PAIR_STAGE_BYTES;
+  constexpr int STAGES = pair_stages(BN), STAGE_BYTES = pair_stage_bytes(BN);
   constexpr int NEPI = EPI8 ? 8 : 4;
   constexpr uint32_t IDESC = make_idesc_bf16(2 * BM, BN);
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -1048,7 +1112,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
     __syncwarp();
   } else if (warp == 1) {
     // =================================== MMA issuer (leader CTA only) ===============================
-    if (leader && lane == 0) {
+    // (all lanes run the loop and one elected lane issues: under `lane == 0` every tcgen05.mma takes ~115 clocks to issue, and the issuer paces the kernel.
+    // 8192 tokens, bf16 rows: 8192 x 2048 229 -> 198 us, 1152 x 4304 82 -> 77, 2048 x 8192 262 -> 225)
+    if (leader) {
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -1063,10 +1129,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
           const uint32_t sa = smem_base + stage * STAGE_BYTES;
           const uint64_t adesc = make_sdesc_k_sw128(sa);
           const uint64_t bdesc = make_sdesc_k_sw128(sa + A_TILE_BYTES);
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) umma_f16_pair(d_tmem, adesc + 2 * k, bdesc + 2 * k, IDESC, (kb > 0 || k > 0) ? 1u : 0u);
-          umma_commit_pair(empty_bar(stage));
-          if (kb == total_kb - 1) umma_commit_pair(tfull_bar(acc));
+            for (int k = 0; k < BK / 16; ++k) umma_f16_pair(d_tmem, adesc + 2 * k, bdesc + 2 * k, IDESC, (kb > 0 || k > 0) ? 1u : 0u);
+            umma_commit_pair(empty_bar(stage));
+            if (kb == total_kb - 1) umma_commit_pair(tfull_bar(acc));
+          }
+          __syncwarp();
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         if (++acc == ACC_STAGES) { acc = 0; acc_phase ^= 1; }
@@ -1100,12 +1169,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
   }
 }
 
-template <bool EPI8, bool ROPE>
+template <int BN, bool EPI8, bool ROPE>
 static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& a, int num_tiles, cudaStream_t st) {
   static bool configured[kMaxDevices] = {};
   const int dev = current_device();
   if (!configured[dev]) {
-    if (cudaFuncSetAttribute(gemm_pair_kernel<EPI8, ROPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM) != cudaSuccess) {
+    if (cudaFuncSetAttribute(gemm_pair_kernel<BN, EPI8, ROPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, pair_smem(BN)) != cudaSuccess) {
       cudaGetLastError();
       return PG_ERR_CUDA;
     }
@@ -1113,7 +1182,7 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmA
   }
   const int pairs = num_sms() / 2;
   const int grid = 2 * (num_tiles < pairs ? num_tiles : pairs);
-  return launch_kernel(gemm_pair_kernel<EPI8, ROPE>, dim3(grid), dim3(EPI8 ? 320 : NUM_THREADS), PAIR_SMEM, st, ta, tb, a) == cudaSuccess
+  return launch_kernel(gemm_pair_kernel<BN, EPI8, ROPE>, dim3(grid), dim3(EPI8 ? 320 : NUM_THREADS), pair_smem(BN), st, ta, tb, a) == cudaSuccess
              ? PG_OK : PG_ERR_CUDA;
 }
 
@@ -1135,9 +1204,9 @@ extern "C" int pg_debug_set_gemm_pair(int mode, int min_tiles) {
   if (min_tiles > 0) g_pair_min_tiles = min_tiles;
   return 0;
 }
-static int g_force_bn = 0;  // tuning sweeps only: 64 / 128 / 256 overrides the token-major kernel's N tile, 0 = automatic
+static int g_force_bn = 0;  // tuning sweeps only: 64 / 128 / 192 / 256 overrides the token-major kernels' N tile, 0 = automatic
 extern "C" int pg_debug_set_gemm_bn(int bn) {
-  if (bn != 0 && bn != 64 && bn != 128 && bn != 256) return PG_ERR_ARG;
+  if (bn != 0 && bn != 64 && bn != 128 && bn != 192 && bn != 256) return PG_ERR_ARG;
   g_force_bn = bn;
   return 0;
 }
@@ -1200,6 +1269,8 @@ static bool cluster_form(const GemmArgs& a, long long ldr, int swap, bool beside
   if (a.K <= 128) return true;
   const int sms = num_sms(), pairs = sms / 2, pair_tiles = ((a.tokens + 2 * BM - 1) / (2 * BM)) * ((a.features + 255) / 256);
   const float steps = static_cast<float>((a.K + BK - 1) / BK);
+  if (act && a.K > 1536 && pair_tiles >= pairs)  // (the pair kernel: 560 clocks a step since one elected lane issues)
+    return plan.waves == 1 || plan.clocks * 1.2f < (pair_tiles + pairs - 1) / pairs * (steps * 560.f + 1500.f) + 5000.f;
   if (act) {
     const int tiles = ((a.tokens + BM - 1) / BM) * ((a.features + 255) / 256);
     return plan.waves == 1 || plan.clocks < (tiles + sms - 1) / sms * (steps * 640.f + 4500.f) + 8000.f;
@@ -1222,6 +1293,16 @@ bool pg_gemm_sums_once(int tokens, int features, int K, const void* out, long lo
   if (!cluster_form(a, 0, swap)) return false;
   const int tiles = (features + BM - 1) / BM;
   return !(swap && tokens <= 64 && tiles * 10 < num_sms() * 7 && static_cast<long long>(features) * K >= 20000000 && plan_cluster_gemm(tokens, features, K).split == 1);
+}
+
+// 192-column tiles instead of 256.  A round of them on the busiest CTA costs about 0.87 of a round of 256 columns -- operand delivery and the barriers of a step do not
+// shrink with the tile -- so they pay where they take no round more: mostly where the last feature tile or the last round of 256 columns is half empty.  Short
+// products into fp32 rows are paced by their epilogue and take one more in eight.  us, 256 / 192 columns (rounds), N x K weights, bf16 rows unless noted:
+//   8192 tokens: 1152 x 4304 76.7 / 66.2 (3, 3), with residual 84.8 / 74.0; 1152 x 1152 28.3 / 27.1 (3, 3), with residual 37.6 / 32.3; 3456 x 1152 61.4 / 63.8 (7, 8),
+//   with residual 94.6 / 88.1; 2560 x 2048 71.4 / 73.6 (5, 7); 2048 x 2048 60.8 / 61.8 (4, 5).  2100 tokens: 2560 x 2048 30.7 / 27.0 (2, 2); 3456 x 1152 22.6 / 26.0 (2, 3).
+//   One CTA per tile (activations): 8192 tokens 1152 x 1152 34.7 / 32.8, 3456 x 1152 73.1 / 75.9 (7, 8).
+static bool narrow_tiles(int tiles256, int tiles192, int at_once, bool f32_short) {
+  return ((tiles192 + at_once - 1) / at_once) * (f32_short ? 0.87f : 1.0f) <= (tiles256 + at_once - 1) / at_once;
 }
 
 static int gemm_bf16(const void* x, long long ldx, const void* w, long long ldw, void* out, long long ldo, const float* bias, const float* resid, long long ldr, int tokens,
@@ -1289,6 +1370,8 @@ static int gemm_bf16(const void* x, long long ldx, const void* w, long long ldw,
   a.f32_coalesced = (!swap && mode == PG_EPI_F32 && (features % 4) == 0 && (ldo % 4) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 &&
                      (bias == nullptr || (reinterpret_cast<uintptr_t>(bias) & 15) == 0) &&
                      (resid == nullptr || ((ldr % 4) == 0 && (reinterpret_cast<uintptr_t>(resid) & 15) == 0))) ? 1 : 0;
+  a.bf16_pieces = (!swap && mode == PG_EPI_BF16 && (features % 8) == 0 && (ldo % 8) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 &&
+                   (bias == nullptr || (reinterpret_cast<uintptr_t>(bias) & 15) == 0)) ? 1 : 0;
   a.trace = g_gemm_trace ? g_gemm_trace + 8 * (g_gemm_trace_idx++ % 64) : nullptr;
 
   if (cluster_form(a, ldr, swap, beside)) {
@@ -1316,29 +1399,47 @@ static int gemm_bf16(const void* x, long long ldx, const void* w, long long ldw,
   } else {
     // largest N tile that still gives the persistent grid ~a wave of CTAs (small token counts: latency path)
     const int m_blocks = (tokens + BM - 1) / BM;
+    // many tokens: a PAIR of CTAs per 256 x 256 tile (cta_group::2), each staging half of the weight tile.  (Activations of a short K: from five rounds of tiles on; us,
+    // one CTA / pair, gelu, 4304 x 1152: 2048 tokens 22.2 / 22.7, 4096 37.2 / 37.7, 8192 70.5 / 68.7; 8192 x 2048: 1500 tokens 42.7 / 40.7, 8192 196 / 181.)
+    const int pair_tiles = ((tokens + 2 * BM - 1) / (2 * BM)) * ((features + 255) / 256);
+    const bool pair = g_pair_mode != 0 && features > 128 && split_k == 1 && mode != PG_EPI_ATOMIC_F32 && pair_tiles >= g_pair_min_tiles && (g_force_bn == 0 || g_force_bn >= 192) &&
+                      (mode != PG_EPI_GEGLU || (features >= 256 && 2 * pair_tiles >= 120)) &&
+                      !(mode == PG_EPI_BF16 && act_gelu && K <= 1536 && pair_tiles < 5 * (num_sms() / 2));
     auto ntiles = [&](int bn) { return m_blocks * ((features + bn - 1) / bn) * split_k; };
     int BN;
     if (mode == PG_EPI_GEGLU) {
       BN = (features >= 256 && ntiles(256) >= 120) ? 256 : 128;
     } else {
       BN = features > 128 ? 256 : features > 64 ? 128 : 64;
-      while (BN > 64 && ntiles(BN) < 120) BN /= 2;
-      if (g_force_bn) BN = g_force_bn;
+      if (mode == PG_EPI_ATOMIC_F32) {
+        while (BN > 64 && ntiles(BN) < 120) BN /= 2;
+      } else if (!pair) {
+        // the tile whose rounds on the busiest CTA cost least (a step of a 192, 128 and 64 wide tile: 0.87, 0.79 and 0.65 of a 256 wide one's).
+        // us, halved until there are 120 tiles / now: 1500 tokens 2048 x 16384 160 / 90 (two rounds of 128 columns, one of 192), 1152 x 4304 45 / 24, 2048 x 2048 27 / 15
+        float least = 0.f;
+        for (int bn = BN, best = BN;; bn = bn == 256 ? 192 : bn == 192 ? 128 : bn / 2) {
+          if (bn < 64) { BN = best; break; }
+          const float cost = static_cast<float>((ntiles(bn) + num_sms() - 1) / num_sms()) * (bn == 256 ? 1.f : bn == 192 ? 0.87f : bn == 128 ? 0.79f : 0.65f);
+          if (least == 0.f || cost < least) { least = cost; best = bn; }
+        }
+      }
+      if (g_force_bn) BN = pair && g_force_bn == 192 ? 256 : g_force_bn;
     }
     if ((rc = make_tmap_2d(&ta, x, tokens, K, ldx, BM)) != PG_OK) return rc;
-    // many tokens: a PAIR of CTAs per 256 x 256 tile (cta_group::2), each staging half of the weight tile
-    const int pair_tiles = ((tokens + 2 * BM - 1) / (2 * BM)) * ((features + 255) / 256);
-    // (against one CTA per tile: +2 .. 16 % per call site but for the gelu epilogue of fc1: 4 vision layers on 8 x 1024 patches 1862 -> 1893 us)
-    if (g_pair_mode != 0 && BN == 256 && split_k == 1 && pair_tiles >= g_pair_min_tiles && !(mode == PG_EPI_BF16 && act_gelu)) {
+    if (pair) {
       if (band_rows > 0) a.n_fast = 2 + (static_cast<int>(band_rows) / (2 * BM) > 0 ? static_cast<int>(band_rows) / (2 * BM) : 1);
-      if ((rc = make_tmap_2d(&tb, w, features, K, ldw, PAIR_BN / 2)) != PG_OK) return rc;
+      const int tiles192 = ((tokens + 2 * BM - 1) / (2 * BM)) * ((features + 191) / 192);
+      const bool narrow = mode != PG_EPI_GEGLU && (g_force_bn == 192 || (g_force_bn == 0 && narrow_tiles(pair_tiles, tiles192, num_sms() / 2, mode == PG_EPI_F32 && K <= 1536)));
+      if ((rc = make_tmap_2d(&tb, w, features, K, ldw, narrow ? 192 / 2 : 256 / 2)) != PG_OK) return rc;
       // eight epilogue warps where the epilogue outlasts the main loop: short K, and the fp32 residual epilogue (8 bytes of
       // residual traffic per element) up to K = 2048 -- o_proj 142 -> 122 us at 16.6k tokens; gate||up and K >= 4304 prefer four
       const bool epi8 = g_epi8_mode == 1 ? true : (g_epi8_mode == 2 ? false : (K <= 1536 || (mode == PG_EPI_F32 && K <= 2048)));
-      return epi8 ? launch_pair<true, false>(ta, tb, a, pair_tiles, st) : launch_pair<false, false>(ta, tb, a, pair_tiles, st);
+      if (narrow) return epi8 ? launch_pair<192, true, false>(ta, tb, a, tiles192, st) : launch_pair<192, false, false>(ta, tb, a, tiles192, st);
+      return epi8 ? launch_pair<256, true, false>(ta, tb, a, pair_tiles, st) : launch_pair<256, false, false>(ta, tb, a, pair_tiles, st);
     }
     if (band_rows > 0) a.n_fast = 2 + (static_cast<int>(band_rows) / BM > 0 ? static_cast<int>(band_rows) / BM : 1);
     if ((rc = make_tmap_2d(&tb, w, features, K, ldw, BN)) != PG_OK) return rc;
+    if (BN == 192) return launch<192, false, true>(ta, tb, a, m_blocks * ((features + 191) / 192), st);
     const int tiles = ((tokens + BM - 1) / BM) * ((features + BN - 1) / BN) * split_k;
     // short reduction (K <= 1536: the SigLIP projections): the epilogue outlasts the main loop, so it gets eight warps
     if (BN == 256 && K <= 1536) return launch<256, false, true>(ta, tb, a, tiles, st);
@@ -1398,8 +1499,8 @@ extern "C" int pg_gemm_qkv_rope(const void* x, long long ldx, const void* w, lon
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int pair_tiles = ((tokens + 2 * BM - 1) / (2 * BM)) * (Hq + 2 * Hkv);
   if (dh == 256 && g_pair_mode != 0 && pair_tiles >= g_pair_min_tiles) {  // CTA pair: 256 tokens x one head per tile
-    if ((rc = make_tmap_2d(&tb, w, features, K, ldw, PAIR_BN / 2)) != PG_OK) return rc;
-    return launch_pair<false, true>(ta, tb, a, pair_tiles, st);
+    if ((rc = make_tmap_2d(&tb, w, features, K, ldw, 256 / 2)) != PG_OK) return rc;
+    return launch_pair<256, false, true>(ta, tb, a, pair_tiles, st);
   }
   return dh == 256 ? launch<256, false, false, true>(ta, tb, a, tiles, st) : launch<64, false, false, true>(ta, tb, a, tiles, st);
 }
