@@ -327,6 +327,12 @@ int pg_prefetch_l2(const void* ptr, long long bytes, int ctas, int evict_last, v
  * (act_f32 = 0) or fp32 (act_f32 = 1); norms, scores, probabilities, states and residual sums are always fp32.
  * ------------------------------------------------------------------------------------------------------------------- */
 
+/* fp32 products of many tokens on the tensor cores (three bf16 terms a value, 64-deep partial sums added in fp32).  pg_gemm_fp32_scratch: bytes of scratch that
+ * pg_gemm_fp32_split wants for these sizes, 0 where the plain-FMA products are faster or the sizes do not fit (K a multiple of 8, features of 4).
+ * pg_gemm_fp32_split: out (+)= (x w^T + bias) * scale, as pg_gemm_simt_bias; rows, bases and scratch on 16-byte boundaries (else PG_ERR_ARG). */
+long long pg_gemm_fp32_scratch(int tokens, int features, int K);
+int pg_gemm_fp32_split(const float* x, long long ldx, const float* w, long long ldw, float* out, long long ldo, const float* bias, int accumulate, float scale, int tokens,
+                       int features, int K, void* scratch, long long scratch_bytes, void* stream);
 /* out[t, f] = sum_k x[t, k] w[f, k] with plain fp32 FMAs (no tensor-core mode): the exact-precision matrix product of
  * the fp32 serving mode, and the bf16 product for shapes the TMA kernels cannot take (K or a pitch not a multiple of 8).
  * in_f32: x and w are fp32 (else bf16); out_f32: out is fp32 (else bf16). */

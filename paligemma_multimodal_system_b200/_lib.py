@@ -73,6 +73,8 @@ SIGNATURES = {
     "pg_group_rmsnorm_add": [p, i64, p, p, p, i32, i32, i32, f32, i32, p],
     "pg_rmsnorm_gate": [p, p, p, i64, p, i32, i32, f32, i32, p],
     "pg_geglu": [p, i64, p, i64, i32, i32, i32, p],
+    "pg_gemm_fp32_scratch": [i32, i32, i32],
+    "pg_gemm_fp32_split": [p, i64, p, i64, p, i64, p, i32, f32, i32, i32, i32, p, i64, p],
     "pg_token_side": [p, p, p, p, i64, i32, p, p, p, p, i32, i32, i32, i32, f32, i32, p],
     "pg_side_gate": [p, i64, p, p, i64, i32, p, i64, i32, i32, i32, i32, p],
     "pg_attn_prepare": [p, i64, p, p, p, i32, i32, p, p, p, p, p, p, i32, i32, i32, i32, i32, i32, f32, i32, i32, i32, f32, p, i64, f32, i32, p],
@@ -117,7 +119,7 @@ SIGNATURES = {
     "pg_gated_layernorm_add": [p, i64, p, i64, p, p, p, p, p, p, p, i32, i32, f32, i32, i32, p],
     "pg_glu": [p, i64, p, i64, i32, i32, i32, f32, f32, i32, p],
 }
-_RESTYPE = {"pg_launch_count": i64}
+_RESTYPE = {"pg_launch_count": i64, "pg_gemm_fp32_scratch": i64}
 
 
 

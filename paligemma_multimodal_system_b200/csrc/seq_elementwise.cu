@@ -11,7 +11,8 @@ using bf16 = __nv_bfloat16;
 
 // seq_gemm_fp32.cu
 int pg_gemm_fp32(const float* x, long long ldx, long long bsx, const float* w, long long ldw, long long bsw, float* out, long long ldo, long long bso,
-                 const float* bias, int accumulate, float scale, int T, int F, int K, int batch, cudaStream_t st);
+                 const float* bias, int accumulate, float scale, int T, int F, int K, int batch, cudaStream_t st,
+                 const int* only_if = nullptr);
 
 #define PG_ST(s) reinterpret_cast<cudaStream_t>(s)
 #define PG_RET()                                                   \

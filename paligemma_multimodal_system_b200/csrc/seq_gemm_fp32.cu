@@ -28,6 +28,7 @@ struct Fp32Args {
   int T, F, K, kpart;  // kpart: k values per cluster rank (a multiple of the k step)
   int accumulate;
   float scale;
+  const int* only_if;  // not NULL: a flag on the device that has to be set for anything to be computed (gemm_fp32_split.cu)
 };
 
 __device__ __forceinline__ void fma2(float2& d, float2 a, float2 b) {
@@ -97,6 +98,7 @@ __global__ void __launch_bounds__(WM* WN * 32, 2) gemm_fp32_tile_kernel(Fp32Args
   };
   pg::griddep_wait();
   pg::griddep_launch_dependents();
+  if (p.only_if != nullptr && *p.only_if == 0) return;  // (the whole grid)
   float2 acc[TM][TN];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
@@ -211,6 +213,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32, CTAS) gemm_fp32_rows_kernel(F
   for (int i = 0; i < RF * TT; ++i) acc[i] = make_float2(0.f, 0.f);
   pg::griddep_wait();
   pg::griddep_launch_dependents();
+  if (p.only_if != nullptr && *p.only_if == 0) return;  // (the whole grid)
   float4 b[PF][RF];
 #pragma unroll
   for (int i = 0; i < PF; ++i) weights(b[i], k_lo + i * 128 + lane * 4);
@@ -327,8 +330,9 @@ cudaError_t launch_rows(int batch, int sms, cudaStream_t st, Fp32Args p) {
 
 // batch independent products (bsx / bsw / bso: elements between their operands).  Returns PG_ERR_ARG for what no grid can express.
 int pg_gemm_fp32(const float* x, long long ldx, long long bsx, const float* w, long long ldw, long long bsw, float* out, long long ldo, long long bso,
-                 const float* bias, int accumulate, float scale, int T, int F, int K, int batch, cudaStream_t st) {
-  Fp32Args p{x, w, bias, out, ldx, ldw, ldo, bsx, bsw, bso, T, F, K, 0, accumulate, scale};
+                 const float* bias, int accumulate, float scale, int T, int F, int K, int batch, cudaStream_t st,
+                 const int* only_if) {
+  Fp32Args p{x, w, bias, out, ldx, ldw, ldo, bsx, bsw, bso, T, F, K, 0, accumulate, scale, only_if};
   const int sms = pg::num_sms();
   // 16-byte copies and loads want every row of every operand on a 16-byte boundary
   const bool wide = K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && bsx % 4 == 0 && bsw % 4 == 0 &&

@@ -1,7 +1,8 @@
 """Host wrappers of the ragged-step kernels (csrc/seq_elementwise.cu, csrc/seq_mixers.cu) and the step's batch descriptor.
 
 `Precision` says in which type activations and matrix operands live: bf16 (tcgen05 GEMMs with fp32 accumulation wherever
-the shape allows TMA, the plain-FMA kernel otherwise) or fp32 (plain-FMA GEMMs only, no reduced-precision tensor mode).
+the shape allows TMA, the plain-FMA kernel otherwise) or fp32 (plain FMAs, or for many tokens three bf16 terms a value on the
+tensor cores with an error no larger than theirs; no reduced-precision tensor mode).
 Norm statistics, attention scores and probabilities, recurrent states and the residual stream are fp32 in both.
 """
 import dataclasses
@@ -144,6 +145,19 @@ def _aligned(t, n=16):
 ACT_NONE, ACT_GELU, ACT_RELU2, ACT_SILU_GLU, ACT_GELU_ERF = 0, 1, 2, 3, 6
 
 
+def _linear_fp32_split(x, w, out, bias, accumulate, scale):
+    """fp32 products of many tokens on the tensor cores (three bf16 terms a value); False where the plain-FMA form is faster or has to take the call."""
+    T, K = x.shape
+    F = w.shape[0]
+    need = _lib.lib().pg_gemm_fp32_scratch(T, F, K)
+    if not need or (x.stride(0) | w.stride(0) | out.stride(0)) % 4 or not (x.is_cuda and w.is_cuda and _aligned(x) and _aligned(w) and _aligned(out)):
+        return False
+    scratch = torch.empty(need, device=x.device, dtype=torch.uint8)
+    _lib.check(_lib.lib().pg_gemm_fp32_split(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), _lib.ptr(bias), accumulate, scale,
+                                             T, F, K, scratch.data_ptr(), need, _lib.stream()), "pg_gemm_fp32_split")
+    return True
+
+
 def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: int = ACT_NONE, bias: Optional[torch.Tensor] = None):
     """out[t, f] = act(sum_k x[t, k] w[f, k] + bias[f]) (bias fp32 or None).  x, w share a type (bf16 / fp32); out is bf16 or fp32.  bf16 operands go to the
     tcgen05 kernel when TMA can describe them (16-byte pitches and bases), everything else to the plain-FMA kernel.
@@ -165,8 +179,10 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: int = ACT_N
         return _lib.gemm(x, w, out, mode=_lib.EPI_F32 if out.dtype == torch.float32 else _lib.EPI_BF16, swap=1 if T <= 128 else 0, bias=bias)
     if x.dtype == torch.float32 and out.dtype != torch.float32:
         raise ValueError("fp32 operands produce fp32 outputs")
-    if bias is not None:
-        assert bias.dtype == torch.float32 and bias.numel() == F and bias.is_contiguous()
+    assert bias is None or (bias.dtype == torch.float32 and bias.numel() == F and bias.is_contiguous())
+    if x.dtype == torch.float32 and _linear_fp32_split(x, w, out, bias, 0, 1.0):
+        pass
+    elif bias is not None:
         _lib.check(_lib.lib().pg_gemm_simt_bias(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), bias.data_ptr(), 0, 1.0,
                                                 T, F, K, int(x.dtype == torch.float32), int(out.dtype == torch.float32), _lib.stream()), "pg_gemm_simt_bias")
     else:
@@ -191,6 +207,8 @@ def linear_add(x: torch.Tensor, w: torch.Tensor, resid: torch.Tensor, bias: Opti
             and _aligned(resid)):
         return _lib.gemm_residual(x, w, resid, bias=bias, scale=float(scale))
     assert bias is None or (bias.dtype == torch.float32 and bias.numel() == F and bias.is_contiguous())
+    if x.dtype == torch.float32 and _linear_fp32_split(x, w, resid, bias, 1, float(scale)):
+        return resid
     _lib.check(_lib.lib().pg_gemm_simt_bias(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), resid.data_ptr(), resid.stride(0), _lib.ptr(bias), 1, float(scale),
                                             T, F, K, int(x.dtype == torch.float32), 1, _lib.stream()), "pg_gemm_simt_bias")
     return resid
