@@ -676,6 +676,17 @@ int pg_moe_gather_rows(const void* x, long long ldx, const int* sorted_pair, con
 int pg_moe_products(const void* x, long long ldx, const int* sorted_pair, const int* total_rows, int top, void* xg, const void* w_up, const void* w_down, void* mid,
                     float* eo, const int* plan, int max_tiles, int pairs, int n_real, int D, int F, int act, void* stream);
 
+/* A whole routed feed-forward of few rows (bf16): router product, choice, plan, grouped expert products (pg_moe_products), shared expert
+ * w_down relu(w_up h)^2 (NULL: none; shared_gate: times sigmoid of router column n_all) and the weighted sum, y (+)=.  router [n_pad, D], w_up [n_real, F (2 F for act 3), D],
+ * w_down [n_real, D, F].  scratch: pg_routed_ff_scratch bytes on a 256-byte boundary. */
+typedef struct {
+  const void *router, *w_up, *w_down, *shared_up, *shared_down;
+  const float *correction, *router_b;
+  int tokens, D, F, shared_F, n_all, n_real, n_pad, top, group_count, group_keep, flags, act, shared_gate;
+  float scale;
+} PgRoutedFf;
+long long pg_routed_ff_scratch(const PgRoutedFf* a);
+int pg_routed_ff(const PgRoutedFf* a, const void* h, long long ldh, float* y, int accumulate, void* scratch, long long scratch_bytes, void* stream);
 /* Per-expert dense products over the gathered runs: expert e owns the next counts_host[e] rows (host array, n_real entries);
  * mid[rows, F] = act(xg W_up[e]^T) in bf16, eo[rows, D] = mid W_down[e]^T in fp32, both through pg_gemm_bf16.  bf16 only;
  * D, F and the pitches multiples of 8.  act: 2 relu(x)^2, 6 gelu (erf form); 3: w_up holds [n_real, 2F, D] with gate and up rows in blocks of 64

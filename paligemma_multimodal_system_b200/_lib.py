@@ -75,6 +75,8 @@ SIGNATURES = {
     "pg_geglu": [p, i64, p, i64, i32, i32, i32, p],
     "pg_gemm_fp32_scratch": [i32, i32, i32],
     "pg_gemm_fp32_split": [p, i64, p, i64, p, i64, p, i32, f32, i32, i32, i32, p, i64, p],
+    "pg_routed_ff_scratch": [p],
+    "pg_routed_ff": [p, p, i64, p, i32, p, i64, p],
     "pg_token_side": [p, p, p, p, i64, i32, p, p, p, p, i32, i32, i32, i32, f32, i32, p],
     "pg_side_gate": [p, i64, p, p, i64, i32, p, i64, i32, i32, i32, i32, p],
     "pg_attn_prepare": [p, i64, p, p, p, i32, i32, p, p, p, p, p, p, i32, i32, i32, i32, i32, i32, f32, i32, i32, i32, f32, p, i64, f32, i32, p],
@@ -119,7 +121,7 @@ SIGNATURES = {
     "pg_gated_layernorm_add": [p, i64, p, i64, p, p, p, p, p, p, p, i32, i32, f32, i32, i32, p],
     "pg_glu": [p, i64, p, i64, i32, i32, i32, f32, f32, i32, p],
 }
-_RESTYPE = {"pg_launch_count": i64, "pg_gemm_fp32_scratch": i64}
+_RESTYPE = {"pg_launch_count": i64, "pg_gemm_fp32_scratch": i64, "pg_routed_ff_scratch": i64}
 
 
 
@@ -127,6 +129,13 @@ class AttnScore(C.Structure):
     """Mirror of PgAttnScore (include/paligemma_b200.h): the optional parts of an attention's score and mask."""
     _fields_ = [("window", i32), ("keep_first", i32), ("sink", p), ("dist_a", p), ("dist_b", p), ("head_scale", p), ("logistic", i32),
                 ("head_bias", p), ("out_scale", f32), ("out_ld", i64)]
+
+
+class RoutedFf(C.Structure):
+    """Mirror of PgRoutedFf (include/paligemma_b200.h)."""
+    _fields_ = ([(n, p) for n in ("router", "w_up", "w_down", "shared_up", "shared_down", "correction", "router_b")]
+                + [(n, i32) for n in ("tokens", "D", "F", "shared_F", "n_all", "n_real", "n_pad", "top", "group_count", "group_keep", "flags", "act", "shared_gate")]
+                + [("scale", f32)])
 
 
 class LinearAttnOps(C.Structure):

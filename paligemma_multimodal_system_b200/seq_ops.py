@@ -646,6 +646,17 @@ def moe_combine(expert_out, plan: MoePlan, ids, weights, h, shared_out, y, share
     return y
 
 
+def routed_ff(h, form, y, accumulate):
+    """A whole routed feed-forward by one call (_lib.RoutedFf names the weights and sizes); y fp32 [T, D]."""
+    import ctypes as C
+    assert h.is_cuda and h.dtype == torch.bfloat16 and h.stride(1) == 1 and h.shape == (form.tokens, form.D) and y.dtype == torch.float32 and y.is_contiguous() and y.shape == h.shape
+    need = _lib.lib().pg_routed_ff_scratch(C.addressof(form))
+    scratch = torch.empty(need, device=h.device, dtype=torch.uint8)
+    _lib.check(_lib.lib().pg_routed_ff(C.addressof(form), h.data_ptr(), h.stride(0), y.data_ptr(), int(bool(accumulate)), scratch.data_ptr(), need, _lib.stream()),
+               "pg_routed_ff")
+    return y
+
+
 COMBINE_NORM_MAX_WIDTH = 12288  # a row of sums stays in shared memory
 
 
