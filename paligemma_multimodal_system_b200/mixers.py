@@ -504,17 +504,18 @@ class LatentAttention:
         explicit = (self.explicit_prefill and not prec.f32 and b.singles < b.E and (dim + rot, vdim) in seq_ops.MMA_HEAD_SIZES
                     and R % 8 == 0 and (H * (dim + vdim)) % 8 == 0 and b.dense_pages is not None)
         if not explicit or b.singles:
-            # absorbed form; beside the explicit one it serves the single-token entries only (it still forms the absorbed query
-            # of every row: a mixed step is at most a few hundred rows)
+            # absorbed form; beside the explicit one it serves the single-token entries only, so only the rows between which they lie get an absorbed query
+            # (two portions of 333 tokens beside 40 decoding requests: the two products around the attention 48 -> 11 us)
+            r0, r1 = b.single_rows if explicit and b.single_rows is not None else (0, T)
             qlat = prec.empty(T, H, kd)
-            seq_ops.linear_batched(q[:, :, :dim], self.w_ukT, qlat[:, :, :R])
-            seq_ops.rotate_heads(q[:, :, dim:], qlat[:, :, R:], b.pos, self.freq_d, self.rot_dims, self.rot_gain)
+            seq_ops.linear_batched(q[r0:r1, :, :dim], self.w_ukT, qlat[r0:r1, :, :R])
+            seq_ops.rotate_heads(q[r0:r1, :, dim:], qlat[r0:r1, :, R:], b.pos[r0:r1], self.freq_d, self.rot_dims, self.rot_gain)
             olat = prec.empty(T, H, R)
             seq_ops.attn_ragged(qlat.view(T, H * kd), pages, pages, gate if per_head else None, olat.view(T, H * R), b, H, 1, kd, R, self.scale, 0.0, PAGE,
                                 krow=kd, vrow=kd, gate_per_head=True, only_singles=explicit, score=self.score)
-            seq_ops.linear_batched(olat, self.w_uv, att)
+            seq_ops.linear_batched(olat[r0:r1], self.w_uv, att[r0:r1])
             if not per_head:  # the gate has the values' width: it multiplies after the value up projection
-                seq_ops.sigmoid_gate_mul(att.view(T, H * vdim), gate)
+                seq_ops.sigmoid_gate_mul(att.view(T, H * vdim)[r0:r1], gate[r0:r1])
         if explicit:
             # explicit heads for the multi-token entries (their rows of `att` are written last)
             kx, vx = seq_ops.latent_expand(pages, b, self.w_ukv, H, dim, rot, vdim, R, PAGE, prec)

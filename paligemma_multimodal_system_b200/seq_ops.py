@@ -42,6 +42,7 @@ class StepBatch:
     max_pages: int
     singles: int = 0          # entries with one new token (decode rows)
     max_single_ctx: int = 0   # the longest context among them
+    single_rows: Optional[tuple] = None  # (first, one past the last) row between which all of them lie; None: unknown
     # dense scratch layout of the entries with several new tokens (mixers that rebuild per-head keys / values from a compact
     # cache): entry e owns rows [dense_row0[e], + ctx + n) of a dense matrix, starting on a page boundary, so that
     # dense_pages[e] = consecutive page numbers is a page table over the scratch and the paged attention kernels read it
@@ -53,6 +54,16 @@ class StepBatch:
     # what one layer of the CURRENT step leaves for later ones (rotation tables, a layer's values); a model that uses it starts every step
     # with a fresh one (`step_scope`)
     shared: Optional[dict] = None
+
+
+def _single_rows(ns):
+    """The rows between which the entries of one new token lie."""
+    first, last, r = None, 0, 0
+    for k in ns:
+        if k == 1:
+            first, last = r if first is None else first, r + 1
+        r += k
+    return None if first is None else (first, last)
 
 
 def make_step_batch(entries: Sequence[dict]) -> StepBatch:
@@ -94,7 +105,7 @@ def make_step_batch(entries: Sequence[dict]) -> StepBatch:
     return StepBatch(T=T, E=E, max_n=max(ns), tokens=dev[:T], pos=dev[T:2 * T], row_entry=dev[2 * T:3 * T], row0=dev[o:o + E],
                      n=dev[o + E:o + 2 * E], ctx=dev[o + 2 * E:o + 3 * E], slot=dev[o + 3 * E:o + 4 * E],
                      page_table=dev[o + 4 * E:o2].view(E, max_pages), max_pages=max_pages, singles=sum(k == 1 for k in ns),
-                     max_single_ctx=max([e["ctx"] for e, k in zip(entries, ns) if k == 1], default=0),
+                     max_single_ctx=max([e["ctx"] for e, k in zip(entries, ns) if k == 1], default=0), single_rows=_single_rows(ns),
                      dense_row0=dev[o2:o2 + E], dense_pages=dev[o2 + E:].view(E, dmax), dense_max_pages=dmax, dense_rows=page0 * 64,
                      dense_max_len=max(lens))
 

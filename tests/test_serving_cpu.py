@@ -131,3 +131,11 @@ def test_oracle_matches_reference_on_ragged_requests(regime):
         assert toks[0].tolist() == G[f"{regime}_tokens"][r].tolist()
         ref = torch.as_tensor(G[f"{regime}_prefill_logits"][r])
         assert (logits[0, 0] - ref).abs().max().item() <= 2e-5 * max(ref.abs().max().item(), 1.0)
+
+
+def test_rows_between_which_the_single_tokens_lie():
+    from paligemma_multimodal_system_b200.seq_ops import _single_rows
+    assert _single_rows([333, 333, 1, 1, 1]) == (666, 669)
+    assert _single_rows([1, 5, 1, 7]) == (0, 7)
+    assert _single_rows([1]) == (0, 1)
+    assert _single_rows([2, 9]) is None
