@@ -1,6 +1,8 @@
 // Causal attention of prompt portions over the paged bf16 cache on the tensor cores, with the probabilities kept at fp32
 // precision.
 //
+// (What prompts usually are runs in seq_attention_tc.cu on tensor memory; this kernel is for logistic weights, distance penalties, other page and head sizes.)
+//
 // The design asks for scores and probabilities in 32 bits.  q and k are bf16 here (they are stored so), so S = Q K^T from
 // bf16 x bf16 products accumulated in fp32 is exact to fp32 rounding.  The probabilities P = exp(s - m) stay fp32 in
 // registers; for P V each is cut into THREE bf16 terms p = p1 + p2 + p3 (8 + 8 + 8 mantissa bits) and the product is three
@@ -9,8 +11,7 @@
 //
 // CTA = 64 query rows (token x query head of one k/v head) of one entry, 4 warps x 16 rows; keys in tiles of 64.
 // mma.sync.m16n8k16 fragments: S accumulators of two adjacent 8-key blocks are, element for element, the A operand of one
-// 16-key step of P V, so P never leaves the registers.  (tcgen05 would want P in shared or tensor memory as bf16; three
-// passes from there cost the round trips this kernel avoids.)
+// 16-key step of P V, so P never leaves the registers.  
 //
 // What bounds it: instruction issue (ncu: 47 % of the slots, 16 warps per SM by registers) beside a tensor pipe at half its mma.sync rate.  So what
 // is not arithmetic is kept out of the key loop: one page lookup per tile, a tile ahead, with constant row steps (a division and a lookup per
@@ -22,6 +23,11 @@
 #include "paligemma_b200.h"
 
 using bf16 = __nv_bfloat16;
+
+// seq_attention_tc.cu
+int pg_attn_ragged_tc(const void* q, const void* kp, const void* vp, const void* gate, long long ldg, void* out, const int* row0, const int* n, const int* ctx, const int* pt,
+                      int max_pages, int page, int entries, int max_n, int H, int G, int dim, int vdim, float scale, float softcap, int skip_single, int gate_per_head,
+                      const PgAttnScore& sx, cudaStream_t st);
 
 namespace {
 
@@ -584,6 +590,9 @@ extern "C" int pg_attn_ragged_mma(const void* q, const void* k_pages, const void
       (gate != nullptr && !gate_per_head && ((reinterpret_cast<uintptr_t>(gate) & 3) || (ldg & 1))))
     return PG_ERR_ARG;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const int rc = pg_attn_ragged_tc(q, k_pages, v_pages, gate, ldg, out, entry_row0, entry_n, entry_ctx, page_table, max_pages, page, entries, max_n, H, G, dim, vdim, scale,
+                                   softcap, skip_single, gate_per_head, sx, st);
+  if (rc != 1) return rc;
 #define PG_MMA(D, V) \
   if (dim == D && vdim == V) \
     return launch<D, V>(q, k_pages, v_pages, gate, ldg, out, entry_row0, entry_n, entry_ctx, page_table, max_pages, page, entries, max_n, H, G, scale, \

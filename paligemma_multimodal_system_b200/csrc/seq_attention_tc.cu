@@ -1,0 +1,430 @@
+// Causal attention of prompt portions over the paged bf16 cache on the 5th-generation tensor cores, fp32 probabilities kept (the design notes of
+// seq_attention_mma.cu hold: P is cut into three bf16 terms exactly, P V is three passes).  This kernel takes what prompts usually are -- pages of 64 keys (or a
+// multiple, or 8, 16, 32), softmax scores with nothing but scale, soft cap, window and kept first keys -- and leaves logistic weights, distance penalties and other
+// page sizes to that one.
+//
+// CTA = 128 query rows (token x query head of one k/v head) of one entry, keys in tiles of 64, two CTAs per SM.  Warp 0 brings pages in by TMA, warp 1 issues
+// every tcgen05.mma, warps 2 .. 5 are the softmax, a thread per query row:
+//   * S = Q K^T: 128 x 64 into tensor memory; a thread reads its row of 64 scores, masks, exponentiates -- no exchange between lanes, the row sum is its own;
+//   * P goes back to tensor memory as three 32-column bf16 tiles and is the A operand of P V from there (12 instructions a tile): it never passes through shared memory;
+//   * S of the next tile is multiplied while this tile's exponentials run (values 64 wide; for 128 the 256 columns of a CTA leave no room for S beside P);
+//   * O is rescaled only when a row's maximum grew by more than 2^8 (fp32 sums have the room).
+// What bounds it: the softmax's ~10 instructions a score and the 16 UMMAs of N = 64 a tile, about balanced; mma.sync paid twice the instructions for fragments and splits and
+// ran its three passes at a quarter of this rate.  us, mma.sync / here: 8 prompts of 897 .. 1024 tokens, 32 heads x 64 over 8 k/v heads 235 / 149; 2 portions of 333
+// tokens behind 1400, 32 heads x 96 / 64: 144 / 66.
+#include "common.cuh"
+#include "paligemma_b200.h"
+#include "tmap.cuh"
+
+using bf16 = __nv_bfloat16;
+
+namespace pg {
+namespace {
+
+constexpr int kThreads = 192, kBox = 64 * 128;  // a box: 64 keys x 64 columns
+constexpr float kLog2e = 1.4426950408889634f;
+
+// D[tmem] (+)= A[tmem] * B[smem desc]: 128 x 16 bf16 A in 8 columns (two k values a column)
+PG_DEVINL void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+PG_DEVINL void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]),
+      "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+PG_DEVINL void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// MN-major operand as TMA lays it out ([k rows][64 columns], 128B swizzle); 64-column boxes `box` bytes apart
+PG_DEVINL uint64_t make_sdesc_mn_sw128(uint32_t addr, uint32_t box) {
+  uint64_t d = 0;
+  d |= static_cast<uint64_t>((addr & 0x3FFFF) >> 4);
+  d |= static_cast<uint64_t>((box >> 4) & 0x3FFF) << 16;
+  d |= static_cast<uint64_t>(1024 >> 4) << 32;
+  d |= static_cast<uint64_t>(1) << 46;
+  d |= static_cast<uint64_t>(2) << 61;
+  return d;
+}
+
+PG_DEVINL float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// as in seq_attention_mma.cu: tanh to fp32 accuracy, and the exact split by byte permutation
+PG_DEVINL float tanh32(float x) {
+  const float ax = fabsf(x), x2 = x * x;
+  const float small = x * fmaf(x2, fmaf(x2, 0.13333333f, -0.33333334f), 1.0f);
+  const float big = copysignf(1.0f - __fdividef(2.0f, ex2(ax * 2.885390082f) + 1.0f), x);
+  return ax < 0.1f ? small : big;
+}
+PG_DEVINL void split3(float p, float q, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  const uint32_t up = __float_as_uint(p), uq = __float_as_uint(q);
+  hi = __byte_perm(up, uq, 0x7632);
+  const float rp = p - __uint_as_float(up & 0xffff0000u), rq = q - __uint_as_float(uq & 0xffff0000u);
+  const uint32_t vp = __float_as_uint(rp), vq = __float_as_uint(rq);
+  mid = __byte_perm(vp, vq, 0x7632);
+  const float sp = rp - __uint_as_float(vp & 0xffff0000u), sq = rq - __uint_as_float(vq & 0xffff0000u);
+  lo = __byte_perm(__float_as_uint(sp), __float_as_uint(sq), 0x7632);
+}
+
+template <int DIM, int VDIM>
+struct Shape {
+  static constexpr int KB = (DIM + 63) / 64, VB = VDIM / 64;     // 64-column boxes of a key / value tile
+  static constexpr int Q_BYTES = KB * 128 * 128, KV_BYTES = (KB + VB) * kBox;
+  static constexpr int STAGES = (112 * 1024 - Q_BYTES - 256) / KV_BYTES < 4 ? (112 * 1024 - Q_BYTES - 256) / KV_BYTES : 4;
+  static constexpr int SMEM = Q_BYTES + STAGES * KV_BYTES + 256;
+  static constexpr bool ALIAS = VDIM > 64;                       // P over S
+  static constexpr int COL_P = ALIAS ? 0 : 64, COL_O = COL_P + 96;
+  static_assert(COL_O + VDIM <= 256 && STAGES >= 2 && DIM % 16 == 0 && VDIM % 64 == 0, "two CTAs per SM");
+};
+
+template <int DIM, int VDIM>
+__global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
+                                                                     const bf16* __restrict__ q, const bf16* __restrict__ gate, long long ldg, bf16* __restrict__ out,
+                                                                     const int* __restrict__ entry_row0, const int* __restrict__ entry_n, const int* __restrict__ entry_ctx,
+                                                                     const int* __restrict__ page_table, int max_pages, int page, int H, int G, float scale, float softcap,
+                                                                     int skip_single, int gate_per_head, PgAttnScore sx) {
+  using C = Shape<DIM, VDIM>;
+  constexpr uint32_t IDESC_S = make_idesc_bf16(128, 64), IDESC_O = make_idesc_bf16(128, VDIM, 0, 1);
+  griddep_wait();
+  const int e = blockIdx.z, g = blockIdx.y, gsz = H / G;
+  const int n = entry_n[e], ctx = entry_ctx[e], row0 = entry_row0[e];
+  const int rows = n * gsz, r0 = (gridDim.x - 1 - blockIdx.x) * 128;  // the longest rows start first
+  if ((skip_single && n == 1) || r0 >= rows) return;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const uint32_t base = smem_u32(smem);
+  if ((base & 1023u) != 0) __trap();
+  const uint32_t kv0 = base + C::Q_BYTES, bar0 = kv0 + C::STAGES * C::KV_BYTES;
+  auto kv_full = [&](int s) { return bar0 + 8u * s; };
+  auto kv_empty = [&](int s) { return bar0 + 8u * (4 + s); };
+  const uint32_t s_full = bar0 + 64, s_empty = bar0 + 72, p_full = bar0 + 80, o_done = bar0 + 88, tmem_slot = bar0 + 96;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&tmK);
+    tma_prefetch_desc(&tmV);
+    for (int s = 0; s < C::STAGES; ++s) {
+      mbar_init(kv_full(s), 1);
+      mbar_init(kv_empty(s), 1);
+    }
+    mbar_init(s_full, 1);
+    mbar_init(s_empty, 4);
+    mbar_init(p_full, 4);
+    mbar_init(o_done, 1);
+    mbar_fence_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 256);
+    tmem_relinquish();
+  }
+  // query rows, swizzled as TMA would lay them (zeros past the end and past DIM)
+  for (int id = threadIdx.x; id < 128 * C::KB * 8; id += kThreads) {
+    const int r = id / (C::KB * 8), cc = id % (C::KB * 8), rr = r0 + r;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (rr < rows && cc * 8 < DIM)
+      v = *reinterpret_cast<const uint4*>(q + static_cast<long long>(row0 + rr / gsz) * (static_cast<long long>(H) * DIM) + static_cast<long long>(g * gsz + rr % gsz) * DIM + cc * 8);
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(base + (cc >> 3) * (128 * 128) + r * 128 + (((cc & 7) ^ (r & 7)) << 4)), "r"(v.x), "r"(v.y), "r"(v.z),
+                 "r"(v.w) : "memory");
+  }
+  fence_proxy_async_smem();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  griddep_launch_dependents();  // (tensor memory is held)
+  uint32_t tmem;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot) : "memory");
+
+  const int last_row = min(rows, r0 + 128) - 1, kmax = ctx + last_row / gsz;  // last key any row of the CTA sees
+  const int window = sx.window > 0 ? sx.window : 0x3fffffff, keep = sx.window > 0 ? max(sx.keep_first, 0) : 0;
+  const int keep_end = (keep + 63) & ~63, cta_lo = max(0, ctx + r0 / gsz - window + 1) & ~63;
+  // key tiles wholly between the kept first keys and the first key inside the window of the CTA's first row are skipped
+  auto next_tile = [&](int k) {
+    const int nx = k + 64;
+    return (nx >= keep_end && nx < cta_lo) ? cta_lo : nx;
+  };
+  const int k_first = next_tile(-64);
+
+  if (warp == 0) {
+    if (lane == 0) {
+      const int* pt = page_table + static_cast<long long>(e) * max_pages;
+      int stage = 0;
+      uint32_t phase = 0;
+      const int piece = min(page, 64);  // rows of a box: a tile is (part of) a page, or several pages (those past the last key are left out)
+      auto row_at = [&](int key) { return pt[key / page] * page + key % page; };
+      int first = row_at(k_first);
+      for (int k0 = k_first; k0 <= kmax;) {
+        const int nx = next_tile(k0), pieces = min(64, kmax + 1 - k0 + piece - 1) / piece;
+        int row = first;
+        if (nx <= kmax) first = row_at(nx);
+        const uint32_t sk = kv0 + stage * C::KV_BYTES;
+        mbar_wait(kv_empty(stage), phase ^ 1);
+        mbar_expect_tx(kv_full(stage), (C::KB + C::VB) * 128 * piece * pieces);
+        for (int i = 0; i < pieces; ++i) {
+          if (i > 0) row = row_at(k0 + i * piece);
+          const uint32_t dst = sk + i * piece * 128;
+#pragma unroll
+          for (int b = 0; b < C::KB; ++b) tma_load_2d(dst + b * kBox, &tmK, kv_full(stage), g * DIM + 64 * b, row, kEvictNormal);
+#pragma unroll
+          for (int b = 0; b < C::VB; ++b) tma_load_2d(dst + (C::KB + b) * kBox, &tmV, kv_full(stage), g * VDIM + 64 * b, row, kEvictNormal);
+        }
+        if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
+        k0 = nx;
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    auto issue_s = [&](uint32_t sk) {
+      if (elect_one()) {
+#pragma unroll
+        for (int k = 0; k < DIM / 16; ++k)
+          umma_f16(tmem, make_sdesc_k_sw128(base + (k >> 2) * (128 * 128)) + 2 * (k & 3), make_sdesc_k_sw128(sk + (k >> 2) * kBox) + 2 * (k & 3), IDESC_S, k > 0 ? 1u : 0u);
+        umma_commit(s_full);
+      }
+      __syncwarp();
+    };
+    int stage = 0, ahead = 0;  // stages of P V and of S
+    uint32_t ahead_phase = 0, par = 0;
+    mbar_wait(kv_full(0), 0);
+    tc_fence_after();
+    issue_s(kv0);
+    if (++ahead == C::STAGES) { ahead = 0; ahead_phase ^= 1; }
+    for (int k0 = k_first; k0 <= kmax; par ^= 1) {
+      const int nx = next_tile(k0);
+      const uint32_t sk = kv0 + stage * C::KV_BYTES, sv = sk + C::KB * kBox;
+      if (!C::ALIAS && nx <= kmax) {  // S of the next tile as soon as the softmax has read this one
+        mbar_wait(kv_full(ahead), ahead_phase);
+        mbar_wait(s_empty, par);
+        tc_fence_after();
+        issue_s(kv0 + ahead * C::KV_BYTES);
+        if (++ahead == C::STAGES) { ahead = 0; ahead_phase ^= 1; }
+      }
+      if (k0 + 63 > kmax) {  // the last tile: keys nobody sees weigh zero, whatever lies there
+        for (int r = kmax + 1 - k0 + lane; r < 64; r += 32)
+#pragma unroll
+          for (int b = 0; b < C::VB; ++b)
+#pragma unroll
+            for (int c = 0; c < 8; ++c) asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(sv + b * kBox + r * 128 + c * 16), "r"(0) : "memory");
+        fence_proxy_async_smem();
+        __syncwarp();
+      }
+      mbar_wait(p_full, par);
+      tc_fence_after();
+      if (elect_one()) {
+#pragma unroll
+        for (int term = 0; term < 3; ++term)
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            umma_f16_ts(tmem + C::COL_O, tmem + C::COL_P + term * 32 + k * 8, make_sdesc_mn_sw128(sv + k * 2048, kBox), IDESC_O, (k0 > k_first || term > 0 || k > 0) ? 1u : 0u);
+        umma_commit(kv_empty(stage));
+        umma_commit(o_done);
+      }
+      __syncwarp();
+      if (C::ALIAS && nx <= kmax) {  // P lies where S goes
+        mbar_wait(kv_full(ahead), ahead_phase);
+        mbar_wait(o_done, par);
+        tc_fence_after();
+        issue_s(kv0 + ahead * C::KV_BYTES);
+        if (++ahead == C::STAGES) { ahead = 0; ahead_phase ^= 1; }
+      }
+      if (++stage == C::STAGES) stage = 0;
+      k0 = nx;
+    }
+  } else {
+    const int qd = warp & 3, r = qd * 32 + lane, rr = r0 + r;
+    const uint32_t lanes = tmem + (static_cast<uint32_t>(qd * 32) << 16);
+    const bool there = rr < rows;
+    const int head = g * gsz + (there ? rr % gsz : 0);
+    const int lim = there ? ctx + rr / gsz : -1, lo = lim - window + 1;  // last and first key of the row's window
+    // keys of a tile that every row of the warp sees: up to the first row's position, from the last row's window on
+    const int wr = r0 + qd * 32;
+    const bool warp_whole = wr + 32 <= rows;
+    const int all_lim = ctx + wr / gsz, all_lo = ctx + (wr + 31) / gsz - window + 1;
+    const float sc = scale * (sx.head_scale != nullptr ? sx.head_scale[head] : 1.f);
+    const bool plain = !(softcap > 0.f) && sx.head_scale == nullptr && scale > 0.f;  // the maximum commutes with the scale, which rides on the exponent's FMA
+    const float unit = plain ? scale * kLog2e : kLog2e, in = softcap > 0.f ? sc / softcap : 0.f;
+    float m = -INFINITY, l = 0.f;
+    uint32_t par = 0;
+    for (int k0 = k_first; k0 <= kmax; k0 = next_tile(k0), par ^= 1) {
+      mbar_wait(s_full, par);
+      tc_fence_after();
+      float s[64];
+      {
+        uint32_t v[4][16];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) tmem_ld16(lanes + 16 * c, v[c]);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 64; ++i) s[i] = __uint_as_float(v[i >> 4][i & 15]);
+      }
+      if (!C::ALIAS) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(s_empty);
+      }
+      if (!plain) {
+        if (softcap > 0.f) {
+#pragma unroll
+          for (int i = 0; i < 64; ++i) s[i] = softcap * tanh32(s[i] * in);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 64; ++i) s[i] *= sc;
+        }
+      }
+      if (!(warp_whole && k0 + 63 <= all_lim && (k0 >= all_lo || k0 + 64 <= keep))) {
+        const int hi = lim - k0, lw = lo - k0, kp = keep - k0;
+#pragma unroll
+        for (int i = 0; i < 64; ++i)
+          if (!(i <= hi && (i >= lw || i < kp))) s[i] = -INFINITY;
+      }
+      float mx;
+      {
+        float m8[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) m8[i] = s[i];
+#pragma unroll
+        for (int i = 8; i < 64; ++i) m8[i & 7] = fmaxf(m8[i & 7], s[i]);
+        mx = fmaxf(fmaxf(fmaxf(m8[0], m8[1]), fmaxf(m8[2], m8[3])), fmaxf(fmaxf(m8[4], m8[5]), fmaxf(m8[6], m8[7]))) * unit;
+      }
+      const bool need = mx > m + 8.0f;  // (from -inf: every finite maximum)
+      const float mn = need ? mx : m;
+      const float alpha = need ? ex2(m - mn) : 1.0f, off = mn > -INFINITY ? -mn : 0.f;  // rows that see no key yet weigh nothing
+      m = mn;
+      float s4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int i = 0; i < 64; ++i) {
+        s[i] = ex2(fmaf(s[i], unit, off));
+        s4[i & 3] += s[i];
+      }
+      l = l * alpha + ((s4[0] + s4[1]) + (s4[2] + s4[3]));
+      if (k0 > k_first) {
+        mbar_wait(o_done, par ^ 1);  // P V of the tile before: P may be overwritten and O touched
+        tc_fence_after();
+        if (__any_sync(0xffffffffu, need)) {
+#pragma unroll 1
+          for (int c = 0; c < VDIM; c += 16) {
+            uint32_t v[16];
+            tmem_ld16(lanes + C::COL_O + c, v);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
+            tmem_st16(lanes + C::COL_O + c, v);
+          }
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        uint32_t a[16], b[16], c[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) split3(s[32 * h + 2 * i], s[32 * h + 2 * i + 1], a[i], b[i], c[i]);
+        tmem_st16(lanes + C::COL_P + 16 * h, a);
+        tmem_st16(lanes + C::COL_P + 32 + 16 * h, b);
+        tmem_st16(lanes + C::COL_P + 64 + 16 * h, c);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);
+    }
+    mbar_wait(o_done, par ^ 1);
+    tc_fence_after();
+    float osc = 1.f;
+    if (sx.sink != nullptr) {  // the sink joins the denominator once (m is in base-2 units)
+      const float sk = sx.sink[head] * kLog2e, mm = fmaxf(m, sk);
+      osc = exp2f(m - mm);
+      l = l * osc + exp2f(sk - mm);
+    }
+    const float inv = osc / l * (sx.out_scale != 0.f ? sx.out_scale : 1.f);
+    const long long t = row0 + (there ? rr / gsz : 0), ldo = sx.out_ld > 0 ? sx.out_ld : static_cast<long long>(H) * VDIM;
+    bf16* o = out + t * ldo + static_cast<long long>(head) * VDIM;
+    const bf16* gt = gate == nullptr ? nullptr : gate + t * ldg + (gate_per_head ? static_cast<long long>(head) : static_cast<long long>(head) * VDIM);
+    const float gh = gate != nullptr && gate_per_head ? 1.0f / (1.0f + expf(-__bfloat162float(*gt))) : 1.f;
+#pragma unroll 1
+    for (int c = 0; c < VDIM; c += 16) {
+      uint32_t v[16];
+      tmem_ld16(lanes + C::COL_O + c, v);
+      tmem_ld_wait();
+      if (there) {
+        float x[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) x[i] = __uint_as_float(v[i]) * inv;
+        if (gate != nullptr) {
+          if (gate_per_head) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) x[i] *= gh;
+          } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const float2 gg = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(gt + c)[i]);
+              x[2 * i] *= 1.0f / (1.0f + expf(-gg.x));
+              x[2 * i + 1] *= 1.0f / (1.0f + expf(-gg.y));
+            }
+          }
+        }
+        uint4* d = reinterpret_cast<uint4*>(o + c);
+        d[0] = make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
+        d[1] = make_uint4(pack_bf16(x[8], x[9]), pack_bf16(x[10], x[11]), pack_bf16(x[12], x[13]), pack_bf16(x[14], x[15]));
+      }
+      __syncwarp();
+    }
+    tc_fence_before();
+  }
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 256);
+  }
+}
+
+template <int DIM, int VDIM>
+int launch(const void* q, const void* kp, const void* vp, const void* gate, long long ldg, void* out, const int* row0, const int* n, const int* ctx, const int* pt,
+           int max_pages, int page, int entries, int max_n, int H, int G, float scale, float softcap, int skip_single, int gate_per_head, const PgAttnScore& sx,
+           cudaStream_t st) {
+  using C = Shape<DIM, VDIM>;
+  static bool configured[kMaxDevices] = {};
+  const int dev = current_device();
+  if (!configured[dev]) {
+    if (cudaFuncSetAttribute(attn_ragged_tc_kernel<DIM, VDIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess) {
+      cudaGetLastError();
+      return PG_ERR_CUDA;
+    }
+    configured[dev] = true;
+  }
+  // the pools as matrices of rows: only pages named by the table are read, so the row count is a bound and not a size
+  CUtensorMap tk, tv;
+  int rc;
+  if ((rc = make_tmap_2d(&tk, kp, 1LL << 30, static_cast<long long>(G) * DIM, static_cast<long long>(G) * DIM, page < 64 ? page : 64)) != PG_OK) return rc;
+  if ((rc = make_tmap_2d(&tv, vp, 1LL << 30, static_cast<long long>(G) * VDIM, static_cast<long long>(G) * VDIM, page < 64 ? page : 64)) != PG_OK) return rc;
+  launch_spread(attn_ragged_tc_kernel<DIM, VDIM>, dim3((max_n * (H / G) + 127) / 128, G, entries), dim3(kThreads), C::SMEM, st, tk, tv, static_cast<const bf16*>(q),
+                static_cast<const bf16*>(gate), ldg, static_cast<bf16*>(out), row0, n, ctx, pt, max_pages, page, H, G, scale, softcap, skip_single, gate_per_head, sx);
+  pg_count_launch(1);
+  return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
+}
+
+}  // namespace
+}  // namespace pg
+
+// Launches the call when it is one of this file's (PG_OK or an error), else returns 1.  Everything that pg_attn_ragged_mma checks has been checked.
+int pg_attn_ragged_tc(const void* q, const void* kp, const void* vp, const void* gate, long long ldg, void* out, const int* row0, const int* n, const int* ctx, const int* pt,
+                      int max_pages, int page, int entries, int max_n, int H, int G, int dim, int vdim, float scale, float softcap, int skip_single, int gate_per_head,
+                      const PgAttnScore& sx, cudaStream_t st) {
+  // pages that a tile of 64 keys divides, or that divide it in whole swizzle rows
+  if (!(page > 0 && (page % 64 == 0 || (page % 8 == 0 && 64 % page == 0))) || sx.logistic || sx.dist_a != nullptr || sx.out_ld % 8 != 0) return 1;
+#define PG_TC(D, V) \
+  if (dim == D && vdim == V) \
+    return pg::launch<D, V>(q, kp, vp, gate, ldg, out, row0, n, ctx, pt, max_pages, page, entries, max_n, H, G, scale, softcap, skip_single, gate_per_head, sx, st)
+  PG_TC(64, 64);
+  PG_TC(96, 64);
+  PG_TC(128, 128);
+  PG_TC(64, 128);
+  PG_TC(128, 64);
+#undef PG_TC
+  return 1;
+}

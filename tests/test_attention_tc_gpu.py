@@ -1,0 +1,87 @@
+"""Prompt attention on tensor memory where it can go wrong -- tiles of 128 rows and 64 keys, windows and kept first keys, every optional part of the score, pages whose
+unused rows hold NaNs -- against 64-bit sums.  Scores are sums of bf16 products in fp32 and probabilities keep 24 bits, so a result differs by its rounding to bf16
+(2^-9, bound 2^-8) and about 1e-5 of the values' scale; tanh32 adds 2e-7 of the cap to a score."""
+import math
+
+import pytest
+import torch
+
+from paligemma_multimodal_system_b200 import seq_ops
+
+pytestmark = pytest.mark.gpu
+
+
+def _t(*shape, seed, dtype=torch.bfloat16):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return torch.randn(*shape, generator=g, device="cuda").to(dtype)
+
+
+def _want(q, k, v, first, scale, softcap, window, keep, hs, sink):
+    """q [n, H, dim] at positions first .., k / v [L, G, .], in 64 bits."""
+    n, H, _ = q.shape
+    G, L = k.shape[1], k.shape[0]
+    kk, vv = (t.double().repeat_interleave(H // G, 1) for t in (k, v))
+    s = torch.einsum("ihd,jhd->hij", q.double(), kk) * scale
+    if hs is not None:
+        s = s * hs.double()[:, None, None]
+    if softcap:
+        s = softcap * torch.tanh(s / softcap)
+    i, j = torch.arange(first, first + n, device="cuda")[:, None], torch.arange(L, device="cuda")[None]
+    s = s.masked_fill(~((j <= i) & ((i - j < window) | (j < keep)) if window else j <= i), -math.inf)
+    if sink is not None:
+        s = torch.cat([s, sink.double()[:, None, None].expand(H, n, 1)], -1)
+    return torch.einsum("hij,jhd->ihd", torch.softmax(s, -1)[..., :L], vv)
+
+
+@pytest.mark.parametrize("dim,vdim,G,gsz", [(64, 64, 2, 4), (96, 64, 3, 1), (128, 128, 1, 4), (64, 128, 2, 3), (128, 64, 1, 5), (64, 64, 1, 129)])
+@pytest.mark.parametrize("ns,ctxs", [((2, 1, 33, 130), (0, 5, 63, 200)), ((300,), (0,)), ((64, 65), (64, 127)), ((5,), (1000,))])
+@pytest.mark.parametrize("window,keep", [(0, 0), (33, 0), (70, 5), (1, 1), (512, 130)])
+def test_masks(dim, vdim, G, gsz, ns, ctxs, window, keep):
+    _run(dim, vdim, G, gsz, ns, ctxs, window, keep)
+
+
+@pytest.mark.parametrize("dim,vdim", [(64, 64), (96, 64), (128, 128)])
+@pytest.mark.parametrize("opts", [dict(softcap=5.0), dict(hs=True), dict(sink=True), dict(gate="row"), dict(gate="head"), dict(ld=True), dict(softcap=3.0, hs=True, sink=True, gate="head", ld=True),
+                                  dict(scale=-0.1), dict(big=True)])
+def test_options(dim, vdim, opts):
+    _run(dim, vdim, 2, 2, (70, 1, 129), (0, 9, 77), 100, 3, **opts)
+
+
+def _run(dim, vdim, G, gsz, ns, ctxs, window, keep, softcap=0.0, hs=False, sink=False, gate=None, ld=False, scale=None, big=False):
+    H, scale = G * gsz, dim ** -0.5 if scale is None else scale
+    rows, first = [], 0
+    for i, (n, c) in enumerate(zip(ns, ctxs)):
+        p = (n + c + 63) // 64
+        rows.append(dict(tokens=[1] * n, ctx=c, slot=i, pages=list(range(first, first + p))[::-1]))
+        first += p
+    b = seq_ops.make_step_batch(rows)
+    kp = torch.full((first, 64, G * dim), float("nan"), device="cuda", dtype=torch.bfloat16)
+    vp = torch.full((first, 64, G * vdim), float("nan"), device="cuda", dtype=torch.bfloat16)
+    q = _t(b.T, H * dim, seed=1) * (30 if big else 1)  # (big: maxima that grow from tile to tile)
+    ks, vs = [], []
+    for i, (n, c) in enumerate(zip(ns, ctxs)):
+        k, v = _t(n + c, G * dim, seed=10 + i), _t(n + c, G * vdim, seed=20 + i)
+        if big:
+            k = (k * torch.linspace(0.1, 3, n + c, device="cuda")[:, None]).to(torch.bfloat16)
+        for j, p in enumerate(rows[i]["pages"]):
+            part = slice(64 * j, min(64 * j + 64, n + c))
+            kp[p, : part.stop - part.start], vp[p, : part.stop - part.start] = k[part], v[part]
+        ks.append(k.view(-1, G, dim))
+        vs.append(v.view(-1, G, vdim))
+    hst = torch.linspace(-0.7, 1.5, H, device="cuda") if hs else None
+    skt = torch.linspace(-2, 3, H, device="cuda") if sink else None
+    pitch = H * vdim + 8 if ld else H * vdim
+    out = torch.full((b.T, pitch), 7.0, device="cuda", dtype=torch.bfloat16)
+    g = None if gate is None else _t(b.T, H if gate == "head" else H * vdim, seed=5)
+    score = seq_ops.ScoreOptions(H, window or None, keep, sink=skt, head_scale=hst, out_scale=0.5 if ld else 1.0, out_ld=pitch if ld else 0)
+    seq_ops.attn_ragged(q, kp, vp, g, out, b, H, G, dim, vdim, scale, softcap, 64, gate_per_head=gate == "head", score=score, decode_kernel=False)
+    r = 0
+    for i, (n, c) in enumerate(zip(ns, ctxs)):
+        want = _want(q[r:r + n].view(n, H, dim), ks[i], vs[i], c, scale, softcap, window, keep, hst, skt) * (0.5 if ld else 1.0)
+        if g is not None:
+            want = want * torch.sigmoid(g[r:r + n].double()).view(n, H, -1)
+        got = out[r:r + n, : H * vdim].double().view(n, H, vdim)
+        assert ((got - want).abs() <= want.abs() * 2.0 ** -8 + (2e-4 if big else 5e-5)).all(), (i, (got - want).abs().max().item())
+        r += n
+    if ld:
+        assert (out[:, H * vdim:] == 7).all()
