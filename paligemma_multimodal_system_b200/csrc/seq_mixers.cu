@@ -635,17 +635,30 @@ __global__ void attn_decode_merge_kernel(const float* __restrict__ partial, cons
   if (entry_n[e] != 1) return;
   const long long t = entry_row0[e];
   const float* pp = partial + ((long long)e * H + head) * nsplit * (vdim + 2);
-  float M = -INFINITY;
-  for (int s = 0; s < nsplit; ++s) M = fmaxf(M, pp[s * (vdim + 2)]);
+  // the splits' factors once, a lane per split; then every column's loads are independent (a chain of three loads per split and column took 15.7 us for 40 tokens x 32
+  // heads x 256 in 14 splits; now 13.9)
+  __shared__ float fs[64], whole[2];
+  if (threadIdx.x < 32) {
+    float mx = -INFINITY, sum = 0.f;
+    for (int s = threadIdx.x; s < nsplit; s += 32) mx = fmaxf(mx, pp[s * (vdim + 2)]);
+    mx = wmax(mx);
+    for (int s = threadIdx.x; s < nsplit; s += 32) {
+      const float ms = pp[s * (vdim + 2)], f = ms > -INFINITY ? expf(ms - mx) : 0.f;
+      if (s < 64) fs[s] = f;
+      if (f != 0.f) sum = fmaf(f, pp[s * (vdim + 2) + 1], sum);
+    }
+    sum = wsum(sum);
+    if (threadIdx.x == 0) { whole[0] = mx; whole[1] = sum; }
+  }
+  __syncthreads();
+  const float M = whole[0];
   for (int col = threadIdx.x; col < vdim; col += blockDim.x) {
-    float acc = 0.f, ls = 0.f;
+    float acc = 0.f, ls = whole[1];
+#pragma unroll 8
     for (int s = 0; s < nsplit; ++s) {
-      const float ms = pp[s * (vdim + 2)];
-      if (ms > -INFINITY) {
-        const float f = expf(ms - M);
-        acc = fmaf(f, pp[s * (vdim + 2) + 2 + col], acc);
-        ls = fmaf(f, pp[s * (vdim + 2) + 1], ls);
-      }
+      const float ms = s < 64 ? 0.f : pp[s * (vdim + 2)];
+      const float f = s < 64 ? fs[s] : ms > -INFINITY ? expf(ms - M) : 0.f;
+      acc = fmaf(f, f != 0.f ? pp[s * (vdim + 2) + 2 + col] : 0.f, acc);
     }
     if (sink != nullptr) {
       const float sk = sink[head], mm = fmaxf(M, sk), f = expf(M - mm);
