@@ -9,8 +9,8 @@
 //   * P goes back to tensor memory as three 32-column bf16 tiles and is the A operand of P V from there (12 instructions a tile): it never passes through shared memory;
 //   * S of the next tile is multiplied while this tile's exponentials run (values 64 wide; for 128 the 256 columns of a CTA leave no room for S beside P);
 //   * O is rescaled only when a row's maximum grew by more than 2^8 (fp32 sums have the room).
-// What bounds it: the softmax's ~10 instructions a score and the 16 UMMAs of N = 64 a tile, about balanced; mma.sync paid twice the instructions for fragments and splits and
-// ran its three passes at a quarter of this rate.  us, mma.sync / here: 8 prompts of 897 .. 1024 tokens, 32 heads x 64 over 8 k/v heads 235 / 149; 2 portions of 333
+// What bounds it: the softmax warps (clocks a tile, stamped: wait for S 100, its load 75, maxima and exponentials 1000 .. 1330, wait for P V 185, split 520; the products hide
+// behind them).  Two threads a row share the same pipes (146 us for 149), exponentials as polynomials on the FMA pipe cost more than they save (168).  us, mma.sync / here: 8 prompts of 897 .. 1024 tokens, 32 heads x 64 over 8 k/v heads 235 / 149; 2 portions of 333
 // tokens behind 1400, 32 heads x 96 / 64: 144 / 66.
 #include "common.cuh"
 #include "paligemma_b200.h"
