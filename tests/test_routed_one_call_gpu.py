@@ -47,6 +47,3 @@ def test_calls_that_keep_the_separate_launches():
     assert fits._one_call(h.float(), f32) is None
     assert fits._one_call(h.flatten()[4:4 + 39 * 512].view(39, 512), bf) is None  # off a 16-byte boundary
     assert fits._one_call(torch.zeros(600, 512, device="cuda", dtype=torch.bfloat16), bf) is None  # dense runs
-    none = _layer(512, 0, 4, 2, 256, 0)
-    none.pack(bf)
-    assert none._one_call(h, bf) is None and none(h, None, bf).shape == h.shape
