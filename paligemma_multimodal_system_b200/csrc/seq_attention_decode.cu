@@ -293,11 +293,18 @@ int launch(const void* q, const void* kp, const void* vp, const void* gate, long
            long long krow, long long vrow, int gate_per_head, const PgAttnScore& sx, cudaStream_t st) {
   const int gsz = H / G, dimp = (dim + 63) / 64 * 64;
   const size_t smem = ((size_t)gsz * dimp + kWarps * (128 + 8 + (size_t)4 * vdim)) * sizeof(float);
-  if (smem > 200 * 1024) return PG_ERR_ARG;
+  constexpr int kMost = 200 * 1024;
+  if (smem > kMost) return PG_ERR_ARG;
   auto kern = sx.logistic ? attn_decode_vec_kernel<TA, VC, true> : attn_decode_vec_kernel<TA, VC, false>;
-  if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-    cudaGetLastError();
-    return PG_ERR_CUDA;
+  // once a device, to the most that any call asks for: calls of several threads find the same
+  static bool configured[2][pg::kMaxDevices] = {};
+  bool& done = configured[sx.logistic ? 1 : 0][pg::current_device()];
+  if (!done) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost) != cudaSuccess) {
+      cudaGetLastError();
+      return PG_ERR_CUDA;
+    }
+    done = true;
   }
   return pg::launch_kernel(kern, dim3(nsplit, G, entries), dim3(32 * kWarps), smem, st, static_cast<const TA*>(q), static_cast<const TA*>(kp),
                            static_cast<const TA*>(vp), static_cast<const TA*>(gate), ldg, static_cast<TA*>(out), partial, row0, n, ctx, pt, max_pages, page, H, G,
