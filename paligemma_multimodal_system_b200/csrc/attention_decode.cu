@@ -4,8 +4,8 @@
 // One thread-block cluster per (sequence, kv head); every rank owns a contiguous range of 64-key pages that it pulls with
 // TMA tensor loads into 128B-swizzled shared memory.  The page loads are issued BEFORE griddepcontrol.wait: the cache
 // rows of earlier positions, kv_len and the page table were written by kernels that completed before this one could
-// start (every kernel of the decode chain waits on its predecessor before it triggers its dependents), only the fp32
-// qkv row of the new token comes from the immediately preceding GEMM.
+// start: what writes them either does not trigger its dependents at all (pg_rope_kv_append) or lies further back in the decode chain, whose
+// kernels trigger behind their own wait.  Only the fp32 qkv row of the new token comes from the immediately preceding GEMM.
 //
 // Work split inside a CTA (8 warps), chosen so that NO accumulator ever has to be merged across warps:
 //   scores : warp w computes Q K^T for keys [8w, 8w+8) of every resident page (mma.sync m16n8k16, Q fragments live in

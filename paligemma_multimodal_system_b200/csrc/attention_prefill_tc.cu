@@ -224,7 +224,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_gen;
   griddep_wait();
-  griddep_launch_dependents();  // (tensor memory is held by now: a product behind this kernel cannot take it first)
   // ragged batches: keys [key_lens[b], keys) of problem b exist in memory (padding tokens, finite values) but weigh nothing
   const int n_keys = p.key_lens ? max(1, min(p.keys, __ldg(p.key_lens + b))) : p.keys;
   const int n_tiles = (n_keys + BN - 1) / BN;

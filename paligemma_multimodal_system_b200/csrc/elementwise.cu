@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(128) rope_kv_append_kernel(const void* __restr
                                                              const int* __restrict__ slot_base, int tokens_per_seq, int Hq,
                                                              int Hkv, int dh, int page_size, int max_pages,
                                                              const float* __restrict__ inv_freq) {
-  pg::griddep_begin();
+  pg::griddep_begin();  // (writes pages: attn_decode_v3_kernel reads them ahead of its wait)
   const long long t = blockIdx.x;
   const int b = static_cast<int>(t / tokens_per_seq);
   const int half = dh / 2;

@@ -70,7 +70,6 @@ __global__ void __launch_bounds__(32 * kWarps, VC == 1 && sizeof(TA) == 2 ? 3 : 
                                                                          const int* __restrict__ entry_ctx, const int* __restrict__ page_table, int max_pages,
                                                                          int page, int H, int G, int dim, int vdim, float scale, float softcap, long long krow,
                                                                          long long vrow, int gate_per_head, PgAttnScore sx) {
-  if (sizeof(TA) == 2) pg::griddep_launch_dependents();  // (fp32: see griddep_begin)
   constexpr bool EARLY_V = VC == 1 && sizeof(TA) == 2;
   const int e = blockIdx.z, g = blockIdx.y, split = blockIdx.x, nsplit = gridDim.x, gsz = H / G;
   const int ctx = entry_ctx[e];

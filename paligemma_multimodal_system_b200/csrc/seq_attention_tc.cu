@@ -138,7 +138,6 @@ __global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __gri
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  griddep_launch_dependents();  // (tensor memory is held)
   uint32_t tmem;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot) : "memory");
 

@@ -229,13 +229,13 @@ __global__ void __launch_bounds__(256) group_rmsnorm_add_kernel(const float* __r
 }
 
 // The same for groups of whole 128 elements: a thread keeps its up to 4 NV elements of the row, so y, x and w are each requested once and together
-// (w ahead of the dependency wait), and one barrier separates the sums from the result.  What bounds it: decode steps, two round trips (48 rows of 2048 in a
+// and one barrier separates the sums from the result.  What bounds it: decode steps, two round trips (48 rows of 2048 in a
 // step: 4.1 -> 3.1 us); prompts, HBM (10836 rows: 70 us in either form).
 template <typename TO, int NV>
 __global__ void __launch_bounds__(256) group_rmsnorm_add_reg_kernel(const float* __restrict__ y, long long ldy, const float* __restrict__ w,
                                                                     float* __restrict__ x, TO* __restrict__ out_act, int D, int gs, float eps) {
   __shared__ float red[8 * NV];  // sums of 128 neighbouring elements
-  pg::griddep_launch_dependents();
+  pg::griddep_begin();
   const long long t = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float4 v[NV], ww[NV], xv[NV];
@@ -244,7 +244,6 @@ __global__ void __launch_bounds__(256) group_rmsnorm_add_reg_kernel(const float*
     const int i = threadIdx.x + 256 * k;
     if (4 * i < D) ww[k] = reinterpret_cast<const float4*>(w)[i];
   }
-  pg::griddep_wait();
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
     const int i = threadIdx.x + 256 * k;
@@ -320,13 +319,12 @@ __global__ void __launch_bounds__(256) rmsnorm_gate_kernel(const float* __restri
   }
 }
 
-// The same for rows of up to 4096 elements: a thread keeps its elements, so the row, the gate and the weights are requested together (the weights ahead of the
-// dependency wait) and the row once.  48 rows of 2048 in a step: 3.2 -> 2.7 us; 10836 rows: 55 in either form.
+// The same for rows of up to 4096 elements: a thread keeps its elements, so the row, the gate and the weights are requested together and the row once.  48 rows of 2048 in a step: 3.2 -> 2.7 us; 10836 rows: 55 in either form.
 template <typename TA, int NV>
 __global__ void __launch_bounds__(256) rmsnorm_gate_reg_kernel(const float* __restrict__ o, const float* __restrict__ w, const TA* __restrict__ gate,
                                                                long long ldg, TA* __restrict__ out, int D, float eps) {
   __shared__ float red[8];
-  pg::griddep_launch_dependents();
+  pg::griddep_begin();
   const long long t = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float4 v[NV], ww[NV], g[NV];
@@ -335,7 +333,6 @@ __global__ void __launch_bounds__(256) rmsnorm_gate_reg_kernel(const float* __re
     const int i = threadIdx.x + 256 * k;
     if (4 * i < D) ww[k] = reinterpret_cast<const float4*>(w)[i];
   }
-  pg::griddep_wait();
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
     const int i = threadIdx.x + 256 * k;

@@ -179,7 +179,6 @@ __global__ void __launch_bounds__(128) attn_prepare_vec_kernel(const TA* __restr
                                                                TA* __restrict__ v_pages, int rows, int H, int G, int dim, int vdim, int rot, float eps,
                                                                int norm_qk, int norm_v, int v_from_k, float rot_gain, const TA* __restrict__ v_other,
                                                                long long ldvo, float v_mix) {
-  pg::griddep_launch_dependents();
   extern __shared__ float cs[];  // [TOK][cos rot/2 | sin rot/2]
   __shared__ float part[2][TOK][4];
   const int t0 = blockIdx.x * TOK, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -294,7 +293,7 @@ __global__ void __launch_bounds__(256) attn_ragged_kernel(const TA* __restrict__
                                                           const int* __restrict__ entry_ctx, const int* __restrict__ page_table, int max_pages,
                                                           int page, int H, int G, int dim, int vdim, float scale, float softcap, int skip_single,
                                                           long long krow, long long vrow, int gate_per_head, int alias, PgAttnScore sx) {
-  pg::griddep_begin<sizeof(TA) == 2>();
+  pg::griddep_begin();
   const int e = blockIdx.z, g = blockIdx.y, gsz = H / G;
   const int n = entry_n[e], ctx = entry_ctx[e], row0 = entry_row0[e];
   if (skip_single && n == 1) return;
@@ -479,7 +478,7 @@ __global__ void __launch_bounds__(256) attn_decode_kernel(const TA* __restrict__
                                                           const int* __restrict__ entry_ctx, const int* __restrict__ page_table, int max_pages,
                                                           int page, int H, int G, int dim, int vdim, float scale, float softcap, long long krow,
                                                           long long vrow, int gate_per_head, PgAttnScore sx) {
-  pg::griddep_begin<sizeof(TA) == 2>();
+  pg::griddep_begin();
   constexpr int NO = 2 * VC;  // accumulator columns per lane
   const int e = blockIdx.z, g = blockIdx.y, split = blockIdx.x, nsplit = gridDim.x, gsz = H / G;
   if (entry_n[e] != 1) return;
@@ -627,7 +626,7 @@ template <typename TA>
 __global__ void attn_decode_merge_kernel(const float* __restrict__ partial, const TA* __restrict__ gate, long long ldg, TA* __restrict__ out,
                                          const int* __restrict__ entry_row0, const int* __restrict__ entry_n, int H, int vdim, int nsplit,
                                          int gate_per_head, PgAttnScore sx) {
-  pg::griddep_begin<sizeof(TA) == 2>();
+  pg::griddep_begin();
   const float* sink = sx.logistic ? nullptr : sx.sink;
   const long long ldo = sx.out_ld > 0 ? sx.out_ld : (long long)H * vdim;
   const float oscale = sx.out_scale != 0.f ? sx.out_scale : 1.f;
@@ -771,12 +770,10 @@ __global__ void __launch_bounds__(128, RP == 8 ? 7 : 3) linear_attn_scan_vec_ker
                                                                    const int* __restrict__ entry_row0, const int* __restrict__ entry_n,
                                                                    const int* __restrict__ entry_ctx, const int* __restrict__ entry_slot, int H,
                                                                    int dim, int vdim, PgLinearAttnOps ops) {
-  pg::griddep_launch_dependents();
   __shared__ float qs[8 * RP], ksm[8 * RP];
   __shared__ __align__(16) float red[8][64];
   const int e = blockIdx.z, h = blockIdx.y, vb = 64 * blockIdx.x;
   const int n = entry_n[e], row0 = entry_row0[e], slot = entry_slot[e], ctx = entry_ctx[e];
-  const float a = decay[h];
   const bool mine = n >= ops.n_min && n <= ops.n_max;
   const int rg = threadIdx.x >> 4, v = vb + 4 * (threadIdx.x & 15);
   const bool v_ok = v < vdim;
@@ -785,8 +782,9 @@ __global__ void __launch_bounds__(128, RP == 8 ? 7 : 3) linear_attn_scan_vec_ker
   // the state, on its way to L2 while the kernels before still run (only a hint: it is read behind the wait)
   if (mine && ctx != 0 && (threadIdx.x & 7) == 0 && v_ok)
     for (int d = rg; d < dim; d += 8) asm volatile("prefetch.global.L2 [%0];" ::"l"(st + d * pitch));
-  pg::griddep_wait();
+  pg::griddep_begin<true>();
   if (!mine) return;
+  const float a = decay[h];
   float4 S[RP];
 #pragma unroll
   for (int i = 0; i < RP; ++i) {
@@ -861,7 +859,7 @@ __global__ void __launch_bounds__(256, 2) linear_attn_chunked_kernel(const TA* _
                                                                   const int* __restrict__ entry_row0, const int* __restrict__ entry_n,
                                                                   const int* __restrict__ entry_ctx, const int* __restrict__ entry_slot, int H,
                                                                   int dim, int vdim, PgLinearAttnOps ops) {
-  pg::griddep_begin<sizeof(TA) == 2>();
+  pg::griddep_begin();
   constexpr int C = 32;
   const int e = blockIdx.z, h = blockIdx.y, vb = blockIdx.x;
   const int n = entry_n[e], row0 = entry_row0[e];

@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict_
                                                         int* __restrict__ ids, float* __restrict__ weights, int* __restrict__ counts, int T,
                                                         int n_all, int n_real, int top, int group_count, int group_keep, float scale,
                                                         const float* __restrict__ logit_bias, int flags) {
-  pg::griddep_begin();
+  pg::griddep_begin<true>();
   extern __shared__ float sm[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int t = blockIdx.x * 4 + warp;
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict_
 // One warp: 32 experts at a time, prefix sums of their counts and tile numbers by shuffles.
 __global__ void moe_plan_kernel(const int* __restrict__ counts, int* __restrict__ offsets, int* __restrict__ fill, int* __restrict__ plan, int n_real,
                                 int max_tiles) {
-  pg::griddep_begin();
+  pg::griddep_begin<true>();
   const int lane = threadIdx.x;
   int off = 0, nt = 0;
   for (int e0 = 0; e0 < n_real; e0 += 32) {
@@ -202,7 +202,7 @@ __global__ void moe_plan_kernel(const int* __restrict__ counts, int* __restrict_
 
 __global__ void moe_scatter_kernel(const int* __restrict__ ids, const int* __restrict__ offsets, int* __restrict__ fill, int* __restrict__ sorted_pair,
                                    int* __restrict__ pair_row, int pairs, int n_real) {
-  pg::griddep_begin();
+  pg::griddep_begin<true>();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= pairs) return;
   const int e = ids[p];
@@ -449,7 +449,7 @@ __global__ void moe_combine_kernel(const float* __restrict__ expert_out, long lo
                                    const float* __restrict__ weights, const TA* __restrict__ h, long long ldh, const float* __restrict__ shared_out,
                                    long long lds, float* __restrict__ y, int D, int top, const float* __restrict__ shared_gate, long long ldsg,
                                    int accumulate) {
-  pg::griddep_begin();
+  pg::griddep_begin<true>();
   const long long t = blockIdx.x;
   const float sgate = shared_gate != nullptr ? 1.0f / (1.0f + expf(-shared_gate[t * ldsg])) : 1.0f;
   for (int d = threadIdx.x; d < D; d += blockDim.x) {

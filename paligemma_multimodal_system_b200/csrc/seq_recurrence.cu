@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const TA* __restrict__ 
                                                          long long ldo, float* __restrict__ inv, int ldi, PgConvSections sec, int taps, int C,
                                                          const int* __restrict__ entry_row0, const int* __restrict__ entry_n,
                                                          const int* __restrict__ entry_ctx, const int* __restrict__ entry_slot, int chunk) {
-  pg::griddep_begin<sizeof(TA) == 2>();
+  pg::griddep_begin();
   const int e = blockIdx.z, lane = threadIdx.x & 31;
   const int n = entry_n[e], r0 = blockIdx.y * chunk;
   if (r0 >= n) return;
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(128) short_conv_vec_kernel(const bf16* __restr
 // ---------------------------------------------------------------------------------------------------------------------
 template <typename TA, int VEC, int RP>
 __global__ void __launch_bounds__(256) delta_scan_kernel(PgDeltaArgs a, int n_min, int n_max) {
-  pg::griddep_begin<sizeof(TA) == 2>();
+  pg::griddep_begin();
   constexpr int VB = 16 * VEC;
   const int e = blockIdx.z, h = blockIdx.y;
   const int n = a.entry_n[e];
@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(PgDeltaArgs a, int n_mi
 // of value columns (norm_state [slots, blocks, H, dim + 1], m last), so that the CTAs of one head share no slot.
 template <typename TA, int VEC, int RP, int KIND>
 __global__ void __launch_bounds__(256) gated_scan_kernel(PgGatedArgs a, int n_min, int n_max) {
-  pg::griddep_begin<sizeof(TA) == 2>();
+  pg::griddep_begin();
   constexpr int VB = 16 * VEC;
   const int e = blockIdx.z, h = blockIdx.y;
   const int n = a.entry_n[e];

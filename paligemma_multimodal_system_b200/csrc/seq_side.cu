@@ -60,7 +60,6 @@ __global__ void __launch_bounds__(kThreads) token_side_kernel(const TA* act, con
   float* gz = row + D;       // [kMaxInner]
   float* ys = gz + kMaxInner;  // [D / kRanks]
   float* red = ys + D / kRanks;  // [8] warps, [kRanks] ranks
-  pg::griddep_launch_dependents();
   {  // weights do not depend on the kernels before: on their way to L2 ahead of the wait
     const long long lines = (long long)n_pad * D * sizeof(TA) / 128, i = (long long)blockIdx.x * kThreads + threadIdx.x;
     for (long long l = i; l < lines; l += (long long)gridDim.x * kThreads) {
