@@ -318,7 +318,14 @@ inline int current_device() {
 inline int num_sms() {
   static int sms[kMaxDevices] = {};
   const int dev = current_device();
-  if (sms[dev] == 0) cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
+  if (sms[dev] == 0) {
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 2) {  // no GPU: plans divide by this; the launch reports the error
+      cudaGetLastError();
+      return 2;
+    }
+    sms[dev] = n;
+  }
   return sms[dev];
 }
 

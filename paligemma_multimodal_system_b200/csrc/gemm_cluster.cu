@@ -295,7 +295,7 @@ int clusters_at_once(int S) {
     int n = 0;
     if (!configure() || cudaOccupancyMaxActiveClusters(&n, gemm_cluster_kernel<true>, &cfg) != cudaSuccess || n <= 0) {
       cudaGetLastError();
-      n = num_sms() / (S + 1);
+      n = num_sms() / (S + 1) > 0 ? num_sms() / (S + 1) : 1;
     }
     known[dev][S] = n;
   }
