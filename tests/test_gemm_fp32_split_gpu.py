@@ -80,6 +80,38 @@ def test_range_of_fp32():
     assert ((out.double() - 1.5e-36).abs() <= 2 ** -16 * 1.5e-36).all()
 
 
+@pytest.mark.parametrize("K", [64, 1000])
+@pytest.mark.parametrize("xs,ws", [(1e30, 1e30), (3e38, 3e38), (2.5e18, 7e19), (1e-10, 3.3e38), (1.0, 3.4e38)])
+def test_products_at_the_end_of_the_range(xs, ws, K):
+    """Finite operands, products near or above the largest fp32 and with all three terms: infinities where plain FMAs have infinities, never a NaN in their place."""
+    T, F = 300, 260
+    x, w = _t(T, K, seed=31).sign() * (1 + 0.1 * _t(T, K, seed=32).clamp(-1, 0)) * xs, _t(F, K, seed=33).abs().clamp(0.9, 1) * ws
+    x[:100] = x[:100].abs()  # rows whose sums overflow to one side only
+    assert torch.isfinite(x).all() and torch.isfinite(w).all()
+    a, b = torch.empty(T, F, device="cuda"), torch.empty(T, F, device="cuda")
+    assert _split(x, w, a) == 0
+    _lib.check(_lib.lib().pg_gemm_simt(x.data_ptr(), K, w.data_ptr(), K, b.data_ptr(), F, T, F, K, 1, 1, _lib.stream()), "simt")
+    assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
+    ok = torch.isfinite(b)
+    assert torch.equal(a[~ok & ~b.isnan()], b[~ok & ~b.isnan()])
+    # finite sums: either is within K 2^-24 of the sum of the terms' sizes
+    size = (x.double().abs() @ w.double().abs().T)[ok]
+    assert ((a.double()[ok] - b.double()[ok]).abs() <= size * (2.0 ** -23 * K)).all()
+
+
+@pytest.mark.parametrize("ex,ew,K,split", [(63, 62, 64, False), (54, 64, 64, True), (55, 64, 64, False), (94, 20, 1024, True), (95, 20, 1024, False), (-120, 126, 64, True)])
+def test_the_line_to_the_plain_products(ex, ew, K, split):
+    """Operands of 1.5 x 2^e: split while the two exponents and log2 K add up to 124 at most (2^(e_x + e_w + 2) K <= 2^126), and the sums are right on either side."""
+    T, F = 64, 64
+    x, w = torch.full((T, K), 1.5 * 2.0 ** ex, device="cuda"), torch.full((F, K), 1.5 * 2.0 ** ew, device="cuda")
+    scratch = torch.zeros(1 << 22, device="cuda", dtype=torch.uint8)
+    out = torch.empty(T, F, device="cuda")
+    assert _lib.lib().pg_gemm_fp32_split(x.data_ptr(), K, w.data_ptr(), K, out.data_ptr(), F, 0, 0, 1.0, T, F, K, scratch.data_ptr(), scratch.numel(), _lib.stream()) == 0
+    assert scratch[:4].view(torch.int32).item() == int(not split)
+    want = (x.double() @ w.double().T).float()
+    assert torch.equal(out.isinf(), want.isinf()) and torch.allclose(out, want, rtol=1e-6)
+
+
 def test_what_has_no_split_form():
     x, w, out = _t(64, 68, seed=1), _t(64, 68, seed=2), torch.empty(64, 64, device="cuda")
     assert _split(x, w, out) != 0                                     # K not a multiple of 8
