@@ -287,28 +287,41 @@ Plan plan(int T, int F, int K) {
   return best;
 }
 
-long long up16(long long n) { return (n + 15) / 16 * 16; }
+long long scratch_of(int T, int F, int K, int split_k) { return 16 + 6LL * (static_cast<long long>(T) + F) * K + (split_k > 1 ? 4LL * split_k * T * F : 0); }
+
+// The planes are half as large again as the operands.  A call takes at most 256 MB of scratch, whatever its operands: larger ones (a vocabulary) go in blocks of whole
+// tiles that use it one after the other.  Where not even one tile fits the plain FMAs compute the call.  (750 tokens x 16384 x 2048 takes 211 MB.)
+constexpr long long kMaxScratch = 256LL << 20;
+
+struct Blocks { int tokens, features; Plan plan; };  // of one block; tokens 0: none fits
+Blocks blocks(int T, int F, int K) {
+  Blocks b{T, F, plan(T, F, K)};
+  while (scratch_of(b.tokens, b.features, K, b.plan.split_k) > kMaxScratch) {
+    int& larger = b.tokens > b.features ? b.tokens : b.features;
+    if (larger <= kTile) return Blocks{0, 0, Plan{1, false}};
+    larger = ((larger + 1) / 2 + kTile - 1) / kTile * kTile;
+    b.plan = plan(b.tokens, b.features, K);
+  }
+  return b;
+}
 
 }  // namespace
 }  // namespace pg
 
 extern "C" long long pg_gemm_fp32_scratch(int tokens, int features, int K) {
   if (tokens < 32 || features < 64 || K < 64 || K % 8 != 0 || features % 4 != 0) return 0;
-  const pg::Plan p = pg::plan(tokens, features, K);
-  if (!p.use) return 0;
-  return 16 + 6LL * (static_cast<long long>(tokens) + features) * K + (p.split_k > 1 ? 4LL * p.split_k * tokens * features : 0);
+  const pg::Blocks b = pg::blocks(tokens, features, K);
+  return b.plan.use ? pg::scratch_of(b.tokens, b.features, K, b.plan.split_k) : 0;
 }
 
-extern "C" int pg_gemm_fp32_split(const float* x, long long ldx, const float* w, long long ldw, float* out, long long ldo, const float* bias, int accumulate, float scale,
-                                  int tokens, int features, int K, void* scratch, long long scratch_bytes, void* stream) {
-  using namespace pg;
-  if (tokens <= 0 || features <= 0 || K <= 0 || x == nullptr || w == nullptr || out == nullptr || scratch == nullptr) return PG_ERR_ARG;
-  const uintptr_t all = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(scratch);
-  if (K % 8 != 0 || features % 4 != 0 || ldx % 4 != 0 || ldw % 4 != 0 || ldo % 4 != 0 || (all & 15) != 0) return PG_ERR_ARG;
-  const int split_k = plan(tokens, features, K).split_k;
-  const long long xn = 3LL * tokens * K * 2, wn = 3LL * features * K * 2, pn = split_k > 1 ? 4LL * split_k * tokens * features : 0;
-  if (scratch_bytes < 16 + xn + wn + pn || 3LL * features > 0x7fffffff || 3LL * tokens > 0x7fffffff) return PG_ERR_ARG;
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+namespace pg {
+namespace {
+// one block of the call
+int split_block(const float* x, long long ldx, const float* w, long long ldw, float* out, long long ldo, const float* bias, int accumulate, float scale, int tokens, int features,
+                int K, void* scratch, long long scratch_bytes, cudaStream_t st) {
+  int split_k = plan(tokens, features, K).split_k;
+  if (scratch_bytes < scratch_of(tokens, features, K, split_k)) split_k = 1;  // (the last block of a row: its parts may want more than a whole block does)
+  const long long xn = 3LL * tokens * K * 2, wn = 3LL * features * K * 2;
   char* s = static_cast<char*>(scratch);
   int* flag = reinterpret_cast<int*>(s);
   uint4* xp = reinterpret_cast<uint4*>(s + 16);
@@ -341,4 +354,24 @@ extern "C" int pg_gemm_fp32_split(const float* x, long long ldx, const float* w,
       launch_kernel(fp32_split_sum_kernel, dim3(static_cast<unsigned>((static_cast<long long>(tokens) * features / 4 + 255) / 256)), dim3(256), 0, st, part, a, out) != cudaSuccess)
     return PG_ERR_CUDA;
   return pg_gemm_fp32(x, ldx, 0, w, ldw, 0, out, ldo, 0, bias, accumulate, scale, tokens, features, K, 1, st, flag);
+}
+}  // namespace
+}  // namespace pg
+
+extern "C" int pg_gemm_fp32_split(const float* x, long long ldx, const float* w, long long ldw, float* out, long long ldo, const float* bias, int accumulate, float scale,
+                                  int tokens, int features, int K, void* scratch, long long scratch_bytes, void* stream) {
+  using namespace pg;
+  if (tokens <= 0 || features <= 0 || K <= 0 || x == nullptr || w == nullptr || out == nullptr || scratch == nullptr) return PG_ERR_ARG;
+  const uintptr_t all = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(scratch);
+  if (K % 8 != 0 || features % 4 != 0 || ldx % 4 != 0 || ldw % 4 != 0 || ldo % 4 != 0 || (all & 15) != 0) return PG_ERR_ARG;
+  const Blocks b = blocks(tokens, features, K);
+  if (b.tokens == 0 || scratch_bytes < scratch_of(b.tokens, b.features, K, b.plan.split_k)) return PG_ERR_ARG;
+  for (long long t = 0; t < tokens; t += b.tokens)
+    for (long long f = 0; f < features; f += b.features) {
+      const int nt = static_cast<int>(tokens - t < b.tokens ? tokens - t : b.tokens), nf = static_cast<int>(features - f < b.features ? features - f : b.features);
+      const int rc = split_block(x + t * ldx, ldx, w + f * ldw, ldw, out + t * ldo + f, ldo, bias == nullptr ? nullptr : bias + f, accumulate, scale, nt, nf, K, scratch,
+                                 scratch_bytes, reinterpret_cast<cudaStream_t>(stream));
+      if (rc != PG_OK) return rc;
+    }
+  return PG_OK;
 }

@@ -157,7 +157,8 @@ ACT_NONE, ACT_GELU, ACT_RELU2, ACT_SILU_GLU, ACT_GELU_ERF = 0, 1, 2, 3, 6
 
 
 def _linear_fp32_split(x, w, out, bias, accumulate, scale):
-    """fp32 products of many tokens on the tensor cores (three bf16 terms a value); False where the plain-FMA form is faster or has to take the call."""
+    """fp32 products of many tokens on the tensor cores (three bf16 terms a value); False where the plain-FMA form is faster or has to take the call: it needs no
+    scratch, so a device without room for that (256 MB at most) is served as well."""
     T, K = x.shape
     F = w.shape[0]
     if not (x.is_cuda and w.is_cuda and _aligned(x) and _aligned(w) and _aligned(out)) or (x.stride(0) | w.stride(0) | out.stride(0)) % 4:
@@ -165,7 +166,10 @@ def _linear_fp32_split(x, w, out, bias, accumulate, scale):
     need = _lib.lib().pg_gemm_fp32_scratch(T, F, K)
     if not need:
         return False
-    scratch = torch.empty(need, device=x.device, dtype=torch.uint8)
+    try:
+        scratch = torch.empty(need, device=x.device, dtype=torch.uint8)
+    except torch.OutOfMemoryError:
+        return False
     _lib.check(_lib.lib().pg_gemm_fp32_split(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), _lib.ptr(bias), accumulate, scale,
                                              T, F, K, scratch.data_ptr(), need, _lib.stream()), "pg_gemm_fp32_split")
     return True

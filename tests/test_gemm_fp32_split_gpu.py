@@ -112,6 +112,55 @@ def test_the_line_to_the_plain_products(ex, ew, K, split):
     assert torch.equal(out.isinf(), want.isinf()) and torch.allclose(out, want, rtol=1e-6)
 
 
+@pytest.mark.parametrize("T,F,K", [(300, 40000, 2048), (30000, 260, 2048), (11000, 11004, 4096), (300, 22020, 2048), (300, 4100, 16384)])
+def test_large_operands_in_blocks(T, F, K):
+    """More than 256 MB of planes: blocks of features, of tokens, of both; the last block short.  Views, bias, scale, an output that is added to."""
+    L = _lib.lib()
+    need = L.pg_gemm_fp32_scratch(T, F, K)
+    assert 0 < need <= 256 << 20 < 6 * (T + F) * K
+    x, w, bias = _t(T, K + 4, seed=41)[:, :K], _t(F, K, seed=42, scale=K ** -0.5), _t(F, seed=43)
+    whole = _t(T, F + 4, seed=44)
+    out, before = whole[:, :F], whole.clone()
+    scratch = torch.full((need + 64,), 0xFF, device="cuda", dtype=torch.uint8)
+    assert L.pg_gemm_fp32_split(x.data_ptr(), x.stride(0), w.data_ptr(), K, out.data_ptr(), out.stride(0), bias.data_ptr(), 1, 0.7, T, F, K, scratch.data_ptr(), need,
+                                _lib.stream()) == 0
+    assert (scratch[need:] == 0xFF).all() and torch.equal(whole[:, F:], before[:, F:])
+    xd = x.double()
+    for f in range(0, F, 4096):
+        want = (xd @ w[f:f + 4096].double().T + bias[f:f + 4096].double()) * 0.7 + before[:, f:min(F, f + 4096)].double()
+        assert ((out[:, f:f + 4096].double() - want).norm() / want.norm()).item() < 4e-7
+    assert L.pg_gemm_fp32_split(x.data_ptr(), x.stride(0), w.data_ptr(), K, out.data_ptr(), out.stride(0), 0, 0, 1.0, T, F, K, scratch.data_ptr(), need - 1, _lib.stream()) != 0
+
+
+def test_scratch_is_bounded():
+    L = _lib.lib()
+    for T in (32, 100, 750, 5000, 100000):
+        for F, K in ((257216, 2048), (16384, 2048), (2048, 16384), (64, 64), (1 << 20, 8192), (256, 1 << 20)):
+            assert 0 <= L.pg_gemm_fp32_scratch(T, F, K) <= 256 << 20
+    assert L.pg_gemm_fp32_scratch(750, 16384, 2048) == 16 + 6 * (750 + 16384) * 2048  # (one block)
+
+
+def test_no_room_for_the_scratch(monkeypatch):
+    """A device without memory for the planes: the plain FMAs, with the bits they have."""
+    K = 2048
+    x, w = _t(700, K, seed=51), _t(K, K, seed=52)
+    assert _lib.lib().pg_gemm_fp32_scratch(700, K, K) > 0
+    real, out, acc = torch.empty, torch.empty(700, K, device="cuda"), _t(700, K, seed=53)
+
+    def full(*a, dtype=None, **kw):
+        if dtype == torch.uint8:
+            raise torch.OutOfMemoryError("no room")
+        return real(*a, dtype=dtype, **kw)
+
+    want = torch.empty(700, K, device="cuda")
+    _lib.check(_lib.lib().pg_gemm_simt(x.data_ptr(), K, w.data_ptr(), K, want.data_ptr(), K, 700, K, K, 1, 1, _lib.stream()), "simt")
+    want_acc = acc.clone()
+    _lib.check(_lib.lib().pg_gemm_simt_bias(x.data_ptr(), K, w.data_ptr(), K, want_acc.data_ptr(), K, 0, 1, 0.5, 700, K, K, 1, 1, _lib.stream()), "simt")
+    monkeypatch.setattr(seq_ops.torch, "empty", full)
+    assert torch.equal(seq_ops.linear(x, w, out), want)
+    assert torch.equal(seq_ops.linear_add(x, w, acc, scale=0.5), want_acc)
+
+
 def test_what_has_no_split_form():
     x, w, out = _t(64, 68, seed=1), _t(64, 68, seed=2), torch.empty(64, 64, device="cuda")
     assert _split(x, w, out) != 0                                     # K not a multiple of 8
