@@ -696,7 +696,7 @@ class RoutedFeedForward:
         z = seq_ops.linear(h, self.w_router, torch.empty(T, self.w_router.shape[0], device="cuda", dtype=torch.float32))
         ids, wts, counts = seq_ops.moe_route(z[:, :self.n_all], self.correction, self.n_real, self.top, self.group_count, self.group_keep, self.scale,
                                              logit_bias=self.router_b, flags=self.route_flags)
-        plan = seq_ops.MoePlan(ids, counts, max(1, self.n_real))
+        plan = seq_ops.MoePlan(ids, counts, self.n_real)
         return z, ids, wts, plan, self.expert_products(h, plan, counts, prec) if self.n_real else None
 
     def add_normed(self, h, prec, norm_w, x, out_act, eps):

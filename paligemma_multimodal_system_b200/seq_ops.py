@@ -599,12 +599,16 @@ def moe_route(logits, correction, n_real, top, group_count, group_keep, scale, l
 
 
 class MoePlan:
-    """Device-side order of the (token, choice) pairs by expert and the list of row tiles the grouped products walk."""
+    """Device-side order of the (token, choice) pairs by expert and the list of row tiles the grouped products walk.  n_real 0 (identity outputs only): no pair has an
+    expert row, there is nothing to walk and no count to read."""
 
     def __init__(self, ids, counts, n_real):
         L = _lib.lib()
         T, top = ids.shape
         self.pairs, self.top = T * top, top
+        if not n_real:
+            self.pair_row = torch.full((self.pairs,), -1, device=ids.device, dtype=torch.int32)
+            return
         self.max_tiles = -(-self.pairs // L.pg_moe_tile_rows()) + n_real
         i32 = dict(device="cuda", dtype=torch.int32)
         self.offsets = torch.empty(n_real + 1, **i32)
@@ -653,6 +657,7 @@ def moe_combine(expert_out, plan: MoePlan, ids, weights, h, shared_out, y, share
     """y[t] (+)= sum_k weights[t, k] * expert row (or h[t] for an identity expert) + sigmoid(shared_gate[t]) * shared_out[t]; shared_gate:
     fp32 logits, one per token (a strided column view), None: the shared term counts fully; accumulate: add into y."""
     T, D = y.shape
+    assert expert_out is not None or not hasattr(plan, "plan")  # (without expert rows no pair may have one)
     assert shared_gate is None or (shared_gate.dtype == torch.float32 and shared_gate.shape[0] == T)
     assert y.dtype == torch.float32 and y.is_contiguous() and h.stride(1) == 1
     assert expert_out is None or (expert_out.dtype == torch.float32 and expert_out.stride(1) == 1)
