@@ -9,8 +9,9 @@
 //
 // Three launches: split (both operands into planes of a scratch the caller owns), product, and -- where the output has too few tiles for the SMs, K is shared out
 // between pairs of CTAs -- a sum of the partial outputs, part after part.  Infinities and NaNs have no such split, and where products come near the end of the range one
-// term may overflow to either side and the sum of two be no number (inf - inf).  So the split kernel keeps the largest exponent of either operand; where the sums could
-// reach 2^127 (too_large) the product writes nothing, and the plain-FMA kernel launched behind it, which otherwise returns at once, computes the call.
+// term may overflow to either side and the sum of two be no number (inf - inf).  So the split kernel raises a flag for values so large that a
+// sum could reach 2^127 (safe_exponent; 2^57 for K = 2048), the product then writes nothing, and the plain-FMA kernel launched behind it, which otherwise returns at once,
+// computes the call.  (A bound of the operands' largest exponents together would let more through; their maxima as atomics cost a decode burst of five requests 8 %.)
 //
 // What it holds: operands above about 1e-33 keep their 24 bits; below, the third term and then the second fall under the smallest bf16 (at 2e-36 16 bits are left).
 //
@@ -45,42 +46,38 @@ PG_DEVINL void split3(float v, uint32_t& a, uint32_t& b, uint32_t& c) {
   c = (u3 + 0x7fffu + ((u3 >> 16) & 1)) >> 16;
 }
 
-// Biased exponents of the largest operands: a value is below 2^(e - 126), the six terms of a product are together below 1.02 times that of their operands, and K of them are
-// added: all below 2^127 while e_x + e_w + log2 K is at most 378.
-PG_DEVINL bool too_large(int ex, int ew, int K) { return max(ex, ew) == 255 || ex + ew + (32 - __clz(K - 1)) > 378; }
+// The largest biased exponent of an operand that cannot bring a sum to 2^127: a value is below 2^(e - 126), the six terms of a product are together below 1.02 times that of
+// their operands, and K of them are added, so 2 e + log2 K is at most 378.
+int safe_exponent(int K) {
+  int log_k = 0;
+  while (log_k < 31 && (1LL << log_k) < K) ++log_k;
+  return (378 - log_k) / 2;
+}
 
 // rows of x, then rows of w -> planes [3][T][K] and [3][F][K]; eight values a thread
 __global__ void __launch_bounds__(256) fp32_split_kernel(const float* __restrict__ x, long long ldx, int T, const float* __restrict__ w, long long ldw, int F, int K,
-                                                         uint4* __restrict__ xp, uint4* __restrict__ wp, int* __restrict__ flag) {
+                                                         uint4* __restrict__ xp, uint4* __restrict__ wp, int* __restrict__ flag, int safe) {
   griddep_wait();
   const int per = K / 8;
   const long long id = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x, nx = static_cast<long long>(T) * per, nw = static_cast<long long>(F) * per;
+  if (id >= nx + nw) return;
   const bool is_x = id < nx;
-  int exponent = 0;  // the largest of the thread's values, biased; 255 infinities and NaNs
-  if (id < nx + nw) {
-    const long long i = is_x ? id : id - nx, n = is_x ? nx : nw;
-    const float* src = (is_x ? x + i / per * ldx : w + i / per * ldw) + i % per * 8;
-    const float4 p = reinterpret_cast<const float4*>(src)[0], q = reinterpret_cast<const float4*>(src)[1];
-    const float v[8] = {p.x, p.y, p.z, p.w, q.x, q.y, q.z, q.w};
-    uint32_t o[3][8];
+  const long long i = is_x ? id : id - nx, n = is_x ? nx : nw;
+  const float* src = (is_x ? x + i / per * ldx : w + i / per * ldw) + i % per * 8;
+  const float4 p = reinterpret_cast<const float4*>(src)[0], q = reinterpret_cast<const float4*>(src)[1];
+  const float v[8] = {p.x, p.y, p.z, p.w, q.x, q.y, q.z, q.w};
+  uint32_t o[3][8];
+  bool large = false;  // (infinities and NaNs have the largest exponent)
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      exponent = max(exponent, static_cast<int>((__float_as_uint(v[k]) & 0x7f800000u) >> 23));
-      split3(v[k], o[0][k], o[1][k], o[2][k]);
-    }
-    uint4* dst = (is_x ? xp : wp) + i;
+  for (int k = 0; k < 8; ++k) {
+    large = large || static_cast<int>((__float_as_uint(v[k]) & 0x7f800000u) >> 23) > safe;
+    split3(v[k], o[0][k], o[1][k], o[2][k]);
+  }
+  uint4* dst = (is_x ? xp : wp) + i;
 #pragma unroll
-    for (int t = 0; t < 3; ++t)
-      dst[t * n] = make_uint4(o[t][0] | o[t][1] << 16, o[t][2] | o[t][3] << 16, o[t][4] | o[t][5] << 16, o[t][6] | o[t][7] << 16);
-  }
-  // (a maximum that is there already needs no atomic: after the first few warps hardly one is left)
-  const int ex = __reduce_max_sync(0xffffffffu, is_x ? exponent : 0), ew = __reduce_max_sync(0xffffffffu, is_x ? 0 : exponent);
-  if ((threadIdx.x & 31) == 0 && (ex > *static_cast<volatile int*>(flag + 1) || ew > *static_cast<volatile int*>(flag + 2))) {
-    atomicMax(flag + 1, ex);
-    atomicMax(flag + 2, ew);
-    __threadfence();  // of two warps that raise one maximum each, one sees both
-    if (too_large(atomicMax(flag + 1, 0), atomicMax(flag + 2, 0), K)) *flag = 1;
-  }
+  for (int t = 0; t < 3; ++t)
+    dst[t * n] = make_uint4(o[t][0] | o[t][1] << 16, o[t][2] | o[t][3] << 16, o[t][4] | o[t][5] << 16, o[t][6] | o[t][7] << 16);
+  if (large) *flag = 1;
 }
 
 struct SplitArgs {
@@ -340,12 +337,12 @@ int split_block(const float* x, long long ldx, const float* w, long long ldw, fl
   int rc;
   if ((rc = make_tmap_2d(&tx, xp, 3LL * tokens, K, K, kRows)) != PG_OK) return rc;
   if ((rc = make_tmap_2d(&tw, wp, 3LL * features, K, K, kRows)) != PG_OK) return rc;
-  if (cudaMemsetAsync(flag, 0, 3 * sizeof(int), st) != cudaSuccess) {
+  if (cudaMemsetAsync(flag, 0, sizeof(int), st) != cudaSuccess) {
     cudaGetLastError();
     return PG_ERR_CUDA;
   }
   const long long pieces = (static_cast<long long>(tokens) + features) * (K / 8);
-  if (launch_kernel(fp32_split_kernel, dim3(static_cast<unsigned>((pieces + 255) / 256)), dim3(256), 0, st, x, ldx, tokens, w, ldw, features, K, xp, wp, flag) != cudaSuccess)
+  if (launch_kernel(fp32_split_kernel, dim3(static_cast<unsigned>((pieces + 255) / 256)), dim3(256), 0, st, x, ldx, tokens, w, ldw, features, K, xp, wp, flag, safe_exponent(K)) != cudaSuccess)
     return PG_ERR_CUDA;
   SplitArgs a{split_k > 1 ? part : out, bias, flag, ldo, tokens, features, K, split_k, accumulate, scale};
   const int tiles = ((tokens + kTile - 1) / kTile) * ((features + kTile - 1) / kTile) * split_k, pairs = num_sms() / 2;

@@ -99,9 +99,10 @@ def test_products_at_the_end_of_the_range(xs, ws, K):
     assert ((a.double()[ok] - b.double()[ok]).abs() <= size * (2.0 ** -23 * K)).all()
 
 
-@pytest.mark.parametrize("ex,ew,K,split", [(63, 62, 64, False), (54, 64, 64, True), (55, 64, 64, False), (94, 20, 1024, True), (95, 20, 1024, False), (-120, 126, 64, True)])
+@pytest.mark.parametrize("ex,ew,K,split", [(59, 59, 64, True), (60, 3, 64, False), (-100, 60, 64, False), (57, 57, 1000, True), (57, 57, 1024, True), (58, 0, 1024, False), (-120, 56, 1032, True), (57, -3, 1032, False),
+                                           (63, 62, 64, False), (-110, 126, 64, False)])
 def test_the_line_to_the_plain_products(ex, ew, K, split):
-    """Operands of 1.5 x 2^e: split while the two exponents and log2 K add up to 124 at most (2^(e_x + e_w + 2) K <= 2^126), and the sums are right on either side."""
+    """Operands of 1.5 x 2^e: split while e of each is at most (124 - log2 K) / 2 (then 2^(e_x + e_w + 2) K is at most 2^126), and the sums are right on either side."""
     T, F = 64, 64
     x, w = torch.full((T, K), 1.5 * 2.0 ** ex, device="cuda"), torch.full((F, K), 1.5 * 2.0 ** ew, device="cuda")
     scratch = torch.zeros(1 << 22, device="cuda", dtype=torch.uint8)
