@@ -8,7 +8,10 @@
 //   * S = Q K^T: 128 x 64 into tensor memory; a thread reads its row of 64 scores, masks, exponentiates -- no exchange between lanes, the row sum is its own;
 //   * P goes back to tensor memory as three 32-column bf16 tiles and is the A operand of P V from there (12 instructions a tile): it never passes through shared memory;
 //   * S of the next tile is multiplied while this tile's exponentials run (values 64 wide; for 128 the 256 columns of a CTA leave no room for S beside P);
-//   * O is rescaled only when a row's maximum grew by more than 2^8 (fp32 sums have the room).
+//   * O is rescaled only when a row's maximum grew by more than 2^8 (fp32 sums have the room);
+//   * P V runs over all 128 rows with zero weights where a row does not see a key, and zero times a value that is not finite is no zero.  So a row whose sums are not finite is
+//     computed again from the keys that it sees (row_from_visible_keys): a broken value reaches the rows that see it and no others.  (Rows that end or begin inside the loop
+//     instead cost every prompt: 8 x 1024 tokens 140 -> 147 us; the check 142.)
 // What bounds it: the softmax warps (clocks a tile, stamped: wait for S 100, its load 75, maxima and exponentials 1000 .. 1330, wait for P V 185, split 520; the products hide
 // behind them).  Two threads a row share the same pipes (146 us for 149), exponentials as polynomials on the FMA pipe cost more than they save (168).  us, mma.sync / here: 8 prompts of 897 .. 1024 tokens, 32 heads x 64 over 8 k/v heads 235 / 149; 2 portions of 333
 // tokens behind 1400, 32 heads x 96 / 64: 144 / 66.
@@ -87,9 +90,65 @@ struct Shape {
   static_assert(COL_O + VDIM <= 256 && STAGES >= 2 && DIM % 16 == 0 && VDIM % 64 == 0, "two CTAs per SM");
 };
 
+// One query row by a warp, from the keys that it sees and no others: for rows whose sums are not finite (see above).  Scores, probabilities and sums in fp32; a lane has a key of
+// 32 for the scores and VDIM / 32 columns of the values.
+template <int DIM, int VDIM>
+__device__ __noinline__ void row_from_visible_keys(const bf16* __restrict__ q, const bf16* __restrict__ k_pages, const bf16* __restrict__ v_pages, const int* __restrict__ pt, int page,
+                                                   long long krow, long long vrow, int lim, int lo, int keep, float sc, float softcap, const float* sink, float out_scale,
+                                                   const bf16* __restrict__ gate, int gate_per_head, bf16* __restrict__ out) {
+  constexpr int NC = VDIM / 32;
+  const int lane = threadIdx.x & 31;
+  float m = -INFINITY, l = 0.f, acc[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) acc[c] = 0.f;
+  for (int k0 = 0; k0 <= lim; k0 += 32) {
+    if (k0 >= keep && k0 + 31 < lo) k0 = lo & ~31;
+    const int j = k0 + lane;
+    const bool vis = j <= lim && (j >= lo || j < keep);
+    const unsigned seen = __ballot_sync(0xffffffffu, vis);
+    const long long row = vis ? static_cast<long long>(pt[j / page]) * page + j % page : 0;
+    float t = -INFINITY;
+    if (vis) {
+      float d = 0.f;
+      for (int i = 0; i < DIM; ++i) d = fmaf(__bfloat162float(q[i]), __bfloat162float(k_pages[row * krow + i]), d);
+      t = (softcap > 0.f ? softcap * tanh32(d * (sc / softcap)) : d * sc) * kLog2e;
+    }
+    float mx = t;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    const float mn = fmaxf(m, mx), off = mn > -INFINITY ? mn : 0.f, alpha = ex2(m - off), p = vis ? ex2(t - off) : 0.f;
+    m = mn;
+    l = l * alpha + p;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) acc[c] *= alpha;
+    for (unsigned left = seen; left != 0; left &= left - 1) {
+      const int src = __ffs(left) - 1;
+      const float pj = __shfl_sync(0xffffffffu, p, src);
+      const bf16* v = v_pages + __shfl_sync(0xffffffffu, row, src) * vrow + NC * lane;
+#pragma unroll
+      for (int c = 0; c < NC; ++c) acc[c] = fmaf(pj, __bfloat162float(v[c]), acc[c]);
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+  float osc = 1.f;
+  if (sink != nullptr) {
+    const float sk = *sink * kLog2e, mm = fmaxf(m, sk);
+    osc = exp2f(m - mm);
+    l = l * osc + exp2f(sk - mm);
+  }
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    float x = acc[c] * (osc / l * out_scale);
+    if (gate != nullptr) x *= 1.0f / (1.0f + expf(-__bfloat162float(gate[gate_per_head ? 0 : NC * lane + c])));
+    out[NC * lane + c] = __float2bfloat16_rn(x);
+  }
+}
+
 template <int DIM, int VDIM>
 __global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
-                                                                     const bf16* __restrict__ q, const bf16* __restrict__ gate, long long ldg, bf16* __restrict__ out,
+                                                                     const bf16* __restrict__ q, const bf16* __restrict__ k_pages, const bf16* __restrict__ v_pages,
+                                                                     const bf16* __restrict__ gate, long long ldg, bf16* __restrict__ out,
                                                                      const int* __restrict__ entry_row0, const int* __restrict__ entry_n, const int* __restrict__ entry_ctx,
                                                                      const int* __restrict__ page_table, int max_pages, int page, int H, int G, float scale, float softcap,
                                                                      int skip_single, int gate_per_head, PgAttnScore sx) {
@@ -344,6 +403,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __gri
     const long long t = row0 + (there ? rr / gsz : 0), ldo = sx.out_ld > 0 ? sx.out_ld : static_cast<long long>(H) * VDIM;
     bf16* o = out + t * ldo + static_cast<long long>(head) * VDIM;
     const bf16* gt = gate == nullptr ? nullptr : gate + t * ldg + (gate_per_head ? static_cast<long long>(head) : static_cast<long long>(head) * VDIM);
+    bool odd = false;  // a sum of the row is not finite
     const float gh = gate != nullptr && gate_per_head ? 1.0f / (1.0f + expf(-__bfloat162float(*gt))) : 1.f;
 #pragma unroll 1
     for (int c = 0; c < VDIM; c += 16) {
@@ -353,7 +413,10 @@ __global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __gri
       if (there) {
         float x[16];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) x[i] = __uint_as_float(v[i]) * inv;
+        for (int i = 0; i < 16; ++i) {
+          odd = odd || (v[i] & 0x7f800000u) == 0x7f800000u;
+          x[i] = __uint_as_float(v[i]) * inv;
+        }
         if (gate != nullptr) {
           if (gate_per_head) {
 #pragma unroll
@@ -372,6 +435,16 @@ __global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __gri
         d[1] = make_uint4(pack_bf16(x[8], x[9]), pack_bf16(x[10], x[11]), pack_bf16(x[12], x[13]), pack_bf16(x[14], x[15]));
       }
       __syncwarp();
+    }
+    for (unsigned left = __ballot_sync(0xffffffffu, odd); left != 0; left &= left - 1) {
+      const int row = r0 + qd * 32 + __ffs(left) - 1, hd = g * gsz + row % gsz, last = ctx + row / gsz;
+      const long long tk = row0 + row / gsz;
+      row_from_visible_keys<DIM, VDIM>(q + (tk * H + hd) * DIM, k_pages + static_cast<long long>(g) * DIM, v_pages + static_cast<long long>(g) * VDIM,
+                                       page_table + static_cast<long long>(e) * max_pages, page, static_cast<long long>(G) * DIM, static_cast<long long>(G) * VDIM, last, last - window + 1, keep,
+                                       scale * (sx.head_scale != nullptr ? sx.head_scale[hd] : 1.f), softcap, sx.sink != nullptr ? sx.sink + hd : nullptr,
+                                       sx.out_scale != 0.f ? sx.out_scale : 1.f,
+                                       gate == nullptr ? nullptr : gate + tk * ldg + (gate_per_head ? static_cast<long long>(hd) : static_cast<long long>(hd) * VDIM), gate_per_head,
+                                       out + tk * ldo + static_cast<long long>(hd) * VDIM);
     }
     tc_fence_before();
   }
@@ -402,7 +475,8 @@ int launch(const void* q, const void* kp, const void* vp, const void* gate, long
   if ((rc = make_tmap_2d(&tk, kp, 1LL << 30, static_cast<long long>(G) * DIM, static_cast<long long>(G) * DIM, page < 64 ? page : 64)) != PG_OK) return rc;
   if ((rc = make_tmap_2d(&tv, vp, 1LL << 30, static_cast<long long>(G) * VDIM, static_cast<long long>(G) * VDIM, page < 64 ? page : 64)) != PG_OK) return rc;
   launch_spread(attn_ragged_tc_kernel<DIM, VDIM>, dim3((max_n * (H / G) + 127) / 128, G, entries), dim3(kThreads), C::SMEM, st, tk, tv, static_cast<const bf16*>(q),
-                static_cast<const bf16*>(gate), ldg, static_cast<bf16*>(out), row0, n, ctx, pt, max_pages, page, H, G, scale, softcap, skip_single, gate_per_head, sx);
+                static_cast<const bf16*>(kp), static_cast<const bf16*>(vp), static_cast<const bf16*>(gate), ldg, static_cast<bf16*>(out), row0, n, ctx, pt, max_pages, page, H, G,
+                scale, softcap, skip_single, gate_per_head, sx);
   pg_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
 }

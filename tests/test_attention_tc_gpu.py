@@ -85,3 +85,65 @@ def _run(dim, vdim, G, gsz, ns, ctxs, window, keep, softcap=0.0, hs=False, sink=
         r += n
     if ld:
         assert (out[:, H * vdim:] == 7).all()
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("dim,vdim,G,gsz,window,keep", [(64, 64, 2, 4, 0, 0), (64, 64, 1, 1, 0, 0), (128, 128, 1, 4, 0, 0), (96, 64, 2, 1, 70, 0), (64, 128, 1, 2, 33, 40),
+                                                        (128, 64, 1, 129, 0, 0), (64, 64, 3, 2, 90, 5)])
+@pytest.mark.parametrize("opts", [dict(), dict(softcap=5.0, hs=True, sink=True, gate="head", ld=True), dict(gate="row")])
+def test_values_that_are_not_finite(dim, vdim, G, gsz, window, keep, opts, bad):
+    """A broken value reaches the rows that see it and no others: not those before it in their block, nor those whose window begins behind it."""
+    n, ctx, at = 300, 30, 207
+    H, L, softcap = G * gsz, ctx + n, opts.get("softcap", 0.0)
+    b = seq_ops.make_step_batch([dict(tokens=[1] * n, ctx=ctx, slot=0, pages=list(range((L + 63) // 64)))])
+    kp, vp = (_t((L + 63) // 64, 64, G * d, seed=s) for d, s in ((dim, 2), (vdim, 3)))
+    vp[at // 64, at % 64] = bad
+    pitch = H * vdim + (8 if "ld" in opts else 0)
+    q, out = _t(n, H * dim, seed=1), torch.full((n, pitch), 7.0, device="cuda", dtype=torch.bfloat16)
+    hs = torch.linspace(-0.7, 1.5, H, device="cuda") if "hs" in opts else None
+    sink = torch.linspace(-2, 3, H, device="cuda") if "sink" in opts else None
+    gate = opts.get("gate")
+    g = None if gate is None else _t(n, H if gate == "head" else H * vdim, seed=5)
+    score = seq_ops.ScoreOptions(H, window or None, keep, sink=sink, head_scale=hs, out_scale=0.5 if "ld" in opts else 1.0, out_ld=pitch if "ld" in opts else 0)
+    seq_ops.attn_ragged(q, kp, vp, g, out, b, H, G, dim, vdim, dim ** -0.5, softcap, 64, gate_per_head=gate == "head", score=score, decode_kernel=False)
+    k, v = kp.view(-1, G, dim)[:L], vp.view(-1, G, vdim)[:L].clone()
+    v[at] = 0
+    want = _want(q.view(n, H, dim), k, v, ctx, dim ** -0.5, softcap, window, keep, hs, sink) * (0.5 if "ld" in opts else 1.0)
+    if g is not None:
+        want = want * torch.sigmoid(g.double()).view(n, H, -1)
+    pos = torch.arange(ctx, L, device="cuda")
+    sees = (pos >= at) & (pos - at < window) if window else pos >= at  # (207 is none of the kept first keys)
+    got = out[:, : H * vdim].double().view(n, H, vdim)
+    assert (~torch.isfinite(got[sees])).all()
+    assert ((got[~sees] - want[~sees]).abs() <= want[~sees].abs() * 2.0 ** -8 + 5e-5).all()
+    if pitch > H * vdim:
+        assert (out[:, H * vdim:] == 7).all()
+
+
+@pytest.mark.parametrize("page", [8, 16, 32, 128, 192])
+@pytest.mark.parametrize("dim,vdim", [(64, 64), (128, 128)])
+def test_page_sizes(page, dim, vdim):
+    """A tile of 64 keys as several pages, the last of them missing, and as part of a page."""
+    G, gsz, ns, ctxs, window, keep = 2, 2, (70, 1, 9, 130), (0, 5, 63, 200), 100, 3
+    H, rows, first = G * gsz, [], 0
+    for i, (n, c) in enumerate(zip(ns, ctxs)):
+        p = (n + c + page - 1) // page
+        rows.append(dict(tokens=[1] * n, ctx=c, slot=i, pages=list(range(first, first + p))[::-1] + [0] * ((n + c + 63) // 64 - p)))  # (at least one a 64 keys is asked for)
+        first += p
+    b = seq_ops.make_step_batch(rows)
+    kp, vp = (torch.full((first, page, G * d), float("nan"), device="cuda", dtype=torch.bfloat16) for d in (dim, vdim))
+    q, out, ks, vs = _t(b.T, H * dim, seed=1), torch.full((b.T, H * vdim), 7.0, device="cuda", dtype=torch.bfloat16), [], []
+    for i, (n, c) in enumerate(zip(ns, ctxs)):
+        k, v = _t(n + c, G * dim, seed=10 + i), _t(n + c, G * vdim, seed=20 + i)
+        for j, p in enumerate(rows[i]["pages"][: (n + c + page - 1) // page]):
+            part = slice(page * j, min(page * j + page, n + c))
+            kp[p, : part.stop - part.start], vp[p, : part.stop - part.start] = k[part], v[part]
+        ks.append(k.view(-1, G, dim))
+        vs.append(v.view(-1, G, vdim))
+    seq_ops.attn_ragged(q, kp, vp, None, out, b, H, G, dim, vdim, dim ** -0.5, 0.0, page, score=seq_ops.ScoreOptions(H, window, keep), decode_kernel=False)
+    r = 0
+    for i, (n, c) in enumerate(zip(ns, ctxs)):
+        want = _want(q[r:r + n].view(n, H, dim), ks[i], vs[i], c, dim ** -0.5, 0.0, window, keep, None, None)
+        got = out[r:r + n].double().view(n, H, vdim)
+        assert ((got - want).abs() <= want.abs() * 2.0 ** -8 + 5e-5).all(), (i, (got - want).abs().max().item())
+        r += n
