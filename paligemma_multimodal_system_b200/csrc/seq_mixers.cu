@@ -762,10 +762,11 @@ __global__ void __launch_bounds__(256) linear_attn_scan_kernel(const TA* __restr
 }
 
 // The same with the state in 16-byte pieces (vdim a multiple of four, dim <= 8 RP): thread = four value columns x every eighth key dimension, CTA = 64 columns of
-// a head.  A step of single tokens moves the state once in and once out and is bound by that (48 requests x 32 heads x 64 x 64, 50 MB: 19.6 -> 13 us): all
-// its pieces are requested at once, beside the token's q, k and v.
+// a head.  A step of single tokens moves the state once in and once out and is bound by that (back to back, 48 requests x 32 heads x 64 x 64, 50 MB: 18.4 -> 9.1 us; 300 requests 131 -> 55): all
+// its pieces are requested at once, beside the token's q, k and v.  A long portion is bound by the chain of its tokens: their q, k and v are requested a token ahead, and five
+// CTAs leave a thread its registers (one portion of 1000 tokens, 8 heads 794 -> 597 us; with seven CTAs and no request ahead 1113).
 template <typename TA, int RP>
-__global__ void __launch_bounds__(128, RP == 8 ? 7 : 3) linear_attn_scan_vec_kernel(const TA* __restrict__ qkv, long long ld, float* __restrict__ state,
+__global__ void __launch_bounds__(128, RP == 8 ? 5 : 3) linear_attn_scan_vec_kernel(const TA* __restrict__ qkv, long long ld, float* __restrict__ state,
                                                                    const float* __restrict__ decay, float* __restrict__ out,
                                                                    const int* __restrict__ entry_row0, const int* __restrict__ entry_n,
                                                                    const int* __restrict__ entry_ctx, const int* __restrict__ entry_slot, int H,
@@ -792,30 +793,39 @@ __global__ void __launch_bounds__(128, RP == 8 ? 7 : 3) linear_attn_scan_vec_ker
     S[i] = (ctx != 0 && d < dim && v_ok) ? st[d * pitch] : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   const long long qo = (long long)h * dim, ko = (long long)H * dim + (long long)h * dim, vo = 2LL * H * dim + (long long)h * vdim;
-  for (int t = 0; t < n; ++t) {
+  // a token's q, k and v are requested a token ahead (dim <= 128: one element or pair a thread)
+  const int d0 = ops.silu ? threadIdx.x : 2 * threadIdx.x;
+  const bool one = d0 < dim, two = !ops.silu && d0 + 1 < dim;
+  TA nq[2], nk[2], nv[4];
+  auto request = [&](int t) {
     const TA* row = qkv + (long long)(row0 + t) * ld;
+    if (one) { nq[0] = row[qo + d0]; nk[0] = row[ko + d0]; }
+    if (two) { nq[1] = row[qo + d0 + 1]; nk[1] = row[ko + d0 + 1]; }
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      if (v_ok) nv[c] = row[vo + v + c];
+  };
+  if (n > 0) request(0);
+  for (int t = 0; t < n; ++t) {
     float vv[4];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) vv[c] = v_ok ? ldf(row, vo + v + c) : 0.f;
+    for (int c = 0; c < 4; ++c) vv[c] = v_ok ? ldf(nv, c) : 0.f;
     if (ops.silu) {
-      for (int d = threadIdx.x; d < dim; d += 128) {
-        qs[d] = silu(ldf(row, qo + d));
-        ksm[d] = silu(ldf(row, ko + d));
+      if (one) {
+        qs[d0] = silu(ldf(nq, 0));
+        ksm[d0] = silu(ldf(nk, 0));
       }
 #pragma unroll
       for (int c = 0; c < 4; ++c) vv[c] = silu(vv[c]);
-    } else {
-      for (int i = threadIdx.x; 2 * i < dim; i += 128) {
-        const int d = 2 * i;
-        const bool two = d + 1 < dim;
-        float q0 = ldf(row, qo + d), q1 = two ? ldf(row, qo + d + 1) : 0.f, k0 = ldf(row, ko + d), k1 = two ? ldf(row, ko + d + 1) : 0.f;
-        enter_pair(ops, row0 + t, i, 1.0f, q0, q1);
-        enter_pair(ops, row0 + t, i, ops.kscale, k0, k1);
-        qs[d] = q0;
-        ksm[d] = k0;
-        if (two) { qs[d + 1] = q1; ksm[d + 1] = k1; }
-      }
+    } else if (one) {
+      float q0 = ldf(nq, 0), q1 = two ? ldf(nq, 1) : 0.f, k0 = ldf(nk, 0), k1 = two ? ldf(nk, 1) : 0.f;
+      enter_pair(ops, row0 + t, threadIdx.x, 1.0f, q0, q1);
+      enter_pair(ops, row0 + t, threadIdx.x, ops.kscale, k0, k1);
+      qs[d0] = q0;
+      ksm[d0] = k0;
+      if (two) { qs[d0 + 1] = q1; ksm[d0 + 1] = k1; }
     }
+    if (t + 1 < n) request(t + 1);
     __syncthreads();
     float4 part = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll

@@ -87,6 +87,46 @@ def test_recurrent_scan(dtype, H, dim, vdim):
 
 
 @pytest.mark.parametrize("dtype", DT)
+@pytest.mark.parametrize("H,dim,vdim", [(2, 64, 64), (1, 128, 128), (2, 20, 68), (1, 7, 4)])
+@pytest.mark.parametrize("turned", [False, True])
+def test_recurrent_scan_of_long_portions(dtype, H, dim, vdim, turned):
+    """Token by token where blocks are the rule: every token's q, k and v are requested a token ahead."""
+    ns, ctxs = [33, 1, 70], [4, 0, 0]
+    b = seq_ops.make_step_batch([dict(tokens=[1] * n, ctx=c, slot=s, pages=[2 * s, 2 * s + 1]) for n, c, s in zip(ns, ctxs, [2, 0, 1])])
+    qkv, state = _t(b.T, H * (2 * dim + vdim), seed=4, dtype=dtype), _t(3, H, dim, vdim, seed=5)
+    want_state, decay, out = state.double().clone(), torch.linspace(0.7, 0.95, H, device="cuda"), torch.empty(b.T, H * vdim, device="cuda")
+    angles = torch.linspace(0, 3, b.T, device="cuda", dtype=torch.float64)[:, None] * torch.linspace(1, 0.1, (dim + 7) // 8 * 4, device="cuda", dtype=torch.float64)
+    table = torch.stack([angles.cos(), angles.sin()], 1).float().contiguous() if turned else None
+    if turned:
+        seq_ops.retention(qkv, state, decay, out, b, H, dim, vdim, kscale=0.5, rotate=table, blocks=False)
+    else:
+        seq_ops.linear_attn(qkv, state, decay, out, b, H, dim, vdim, chunked=False)
+
+    def turn(x, t):
+        y = x.clone()
+        for i in range(dim // 2):
+            c, s = table[t, 0, i].double(), table[t, 1, i].double()
+            y[:, 2 * i], y[:, 2 * i + 1] = x[:, 2 * i] * c - x[:, 2 * i + 1] * s, x[:, 2 * i + 1] * c + x[:, 2 * i] * s
+        if dim % 2:  # the last element has no partner (its pair's other half is zero)
+            y[:, dim - 1] = x[:, dim - 1] * table[t, 0, dim // 2].double()
+        return y
+
+    r = 0
+    for n, c, slot in zip(ns, ctxs, [2, 0, 1]):
+        S = want_state[slot] if c else torch.zeros_like(want_state[slot])
+        for _ in range(n):
+            x = qkv[r].double() if turned else torch.nn.functional.silu(qkv[r].double())
+            q, k, v = x[: H * dim].view(H, dim), x[H * dim: 2 * H * dim].view(H, dim), x[2 * H * dim:].view(H, vdim)
+            if turned:
+                q, k = turn(q, r), turn(k, r) * 0.5
+            S = decay.double()[:, None, None] * S + k[:, :, None] * v[:, None, :]
+            _close(out[r], torch.einsum("hdv,hd->hv", S, q).reshape(-1), torch.float32, scale=20.0)
+            r += 1
+        want_state[slot] = S
+    _close(state, want_state, torch.float32, scale=20.0)
+
+
+@pytest.mark.parametrize("dtype", DT)
 @pytest.mark.parametrize("D,groups", [(128, 1), (1024, 8), (1152, 3), (2048, 4), (4096, 1), (3968, 31)])
 def test_norms_that_keep_their_row(dtype, D, groups):
     rows, eps = 5, 1e-5
