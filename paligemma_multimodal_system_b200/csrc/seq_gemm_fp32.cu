@@ -278,26 +278,16 @@ __global__ void __launch_bounds__(kRowsWarps * 32, CTAS) gemm_fp32_rows_kernel(F
 
 int part(int K, int S, int step) { return ((K + S - 1) / S + step - 1) / step * step; }  // k values of a cluster rank
 
-// SPREAD: no more CTAs to an SM than an even spread gives it: launched while the kernel before still holds most SMs, they would share the few that are free (24 tokens,
-// 2048 x 2048: 16 -> 34 us).  (228 KB an SM, 1 KB a CTA beside its own.)
-constexpr size_t kOnePerSm = 114 * 1024, kTwoPerSm = 76 * 1024;
-
-template <void (*KERNEL)(Fp32Args), bool SPREAD>
+template <void (*KERNEL)(Fp32Args)>
 cudaError_t launch(dim3 grid, int threads, size_t smem, int S, cudaStream_t st, const Fp32Args& p) {
-  // The attributes belong to the kernel, not to the call: set once a device, to the most that any call asks for, so that calls of several threads find the same.
+  // (the size belongs to the kernel: set once a device, so that calls of several threads find the same)
   static bool configured[pg::kMaxDevices] = {};
   const int dev = pg::current_device();
   if (!configured[dev]) {
-    const size_t most = SPREAD && smem < kOnePerSm ? kOnePerSm : smem;
-    cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most));
-    // (all of the SM's memory: a share sized for one such CTA would keep the next kernel's CTAs out until the SM has drained)
-    if (e == cudaSuccess && SPREAD) e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    const cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  const long long ctas = (long long)grid.x * grid.y * grid.z, sms = pg::num_sms();
-  if (SPREAD && ctas <= sms) smem = smem > kOnePerSm ? smem : kOnePerSm;
-  else if (SPREAD && ctas <= 2 * sms) smem = smem > kTwoPerSm ? smem : kTwoPerSm;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
@@ -321,8 +311,8 @@ cudaError_t launch_tile(bool wide, int S, int batch, cudaStream_t st, const Fp32
   const dim3 grid((p.F + BN - 1) / BN * S, (p.T + BM - 1) / BM, batch);
   if (grid.y > 65535) return cudaErrorInvalidConfiguration;
   const size_t smem = sizeof(float) * kStages * (BM + BN) * kPitch;
-  return wide ? launch<gemm_fp32_tile_kernel<WM, WN, TM, TN, 16>, true>(grid, WM * WN * 32, smem, S, st, p)
-              : launch<gemm_fp32_tile_kernel<WM, WN, TM, TN, 4>, true>(grid, WM * WN * 32, smem, S, st, p);
+  return wide ? launch<gemm_fp32_tile_kernel<WM, WN, TM, TN, 16>>(grid, WM * WN * 32, smem, S, st, p)
+              : launch<gemm_fp32_tile_kernel<WM, WN, TM, TN, 4>>(grid, WM * WN * 32, smem, S, st, p);
 }
 
 template <int TT, int RF, int PF, int CTAS>
@@ -333,7 +323,7 @@ cudaError_t launch_rows(int batch, int sms, cudaStream_t st, Fp32Args p) {
   int S = 1;
   while (S < 8 && tiles * batch * S < 2 * sms && p.K >= 2 * S * kRowsK) S *= 2;
   p.kpart = part(p.K, S, kRowsK);
-  return launch<gemm_fp32_rows_kernel<TT, RF, PF, CTAS>, false>(dim3(tiles * S, 1, batch), kRowsWarps * 32, sizeof(float) * 2 * TT * kRowsK, S, st, p);
+  return launch<gemm_fp32_rows_kernel<TT, RF, PF, CTAS>>(dim3(tiles * S, 1, batch), kRowsWarps * 32, sizeof(float) * 2 * TT * kRowsK, S, st, p);
 }
 
 }  // namespace
