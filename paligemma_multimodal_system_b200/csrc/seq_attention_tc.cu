@@ -490,6 +490,11 @@ int pg_attn_ragged_tc(const void* q, const void* kp, const void* vp, const void*
                       const PgAttnScore& sx, cudaStream_t st) {
   // pages that a tile of 64 keys divides, or that divide it in whole swizzle rows
   if (!(page > 0 && (page % 64 == 0 || (page % 8 == 0 && 64 % page == 0))) || sx.logistic || sx.dist_a != nullptr || sx.out_ld % 8 != 0) return 1;
+  // Blocks of 128 rows do not pay for a handful of rows in more CTAs than SMs (the mma.sync kernel's warps without rows idle; us, mma.sync / here, 16 heads of 64: 16 x 8 tokens
+  // behind 2000 57 / 72, behind 500 19 / 25; 4 x 8 tokens behind 2000 50 / 49), nor, for 64 / 128, whose S waits for P V, while that kernel's twice as many CTAs are one
+  // wave (16 heads: 400 tokens behind 2000 74 / 82, 200 tokens 12.7 / 15.4; 4 x 200 tokens, 256 CTAs, behind 500 41 / 29).
+  const long long rows = static_cast<long long>(max_n) * (H / G), units = static_cast<long long>(G) * entries;
+  if ((rows <= 16 && units > pg::num_sms()) || (dim == 64 && vdim == 128 && (rows + 63) / 64 * units <= pg::num_sms())) return 1;
 #define PG_TC(D, V) \
   if (dim == D && vdim == V) \
     return pg::launch<D, V>(q, kp, vp, gate, ldg, out, row0, n, ctx, pt, max_pages, page, entries, max_n, H, G, scale, softcap, skip_single, gate_per_head, sx, st)

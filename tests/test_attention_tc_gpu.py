@@ -47,6 +47,18 @@ def test_options(dim, vdim, opts):
     _run(dim, vdim, 2, 2, (70, 1, 129), (0, 9, 77), 100, 3, **opts)
 
 
+@pytest.mark.parametrize("ns,ctxs", [((2, 1, 33, 130), (0, 5, 63, 200)), ((300,), (0,)), ((64, 65), (64, 127)), ((5,), (1000,))])
+@pytest.mark.parametrize("window,keep", [(0, 0), (33, 0), (70, 5), (512, 130)])
+def test_masks_of_many_heads(ns, ctxs, window, keep):
+    """Heads of 64 / 128 in more CTAs than SMs (fewer stay with mma.sync, as do a handful of rows in many CTAs)."""
+    _run(64, 128, 160, 1, ns, ctxs, window, keep)
+
+
+@pytest.mark.parametrize("n", [1, 4, 5])
+def test_either_side_of_a_handful_of_rows(n):
+    _run(64, 64, 40, 4, (n, 2, n, 1), (70, 0, 300, 5), 0, 0)  # 16 and 20 rows in 160 CTAs
+
+
 def _run(dim, vdim, G, gsz, ns, ctxs, window, keep, softcap=0.0, hs=False, sink=False, gate=None, ld=False, scale=None, big=False):
     H, scale = G * gsz, dim ** -0.5 if scale is None else scale
     rows, first = [], 0
@@ -88,7 +100,7 @@ def _run(dim, vdim, G, gsz, ns, ctxs, window, keep, softcap=0.0, hs=False, sink=
 
 
 @pytest.mark.parametrize("bad", [float("nan"), float("inf")])
-@pytest.mark.parametrize("dim,vdim,G,gsz,window,keep", [(64, 64, 2, 4, 0, 0), (64, 64, 1, 1, 0, 0), (128, 128, 1, 4, 0, 0), (96, 64, 2, 1, 70, 0), (64, 128, 1, 2, 33, 40),
+@pytest.mark.parametrize("dim,vdim,G,gsz,window,keep", [(64, 64, 2, 4, 0, 0), (64, 64, 1, 1, 0, 0), (128, 128, 1, 4, 0, 0), (96, 64, 2, 1, 70, 0), (64, 128, 16, 2, 33, 40),
                                                         (128, 64, 1, 129, 0, 0), (64, 64, 3, 2, 90, 5)])
 @pytest.mark.parametrize("opts", [dict(), dict(softcap=5.0, hs=True, sink=True, gate="head", ld=True), dict(gate="row")])
 def test_values_that_are_not_finite(dim, vdim, G, gsz, window, keep, opts, bad):
