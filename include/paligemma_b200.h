@@ -328,11 +328,13 @@ int pg_prefetch_l2(const void* ptr, long long bytes, int ctas, int evict_last, v
  * ------------------------------------------------------------------------------------------------------------------- */
 
 /* fp32 products of many tokens on the tensor cores (three bf16 terms a value, 64-deep partial sums added in fp32).  pg_gemm_fp32_scratch: bytes of scratch that
- * pg_gemm_fp32_split wants for these sizes (256 MB at most: larger operands go through it block by block), 0 where the plain-FMA products are faster or the sizes do not fit (K a multiple of 8, features of 4).
+ * pg_gemm_fp32_split wants for these sizes (256 MB at most: larger operands go through it block by block), 0 where the plain-FMA products are faster or the sizes do not fit (K a multiple of 8, features of 4);
+ * pg_gemm_fp32_scratch_add: the same for a call that adds to its output, whose line lies elsewhere.
  * pg_gemm_fp32_split: out (+)= (x w^T + bias) * scale, as pg_gemm_simt_bias; rows, bases and scratch on 16-byte boundaries (else PG_ERR_ARG).  Operands keep their 24
  * bits down to about 1e-33 (16 bits are left at 2e-36), and of the terms of a product those below 2^-24 of it are dropped.  Operands that are not finite, or so large that a
  * sum could reach 2^127 (from 2^57 on for K = 2048), are computed by the plain FMAs. */
 long long pg_gemm_fp32_scratch(int tokens, int features, int K);
+long long pg_gemm_fp32_scratch_add(int tokens, int features, int K);
 int pg_gemm_fp32_split(const float* x, long long ldx, const float* w, long long ldw, float* out, long long ldo, const float* bias, int accumulate, float scale, int tokens,
                        int features, int K, void* scratch, long long scratch_bytes, void* stream);
 /* out[t, f] = sum_k x[t, k] w[f, k] with plain fp32 FMAs (no tensor-core mode): the exact-precision matrix product of

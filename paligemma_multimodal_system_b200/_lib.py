@@ -74,6 +74,7 @@ SIGNATURES = {
     "pg_rmsnorm_gate": [p, p, p, i64, p, i32, i32, f32, i32, p],
     "pg_geglu": [p, i64, p, i64, i32, i32, i32, p],
     "pg_gemm_fp32_scratch": [i32, i32, i32],
+    "pg_gemm_fp32_scratch_add": [i32, i32, i32],
     "pg_gemm_fp32_split": [p, i64, p, i64, p, i64, p, i32, f32, i32, i32, i32, p, i64, p],
     "pg_routed_ff_scratch": [p],
     "pg_routed_ff": [p, p, i64, p, i32, p, i64, p],
@@ -121,7 +122,7 @@ SIGNATURES = {
     "pg_gated_layernorm_add": [p, i64, p, i64, p, p, p, p, p, p, p, i32, i32, f32, i32, i32, p],
     "pg_glu": [p, i64, p, i64, i32, i32, i32, f32, f32, i32, p],
 }
-_RESTYPE = {"pg_launch_count": i64, "pg_gemm_fp32_scratch": i64, "pg_routed_ff_scratch": i64}
+_RESTYPE = {"pg_launch_count": i64, "pg_gemm_fp32_scratch": i64, "pg_gemm_fp32_scratch_add": i64, "pg_routed_ff_scratch": i64}
 
 
 

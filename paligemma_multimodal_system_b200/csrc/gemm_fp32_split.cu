@@ -26,6 +26,7 @@
 // seq_gemm_fp32.cu; only_if: the call is computed only where this flag is set
 int pg_gemm_fp32(const float* x, long long ldx, long long bsx, const float* w, long long ldw, long long bsw, float* out, long long ldo, long long bso,
                  const float* bias, int accumulate, float scale, int T, int F, int K, int batch, cudaStream_t st, const int* only_if);
+double pg_gemm_fp32_estimate(int T, int F, int K, int accumulate);  // us of the plain-FMA form
 
 namespace pg {
 namespace {
@@ -265,22 +266,26 @@ __global__ void __launch_bounds__(256) fp32_split_sum_kernel(const float* __rest
   *reinterpret_cast<float4*>(o) = finished(v, args.bias == nullptr ? nullptr : args.bias + f, args.scale, args.accumulate ? o : nullptr);
 }
 
-// How a call is cut, and its estimated time in clocks (split, product, sum) beside the plain-FMA form's (45 TFLOP/s).  The split of the weights (10 bytes
-// a value) is what few tokens pay for: us, FMAs / here: 64 tokens 16384 x 2048 116 / 141, 100 tokens 2048 x 2048 37 / 34, 128 tokens 8192 x 2048 115 / 85; 200 tokens
-// 1024 x 1024 25 / 26; short K 1000 tokens 2048 x 64 11 / 21.
+// How a call is cut, and whether it is the faster form.  The split of the weights (10 bytes a value) is what few tokens pay for, the rows what a short K pays for.  Both sides
+// are estimated in us; the constants were fitted to 1836 products timed in turn on both sides (32 .. 1000 tokens, 64 .. 16384 x 64 .. 8192), with this line 1.0 % slower on
+// average than the better side each time.  us, FMAs / here: 64 tokens 16384 x 2048 116 / 141, 128 tokens 8192 x 2048 115 / 85; 200 tokens 1024 x 1024 25 / 26,
+// 512 x 8192 109 / 48; added to an output: 750 tokens 16384 x 64 74 / 100, 400 tokens 2048 x 512 31 / 58.
 struct Plan { int split_k; bool use; };
-Plan plan(int T, int F, int K) {
+Plan plan(int T, int F, int K, int accumulate) {
   const int pairs = num_sms() / 2, kb = (K + kKb - 1) / kKb, tiles = ((T + kTile - 1) / kTile) * ((F + kTile - 1) / kTile);
   Plan best{1, false};
   double least = 0;
+  int steps = 0;  // 64-deep steps of the busiest pair
   for (int s = 1; s <= 16 && s <= kb; ++s) {
     const int per = (kb + s - 1) / s;
     if ((kb + per - 1) / per != s) continue;  // no empty part
-    const double clocks = static_cast<double>((tiles * s + pairs - 1) / pairs) * (per * 1700.0 + 6000.0) + (s > 1 ? 4000.0 + 4.0 * (s + 1) * T * F / 2500.0 : 0.0);
-    if (s == 1 || clocks < least) { least = clocks; best.split_k = s; }
+    const int rounds = (tiles * s + pairs - 1) / pairs;
+    const double clocks = rounds * (per * 1700.0 + 6000.0) + (s > 1 ? 4000.0 + 4.0 * (s + 1) * T * F / 2500.0 : 0.0);
+    if (s == 1 || clocks < least) { least = clocks; best.split_k = s; steps = rounds * per; }
   }
-  const double ours = least + 14000.0 + 10.0 * (static_cast<double>(F) + T) * K / 2700.0, fmas = 2.0 * T * F * static_cast<double>(K) / 22500.0 + 6000.0;
-  best.use = ours < 0.9 * fmas;
+  const double mb = 4e-6 * T * F;
+  const double ours = 18.7 + 1.95e-6 * (static_cast<double>(F) + T) * K + 2.0 * steps + 0.67 * mb * (accumulate ? 2 : 1) + (best.split_k > 1 ? 0.16 * mb * (best.split_k + 1) : 0.0);
+  best.use = ours < 0.9 * pg_gemm_fp32_estimate(T, F, K, accumulate);
   return best;
 }
 
@@ -291,13 +296,13 @@ long long scratch_of(int T, int F, int K, int split_k) { return 16 + 6LL * (stat
 constexpr long long kMaxScratch = 256LL << 20;
 
 struct Blocks { int tokens, features; Plan plan; };  // of one block; tokens 0: none fits
-Blocks blocks(int T, int F, int K) {
-  Blocks b{T, F, plan(T, F, K)};
+Blocks blocks(int T, int F, int K, int accumulate) {
+  Blocks b{T, F, plan(T, F, K, accumulate)};
   while (scratch_of(b.tokens, b.features, K, b.plan.split_k) > kMaxScratch) {
     int& larger = b.tokens > b.features ? b.tokens : b.features;
     if (larger <= kTile) return Blocks{0, 0, Plan{1, false}};
     larger = ((larger + 1) / 2 + kTile - 1) / kTile * kTile;
-    b.plan = plan(b.tokens, b.features, K);
+    b.plan = plan(b.tokens, b.features, K, accumulate);
   }
   return b;
 }
@@ -305,18 +310,20 @@ Blocks blocks(int T, int F, int K) {
 }  // namespace
 }  // namespace pg
 
-extern "C" long long pg_gemm_fp32_scratch(int tokens, int features, int K) {
+static long long scratch_where_faster(int tokens, int features, int K, int accumulate) {
   if (tokens < 32 || features < 64 || K < 64 || K % 8 != 0 || features % 4 != 0) return 0;
-  const pg::Blocks b = pg::blocks(tokens, features, K);
+  const pg::Blocks b = pg::blocks(tokens, features, K, accumulate);
   return b.plan.use ? pg::scratch_of(b.tokens, b.features, K, b.plan.split_k) : 0;
 }
+extern "C" long long pg_gemm_fp32_scratch(int tokens, int features, int K) { return scratch_where_faster(tokens, features, K, 0); }
+extern "C" long long pg_gemm_fp32_scratch_add(int tokens, int features, int K) { return scratch_where_faster(tokens, features, K, 1); }
 
 namespace pg {
 namespace {
 // one block of the call
 int split_block(const float* x, long long ldx, const float* w, long long ldw, float* out, long long ldo, const float* bias, int accumulate, float scale, int tokens, int features,
                 int K, void* scratch, long long scratch_bytes, cudaStream_t st) {
-  int split_k = plan(tokens, features, K).split_k;
+  int split_k = plan(tokens, features, K, accumulate).split_k;
   if (scratch_bytes < scratch_of(tokens, features, K, split_k)) split_k = 1;  // (the last block of a row: its parts may want more than a whole block does)
   const long long xn = 3LL * tokens * K * 2, wn = 3LL * features * K * 2;
   char* s = static_cast<char*>(scratch);
@@ -361,7 +368,7 @@ extern "C" int pg_gemm_fp32_split(const float* x, long long ldx, const float* w,
   if (tokens <= 0 || features <= 0 || K <= 0 || x == nullptr || w == nullptr || out == nullptr || scratch == nullptr) return PG_ERR_ARG;
   const uintptr_t all = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(scratch);
   if (K % 8 != 0 || features % 4 != 0 || ldx % 4 != 0 || ldw % 4 != 0 || ldo % 4 != 0 || (all & 15) != 0) return PG_ERR_ARG;
-  const Blocks b = blocks(tokens, features, K);
+  const Blocks b = blocks(tokens, features, K, accumulate);
   if (b.tokens == 0 || scratch_bytes < scratch_of(b.tokens, b.features, K, b.plan.split_k)) return PG_ERR_ARG;
   for (long long t = 0; t < tokens; t += b.tokens)
     for (long long f = 0; f < features; f += b.features) {

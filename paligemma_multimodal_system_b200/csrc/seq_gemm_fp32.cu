@@ -328,6 +328,33 @@ cudaError_t launch_rows(int batch, int sms, cudaStream_t st, Fp32Args p) {
 
 }  // namespace
 
+// The tile and the number of cluster ranks whose busiest SM has the least to do (that in return: outputs times k steps); smaller tiles read shared memory more often per FMA.
+static float cheapest_tile(int T, int F, int K, int batch, int& best, int& S) {
+  struct Form { int bm, bn; float weight; };
+  const Form forms[3] = {{64, 128, 1.0f}, {64, 64, 1.05f}, {32, 64, 1.3f}};
+  const int sms = pg::num_sms();
+  float least = 0.f;
+  best = 0;
+  S = 1;
+  for (int i = 0; i < 3; ++i) {
+    if (i > 0 && (T + forms[i].bm - 1) / forms[i].bm > 65535) break;
+    for (int s = 1; s <= 8; s *= 2) {
+      if (s > 1 && K < s * 8 * kStep) break;
+      const long long ctas = (long long)((F + forms[i].bn - 1) / forms[i].bn) * ((T + forms[i].bm - 1) / forms[i].bm) * batch * s;
+      // a rank that joins the others' sums costs about as much as 48 k values more
+      const float cost = (float)((ctas + sms - 1) / sms) * forms[i].bm * forms[i].bn * (part(K, s, kStep) + (s > 1 ? 48 : 0)) * forms[i].weight;
+      if ((i == 0 && s == 1) || cost < least) { least = cost; best = i; S = s; }
+    }
+  }
+  return least;
+}
+
+// us of a product of more than 16 tokens by the tiles (20 tokens to 1000, 64 to 16384 wide and 64 to 8192 deep: half of them within 10 %)
+double pg_gemm_fp32_estimate(int T, int F, int K, int accumulate) {
+  int best, S;
+  return 5.6 + 6.8e-6 * cheapest_tile(T, F, K, 1, best, S) + 0.28e-6 * 4.0 * T * F * (accumulate ? 2 : 1);
+}
+
 // batch independent products (bsx / bsw / bso: elements between their operands).  Returns PG_ERR_ARG for what no grid can express.
 int pg_gemm_fp32(const float* x, long long ldx, long long bsx, const float* w, long long ldw, long long bsw, float* out, long long ldo, long long bso,
                  const float* bias, int accumulate, float scale, int T, int F, int K, int batch, cudaStream_t st,
@@ -347,21 +374,8 @@ int pg_gemm_fp32(const float* x, long long ldx, long long bsx, const float* w, l
         : T <= 8 ? launch_rows<8, 2, 4, 2>(batch, sms, st, p)
                  : launch_rows<16, 4, 4, 1>(batch, sms, st, p);
   } else {
-    // the tile and the number of cluster ranks whose busiest SM has the least to do; smaller tiles read shared memory more often per FMA
-    struct Form { int bm, bn; float weight; };
-    const Form forms[3] = {{64, 128, 1.0f}, {64, 64, 1.05f}, {32, 64, 1.3f}};
-    int best = 0, S = 1;
-    float least = 0.f;
-    for (int i = 0; i < 3; ++i) {
-      if (i > 0 && (T + forms[i].bm - 1) / forms[i].bm > 65535) break;
-      for (int s = 1; s <= 8; s *= 2) {
-        if (s > 1 && K < s * 8 * kStep) break;
-        const long long ctas = (long long)((F + forms[i].bn - 1) / forms[i].bn) * ((T + forms[i].bm - 1) / forms[i].bm) * batch * s;
-        // a rank that joins the others' sums costs about as much as 48 k values more
-        const float cost = (float)((ctas + sms - 1) / sms) * forms[i].bm * forms[i].bn * (part(K, s, kStep) + (s > 1 ? 48 : 0)) * forms[i].weight;
-        if ((i == 0 && s == 1) || cost < least) { least = cost; best = i; S = s; }
-      }
-    }
+    int best, S;
+    cheapest_tile(T, F, K, batch, best, S);
     p.kpart = part(K, S, kStep);
     e = best == 0   ? launch_tile<2, 2, 8, 8>(wide, S, batch, st, p)
         : best == 1 ? launch_tile<2, 2, 8, 4>(wide, S, batch, st, p)

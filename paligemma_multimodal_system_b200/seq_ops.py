@@ -163,7 +163,7 @@ def _linear_fp32_split(x, w, out, bias, accumulate, scale):
     F = w.shape[0]
     if not (x.is_cuda and w.is_cuda and _aligned(x) and _aligned(w) and _aligned(out)) or (x.stride(0) | w.stride(0) | out.stride(0)) % 4:
         return False
-    need = _lib.lib().pg_gemm_fp32_scratch(T, F, K)
+    need = (_lib.lib().pg_gemm_fp32_scratch_add if accumulate else _lib.lib().pg_gemm_fp32_scratch)(T, F, K)
     if not need:
         return False
     try:
