@@ -45,6 +45,7 @@ struct Params {
   const int* key_lens;  // optional [B]: problem b only attends to its first key_lens[b] keys (ragged prompts); else nullptr
   int stagger;          // QT = 2 (tuning): clock cycles the softmax group of query tile 1 idles after its first S tile is ready
   long long* trace;     // optional clock64 stamps of CTA (0,0,0): [role][tile][event]
+  int trigger;          // the next kernel may come (weights_follow)
 };
 
 template <int DH, int QT>
@@ -223,7 +224,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_gen;
-  griddep_wait();
+  griddep_begin_if(p.trigger);  // (tensor memory is held by now: a product behind this kernel cannot take it first)
   // ragged batches: keys [key_lens[b], keys) of problem b exist in memory (padding tokens, finite values) but weigh nothing
   const int n_keys = p.key_lens ? max(1, min(p.keys, __ldg(p.key_lens + b))) : p.keys;
   const int n_tiles = (n_keys + BN - 1) / BN;
@@ -596,6 +597,7 @@ int pg_attention_prefill_tc(const void* q, const void* k, const void* v, void* o
   p.sl2 = scale * 1.4426950408889634f;
   p.key_lens = key_lens;
   p.trace = g_trace;
+  p.trigger = weights_follow();
   p.stagger = g_stagger;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   // softmax warps per TMEM lane quadrant: two (column halves) for the one-tile dh <= 128 variant, else one

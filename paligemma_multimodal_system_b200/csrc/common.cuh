@@ -150,13 +150,18 @@ PG_DEVINL void griddep_launch_dependents() { asm volatile("griddepcontrol.launch
 //   * griddep_begin(): waits; the next kernel comes when this one has ended, as after a plain launch, but with its launch behind it.  Everything that writes 16-bit rows (they can be
 //     the weight operand of the product behind), pages or positions.
 //   * griddep_begin<true>(): waits, then triggers.  Kernels whose results are fp32 rows and integers that are read behind a wait only (routing, scans).
-// What it costs, every kernel triggering ahead of its wait / behind it / this: tower of four layers, one image 252 / 246 / 252 us, 48 requests with 24 decode steps 16.5 / 16.4 /
-// 16.9 ms, a routed feed-forward 91 us all three.
+//   * griddep_begin_if(weights_follow()): where a whole layer is issued by one call (layers.cu) it is known that the product behind a norm or an attention takes a weight.
+// What that costs against every kernel triggering ahead of its wait: 48 requests with 24 decode steps 16.5 -> 16.9 ms, one request through four narrow layers 5 %; a tower of
+// four layers, one image 252 -> 247 us, a routed feed-forward 91 us both.
 // (Products trigger behind their wait: their outputs are not weights.  rmsnorm_kernel of the Gemma decode chain triggers early: see there.)
 template <bool TRIGGER = false>
 PG_DEVINL void griddep_begin() {
   griddep_wait();
   if (TRIGGER) griddep_launch_dependents();
+}
+PG_DEVINL void griddep_begin_if(int trigger) {  // trigger: weights_follow() of the launch
+  griddep_wait();
+  if (trigger) griddep_launch_dependents();
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -328,6 +333,15 @@ inline int num_sms() {
   }
   return sms[dev];
 }
+
+// While a thread issues whole layers by one call (layers.cu) the product behind a norm or an attention is that layer's, and its operand a weight: there they trigger behind their
+// wait.  Counted per thread, for the length of that call.
+inline thread_local int t_weights_follow = 0;
+inline int weights_follow() { return t_weights_follow > 0 ? 1 : 0; }
+struct WeightsFollow {
+  WeightsFollow() { ++t_weights_follow; }
+  ~WeightsFollow() { --t_weights_follow; }
+};
 
 // Host-side launch through cudaLaunchKernelEx, as a programmatic dependent launch unless that is switched off (the caller counts it).  Every kernel launched this
 // way executes griddepcontrol.wait before its first dependent global access.

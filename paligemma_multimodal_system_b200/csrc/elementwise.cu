@@ -34,8 +34,8 @@ PG_DEVINL float block_sum(float v, float* red) {
 // ---------------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) layernorm_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
                                                         const float* __restrict__ beta, bf16* __restrict__ y_bf,
-                                                        float* __restrict__ y_f, int D, float eps) {
-  pg::griddep_begin();
+                                                        float* __restrict__ y_f, int D, float eps, int trigger) {
+  pg::griddep_begin_if(trigger);
   extern __shared__ float row[];  // D floats + 33
   float* red = row + D;
   const long long r = blockIdx.x;
@@ -99,8 +99,8 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* __restrict__ 
 template <int NV>
 __global__ void __launch_bounds__(256) layernorm_warp_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
                                                              const float* __restrict__ beta, bf16* __restrict__ y_bf,
-                                                             float* __restrict__ y_f, int rows, int D, float eps) {
-  pg::griddep_begin();
+                                                             float* __restrict__ y_f, int rows, int D, float eps, int trigger) {
+  pg::griddep_begin_if(trigger);
   const int lane = threadIdx.x & 31;
   const long long r = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (r >= rows) return;
@@ -140,8 +140,8 @@ __global__ void __launch_bounds__(256) layernorm_warp_kernel(const float* __rest
 
 template <int NV>
 __global__ void __launch_bounds__(256) rmsnorm_warp_kernel(const float* __restrict__ x, const float* __restrict__ w,
-                                                           bf16* __restrict__ y, int rows, int D, float eps) {
-  pg::griddep_begin();
+                                                           bf16* __restrict__ y, int rows, int D, float eps, int trigger) {
+  pg::griddep_begin_if(trigger);
   const int lane = threadIdx.x & 31;
   const long long r = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (r >= rows) return;
@@ -457,10 +457,10 @@ extern "C" int pg_layernorm(const float* x, const float* gamma, const float* bet
   const bool al = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(beta) |
                     reinterpret_cast<uintptr_t>(y_bf16) | reinterpret_cast<uintptr_t>(y_f32)) & 15) == 0;
   if (rows >= 1024 && (D % 128) == 0 && D <= 2048 && al) {  // prefill: one warp per row, the row stays in registers
-    pg::launch_dependent(layernorm_warp_kernel<16>, (rows + 7) / 8, 256, 0, PG_ST(stream), x, gamma, beta, static_cast<bf16*>(y_bf16), y_f32, rows, D, eps);
+    pg::launch_dependent(layernorm_warp_kernel<16>, (rows + 7) / 8, 256, 0, PG_ST(stream), x, gamma, beta, static_cast<bf16*>(y_bf16), y_f32, rows, D, eps, pg::weights_follow());
     PG_RET();
   }
-  pg::launch_dependent(layernorm_kernel, rows, 256, (D + 33) * sizeof(float), PG_ST(stream), x, gamma, beta, static_cast<bf16*>(y_bf16), y_f32, D, eps);
+  pg::launch_dependent(layernorm_kernel, rows, 256, (D + 33) * sizeof(float), PG_ST(stream), x, gamma, beta, static_cast<bf16*>(y_bf16), y_f32, D, eps, pg::weights_follow());
   PG_RET();
 }
 
@@ -471,7 +471,7 @@ extern "C" int pg_rmsnorm(const float* x, const float* w, void* y_bf16, int rows
   if (rows <= 0 || D <= 0 || (D % 4) != 0 || D > 8192) return PG_ERR_ARG;
   if (rows >= 1024 && (D % 128) == 0 && D <= 2048 &&
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y_bf16)) & 15) == 0) {
-    pg::launch_dependent(rmsnorm_warp_kernel<16>, (rows + 7) / 8, 256, 0, PG_ST(stream), x, w, static_cast<bf16*>(y_bf16), rows, D, eps);
+    pg::launch_dependent(rmsnorm_warp_kernel<16>, (rows + 7) / 8, 256, 0, PG_ST(stream), x, w, static_cast<bf16*>(y_bf16), rows, D, eps, pg::weights_follow());
     PG_RET();
   }
   return launch_kernel(rmsnorm_kernel, dim3(rows), dim3(256), (D + 33) * sizeof(float), PG_ST(stream), x, w,

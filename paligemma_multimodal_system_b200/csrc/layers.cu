@@ -58,6 +58,7 @@ extern "C" int pg_linear_f32(const void* x, long long ldx, const void* w, long l
 extern "C" int pg_siglip_layers(const PgSiglipLayer* layers, int count, float* x, void* hn, void* qkv, void* att, void* mid, int images, int patches,
                                 int D, int F, int heads, float eps, void* stream) {
   if (layers == nullptr || count < 0 || images <= 0 || patches <= 0 || heads <= 0 || D <= 0 || D % heads != 0) return PG_ERR_ARG;
+  const pg::WeightsFollow chain;
   const int M = images * patches, dh = D / heads;
   const long long N = patches, D3 = 3LL * D;
   const char* q = static_cast<const char*>(qkv);
@@ -77,6 +78,7 @@ extern "C" int pg_siglip_layers(const PgSiglipLayer* layers, int count, float* x
 
 extern "C" int pg_gemma_prefill_layers(const PgGemmaLayer* layers, int count, const PgGemmaPrefill* a, void* stream) {
   if (layers == nullptr || a == nullptr || count < 0 || a->B <= 0 || a->S <= 0 || a->Hkv <= 0 || a->Hq % a->Hkv != 0) return PG_ERR_ARG;
+  const pg::WeightsFollow chain;
   const int T = a->B * a->S, D = a->D, F = a->F, Hq = a->Hq, Hkv = a->Hkv, dh = a->dh, G = Hq / Hkv, swap = T > 128 ? 0 : 1;
   const long long W = (Hq + 2LL * Hkv) * dh, S = a->S, qs = a->fused ? W : (long long)Hq * dh, kvs = a->fused ? W : (long long)Hkv * dh, os = (long long)Hq * dh;
   const char* qkv = static_cast<const char*>(a->qkv);
