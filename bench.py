@@ -4,7 +4,7 @@
     python bench.py --gpus N --steps K --warmup W            # this repo's sm_100a path
     python bench.py --impl reference --gpus N ...            # the reference's own CPU path on the host cores
 
-Workload = BASELINE.json configs[2]: 3B-224 architecture (random init, bf16-representable, regime R2), 64 requests per
+Workload: 3B-224 architecture (random init, bf16-representable, regime R2), 64 requests per
 GPU (weak scaling: batch-sharded replicas, no collective on the data path), prompt `<image>*256 <bos> t1 t2 \\n`
 (S = 260), temperature 0.8 / top-p 0.9 sampling, 128 generated tokens.  One "step" = one whole generate() job
 (prefill of 64 images + 127 graph-replayed decode steps).
@@ -15,9 +15,9 @@ GPU (weak scaling: batch-sharded replicas, no collective on the data path), prom
               inside the timed region, prefill included (all 128 tokens counted).
   roofline    dominant kernel (gate||up weight-streaming tcgen05 GEMM of the decode step) timed alone with CUDA events, rotating over the 18 layers' weights
               (2.4 GB > L2) against the measured HBM peak; `roofline_step` is the whole decode step (5.40 GB algorithmic
-              bytes, SURVEY.md 8(d)) from the graph replays of the timed region.
-  configs     the other BASELINE.json configurations measured in the same process: cfg2 (B = 1 greedy-32 latency),
-              cfg4 (448 px, 32 requests), cfg5 (896 px, 8 requests), and the strong-scaling split of configs[2]
+              bytes) from the graph replays of the timed region.
+  configs     the other configurations measured in the same process: cfg2 (B = 1 greedy-32 latency),
+              cfg4 (448 px, 32 requests), cfg5 (896 px, 8 requests), and the strong-scaling split of the main workload
               (global batch 64 => 64 / N requests per GPU).
   parity      measured GPU-vs-oracle figures at the 3B widths (profiles/parity_r02.json, written by tests/test_bench_3b_gpu.py).
   cpu_baseline  the UNMODIFIED reference (staged under baseline/_ref, kind "reference") or, when that copy is absent, the
@@ -49,7 +49,7 @@ TRAFFIC_CAPTURE = os.path.join(ROOT, "profiles", "r02i_decode_gemm_ncu_full.csv"
 
 
 def algorithmic_bytes_per_decode_step(cfg, batch, kv_len_avg):
-    """every LM weight once (bf16) + KV read + KV write; vision tower / dead logits excluded."""
+    """Every LM weight once (bf16) + KV read + KV write; vision tower / dead logits excluded."""
     tc = cfg["text_config"]
     D, F, L, V = tc["hidden_size"], tc["intermediate_size"], tc["num_hidden_layers"], tc["vocab_size"]
     Hq, Hkv, dh = tc["num_attention_heads"], tc["num_key_value_heads"], tc["head_dim"]
@@ -61,7 +61,7 @@ def algorithmic_bytes_per_decode_step(cfg, batch, kv_len_avg):
 
 
 def algorithmic_flops_per_image(cfg, S):
-    """full non-causal attention as in the reference, last-position lm_head only."""
+    """Full non-causal attention as in the reference, last-position lm_head only."""
     vc, tc = cfg["vision_config"], cfg["text_config"]
     Dv, Fv, Lv = vc["hidden_size"], vc["intermediate_size"], vc["num_hidden_layers"]
     N = (vc["image_size"] // vc["patch_size"]) ** 2
@@ -186,7 +186,7 @@ def time_dominant_kernel(model, batch, iters=3):
 
 
 # ----------------------------------------------------------------------------------------------------------------------
-# CPU arms: the unmodified reference (baseline/_ref, staged by __graft_entry__.build() where /root/reference exists) or the
+# CPU arms: the unmodified reference (baseline/_ref, staged by __graft_entry__.build() where the reference is mounted) or the
 # oracle port
 # ----------------------------------------------------------------------------------------------------------------------
 def reference_staged():
@@ -194,7 +194,7 @@ def reference_staged():
 
 
 def load_reference(cfg, sd_cpu):
-    """The reference's own classes from baseline/_ref (an unmodified copy of /root/reference/*.py), its stock constructor,
+    """The reference's own classes from baseline/_ref (an unmodified copy of its modules), its stock constructor,
     load_state_dict and tie_weights.  `fire` (its CLI dependency, absent from this image) is stubbed: the CLI is not on the path."""
     import copy
     if REF_DIR not in sys.path:
@@ -211,7 +211,7 @@ def load_reference(cfg, sd_cpu):
 
 @torch.no_grad()
 def cpu_reference_sample(ref, inp, new_tokens, do_sample):
-    """The stock loop of inference.py:45-79 at model level (B = 1: the reference cannot decode a batch, SURVEY 8(c)), its own
+    """The stock loop of inference.py:45-79 at model level (B = 1: the reference cannot decode a batch), its own
     forward / KVCache / _sample_top_p, stdout silenced (the reference prints shapes).  Vision tower re-run every step, as it does."""
     model, KVCache, ref_inference = ref
     ids, mask, px = inp["input_ids"], inp["attention_mask"], inp["pixel_values"]
@@ -272,7 +272,7 @@ def cpu_baseline_entry(cfg, sd_cpu, threads, tokens, do_sample):
 
 
 def measure_serving(model, cfg, n_requests=256, slots=64, stage=32, min_admit=16, steps_per_replay=8, greedy=False, static=True):
-    """a ragged request stream (text prompts of 2..12 tokens, token budgets uniform in [16, 128] standing
+    """A ragged request stream (text prompts of 2..12 tokens, token budgets uniform in [16, 128] standing
     in for EOS-terminated answers) through serving.ContinuousBatcher, beside static batching of the same stream through
     generate() (arrival order, `slots` at a time, each batch runs to its longest budget; one prompt length per batch, i.e.
     with perfect length bucketing).  Useful tokens = sum of the budgets in both arms; wall clock around the whole stream,
@@ -523,7 +523,7 @@ def main():
             except Exception as e:  # a reported extra, never allowed to take the headline line down
                 serving = {"error": f"{type(e).__name__}: {e}"}
 
-    # ---------------- the other BASELINE configurations, same process ----------------
+    # ---------------- the other configurations, same process ----------------
     # [cfg2 prefill, cfg2 decode, strong prefill, strong decode, cfg4 prefill, cfg4 decode, cfg5 prefill, cfg5 decode]
     extra = [0.0] * 8
     extra_meta = {}
@@ -532,7 +532,7 @@ def main():
         greedy = dict(do_sample=False)
         pre2, dec2, _ = time_generate(model, cfg, 1, 32, greedy, runs=5, warmup=3)            # cfg-2: latency path
         extra[0], extra[1] = pre2 / 5, dec2 / 5
-        bs = max(1, BATCH_PER_GPU // world)                                                   # strong scaling of configs[2]
+        bs = max(1, BATCH_PER_GPU // world)                                                   # strong scaling of the main workload
         if world == 1:
             extra[2], extra[3] = pre_ms / args.steps, dec_ms / args.steps
         else:

@@ -204,7 +204,7 @@ int pg_attention_prefill(const void* q, const void* k, const void* v, void* o, i
                          long long o_hs, long long o_head_off, float scale, void* stream);
 
 /*
- * pg_attention_prefill for a ragged batch (SURVEY 8(f) rank 1: prompts of different lengths in one prefill; the reference
+ * pg_attention_prefill for a ragged batch (prompts of different lengths in one prefill; the reference
  * runs B = 1, inference.py:69, and never masks padding, modeling_paligemma.py:154-156): problem b attends only to its first
  * key_lens[b] keys (int32 [B] on the device, clamped to [1, keys]).  Rows past a problem's length are computed and must be
  * ignored by the caller; K/V rows in [key_lens[b], keys) must hold finite values.  tcgen05 kernel only (dh 64 / 72 / 256,

@@ -4,8 +4,8 @@ A plain-PyTorch (CPU, fp32) restatement of the algorithm of prtk1729/Paligemma-M
 PaliGemmaForConditionalGeneration.forward + KVCache + the inference.py sampling loop.  Only tests/, __graft_entry__.smoke()
 and bench.py's cpu_baseline / `--impl reference` legs may import this module; the product package never does.
 
-Parity pin: the reference has NO tests / golden vectors for this path (SURVEY.md 4, 8(c)), so this restatement is pinned
-against outputs of the UNMODIFIED reference itself, executed in the build container by tests/golden/make_golden.py
+Parity pin: the reference has NO tests / golden vectors for this path, so this restatement is pinned
+against outputs of the UNMODIFIED reference itself, executed by tests/golden/make_golden.py
 (fixtures committed under tests/golden/, checked by tests/test_oracle_golden.py on every run).
 
 It is written functionally over a state dict that uses the reference's parameter names.  Each function cites the

@@ -3,7 +3,7 @@
     image.resize((S, S), resample=Image.Resampling.BICUBIC)   (:17-19)   -> np.array(image.convert("RGB"))   (:52)
     -> * 1/255 as float32  (:21-23, 56-59)  -> (x - 0.5) / 0.5  (:25-33, 64-68)  -> HWC -> CHW  (:71)
 
-The resize itself lives in a third-party dependency that is not part of /root/reference: Pillow (no version is pinned by
+The resize itself lives in a third-party dependency that is not part of the reference: Pillow (no version is pinned by
 the reference; this image ships Pillow 12.2.0).  Its published algorithm for 8-bit images (src/libImaging/Resample.c:
 precompute_coeffs, normalize_coeffs_8bpc, ImagingResampleHorizontal_8bpc / Vertical_8bpc) is restated here in numpy:
 per output pixel a window of `support = 2 * max(scale, 1)` input pixels either side of the centre, weights from the

@@ -1,6 +1,6 @@
 """Builds libpaligemma_b200.so (every .cu under csrc/) for sm_100a with nvcc, in-tree.
 
-nvcc cross-compiles without a GPU; the resulting .so travels to the GPU box with the repo snapshot.
+nvcc cross-compiles without a GPU; the resulting .so stays in the tree.
 """
 import hashlib
 import os

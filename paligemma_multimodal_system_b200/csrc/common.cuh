@@ -87,7 +87,7 @@ PG_DEVINL bool mbar_try_wait(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait: a protocol bug traps (CUDA error) instead of hanging the GPU box.
+// Bounded wait: a protocol bug traps (CUDA error) instead of hanging the GPU.
 PG_DEVINL void mbar_wait(uint32_t bar, uint32_t parity) {
   if (mbar_try_wait(bar, parity)) return;
   long long t0 = clock64();
@@ -361,7 +361,7 @@ inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 bl
 }
 
 // For kernels that run long with few CTAs per SM: behind the whole of the kernel before.  CTAs that become resident while that one still holds most SMs share the few
-// that are free, and stay there (an fp32 product of 24 tokens behind the merge of a decode attention: 16 -> 34 us).
+// that are free, and stay there (an fp32 product of 24 tokens behind a kernel that triggered early: 16 -> 34 us).
 template <typename... KArgs, typename... Args>
 inline void launch_spread(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
   kernel<<<grid, block, smem, st>>>(static_cast<KArgs>(args)...);

@@ -1237,7 +1237,8 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& 
 //   activations (bf16 rows): this file's one-CTA kernel (640 clocks a 64-deep step, 4500 a tile).  8192 x 2048, 640 tokens 36.4 / 23.0; 16384 x 2048, 1408 tokens 84.6 / 99.2.
 //   fewer than 74 pair tiles: 3456 x 1152, 263 tokens 14.4 / 8.2; 2048 x 16384 with residual, 1300 tokens 163 / 86.  (Plain bf16 rows of a short K that three and more share
 //     lose a little: 512 x 512, 1200 tokens 6.6 / 7.3; 1152 x 1152, 769 tokens 10.0 / 10.8, 400 tokens 9.4 / 8.2.)
-//   else the pair kernel (740 clocks a step, 1500 a tile).  A second wave of CTAs starts one by one, not as a whole, and fp32 rows with their residual are moved after
+//   else the pair kernel (740 clocks a step, 1500 a tile: fitted, like the 640 above, when one lane of a warp issued every product; an elected lane takes 560, which only the
+//     line for activations of a long K reckons with -- the others have not been fitted again and may send a product of many features to the slower side).  A second wave of CTAs starts one by one, not as a whole, and fp32 rows with their residual are moved after
 //     the products of a tile and not beside them: 12 % more, bf16 rows 20, fp32 rows 30.  8192 x 2048: bf16 640 tokens 27.8 / 21.0, 1200 tokens 38.4 / 40.5; residual 640
 //     tokens 34.6 / 26.9, 1200 tokens 48.7 / 56.1; 16384 x 2048 residual 1025 tokens 78.1 / 96.0; gate || up 32768 x 2048 263 tokens 54 / 39, 1024 tokens 101 / 133.
 //

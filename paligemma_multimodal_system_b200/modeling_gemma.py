@@ -386,7 +386,7 @@ class GemmaForCausalLM(nn.Module):
         attention, O GEMM, RMSNorm, gate||up GEGLU GEMM, down GEMM (+ one L2 weight prefetch on a forked stream, see below); the three small-output GEMMs split K over CTAs and
         red.add their fp32 partials straight into the residual stream / the zeroed `qkv` accumulator, which the o_proj launch
         resets for the next layer.  (Folding the norms into the GEMMs -- the consumer converting the fp32 residual stream into its
-        own bf16 operand tiles -- was built and measured: slower)
+        own bf16 operand tiles -- was built and measured: slower.)
         Then the final RMSNorm and the lm_head (modeling_gemma.py:523-525), whose epilogue also leaves the softmax statistics
         of every 32-token vocabulary segment at `inv_temperature` in bufs['stats'] (pg_sample_top_p_stats / pg_argmax_stats).
         Every launch reads its sizes from device counters, so the sequence can be captured in a CUDA graph."""

@@ -1,9 +1,8 @@
-"""PaliGemmaProcessor with the reference's interface (processing_paligemma.py:94-212): upstream of the hot path
-(SURVEY.md 8(f) "next" rows 3-4), kept as thin host code so that `inference.test_inference` is usable with a real
+"""PaliGemmaProcessor with the reference's interface (processing_paligemma.py:94-212): upstream of the hot path, kept as thin host code so that `inference.test_inference` is usable with a real
 tokenizer.  Image path: bicubic resize -> /255 -> (x - 0.5) / 0.5 -> CHW float32; text path:
 `<image>` * N + bos + prompt + "\\n" (processing_paligemma.py:77-89), tokenised by the caller's HF tokenizer.
 
-Deliberate fixes relative to the reference, both noted in SURVEY.md: batches of prompts/images are accepted (the
+Deliberate fixes relative to the reference: batches of prompts/images are accepted (the
 reference asserts exactly one, :174), and each prompt string itself is formatted into the template (the reference
 formats the *list*, :197, producing "...<bos>['caption en']\\n").
 """

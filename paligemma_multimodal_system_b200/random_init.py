@@ -4,7 +4,7 @@
 modeling_paligemma.py:71-90 / modeling_siglip.py / modeling_gemma.py), every value rounded to a bf16-representable
 fp32 number so that the fp32 CPU reference, the oracle and the bf16 GPU model hold IDENTICAL weights.
 
-Init regimes (SURVEY.md 8(c)):
+Init regimes:
   R0  "literal"  : PyTorch default init distributions (Linear/Conv2d U(+-1/sqrt(fan_in)), Embedding N(0,1),
                    LayerNorm 1/0, GemmaRMSNorm 0 as in modeling_gemma.py:163)
   R1  "wellcond" : tied embedding N(0, 0.02), LM matrices N(0, 1/sqrt(fan_in)), vision tower as R0
@@ -107,7 +107,7 @@ def make_state_dict(config: dict, regime: str = "R1", seed: int = 0, device="cpu
 
 
 def make_inputs(config: dict, batch: int, prompt_len: int = 4, seed: int = 0, device="cpu"):
-    """Synthetic request batch (SURVEY.md 8(d)): `<image>`*N + bos(2) + random prompt tokens + "\\n"(108); all-ones
+    """Synthetic request batch: `<image>`*N + bos(2) + random prompt tokens + "\\n"(108); all-ones
     attention mask; pixel values uniform in [-1, 1], bf16-representable.  Row r is seeded with seed + r."""
     vc, tc = config["vision_config"], config["text_config"]
     N = (vc["image_size"] // vc["patch_size"]) ** 2

@@ -465,7 +465,9 @@ def attn_ragged(q, k_pages, v_pages, gate, out, b: StepBatch, H, G, dim, vdim, s
                                               vdim, gph, 0, 0, _lib.stream()), "pg_attn_decode_merge")
     elif singles and not skip_singles:
         tiles = (reach - 1) // 32 + 1
-        # three CTAs of four warps per SM at once: what one wave holds, and at least two 32-key tiles for every warp
+        # three CTAs of four warps per SM at once: what one wave holds, and at least two 32-key tiles for every warp.  The general kernel has eight warps and two CTAs an SM, and
+        # takes the same split: us, this / two waves of CTAs with two tiles a warp, bf16 128 / 256 64 x 2250 318 / 347, 1 x 3000 89 / 134; fp32 latent 288 / 256 5 x 1100
+        # 681 / 1099, 1 x 3000 795 / 1307
         nsplit = max(1, min(3 * _lib.num_sms() // (G * singles), tiles // 8, 32))
         partial = torch.empty(b.E * H * nsplit * (vdim + 2), device="cuda", dtype=torch.float32) if nsplit > 1 else None
         _lib.check(L.pg_attn_decode(q.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), _lib.ptr(gate), ldg, out.data_ptr(), _lib.ptr(partial),

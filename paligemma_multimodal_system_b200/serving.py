@@ -1,4 +1,4 @@
-"""Variable-length prompts and continuous batching on top of the paged KVCache (SURVEY 8(f) rank 1).
+"""Variable-length prompts and continuous batching on top of the paged KVCache.
 
 The reference loop (inference.py:45-79) serves ONE request (`assert next_token.size() == (1, 1)`, :69): prefill, then one
 token per step until EOS has been appended (:71-74) or `max_tokens_to_generate` is reached.  Here B such loops share one

@@ -1,6 +1,6 @@
 """load_hf_model with the reference's signature (utils.py:9-37): safetensors shards + config.json -> packed bf16 model.
 
-SURVEY.md 8(f) "next" row 2.  Like the reference it reads every `*.safetensors` shard, builds the model from
+Like the reference it reads every `*.safetensors` shard, builds the model from
 `config.json`, loads the tensors and ties the weights.  Where the reference's `strict=False` hides real differences, this
 loader accounts for every key instead:
 

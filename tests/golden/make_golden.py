@@ -1,6 +1,6 @@
-"""Generates tests/golden/*.npz by executing the UNMODIFIED reference (/root/reference) on CPU fp32.
+"""Generates tests/golden/*.npz by executing the UNMODIFIED reference (read from /root/reference) on CPU fp32.
 
-Run in the build container only (the GPU box has no /root/reference):
+Run where the reference is mounted:
     python tests/golden/make_golden.py
 Weights and inputs come from paligemma_multimodal_system_b200.random_init (seeded, bf16-representable), loaded into the
 reference modules with load_state_dict(strict=True) + tie_weights(), so tests can rebuild the identical state dict.

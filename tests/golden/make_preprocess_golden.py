@@ -1,6 +1,6 @@
 """Writes tests/golden/preprocess_reference.npz: outputs of the UNMODIFIED reference process_images
-(/root/reference/processing_paligemma.py:36-73, i.e. Pillow's bicubic resize + numpy rescale / normalise / transpose)
-on small seeded synthetic images.  Run in the build container (needs /root/reference and Pillow)."""
+(processing_paligemma.py:36-73, i.e. Pillow's bicubic resize + numpy rescale / normalise / transpose)
+on small seeded synthetic images.  Run where the reference is mounted at /root/reference and Pillow is installed."""
 import os
 import sys
 
@@ -20,7 +20,7 @@ def make_image(H, W, seed):
 def main():
     from PIL import Image
     sys.path.insert(0, "/root/reference")
-    import processing_paligemma as ref  # the unmodified reference (build container only)
+    import processing_paligemma as ref  # the unmodified reference (where it is mounted)
     out = {}
     for i, (H, W, S) in enumerate(CASES):
         img = make_image(H, W, 100 + i)

@@ -1,6 +1,6 @@
-"""Generates tests/golden/serving_reference.npz by executing the UNMODIFIED reference (/root/reference) on CPU fp32.
+"""Generates tests/golden/serving_reference.npz by executing the UNMODIFIED reference on CPU fp32.
 
-Run in the build container only:  python tests/golden/make_serving_golden.py
+Run where the reference is mounted:  python tests/golden/make_serving_golden.py
 The reference serves one request at a time (inference.py:69), so every request of the ragged stream
 (random_init.make_requests) is run through its loop on its own, unpadded: these are the answers a continuous batcher must
 reproduce row by row (tests/test_serving_gpu.py) and the oracle must reproduce on CPU (tests/test_oracle_golden.py).
@@ -13,7 +13,7 @@ import torch
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, HERE)
-from make_golden import build_reference, run_reference_loop  # noqa: E402  (also puts /root/reference on sys.path)
+from make_golden import build_reference, run_reference_loop  # noqa: E402  (also puts the reference on sys.path)
 
 from paligemma_multimodal_system_b200.random_init import TINY_CONFIG, make_requests, make_state_dict  # noqa: E402
 

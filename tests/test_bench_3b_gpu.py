@@ -6,7 +6,7 @@
     against the oracle's kept set;
   * 3B-448 (1024 image tokens) and 3B-896 (4096 image tokens), B = 1: prefill + 4 teacher-forced decode steps.
 
-Tolerance (north_star: bf16 tolerance stated in the test): last-position logits cosine >= 0.9999 and max-abs <= 1 % of the
+Tolerance (bf16): last-position logits cosine >= 0.9999 and max-abs <= 1 % of the
 oracle logit absmax in R1; cosine >= 0.999 and <= 3 % in the diffuse regime R2; greedy tokens identical to the oracle's
 whenever its top-2 margin exceeds 4x the measured error (all 32 steps in R1).  Every measured figure is also written to
 build/parity_r02.json (copied to profiles/parity_r02.json, which bench.py attaches to its line as `parity`)."""
@@ -93,7 +93,7 @@ def test_3b_greedy_32_tokens_identical_and_batch_rows_independent(setup_3b):
 
 
 # ---------------------------------------------------------------------------------------------------------------------
-# the benchmarked workload (BASELINE configs[2]): R2, 64 requests, S = 260
+# the benchmarked workload: R2, 64 requests, S = 260
 # ---------------------------------------------------------------------------------------------------------------------
 ROWS = (0, 21, 42, 63)
 
@@ -170,7 +170,7 @@ def test_3b_r2_batch64_top_p_draws_in_oracle_kept_set(setup_3b_r2):
 
 
 # ---------------------------------------------------------------------------------------------------------------------
-# 448 px / 896 px geometries at full widths (BASELINE configs[3] / [4])
+# 448 px / 896 px geometries at full widths
 # ---------------------------------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("image_size", [448, 896])
 def test_3b_long_image_sequences_prefill_and_decode(setup_3b, image_size):

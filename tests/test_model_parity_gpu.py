@@ -1,6 +1,6 @@
 """End-to-end parity of the sm_100a model against the CPU fp32 oracle and the committed reference golden vectors.
 
-Tolerances (bf16 operands, fp32 accumulation / residual stream / softmax; SURVEY.md 8(c) protocol):
+Tolerances (bf16 operands, fp32 accumulation / residual stream / softmax):
   logits:  cosine >= 0.9999 and max-abs <= 1 % of the oracle's logit absmax in the well-conditioned regimes (R0, R1);
            cosine >= 0.999 / 3 % in the diffuse regime R2 (tiny model, where bf16 noise is amplified);
   greedy:  token sequences identical in R0/R1 (16 tokens tiny), and wherever the oracle's top-2 margin exceeds 4x the
@@ -151,7 +151,7 @@ def test_graphed_prefill_of_the_latency_path_follows_its_inputs():
 
 @pytest.mark.parametrize("image_size,batch", [(448, 2), (896, 1)])
 def test_long_image_sequences_1024_and_4096_image_tokens(image_size, batch):
-    """BASELINE configs[3] / [4] geometry (1024 / 4096 image tokens, position table, merge, many key tiles in both prefill
+    """Geometry of the 448 px and 896 px models (1024 / 4096 image tokens, position table, merge, many key tiles in both prefill
     attentions, a KV cache of 17 / 65 pages) on the tiny widths, so that the CPU oracle stays cheap: prefill + teacher-forced
     decode logits and free-running greedy tokens against the oracle."""
     import copy
@@ -173,7 +173,7 @@ def test_long_image_sequences_1024_and_4096_image_tokens(image_size, batch):
 
 
 def test_batched_generate_rows_equal_single_row_runs():
-    """B > 1 (not runnable in the reference): every row must reproduce its own B = 1 run, oracle as the judge."""
+    """B > 1 (not runnable in the reference): every row must reproduce its own B = 1 run, against the oracle."""
     sd = make_state_dict(TINY_CONFIG, "R2", seed=3)
     model = build_model(TINY_CONFIG, sd)
     inp = make_inputs(TINY_CONFIG, batch=5, prompt_len=5, seed=9)

@@ -1,5 +1,5 @@
 """Pins the CPU oracle (oracle/paligemma_oracle.py) to the UNMODIFIED reference: every golden vector in
-tests/golden/tiny_reference.npz was produced by running /root/reference itself (tests/golden/make_golden.py)."""
+tests/golden/tiny_reference.npz was produced by running the reference itself (tests/golden/make_golden.py)."""
 import os
 import sys
 

@@ -1,6 +1,6 @@
-"""Variable-length prompts + continuous batching (serving.py; SURVEY 8(f) rank 1) on the GPU, through the C ABI.
+"""Variable-length prompts + continuous batching (serving.py) on the GPU, through the C ABI.
 
-Judges: plain PyTorch fp32 for the ragged attention kernel; vectors of the UNMODIFIED reference run one request at a time
+Compared with: plain PyTorch fp32 for the ragged attention kernel; vectors of the UNMODIFIED reference run one request at a time
 (tests/golden/serving_reference.npz) and this package's own B = 1 generate() for the batcher."""
 import os
 import sys
@@ -124,7 +124,7 @@ def test_continuous_batching_stops_at_eos_and_refills(stage):
 def test_ragged_prefill_logits_and_single_request_runs_R2():
     """Diffuse regime: the first token's logits of every admitted row against the reference's B = 1 prefill logits (stated
     tolerance of the tiny R2 regime: cosine >= 0.999, max-abs <= 3 % of absmax); free-running tokens are compared with
-    this package's own B = 1 generate() and reported (greedy in R2 is not stable under bf16 noise, SURVEY 8(c.2))."""
+    this package's own B = 1 generate() and reported (greedy in R2 is not stable under bf16 noise)."""
     from paligemma_multimodal_system_b200.serving import ContinuousBatcher
     model = build_model(TINY_CONFIG, make_state_dict(TINY_CONFIG, "R2", seed=11))
     reqs = make_requests(TINY_CONFIG, 10, 2, 8, seed=21)
