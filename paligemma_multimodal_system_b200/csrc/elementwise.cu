@@ -92,79 +92,72 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* __restrict__ 
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// Warp-per-row variants for the prefill (tens of thousands of short rows): the row lives in registers (D/128 float4 per
-// lane), the two reductions are warp shuffles, nothing goes through shared memory or a block barrier.  D % 128 == 0,
-// D <= 128 * NV * ... (NV float4 per lane).
+// Warp-per-row variants for the prefill (tens of thousands of short rows): the row lives in registers (NV = D / 128 float4 per
+// lane), the two reductions are warp shuffles, nothing goes through shared memory or a block barrier.  D % 128 == 0, D <= 2048.
+// Bound by HBM with enough rows under way: NV is the row's own width, so that a narrow row takes the registers of its width only and more warps fit.  us with the caches
+// flushed before / launch after launch, registers of 2048-wide rows for all widths -> now: layer norm 8192 x 1152 24.6 / 12.2 -> 18.5 / 9.3 (two CTAs per SM, four), 16640 x 2048
+// 55 / 47 -> 39 / 34; 8238 x 2048 without a mean 26.6 / 17.2 -> 24.6 / 16.4.
 // ---------------------------------------------------------------------------------------------------------
+// CTAs of 256 threads per SM that the row's registers leave room for (`extra`: what the kernel keeps beside the row)
+constexpr int row_ctas(int nv, int extra) { return 4 * nv + extra <= 64 ? 4 : 4 * nv + extra <= 80 ? 3 : 2; }
+
 template <int NV>
-__global__ void __launch_bounds__(256) layernorm_warp_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
+__global__ void __launch_bounds__(256, row_ctas(NV, 24)) layernorm_warp_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
                                                              const float* __restrict__ beta, bf16* __restrict__ y_bf,
                                                              float* __restrict__ y_f, int rows, int D, float eps, int trigger) {
   pg::griddep_begin_if(trigger);
   const int lane = threadIdx.x & 31;
   const long long r = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (r >= rows) return;
-  const int nv = D >> 7;  // float4 per lane
   const float4* xr = reinterpret_cast<const float4*>(x + r * D);
   float4 v[NV];
   float s = 0.f;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    if (i < nv) {
-      v[i] = xr[lane + 32 * i];
-      s += v[i].x + v[i].y + v[i].z + v[i].w;
-    }
+    v[i] = xr[lane + 32 * i];
+    s += v[i].x + v[i].y + v[i].z + v[i].w;
   }
   const float mean = warp_sum(s) / D;
   float ss = 0.f;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    if (i < nv) {
-      const float a = v[i].x - mean, b = v[i].y - mean, c = v[i].z - mean, d = v[i].w - mean;
-      ss += a * a + b * b + c * c + d * d;
-    }
+    const float a = v[i].x - mean, b = v[i].y - mean, c = v[i].z - mean, d = v[i].w - mean;
+    ss += a * a + b * b + c * c + d * d;
   }
   const float rstd = rsqrtf(warp_sum(ss) / D + eps);
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    if (i < nv) {
-      const int c4 = lane + 32 * i;
-      const float4 g = __ldg(reinterpret_cast<const float4*>(gamma) + c4), bt = __ldg(reinterpret_cast<const float4*>(beta) + c4);
-      const float a = (v[i].x - mean) * rstd * g.x + bt.x, b = (v[i].y - mean) * rstd * g.y + bt.y;
-      const float c = (v[i].z - mean) * rstd * g.z + bt.z, d = (v[i].w - mean) * rstd * g.w + bt.w;
-      if (y_bf) reinterpret_cast<uint2*>(y_bf + r * D)[c4] = make_uint2(pack_bf16(a, b), pack_bf16(c, d));
-      if (y_f) reinterpret_cast<float4*>(y_f + r * D)[c4] = make_float4(a, b, c, d);
-    }
+    const int c4 = lane + 32 * i;
+    const float4 g = __ldg(reinterpret_cast<const float4*>(gamma) + c4), bt = __ldg(reinterpret_cast<const float4*>(beta) + c4);
+    const float a = (v[i].x - mean) * rstd * g.x + bt.x, b = (v[i].y - mean) * rstd * g.y + bt.y;
+    const float c = (v[i].z - mean) * rstd * g.z + bt.z, d = (v[i].w - mean) * rstd * g.w + bt.w;
+    if (y_bf) reinterpret_cast<uint2*>(y_bf + r * D)[c4] = make_uint2(pack_bf16(a, b), pack_bf16(c, d));
+    if (y_f) reinterpret_cast<float4*>(y_f + r * D)[c4] = make_float4(a, b, c, d);
   }
 }
 
 template <int NV>
-__global__ void __launch_bounds__(256) rmsnorm_warp_kernel(const float* __restrict__ x, const float* __restrict__ w,
+__global__ void __launch_bounds__(256, row_ctas(NV, 16)) rmsnorm_warp_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                            bf16* __restrict__ y, int rows, int D, float eps, int trigger) {
   pg::griddep_begin_if(trigger);
   const int lane = threadIdx.x & 31;
   const long long r = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (r >= rows) return;
-  const int nv = D >> 7;
   const float4* xr = reinterpret_cast<const float4*>(x + r * D);
   float4 v[NV];
   float ss = 0.f;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    if (i < nv) {
-      v[i] = xr[lane + 32 * i];
-      ss += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
-    }
+    v[i] = xr[lane + 32 * i];
+    ss += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
   }
   const float rstd = rsqrtf(warp_sum(ss) / D + eps);
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    if (i < nv) {
-      const int c4 = lane + 32 * i;
-      const float4 g = __ldg(reinterpret_cast<const float4*>(w) + c4);
-      reinterpret_cast<uint2*>(y + r * D)[c4] = make_uint2(pack_bf16(v[i].x * rstd * (1.0f + g.x), v[i].y * rstd * (1.0f + g.y)),
-                                                          pack_bf16(v[i].z * rstd * (1.0f + g.z), v[i].w * rstd * (1.0f + g.w)));
-    }
+    const int c4 = lane + 32 * i;
+    const float4 g = __ldg(reinterpret_cast<const float4*>(w) + c4);
+    reinterpret_cast<uint2*>(y + r * D)[c4] = make_uint2(pack_bf16(v[i].x * rstd * (1.0f + g.x), v[i].y * rstd * (1.0f + g.y)),
+                                                        pack_bf16(v[i].z * rstd * (1.0f + g.z), v[i].w * rstd * (1.0f + g.w)));
   }
 }
 
@@ -457,7 +450,12 @@ extern "C" int pg_layernorm(const float* x, const float* gamma, const float* bet
   const bool al = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(beta) |
                     reinterpret_cast<uintptr_t>(y_bf16) | reinterpret_cast<uintptr_t>(y_f32)) & 15) == 0;
   if (rows >= 1024 && (D % 128) == 0 && D <= 2048 && al) {  // prefill: one warp per row, the row stays in registers
-    pg::launch_dependent(layernorm_warp_kernel<16>, (rows + 7) / 8, 256, 0, PG_ST(stream), x, gamma, beta, static_cast<bf16*>(y_bf16), y_f32, rows, D, eps, pg::weights_follow());
+    switch (D / 128) {
+#define PG_LN(NV) \
+  case NV: pg::launch_dependent(layernorm_warp_kernel<NV>, (rows + 7) / 8, 256, 0, PG_ST(stream), x, gamma, beta, static_cast<bf16*>(y_bf16), y_f32, rows, D, eps, pg::weights_follow()); break;
+      PG_LN(1) PG_LN(2) PG_LN(3) PG_LN(4) PG_LN(5) PG_LN(6) PG_LN(7) PG_LN(8) PG_LN(9) PG_LN(10) PG_LN(11) PG_LN(12) PG_LN(13) PG_LN(14) PG_LN(15) PG_LN(16)
+#undef PG_LN
+    }
     PG_RET();
   }
   pg::launch_dependent(layernorm_kernel, rows, 256, (D + 33) * sizeof(float), PG_ST(stream), x, gamma, beta, static_cast<bf16*>(y_bf16), y_f32, D, eps, pg::weights_follow());
@@ -471,7 +469,12 @@ extern "C" int pg_rmsnorm(const float* x, const float* w, void* y_bf16, int rows
   if (rows <= 0 || D <= 0 || (D % 4) != 0 || D > 8192) return PG_ERR_ARG;
   if (rows >= 1024 && (D % 128) == 0 && D <= 2048 &&
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y_bf16)) & 15) == 0) {
-    pg::launch_dependent(rmsnorm_warp_kernel<16>, (rows + 7) / 8, 256, 0, PG_ST(stream), x, w, static_cast<bf16*>(y_bf16), rows, D, eps, pg::weights_follow());
+    switch (D / 128) {
+#define PG_RMS(NV) \
+  case NV: pg::launch_dependent(rmsnorm_warp_kernel<NV>, (rows + 7) / 8, 256, 0, PG_ST(stream), x, w, static_cast<bf16*>(y_bf16), rows, D, eps, pg::weights_follow()); break;
+      PG_RMS(1) PG_RMS(2) PG_RMS(3) PG_RMS(4) PG_RMS(5) PG_RMS(6) PG_RMS(7) PG_RMS(8) PG_RMS(9) PG_RMS(10) PG_RMS(11) PG_RMS(12) PG_RMS(13) PG_RMS(14) PG_RMS(15) PG_RMS(16)
+#undef PG_RMS
+    }
     PG_RET();
   }
   return launch_kernel(rmsnorm_kernel, dim3(rows), dim3(256), (D + 33) * sizeof(float), PG_ST(stream), x, w,

@@ -1,0 +1,26 @@
+"""The norms that keep a row in one warp's registers: every row width they are built for, an odd number of rows, against 64 bits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("D", range(128, 2049, 128))
+def test_widths(D):
+    from paligemma_multimodal_system_b200 import _lib
+    rows, eps = 1027, 1e-6
+    g = torch.Generator(device="cuda").manual_seed(D)
+    x = torch.randn(rows, D, generator=g, device="cuda") * 3 + 0.5
+    w, b = (torch.randn(D, generator=g, device="cuda") for _ in range(2))
+    y, f = torch.empty(rows, D, device="cuda", dtype=torch.bfloat16), torch.empty(rows, D, device="cuda")
+    xd = x.double()
+    m = xd.mean(-1, keepdim=True)
+    want = (xd - m) / torch.sqrt(((xd - m) ** 2).mean(-1, keepdim=True) + eps) * w.double() + b.double()
+    _lib.layernorm(x, w, b, eps, out_bf16=y)
+    _lib.layernorm(x, w, b, eps, out_f32=f)
+    # sums of up to 2048 fp32 values: 2^-20 of the normalised values (up to 5 here) before the weight; bf16 rounds by 2^-9
+    assert ((f.double() - want).abs() <= 2.0 ** -19 * (1 + want.abs()) * 5).all()
+    assert ((y.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -16).all()
+    _lib.rmsnorm(x, w, y, eps)
+    want = xd / torch.sqrt((xd * xd).mean(-1, keepdim=True) + eps) * (1 + w.double())
+    assert ((y.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -16).all()
