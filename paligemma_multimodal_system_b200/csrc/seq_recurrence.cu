@@ -627,20 +627,23 @@ __global__ void __launch_bounds__(256) group_norm_gate_kernel(const float* __res
   }
 }
 
-// Groups of 4 * NV * 2^k columns whose lanes fit a warp: lane <-> NV float4 of one group, several groups per warp, the row read once.
+// Groups of 4 * NV * 2^k columns whose lanes fit a warp: lane <-> NV float4 of one group, several groups per warp, the row read once.  Group and lane counts are powers
+// of two and come as shifts, the row of a group is a 32-bit division: 64-bit divisions were two thirds of the instructions that bounded the kernel (3795 rows of 2048 in
+// groups of 64, gated, us with the caches flushed before / launch after launch: 26.6 / 21.3 -> 20.5 / 11.4).
 __device__ __forceinline__ float fast_sigmoid(float z) { return __fdividef(1.0f, 1.0f + __expf(-z)); }
 
 template <typename TA, int NV>
 __global__ void __launch_bounds__(256) group_norm_gate_flat_kernel(const float* __restrict__ o, const float* __restrict__ w, int w_n,
                                                                    const TA* __restrict__ gate, long long ldg, int gate_mode, TA* __restrict__ out,
-                                                                   long long ldo, int D, int gs, long long total_groups, float eps, float scale) {
+                                                                   long long ldo, int D, int gs_bits, int lane_bits, unsigned total_groups, float eps, float scale) {
   pg::griddep_begin();
-  const int lanes = gs / (4 * NV), groups = D / gs;
-  const long long id = (long long)blockIdx.x * (256 / lanes) + threadIdx.x / lanes;  // (row, group)
+  const int lanes = 1 << lane_bits, groups = D >> gs_bits;
+  const unsigned id = blockIdx.x * (256u >> lane_bits) + (threadIdx.x >> lane_bits);  // (row, group)
   const int l = threadIdx.x & (lanes - 1);
   const bool ok = id < total_groups;
-  const long long t = ok ? id / groups : 0;
-  const int col0 = (ok ? (int)(id % groups) : 0) * gs;
+  const unsigned row = ok ? id / (unsigned)groups : 0u;
+  const long long t = row;
+  const int col0 = (ok ? (int)(id - row * (unsigned)groups) : 0) << gs_bits;
   float v[NV][4], z[NV][4], s = 0.f;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
@@ -666,12 +669,12 @@ __global__ void __launch_bounds__(256) group_norm_gate_flat_kernel(const float* 
     }
   for (int x = lanes / 2; x > 0; x >>= 1) s += __shfl_xor_sync(0xffffffffu, s, x);
   if (!ok) return;
-  const float iv = scale / sqrtf(s / (float)gs + eps);
+  const float iv = scale / sqrtf(s * __int_as_float((127 - gs_bits) << 23) + eps);
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int in = (i * lanes + l) * 4;
     float ww[4];
-    if (w != nullptr) ldv<4>(w, w_n == gs ? in : col0 + in, ww);
+    if (w != nullptr) ldv<4>(w, w_n == (1 << gs_bits) ? in : col0 + in, ww);
 #pragma unroll
     for (int k = 0; k < 4; ++k) v[i][k] *= (w != nullptr ? iv * ww[k] : iv) * ((gate_mode & 1) ? z[i][k] : 1.0f);
     stv<4>(out, t * ldo + col0 + in, v[i]);
@@ -851,18 +854,21 @@ extern "C" int pg_group_norm_gate(const float* o, const float* w, int w_n, const
     return gs % v == 0 && ldg % v == 0 && ldo % v == 0 && al(o, 4 * v) && al(w, 4 * v) && al(gate, ab * v) && al(out, ab * v);
   };
   cudaStream_t st = PG_ST(stream);
-  if (fits(4)) {
-    const long long total = (long long)rows * groups;
-    for (int nv = 1; nv <= 8; nv *= 2) {
-      const int lanes = gs / (4 * nv);
-      if (lanes * 4 * nv != gs || lanes > 32 || (lanes & (lanes - 1))) continue;
-      const unsigned blocks = (unsigned)((total + 256 / lanes - 1) / (256 / lanes));
-#define PG_GF(TA, NV) pg::launch_dependent(group_norm_gate_flat_kernel<TA, NV>, blocks, 256, 0, st, o, w, w_n, static_cast<const TA*>(gate), ldg, gate_mode, static_cast<TA*>(out), ldo, D, gs, total, eps, scale)
-      if (act_f32) { if (nv == 1) PG_GF(float, 1); else if (nv == 2) PG_GF(float, 2); else if (nv == 4) PG_GF(float, 4); else PG_GF(float, 8); }
-      else { if (nv == 1) PG_GF(bf16, 1); else if (nv == 2) PG_GF(bf16, 2); else if (nv == 4) PG_GF(bf16, 4); else PG_GF(bf16, 8); }
+  const long long total = (long long)rows * groups;
+  if (fits(4) && (gs & (gs - 1)) == 0 && gs <= 4 * 8 * 32 && total < 0x7fffff00) {
+    int gs_bits = 2;
+    while (1 << gs_bits < gs) ++gs_bits;
+    // float4 per lane: one while that leaves CTAs few (a decode step is a chain of latencies), two where there are many (root, division and row lookup are
+    // per lane), more where a warp would not hold the group
+    int nv = gs >= 8 && total * gs > 256LL * 1024 * 4 ? 2 : 1;
+    while (gs / (4 * nv) > 32) nv *= 2;
+    const int lane_bits = gs_bits - 2 - (nv == 8 ? 3 : nv / 2);
+    const unsigned blocks = (unsigned)((total + (256 >> lane_bits) - 1) / (256 >> lane_bits));
+#define PG_GF(TA, NV) pg::launch_dependent(group_norm_gate_flat_kernel<TA, NV>, blocks, 256, 0, st, o, w, w_n, static_cast<const TA*>(gate), ldg, gate_mode, static_cast<TA*>(out), ldo, D, gs_bits, lane_bits, (unsigned)total, eps, scale)
+    if (act_f32) { if (nv == 1) PG_GF(float, 1); else if (nv == 2) PG_GF(float, 2); else if (nv == 4) PG_GF(float, 4); else PG_GF(float, 8); }
+    else { if (nv == 1) PG_GF(bf16, 1); else if (nv == 2) PG_GF(bf16, 2); else if (nv == 4) PG_GF(bf16, 4); else PG_GF(bf16, 8); }
 #undef PG_GF
-      PG_RET();
-    }
+    PG_RET();
   }
 #define PG_GN(TA, V) pg::launch_dependent(group_norm_gate_kernel<TA, V>, rows, 256, 0, st, o, w, w_n, static_cast<const TA*>(gate), ldg, gate_mode, static_cast<TA*>(out), ldo, D, groups, eps, scale)
   if (act_f32) {
