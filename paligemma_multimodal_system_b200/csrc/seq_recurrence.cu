@@ -225,8 +225,25 @@ __device__ __forceinline__ void pack(const float* v, uint4& u) {
   u = make_uint4(pg::pack_bf16(v[0], v[1]), pg::pack_bf16(v[2], v[3]), pg::pack_bf16(v[4], v[5]), pg::pack_bf16(v[6], v[7]));
 }
 
+// a pair of fp32 products and sums by one instruction, rounded as two fmaf
+__device__ __forceinline__ uint64_t pair2(float a, float b) { return (uint64_t)__float_as_uint(b) << 32 | __float_as_uint(a); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+// silu of a value that is rounded to bf16 at once: the hardware exponential and reciprocal are far below its rounding
+__device__ __forceinline__ float silu_bf16(float a) {
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(a * -1.4426950408889634f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+  return a * r;
+}
+
+// What bounds it: instructions (3795 rows x 6144 channels, 4 taps, two thirds of them normed: 45 per element and 53 us before pairs of products, a reduction
+// that leaves one row per lane, row pointers that advance and longer runs; 28 now launch after launch, 48 before; its bytes 15 us).
 template <int TAPS, int V>
-__global__ void __launch_bounds__(128) short_conv_vec_kernel(const bf16* __restrict__ x, long long ldx, const float* __restrict__ w,
+__global__ void __launch_bounds__(128, V == 4 && TAPS == 4 ? 6 : 1) short_conv_vec_kernel(const bf16* __restrict__ x, long long ldx, const float* __restrict__ w,
                                                              const float* __restrict__ bias, float* __restrict__ state, bf16* __restrict__ out,
                                                              long long ldo, float* __restrict__ inv, int ldi, PgConvSections sec, int taps, int C,
                                                              const int* __restrict__ entry_row0, const int* __restrict__ entry_n,
@@ -237,85 +254,138 @@ __global__ void __launch_bounds__(128) short_conv_vec_kernel(const bf16* __restr
   const int e = blockIdx.z, lane = threadIdx.x & 31;
   const int n = entry_n[e], r0 = blockIdx.y * chunk;
   if (r0 >= n) return;
-  int g = blockIdx.x * 4 + (threadIdx.x >> 5), s = 0, unit_base = 0;
-  while (s < sec.count && g >= (sec.total[s] + WC - 1) / WC) {
-    g -= (sec.total[s] + WC - 1) / WC;
-    if (sec.unit[s]) unit_base += sec.groups[s];
-    ++s;
+  // the warp's section, its fields by selects (a section taken by a running index is a chain of indexed constant loads)
+  int g = blockIdx.x * 4 + (threadIdx.x >> 5), unit_base = 0, s_total = -1, s_size = V, s_xcol = 0, s_ccol = 0;
+  bool unit = false;
+  float unit_scale = 0.f;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    if (i >= sec.count || s_total >= 0) continue;
+    const int w = (sec.total[i] + WC - 1) / WC;
+    if (g < w) {
+      s_total = sec.total[i]; s_size = sec.size[i]; s_xcol = sec.xcol[i]; s_ccol = sec.ccol[i];
+      unit = sec.unit[i] != 0; unit_scale = sec.scale[i];
+    } else {
+      g -= w;
+      if (sec.unit[i]) unit_base += sec.groups[i];
+    }
   }
-  if (s >= sec.count) return;
+  if (s_total < 0) return;
   const int c = g * WC + lane * V;    // channel inside the section
-  const bool ok = c < sec.total[s];   // totals are multiples of V
-  const int lanes = sec.size[s] / V;  // lanes of one group
+  const bool ok = c < s_total;        // totals are multiples of V
+  const int lanes = s_size / V;       // lanes of one group
   const long long row0 = entry_row0[e];
-  const bf16* xp = x + row0 * ldx + sec.xcol[s] + (ok ? c : 0);
-  bf16* op = out + row0 * ldo + sec.ccol[s] + (ok ? c : 0);
-  const int cc = sec.ccol[s] + (ok ? c : 0), K = taps - 1;
+  const bf16* xp = x + row0 * ldx + s_xcol + (ok ? c : 0);
+  bf16* op = out + (row0 + r0) * ldo + s_ccol + (ok ? c : 0);
+  const int cc = s_ccol + (ok ? c : 0), K = taps - 1;
   float* slot = state + (long long)entry_slot[e] * K * C + cc;
-  float wt[TAPS][V], bs[V], hist[TAPS - 1][V];
+  uint64_t wt[TAPS][V / 2], bs[V / 2], hist[TAPS - 1][V / 2];  // pairs of adjacent channels
   auto ldf = [](const float* p, float* v) {
 #pragma unroll
     for (int i = 0; i < V; i += 4) ldv<4>(p, i, v + i);
   };
-  auto zero = [](float* v) {
+  auto pairs = [](const float* v, uint64_t* p) {
 #pragma unroll
-    for (int i = 0; i < V; ++i) v[i] = 0.f;
+    for (int i = 0; i < V / 2; ++i) p[i] = pair2(v[2 * i], v[2 * i + 1]);
+  };
+  auto ldp = [&](const float* p, uint64_t* to) {
+    float v[V];
+    ldf(p, v);
+    pairs(v, to);
   };
   auto row_at = [&](int r) { return *reinterpret_cast<const P*>(xp + (long long)r * ldx); };
-  if (bias != nullptr) ldf(bias + cc, bs); else zero(bs);
+  if (bias != nullptr) ldp(bias + cc, bs);
+  else {
+#pragma unroll
+    for (int i = 0; i < V / 2; ++i) bs[i] = 0;
+  }
 #pragma unroll
   for (int j = 0; j < TAPS; ++j) {
     const int tj = j - (TAPS - taps);
-    if (tj >= 0) ldf(w + (long long)tj * C + cc, wt[j]); else zero(wt[j]);
+    if (tj >= 0) ldp(w + (long long)tj * C + cc, wt[j]);
+    else {
+#pragma unroll
+      for (int i = 0; i < V / 2; ++i) wt[j][i] = 0;
+    }
   }
 #pragma unroll
   for (int j = 0; j < TAPS - 1; ++j) {
     const int row = r0 - (TAPS - 1) + j;
-    if (row >= 0) unpack(row_at(row), hist[j]);
-    else if (entry_ctx[e] > 0 && K + row >= 0) ldf(slot + (long long)(K + row) * C, hist[j]);
-    else zero(hist[j]);
+    if (row >= 0) {
+      float v[V];
+      unpack(row_at(row), v);
+      pairs(v, hist[j]);
+    } else if (entry_ctx[e] > 0 && K + row >= 0) {
+      ldp(slot + (long long)(K + row) * C, hist[j]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < V / 2; ++i) hist[j][i] = 0;
+    }
   }
   const int r1 = min(n, r0 + chunk);
-  const bool unit = sec.unit[s] != 0;
-  const float unit_scale = sec.scale[s];
-  float* ip = (unit && ok && (lane & (lanes - 1)) == 0) ? inv + row0 * ldi + unit_base + c / sec.size[s] : nullptr;
+  // With four lanes or more the sums of AHEAD rows are spread as they are added: a lane ends with the whole sum of one row, and the first of those that hold a row stores it
+  const bool spread = lanes >= AHEAD;
+  const int keep_bits = spread ? ((lane & (lanes / 2)) ? 2 : 0) + ((lane & (lanes / 4)) ? 1 : 0) : 0;
+  float* ip = nullptr;
+  if (unit && ok && (lane & ((spread ? lanes / 4 : lanes) - 1)) == 0) ip = inv + (row0 + r0 + keep_bits) * ldi + unit_base + c / s_size;
+  const bf16* np = xp + (long long)r0 * ldx;
   P nxt[AHEAD];
 #pragma unroll
-  for (int i = 0; i < AHEAD; ++i) nxt[i] = row_at(min(r0 + i, r1 - 1));
+  for (int i = 0; i < AHEAD; ++i, np += ldx) nxt[i] = r0 + i < r1 ? *reinterpret_cast<const P*>(np) : P{};
   for (int rb = r0; rb < r1; rb += AHEAD) {
     float ss[AHEAD];
 #pragma unroll
     for (int i = 0; i < AHEAD; ++i) {
-      const int r = rb + i;  // rows past the run are computed from a repeated row and not stored
+      const int r = rb + i;  // rows past the run are computed from whatever is there and not stored
       float cur[V], y[V];
+      uint64_t cp[V / 2];
       unpack(nxt[i], cur);
-      nxt[i] = row_at(min(r + AHEAD, r1 - 1));
+      pairs(cur, cp);
+      if (r + AHEAD < r1) nxt[i] = *reinterpret_cast<const P*>(np);
+      np += ldx;
 #pragma unroll
-      for (int v = 0; v < V; ++v) {
-        float a = fmaf(wt[TAPS - 1][v], cur[v], bs[v]);
+      for (int v = 0; v < V / 2; ++v) {
+        uint64_t a = fma2(wt[TAPS - 1][v], cp[v], bs[v]);
 #pragma unroll
-        for (int j = 0; j < TAPS - 1; ++j) a = fmaf(wt[j][v], hist[j][v], a);
+        for (int j = 0; j < TAPS - 1; ++j) a = fma2(wt[j][v], hist[j][v], a);
 #pragma unroll
         for (int j = 0; j < TAPS - 2; ++j) hist[j][v] = hist[j + 1][v];
-        hist[TAPS - 2][v] = cur[v];
-        y[v] = __fdividef(a, 1.0f + __expf(-a));  // a bf16 activation: the hardware exponential is far below its rounding
+        hist[TAPS - 2][v] = cp[v];
+        y[2 * v] = silu_bf16(__uint_as_float((uint32_t)a));
+        y[2 * v + 1] = silu_bf16(__uint_as_float((uint32_t)(a >> 32)));
       }
       P pk;
       pack(y, pk);
-      if (ok && r < r1) *reinterpret_cast<P*>(op + (long long)r * ldo) = pk;
+      if (ok && r < r1) *reinterpret_cast<P*>(op) = pk;
+      op += ldo;
+      if (!unit) continue;
       unpack(pk, y);  // the norm is that of the stored activations
       ss[i] = 0.f;
 #pragma unroll
       for (int v = 0; v < V; ++v) ss[i] = fmaf(y[v], y[v], ss[i]);
     }
-    if (unit) {
+    if (!unit) continue;
+    if (spread) {
+      const bool up = (lane & (lanes / 2)) != 0, odd = (lane & (lanes / 4)) != 0;
+      float a0 = up ? ss[2] : ss[0], a1 = up ? ss[3] : ss[1];
+      a0 += __shfl_xor_sync(0xffffffffu, up ? ss[0] : ss[2], lanes / 2);
+      a1 += __shfl_xor_sync(0xffffffffu, up ? ss[1] : ss[3], lanes / 2);
+      float a = odd ? a1 : a0;
+      a += __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, lanes / 4);
+      for (int o = lanes / 8; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+      if (ip != nullptr) {
+        if (rb + keep_bits < r1) *ip = unit_scale / sqrtf(a + 1e-6f);
+        ip += (long long)AHEAD * ldi;
+      }
+    } else {
       for (int o = lanes / 2; o > 0; o >>= 1)
 #pragma unroll
         for (int i = 0; i < AHEAD; ++i) ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], o);
       if (ip != nullptr) {
 #pragma unroll
         for (int i = 0; i < AHEAD; ++i)
-          if (rb + i < r1) ip[(long long)(rb + i) * ldi] = unit_scale / sqrtf(ss[i] + 1e-6f);
+          if (rb + i < r1) ip[(long long)i * ldi] = unit_scale / sqrtf(ss[i] + 1e-6f);
+        ip += (long long)AHEAD * ldi;
       }
     }
   }
@@ -325,7 +395,10 @@ __global__ void __launch_bounds__(128) short_conv_vec_kernel(const bf16* __restr
       float h[V];
       if (row >= 0) unpack(row_at(row), h);
       else if (entry_ctx[e] > 0) ldf(slot + (long long)(n + j) * C, h);
-      else zero(h);
+      else {
+#pragma unroll
+        for (int i = 0; i < V; ++i) h[i] = 0.f;
+      }
 #pragma unroll
       for (int i = 0; i < V; i += 4) stv<4>(slot, (long long)j * C + i, h + i);
     }
@@ -719,8 +792,12 @@ int launch_conv_vec(const void* x, long long ldx, const float* w, const float* b
                     cudaStream_t st) {
   int warps = 0;
   for (int s = 0; s < sec.count; ++s) warps += (sec.total[s] + 32 * V - 1) / (32 * V);
+  // runs of 64 rows, shortened while an SM would have fewer than 24 warps; below 16 rows a warp's weights and section cost more than the rows, so runs of 8 only
+  // where even those leave an SM with fewer than 8 (3795 rows, 48 warps wide: runs of 16 / 32 42 / 28 us)
   int chunk = 64;
-  while (chunk > 8 && (long long)warps * entries * ((max_n + chunk - 1) / chunk) < 48LL * pg::num_sms()) chunk /= 2;
+  auto runs = [&](int c) { return (long long)warps * entries * ((max_n + c - 1) / c); };
+  while (chunk > 16 && runs(chunk) < 24LL * pg::num_sms()) chunk /= 2;
+  if (chunk == 16 && runs(16) < 8LL * pg::num_sms()) chunk = 8;
   const dim3 grid((warps + 3) / 4, (max_n + chunk - 1) / chunk, entries);
   pg::launch_dependent(short_conv_vec_kernel<TAPS, V>, grid, 128, 0, st, static_cast<const bf16*>(x), ldx, w, bias, state, static_cast<bf16*>(out), ldo, inv, ldi, sec, taps, C, row0,
                                                         n, ctx, slot, chunk);
