@@ -147,8 +147,10 @@ __global__ void __launch_bounds__(128) attn_prepare_kernel(const TA* __restrict_
 
 // The same for heads of whole 16-byte groups (8 elements a lane, so dim / 8 lanes -- a power of two -- hold a head and its norm stays inside them): the
 // row is read once, in 16-byte pieces, all of them under way together.  A CTA takes TOK tokens, so that the double-precision angles -- a chain of ~60
-// dependent operations that only dim / 2 threads had work in -- run on all of its threads.  What bounds it: prompts, HBM (8192 rows of 32 + 8 + 8 heads x 64,
-// 100 MB: 65 -> 28 us, with norms 101 -> 37); a decode step, the latency of its loads (48 rows: 7.9 -> 3.5 us, with norms 12.8 -> 4.5).
+// dependent operations that only dim / 2 threads had work in -- run on all of its threads; with several tokens a CTA behind its first pieces' requests.  With four tokens the
+// sums of their norms are spread as they are added (a lane ends with one token's, and takes one root and one division instead of four).  What bounds it: prompts,
+// instructions and their fetch, then HBM (7.8k rows of 32 + 8 + 8 heads x 64, 94 MB: 26 us launch after launch as a loop unrolled twice over pieces held as fp32, 18 now; with norms,
+// 10.8k rows, 50 and 32; element by element 65); a decode step, the latency of its loads (48 rows: 7.9 -> 3.5 us, with norms 12.8 -> 4.5).
 template <typename TA>
 __device__ __forceinline__ void ld8(float (&v)[8], const TA* p);
 template <>
@@ -171,7 +173,31 @@ __device__ __forceinline__ void st8(bf16* p, const float (&v)[8]) {
   *reinterpret_cast<uint4*>(p) = make_uint4(pg::pack_bf16(v[0], v[1]), pg::pack_bf16(v[2], v[3]), pg::pack_bf16(v[4], v[5]), pg::pack_bf16(v[6], v[7]));
 }
 
-template <typename TA, int TOK>
+// eight elements as they lie in memory
+template <typename TA>
+struct Raw8 {
+  uint4 u[sizeof(TA) / 2];
+};
+template <typename TA>
+__device__ __forceinline__ Raw8<TA> ldraw(const TA* p) {
+  Raw8<TA> r;
+#pragma unroll
+  for (int i = 0; i < (int)(sizeof(TA) / 2); ++i) r.u[i] = reinterpret_cast<const uint4*>(p)[i];
+  return r;
+}
+__device__ __forceinline__ void unraw(float (&v)[8], const Raw8<bf16>& r) {
+  const uint32_t w[4] = {r.u[0].x, r.u[0].y, r.u[0].z, r.u[0].w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) { v[2 * i] = __uint_as_float(w[i] << 16); v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
+}
+__device__ __forceinline__ void unraw(float (&v)[8], const Raw8<float>& r) {
+  const uint32_t w[8] = {r.u[0].x, r.u[0].y, r.u[0].z, r.u[0].w, r.u[1].x, r.u[1].y, r.u[1].z, r.u[1].w};
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(w[i]);
+}
+
+// ROT8: rot is a multiple of 8, so the four pairs of a lane are rotated or not as one
+template <typename TA, int TOK, bool ROT8>
 __global__ void __launch_bounds__(128) attn_prepare_vec_kernel(const TA* __restrict__ qkv, long long ld, const int* __restrict__ pos,
                                                                const int* __restrict__ row_entry, const int* __restrict__ page_table, int max_pages,
                                                                int page, const double* __restrict__ freq, const float* __restrict__ qn,
@@ -179,15 +205,28 @@ __global__ void __launch_bounds__(128) attn_prepare_vec_kernel(const TA* __restr
                                                                TA* __restrict__ v_pages, int rows, int H, int G, int dim, int vdim, int rot, float eps,
                                                                int norm_qk, int norm_v, int v_from_k, float rot_gain, const TA* __restrict__ v_other,
                                                                long long ldvo, float v_mix) {
-  extern __shared__ float cs[];  // [TOK][cos rot/2 | sin rot/2]
+  extern __shared__ __align__(16) float cs[];  // [TOK][cos rot/2 | sin rot/2]
   __shared__ float part[2][TOK][4];
   const int t0 = blockIdx.x * TOK, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nq = H * dim / 8, nk = k_pages != nullptr ? G * dim / 8 : 0, nv = k_pages != nullptr ? G * vdim / 8 : 0, half = rot / 2;
+  const int total = nq + nk + nv, lph = dim / 8;  // (a value norm wants vdim == dim: one head width for all shuffles)
   long long pg_row[TOK];
 #pragma unroll
   for (int k = 0; k < TOK; ++k) {
     const int t = min(t0 + k, rows - 1), p = pos[t];
     pg_row[k] = nk > 0 ? (long long)page_table[(long long)row_entry[t] * max_pages + p / page] * page + p % page : 0;
+  }
+  constexpr int DEEP = TOK == 1 ? 3 : 1;  // pieces of a row under way: one token has too few rows in flight otherwise
+  Raw8<TA> ahead[DEEP][TOK];
+  auto request = [&](Raw8<TA>(&x)[TOK], int c) {
+    if (c >= total) return;
+    const TA* p = qkv + (long long)t0 * ld + (v_from_k && c >= nq + nk ? 8LL * (c - nk) : 8LL * c);
+#pragma unroll
+    for (int k = 0; k < TOK; ++k) x[k] = ldraw<TA>(p + (t0 + k < rows ? k : rows - 1 - t0) * ld);
+  };
+  if (TOK > 1) {
+    pg::griddep_wait();
+    request(ahead[0], threadIdx.x);
   }
   for (int i = threadIdx.x; i < TOK * half; i += 128) {
     const int k = i / half, j = i - k * half;
@@ -196,9 +235,13 @@ __global__ void __launch_bounds__(128) attn_prepare_vec_kernel(const TA* __restr
     cs[k * rot + j] = rot_gain * (float)c;
     cs[k * rot + half + j] = rot_gain * (float)s;
   }
-  pg::griddep_wait();  // (positions, pages and frequencies are the host's)
-  if (norm_qk == 2) {  // one root mean square for all of q, one for all of k
+  if (TOK == 1) {  // (positions, pages and frequencies are the host's)
+    pg::griddep_wait();
 #pragma unroll
+    for (int d = 0; d < DEEP; ++d) request(ahead[d], threadIdx.x + 128 * d);
+  }
+  if (norm_qk == 2) {  // one root mean square for all of q, one for all of k
+#pragma unroll 1
     for (int k = 0; k < TOK; ++k) {
       const TA* row = qkv + (long long)min(t0 + k, rows - 1) * ld;
       float sq = 0.f, sk = 0.f;
@@ -215,68 +258,114 @@ __global__ void __launch_bounds__(128) attn_prepare_vec_kernel(const TA* __restr
     }
   }
   __syncthreads();
-  const int total = nq + nk + nv;
-#pragma unroll 2
-  for (int c = threadIdx.x; c < (total + 31) / 32 * 32; c += 128) {  // whole warps: the norms shuffle
+  auto piece = [&](Raw8<TA>(&x)[TOK], int c) {
     const bool in = c < total, is_q = c < nq, is_k = !is_q && c < nq + nk;
-    const int cc = is_q ? c : is_k ? c - nq : c - nq - nk, lph = (is_q || is_k ? dim : vdim) / 8;  // lanes of the head
-    const int d0 = (cc & (lph - 1)) * 8;
-    const long long off = is_q || is_k ? 8LL * c : v_from_k ? 8LL * (c - nk) : 8LL * c;
-    const float* w = is_q ? qn : kn;  // NULL: a norm without a weight
-    if (w != nullptr) w += norm_qk == 2 ? 8LL * cc : d0;
-    float x[TOK][8];
+    const int cc = is_q ? c : is_k ? c - nq : c - nq - nk;
+    const int d0 = (cc & ((is_q || is_k ? dim : vdim) / 8 - 1)) * 8;
+    float inv[TOK];
 #pragma unroll
-    for (int k = 0; k < TOK; ++k)
-      if (in) ld8<TA>(x[k], qkv + (long long)min(t0 + k, rows - 1) * ld + off);
+    for (int k = 0; k < TOK; ++k) inv[k] = 1.0f;
+    if (norm_qk == 1 || norm_v) {  // (uniform: every lane takes part in the shuffles, whatever it holds; sums that are not wanted are not used)
+      const bool wanted = (is_q || is_k) ? norm_qk == 1 : norm_v != 0;
+      float s[TOK];
 #pragma unroll
-    for (int k = 0; k < TOK; ++k) {
-      float inv = 1.0f;
-      if (norm_qk == 1 || norm_v) {  // (uniform: every lane takes part in the shuffles, whatever it holds; sums that are not wanted are not used)
-        float s = 0.f;
+      for (int k = 0; k < TOK; ++k) {
+        float v[8];
+        unraw(v, x[k]);
+        s[k] = 0.f;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) s = in ? fmaf(x[k][i], x[k][i], s) : 0.f;
-        for (int o = 1; o < 32; o <<= 1) {
-          const float u = __shfl_xor_sync(0xffffffffu, s, o);
-          if (o < lph) s += u;
-        }
-        if ((is_q || is_k) ? norm_qk == 1 : norm_v) inv = 1.0f / sqrtf(s / (float)(8 * lph) + eps);
+        for (int i = 0; i < 8; ++i) s[k] = in ? fmaf(v[i], v[i], s[k]) : 0.f;
       }
-      if ((is_q || is_k) && norm_qk == 2) {
-        const float* ps = part[is_q ? 0 : 1][k];
-        inv = 1.0f / sqrtf((ps[0] + ps[1] + ps[2] + ps[3]) / (float)(8 * (is_q ? nq : nk)) + eps);
-      }
-      const int t = t0 + k;
-      if (!in || t >= rows) continue;
+      if (TOK == 4 && lph >= 4) {
+        const bool up = (lane & (lph / 2)) != 0, odd = (lane & (lph / 4)) != 0;
+        float a0 = (up ? s[2 % TOK] : s[0]) + __shfl_xor_sync(0xffffffffu, up ? s[0] : s[2 % TOK], lph / 2);
+        float a1 = (up ? s[3 % TOK] : s[1 % TOK]) + __shfl_xor_sync(0xffffffffu, up ? s[1 % TOK] : s[3 % TOK], lph / 2);
+        float a = (odd ? a1 : a0) + __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, lph / 4);
+        for (int o = lph / 8; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        a = 1.0f / sqrtf(a / (float)dim + eps);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) x[k][i] *= inv;
-      if (is_q || is_k) {
-        if (w != nullptr) {
-          float ww[8];
-          ld8<float>(ww, w);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) x[k][i] *= ww[i];
+        for (int k = 0; k < TOK; ++k) {
+          const float u = __shfl_sync(0xffffffffu, a, (lane & ~(lph - 1)) + (k >> 1) * (lph / 2) + (k & 1) * (lph / 4));
+          if (wanted) inv[k] = u;
         }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int pair = d0 / 2 + i;
-          if (pair < half) {
-            const float c0 = cs[k * rot + pair], s0 = cs[k * rot + half + pair], a = x[k][2 * i], b = x[k][2 * i + 1];
-            x[k][2 * i] = a * c0 - b * s0;
-            x[k][2 * i + 1] = b * c0 + a * s0;
-          }
-        }
-        if (is_q) st8(q_out + (long long)t * H * dim + 8LL * cc, x[k]);
-        else st8(k_pages + pg_row[k] * ((long long)G * dim) + 8LL * cc, x[k]);
       } else {
-        if (v_other != nullptr) {
-          float o[8];
-          ld8<TA>(o, v_other + (long long)t * ldvo + 8LL * cc);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) x[k][i] = (1.0f - v_mix) * x[k][i] + v_mix * o[i];
+        for (int k = 0; k < TOK; ++k) {
+          for (int o = lph / 2; o > 0; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+          if (wanted) inv[k] = 1.0f / sqrtf(s[k] / (float)dim + eps);
         }
-        st8(v_pages + pg_row[k] * ((long long)G * vdim) + 8LL * cc, x[k]);
       }
     }
+    if (norm_qk == 2 && (is_q || is_k)) {
+#pragma unroll
+      for (int k = 0; k < TOK; ++k) {
+        const float* ps = part[is_q ? 0 : 1][k];
+        inv[k] = 1.0f / sqrtf((ps[0] + ps[1] + ps[2] + ps[3]) / (float)(8 * (is_q ? nq : nk)) + eps);
+      }
+    }
+    if (in) {
+      const float* w = is_q ? qn : is_k ? kn : nullptr;  // NULL: a norm without a weight
+      float ww[8];
+      if (w != nullptr) ld8<float>(ww, w + (norm_qk == 2 ? 8LL * cc : d0));
+      const int pair0 = d0 / 2;
+      const bool turn = (is_q || is_k) && pair0 < half;
+#pragma unroll
+      for (int k = 0; k < TOK; ++k) {
+        const int t = t0 + k;
+        if (t >= rows) break;
+        float v[8];
+        unraw(v, x[k]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] *= inv[k];
+        if (w != nullptr) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) v[i] *= ww[i];
+        }
+        if (turn) {
+          float cv[4], sv[4];
+          const float* ck = cs + k * rot + pair0;
+          if (ROT8) {
+            const float4 c4 = *reinterpret_cast<const float4*>(ck), s4 = *reinterpret_cast<const float4*>(ck + half);
+            cv[0] = c4.x; cv[1] = c4.y; cv[2] = c4.z; cv[3] = c4.w;
+            sv[0] = s4.x; sv[1] = s4.y; sv[2] = s4.z; sv[3] = s4.w;
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              cv[i] = pair0 + i < half ? ck[i] : 1.f;
+              sv[i] = pair0 + i < half ? ck[half + i] : 0.f;
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (!ROT8 && pair0 + i >= half) break;
+            const float a = v[2 * i], b = v[2 * i + 1];
+            v[2 * i] = a * cv[i] - b * sv[i];
+            v[2 * i + 1] = b * cv[i] + a * sv[i];
+          }
+        }
+        if (is_q) {
+          st8(q_out + (long long)t * H * dim + 8LL * cc, v);
+        } else if (is_k) {
+          st8(k_pages + pg_row[k] * ((long long)G * dim) + 8LL * cc, v);
+        } else {
+          if (v_other != nullptr) {
+            float o[8];
+            ld8<TA>(o, v_other + (long long)t * ldvo + 8LL * cc);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = (1.0f - v_mix) * v[i] + v_mix * o[i];
+          }
+          st8(v_pages + pg_row[k] * ((long long)G * vdim) + 8LL * cc, v);
+        }
+      }
+    }
+    request(x, c + 128 * DEEP);
+  };
+  const int whole = (total + 31) / 32 * 32;  // whole warps: the norms shuffle
+#pragma unroll 1
+  for (int c = threadIdx.x; c < whole; c += 128 * DEEP) {
+#pragma unroll
+    for (int d = 0; d < DEEP; ++d)
+      if (c + 128 * d < whole) piece(ahead[d], c + 128 * d);
   }
 }
 
@@ -1099,8 +1188,13 @@ extern "C" int pg_attn_prepare(const void* qkv, long long ld, const int* pos, co
           static_cast<TA*>(v_pages), rows, H, G, dim, vdim, rot_dims, eps, norm_qk, norm_v, v_from_k, rot_gain, static_cast<const TA*>(v_other), ld_v_other, v_mix);
     };
     // four tokens a CTA once that still fills the SMs
-    if (act_f32) rows >= 4 * 4 * pg::num_sms() ? go(attn_prepare_vec_kernel<float, 4>, float(), 4) : go(attn_prepare_vec_kernel<float, 1>, float(), 1);
-    else rows >= 4 * 4 * pg::num_sms() ? go(attn_prepare_vec_kernel<bf16, 4>, bf16(), 4) : go(attn_prepare_vec_kernel<bf16, 1>, bf16(), 1);
+    const bool four = rows >= 4 * 4 * pg::num_sms(), rot8 = rot_dims % 8 == 0;
+#define PG_AP(TA) \
+  four ? (rot8 ? go(attn_prepare_vec_kernel<TA, 4, true>, TA(), 4) : go(attn_prepare_vec_kernel<TA, 4, false>, TA(), 4)) \
+       : (rot8 ? go(attn_prepare_vec_kernel<TA, 1, true>, TA(), 1) : go(attn_prepare_vec_kernel<TA, 1, false>, TA(), 1))
+    if (act_f32) PG_AP(float);
+    else PG_AP(bf16);
+#undef PG_AP
     PG_RET();
   }
   const size_t smem = (size_t)(rot_dims + 2) * sizeof(float);
