@@ -154,31 +154,58 @@ __global__ void __launch_bounds__(256) latent_gather_kernel(const TA* __restrict
 }
 
 // per dense row: k[row, h, :] = [up[row, h * dim ..] | rotated part of the cached row], v[row, h, :] = up[row, H * dim + h * vdim ..]
+// A warp takes rows of all entries in turn: a CTA sums the lengths of 256 entries at a time (single-token entries own no rows) and finds a row's entry among them by halving, so
+// that a step of a few portions beside many single tokens has neither CTAs without rows nor rows that wait for one another.  A warp's eight loads are under way together.
+// Bound by the latency of table, row and copy, one row per warp.  2 x 1733 rows beside 40 singles, 32 heads x (64 + 32 | 64): a CTA per 16 rows of the longest entry and entry,
+// 20 us; now 12.
 template <typename TA, bool VEC>
 __global__ void __launch_bounds__(256) latent_pack_kv_kernel(const TA* __restrict__ up, long long ld_up, const TA* __restrict__ pages,
                                                              const int* __restrict__ page_table, int max_pages, int page, const int* __restrict__ dense_row0,
                                                              const int* __restrict__ entry_n, const int* __restrict__ entry_ctx, TA* __restrict__ k_out,
-                                                             TA* __restrict__ v_out, int H, int dim, int rot, int vdim, int rank) {
-  pg::griddep_begin();
+                                                             TA* __restrict__ v_out, int entries, int H, int dim, int rot, int vdim, int rank) {
   constexpr int E = VEC ? 16 / sizeof(TA) : 1;
   using P = typename Piece<TA, VEC>::type;
-  const int e = blockIdx.y;
-  if (entry_n[e] == 1) return;
-  const int len = entry_ctx[e] + entry_n[e], lane = threadIdx.x & 31, nw = gridDim.x * 8;
+  __shared__ int ends[256], sums[8];  // ends[i]: rows of the entries e0 .. e0 + i
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = gridDim.x * 8;
   const int kd = (dim + rot) / E, plain = dim / E;
-  for (int j = blockIdx.x * 8 + (threadIdx.x >> 5); j < len; j += nw) {
-    const long long row = dense_row0[e] + j;
-    const P* src = reinterpret_cast<const P*>(pages + ((long long)page_table[(long long)e * max_pages + j / page] * page + j % page) * (long long)(rank + rot) + rank);
-    const P* u = reinterpret_cast<const P*>(up + row * ld_up);
-    P* ko = reinterpret_cast<P*>(k_out + row * (long long)H * (dim + rot));
-    P* vo = reinterpret_cast<P*>(v_out + row * (long long)H * vdim);
-#pragma unroll 4
-    for (int i = lane; i < H * kd; i += 32) {
-      const int h = i / kd, d = i - h * kd;
-      ko[i] = d < plain ? u[h * plain + d] : src[d - plain];
+  int mine = blockIdx.x * 8 + warp;  // row of this warp, counted from the first entry of the 256
+  pg::griddep_begin();
+  for (int e0 = 0; e0 < entries; e0 += 256) {
+    const int e = e0 + (int)threadIdx.x, n = e < entries ? entry_n[e] : 1;
+    int len = n > 1 ? entry_ctx[e] + n : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, len, o);
+      if (lane >= o) len += u;
     }
-#pragma unroll 4
-    for (int i = lane; i < H * vdim / E; i += 32) vo[i] = u[H * plain + i];
+    __syncthreads();  // the 256 before are done with
+    if (lane == 31) sums[warp] = len;
+    __syncthreads();
+    for (int w = 0; w < warp; ++w) len += sums[w];
+    ends[threadIdx.x] = len;
+    __syncthreads();
+    const int rows = ends[255];
+    for (; mine < rows; mine += nw) {
+      int lo = 0, hi = 255;  // the first entry that ends behind the row
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (ends[mid] > mine) hi = mid; else lo = mid + 1;
+      }
+      const int j = mine - (lo > 0 ? ends[lo - 1] : 0);
+      const long long ent = e0 + lo, row = dense_row0[ent] + j;
+      const P* __restrict__ src = reinterpret_cast<const P*>(pages + ((long long)page_table[ent * max_pages + j / page] * page + j % page) * (long long)(rank + rot) + rank);
+      const P* __restrict__ u = reinterpret_cast<const P*>(up + row * ld_up);
+      P* __restrict__ ko = reinterpret_cast<P*>(k_out + row * (long long)H * (dim + rot));
+      P* __restrict__ vo = reinterpret_cast<P*>(v_out + row * (long long)H * vdim);
+#pragma unroll 8
+      for (int i = lane; i < H * vdim / E; i += 32) vo[i] = u[H * plain + i];
+#pragma unroll 8
+      for (int i = lane; i < H * kd; i += 32) {
+        const int h = i / kd, d = i - h * kd;
+        ko[i] = d < plain ? u[h * plain + d] : src[d - plain];
+      }
+    }
+    mine -= rows;
   }
 }
 
@@ -241,12 +268,14 @@ extern "C" int pg_latent_pack_kv(const void* up, long long ld_up, const void* pa
                                  const int* dense_row0, const int* entry_n, const int* entry_ctx, void* k_out, void* v_out, int entries, int max_len,
                                  int H, int dim, int rot, int vdim, int rank, int act_f32, void* stream) {
   if (entries <= 0 || entries > 65535 || max_len <= 0 || H <= 0 || dim <= 0 || rot < 0 || vdim <= 0 || rank <= 0 || page <= 0) return PG_ERR_ARG;
-  const dim3 grid((max_len + kRowsPerCta - 1) / kRowsPerCta < 4096 ? (max_len + kRowsPerCta - 1) / kRowsPerCta : 4096, entries);
+  // a warp per row as far as the rows can be known here, up to what is resident at once (six CTAs per SM)
+  const long long most = ((long long)entries * max_len + 7) / 8;
+  const dim3 grid((unsigned)(most < 6LL * pg::num_sms() ? most : 6LL * pg::num_sms()));
   const bool vec = whole_pieces(act_f32 ? 4 : 2, {dim, rot, vdim, rank, ld_up}, {up, pages, k_out, v_out});
   auto go = [&](auto kernel, auto t) {
     using TA = decltype(t);
     pg::launch_dependent(kernel, grid, 256, 0, PG_ST(stream), static_cast<const TA*>(up), ld_up, static_cast<const TA*>(pages), page_table, max_pages, page, dense_row0, entry_n,
-                                            entry_ctx, static_cast<TA*>(k_out), static_cast<TA*>(v_out), H, dim, rot, vdim, rank);
+                                            entry_ctx, static_cast<TA*>(k_out), static_cast<TA*>(v_out), entries, H, dim, rot, vdim, rank);
   };
   if (act_f32) vec ? go(latent_pack_kv_kernel<float, true>, float()) : go(latent_pack_kv_kernel<float, false>, float());
   else vec ? go(latent_pack_kv_kernel<bf16, true>, bf16()) : go(latent_pack_kv_kernel<bf16, false>, bf16());

@@ -72,3 +72,25 @@ def test_latent_rows(dtype, H, dim, rot, vdim, rank):
         assert torch.equal(ks[:, :, dim:], rows[:, None, rank:].expand(-1, H, -1))
         assert (ks[:, :, :dim].double() - up[:, :H * dim].view(-1, H, dim)).abs().max() <= tol * up.abs().max()
         assert (vs.double() - up[:, H * dim:].view(-1, H, vdim)).abs().max() <= tol * up.abs().max()
+
+
+@pytest.mark.parametrize("at", [0, 255, 256, 300])
+def test_latent_rows_of_one_entry_among_many(at):
+    H, dim, rot, vdim, rank = 3, 16, 8, 16, 32
+    entries = [(1, 5)] * 310
+    entries[at], entries[(at + 7) % 310] = (70, 30), (2, 0)
+    b, pages = _batch(entries)
+    cache = torch.randn(pages, 64, rank + rot, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(H * (dim + vdim), rank, device="cuda") * rank ** -0.5).to(torch.bfloat16)
+    k, v = seq_ops.latent_expand(cache, b, w, H, dim, rot, vdim, rank, 64, seq_ops.Precision(torch.bfloat16))
+    for e, (n, ctx) in enumerate(entries):
+        if n == 1:
+            continue
+        first = int(b.page_table[e, 0])
+        rows = cache[first:first + (n + ctx + 63) // 64].reshape(-1, rank + rot)[:n + ctx]
+        at = int(b.dense_row0[e])
+        up = rows[:, :rank].double() @ w.double().T
+        ks, vs = k[at:at + n + ctx].view(-1, H, dim + rot), v[at:at + n + ctx].view(-1, H, vdim)
+        assert torch.equal(ks[:, :, dim:], rows[:, None, rank:].expand(-1, H, -1))
+        assert (ks[:, :, :dim].double() - up[:, :H * dim].view(-1, H, dim)).abs().max() <= 2.0 ** -7 * up.abs().max()
+        assert (vs.double() - up[:, H * dim:].view(-1, H, vdim)).abs().max() <= 2.0 ** -7 * up.abs().max()
