@@ -501,7 +501,7 @@ int pg_attn_latent_decode_mma(const void* q, const void* pages, const void* gate
  * per head S <- decay[h] * S + k v^T, out[t, h * vdim + :] = S^T q (fp32).  state: fp32 [slots, H, dim, vdim]; entry e
  * continues state[entry_slot[e]] (from zero when entry_ctx[e] == 0) and leaves its new state there.
  * pg_linear_attn_scan steps token by token; pg_linear_attn_chunked advances in blocks of 32 tokens (same results up to
- * fp32 summation order) and is meant for prompt portions; pg_linear_attn_blocks does so on the tensor cores (bf16, silu == 0, dim <= 128,
+ * fp32 summation order) and is meant for prompt portions; pg_linear_attn_blocks does so on the tensor cores (bf16, dim <= 128,
  * dim and vdim multiples of 8, 16-byte aligned rows; every fp32 operand as three bf16 terms).
  * options (NULL: silu on q, k and v, every entry): silu == 0 -- q and k are turned in pairs (2i, 2i + 1) by the table `rotate` (fp32
  * [rows, 2, pairs]: cosines, then sines, of the step's rows, made by pg_rotary_table; NULL: not turned), k is multiplied by kscale, and

@@ -42,6 +42,7 @@ class StepBatch:
     max_pages: int
     singles: int = 0          # entries with one new token (decode rows)
     max_single_ctx: int = 0   # the longest context among them
+    min_n: int = 1            # the fewest new tokens of an entry (1 where that is not known)
     single_rows: Optional[tuple] = None  # (first, one past the last) row between which all of them lie; None: unknown
     # dense scratch layout of the entries with several new tokens (mixers that rebuild per-head keys / values from a compact
     # cache): entry e owns rows [dense_row0[e], + ctx + n) of a dense matrix, starting on a page boundary, so that
@@ -102,7 +103,7 @@ def make_step_batch(entries: Sequence[dict]) -> StepBatch:
         r += k
     dev = torch.from_numpy(buf).pin_memory().to("cuda", non_blocking=True)
     o = 3 * T
-    return StepBatch(T=T, E=E, max_n=max(ns), tokens=dev[:T], pos=dev[T:2 * T], row_entry=dev[2 * T:3 * T], row0=dev[o:o + E],
+    return StepBatch(T=T, E=E, max_n=max(ns), min_n=min(ns), tokens=dev[:T], pos=dev[T:2 * T], row_entry=dev[2 * T:3 * T], row0=dev[o:o + E],
                      n=dev[o + E:o + 2 * E], ctx=dev[o + 2 * E:o + 3 * E], slot=dev[o + 3 * E:o + 4 * E],
                      page_table=dev[o + 4 * E:o2].view(E, max_pages), max_pages=max_pages, singles=sum(k == 1 for k in ns),
                      max_single_ctx=max([e["ctx"] for e, k in zip(entries, ns) if k == 1], default=0), single_rows=_single_rows(ns),
@@ -699,12 +700,31 @@ LINEAR_ATTN_CHUNK_MIN = 8
 
 
 def linear_attn(qkv, state, decay, out, b: StepBatch, H, dim, vdim, chunked=None):
+    """S <- decay S + k v^T, out = S^T q per head (fp32 [T, H * vdim]) with q, k and v through silu.  Portions of some length go in blocks -- on the tensor cores for bf16
+    head sizes that fit, there an entry's own length decides -- the others token by token (chunked True / False: one form for every entry)."""
+    import ctypes as C
     assert state.dtype == torch.float32 and out.dtype == torch.float32 and out.is_contiguous() and qkv.stride(1) == 1
-    if chunked is None:
-        chunked = b.max_n >= LINEAR_ATTN_CHUNK_MIN
-    fn = _lib.lib().pg_linear_attn_chunked if chunked else _lib.lib().pg_linear_attn_scan
-    _lib.check(fn(qkv.data_ptr(), qkv.stride(0), state.data_ptr(), decay.data_ptr(), out.data_ptr(), b.row0.data_ptr(), b.n.data_ptr(),
-                  b.ctx.data_ptr(), b.slot.data_ptr(), b.E, H, dim, vdim, 0, int(qkv.dtype == torch.float32), _lib.stream()), "pg_linear_attn")
+    f32 = int(qkv.dtype == torch.float32)
+    n_min = {None: LINEAR_ATTN_CHUNK_MIN, True: 1, False: FOREVER}[chunked]
+    # not for a few heads of a few sequences: there the other block form has more CTAs (its value blocks get narrower), and a chain of blocks is what takes the time (us, FMA / tensor:
+    # 32 CTAs of 64 columns, 2000 tokens 330 / 370, 2 x 1000 tokens 171 / 191; 64 CTAs of 2000 tokens 458 / 371, of 100 tokens 35 / 29)
+    tensor_cores = (not f32 and dim % 8 == 0 and dim <= 128 and vdim % 8 == 0 and qkv.stride(0) % 8 == 0 and _aligned(qkv)
+                    and b.E * H * ((vdim + 63) // 64) >= 64)
+
+    def go(fn, lo, hi, *tail):
+        ops = _lib.LinearAttnOps(1, 1.0, 0, 0, lo, hi)
+        _lib.check(fn(qkv.data_ptr(), qkv.stride(0), state.data_ptr(), decay.data_ptr(), out.data_ptr(), b.row0.data_ptr(), b.n.data_ptr(), b.ctx.data_ptr(),
+                      b.slot.data_ptr(), b.E, H, dim, vdim, C.addressof(ops), *tail, _lib.stream()), "pg_linear_attn")
+
+    L = _lib.lib()
+    if b.max_n < n_min:
+        go(L.pg_linear_attn_scan, 1, FOREVER, f32)
+    elif not tensor_cores:
+        go(L.pg_linear_attn_chunked, 1, FOREVER, f32)
+    else:
+        go(L.pg_linear_attn_blocks, n_min, FOREVER)
+        if b.min_n < n_min:
+            go(L.pg_linear_attn_scan, 1, n_min - 1, f32)
 
 
 def rotary_table(b: StepBatch, freq, rot_dims, dim, gain=1.0):
