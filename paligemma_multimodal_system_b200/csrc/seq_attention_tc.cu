@@ -7,14 +7,21 @@
 // every tcgen05.mma, warps 2 .. 5 are the softmax, a thread per query row:
 //   * S = Q K^T: 128 x 64 into tensor memory; a thread reads its row of 64 scores, masks, exponentiates -- no exchange between lanes, the row sum is its own;
 //   * P goes back to tensor memory as three 32-column bf16 tiles and is the A operand of P V from there (12 instructions a tile): it never passes through shared memory;
-//   * S of the next tile is multiplied while this tile's exponentials run (values 64 wide; for 128 the 256 columns of a CTA leave no room for S beside P);
+//   * P lies over its own S (read by then) and 32 columns more, and there are two such areas (values 64 wide; for 128 the 256 columns of a CTA leave room for one): the next
+//     tile's S is multiplied while this tile's exponentials run, and no tile waits for P V of the one before unless it rescales O.  So a warp cuts one piece of a row
+//     (logic pipe) while the exponentials of the next are under way (MUFU);
+//   * query rows come by TMA where a CTA has 128 of them and whole tokens, else with all of a thread's pieces requested together;
 //   * O is rescaled only when a row's maximum grew by more than 2^8 (fp32 sums have the room);
 //   * P V runs over all 128 rows with zero weights where a row does not see a key, and zero times a value that is not finite is no zero.  So a row whose sums are not finite is
 //     computed again from the keys that it sees (row_from_visible_keys): a broken value reaches the rows that see it and no others.  (Rows that end or begin inside the loop
 //     instead cost every prompt: 8 x 1024 tokens 140 -> 147 us; the check 142.)
-// What bounds it: the softmax warps (clocks a tile, stamped: wait for S 100, its load 75, maxima and exponentials 1000 .. 1330, wait for P V 185, split 520; the products hide
-// behind them).  Two threads a row share the same pipes (146 us for 149), exponentials as polynomials on the FMA pipe cost more than they save (168).  us, mma.sync / here: 8 prompts of 897 .. 1024 tokens, 32 heads x 64 over 8 k/v heads 235 / 149; 2 portions of 333
-// tokens behind 1400, 32 heads x 96 / 64: 144 / 66.
+// What bounds it: the softmax warps (MUFU 512 clocks a tile and warp, logic and permutes for the split 450, two warps on each pipe) and, with few tiles a CTA, its start (entry, page
+// table, first tile: each a trip to memory).  Two threads a row share the same pipes, exponentials as polynomials on the FMA pipe cost more than they save.
+// us, mma.sync / here: 8 prompts of 897 .. 1024 tokens, 32 heads x 64 over 8 k/v heads 235 / 103; 2 portions of 333
+// tokens behind 1400, 32 heads x 96 / 64: 144 / 58 (with P beside S, every tile waiting for P V of the one before, and query rows copied one piece after the other: 142 and 65;
+// there a CTA of eight tiles spent 6500 of 31700 clocks before its first barrier).
+#include <string.h>
+
 #include "common.cuh"
 #include "paligemma_b200.h"
 #include "tmap.cuh"
@@ -44,6 +51,11 @@ PG_DEVINL void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
       "r"(r[14]), "r"(r[15])
       : "memory");
 }
+PG_DEVINL void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
+               "r"(r[7])
+               : "memory");
+}
 PG_DEVINL void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // MN-major operand as TMA lays it out ([k rows][64 columns], 128B swizzle); 64-column boxes `box` bytes apart
@@ -69,14 +81,28 @@ PG_DEVINL float tanh32(float x) {
   const float big = copysignf(1.0f - __fdividef(2.0f, ex2(ax * 2.885390082f) + 1.0f), x);
   return ax < 0.1f ? small : big;
 }
-PG_DEVINL void split3(float p, float q, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  const uint32_t up = __float_as_uint(p), uq = __float_as_uint(q);
-  hi = __byte_perm(up, uq, 0x7632);
-  const float rp = p - __uint_as_float(up & 0xffff0000u), rq = q - __uint_as_float(uq & 0xffff0000u);
-  const uint32_t vp = __float_as_uint(rp), vq = __float_as_uint(rq);
-  mid = __byte_perm(vp, vq, 0x7632);
-  const float sp = rp - __uint_as_float(vp & 0xffff0000u), sq = rq - __uint_as_float(vq & 0xffff0000u);
-  lo = __byte_perm(__float_as_uint(sp), __float_as_uint(sq), 0x7632);
+// two fp32 values side by side: one instruction for two sums or products, rounded as two (the softmax warps are short of issue slots)
+PG_DEVINL uint64_t pair_of(uint32_t lo, uint32_t hi) { return static_cast<uint64_t>(hi) << 32 | lo; }
+PG_DEVINL uint64_t pair_of(float lo, float hi) { return pair_of(__float_as_uint(lo), __float_as_uint(hi)); }
+PG_DEVINL uint32_t lo_of(uint64_t p) { return static_cast<uint32_t>(p); }
+PG_DEVINL uint32_t hi_of(uint64_t p) { return static_cast<uint32_t>(p >> 32); }
+PG_DEVINL uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+PG_DEVINL uint64_t add_pair(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+PG_DEVINL void split3(uint64_t p, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  constexpr uint64_t minus = 0xbf800000bf800000ull;
+  hi = __byte_perm(lo_of(p), hi_of(p), 0x7632);
+  const uint64_t r = fma_pair(pair_of(lo_of(p) & 0xffff0000u, hi_of(p) & 0xffff0000u), minus, p);
+  mid = __byte_perm(lo_of(r), hi_of(r), 0x7632);
+  const uint64_t t = fma_pair(pair_of(lo_of(r) & 0xffff0000u, hi_of(r) & 0xffff0000u), minus, r);
+  lo = __byte_perm(lo_of(t), hi_of(t), 0x7632);
 }
 
 template <int DIM, int VDIM>
@@ -85,8 +111,8 @@ struct Shape {
   static constexpr int Q_BYTES = KB * 128 * 128, KV_BYTES = (KB + VB) * kBox;
   static constexpr int STAGES = (112 * 1024 - Q_BYTES - 256) / KV_BYTES < 4 ? (112 * 1024 - Q_BYTES - 256) / KV_BYTES : 4;
   static constexpr int SMEM = Q_BYTES + STAGES * KV_BYTES + 256;
-  static constexpr bool ALIAS = VDIM > 64;                       // P over S
-  static constexpr int COL_P = ALIAS ? 0 : 64, COL_O = COL_P + 96;
+  static constexpr int NBUF = VDIM > 64 ? 1 : 2;                 // areas of 96 columns: S, then P over it
+  static constexpr int COL_O = 96 * NBUF;
   static_assert(COL_O + VDIM <= 256 && STAGES >= 2 && DIM % 16 == 0 && VDIM % 64 == 0, "two CTAs per SM");
 };
 
@@ -146,27 +172,59 @@ __device__ __noinline__ void row_from_visible_keys(const bf16* __restrict__ q, c
 }
 
 template <int DIM, int VDIM>
-__global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
+__global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                                                                     const __grid_constant__ CUtensorMap tmV,
                                                                      const bf16* __restrict__ q, const bf16* __restrict__ k_pages, const bf16* __restrict__ v_pages,
                                                                      const bf16* __restrict__ gate, long long ldg, bf16* __restrict__ out,
                                                                      const int* __restrict__ entry_row0, const int* __restrict__ entry_n, const int* __restrict__ entry_ctx,
                                                                      const int* __restrict__ page_table, int max_pages, int page, int H, int G, float scale, float softcap,
-                                                                     int skip_single, int gate_per_head, PgAttnScore sx) {
+                                                                     int skip_single, int gate_per_head, int q_tma, int entries, PgAttnScore sx) {
   using C = Shape<DIM, VDIM>;
   constexpr uint32_t IDESC_S = make_idesc_bf16(128, 64), IDESC_O = make_idesc_bf16(128, VDIM, 0, 1);
   griddep_wait();
-  const int e = blockIdx.z, g = blockIdx.y, gsz = H / G;
+  // The longest rows of all entries and heads come first (48 prompts of 193 .. 256 tokens, soft-capped: 243 us entry by entry, 198 so).  Where single tokens are left to another
+  // kernel, the entries with rows are counted and numbered first, so that CTAs without any stand at the end and not between two blocks of rows (2 portions + 40 singles, 4032
+  // CTAs of which 192 have rows: 58 us entry by entry, 71 with the 2700 empty ones of the first two blocks in front of the third).
+  const unsigned idx = blockIdx.x, blocks = gridDim.x / static_cast<unsigned>(entries * G);
+  unsigned with_rows = entries;
+  if (skip_single) {
+    with_rows = 0;
+    for (int i = 0; i < entries; i += 32) {
+      const int at = i + static_cast<int>(lane_id());
+      with_rows += __popc(__ballot_sync(0xffffffffu, at < entries && entry_n[at] != 1));
+    }
+  }
+  if (idx >= blocks * with_rows * G) return;
+  const unsigned unit = idx % (with_rows * G);
+  int e = unit / G;
+  if (skip_single) {
+    int left = e;
+    for (int i = 0;; i += 32) {
+      const int at = i + static_cast<int>(lane_id());
+      const unsigned here = __ballot_sync(0xffffffffu, at < entries && entry_n[at] != 1);
+      if (left < __popc(here)) {
+        e = i + __fns(here, 0, left + 1);
+        break;
+      }
+      left -= __popc(here);
+    }
+  }
+  const int g = unit % G, gsz = H / G;
   const int n = entry_n[e], ctx = entry_ctx[e], row0 = entry_row0[e];
-  const int rows = n * gsz, r0 = (gridDim.x - 1 - blockIdx.x) * 128;  // the longest rows start first
-  if ((skip_single && n == 1) || r0 >= rows) return;
+  const int rows = n * gsz, r0 = static_cast<int>(blocks - 1 - idx / (with_rows * G)) * 128;
+  if (r0 >= rows) return;
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t base = smem_u32(smem);
   if ((base & 1023u) != 0) __trap();
   const uint32_t kv0 = base + C::Q_BYTES, bar0 = kv0 + C::STAGES * C::KV_BYTES;
   auto kv_full = [&](int s) { return bar0 + 8u * s; };
   auto kv_empty = [&](int s) { return bar0 + 8u * (4 + s); };
-  const uint32_t s_full = bar0 + 64, s_empty = bar0 + 72, p_full = bar0 + 80, o_done = bar0 + 88, tmem_slot = bar0 + 96;
+  auto s_full = [&](int b) { return bar0 + 64u + 8u * b; };
+  auto p_full = [&](int b) { return bar0 + 80u + 8u * b; };
+  auto o_done = [&](int b) { return bar0 + 96u + 8u * b; };  // (two: with one, a wait for tile j - 1 would pass while j - 2 is still under way)
+  const uint32_t q_full = bar0 + 112, tmem_slot = bar0 + 120;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool by_tma = q_tma && r0 + 128 <= rows;  // (rows past the entry's may lie past the end of q)
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmV);
@@ -174,26 +232,42 @@ __global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __gri
       mbar_init(kv_full(s), 1);
       mbar_init(kv_empty(s), 1);
     }
-    mbar_init(s_full, 1);
-    mbar_init(s_empty, 4);
-    mbar_init(p_full, 4);
-    mbar_init(o_done, 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(s_full(b), 1);
+      mbar_init(p_full(b), 4);
+      mbar_init(o_done(b), 1);
+    }
+    mbar_init(q_full, 1);
     mbar_fence_init();
+    if (by_tma) {
+      mbar_expect_tx(q_full, C::Q_BYTES);
+#pragma unroll
+      for (int b = 0; b < C::KB; ++b) tma_load_3d(base + b * (128 * 128), &tmQ, q_full, 64 * b, g * gsz, row0 + r0 / gsz, kEvictNormal);
+    }
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 256);
     tmem_relinquish();
   }
-  // query rows, swizzled as TMA would lay them (zeros past the end and past DIM)
-  for (int id = threadIdx.x; id < 128 * C::KB * 8; id += kThreads) {
-    const int r = id / (C::KB * 8), cc = id % (C::KB * 8), rr = r0 + r;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (rr < rows && cc * 8 < DIM)
-      v = *reinterpret_cast<const uint4*>(q + static_cast<long long>(row0 + rr / gsz) * (static_cast<long long>(H) * DIM) + static_cast<long long>(g * gsz + rr % gsz) * DIM + cc * 8);
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(base + (cc >> 3) * (128 * 128) + r * 128 + (((cc & 7) ^ (r & 7)) << 4)), "r"(v.x), "r"(v.y), "r"(v.z),
-                 "r"(v.w) : "memory");
+  if (!by_tma) {  // query rows, swizzled as TMA would lay them (zeros past the end and past DIM)
+    constexpr int N = (128 * C::KB * 8 + kThreads - 1) / kThreads;
+    uint4 v[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int id = threadIdx.x + i * kThreads, r = id / (C::KB * 8), cc = id % (C::KB * 8), rr = r0 + r;
+      v[i] = make_uint4(0, 0, 0, 0);
+      if (r < 128 && rr < rows && cc * 8 < DIM)
+        v[i] = *reinterpret_cast<const uint4*>(q + static_cast<long long>(row0 + rr / gsz) * (static_cast<long long>(H) * DIM) + static_cast<long long>(g * gsz + rr % gsz) * DIM + cc * 8);
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int id = threadIdx.x + i * kThreads, r = id / (C::KB * 8), cc = id % (C::KB * 8);
+      if (r < 128)
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(base + (cc >> 3) * (128 * 128) + r * 128 + (((cc & 7) ^ (r & 7)) << 4)), "r"(v[i].x), "r"(v[i].y), "r"(v[i].z),
+                     "r"(v[i].w) : "memory");
+    }
+    fence_proxy_async_smem();
   }
-  fence_proxy_async_smem();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -239,31 +313,30 @@ __global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __gri
     }
     __syncwarp();
   } else if (warp == 1) {
-    auto issue_s = [&](uint32_t sk) {
+    // tile j: S in area j % NBUF, its P over it; S of tile j + NBUF behind P V of tile j, whose area it takes (one thread's products run in order)
+    int stage = 0, ahead = 0, ks = k_first, js = 0;  // stages of P V and of S; key and number of the next S
+    uint32_t ahead_phase = 0;
+    auto issue_s = [&]() {
+      mbar_wait(kv_full(ahead), ahead_phase);
+      tc_fence_after();
+      const uint32_t sk = kv0 + ahead * C::KV_BYTES, to = tmem + 96 * (js % C::NBUF);
       if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < DIM / 16; ++k)
-          umma_f16(tmem, make_sdesc_k_sw128(base + (k >> 2) * (128 * 128)) + 2 * (k & 3), make_sdesc_k_sw128(sk + (k >> 2) * kBox) + 2 * (k & 3), IDESC_S, k > 0 ? 1u : 0u);
-        umma_commit(s_full);
+          umma_f16(to, make_sdesc_k_sw128(base + (k >> 2) * (128 * 128)) + 2 * (k & 3), make_sdesc_k_sw128(sk + (k >> 2) * kBox) + 2 * (k & 3), IDESC_S, k > 0 ? 1u : 0u);
+        umma_commit(s_full(js % C::NBUF));
       }
       __syncwarp();
+      if (++ahead == C::STAGES) { ahead = 0; ahead_phase ^= 1; }
+      ks = next_tile(ks);
+      ++js;
     };
-    int stage = 0, ahead = 0;  // stages of P V and of S
-    uint32_t ahead_phase = 0, par = 0;
-    mbar_wait(kv_full(0), 0);
-    tc_fence_after();
-    issue_s(kv0);
-    if (++ahead == C::STAGES) { ahead = 0; ahead_phase ^= 1; }
-    for (int k0 = k_first; k0 <= kmax; par ^= 1) {
-      const int nx = next_tile(k0);
-      const uint32_t sk = kv0 + stage * C::KV_BYTES, sv = sk + C::KB * kBox;
-      if (!C::ALIAS && nx <= kmax) {  // S of the next tile as soon as the softmax has read this one
-        mbar_wait(kv_full(ahead), ahead_phase);
-        mbar_wait(s_empty, par);
-        tc_fence_after();
-        issue_s(kv0 + ahead * C::KV_BYTES);
-        if (++ahead == C::STAGES) { ahead = 0; ahead_phase ^= 1; }
-      }
+    if (by_tma) mbar_wait(q_full, 0);
+    for (int b = 0; b < C::NBUF; ++b)
+      if (ks <= kmax) issue_s();
+    int j = 0;
+    for (int k0 = k_first; k0 <= kmax; k0 = next_tile(k0), ++j) {
+      const uint32_t sv = kv0 + stage * C::KV_BYTES + C::KB * kBox, area = tmem + 96 * (j % C::NBUF);
       if (k0 + 63 > kmax) {  // the last tile: keys nobody sees weigh zero, whatever lies there
         for (int r = kmax + 1 - k0 + lane; r < 64; r += 32)
 #pragma unroll
@@ -273,27 +346,20 @@ __global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __gri
         fence_proxy_async_smem();
         __syncwarp();
       }
-      mbar_wait(p_full, par);
+      mbar_wait(p_full(j & 1), (j >> 1) & 1);
       tc_fence_after();
       if (elect_one()) {
 #pragma unroll
         for (int term = 0; term < 3; ++term)
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            umma_f16_ts(tmem + C::COL_O, tmem + C::COL_P + term * 32 + k * 8, make_sdesc_mn_sw128(sv + k * 2048, kBox), IDESC_O, (k0 > k_first || term > 0 || k > 0) ? 1u : 0u);
+            umma_f16_ts(tmem + C::COL_O, area + term * 32 + k * 8, make_sdesc_mn_sw128(sv + k * 2048, kBox), IDESC_O, (j > 0 || term > 0 || k > 0) ? 1u : 0u);
         umma_commit(kv_empty(stage));
-        umma_commit(o_done);
+        umma_commit(o_done(j & 1));
       }
       __syncwarp();
-      if (C::ALIAS && nx <= kmax) {  // P lies where S goes
-        mbar_wait(kv_full(ahead), ahead_phase);
-        mbar_wait(o_done, par);
-        tc_fence_after();
-        issue_s(kv0 + ahead * C::KV_BYTES);
-        if (++ahead == C::STAGES) { ahead = 0; ahead_phase ^= 1; }
-      }
+      if (ks <= kmax) issue_s();
       if (++stage == C::STAGES) stage = 0;
-      k0 = nx;
     }
   } else {
     const int qd = warp & 3, r = qd * 32 + lane, rr = r0 + r;
@@ -309,23 +375,19 @@ __global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __gri
     const bool plain = !(softcap > 0.f) && sx.head_scale == nullptr && scale > 0.f;  // the maximum commutes with the scale, which rides on the exponent's FMA
     const float unit = plain ? scale * kLog2e : kLog2e, in = softcap > 0.f ? sc / softcap : 0.f;
     float m = -INFINITY, l = 0.f;
-    uint32_t par = 0;
-    for (int k0 = k_first; k0 <= kmax; k0 = next_tile(k0), par ^= 1) {
-      mbar_wait(s_full, par);
+    int j = 0;
+    for (int k0 = k_first; k0 <= kmax; k0 = next_tile(k0), ++j) {
+      const uint32_t area = lanes + 96 * (j % C::NBUF);
+      mbar_wait(s_full(j % C::NBUF), (j / C::NBUF) & 1);
       tc_fence_after();
       float s[64];
       {
         uint32_t v[4][16];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_ld16(lanes + 16 * c, v[c]);
+        for (int c = 0; c < 4; ++c) tmem_ld16(area + 16 * c, v[c]);
         tmem_ld_wait();
 #pragma unroll
         for (int i = 0; i < 64; ++i) s[i] = __uint_as_float(v[i >> 4][i & 15]);
-      }
-      if (!C::ALIAS) {
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(s_empty);
       }
       if (!plain) {
         if (softcap > 0.f) {
@@ -355,43 +417,53 @@ __global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __gri
       const float mn = need ? mx : m;
       const float alpha = need ? ex2(m - mn) : 1.0f, off = mn > -INFINITY ? -mn : 0.f;  // rows that see no key yet weigh nothing
       m = mn;
-      float s4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int i = 0; i < 64; ++i) {
-        s[i] = ex2(fmaf(s[i], unit, off));
-        s4[i & 3] += s[i];
-      }
-      l = l * alpha + ((s4[0] + s4[1]) + (s4[2] + s4[3]));
-      if (k0 > k_first) {
-        mbar_wait(o_done, par ^ 1);  // P V of the tile before: P may be overwritten and O touched
+      if (__any_sync(0xffffffffu, need) && j > 0) {
+        mbar_wait(o_done((j - 1) & 1), ((j - 1) >> 1) & 1);  // P V of the tile before
         tc_fence_after();
-        if (__any_sync(0xffffffffu, need)) {
 #pragma unroll 1
-          for (int c = 0; c < VDIM; c += 16) {
-            uint32_t v[16];
-            tmem_ld16(lanes + C::COL_O + c, v);
-            tmem_ld_wait();
+        for (int c = 0; c < VDIM; c += 16) {
+          uint32_t v[16];
+          tmem_ld16(lanes + C::COL_O + c, v);
+          tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-            tmem_st16(lanes + C::COL_O + c, v);
-          }
+          for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
+          tmem_st16(lanes + C::COL_O + c, v);
         }
       }
+      // pieces of 16 scores: the exponentials of a piece are requested before the piece in front is cut and stored
+      uint64_t s2[2] = {0, 0}, pp[2][8];
+      const uint64_t unit2 = pair_of(unit, unit), off2 = pair_of(off, off);
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        uint32_t a[16], b[16], c[16];
+      for (int c = 0; c < 5; ++c) {
+        if (c < 4) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) split3(s[32 * h + 2 * i], s[32 * h + 2 * i + 1], a[i], b[i], c[i]);
-        tmem_st16(lanes + C::COL_P + 16 * h, a);
-        tmem_st16(lanes + C::COL_P + 32 + 16 * h, b);
-        tmem_st16(lanes + C::COL_P + 64 + 16 * h, c);
+          for (int i = 0; i < 8; ++i) {
+            const int at = (16 * c + 2 * i) & 63;
+            const uint64_t x = fma_pair(pair_of(s[at], s[at + 1]), unit2, off2);
+            pp[c & 1][i] = pair_of(ex2(__uint_as_float(lo_of(x))), ex2(__uint_as_float(hi_of(x))));
+          }
+        }
+        if (c > 0) {
+          uint32_t hi[8], mid[8], low[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const uint64_t p = pp[(c - 1) & 1][i];
+            s2[i & 1] = add_pair(s2[i & 1], p);
+            split3(p, hi[i], mid[i], low[i]);
+          }
+          tmem_st8(area + 8 * (c - 1), hi);
+          tmem_st8(area + 32 + 8 * (c - 1), mid);
+          tmem_st8(area + 64 + 8 * (c - 1), low);
+        }
       }
+      s2[0] = add_pair(s2[0], s2[1]);
+      l = l * alpha + (__uint_as_float(lo_of(s2[0])) + __uint_as_float(hi_of(s2[0])));
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(p_full);
+      if (lane == 0) mbar_arrive(p_full(j & 1));
     }
-    mbar_wait(o_done, par ^ 1);
+    mbar_wait(o_done((j - 1) & 1), ((j - 1) >> 1) & 1);
     tc_fence_after();
     float osc = 1.f;
     if (sx.sink != nullptr) {  // the sink joins the denominator once (m is in base-2 units)
@@ -406,11 +478,16 @@ __global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __gri
     bool odd = false;  // a sum of the row is not finite
     const float gh = gate != nullptr && gate_per_head ? 1.0f / (1.0f + expf(-__bfloat162float(*gt))) : 1.f;
 #pragma unroll 1
-    for (int c = 0; c < VDIM; c += 16) {
-      uint32_t v[16];
-      tmem_ld16(lanes + C::COL_O + c, v);
+    for (int c0 = 0; c0 < VDIM; c0 += 64) {
+      uint32_t all[4][16];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) tmem_ld16(lanes + C::COL_O + c0 + 16 * i, all[i]);
       tmem_ld_wait();
-      if (there) {
+#pragma unroll
+      for (int part = 0; part < 4; ++part) {
+        if (!there) break;
+        const int c = c0 + 16 * part;
+        const uint32_t(&v)[16] = all[part];
         float x[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
@@ -460,6 +537,8 @@ int launch(const void* q, const void* kp, const void* vp, const void* gate, long
            int max_pages, int page, int entries, int max_n, int H, int G, float scale, float softcap, int skip_single, int gate_per_head, const PgAttnScore& sx,
            cudaStream_t st) {
   using C = Shape<DIM, VDIM>;
+  const long long ctas = (static_cast<long long>(max_n) * (H / G) + 127) / 128 * G * entries;
+  if (ctas > 0x7fffffff) return 1;
   static bool configured[kMaxDevices] = {};
   const int dev = current_device();
   if (!configured[dev]) {
@@ -469,14 +548,24 @@ int launch(const void* q, const void* kp, const void* vp, const void* gate, long
     }
     configured[dev] = true;
   }
+  const int gsz = H / G;
+  // query rows of whole tokens: boxes of [128 / gsz tokens][gsz heads][64 columns]; only rows of the step are read, so the token count is a bound and not a size
+  const int q_tma = 128 % gsz == 0;
+  CUtensorMap tq;
+  if (q_tma) {
+    const int rcq = make_tmap_rows3(&tq, q, DIM, H, 1LL << 24, gsz, 128 / gsz);
+    if (rcq != PG_OK) return rcq;
+  } else {
+    memset(&tq, 0, sizeof(tq));
+  }
   // the pools as matrices of rows: only pages named by the table are read, so the row count is a bound and not a size
   CUtensorMap tk, tv;
   int rc;
   if ((rc = make_tmap_2d(&tk, kp, 1LL << 30, static_cast<long long>(G) * DIM, static_cast<long long>(G) * DIM, page < 64 ? page : 64)) != PG_OK) return rc;
   if ((rc = make_tmap_2d(&tv, vp, 1LL << 30, static_cast<long long>(G) * VDIM, static_cast<long long>(G) * VDIM, page < 64 ? page : 64)) != PG_OK) return rc;
-  launch_spread(attn_ragged_tc_kernel<DIM, VDIM>, dim3((max_n * (H / G) + 127) / 128, G, entries), dim3(kThreads), C::SMEM, st, tk, tv, static_cast<const bf16*>(q),
+  launch_spread(attn_ragged_tc_kernel<DIM, VDIM>, dim3(static_cast<unsigned>(ctas)), dim3(kThreads), C::SMEM, st, tq, tk, tv, static_cast<const bf16*>(q),
                 static_cast<const bf16*>(kp), static_cast<const bf16*>(vp), static_cast<const bf16*>(gate), ldg, static_cast<bf16*>(out), row0, n, ctx, pt, max_pages, page, H, G,
-                scale, softcap, skip_single, gate_per_head, sx);
+                scale, softcap, skip_single, gate_per_head, q_tma, entries, sx);
   pg_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
 }

@@ -36,4 +36,18 @@ inline int make_tmap_2d(CUtensorMap* m, const void* ptr, long long rows, long lo
   return r == CUDA_SUCCESS ? PG_OK : PG_ERR_TMAP;
 }
 
+// 3D bf16 [outer][mid][cols], dense, box = [box_outer][box_mid][64 cols = 128 B], 128B swizzle, OOB -> zeros
+inline int make_tmap_rows3(CUtensorMap* m, const void* ptr, long long cols, long long mid, long long outer, int box_mid, int box_outer) {
+  EncodeTiledFn enc = get_encode_fn();
+  if (!enc) return PG_ERR_DRIVER;
+  cuuint64_t gdim[3] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(mid), static_cast<cuuint64_t>(outer)};
+  cuuint64_t gstr[2] = {static_cast<cuuint64_t>(cols) * 2, static_cast<cuuint64_t>(cols) * 2 * static_cast<cuuint64_t>(mid)};
+  cuuint32_t box[3] = {64u, static_cast<cuuint32_t>(box_mid), static_cast<cuuint32_t>(box_outer)};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), gdim, gstr, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? PG_OK : PG_ERR_TMAP;
+}
+
 }  // namespace pg

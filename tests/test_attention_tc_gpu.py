@@ -59,7 +59,16 @@ def test_either_side_of_a_handful_of_rows(n):
     _run(64, 64, 40, 4, (n, 2, n, 1), (70, 0, 300, 5), 0, 0)  # 16 and 20 rows in 160 CTAs
 
 
-def _run(dim, vdim, G, gsz, ns, ctxs, window, keep, softcap=0.0, hs=False, sink=False, gate=None, ld=False, scale=None, big=False):
+@pytest.mark.parametrize("dim,vdim,G,gsz", [(64, 64, 2, 4), (96, 64, 3, 1), (128, 128, 1, 2)])
+@pytest.mark.parametrize("at", [0, 31, 32, 69])
+def test_portions_among_many_single_tokens(dim, vdim, G, gsz, at):
+    """Single tokens left to another kernel: the entries with rows are found by their number among 32, 64 and more."""
+    ns, ctxs = [1] * 70, [0] * 70
+    ns[at], ctxs[at], ns[(at + 33) % 70], ctxs[(at + 33) % 70] = 200, 40, 3, 90
+    _run(dim, vdim, G, gsz, ns, ctxs, 0, 0, skip=True)
+
+
+def _run(dim, vdim, G, gsz, ns, ctxs, window, keep, softcap=0.0, hs=False, sink=False, gate=None, ld=False, scale=None, big=False, skip=False):
     H, scale = G * gsz, dim ** -0.5 if scale is None else scale
     rows, first = [], 0
     for i, (n, c) in enumerate(zip(ns, ctxs)):
@@ -86,14 +95,17 @@ def _run(dim, vdim, G, gsz, ns, ctxs, window, keep, softcap=0.0, hs=False, sink=
     out = torch.full((b.T, pitch), 7.0, device="cuda", dtype=torch.bfloat16)
     g = None if gate is None else _t(b.T, H if gate == "head" else H * vdim, seed=5)
     score = seq_ops.ScoreOptions(H, window or None, keep, sink=skt, head_scale=hst, out_scale=0.5 if ld else 1.0, out_ld=pitch if ld else 0)
-    seq_ops.attn_ragged(q, kp, vp, g, out, b, H, G, dim, vdim, scale, softcap, 64, gate_per_head=gate == "head", score=score, decode_kernel=False)
+    seq_ops.attn_ragged(q, kp, vp, g, out, b, H, G, dim, vdim, scale, softcap, 64, gate_per_head=gate == "head", score=score, decode_kernel=False, skip_singles=skip)
     r = 0
     for i, (n, c) in enumerate(zip(ns, ctxs)):
         want = _want(q[r:r + n].view(n, H, dim), ks[i], vs[i], c, scale, softcap, window, keep, hst, skt) * (0.5 if ld else 1.0)
         if g is not None:
             want = want * torch.sigmoid(g[r:r + n].double()).view(n, H, -1)
         got = out[r:r + n, : H * vdim].double().view(n, H, vdim)
-        assert ((got - want).abs() <= want.abs() * 2.0 ** -8 + (2e-4 if big else 5e-5)).all(), (i, (got - want).abs().max().item())
+        if skip and n == 1:
+            assert (got == 7).all()
+        else:
+            assert ((got - want).abs() <= want.abs() * 2.0 ** -8 + (2e-4 if big else 5e-5)).all(), (i, (got - want).abs().max().item())
         r += n
     if ld:
         assert (out[:, H * vdim:] == 7).all()
