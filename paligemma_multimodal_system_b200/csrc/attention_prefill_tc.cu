@@ -17,7 +17,7 @@
 //               bf16 in the swizzled A-operand layout.  The running maximum is only advanced when it grew by more than 2^8
 //               (the O accumulator in TMEM then gets rescaled in place), which keeps the accumulator round trip off the
 //               common path.  dh <= 128: QT = 2 -- warps 2-5 own query tile 0, warps 6-9 tile 1, sharing every K / V tile;
-//               3 of 8 exponentials run on the FMA pipe (exp2_fma), the row sums of dh = 72 come from the tensor core (a
+//               3 of 8 exponentials run on the FMA pipe (exp2_fma_pair), the row sums of dh = 72 come from the tensor core (a
 //               ones column in the padded V tile).  dh = 256: QT = 1, four softmax warps (SW = 1).  SW = 2 (eight warps, two
 //               column halves of one row exchanging their maxima through shared memory) remains for single-tile problems.
 // S_{j+1} is computed while the softmax of tile j runs, and P_j V_j runs while the softmax of tile j+1 runs.
@@ -28,8 +28,8 @@
 #include "paligemma_b200.h"
 #include "tmap.cuh"
 
-#ifndef PG_AP_POLY8
-#define PG_AP_POLY8 3
+#ifndef PG_AP_POLY16
+#define PG_AP_POLY16 6
 #endif
 
 namespace pg {
@@ -46,6 +46,8 @@ struct Params {
   int stagger;          // QT = 2 (tuning): clock cycles the softmax group of query tile 1 idles after its first S tile is ready
   long long* trace;     // optional clock64 stamps of CTA (0,0,0): [role][tile][event]
   int trigger;          // the next kernel may come (weights_follow)
+  int m_blks, heads;    // blocks of QT query tiles of a (head, batch); heads
+  int whole;            // CTAs with QT query tiles; those behind them take one tile of a block each
 };
 
 template <int DH, int QT>
@@ -145,14 +147,15 @@ PG_DEVINL float exp2_mufu(float x) {
 // probability that follows), n added into the exponent field.  x <= 8 by the lazy maximum; x = -inf (masked keys) clamps to
 // 2^-126, which rounds to a bf16 denormal that weighs nothing.
 // (An earlier measurement showed "no gain": at that time the single MMA-issuing thread, not the softmax, paced the kernel.)
-PG_DEVINL float exp2_fma(float x) {
-  x = fmaxf(x, -126.0f);
-  const float t = x + 12582912.0f;
-  const float f = x - (t - 12582912.0f);
-  float p = fmaf(f, 0.05518874f, 0.24261212f);  // minimax cubic of 2^f on [-0.5, 0.5]: max relative error 7.5e-5
-  p = fmaf(p, f, 0.69325641f);
-  p = fmaf(p, f, 0.99992746f);
-  return __int_as_float(__float_as_int(p) + (__float_as_int(t) << 23));
+// Two at a time: five issue slots a score instead of nine.
+PG_DEVINL uint64_t exp2_fma_pair(uint64_t x) {
+  x = pair_of(fmaxf(lo_f32(x), -126.0f), fmaxf(hi_f32(x), -126.0f));
+  const uint64_t t = add_pair(x, pair_of(12582912.0f, 12582912.0f));
+  const uint64_t f = fma_pair(add_pair(t, pair_of(-12582912.0f, -12582912.0f)), pair_of(-1.0f, -1.0f), x);
+  uint64_t p = fma_pair(f, pair_of(0.05518874f, 0.05518874f), pair_of(0.24261212f, 0.24261212f));  // minimax cubic of 2^f on [-0.5, 0.5]: max relative error 7.5e-5
+  p = fma_pair(p, f, pair_of(0.69325641f, 0.69325641f));
+  p = fma_pair(p, f, pair_of(0.99992746f, 0.99992746f));
+  return pair_of(lo_of(p) + (lo_of(t) << 23), hi_of(p) + (hi_of(t) << 23));
 }
 // QT = query tiles (128 rows each) per CTA.  QT = 2 (dh <= 128): both tiles run against the SAME K / V tiles in shared
 // memory -- the kernel is bound by K/V delivery through the crossbar (profiles/r01d_prefill_attn72_ncu_full.csv), and two
@@ -168,9 +171,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   // the row sums of the (bf16) probabilities on the tensor core and the softmax warps -- bound by instruction issue, ~4.5
   // instructions per score -- drop the FADD per score.  The lazy rescale of O carries the column along.
   constexpr bool TCSUM = DHP > DH;
-  // scores per 8 whose exponential runs on the FMA pipe (exp2_fma): MUFU and FMA / issue time balance near 3 of 8 for dh <= 128;
+  // scores per 16 whose exponential runs on the FMA pipe (exp2_fma_pair): MUFU and FMA / issue time balance near 6 of 16 for dh <= 128;
   // dh = 256 has four times the tensor work per score and is not softmax-bound
-  constexpr int POLY8 = DH <= 128 ? PG_AP_POLY8 : 0;
+  constexpr int POLY16 = DH <= 128 ? PG_AP_POLY16 : 0;
   constexpr uint32_t IDESC_S = make_idesc_bf16(BM, BN);
   constexpr uint32_t IDESC_O = make_idesc_bf16(BM, DHP, 0, 1);  // B (= V) is MN-major
   extern __shared__ __align__(1024) uint8_t smem_ap[];
@@ -193,9 +196,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   volatile uint32_t* tmem_slot_gen = reinterpret_cast<volatile uint32_t*>(smem_ap + C::OFF_BAR + 8 * C::NBAR);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m_blk = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  // the last CTAs may take one query tile of a block instead of QT (see the launch)
+  const int part = static_cast<int>(blockIdx.x) - p.whole, blk = part < 0 ? static_cast<int>(blockIdx.x) : p.whole + part / QT;
+  const int m_blk = blk % p.m_blks, h = blk / p.m_blks % p.heads, b = blk / p.m_blks / p.heads;
+  const int tile0 = m_blk * QT + (part < 0 ? 0 : part % QT), nqt = part < 0 ? QT : 1;  // query tiles of this CTA
+  if (tile0 * BM >= p.rows) return;
   // profiling stamps (tiles 0..31 of CTA (0,0,0)): role 0 = MMA issuer, 1 = softmax warp 2, 2 = softmax warp 6; 8 events per tile
-  const bool tr_on = p.trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && lane == 0;
+  const bool tr_on = p.trace != nullptr && blockIdx.x == 0 && lane == 0;
   auto stamp = [&](int role, int j, int ev) {
     if (tr_on && j < 32) p.trace[(role * 32 + j) * 8 + ev] = clock64();
   };
@@ -232,10 +239,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   if (warp == 0) {
     // ============================== TMA producer ==============================
     if (lane == 0) {
-      mbar_expect_tx(q_full, QT * C::Q_BYTES);
+      mbar_expect_tx(q_full, nqt * C::Q_BYTES);
 #pragma unroll
       for (int qt = 0; qt < QT; ++qt) {
-        const int t0 = ((m_blk * QT + qt) * BM) / p.group;  // first token of this row tile (128 % group == 0)
+        if (qt >= nqt) break;
+        const int t0 = ((tile0 + qt) * BM) / p.group;  // first token of this row tile (128 % group == 0)
 #pragma unroll
         for (int kb = 0; kb < NKB; ++kb)
           tma_load_5d(sbase + qt * C::Q_BYTES + kb * C::Q_BOX, &tmQ, q_full, kb * 64, 0, t0, h, b);
@@ -266,6 +274,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       const uint32_t kaddr = sbase + C::OFF_K + ks * C::KV_BYTES;
 #pragma unroll
       for (int qt = 0; qt < QT; ++qt) {
+        if (qt >= nqt) break;
         mbar_wait(s_empty(qt, sb), ((j >> 1) & 1) ^ 1);
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + C::COL_S + (qt * 2 + sb) * BN;
@@ -277,7 +286,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             umma_f16(d_tmem, adesc, bdesc, IDESC_S, k > 0 ? 1u : 0u);
           }
           umma_commit(s_full(qt, sb));
-          if (qt == QT - 1) umma_commit(k_empty(ks));
+          if (qt == nqt - 1) umma_commit(k_empty(ks));
         }
         __syncwarp();
       }
@@ -312,6 +321,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       stamp(0, j, 3);
 #pragma unroll
       for (int qt = 0; qt < QT; ++qt) {
+        if (qt >= nqt) break;
         mbar_wait(p_full(qt, pb), (j >> 1) & 1);
         if (qt == 0) stamp(0, j, 4);
         tc_fence_after();
@@ -325,13 +335,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             umma_f16(d_tmem, adesc, bdesc, IDESC_O, (j > 0 || k > 0) ? 1u : 0u);
           }
           umma_commit(o_done(qt, pb));
-          if (qt == QT - 1) umma_commit(v_empty(vs));
+          if (qt == nqt - 1) umma_commit(v_empty(vs));
         }
         __syncwarp();
       }
       stamp(0, j, 5);
     }
-  } else {
+  } else if (QT == 1 || ((warp - 2) >> 2) < nqt) {
     // ============================== softmax / epilogue ========================
     constexpr int HB = BN / SW;         // score columns of a tile owned by one thread
     const int q = warp & 3;             // TMEM lane quadrant this warp may access
@@ -340,7 +350,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     const int qt = QT == 2 ? grp : 0;
     const int r = q * 32 + lane;        // row inside the tile == TMEM lane
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
-    const int row = (m_blk * QT + qt) * BM + r;
+    const int row = (tile0 + qt) * BM + r;
     const uint32_t col_s = C::COL_S + qt * 2 * BN, col_o = C::COL_O + qt * C::O_STRIDE;
     float* xch = reinterpret_cast<float*>(smem_ap + C::OFF_X);  // [2][2][128]
     auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory"); };  // the two warps of a quadrant
@@ -394,8 +404,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 #pragma unroll
         for (int i = 0; i < 8; ++i) m8[i] = s[i];
 #pragma unroll
-        for (int i = 8; i < HB; ++i) m8[i & 7] = fmaxf(m8[i & 7], s[i]);
-        mx = fmaxf(fmaxf(fmaxf(m8[0], m8[1]), fmaxf(m8[2], m8[3])), fmaxf(fmaxf(m8[4], m8[5]), fmaxf(m8[6], m8[7])));
+        for (int i = 8; i < HB - 8; i += 16)
+#pragma unroll
+          for (int k = 0; k < 8; ++k) m8[k] = max3(m8[k], s[i + k], s[i + 8 + k]);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) m8[k] = fmaxf(m8[k], s[HB - 8 + k]);
+        mx = max3(max3(m8[0], m8[1], m8[2]), max3(m8[3], m8[4], m8[5]), fmaxf(m8[6], m8[7]));
       }
       mx *= p.sl2;
       if constexpr (SW == 2) {  // row maximum over both halves (buffer sb is rewritten two tiles later, one barrier apart)
@@ -409,32 +423,34 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       const float m_new = need ? mx : m_used;
       const float alpha = need ? exp2f(m_used - m_new) : 1.0f;  // first tile: m_used = -inf -> 0 (O is overwritten)
       m_used = m_new;
-      float sum = 0.f;
+      uint64_t sum = 0;
       const uint32_t pdst = p_row + sb * C::P_BYTES;
       // Three separate passes over the thread's HB scores (exponent arguments, then the MUFU exponentials back to back, then
       // pack + store): interleaved chunk by chunk, each exp2 -> pack -> store chain exposed the ~40 clk MUFU latency with two
       // or three exponentials in flight (900 clk per 64 scores for a warp ALONE on its sub-partition's MUFU pipe, which
       // could do them in 512).
+      const uint64_t sl2 = pair_of(p.sl2, p.sl2), off = pair_of(-m_new, -m_new);
+      uint64_t x[HB / 2];
 #pragma unroll
-      for (int i = 0; i < HB; ++i) s[i] = fmaf(s[i], p.sl2, -m_new);
+      for (int i = 0; i < HB / 2; ++i) x[i] = fma_pair(pair_of(s[2 * i], s[2 * i + 1]), sl2, off);
       // (an earlier variant with floorf / float->int range reduction was 40 % SLOWER: those conversions run on the XU pipe
       //  as well, so it added XU work instead of removing it)
 #pragma unroll
-      for (int i = 0; i < HB; ++i) s[i] = (POLY8 > 0 && (i & 7) >= 8 - POLY8) ? exp2_fma(s[i]) : exp2_mufu(s[i]);
+      for (int i = 0; i < HB / 2; ++i) x[i] = (i & 7) >= 8 - POLY16 / 2 ? exp2_fma_pair(x[i]) : pair_of(exp2_mufu(lo_f32(x[i])), exp2_mufu(hi_f32(x[i])));
 #pragma unroll
       for (int cc = 0; cc < HB / 8; ++cc) {  // 16-byte chunks of 8 keys
         uint32_t pk[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float p0 = s[cc * 8 + 2 * e], p1 = s[cc * 8 + 2 * e + 1];
-          if constexpr (!TCSUM) sum += p0 + p1;
-          pk[e] = pack_bf16(p0, p1);
+          const uint64_t pp = x[cc * 4 + e];
+          if constexpr (!TCSUM) sum = add_pair(sum, pp);
+          pk[e] = pack_bf16(lo_f32(pp), hi_f32(pp));
         }
         const int c = half * (HB / 8) + cc;  // chunk index inside the whole tile row
         const uint32_t addr = pdst + (c >> 3) * C::P_BOX + (((c & 7) ^ (r & 7)) << 4);
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
       }
-      l_run = l_run * alpha + sum;  // (SW == 2: the sum over this thread's columns only; the halves are added at the end)
+      l_run = l_run * alpha + (lo_f32(sum) + hi_f32(sum));  // (SW == 2: the sum over this thread's columns only; the halves are added at the end)
       if (trole < 3) stamp(trole, j, 4);
       if (j > 0) {
         if (__any_sync(0xffffffffu, need)) {  // (both warps of a quadrant see the same maxima, hence the same decision)
@@ -537,8 +553,18 @@ static int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
     }
     configured[dev] = true;
   }
-  dim3 grid((p.rows + C::BM * QT - 1) / (C::BM * QT), H, B);
-  return launch_kernel(attn_prefill_tc_kernel<DH, SW, QT>, grid, dim3(96 + 128 * SW * QT), C::SMEM, st, tq, tk, tv, p) == cudaSuccess ? PG_OK : PG_ERR_CUDA;
+  // One CTA per SM.  Where the last round has at most half as many blocks as SMs, its two query tiles go to two CTAs: a tile alone on an SM takes a little over half of what two
+  // together take (64 blocks of 1024 keys 25 -> 19 us, 192 47 -> 40, 512 of 4096 keys 295 -> 258, the packed exponentials of 3 % included).
+  Params pp = p;
+  pp.m_blks = (p.rows + C::BM * QT - 1) / (C::BM * QT);
+  pp.heads = H;
+  const long long blks = static_cast<long long>(pp.m_blks) * H * B;
+  if (blks * QT > 0x7fffffff) return PG_ERR_ARG;
+  const int rest = static_cast<int>(blks % num_sms());
+  const bool split = QT == 2 && 2 * rest <= num_sms();
+  pp.whole = static_cast<int>(split ? blks - rest : blks);
+  const unsigned grid = static_cast<unsigned>(split ? blks + rest : blks);
+  return launch_kernel(attn_prefill_tc_kernel<DH, SW, QT>, grid, dim3(96 + 128 * SW * QT), C::SMEM, st, tq, tk, tv, pp) == cudaSuccess ? PG_OK : PG_ERR_CUDA;
 }
 
 }  // namespace ap

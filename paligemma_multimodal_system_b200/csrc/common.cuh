@@ -58,6 +58,30 @@ PG_DEVINL float gelu_tanh_fast(float x) {
   return 0.5f * x * (1.0f + t);
 }
 
+// Two fp32 values side by side: one instruction for two sums or products, each rounded as by itself.  The pipe takes as long as for two (measured 2.0 clocks a warp for 1.0), what
+// is saved are issue slots; a maximum of three likewise.
+PG_DEVINL uint64_t pair_of(uint32_t lo, uint32_t hi) { return static_cast<uint64_t>(hi) << 32 | lo; }
+PG_DEVINL uint64_t pair_of(float lo, float hi) { return pair_of(__float_as_uint(lo), __float_as_uint(hi)); }
+PG_DEVINL uint32_t lo_of(uint64_t p) { return static_cast<uint32_t>(p); }
+PG_DEVINL uint32_t hi_of(uint64_t p) { return static_cast<uint32_t>(p >> 32); }
+PG_DEVINL float lo_f32(uint64_t p) { return __uint_as_float(lo_of(p)); }
+PG_DEVINL float hi_f32(uint64_t p) { return __uint_as_float(hi_of(p)); }
+PG_DEVINL uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+PG_DEVINL uint64_t add_pair(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+PG_DEVINL float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
 PG_DEVINL uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);

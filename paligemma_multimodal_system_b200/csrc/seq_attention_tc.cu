@@ -81,21 +81,6 @@ PG_DEVINL float tanh32(float x) {
   const float big = copysignf(1.0f - __fdividef(2.0f, ex2(ax * 2.885390082f) + 1.0f), x);
   return ax < 0.1f ? small : big;
 }
-// two fp32 values side by side: one instruction for two sums or products, rounded as two (the softmax warps are short of issue slots)
-PG_DEVINL uint64_t pair_of(uint32_t lo, uint32_t hi) { return static_cast<uint64_t>(hi) << 32 | lo; }
-PG_DEVINL uint64_t pair_of(float lo, float hi) { return pair_of(__float_as_uint(lo), __float_as_uint(hi)); }
-PG_DEVINL uint32_t lo_of(uint64_t p) { return static_cast<uint32_t>(p); }
-PG_DEVINL uint32_t hi_of(uint64_t p) { return static_cast<uint32_t>(p >> 32); }
-PG_DEVINL uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-PG_DEVINL uint64_t add_pair(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
 PG_DEVINL void split3(uint64_t p, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
   constexpr uint64_t minus = 0xbf800000bf800000ull;
   hi = __byte_perm(lo_of(p), hi_of(p), 0x7632);
@@ -410,8 +395,12 @@ __global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __gri
 #pragma unroll
         for (int i = 0; i < 8; ++i) m8[i] = s[i];
 #pragma unroll
-        for (int i = 8; i < 64; ++i) m8[i & 7] = fmaxf(m8[i & 7], s[i]);
-        mx = fmaxf(fmaxf(fmaxf(m8[0], m8[1]), fmaxf(m8[2], m8[3])), fmaxf(fmaxf(m8[4], m8[5]), fmaxf(m8[6], m8[7]))) * unit;
+        for (int i = 8; i < 56; i += 16)
+#pragma unroll
+          for (int k = 0; k < 8; ++k) m8[k] = max3(m8[k], s[i + k], s[i + 8 + k]);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) m8[k] = fmaxf(m8[k], s[56 + k]);
+        mx = max3(max3(m8[0], m8[1], m8[2]), max3(m8[3], m8[4], m8[5]), fmaxf(m8[6], m8[7])) * unit;
       }
       const bool need = mx > m + 8.0f;  // (from -inf: every finite maximum)
       const float mn = need ? mx : m;
@@ -440,7 +429,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __gri
           for (int i = 0; i < 8; ++i) {
             const int at = (16 * c + 2 * i) & 63;
             const uint64_t x = fma_pair(pair_of(s[at], s[at + 1]), unit2, off2);
-            pp[c & 1][i] = pair_of(ex2(__uint_as_float(lo_of(x))), ex2(__uint_as_float(hi_of(x))));
+            pp[c & 1][i] = pair_of(ex2(lo_f32(x)), ex2(hi_f32(x)));
           }
         }
         if (c > 0) {
@@ -457,7 +446,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __gri
         }
       }
       s2[0] = add_pair(s2[0], s2[1]);
-      l = l * alpha + (__uint_as_float(lo_of(s2[0])) + __uint_as_float(hi_of(s2[0])));
+      l = l * alpha + (lo_f32(s2[0]) + hi_f32(s2[0]));
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();

@@ -225,13 +225,6 @@ __device__ __forceinline__ void pack(const float* v, uint4& u) {
   u = make_uint4(pg::pack_bf16(v[0], v[1]), pg::pack_bf16(v[2], v[3]), pg::pack_bf16(v[4], v[5]), pg::pack_bf16(v[6], v[7]));
 }
 
-// a pair of fp32 products and sums by one instruction, rounded as two fmaf
-__device__ __forceinline__ uint64_t pair2(float a, float b) { return (uint64_t)__float_as_uint(b) << 32 | __float_as_uint(a); }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
 // silu of a value that is rounded to bf16 at once: the hardware exponential and reciprocal are far below its rounding
 __device__ __forceinline__ float silu_bf16(float a) {
   float e, r;
@@ -286,7 +279,7 @@ __global__ void __launch_bounds__(128, V == 4 && TAPS == 4 ? 6 : 1) short_conv_v
   };
   auto pairs = [](const float* v, uint64_t* p) {
 #pragma unroll
-    for (int i = 0; i < V / 2; ++i) p[i] = pair2(v[2 * i], v[2 * i + 1]);
+    for (int i = 0; i < V / 2; ++i) p[i] = pg::pair_of(v[2 * i], v[2 * i + 1]);
   };
   auto ldp = [&](const float* p, uint64_t* to) {
     float v[V];
@@ -345,9 +338,9 @@ __global__ void __launch_bounds__(128, V == 4 && TAPS == 4 ? 6 : 1) short_conv_v
       np += ldx;
 #pragma unroll
       for (int v = 0; v < V / 2; ++v) {
-        uint64_t a = fma2(wt[TAPS - 1][v], cp[v], bs[v]);
+        uint64_t a = pg::fma_pair(wt[TAPS - 1][v], cp[v], bs[v]);
 #pragma unroll
-        for (int j = 0; j < TAPS - 1; ++j) a = fma2(wt[j][v], hist[j][v], a);
+        for (int j = 0; j < TAPS - 1; ++j) a = pg::fma_pair(wt[j][v], hist[j][v], a);
 #pragma unroll
         for (int j = 0; j < TAPS - 2; ++j) hist[j][v] = hist[j + 1][v];
         hist[TAPS - 2][v] = cp[v];
