@@ -21,6 +21,9 @@
 //               ones column in the padded V tile).  dh = 256: QT = 1, four softmax warps (SW = 1).  SW = 2 (eight warps, two
 //               column halves of one row exchanging their maxima through shared memory) remains for single-tile problems.
 // S_{j+1} is computed while the softmax of tile j runs, and P_j V_j runs while the softmax of tile j+1 runs.
+// A CTA takes blocks in turn, one CTA per SM: rings, S buffers and their barriers run on from block to block, so the next block's queries, keys and first scores are there
+// while the softmax warps still write the last one's rows (a CTA per block spent 7 us of each on its start and end: 64 x 256 keys 74 us, 57 now; 8 x 1024 83, 78 now; a single
+// round of 17 blocks of 256-wide heads 13.3, 13.9 now).
 // Zero padding comes from TMA: columns beyond dh (72 -> 80) and key / query rows beyond the sequence are out-of-bounds
 // box elements and arrive as zeros; padded keys are masked to -inf before the softmax.
 // Timelines of one CTA: clock64 stamps through Params::trace.
@@ -47,7 +50,7 @@ struct Params {
   long long* trace;     // optional clock64 stamps of CTA (0,0,0): [role][tile][event]
   int trigger;          // the next kernel may come (weights_follow)
   int m_blks, heads;    // blocks of QT query tiles of a (head, batch); heads
-  int whole;            // CTAs with QT query tiles; those behind them take one tile of a block each
+  int whole, items;     // blocks of QT query tiles; with those behind them, one tile of a block each
 };
 
 template <int DH, int QT>
@@ -67,14 +70,14 @@ struct Cfg {
   static constexpr int OFF_V = OFF_K + KST * KV_BYTES;
   static constexpr int OFF_P = OFF_V + VST * KV_BYTES;  // [QT][2 buffers][P_BYTES]
   static constexpr int OFF_BAR = OFF_P + QT * 2 * P_BYTES;
-  static constexpr int OFF_X = OFF_BAR + 256;          // float [2 S buffers][2 halves][128 rows]: tile maxima / row sums (SW = 2)
+  static constexpr int OFF_X = OFF_BAR + 320;          // float [2 S buffers][2 halves][128 rows]: tile maxima / row sums (SW = 2)
   static constexpr int SMEM = OFF_X + 2048;
   static constexpr int TMEM_COLS = 512;
   static constexpr int COL_S = 0, COL_O = 2 * QT * BN;  // S: [QT][2 buffers][BN] columns, then O: [QT] accumulators
   static constexpr int O_STRIDE = QT == 2 ? 128 : DHP;  // (two accumulators: each starts on a 128-column boundary)
-  static constexpr int NBAR = 1 + 2 * KST + 2 * VST + 8 * QT;
+  static constexpr int NBAR = 2 + 2 * KST + 2 * VST + 9 * QT;
   static_assert(2 * QT * BN + (QT - 1) * O_STRIDE + DHP <= 512, "TMEM budget");
-  static_assert(8 * NBAR + 8 <= 256, "barrier area");
+  static_assert(8 * NBAR + 8 <= 320, "barrier area");
   static_assert(SMEM <= 232448, "shared memory budget");
 };
 
@@ -192,15 +195,28 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   auto s_empty = [&](int qt, int s) { return bar0 + 8u * (S0 + 2 * QT + qt * 2 + s); };
   auto p_full = [&](int qt, int s) { return bar0 + 8u * (S0 + 4 * QT + qt * 2 + s); };
   auto o_done = [&](int qt, int s) { return bar0 + 8u * (S0 + 6 * QT + qt * 2 + s); };  // P_j V_j complete: barrier j % 2
+  const uint32_t q_empty = bar0 + 8u * (S0 + 8 * QT);                       // every S of the block has been multiplied
+  auto o_empty = [&](int qt) { return bar0 + 8u * (S0 + 8 * QT + 1 + qt); };  // the block's O has been read
   const uint32_t tmem_slot = bar0 + 8u * C::NBAR;
   volatile uint32_t* tmem_slot_gen = reinterpret_cast<volatile uint32_t*>(smem_ap + C::OFF_BAR + 8 * C::NBAR);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // the last CTAs may take one query tile of a block instead of QT (see the launch)
-  const int part = static_cast<int>(blockIdx.x) - p.whole, blk = part < 0 ? static_cast<int>(blockIdx.x) : p.whole + part / QT;
-  const int m_blk = blk % p.m_blks, h = blk / p.m_blks % p.heads, b = blk / p.m_blks / p.heads;
-  const int tile0 = m_blk * QT + (part < 0 ? 0 : part % QT), nqt = part < 0 ? QT : 1;  // query tiles of this CTA
-  if (tile0 * BM >= p.rows) return;
+  // block `idx` of the launch; the last ones may be one query tile of a block instead of QT (see the launch): a CTA's blocks of two tiles come before its single ones
+  struct Item {
+    int tile0, nqt, h, b;  // first query tile, query tiles (0: none), head, problem
+  };
+  auto item = [&](int idx) {
+    Item it;
+    const int part = idx - p.whole, blk = part < 0 ? idx : p.whole + part / QT, m_blk = blk % p.m_blks;
+    it.h = blk / p.m_blks % p.heads;
+    it.b = blk / p.m_blks / p.heads;
+    it.tile0 = m_blk * QT + (part < 0 ? 0 : part % QT);
+    it.nqt = it.tile0 * BM >= p.rows ? 0 : part < 0 ? QT : 1;
+    return it;
+  };
+  // ragged batches: keys [key_lens[b], keys) of problem b exist in memory (padding tokens, finite values) but weigh nothing
+  // (The issuing warps and the softmax take them from lane 0: tile counts then stay uniform over the warp for the compiler, and with them descriptors and addresses.)
+  auto keys = [&](const Item& it) { return p.key_lens ? max(1, min(p.keys, __ldg(p.key_lens + it.b))) : p.keys; };
   // profiling stamps (tiles 0..31 of CTA (0,0,0)): role 0 = MMA issuer, 1 = softmax warp 2, 2 = softmax warp 6; 8 events per tile
   const bool tr_on = p.trace != nullptr && blockIdx.x == 0 && lane == 0;
   auto stamp = [&](int role, int j, int ev) {
@@ -211,6 +227,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmV);
     mbar_init(q_full, 1);
+    mbar_init(q_empty, 1);
     for (int s = 0; s < KST; ++s) { mbar_init(k_full(s), 1); mbar_init(k_empty(s), 1); }
     for (int s = 0; s < VST; ++s) { mbar_init(v_full(s), 1); mbar_init(v_empty(s), 1); }
     for (int qt = 0; qt < QT; ++qt) {
@@ -218,6 +235,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         mbar_init(s_full(qt, s), 1); mbar_init(s_empty(qt, s), 4 * SW);
         mbar_init(p_full(qt, s), 4 * SW);
       }
+      mbar_init(o_empty(qt), 4 * SW);
       mbar_init(o_done(qt, 0), 1);
       mbar_init(o_done(qt, 1), 1);
     }
@@ -227,39 +245,44 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     tmem_alloc(tmem_slot, C::TMEM_COLS);
     tmem_relinquish();
   }
+  const Item item0 = item(blockIdx.x);  // (its divisions pass while barriers and tensor memory are set up)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_gen;
   griddep_begin_if(p.trigger);  // (tensor memory is held by now: a product behind this kernel cannot take it first)
-  // ragged batches: keys [key_lens[b], keys) of problem b exist in memory (padding tokens, finite values) but weigh nothing
-  const int n_keys = p.key_lens ? max(1, min(p.keys, __ldg(p.key_lens + b))) : p.keys;
-  const int n_tiles = (n_keys + BN - 1) / BN;
-
   if (warp == 0) {
     // ============================== TMA producer ==============================
     if (lane == 0) {
-      mbar_expect_tx(q_full, nqt * C::Q_BYTES);
+      int jt = 0, n = 0;  // key tiles and blocks so far
+      for (int idx = blockIdx.x; idx < p.items; idx += gridDim.x) {
+        const Item it = idx == static_cast<int>(blockIdx.x) ? item0 : item(idx);
+        if (it.nqt == 0) continue;
+        const int n_keys = keys(it), n_tiles = (n_keys + BN - 1) / BN;
+        mbar_wait(q_empty, (n & 1) ^ 1);
+        mbar_expect_tx(q_full, it.nqt * C::Q_BYTES);
 #pragma unroll
-      for (int qt = 0; qt < QT; ++qt) {
-        if (qt >= nqt) break;
-        const int t0 = ((tile0 + qt) * BM) / p.group;  // first token of this row tile (128 % group == 0)
+        for (int qt = 0; qt < QT; ++qt) {
+          if (qt >= it.nqt) break;
+          const int t0 = ((it.tile0 + qt) * BM) / p.group;  // first token of this row tile (128 % group == 0)
 #pragma unroll
-        for (int kb = 0; kb < NKB; ++kb)
-          tma_load_5d(sbase + qt * C::Q_BYTES + kb * C::Q_BOX, &tmQ, q_full, kb * 64, 0, t0, h, b);
-      }
-      for (int j = 0; j < n_tiles; ++j) {
-        const int ks = j % KST, vs = j % VST;
-        mbar_wait(k_empty(ks), ((j / KST) & 1) ^ 1);
-        mbar_expect_tx(k_full(ks), C::KV_BYTES);
+          for (int kb = 0; kb < NKB; ++kb)
+            tma_load_5d(sbase + qt * C::Q_BYTES + kb * C::Q_BOX, &tmQ, q_full, kb * 64, 0, t0, it.h, it.b);
+        }
+        for (int j = 0; j < n_tiles; ++j, ++jt) {
+          const int ks = jt % KST, vs = jt % VST;
+          mbar_wait(k_empty(ks), ((jt / KST) & 1) ^ 1);
+          mbar_expect_tx(k_full(ks), C::KV_BYTES);
 #pragma unroll
-        for (int kb = 0; kb < NKB; ++kb)
-          tma_load_4d(sbase + C::OFF_K + ks * C::KV_BYTES + kb * C::KV_BOX, &tmK, k_full(ks), kb * 64, j * BN, h, b);
-        mbar_wait(v_empty(vs), ((j / VST) & 1) ^ 1);
-        mbar_expect_tx(v_full(vs), C::KV_BYTES);
+          for (int kb = 0; kb < NKB; ++kb)
+            tma_load_4d(sbase + C::OFF_K + ks * C::KV_BYTES + kb * C::KV_BOX, &tmK, k_full(ks), kb * 64, j * BN, it.h, it.b);
+          mbar_wait(v_empty(vs), ((jt / VST) & 1) ^ 1);
+          mbar_expect_tx(v_full(vs), C::KV_BYTES);
 #pragma unroll
-        for (int kb = 0; kb < NKB; ++kb)
-          tma_load_4d(sbase + C::OFF_V + vs * C::KV_BYTES + kb * C::KV_BOX, &tmV, v_full(vs), kb * 64, j * BN, h, b);
+          for (int kb = 0; kb < NKB; ++kb)
+            tma_load_4d(sbase + C::OFF_V + vs * C::KV_BYTES + kb * C::KV_BOX, &tmV, v_full(vs), kb * 64, j * BN, it.h, it.b);
+        }
+        ++n;
       }
     }
     __syncwarp();
@@ -268,7 +291,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     // All 32 lanes run the loop and ONE elected lane issues: with uniform control flow the compiler keeps the descriptors
     // and TMEM addresses uniform over the warp.  (Under `if (lane == 0)` every tcgen05.mma took ~115 clk to issue: the issuer, not the
     // softmax or the tensor pipe, paced the kernel.)
-    auto issue_s = [&](int j) {  // S_j = Q K_j^T of every query tile into its S buffer j % 2
+    auto issue_s = [&](int j, int nqt, bool last) {  // S_j = Q K_j^T of every query tile into its S buffer j % 2 (j: tiles of all blocks so far)
       const int ks = j % KST, sb = j & 1;
       mbar_wait(k_full(ks), (j / KST) & 1);
       const uint32_t kaddr = sbase + C::OFF_K + ks * C::KV_BYTES;
@@ -287,6 +310,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
           }
           umma_commit(s_full(qt, sb));
           if (qt == nqt - 1) umma_commit(k_empty(ks));
+          if (qt == nqt - 1 && last) umma_commit(q_empty);
         }
         __syncwarp();
       }
@@ -294,54 +318,70 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     // The S issuer (this warp) and the P V issuer (the last warp) are separate instruction streams: a tcgen05.mma blocks its
     // issuing thread while the tensor pipe's queue is full, so one stream serialised S_{j+1}, its barrier round trips, the
     // ones column and P_j V_j into 2300 clk per 128-key tile -- longer than the softmax it was supposed to hide behind.
-    mbar_wait(q_full, 0);
-    for (int j = 0; j < n_tiles; ++j) {
-      stamp(0, j, 0);
-      issue_s(j);
-      stamp(0, j, 1);
+    int jt = 0, n = 0;
+    for (int idx = blockIdx.x; idx < p.items; idx += gridDim.x) {
+      const Item it = idx == static_cast<int>(blockIdx.x) ? item0 : item(idx);
+      if (it.nqt == 0) continue;
+      const int n_keys = __shfl_sync(0xffffffffu, keys(it), 0), n_tiles = (n_keys + BN - 1) / BN;
+      mbar_wait(q_full, n & 1);
+      for (int j = 0; j < n_tiles; ++j, ++jt) {
+        stamp(0, jt, 0);
+        issue_s(jt, it.nqt, j == n_tiles - 1);
+        stamp(0, jt, 1);
+      }
+      ++n;
     }
   } else if (warp == 2 + 4 * SW * QT) {
     // ============================== P V issuer ================================
-    for (int j = 0; j < n_tiles; ++j) {
-      const int vs = j % VST, pb = j & 1;
-      mbar_wait(v_full(vs), (j / VST) & 1);
-      stamp(0, j, 2);
-      const uint32_t vaddr = sbase + C::OFF_V + vs * C::KV_BYTES;
-      if constexpr (TCSUM) {
-        // every lane plants its share of the ones column into the V tile that just landed:
-        // column DH (= 72) lives in box DH / 64, 16-byte chunk (DH % 64) / 8, element DH % 8 of key row r (128B swizzle)
-        constexpr uint32_t BOX = DH / 64, CH = (DH % 64) / 8, EL = DH % 8;
-        for (int r = lane; r < BN; r += 32) {
-          const uint32_t addr = vaddr + BOX * C::KV_BOX + r * 128 + ((CH ^ (r & 7)) << 4) + EL * 2;
-          asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"(static_cast<unsigned short>(0x3F80)) : "memory");
-        }
-        fence_proxy_async_smem();
-        __syncwarp();
-      }
-      stamp(0, j, 3);
-#pragma unroll
-      for (int qt = 0; qt < QT; ++qt) {
-        if (qt >= nqt) break;
-        mbar_wait(p_full(qt, pb), (j >> 1) & 1);
-        if (qt == 0) stamp(0, j, 4);
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + C::COL_O + qt * C::O_STRIDE;
-        const uint32_t paddr = sbase + C::OFF_P + (qt * 2 + pb) * C::P_BYTES;
-        if (elect_one()) {
-#pragma unroll
-          for (int k = 0; k < BN / 16; ++k) {
-            const uint64_t adesc = make_sdesc_k_sw128(paddr + (k >> 2) * C::P_BOX) + 2 * (k & 3);
-            const uint64_t bdesc = make_sdesc_mn_sw128(vaddr + k * 2048, C::KV_BOX);  // 16 keys = two 8-row groups
-            umma_f16(d_tmem, adesc, bdesc, IDESC_O, (j > 0 || k > 0) ? 1u : 0u);
+    int jt = 0, n = 0;
+    for (int idx = blockIdx.x; idx < p.items; idx += gridDim.x) {
+      const Item it = idx == static_cast<int>(blockIdx.x) ? item0 : item(idx);
+      if (it.nqt == 0) continue;
+      const int n_keys = __shfl_sync(0xffffffffu, keys(it), 0), n_tiles = (n_keys + BN - 1) / BN;
+      for (int first = jt; jt < first + n_tiles; ++jt) {
+        const int j = jt;
+        const int vs = j % VST, pb = j & 1;
+        mbar_wait(v_full(vs), (j / VST) & 1);
+        stamp(0, j, 2);
+        const uint32_t vaddr = sbase + C::OFF_V + vs * C::KV_BYTES;
+        if constexpr (TCSUM) {
+          // every lane plants its share of the ones column into the V tile that just landed:
+          // column DH (= 72) lives in box DH / 64, 16-byte chunk (DH % 64) / 8, element DH % 8 of key row r (128B swizzle)
+          constexpr uint32_t BOX = DH / 64, CH = (DH % 64) / 8, EL = DH % 8;
+          for (int r = lane; r < BN; r += 32) {
+            const uint32_t addr = vaddr + BOX * C::KV_BOX + r * 128 + ((CH ^ (r & 7)) << 4) + EL * 2;
+            asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"(static_cast<unsigned short>(0x3F80)) : "memory");
           }
-          umma_commit(o_done(qt, pb));
-          if (qt == nqt - 1) umma_commit(v_empty(vs));
+          fence_proxy_async_smem();
+          __syncwarp();
         }
-        __syncwarp();
+        stamp(0, j, 3);
+#pragma unroll
+        for (int qt = 0; qt < QT; ++qt) {
+          if (qt >= it.nqt) break;
+          if (j == first) mbar_wait(o_empty(qt), (n & 1) ^ 1);  // the softmax has read the accumulator of the block before
+          mbar_wait(p_full(qt, pb), (j >> 1) & 1);
+          if (qt == 0) stamp(0, j, 4);
+          tc_fence_after();
+          const uint32_t d_tmem = tmem_base + C::COL_O + qt * C::O_STRIDE;
+          const uint32_t paddr = sbase + C::OFF_P + (qt * 2 + pb) * C::P_BYTES;
+          if (elect_one()) {
+#pragma unroll
+            for (int k = 0; k < BN / 16; ++k) {
+              const uint64_t adesc = make_sdesc_k_sw128(paddr + (k >> 2) * C::P_BOX) + 2 * (k & 3);
+              const uint64_t bdesc = make_sdesc_mn_sw128(vaddr + k * 2048, C::KV_BOX);  // 16 keys = two 8-row groups
+              umma_f16(d_tmem, adesc, bdesc, IDESC_O, (j > first || k > 0) ? 1u : 0u);
+            }
+            umma_commit(o_done(qt, pb));
+            if (qt == it.nqt - 1) umma_commit(v_empty(vs));
+          }
+          __syncwarp();
+        }
+        stamp(0, j, 5);
       }
-      stamp(0, j, 5);
+      ++n;
     }
-  } else if (QT == 1 || ((warp - 2) >> 2) < nqt) {
+  } else {
     // ============================== softmax / epilogue ========================
     constexpr int HB = BN / SW;         // score columns of a tile owned by one thread
     const int q = warp & 3;             // TMEM lane quadrant this warp may access
@@ -350,162 +390,183 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     const int qt = QT == 2 ? grp : 0;
     const int r = q * 32 + lane;        // row inside the tile == TMEM lane
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
-    const int row = (tile0 + qt) * BM + r;
     const uint32_t col_s = C::COL_S + qt * 2 * BN, col_o = C::COL_O + qt * C::O_STRIDE;
     float* xch = reinterpret_cast<float*>(smem_ap + C::OFF_X);  // [2][2][128]
     auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory"); };  // the two warps of a quadrant
-    float m_used = -INFINITY, l_run = 0.f;
     const uint32_t p_row = sbase + C::OFF_P + qt * 2 * C::P_BYTES + r * 128;
-    for (int j = 0; j < n_tiles; ++j) {
-      const int sb = j & 1;
-      const int trole = warp == 2 ? 1 : (warp == 6 ? 2 : 3);
-      if (trole < 3) stamp(trole, j, 0);
-      // S_j is ready AND P_{j-2} V_{j-2} has completed (its P buffer is the one this tile writes): both barrier round trips
-      // (~150 clk each even when the phase completed long ago) are in flight together.  P_{j-1} V_{j-1}, which the old loop
-      // waited for at the end of every tile, only matters to the rare O rescale below.
-      if (j >= 2) mbar_wait2(s_full(qt, sb), (j >> 1) & 1, o_done(qt, sb), ((j - 2) >> 1) & 1);
-      else mbar_wait(s_full(qt, sb), (j >> 1) & 1);
-      if constexpr (QT == 2) {
-        if (j == 0 && qt == 1 && p.stagger > 0) {
-          const long long t0 = clock64();
-          while (clock64() - t0 < p.stagger) {}
-        }
-      }
-      if (trole < 3) stamp(trole, j, 1);
-      tc_fence_after();
-      float s[HB];
-      {
-        // every 16-column slice is requested before the one wait: the slices' TMEM round trips overlap instead of queueing
-        // (ncu at 4096 keys: tensor pipe 28 %, XU 45 %, issue 33 % -- nothing saturated, the softmax warps sit in latencies)
-        uint32_t v[HB / 16][16];
-#pragma unroll
-        for (int c0 = 0; c0 < HB; c0 += 16) tmem_ld16(lane_addr + col_s + sb * BN + half * HB + c0, v[c0 / 16]);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < HB; ++i) s[i] = __uint_as_float(v[i / 16][i % 16]);  // raw scores: the scale rides on the FFMA below
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (trole < 3) stamp(trole, j, 2);
-      if (lane == 0) mbar_arrive(s_empty(qt, sb));  // the S buffer may be overwritten by S_{j+2}
-      // The softmax warps are bound by instruction issue (ncu: ~9 instructions per score, XU pipe 39 %, tensor pipe 24 %), so
-      // the per-score work is kept to FMNMX, FFMA, MUFU, FADD and half an F2FP: keys are only masked in the one tile that
-      // has padding, and the softmax scale is folded into the exponent's FFMA (scale > 0: max commutes with it).
-      const int nvalid = n_keys - j * BN - half * HB;  // columns of this thread that are real keys
-      if (nvalid < HB) {
-#pragma unroll
-        for (int i = 0; i < HB; ++i)
-          if (i >= nvalid) s[i] = -INFINITY;
-      }
-      float mx;
-      {
-        // eight independent running maxima, then a tree: a single FMNMX chain over HB scores is HB dependent instructions
-        float m8[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) m8[i] = s[i];
-#pragma unroll
-        for (int i = 8; i < HB - 8; i += 16)
-#pragma unroll
-          for (int k = 0; k < 8; ++k) m8[k] = max3(m8[k], s[i + k], s[i + 8 + k]);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) m8[k] = fmaxf(m8[k], s[HB - 8 + k]);
-        mx = max3(max3(m8[0], m8[1], m8[2]), max3(m8[3], m8[4], m8[5]), fmaxf(m8[6], m8[7]));
-      }
-      mx *= p.sl2;
-      if constexpr (SW == 2) {  // row maximum over both halves (buffer sb is rewritten two tiles later, one barrier apart)
-        xch[(sb * 2 + half) * 128 + r] = mx;
-        pair_sync();
-        mx = fmaxf(mx, xch[(sb * 2 + (half ^ 1)) * 128 + r]);
-      }
-      if (trole < 3) stamp(trole, j, 3);
-      // lazy running maximum: only move it when it grew by more than 8 (log2 units); probabilities stay <= 2^8
-      const bool need = mx > m_used + 8.0f;
-      const float m_new = need ? mx : m_used;
-      const float alpha = need ? exp2f(m_used - m_new) : 1.0f;  // first tile: m_used = -inf -> 0 (O is overwritten)
-      m_used = m_new;
-      uint64_t sum = 0;
-      const uint32_t pdst = p_row + sb * C::P_BYTES;
-      // Three separate passes over the thread's HB scores (exponent arguments, then the MUFU exponentials back to back, then
-      // pack + store): interleaved chunk by chunk, each exp2 -> pack -> store chain exposed the ~40 clk MUFU latency with two
-      // or three exponentials in flight (900 clk per 64 scores for a warp ALONE on its sub-partition's MUFU pipe, which
-      // could do them in 512).
-      const uint64_t sl2 = pair_of(p.sl2, p.sl2), off = pair_of(-m_new, -m_new);
-      uint64_t x[HB / 2];
-#pragma unroll
-      for (int i = 0; i < HB / 2; ++i) x[i] = fma_pair(pair_of(s[2 * i], s[2 * i + 1]), sl2, off);
-      // (an earlier variant with floorf / float->int range reduction was 40 % SLOWER: those conversions run on the XU pipe
-      //  as well, so it added XU work instead of removing it)
-#pragma unroll
-      for (int i = 0; i < HB / 2; ++i) x[i] = (i & 7) >= 8 - POLY16 / 2 ? exp2_fma_pair(x[i]) : pair_of(exp2_mufu(lo_f32(x[i])), exp2_mufu(hi_f32(x[i])));
-#pragma unroll
-      for (int cc = 0; cc < HB / 8; ++cc) {  // 16-byte chunks of 8 keys
-        uint32_t pk[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const uint64_t pp = x[cc * 4 + e];
-          if constexpr (!TCSUM) sum = add_pair(sum, pp);
-          pk[e] = pack_bf16(lo_f32(pp), hi_f32(pp));
-        }
-        const int c = half * (HB / 8) + cc;  // chunk index inside the whole tile row
-        const uint32_t addr = pdst + (c >> 3) * C::P_BOX + (((c & 7) ^ (r & 7)) << 4);
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
-      }
-      l_run = l_run * alpha + (lo_f32(sum) + hi_f32(sum));  // (SW == 2: the sum over this thread's columns only; the halves are added at the end)
-      if (trole < 3) stamp(trole, j, 4);
-      if (j > 0) {
-        if (__any_sync(0xffffffffu, need)) {  // (both warps of a quadrant see the same maxima, hence the same decision)
-          mbar_wait(o_done(qt, (j - 1) & 1), ((j - 1) >> 1) & 1);  // P_{j-1} V_{j-1} has completed: O may be touched
-          tc_fence_after();
-#pragma unroll 1
-          for (int c0 = half * 16; c0 < DHP; c0 += 16 * SW) {  // the halves take alternate 16-column slices of O
-            uint32_t v[16];
-            tmem_ld16(lane_addr + col_o + c0, v);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-            tmem_st16(lane_addr + col_o + c0, v);
+    int jt = 0;
+    for (int idx = blockIdx.x; idx < p.items; idx += gridDim.x) {
+      const Item it = idx == static_cast<int>(blockIdx.x) ? item0 : item(idx);
+      if (it.nqt == 0) continue;
+      const int n_keys = __shfl_sync(0xffffffffu, keys(it), 0), n_tiles = (n_keys + BN - 1) / BN;
+      if (qt >= it.nqt) break;  // (single tiles come last)
+      const int row = (it.tile0 + qt) * BM + r, first = jt;
+      float m_used = -INFINITY, l_run = 0.f;
+      for (; jt < first + n_tiles; ++jt) {
+        const int j = jt;
+        const int sb = j & 1;
+        const int trole = warp == 2 ? 1 : (warp == 6 ? 2 : 3);
+        if (trole < 3) stamp(trole, j, 0);
+        // S_j is ready AND P_{j-2} V_{j-2} has completed (its P buffer is the one this tile writes): both barrier round trips
+        // (~150 clk each even when the phase completed long ago) are in flight together.  P_{j-1} V_{j-1}, which the old loop
+        // waited for at the end of every tile, only matters to the rare O rescale below.
+        if (j >= 2) mbar_wait2(s_full(qt, sb), (j >> 1) & 1, o_done(qt, sb), ((j - 2) >> 1) & 1);
+        else mbar_wait(s_full(qt, sb), (j >> 1) & 1);
+        if constexpr (QT == 2) {
+          if (j == 0 && qt == 1 && p.stagger > 0) {
+            const long long t0 = clock64();
+            while (clock64() - t0 < p.stagger) {}
           }
-          tmem_st_wait();
+        }
+        if (trole < 3) stamp(trole, j, 1);
+        tc_fence_after();
+        float s[HB];
+        {
+          // every 16-column slice is requested before the one wait: the slices' TMEM round trips overlap instead of queueing
+          // (ncu at 4096 keys: tensor pipe 28 %, XU 45 %, issue 33 % -- nothing saturated, the softmax warps sit in latencies)
+          uint32_t v[HB / 16][16];
+#pragma unroll
+          for (int c0 = 0; c0 < HB; c0 += 16) tmem_ld16(lane_addr + col_s + sb * BN + half * HB + c0, v[c0 / 16]);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < HB; ++i) s[i] = __uint_as_float(v[i / 16][i % 16]);  // raw scores: the scale rides on the FFMA below
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (trole < 3) stamp(trole, j, 2);
+        if (lane == 0) mbar_arrive(s_empty(qt, sb));  // the S buffer may be overwritten by S_{j+2}
+        // The softmax warps are bound by instruction issue (ncu: ~9 instructions per score, XU pipe 39 %, tensor pipe 24 %), so
+        // the per-score work is kept to FMNMX, FFMA, MUFU, FADD and half an F2FP: keys are only masked in the one tile that
+        // has padding, and the softmax scale is folded into the exponent's FFMA (scale > 0: max commutes with it).
+        const int nvalid = n_keys - (j - first) * BN - half * HB;  // columns of this thread that are real keys
+        if (nvalid < HB) {
+#pragma unroll
+          for (int i = 0; i < HB; ++i)
+            if (i >= nvalid) s[i] = -INFINITY;
+        }
+        float mx;
+        {
+          // eight independent running maxima, then a tree: a single FMNMX chain over HB scores is HB dependent instructions
+          float m8[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) m8[i] = s[i];
+#pragma unroll
+          for (int i = 8; i < HB - 8; i += 16)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) m8[k] = max3(m8[k], s[i + k], s[i + 8 + k]);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) m8[k] = fmaxf(m8[k], s[HB - 8 + k]);
+          mx = max3(max3(m8[0], m8[1], m8[2]), max3(m8[3], m8[4], m8[5]), fmaxf(m8[6], m8[7]));
+        }
+        mx *= p.sl2;
+        if constexpr (SW == 2) {  // row maximum over both halves (buffer sb is rewritten two tiles later, one barrier apart)
+          xch[(sb * 2 + half) * 128 + r] = mx;
+          pair_sync();
+          mx = fmaxf(mx, xch[(sb * 2 + (half ^ 1)) * 128 + r]);
+        }
+        if (trole < 3) stamp(trole, j, 3);
+        // lazy running maximum: only move it when it grew by more than 8 (log2 units); probabilities stay <= 2^8
+        const bool need = mx > m_used + 8.0f;
+        const float m_new = need ? mx : m_used;
+        const float alpha = need ? exp2f(m_used - m_new) : 1.0f;  // first tile: m_used = -inf -> 0 (O is overwritten)
+        m_used = m_new;
+        uint64_t sum = 0;
+        const uint32_t pdst = p_row + sb * C::P_BYTES;
+        // Three separate passes over the thread's HB scores (exponent arguments, then the MUFU exponentials back to back, then
+        // pack + store): interleaved chunk by chunk, each exp2 -> pack -> store chain exposed the ~40 clk MUFU latency with two
+        // or three exponentials in flight (900 clk per 64 scores for a warp ALONE on its sub-partition's MUFU pipe, which
+        // could do them in 512).
+        const uint64_t sl2 = pair_of(p.sl2, p.sl2), off = pair_of(-m_new, -m_new);
+        uint64_t x[HB / 2];
+#pragma unroll
+        for (int i = 0; i < HB / 2; ++i) x[i] = fma_pair(pair_of(s[2 * i], s[2 * i + 1]), sl2, off);
+        // (an earlier variant with floorf / float->int range reduction was 40 % SLOWER: those conversions run on the XU pipe
+        //  as well, so it added XU work instead of removing it)
+#pragma unroll
+        for (int i = 0; i < HB / 2; ++i) x[i] = (i & 7) >= 8 - POLY16 / 2 ? exp2_fma_pair(x[i]) : pair_of(exp2_mufu(lo_f32(x[i])), exp2_mufu(hi_f32(x[i])));
+#pragma unroll
+        for (int cc = 0; cc < HB / 8; ++cc) {  // 16-byte chunks of 8 keys
+          uint32_t pk[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const uint64_t pp = x[cc * 4 + e];
+            if constexpr (!TCSUM) sum = add_pair(sum, pp);
+            pk[e] = pack_bf16(lo_f32(pp), hi_f32(pp));
+          }
+          const int c = half * (HB / 8) + cc;  // chunk index inside the whole tile row
+          const uint32_t addr = pdst + (c >> 3) * C::P_BOX + (((c & 7) ^ (r & 7)) << 4);
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
+        }
+        l_run = l_run * alpha + (lo_f32(sum) + hi_f32(sum));  // (SW == 2: the sum over this thread's columns only; the halves are added at the end)
+        if (trole < 3) stamp(trole, j, 4);
+        if (j > first) {
+          if (__any_sync(0xffffffffu, need)) {  // (both warps of a quadrant see the same maxima, hence the same decision)
+            mbar_wait(o_done(qt, (j - 1) & 1), ((j - 1) >> 1) & 1);  // P_{j-1} V_{j-1} has completed: O may be touched
+            tc_fence_after();
+#pragma unroll 1
+            for (int c0 = half * 16; c0 < DHP; c0 += 16 * SW) {  // the halves take alternate 16-column slices of O
+              uint32_t v[16];
+              tmem_ld16(lane_addr + col_o + c0, v);
+              tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
+              tmem_st16(lane_addr + col_o + c0, v);
+            }
+            tmem_st_wait();
+          }
+        }
+        if (trole < 3) stamp(trole, j, 5);
+        fence_proxy_async_smem();  // P (generic-proxy stores) -> visible to the tensor core's async-proxy reads
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_full(qt, sb));
+        if (trole < 3) stamp(trole, j, 6);
+      }
+      // ---- epilogue: O / l -> bf16 ----
+      if constexpr (SW == 2 && !TCSUM) {  // total row sum = sum over both halves
+        pair_sync();            // the partner has read the last tile's maximum: the exchange area is free
+        xch[half * 128 + r] = l_run;
+        pair_sync();
+        l_run += xch[(half ^ 1) * 128 + r];
+      }
+      mbar_wait(o_done(qt, (jt - 1) & 1), ((jt - 1) >> 1) & 1);
+      tc_fence_after();
+      if constexpr (TCSUM) {  // the row sum is column DH of the accumulator (ones column of V); any warp of the quadrant may read it
+        uint32_t v[16];
+        tmem_ld16(lane_addr + col_o + (DH / 16) * 16, v);
+        tmem_ld_wait();
+        l_run = __uint_as_float(v[DH % 16]);
+      }
+      const float inv = 1.0f / l_run;
+      const bool row_ok = row < p.rows;
+      bf16* orow = p.o + it.b * p.o_bs + it.h * p.o_head_off + static_cast<long long>(row / p.group) * p.o_ts +
+                   static_cast<long long>(row % p.group) * p.o_hs;
+      constexpr int EB = SW == 1 && DHP <= 80 ? DHP / 16 : 4;  // 16-column slices requested together
+#pragma unroll 1
+      for (int c1 = half * 16; c1 < DHP; c1 += 16 * SW * EB) {
+        uint32_t all[EB][16];
+#pragma unroll
+        for (int i = 0; i < EB; ++i)
+          if (c1 + 16 * SW * i < DHP) tmem_ld16(lane_addr + col_o + c1 + 16 * SW * i, all[i]);
+        tmem_ld_wait();
+        if (c1 + 16 * SW * EB >= DHP) {  // O has been read: the next block's may be summed
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(o_empty(qt));
+        }
+#pragma unroll
+        for (int i = 0; i < EB; ++i) {
+          const int c0 = c1 + 16 * SW * i;
+          const uint32_t(&v)[16] = all[i];
+          if (c0 >= DHP || !row_ok) continue;
+          uint32_t pk[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) pk[k] = pack_bf16(__uint_as_float(v[2 * k]) * inv, __uint_as_float(v[2 * k + 1]) * inv);
+          if (c0 + 8 <= p.dh) *reinterpret_cast<uint4*>(orow + c0) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+          if (c0 + 16 <= p.dh) *reinterpret_cast<uint4*>(orow + c0 + 8) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
         }
       }
-      if (trole < 3) stamp(trole, j, 5);
-      fence_proxy_async_smem();  // P (generic-proxy stores) -> visible to the tensor core's async-proxy reads
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(p_full(qt, sb));
-      if (trole < 3) stamp(trole, j, 6);
-    }
-    // ---- epilogue: O / l -> bf16 ----
-    if constexpr (SW == 2 && !TCSUM) {  // total row sum = sum over both halves
-      pair_sync();            // the partner has read the last tile's maximum: the exchange area is free
-      xch[half * 128 + r] = l_run;
-      pair_sync();
-      l_run += xch[(half ^ 1) * 128 + r];
-    }
-    mbar_wait(o_done(qt, (n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1);
-    tc_fence_after();
-    if constexpr (TCSUM) {  // the row sum is column DH of the accumulator (ones column of V); any warp of the quadrant may read it
-      uint32_t v[16];
-      tmem_ld16(lane_addr + col_o + (DH / 16) * 16, v);
-      tmem_ld_wait();
-      l_run = __uint_as_float(v[DH % 16]);
-    }
-    const float inv = 1.0f / l_run;
-    const bool row_ok = row < p.rows;
-    bf16* orow = p.o + b * p.o_bs + h * p.o_head_off + static_cast<long long>(row / p.group) * p.o_ts +
-                 static_cast<long long>(row % p.group) * p.o_hs;
-#pragma unroll 1
-    for (int c0 = half * 16; c0 < DHP; c0 += 16 * SW) {
-      uint32_t v[16];
-      tmem_ld16(lane_addr + col_o + c0, v);
-      tmem_ld_wait();
-      if (row_ok) {
-        uint32_t pk[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) pk[i] = pack_bf16(__uint_as_float(v[2 * i]) * inv, __uint_as_float(v[2 * i + 1]) * inv);
-        if (c0 + 8 <= p.dh) *reinterpret_cast<uint4*>(orow + c0) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-        if (c0 + 16 <= p.dh) *reinterpret_cast<uint4*>(orow + c0 + 8) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-      }
+      if constexpr (SW == 2) pair_sync();  // the partner has read the sums: the exchange area is free for the next block
     }
     tc_fence_before();
   }
@@ -553,7 +614,7 @@ static int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
     }
     configured[dev] = true;
   }
-  // One CTA per SM.  Where the last round has at most half as many blocks as SMs, its two query tiles go to two CTAs: a tile alone on an SM takes a little over half of what two
+  // One CTA per SM.  Where the last round has at most half as many blocks as SMs, the two query tiles of each go to two CTAs: a tile alone on an SM takes a little over half of what two
   // together take (64 blocks of 1024 keys 25 -> 19 us, 192 47 -> 40, 512 of 4096 keys 295 -> 258, the packed exponentials of 3 % included).
   Params pp = p;
   pp.m_blks = (p.rows + C::BM * QT - 1) / (C::BM * QT);
@@ -563,7 +624,8 @@ static int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
   const int rest = static_cast<int>(blks % num_sms());
   const bool split = QT == 2 && 2 * rest <= num_sms();
   pp.whole = static_cast<int>(split ? blks - rest : blks);
-  const unsigned grid = static_cast<unsigned>(split ? blks + rest : blks);
+  pp.items = static_cast<int>(split ? blks + rest : blks);
+  const unsigned grid = static_cast<unsigned>(pp.items < num_sms() ? pp.items : num_sms());
   return launch_kernel(attn_prefill_tc_kernel<DH, SW, QT>, grid, dim3(96 + 128 * SW * QT), C::SMEM, st, tq, tk, tv, pp) == cudaSuccess ? PG_OK : PG_ERR_CUDA;
 }
 
