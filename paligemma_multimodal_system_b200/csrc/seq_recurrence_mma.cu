@@ -34,6 +34,12 @@ namespace {
 constexpr float LOG2E = 1.4426950408889634f;
 
 __device__ __forceinline__ float softplus(float z) { return fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))); }
+// 2^x by the hardware alone: exponents are differences <= 0, and what underflows weighs nothing
+__device__ __forceinline__ float ex2_ftz(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 __device__ __forceinline__ float lo_f(uint32_t u) { return __uint_as_float(u << 16); }
 __device__ __forceinline__ float hi_f(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
 
@@ -491,7 +497,7 @@ __global__ void __launch_bounds__(128) delta_blocks_kernel(PgDeltaArgs a, float*
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const float z = lg[it][i] + bias;
-      const float sp = fmaxf(z, 0.f) + log1pf(exp2f(-fabsf(z) * LOG2E));
+      const float sp = fmaxf(z, 0.f) + log1pf(ex2_ftz(-fabsf(z) * LOG2E));
       if (i < nt) run = fmaf(rate, sp, run);
       lg[it][i] = run;
     }
@@ -502,7 +508,7 @@ __global__ void __launch_bounds__(128) delta_blocks_kernel(PgDeltaArgs a, float*
       Lg[o + i * LD] = lg[it][i];
       Kn[o + i * LD] = kv;
       Qn[o + i * LD] = qv;
-      const float f = exp2f(half == 0 ? run - lg[it][i] : lg[it][i]);
+      const float f = ex2_ftz(half == 0 ? run - lg[it][i] : lg[it][i]);
       Kf[o + i * LD] = kv * f;
       if (half == 1) Qf[i * LD + d] = qv * f;
     }
@@ -531,7 +537,7 @@ __global__ void __launch_bounds__(128) delta_blocks_kernel(PgDeltaArgs a, float*
         const float4 lt = *reinterpret_cast<const float4*>(Lg + t * LD + d), lj = *reinterpret_cast<const float4*>(Lg + j * LD + d);
         const float4 kt = *reinterpret_cast<const float4*>(Kn + t * LD + d), kj = *reinterpret_cast<const float4*>(Kn + j * LD + d);
         const float4 qt = *reinterpret_cast<const float4*>(Qn + t * LD + d);
-        const float e0 = exp2f(lt.x - lj.x) * kj.x, e1 = exp2f(lt.y - lj.y) * kj.y, e2 = exp2f(lt.z - lj.z) * kj.z, e3 = exp2f(lt.w - lj.w) * kj.w;
+        const float e0 = ex2_ftz(lt.x - lj.x) * kj.x, e1 = ex2_ftz(lt.y - lj.y) * kj.y, e2 = ex2_ftz(lt.z - lj.z) * kj.z, e3 = ex2_ftz(lt.w - lj.w) * kj.w;
         sa = fmaf(kt.x, e0, fmaf(kt.y, e1, fmaf(kt.z, e2, fmaf(kt.w, e3, sa))));
         sb = fmaf(qt.x, e0, fmaf(qt.y, e1, fmaf(qt.z, e2, fmaf(qt.w, e3, sb))));
       }
@@ -595,19 +601,32 @@ __global__ void __launch_bounds__(128) delta_blocks_kernel(PgDeltaArgs a, float*
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
-// Delta rule, the sequential part.  128 threads, warp = 16 value columns.  The operand tiles kg, qg, ke of block b + 1 are formed (from
+// Delta rule, the sequential part.  Four warps of 16 value columns each.  The operand tiles kg, qg, ke of block b + 1 are formed (from
 // q, k and cumulative decays fetched into registers a block earlier) while block b's tiles are multiplied; one barrier per block.
+// SPLIT (heads up to 64 wide): by four warps of their own, which leave the other four the registers -- launched with 128 a thread, so that two CTAs fit an SM.  What bounds it: the
+// mma.sync pipe of the SMs that hold two chains (168 products a block and warp, 12 clocks each), elsewhere their order through S, U and S again (6 prompts of 550 .. 700 tokens, 32 heads of 64, 192
+// CTAs: with the tiles formed in the chain's own warps 128 us, 120 now).
 // ---------------------------------------------------------------------------------------------------------------------
+template <int N>
+__device__ __forceinline__ void more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
 template <int DIM>
-__global__ void __launch_bounds__(128) delta_chain_kernel(PgDeltaArgs a, const uint4* __restrict__ scratch, int n_min) {
+__global__ void __launch_bounds__(DIM <= 64 ? 256 : 128, DIM <= 64 ? 2 : 1) delta_chain_kernel(PgDeltaArgs a, const uint4* __restrict__ scratch, int n_min) {
   pg::griddep_begin();
+  constexpr bool SPLIT = DIM <= 64;
   constexpr int LD = DIM + 8, LV = 72, NI = (DIM + 63) / 64, TILE = 16 * LD;
   const int e = blockIdx.z, h = blockIdx.y;
   const int n = a.entry_n[e];
   if (n < n_min) return;
   const int dim = a.dim, vdim = a.vdim, H = a.H;
   const long long row0 = a.entry_row0[e];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gq = lane >> 2, tq = lane & 3;
+  const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) & 3, gq = lane >> 2, tq = lane & 3, tid = threadIdx.x & 127;
+  auto block_barrier = [&]() {
+    if constexpr (SPLIT) asm volatile("bar.sync 1, 256;" ::: "memory");
+    else __syncthreads();
+  };
   extern __shared__ __align__(16) unsigned char smraw[];
   bf16* Tl = reinterpret_cast<bf16*>(smraw);  // [2][3 matrices kg, qg, ke][3 terms][16][LD]
   bf16* Vs = Tl + 18 * TILE;                  // [2][16][LV]
@@ -618,8 +637,6 @@ __global__ void __launch_bounds__(128) delta_chain_kernel(PgDeltaArgs a, const u
   const bf16* vp = static_cast<const bf16*>(a.v) + (long long)h * vdim + v_base;
   const float* lgp = a.decay + (long long)h * dim;
   float* stp = a.state + (((long long)a.entry_slot[e] * H + h) * dim) * vdim;
-  float S[DIM / 8][4];
-  load_state<DIM>(S, stp, dim, vdim, vcol, tq, a.entry_ctx[e] == 0);
   const int r = tid >> 3, c8 = tid & 7;  // this thread's token row and first group of 8 channels of a tile
   uint4 rk[NI], rq[NI];
   float4 rl[NI][2], re[NI][2];
@@ -661,18 +678,18 @@ __global__ void __launch_bounds__(128) delta_chain_kernel(PgDeltaArgs a, const u
       uint32_t t[9][4];
 #pragma unroll
       for (int p = 0; p < 4; ++p) {
-        const float f0 = exp2f(l[2 * p]), f1 = exp2f(l[2 * p + 1]);
+        const float f0 = ex2_ftz(l[2 * p]), f1 = ex2_ftz(l[2 * p + 1]);
         const float k0 = lo_f(kw[p]) * ik, k1 = hi_f(kw[p]) * ik;
         cut3(k0 * f0, k1 * f1, t[0][p], t[1][p], t[2][p]);
         cut3(lo_f(qw[p]) * iq * f0, hi_f(qw[p]) * iq * f1, t[3][p], t[4][p], t[5][p]);
         // a row past the end has k = 0; its exponent must only not overflow
-        cut3(k0 * exp2f(fminf(le[2 * p] - l[2 * p], 0.f)), k1 * exp2f(fminf(le[2 * p + 1] - l[2 * p + 1], 0.f)), t[6][p], t[7][p], t[8][p]);
+        cut3(k0 * ex2_ftz(fminf(le[2 * p] - l[2 * p], 0.f)), k1 * ex2_ftz(fminf(le[2 * p + 1] - l[2 * p + 1], 0.f)), t[6][p], t[7][p], t[8][p]);
       }
 #pragma unroll
       for (int m = 0; m < 9; ++m) *reinterpret_cast<uint4*>(base + m * TILE + c) = make_uint4(t[m][0], t[m][1], t[m][2], t[m][3]);
       if (r == 0) {
 #pragma unroll
-        for (int x = 0; x < 8; ++x) Ge[buf * DIM + c + x] = exp2f(le[x]);
+        for (int x = 0; x < 8; ++x) Ge[buf * DIM + c + x] = ex2_ftz(le[x]);
       }
     }
   };
@@ -680,23 +697,44 @@ __global__ void __launch_bounds__(128) delta_chain_kernel(PgDeltaArgs a, const u
   const int b_row = (lane & 7) + ((lane >> 4) & 1) * 8, b_col = ((lane >> 3) & 1) * 8;
   const uint4* frag = scratch + (block_index(a, e, 0) * H + h) * 6 * 32 + lane;
   const long long frag_step = (long long)H * 6 * 32;
+  auto make = [&]() {  // the tiles, a block ahead of the products
+    fetch_raw(0);
+    fetch_v(0, 0);
+    form_tiles(0);
+    if (16 < n) fetch_raw(16);
+  };
+  auto make_next = [&](int t0, int cur) {
+    if (t0 + 16 >= n) return;
+    fetch_v(t0 + 16, cur ^ 1);
+    form_tiles(cur ^ 1);
+    if (t0 + 32 < n) fetch_raw(t0 + 32);
+  };
+  if constexpr (SPLIT) {
+    if (threadIdx.x >= 128) {
+      fewer_registers<72>();
+      make();
+      int cur = 0;
+      for (int t0 = 0; t0 < n; t0 += 16, cur ^= 1) {
+        pg::cp_async_wait<0>();
+        block_barrier();  // this block's tiles are complete; the products are done with the other buffers
+        make_next(t0, cur);
+      }
+      return;
+    }
+    more_registers<184>();
+  }
+  float S[DIM / 8][4];
+  load_state<DIM>(S, stp, dim, vdim, vcol, tq, a.entry_ctx[e] == 0);
   uint4 fw[3], fb[3];
-  fetch_raw(0);
-  fetch_v(0, 0);
 #pragma unroll
   for (int x = 0; x < 3; ++x) { fw[x] = frag[x * 32]; fb[x] = frag[(3 + x) * 32]; }
-  form_tiles(0);
-  if (16 < n) fetch_raw(16);
+  if constexpr (!SPLIT) make();
   int cur = 0;
   for (int t0 = 0; t0 < n; t0 += 16, cur ^= 1) {
-    pg::cp_async_wait<0>();
-    __syncthreads();  // this block's tiles are complete; every warp is done with the other buffers
+    if constexpr (!SPLIT) pg::cp_async_wait<0>();
+    block_barrier();  // this block's tiles are complete; every warp is done with the other buffers
     const bool more = t0 + 16 < n;
-    if (more) {
-      fetch_v(t0 + 16, cur ^ 1);
-      form_tiles(cur ^ 1);
-      if (t0 + 32 < n) fetch_raw(t0 + 32);
-    }
+    if constexpr (!SPLIT) make_next(t0, cur);
     const bf16* kg = Tl + cur * 9 * TILE;
     const bf16* qg = kg + 3 * TILE;
     const bf16* ke = qg + 3 * TILE;
@@ -798,7 +836,7 @@ int launch_delta(const PgDeltaArgs& a, float* decay, uint4* scratch, int max_n, 
   auto k2 = delta_chain_kernel<DIM>;
   rc = set_smem(k2, s2);
   if (rc != PG_OK) return rc;
-  pg::launch_spread(k2, dim3((a.vdim + 63) / 64, a.H, a.entries), 128, s2, st, a, scratch, n_min);
+  pg::launch_spread(k2, dim3((a.vdim + 63) / 64, a.H, a.entries), DIM <= 64 ? 256 : 128, s2, st, a, scratch, n_min);
   pg_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
 }
