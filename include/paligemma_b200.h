@@ -107,6 +107,10 @@ int pg_gemm_bf16_fused(const void* x, long long ldx, const void* w, long long ld
 int pg_gemm_residual(const void* x, long long ldx, const void* w, long long ldw, float* h, long long ldh, const float* bias, int tokens, int features,
                      int K, float scale, void* stream);
 
+/* Between pg_weights_follow(1) and pg_weights_follow(0) the calling thread promises that the second operand of every product it issues is a weight: nothing that kernels of the same
+ * stream still write.  Norms, gates and attention then let the kernel behind them come early (it requests its weights while they run).  Calls nest. */
+int pg_weights_follow(int on);
+
 /* out[t,f] = sum_k x[t,k] w[f,k] in fp32 rows; few tokens and few output tiles: K is shared out over the GPU. */
 int pg_linear_f32(const void* x, long long ldx, const void* w, long long ldw, float* out, long long ldo, int tokens, int features, int K, void* stream);
 

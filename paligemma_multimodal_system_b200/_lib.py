@@ -41,6 +41,7 @@ SIGNATURES = {
     "pg_gemm_bf16": [p, i64, p, i64, p, i64, p, p, i64, i32, i32, i32, i32, i32, f32, i32, i32, p],
     "pg_gemm_bf16_fused": [p, i64, p, i64, p, i64, p, p, i64, i32, i32, i32, i32, i32, f32, i32, i32, p, p],
     "pg_gemm_residual": [p, i64, p, i64, p, i64, p, i32, i32, i32, f32, p],
+    "pg_weights_follow": [i32],
     "pg_linear_f32": [p, i64, p, i64, p, i64, i32, i32, i32, p],
     "pg_siglip_layers": [p, i32, p, p, p, p, p, i32, i32, i32, i32, i32, f32, p],
     "pg_gemma_prefill_layers": [p, i32, p, p],

@@ -174,7 +174,8 @@ PG_DEVINL void griddep_launch_dependents() { asm volatile("griddepcontrol.launch
 //   * griddep_begin(): waits; the next kernel comes when this one has ended, as after a plain launch, but with its launch behind it.  Everything that writes 16-bit rows (they can be
 //     the weight operand of the product behind), pages or positions.
 //   * griddep_begin<true>(): waits, then triggers.  Kernels whose results are fp32 rows and integers that are read behind a wait only (routing, scans).
-//   * griddep_begin_if(weights_follow()): where a whole layer is issued by one call (layers.cu) it is known that the product behind a norm or an attention takes a weight.
+//   * griddep_begin_if(weights_follow()): where a whole layer is issued by one call (layers.cu), or a model's step by an engine that says so (pg_weights_follow), it is known that the
+//     product behind a norm or an attention takes a weight.
 // What that costs against every kernel triggering ahead of its wait: 48 requests with 24 decode steps 16.5 -> 16.9 ms, one request through four narrow layers 5 %; a tower of
 // four layers, one image 252 -> 247 us, a routed feed-forward 91 us both.
 // (Products trigger behind their wait: their outputs are not weights.  rmsnorm_kernel of the Gemma decode chain triggers early: see there.)
@@ -358,8 +359,8 @@ inline int num_sms() {
   return sms[dev];
 }
 
-// While a thread issues whole layers by one call (layers.cu) the product behind a norm or an attention is that layer's, and its operand a weight: there they trigger behind their
-// wait.  Counted per thread, for the length of that call.
+// While a thread issues whole layers by one call (layers.cu), or a model's step between two calls of pg_weights_follow, the product behind a norm or an attention is that layer's, and
+// its operand a weight: there they trigger behind their wait.  Counted per thread, for the length of that call or step.
 inline thread_local int t_weights_follow = 0;
 inline int weights_follow() { return t_weights_follow > 0 ? 1 : 0; }
 struct WeightsFollow {

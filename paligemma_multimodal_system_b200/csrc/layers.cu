@@ -8,6 +8,11 @@
 
 bool pg_gemm_sums_once(int tokens, int features, int K, const void* out, long long ldo, const float* bias, int swap);  // gemm_tcgen05.cu
 
+extern "C" int pg_weights_follow(int on) {
+  pg::t_weights_follow += on ? 1 : -1;
+  return PG_OK;
+}
+
 extern "C" int pg_gemm_residual(const void* x, long long ldx, const void* w, long long ldw, float* h, long long ldh, const float* bias, int tokens,
                                 int features, int K, float scale, void* stream) {
   if (tokens <= 0 || features <= 0 || K <= 0) return PG_ERR_ARG;

@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(32 * kWarps, VC == 1 && sizeof(TA) == 2 ? 3 : 
                                                                          const int* __restrict__ entry_row0, const int* __restrict__ entry_n,
                                                                          const int* __restrict__ entry_ctx, const int* __restrict__ page_table, int max_pages,
                                                                          int page, int H, int G, int dim, int vdim, float scale, float softcap, long long krow,
-                                                                         long long vrow, int gate_per_head, PgAttnScore sx) {
+                                                                         long long vrow, int gate_per_head, PgAttnScore sx, int trigger) {
   constexpr bool EARLY_V = VC == 1 && sizeof(TA) == 2;
   const int e = blockIdx.z, g = blockIdx.y, split = blockIdx.x, nsplit = gridDim.x, gsz = H / G;
   const int ctx = entry_ctx[e];
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(32 * kWarps, VC == 1 && sizeof(TA) == 2 ? 3 : 
       for (int i = 0; i < dim * (int)sizeof(TA); i += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(k + i));
       for (int i = 0; i < vdim * (int)sizeof(TA); i += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(v + i));
     }
-  pg::griddep_wait();
+  pg::griddep_begin_if(trigger);
   if (!mine) return;
   for (int i = threadIdx.x; i < gsz * dimp; i += 32 * kWarps) {
     const int r = i / dimp, d = i % dimp;
@@ -307,7 +307,7 @@ int launch(const void* q, const void* kp, const void* vp, const void* gate, long
   }
   return pg::launch_kernel(kern, dim3(nsplit, G, entries), dim3(32 * kWarps), smem, st, static_cast<const TA*>(q), static_cast<const TA*>(kp),
                            static_cast<const TA*>(vp), static_cast<const TA*>(gate), ldg, static_cast<TA*>(out), partial, row0, n, ctx, pt, max_pages, page, H, G,
-                           dim, vdim, scale, softcap, krow, vrow, gate_per_head, sx) == cudaSuccess
+                           dim, vdim, scale, softcap, krow, vrow, gate_per_head, sx, pg::weights_follow()) == cudaSuccess
              ? PG_OK : PG_ERR_CUDA;
 }
 

@@ -122,8 +122,8 @@ __global__ void embed_rows_kernel(const int* __restrict__ tokens, const TI* __re
 // The same, eight elements a thread (16-byte rows): the row of 2048 is one request, not sixteen (48 rows back to back 6.2 -> 1.4 us).
 template <typename TI>
 __global__ void __launch_bounds__(256) embed_rows_vec_kernel(const int* __restrict__ tokens, const TI* __restrict__ table, long long ld, int col0,
-                                                             float* __restrict__ out, TI* __restrict__ out_act, int D, float scale) {
-  pg::griddep_begin();
+                                                             float* __restrict__ out, TI* __restrict__ out_act, int D, float scale, int trigger) {
+  pg::griddep_begin_if(trigger);
   const int t = blockIdx.x;
   const TI* row = table + tokens[t] * ld + col0;
   for (int d = 8 * threadIdx.x; d < D; d += 8 * 256) {
@@ -233,9 +233,9 @@ __global__ void __launch_bounds__(256) group_rmsnorm_add_kernel(const float* __r
 // back to back: 4.1 -> 2.1 us); prompts, HBM (10836 rows: 70 us in either form).
 template <typename TO, int NV>
 __global__ void __launch_bounds__(256) group_rmsnorm_add_reg_kernel(const float* __restrict__ y, long long ldy, const float* __restrict__ w,
-                                                                    float* __restrict__ x, TO* __restrict__ out_act, int D, int gs, float eps) {
+                                                                    float* __restrict__ x, TO* __restrict__ out_act, int D, int gs, float eps, int trigger) {
   __shared__ float red[8 * NV];  // sums of 128 neighbouring elements
-  pg::griddep_begin();
+  pg::griddep_begin_if(trigger);
   const long long t = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float4 v[NV], ww[NV], xv[NV];
@@ -322,9 +322,9 @@ __global__ void __launch_bounds__(256) rmsnorm_gate_kernel(const float* __restri
 // The same for rows of up to 4096 elements: a thread keeps its elements, so the row, the gate and the weights are requested together and the row once.  48 rows of 2048 back to back: 4.1 -> 1.9 us; 10836 rows: 55 in either form.
 template <typename TA, int NV>
 __global__ void __launch_bounds__(256) rmsnorm_gate_reg_kernel(const float* __restrict__ o, const float* __restrict__ w, const TA* __restrict__ gate,
-                                                               long long ldg, TA* __restrict__ out, int D, float eps) {
+                                                               long long ldg, TA* __restrict__ out, int D, float eps, int trigger) {
   __shared__ float red[8];
-  pg::griddep_begin();
+  pg::griddep_begin_if(trigger);
   const long long t = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float4 v[NV], ww[NV], g[NV];
@@ -461,9 +461,9 @@ extern "C" int pg_embed_rows(const int* tokens, const void* table, long long ld,
   if (D % 8 == 0 && ld % 8 == 0 && col0 % 8 == 0 &&
       ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(out_act)) & 15) == 0) {
     if (table_f32)
-      pg::launch_dependent(embed_rows_vec_kernel<float>, rows, 256, 0, PG_ST(stream), tokens, static_cast<const float*>(table), ld, col0, out, static_cast<float*>(out_act), D, scale);
+      pg::launch_dependent(embed_rows_vec_kernel<float>, rows, 256, 0, PG_ST(stream), tokens, static_cast<const float*>(table), ld, col0, out, static_cast<float*>(out_act), D, scale, pg::weights_follow());
     else
-      pg::launch_dependent(embed_rows_vec_kernel<bf16>, rows, 256, 0, PG_ST(stream), tokens, static_cast<const bf16*>(table), ld, col0, out, static_cast<bf16*>(out_act), D, scale);
+      pg::launch_dependent(embed_rows_vec_kernel<bf16>, rows, 256, 0, PG_ST(stream), tokens, static_cast<const bf16*>(table), ld, col0, out, static_cast<bf16*>(out_act), D, scale, pg::weights_follow());
     PG_RET();
   }
   if (table_f32)
@@ -482,7 +482,7 @@ extern "C" int pg_group_rmsnorm_add(const float* y, long long ldy, const float* 
                    ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out_act)) & 15) == 0;
   const int gs = D / groups;
   if (vec && gs % 128 == 0 && D <= 4096) {
-#define PG_GNR(TO, NV) pg::launch_dependent(group_rmsnorm_add_reg_kernel<TO, NV>, rows, 256, 0, st, y, ldy, w, x, static_cast<TO*>(out_act), D, gs, eps)
+#define PG_GNR(TO, NV) pg::launch_dependent(group_rmsnorm_add_reg_kernel<TO, NV>, rows, 256, 0, st, y, ldy, w, x, static_cast<TO*>(out_act), D, gs, eps, pg::weights_follow())
     if (out_f32) {
       if (D <= 1024) PG_GNR(float, 1); else if (D <= 2048) PG_GNR(float, 2); else PG_GNR(float, 4);
     } else {
@@ -509,7 +509,7 @@ extern "C" int pg_rmsnorm_gate(const float* o, const float* w, const void* gate,
                    ((reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(out)) & act_mask) == 0;
   cudaStream_t st = PG_ST(stream);
   if (vec && D <= 4096) {
-#define PG_RGR(TA, NV) pg::launch_dependent(rmsnorm_gate_reg_kernel<TA, NV>, rows, 256, 0, st, o, w, static_cast<const TA*>(gate), ldg, static_cast<TA*>(out), D, eps)
+#define PG_RGR(TA, NV) pg::launch_dependent(rmsnorm_gate_reg_kernel<TA, NV>, rows, 256, 0, st, o, w, static_cast<const TA*>(gate), ldg, static_cast<TA*>(out), D, eps, pg::weights_follow())
     if (act_f32) {
       if (D <= 1024) PG_RGR(float, 1); else if (D <= 2048) PG_RGR(float, 2); else PG_RGR(float, 4);
     } else {

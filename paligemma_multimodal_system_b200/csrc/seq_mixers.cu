@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(128) attn_prepare_vec_kernel(const TA* __restr
                                                                const float* __restrict__ kn, TA* __restrict__ q_out, TA* __restrict__ k_pages,
                                                                TA* __restrict__ v_pages, int rows, int H, int G, int dim, int vdim, int rot, float eps,
                                                                int norm_qk, int norm_v, int v_from_k, float rot_gain, const TA* __restrict__ v_other,
-                                                               long long ldvo, float v_mix) {
+                                                               long long ldvo, float v_mix, int trigger) {
   extern __shared__ __align__(16) float cs[];  // [TOK][cos rot/2 | sin rot/2]
   __shared__ float part[2][TOK][4];
   const int t0 = blockIdx.x * TOK, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(128) attn_prepare_vec_kernel(const TA* __restr
     for (int k = 0; k < TOK; ++k) x[k] = ldraw<TA>(p + (t0 + k < rows ? k : rows - 1 - t0) * ld);
   };
   if (TOK > 1) {
-    pg::griddep_wait();
+    pg::griddep_begin_if(trigger);
     request(ahead[0], threadIdx.x);
   }
   for (int i = threadIdx.x; i < TOK * half; i += 128) {
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(128) attn_prepare_vec_kernel(const TA* __restr
     cs[k * rot + half + j] = rot_gain * (float)s;
   }
   if (TOK == 1) {  // (positions, pages and frequencies are the host's)
-    pg::griddep_wait();
+    pg::griddep_begin_if(trigger);
 #pragma unroll
     for (int d = 0; d < DEEP; ++d) request(ahead[d], threadIdx.x + 128 * d);
   }
@@ -1185,7 +1185,8 @@ extern "C" int pg_attn_prepare(const void* qkv, long long ld, const int* pos, co
       using TA = decltype(t);
       pg::launch_dependent(kernel, (rows + tok - 1) / tok, 128, (size_t)(tok * rot_dims + 2) * sizeof(float), PG_ST(stream), 
           static_cast<const TA*>(qkv), ld, pos, row_entry, page_table, max_pages, page, freq, q_norm, k_norm, static_cast<TA*>(q_out), static_cast<TA*>(k_pages),
-          static_cast<TA*>(v_pages), rows, H, G, dim, vdim, rot_dims, eps, norm_qk, norm_v, v_from_k, rot_gain, static_cast<const TA*>(v_other), ld_v_other, v_mix);
+          static_cast<TA*>(v_pages), rows, H, G, dim, vdim, rot_dims, eps, norm_qk, norm_v, v_from_k, rot_gain, static_cast<const TA*>(v_other), ld_v_other, v_mix,
+          pg::weights_follow());
     };
     // four tokens a CTA once that still fills the SMs
     const bool four = rows >= 4 * 4 * pg::num_sms(), rot8 = rot_dims % 8 == 0;

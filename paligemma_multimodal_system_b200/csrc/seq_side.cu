@@ -54,7 +54,7 @@ __device__ __forceinline__ void st_peers(float* p, float v) {  // the same word 
 template <typename TA>
 __global__ void __launch_bounds__(kThreads) token_side_kernel(const TA* act, const TA* __restrict__ wg, const int* __restrict__ tokens, const TA* __restrict__ table,
                                                               long long ldt, int col0, const TA* __restrict__ wp, const float* __restrict__ norm_w, float* x,
-                                                              TA* out_act, int D, int n, int n_pad, float eps) {
+                                                              TA* out_act, int D, int n, int n_pad, float eps, int trigger) {
   extern __shared__ __align__(16) float sm[];
   float* row = sm;           // [D] the activation row
   float* gz = row + D;       // [kMaxInner]
@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(kThreads) token_side_kernel(const TA* act, con
       asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(wp) + l * 128));
     }
   }
-  pg::griddep_wait();
+  pg::griddep_begin_if(trigger);
   const int rank = static_cast<int>(pg::cluster_ctarank()), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long t = blockIdx.x / kRanks;
   const long long tok = tokens[t];
@@ -177,7 +177,7 @@ int launch(const void* act, const void* wg, const int* tokens, const void* table
   cfg.numAttrs = pg_pdl_enabled() ? 2 : 1;
   pg_count_launch(1);
   return cudaLaunchKernelEx(&cfg, token_side_kernel<TA>, static_cast<const TA*>(act), static_cast<const TA*>(wg), tokens, static_cast<const TA*>(table), ldt, col0,
-                            static_cast<const TA*>(wp), norm_w, x, static_cast<TA*>(out_act), D, n, n_pad, eps) == cudaSuccess ? PG_OK : PG_ERR_CUDA;
+                            static_cast<const TA*>(wp), norm_w, x, static_cast<TA*>(out_act), D, n, n_pad, eps, pg::weights_follow()) == cudaSuccess ? PG_OK : PG_ERR_CUDA;
 }
 
 }  // namespace

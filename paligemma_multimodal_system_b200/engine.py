@@ -9,6 +9,7 @@ that has some -- whole prompts, portions of prompts and single decoded tokens si
 
 The model supplies `cache_layout()`, `step(batch, store, want_rows)`, `prec` and `vocab_size` (modeling_mapedra.py).
 """
+import contextlib
 from typing import Dict, List, Optional, Sequence, Tuple
 
 import torch
@@ -17,6 +18,17 @@ from . import _lib
 from .cache import SequenceStore
 from .seq_ops import StaticDecodeBatch, make_step_batch
 from .serving import StepScheduler, TokenRequest
+
+
+@contextlib.contextmanager
+def _weights_follow():
+    """The products of a model's step take weights as their second operand: the kernels in front of them may let them come early."""
+    L = _lib.lib()
+    L.pg_weights_follow(1)
+    try:
+        yield
+    finally:
+        L.pg_weights_follow(0)
 
 
 class SequenceEngine:
@@ -63,7 +75,8 @@ class SequenceEngine:
         elif batch:
             b = make_step_batch(batch)
             rows = torch.tensor(want, dtype=torch.int64).to("cuda", non_blocking=True) if want else None
-            logits = self.model.step(b, store, rows, trace=trace)
+            with _weights_follow():
+                logits = self.model.step(b, store, rows, trace=trace)
             for (rid, toks, _w) in entries:
                 store.commit(rid, len(toks))
         for rid in end:
@@ -91,7 +104,7 @@ class SequenceEngine:
             side.wait_stream(torch.cuda.current_stream())
             with torch.cuda.stream(side):
                 g = torch.cuda.CUDAGraph()
-                with torch.cuda.graph(g, stream=side):
+                with torch.cuda.graph(g, stream=side), _weights_follow():
                     slot["logits"] = self.model.step(st.batch, self.store, st.rows)
             torch.cuda.current_stream().wait_stream(side)
             slot["graph"] = g
@@ -99,7 +112,8 @@ class SequenceEngine:
             slot["graph"].replay()
             full = slot["logits"]
         else:
-            full = self.model.step(st.batch, self.store, st.rows)
+            with _weights_follow():
+                full = self.model.step(st.batch, self.store, st.rows)
         if not want:
             return None
         return full.index_select(0, torch.tensor(want, dtype=torch.int64).to("cuda", non_blocking=True))

@@ -83,6 +83,26 @@ def test_a_product_of_rows_that_the_call_in_front_made(name, T, link):
         assert (out - want).abs().max().item() <= 1e-4 * want.abs().max().item()  # (split K may add its parts in any order)
 
 
+def test_the_engine_takes_its_promise_back():
+    """Products of a model's step have weights behind them and say so; a step that fails must not leave that said."""
+    from paligemma_multimodal_system_b200.engine import SequenceEngine
+
+    class Broken:
+        vocab_size, prec = 8, seq_ops.Precision(torch.bfloat16)
+
+        def cache_layout(self):
+            from paligemma_multimodal_system_b200.mixers import WindowedSoftmaxAttention
+            return [WindowedSoftmaxAttention(64, 2, 1, 32, 32, 1.0, 1e-5).cache_spec()]
+
+        def step(self, *a, **k):
+            raise RuntimeError("broken")
+
+    with pytest.raises(RuntimeError, match="broken"):
+        SequenceEngine(Broken(), 128, 1).step([("a", [1, 2], [1])])
+    for name in ("rmsnorm", "gate", "embed"):
+        test_a_product_of_rows_that_the_call_in_front_made(name, 300, False)
+
+
 def test_norm_weights_that_the_product_in_front_made():
     """w of a norm is the fp32 row of the product in front."""
     x, w = _t(2, 512, seed=5, dtype=torch.bfloat16), _t(D, 512, seed=6, dtype=torch.bfloat16, scale=512 ** -0.5)
