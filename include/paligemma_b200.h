@@ -113,6 +113,8 @@ int pg_weights_follow(int on);
 
 /* out[t,f] = sum_k x[t,k] w[f,k] in fp32 rows; few tokens and few output tiles: K is shared out over the GPU. */
 int pg_linear_f32(const void* x, long long ldx, const void* w, long long ldw, float* out, long long ldo, int tokens, int features, int K, void* stream);
+/* The same into rows that hold zeros: nothing has to be cleared where the parts of K are added up in them. */
+int pg_linear_f32_zeros(const void* x, long long ldx, const void* w, long long ldw, float* out, long long ldo, int tokens, int features, int K, void* stream);
 
 /* The encoder layers of the vision tower (modeling_siglip.py:216-263): seven launches each, issued by one call.  Weights as the entry points above take
  * them (matrices bf16, dense rows; q | k | v projections fused), x fp32 [images * patches, D] in place; hn, att bf16 [., D], qkv bf16 [., 3 D],
@@ -396,6 +398,9 @@ int pg_embed_rows(const int* tokens, const void* table, long long ld, int col0, 
  * consecutive parts and each part is divided by sqrt(mean(part^2) + eps).  x != NULL: x[t, :] += r in place (fp32 residual
  * stream); x == NULL: the bare norm.  out_act != NULL also receives the result (new residual or bare norm) in the activation
  * type -- the operand of the next matrix product. */
+/* (pg_group_rmsnorm_add_clear: and y becomes zero, for a product to sum into.) */
+int pg_group_rmsnorm_add_clear(float* y, long long ldy, const float* w, float* x, void* out_act, int rows, int D, int groups, float eps, int out_f32,
+                               void* stream);
 int pg_group_rmsnorm_add(const float* y, long long ldy, const float* w, float* x, void* out_act, int rows, int D, int groups,
                          float eps, int out_f32, void* stream);
 

@@ -43,6 +43,7 @@ SIGNATURES = {
     "pg_gemm_residual": [p, i64, p, i64, p, i64, p, i32, i32, i32, f32, p],
     "pg_weights_follow": [i32],
     "pg_linear_f32": [p, i64, p, i64, p, i64, i32, i32, i32, p],
+    "pg_linear_f32_zeros": [p, i64, p, i64, p, i64, i32, i32, i32, p],
     "pg_siglip_layers": [p, i32, p, p, p, p, p, i32, i32, i32, i32, i32, f32, p],
     "pg_gemma_prefill_layers": [p, i32, p, p],
     "pg_gemm_qkv_rope": [p, i64, p, i64, p, i64, i32, i32, i32, i32, i32, p, p, p, p, p, p, i32, i32, i32, p],
@@ -72,6 +73,7 @@ SIGNATURES = {
     "pg_gemm_simt": [p, i64, p, i64, p, i64, i32, i32, i32, i32, i32, p],
     "pg_embed_rows": [p, p, i64, i32, p, p, i32, i32, f32, i32, p],
     "pg_group_rmsnorm_add": [p, i64, p, p, p, i32, i32, i32, f32, i32, p],
+    "pg_group_rmsnorm_add_clear": [p, i64, p, p, p, i32, i32, i32, f32, i32, p],
     "pg_rmsnorm_gate": [p, p, p, i64, p, i32, i32, f32, i32, p],
     "pg_geglu": [p, i64, p, i64, i32, i32, i32, p],
     "pg_gemm_fp32_scratch": [i32, i32, i32],

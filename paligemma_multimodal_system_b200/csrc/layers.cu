@@ -37,8 +37,7 @@ extern "C" int pg_gemm_residual(const void* x, long long ldx, const void* w, lon
   return pg_gemm_bf16(x, ldx, w, ldw, h, ldh, bias, nullptr, 0, tokens, features, K, PG_EPI_ATOMIC_F32, 0, scale, swap, split < 1 ? 1 : split, stream);
 }
 
-extern "C" int pg_linear_f32(const void* x, long long ldx, const void* w, long long ldw, float* out, long long ldo, int tokens, int features, int K,
-                             void* stream) {
+static int linear_f32(const void* x, long long ldx, const void* w, long long ldw, float* out, long long ldo, int tokens, int features, int K, bool zeros, void* stream) {
   if (tokens <= 0 || features <= 0 || K <= 0 || out == nullptr) return PG_ERR_ARG;
   const int tiles = (features + 127) / 128, kb = (K + 63) / 64, swap = tokens <= 128 ? 1 : 0;
   int split = 2 * pg::num_sms() / tiles;
@@ -47,11 +46,21 @@ extern "C" int pg_linear_f32(const void* x, long long ldx, const void* w, long l
     return pg_gemm_bf16(x, ldx, w, ldw, out, ldo, nullptr, nullptr, 0, tokens, features, K, PG_EPI_F32, 0, 1.f, swap, 1, stream);
   // few tiles of a long K: split-K partials are red.add-ed into the zeroed output (one row has no pitch: any ldo goes with it)
   const size_t row = features * sizeof(float);
-  if (cudaMemset2DAsync(out, tokens == 1 ? row : ldo * sizeof(float), 0, row, tokens, reinterpret_cast<cudaStream_t>(stream)) != cudaSuccess) {
+  if (!zeros && cudaMemset2DAsync(out, tokens == 1 ? row : ldo * sizeof(float), 0, row, tokens, reinterpret_cast<cudaStream_t>(stream)) != cudaSuccess) {
     cudaGetLastError();  // do not leave a sticky error behind
     return PG_ERR_CUDA;
   }
   return pg_gemm_bf16(x, ldx, w, ldw, out, ldo, nullptr, nullptr, 0, tokens, features, K, PG_EPI_ATOMIC_F32, 0, 1.f, swap, split, stream);
+}
+
+extern "C" int pg_linear_f32(const void* x, long long ldx, const void* w, long long ldw, float* out, long long ldo, int tokens, int features, int K,
+                             void* stream) {
+  return linear_f32(x, ldx, w, ldw, out, ldo, tokens, features, K, false, stream);
+}
+
+extern "C" int pg_linear_f32_zeros(const void* x, long long ldx, const void* w, long long ldw, float* out, long long ldo, int tokens, int features, int K,
+                                   void* stream) {
+  return linear_f32(x, ldx, w, ldw, out, ldo, tokens, features, K, true, stream);
 }
 
 #define PG_TRY(call)                  \

@@ -232,8 +232,8 @@ __global__ void __launch_bounds__(256) group_rmsnorm_add_kernel(const float* __r
 // and one barrier separates the sums from the result.  What bounds it: decode steps, two round trips (48 rows of 2048
 // back to back: 4.1 -> 2.1 us); prompts, HBM (10836 rows: 70 us in either form).
 template <typename TO, int NV>
-__global__ void __launch_bounds__(256) group_rmsnorm_add_reg_kernel(const float* __restrict__ y, long long ldy, const float* __restrict__ w,
-                                                                    float* __restrict__ x, TO* __restrict__ out_act, int D, int gs, float eps, int trigger) {
+__global__ void __launch_bounds__(256) group_rmsnorm_add_reg_kernel(const float* y, long long ldy, const float* __restrict__ w,
+                                                                    float* __restrict__ x, TO* __restrict__ out_act, int D, int gs, float eps, int trigger, float* clear) {
   __shared__ float red[8 * NV];  // sums of 128 neighbouring elements
   pg::griddep_begin_if(trigger);
   const long long t = blockIdx.x;
@@ -277,6 +277,7 @@ __global__ void __launch_bounds__(256) group_rmsnorm_add_reg_kernel(const float*
       reinterpret_cast<float4*>(x + t * D)[i] = r;
     }
     if (out_act != nullptr) st_act4(out_act, t * D + 4LL * i, r);
+    if (clear != nullptr) reinterpret_cast<float4*>(clear + t * ldy)[i] = make_float4(0.f, 0.f, 0.f, 0.f);  // y itself, read above
   }
 }
 
@@ -473,8 +474,8 @@ extern "C" int pg_embed_rows(const int* tokens, const void* table, long long ld,
   PG_RET();
 }
 
-extern "C" int pg_group_rmsnorm_add(const float* y, long long ldy, const float* w, float* x, void* out_act, int rows, int D, int groups,
-                                    float eps, int out_f32, void* stream) {
+static int group_rmsnorm_add(const float* y, long long ldy, const float* w, float* x, void* out_act, int rows, int D, int groups, float eps, int out_f32, float* clear,
+                             void* stream) {
   if (rows <= 0 || D <= 0 || groups <= 0 || (D % groups) != 0 || groups > 4096) return PG_ERR_ARG;
   const size_t smem = (8 + groups) * sizeof(float);
   cudaStream_t st = PG_ST(stream);
@@ -482,7 +483,7 @@ extern "C" int pg_group_rmsnorm_add(const float* y, long long ldy, const float* 
                    ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out_act)) & 15) == 0;
   const int gs = D / groups;
   if (vec && gs % 128 == 0 && D <= 4096) {
-#define PG_GNR(TO, NV) pg::launch_dependent(group_rmsnorm_add_reg_kernel<TO, NV>, rows, 256, 0, st, y, ldy, w, x, static_cast<TO*>(out_act), D, gs, eps, pg::weights_follow())
+#define PG_GNR(TO, NV) pg::launch_dependent(group_rmsnorm_add_reg_kernel<TO, NV>, rows, 256, 0, st, y, ldy, w, x, static_cast<TO*>(out_act), D, gs, eps, pg::weights_follow(), clear)
     if (out_f32) {
       if (D <= 1024) PG_GNR(float, 1); else if (D <= 2048) PG_GNR(float, 2); else PG_GNR(float, 4);
     } else {
@@ -491,6 +492,7 @@ extern "C" int pg_group_rmsnorm_add(const float* y, long long ldy, const float* 
 #undef PG_GNR
     PG_RET();
   }
+  if (clear != nullptr) return 1;
   if (out_f32) {
     if (vec) pg::launch_dependent(group_rmsnorm_add_kernel<float, true>, rows, 256, smem, st, y, ldy, w, x, static_cast<float*>(out_act), D, groups, eps);
     else pg::launch_dependent(group_rmsnorm_add_kernel<float, false>, rows, 256, smem, st, y, ldy, w, x, static_cast<float*>(out_act), D, groups, eps);
@@ -499,6 +501,24 @@ extern "C" int pg_group_rmsnorm_add(const float* y, long long ldy, const float* 
     else pg::launch_dependent(group_rmsnorm_add_kernel<bf16, false>, rows, 256, smem, st, y, ldy, w, x, static_cast<bf16*>(out_act), D, groups, eps);
   }
   PG_RET();
+}
+
+extern "C" int pg_group_rmsnorm_add(const float* y, long long ldy, const float* w, float* x, void* out_act, int rows, int D, int groups,
+                                    float eps, int out_f32, void* stream) {
+  return group_rmsnorm_add(y, ldy, w, x, out_act, rows, D, groups, eps, out_f32, nullptr, stream);
+}
+
+extern "C" int pg_group_rmsnorm_add_clear(float* y, long long ldy, const float* w, float* x, void* out_act, int rows, int D, int groups,
+                                          float eps, int out_f32, void* stream) {
+  const int rc = group_rmsnorm_add(y, ldy, w, x, out_act, rows, D, groups, eps, out_f32, y, stream);
+  if (rc != 1) return rc;
+  const int rc2 = group_rmsnorm_add(y, ldy, w, x, out_act, rows, D, groups, eps, out_f32, nullptr, stream);  // the forms that do not clear
+  if (rc2 != PG_OK) return rc2;
+  if (cudaMemset2DAsync(y, rows == 1 ? D * sizeof(float) : ldy * sizeof(float), 0, D * sizeof(float), rows, PG_ST(stream)) != cudaSuccess) {
+    cudaGetLastError();  // do not leave a sticky error behind
+    return PG_ERR_CUDA;
+  }
+  return PG_OK;
 }
 
 extern "C" int pg_rmsnorm_gate(const float* o, const float* w, const void* gate, long long ldg, void* out, int rows, int D, float eps,

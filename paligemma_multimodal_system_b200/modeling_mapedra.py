@@ -157,9 +157,10 @@ class MapedraForCausalLM:
             xa = x
         for li, blk in enumerate(self.blocks):
             y = blk.mixer(xa, b, store, li, prec)
-            seq_ops.group_rmsnorm_add(y, blk.norm1_d, x, None if prec.f32 else xa, groups, eps)
+            reuse = blk.ff is not None and blk.ff.sums(b.T)
+            seq_ops.group_rmsnorm_add(y, blk.norm1_d, x, None if prec.f32 else xa, groups, eps, clear=reuse)
             if blk.ff is not None:
-                y = blk.ff(xa, b, prec)
+                y = blk.ff(xa, b, prec, zeros=y if reuse else None)
                 seq_ops.group_rmsnorm_add(y, blk.norm2_d, x, None if prec.f32 else xa, groups, eps)
             if blk.side is not None:
                 blk.side.add(xa, b, self.side_embed_d, prec, blk.side_norm_d, x, None if prec.f32 else xa, eps)

@@ -176,10 +176,11 @@ def _linear_fp32_split(x, w, out, bias, accumulate, scale):
     return True
 
 
-def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: int = ACT_NONE, bias: Optional[torch.Tensor] = None):
+def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: int = ACT_NONE, bias: Optional[torch.Tensor] = None, zeros: bool = False):
     """out[t, f] = act(sum_k x[t, k] w[f, k] + bias[f]) (bias fp32 or None).  x, w share a type (bf16 / fp32); out is bf16 or fp32.  bf16 operands go to the
     tcgen05 kernel when TMA can describe them (16-byte pitches and bases), everything else to the plain-FMA kernel.
-    act = ACT_RELU2 (relu squared; out in the operands' type): in the tensor-core kernel's bf16 epilogue, else a pass of its own."""
+    act = ACT_RELU2 (relu squared; out in the operands' type): in the tensor-core kernel's bf16 epilogue, else a pass of its own.
+    zeros: out holds zeros (a product that shares K out over the GPU need not clear it first)."""
     T, K = x.shape
     F = w.shape[0]
     assert x.dtype == w.dtype and w.shape[1] == K and out.shape[0] == T and out.shape[1] == F
@@ -191,7 +192,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: int = ACT_N
             return _lib.gemm(x, w, out, mode=_lib.EPI_BF16, act_gelu=act, swap=1 if T <= 128 else 0, bias=bias)
         if out.dtype == torch.float32 and bias is None:
             assert x.is_cuda and w.is_cuda and w.dim() == 2
-            _lib.check(_lib.lib().pg_linear_f32(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), T, F, K, _lib.stream()),
+            fn = _lib.lib().pg_linear_f32_zeros if zeros else _lib.lib().pg_linear_f32
+            _lib.check(fn(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), T, F, K, _lib.stream()),
                        "pg_linear_f32")
             return out
         return _lib.gemm(x, w, out, mode=_lib.EPI_F32 if out.dtype == torch.float32 else _lib.EPI_BF16, swap=1 if T <= 128 else 0, bias=bias)
@@ -308,13 +310,14 @@ def embed_rows(tokens, table, col0, D, scale, out_act=None):
     return out
 
 
-def group_rmsnorm_add(y, w, x, out_act, groups, eps):
-    """x += gnorm(y) * w (x fp32, in place; x None: bare norm); out_act (bf16 / fp32, may be None) gets a copy of the result."""
+def group_rmsnorm_add(y, w, x, out_act, groups, eps, clear=False):
+    """x += gnorm(y) * w (x fp32, in place; x None: bare norm); out_act (bf16 / fp32, may be None) gets a copy of the result; clear: y becomes zero."""
     rows, D = y.shape
     assert y.dtype == torch.float32 and y.stride(1) == 1 and w.dtype == torch.float32 and w.numel() == D
     assert x is None or (x.dtype == torch.float32 and x.is_contiguous() and x.shape == y.shape)
     assert out_act is None or (out_act.is_contiguous() and out_act.shape == y.shape)
-    _lib.check(_lib.lib().pg_group_rmsnorm_add(y.data_ptr(), y.stride(0), w.data_ptr(), _lib.ptr(x), _lib.ptr(out_act), rows, D, int(groups),
+    fn = _lib.lib().pg_group_rmsnorm_add_clear if clear else _lib.lib().pg_group_rmsnorm_add
+    _lib.check(fn(y.data_ptr(), y.stride(0), w.data_ptr(), _lib.ptr(x), _lib.ptr(out_act), rows, D, int(groups),
                                                float(eps), int(out_act is not None and out_act.dtype == torch.float32), _lib.stream()),
                "pg_group_rmsnorm_add")
 
