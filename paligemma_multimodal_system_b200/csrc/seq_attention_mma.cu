@@ -381,7 +381,9 @@ __global__ void __launch_bounds__(128, (DIM + VDIM <= 128) ? 4 : 2) attn_ragged_
 // P V takes its B operand from the SAME tile with ldmatrix.trans (key-major rows -> the k-pairs an m16n8k16 B fragment wants),
 // so the values are neither stored nor fetched separately; probabilities stay fp32 and enter as three bf16 terms.
 // With several key splits the (max, sum, accumulator) triples go to `partial` in the layout of pg_attn_decode and its merge
-// kernel finishes the rows.  VS > 1: the value columns are shared out over VS CTAs (each recomputes the scores; a thread's accumulators
+// kernel finishes the rows.  What bounds it: latencies -- a CTA of two warps and a few tiles -- and instructions, so the queries are requested together with the first keys, fragments come four
+// at a time and a tile of one page needs one table entry (us with the merge, 32 heads of 288 / 256, before / now: 40 tokens behind 550 .. 1100 46 / 28, 64 behind 3000 97 / 64, one 36 / 20;
+// columns of the values shared out over two warps each: 30, 72, 18).  VS > 1: the value columns are shared out over VS CTAs (each recomputes the scores; a thread's accumulators
 // stay at 128 registers for value parts up to 512 wide).
 // ---------------------------------------------------------------------------------------------------------------------
 template <int DIM, int VDIM, int KT, int VS>
@@ -405,9 +407,8 @@ __global__ void __launch_bounds__(128) attn_latent_decode_mma_kernel(const bf16*
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gq = lane >> 2, tq = lane & 3;
   for (int id = threadIdx.x; id < nrows * (DIM / 8); id += blockDim.x) {
     const int r = id / (DIM / 8), cc = id % (DIM / 8);
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (h0 + r < H) v = *reinterpret_cast<const uint4*>(q + (t * H + h0 + r) * DIM + cc * 8);
-    *reinterpret_cast<uint4*>(Qs + r * LD + cc * 8) = v;
+    if (h0 + r < H) cp_async16(Qs + r * LD + cc * 8, q + (t * H + h0) * DIM + id * 8);
+    else *reinterpret_cast<uint4*>(Qs + r * LD + cc * 8) = make_uint4(0, 0, 0, 0);
   }
   const int rl = warp * 16 + gq, rh = rl + 8;
   float oacc[NV][4];
@@ -422,6 +423,16 @@ __global__ void __launch_bounds__(128) attn_latent_decode_mma_kernel(const bf16*
   const int lm_key = (lane & 7) + ((lane >> 3) & 1) * 8, lm_col = (lane >> 4) * 8;
   auto fetch_tile = [&](int it, bf16* dst) {
     const int k0 = it * KT;
+    if (page % KT == 0) {  // the tile lies in one page (a division and a table entry for each of its pieces were more instructions than its products)
+      const bf16* src = pages + ((long long)pt[k0 / page] * page + k0 % page) * DIM;
+      const int have = min(KT, ctx + 1 - k0) * (DIM / 8);
+      for (int id = threadIdx.x; id < KT * (DIM / 8); id += blockDim.x) {
+        bf16* d = dst + id / (DIM / 8) * LD + id % (DIM / 8) * 8;
+        if (id < have) cp_async16(d, src + id * 8);  // rows of a page follow one another
+        else *reinterpret_cast<uint4*>(d) = make_uint4(0, 0, 0, 0);
+      }
+      return;
+    }
     for (int id = threadIdx.x; id < KT * (DIM / 8); id += blockDim.x) {
       const int r = id / (DIM / 8), cc = id % (DIM / 8), j = k0 + r;
       bf16* d = dst + r * LD + cc * 8;
@@ -445,15 +456,13 @@ __global__ void __launch_bounds__(128) attn_latent_decode_mma_kernel(const bf16*
 #pragma unroll 2
     for (int ks = 0; ks < KS; ++ks) {
       uint32_t a[4];
-      a[0] = *reinterpret_cast<const uint32_t*>(Qs + rl * LD + ks * 16 + 2 * tq);
-      a[1] = *reinterpret_cast<const uint32_t*>(Qs + rh * LD + ks * 16 + 2 * tq);
-      a[2] = *reinterpret_cast<const uint32_t*>(Qs + rl * LD + ks * 16 + 8 + 2 * tq);
-      a[3] = *reinterpret_cast<const uint32_t*>(Qs + rh * LD + ks * 16 + 8 + 2 * tq);
+      ldmatrix_x4(a[0], a[1], a[2], a[3], Qs + (warp * 16 + lm_key) * LD + ks * 16 + lm_col);
 #pragma unroll
-      for (int nb = 0; nb < NB; ++nb) {
-        const uint32_t b0 = *reinterpret_cast<const uint32_t*>(Ks + (nb * 8 + gq) * LD + ks * 16 + 2 * tq);
-        const uint32_t b1 = *reinterpret_cast<const uint32_t*>(Ks + (nb * 8 + gq) * LD + ks * 16 + 8 + 2 * tq);
+      for (int nb = 0; nb < NB; nb += 2) {
+        uint32_t b0, b1, b2, b3;  // keys 0-7 and 8-15 of sixteen, both halves of the depth
+        ldmatrix_x4(b0, b1, b2, b3, Ks + (nb * 8 + (lane & 7) + (lane >> 4) * 8) * LD + ks * 16 + ((lane >> 3) & 1) * 8);
         mma16816(sacc[nb], a, b0, b1);
+        mma16816(sacc[nb + 1], a, b2, b3);
       }
     }
     float mx_l = -INFINITY, mx_h = -INFINITY;
@@ -500,10 +509,10 @@ __global__ void __launch_bounds__(128) attn_latent_decode_mma_kernel(const bf16*
         uint32_t b0, b1, b2, b3;
         ldmatrix_x4_trans(b0, b1, b2, b3, vbase + np * 16);
         mma16816(oacc[2 * np], a1, b0, b1);
-        mma16816(oacc[2 * np], a2, b0, b1);
-        mma16816(oacc[2 * np], a3, b0, b1);
         mma16816(oacc[2 * np + 1], a1, b2, b3);
+        mma16816(oacc[2 * np], a2, b0, b1);
         mma16816(oacc[2 * np + 1], a2, b2, b3);
+        mma16816(oacc[2 * np], a3, b0, b1);
         mma16816(oacc[2 * np + 1], a3, b2, b3);
       }
     }
@@ -529,8 +538,7 @@ __global__ void __launch_bounds__(128) attn_latent_decode_mma_kernel(const bf16*
       if (tq == 0 && v0 == 0) { pp[0] = mrow * 0.6931471805599453f; pp[1] = lsum; }  // the merge kernel works with natural exponentials
 #pragma unroll
       for (int nv = 0; nv < NV; ++nv) {
-        pp[2 + v0 + nv * 8 + 2 * tq] = oacc[nv][2 * half];
-        pp[2 + v0 + nv * 8 + 2 * tq + 1] = oacc[nv][2 * half + 1];
+        *reinterpret_cast<float2*>(pp + 2 + v0 + nv * 8 + 2 * tq) = make_float2(oacc[nv][2 * half], oacc[nv][2 * half + 1]);  // (VDIM is even)
       }
     }
   }

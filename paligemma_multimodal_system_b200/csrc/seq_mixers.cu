@@ -708,14 +708,16 @@ __global__ void __launch_bounds__(256) attn_decode_kernel(const TA* __restrict__
   }
 }
 
-// one value column per thread up to 256 columns: the loop over the splits is a chain of dependent loads per column
-static inline int merge_threads(int vdim) { return vdim <= 64 ? 64 : vdim <= 128 ? 128 : 256; }
+// One value column per thread up to 256 columns (COLS 1), or two where rows of an even width start on 8 bytes (COLS 2).  The first 16 splits' values are requested before the factors
+// are known, so a row takes one trip to memory (factors first, then eight splits at a time: 40 tokens x 32 heads x 256 in 14 splits 14 us, 8 now).
+static inline int merge_threads(int cols) { return cols <= 64 ? 64 : cols <= 128 ? 128 : 256; }
 
-template <typename TA>
+template <typename TA, int COLS>
 __global__ void attn_decode_merge_kernel(const float* __restrict__ partial, const TA* __restrict__ gate, long long ldg, TA* __restrict__ out,
                                          const int* __restrict__ entry_row0, const int* __restrict__ entry_n, int H, int vdim, int nsplit,
                                          int gate_per_head, PgAttnScore sx) {
   pg::griddep_begin();
+  constexpr int AHEAD = 16;
   const float* sink = sx.logistic ? nullptr : sx.sink;
   const long long ldo = sx.out_ld > 0 ? sx.out_ld : (long long)H * vdim;
   const float oscale = sx.out_scale != 0.f ? sx.out_scale : 1.f;
@@ -723,8 +725,22 @@ __global__ void attn_decode_merge_kernel(const float* __restrict__ partial, cons
   if (entry_n[e] != 1) return;
   const long long t = entry_row0[e];
   const float* pp = partial + ((long long)e * H + head) * nsplit * (vdim + 2);
-  // the splits' factors once, a lane per split; then every column's loads are independent (a chain of three loads per split and column took 15.7 us for 40 tokens x 32
-  // heads x 256 in 14 splits; now 13.9)
+  auto value = [&](int s, int col, float (&v)[COLS]) {
+    const float* p = pp + s * (vdim + 2) + 2 + col;
+    if constexpr (COLS == 2) {
+      const float2 f = *reinterpret_cast<const float2*>(p);
+      v[0] = f.x;
+      v[1] = f.y;
+    } else {
+      v[0] = *p;
+    }
+  };
+  const int first = COLS * (int)threadIdx.x;
+  float ahead[AHEAD][COLS];
+#pragma unroll
+  for (int s = 0; s < AHEAD; ++s)
+    if (s < nsplit && first < vdim) value(s, first, ahead[s]);
+  // the splits' factors once, a lane per split
   __shared__ float fs[64], whole[2];
   if (threadIdx.x < 32) {
     float mx = -INFINITY, sum = 0.f;
@@ -740,23 +756,49 @@ __global__ void attn_decode_merge_kernel(const float* __restrict__ partial, cons
   }
   __syncthreads();
   const float M = whole[0];
-  for (int col = threadIdx.x; col < vdim; col += blockDim.x) {
-    float acc = 0.f, ls = whole[1];
-#pragma unroll 8
-    for (int s = 0; s < nsplit; ++s) {
+  for (int col = first; col < vdim; col += COLS * blockDim.x) {
+    float acc[COLS] = {}, ls = whole[1];
+    auto add = [&](float f, const float (&v)[COLS]) {
+#pragma unroll
+      for (int c = 0; c < COLS; ++c) acc[c] = fmaf(f, f != 0.f ? v[c] : 0.f, acc[c]);  // (a split without keys left nothing)
+    };
+#pragma unroll
+    for (int s = 0; s < AHEAD; ++s) {
+      if (s >= nsplit) break;
+      if (col != first) value(s, col, ahead[s]);
+      add(fs[s], ahead[s]);
+    }
+#pragma unroll 4
+    for (int s = AHEAD; s < nsplit; ++s) {
+      float v[COLS];
+      value(s, col, v);
       const float ms = s < 64 ? 0.f : pp[s * (vdim + 2)];
-      const float f = s < 64 ? fs[s] : ms > -INFINITY ? expf(ms - M) : 0.f;
-      acc = fmaf(f, f != 0.f ? pp[s * (vdim + 2) + 2 + col] : 0.f, acc);
+      add(s < 64 ? fs[s] : ms > -INFINITY ? expf(ms - M) : 0.f, v);
     }
     if (sink != nullptr) {
       const float sk = sink[head], mm = fmaxf(M, sk), f = expf(M - mm);
-      acc *= f;
+#pragma unroll
+      for (int c = 0; c < COLS; ++c) acc[c] *= f;
       ls = ls * f + expf(sk - mm);
     }
-    float v = (sx.logistic ? acc : acc / ls) * oscale;
-    if (gate != nullptr) v *= sigmoidf(ldf(gate, t * ldg + (gate_per_head ? (long long)head : (long long)head * vdim + col)));
-    stf(out, t * ldo + (long long)head * vdim + col, v);
+#pragma unroll
+    for (int c = 0; c < COLS; ++c) {
+      float v = (sx.logistic ? acc[c] : acc[c] / ls) * oscale;
+      if (gate != nullptr) v *= sigmoidf(ldf(gate, t * ldg + (gate_per_head ? (long long)head : (long long)head * vdim + col + c)));
+      stf(out, t * ldo + (long long)head * vdim + col + c, v);
+    }
   }
+}
+
+template <typename TA>
+static void launch_merge(const float* partial, const void* gate, long long ldg, void* out, const int* row0, const int* n, int entries, int H, int vdim, int nsplit, int gate_per_head,
+                         const PgAttnScore& sx, cudaStream_t st) {
+  const bool two = vdim % 2 == 0 && (reinterpret_cast<uintptr_t>(partial) & 7) == 0;
+  auto go = [&](auto kern, int cols) {
+    pg::launch_dependent(kern, dim3(H, entries), merge_threads(cols), 0, st, partial, static_cast<const TA*>(gate), ldg, static_cast<TA*>(out), row0, n, H, vdim, nsplit, gate_per_head, sx);
+  };
+  if (two) go(attn_decode_merge_kernel<TA, 2>, vdim / 2);
+  else go(attn_decode_merge_kernel<TA, 1>, vdim);
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -1370,8 +1412,7 @@ static int launch_attn_decode(const void* q, const void* kp, const void* vp, con
                                                      H, G, dim, vdim, scale, softcap, krow, vrow, gate_per_head, sx);
   pg_count_launch(1);
   if (nsplit > 1) {
-    pg::launch_dependent(attn_decode_merge_kernel<TA>, dim3(H, entries), merge_threads(vdim), 0, st, partial, static_cast<const TA*>(gate), ldg, static_cast<TA*>(out), row0, n, H, vdim, nsplit,
-                                                                  gate_per_head, sx);
+    launch_merge<TA>(partial, gate, ldg, out, row0, n, entries, H, vdim, nsplit, gate_per_head, sx, st);
     pg_count_launch(1);
   }
   return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
@@ -1382,12 +1423,8 @@ extern "C" int pg_attn_decode_merge(const float* partial, const void* gate, long
   if (entries <= 0 || entries > 65535 || nsplit <= 0 || H <= 0 || vdim <= 0 || partial == nullptr) return PG_ERR_ARG;
   cudaStream_t st = PG_ST(stream);
   const PgAttnScore sx = score != nullptr ? *score : PgAttnScore{};
-  if (act_f32)
-    pg::launch_dependent(attn_decode_merge_kernel<float>, dim3(H, entries), merge_threads(vdim), 0, st, partial, static_cast<const float*>(gate), ldg, static_cast<float*>(out), entry_row0, entry_n,
-                                                                     H, vdim, nsplit, gate_per_head, sx);
-  else
-    pg::launch_dependent(attn_decode_merge_kernel<bf16>, dim3(H, entries), merge_threads(vdim), 0, st, partial, static_cast<const bf16*>(gate), ldg, static_cast<bf16*>(out), entry_row0, entry_n, H,
-                                                                    vdim, nsplit, gate_per_head, sx);
+  if (act_f32) launch_merge<float>(partial, gate, ldg, out, entry_row0, entry_n, entries, H, vdim, nsplit, gate_per_head, sx, st);
+  else launch_merge<bf16>(partial, gate, ldg, out, entry_row0, entry_n, entries, H, vdim, nsplit, gate_per_head, sx, st);
   PG_RET();
 }
 
