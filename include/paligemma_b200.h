@@ -487,6 +487,11 @@ int pg_attn_ragged_mma(const void* q, const void* k_pages, const void* v_pages, 
                        const int* entry_row0, const int* entry_n, const int* entry_ctx, const int* page_table, int max_pages, int page,
                        int entries, int max_n, int H, int G, int dim, int vdim, float scale, float softcap, int skip_single,
                        int gate_per_head, const PgAttnScore* score, void* stream);
+/* The same with what the host knows of the batch: how many entries have rows for this kernel, and the longest context with its new tokens among them. */
+int pg_attn_ragged_mma_sized(const void* q, const void* k_pages, const void* v_pages, const void* gate, long long ldg, void* out,
+                       const int* entry_row0, const int* entry_n, const int* entry_ctx, const int* page_table, int max_pages, int page,
+                       int entries, int max_n, int H, int G, int dim, int vdim, float scale, float softcap, int skip_single,
+                       int gate_per_head, int portions, int longest, const PgAttnScore* score, void* stream);
 int pg_attn_decode(const void* q, const void* k_pages, const void* v_pages, const void* gate, long long ldg, void* out, float* partial,
                    const int* entry_row0, const int* entry_n, const int* entry_ctx, const int* page_table, int max_pages, int page,
                    int entries, int nsplit, int H, int G, int dim, int vdim, float scale, float softcap, int act_f32, long long krow,

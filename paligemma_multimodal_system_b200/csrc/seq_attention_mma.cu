@@ -27,7 +27,7 @@ using bf16 = __nv_bfloat16;
 // seq_attention_tc.cu
 int pg_attn_ragged_tc(const void* q, const void* kp, const void* vp, const void* gate, long long ldg, void* out, const int* row0, const int* n, const int* ctx, const int* pt,
                       int max_pages, int page, int entries, int max_n, int H, int G, int dim, int vdim, float scale, float softcap, int skip_single, int gate_per_head,
-                      const PgAttnScore& sx, cudaStream_t st);
+                      int portions, int longest, const PgAttnScore& sx, cudaStream_t st);
 
 namespace {
 
@@ -584,10 +584,10 @@ int launch(const void* q, const void* kp, const void* vp, const void* gate, long
 
 }  // namespace
 
-extern "C" int pg_attn_ragged_mma(const void* q, const void* k_pages, const void* v_pages, const void* gate, long long ldg, void* out,
+static int attn_ragged_mma(const void* q, const void* k_pages, const void* v_pages, const void* gate, long long ldg, void* out,
                                   const int* entry_row0, const int* entry_n, const int* entry_ctx, const int* page_table, int max_pages, int page,
                                   int entries, int max_n, int H, int G, int dim, int vdim, float scale, float softcap, int skip_single, int gate_per_head,
-                                  const PgAttnScore* score, void* stream) {
+                                  int portions, int longest, const PgAttnScore* score, void* stream) {
   if (entries <= 0 || max_n <= 0 || H <= 0 || G <= 0 || (H % G) != 0 || entries > 65535 || G > 65535) return PG_ERR_ARG;
   if (score != nullptr && ((score->dist_a == nullptr) != (score->dist_b == nullptr))) return PG_ERR_ARG;
   const PgAttnScore sx = score != nullptr ? *score : PgAttnScore{};
@@ -599,7 +599,7 @@ extern "C" int pg_attn_ragged_mma(const void* q, const void* k_pages, const void
     return PG_ERR_ARG;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int rc = pg_attn_ragged_tc(q, k_pages, v_pages, gate, ldg, out, entry_row0, entry_n, entry_ctx, page_table, max_pages, page, entries, max_n, H, G, dim, vdim, scale,
-                                   softcap, skip_single, gate_per_head, sx, st);
+                                   softcap, skip_single, gate_per_head, portions, longest, sx, st);
   if (rc != 1) return rc;
 #define PG_MMA(D, V) \
   if (dim == D && vdim == V) \
@@ -614,6 +614,20 @@ extern "C" int pg_attn_ragged_mma(const void* q, const void* k_pages, const void
   PG_MMA(128, 64);
 #undef PG_MMA
   return PG_ERR_ARG;  // other head sizes: pg_attn_ragged
+}
+
+extern "C" int pg_attn_ragged_mma(const void* q, const void* k_pages, const void* v_pages, const void* gate, long long ldg, void* out,
+                                  const int* entry_row0, const int* entry_n, const int* entry_ctx, const int* page_table, int max_pages, int page,
+                                  int entries, int max_n, int H, int G, int dim, int vdim, float scale, float softcap, int skip_single, int gate_per_head,
+                                  const PgAttnScore* score, void* stream) {
+  return attn_ragged_mma(q, k_pages, v_pages, gate, ldg, out, entry_row0, entry_n, entry_ctx, page_table, max_pages, page, entries, max_n, H, G, dim, vdim, scale, softcap, skip_single, gate_per_head, 0, 0, score, stream);
+}
+
+extern "C" int pg_attn_ragged_mma_sized(const void* q, const void* k_pages, const void* v_pages, const void* gate, long long ldg, void* out,
+                                  const int* entry_row0, const int* entry_n, const int* entry_ctx, const int* page_table, int max_pages, int page,
+                                  int entries, int max_n, int H, int G, int dim, int vdim, float scale, float softcap, int skip_single, int gate_per_head,
+                                  int portions, int longest, const PgAttnScore* score, void* stream) {
+  return attn_ragged_mma(q, k_pages, v_pages, gate, ldg, out, entry_row0, entry_n, entry_ctx, page_table, max_pages, page, entries, max_n, H, G, dim, vdim, scale, softcap, skip_single, gate_per_head, portions, longest, score, stream);
 }
 
 extern "C" int pg_attn_latent_decode_mma(const void* q, const void* pages, const void* gate, long long ldg, void* out, float* partial,

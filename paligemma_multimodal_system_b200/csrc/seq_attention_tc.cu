@@ -17,8 +17,10 @@
 //     instead cost every prompt: 8 x 1024 tokens 140 -> 147 us; the check 142.)
 // What bounds it: the softmax warps (MUFU 512 clocks a tile and warp, logic and permutes for the split 450, two warps on each pipe) and, with few tiles a CTA, its start (entry, page
 // table, first tile: each a trip to memory).  Two threads a row share the same pipes, exponentials as polynomials on the FMA pipe cost more than they save.
+// SPLIT: two CTAs of a cluster share a block's keys out, half of its tiles each, and the second hands its maxima, sums and O over through its shared memory, where the blocks are too few
+// for the SMs (a portion of 128 tokens behind 1500, 32 blocks: 28 us, 21 so).
 // us, mma.sync / here: 8 prompts of 897 .. 1024 tokens, 32 heads x 64 over 8 k/v heads 235 / 103; 2 portions of 333
-// tokens behind 1400, 32 heads x 96 / 64: 144 / 58 (with P beside S, every tile waiting for P V of the one before, and query rows copied one piece after the other: 142 and 65;
+// tokens behind 1400, 32 heads x 96 / 64: 144 / 49 (with P beside S, every tile waiting for P V of the one before, and query rows copied one piece after the other: 142 and 65;
 // there a CTA of eight tiles spent 6500 of 31700 clocks before its first barrier).
 #include <string.h>
 
@@ -156,21 +158,21 @@ __device__ __noinline__ void row_from_visible_keys(const bf16* __restrict__ q, c
   }
 }
 
-template <int DIM, int VDIM>
+template <int DIM, int VDIM, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                                                                      const __grid_constant__ CUtensorMap tmV,
                                                                      const bf16* __restrict__ q, const bf16* __restrict__ k_pages, const bf16* __restrict__ v_pages,
                                                                      const bf16* __restrict__ gate, long long ldg, bf16* __restrict__ out,
                                                                      const int* __restrict__ entry_row0, const int* __restrict__ entry_n, const int* __restrict__ entry_ctx,
                                                                      const int* __restrict__ page_table, int max_pages, int page, int H, int G, float scale, float softcap,
-                                                                     int skip_single, int gate_per_head, int q_tma, int entries, PgAttnScore sx) {
+                                                                     int skip_single, int gate_per_head, int q_tma, int entries, int units, PgAttnScore sx) {
   using C = Shape<DIM, VDIM>;
   constexpr uint32_t IDESC_S = make_idesc_bf16(128, 64), IDESC_O = make_idesc_bf16(128, VDIM, 0, 1);
   griddep_wait();
   // The longest rows of all entries and heads come first (48 prompts of 193 .. 256 tokens, soft-capped: 243 us entry by entry, 198 so).  Where single tokens are left to another
-  // kernel, the entries with rows are counted and numbered first, so that CTAs without any stand at the end and not between two blocks of rows (2 portions + 40 singles, 4032
-  // CTAs of which 192 have rows: 58 us entry by entry, 71 with the 2700 empty ones of the first two blocks in front of the third).
-  const unsigned idx = blockIdx.x, blocks = gridDim.x / static_cast<unsigned>(entries * G);
+  // kernel, the entries with rows are counted and numbered first, so that CTAs without any stand at the end and not between two blocks of rows; where the host has counted them (`units`)
+  // there are none (2 portions + 40 singles, 192 CTAs with rows: 49 us, 60 with 3840 empty ones behind them, 71 with 2700 in front of the third block).
+  const unsigned idx = SPLIT ? blockIdx.x / 2 : blockIdx.x, blocks = (SPLIT ? gridDim.x / 2 : gridDim.x) / static_cast<unsigned>(units * G);
   unsigned with_rows = entries;
   if (skip_single) {
     with_rows = 0;
@@ -263,11 +265,11 @@ __global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __gri
   const int window = sx.window > 0 ? sx.window : 0x3fffffff, keep = sx.window > 0 ? max(sx.keep_first, 0) : 0;
   const int keep_end = (keep + 63) & ~63, cta_lo = max(0, ctx + r0 / gsz - window + 1) & ~63;
   // key tiles wholly between the kept first keys and the first key inside the window of the CTA's first row are skipped
-  auto next_tile = [&](int k) {
-    const int nx = k + 64;
-    return (nx >= keep_end && nx < cta_lo) ? cta_lo : nx;
-  };
-  const int k_first = next_tile(-64);
+  const bool gap = cta_lo > keep_end;
+  const int before = keep_end / 64, tiles = gap ? before + (kmax - cta_lo) / 64 + 1 : kmax / 64 + 1;
+  auto key_of = [&](int i) { return gap && i >= before ? cta_lo + 64 * (i - before) : 64 * i; };
+  const int rank = SPLIT ? static_cast<int>(cluster_ctarank()) : 0, half = (tiles + 1) / 2;
+  const int t0 = SPLIT && rank ? half : 0, t1 = SPLIT && !rank ? half : tiles;  // this CTA's tiles (the second of a cluster may have none)
 
   if (warp == 0) {
     if (lane == 0) {
@@ -276,30 +278,29 @@ __global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __gri
       uint32_t phase = 0;
       const int piece = min(page, 64);  // rows of a box: a tile is (part of) a page, or several pages (those past the last key are left out)
       auto row_at = [&](int key) { return pt[key / page] * page + key % page; };
-      int first = row_at(k_first);
-      for (int k0 = k_first; k0 <= kmax;) {
-        const int nx = next_tile(k0), pieces = min(64, kmax + 1 - k0 + piece - 1) / piece;
+      int first = t0 < t1 ? row_at(key_of(t0)) : 0;
+      for (int i = t0; i < t1; ++i) {
+        const int k0 = key_of(i), pieces = min(64, kmax + 1 - k0 + piece - 1) / piece;
         int row = first;
-        if (nx <= kmax) first = row_at(nx);
+        if (i + 1 < t1) first = row_at(key_of(i + 1));
         const uint32_t sk = kv0 + stage * C::KV_BYTES;
         mbar_wait(kv_empty(stage), phase ^ 1);
         mbar_expect_tx(kv_full(stage), (C::KB + C::VB) * 128 * piece * pieces);
-        for (int i = 0; i < pieces; ++i) {
-          if (i > 0) row = row_at(k0 + i * piece);
-          const uint32_t dst = sk + i * piece * 128;
+        for (int part = 0; part < pieces; ++part) {
+          if (part > 0) row = row_at(k0 + part * piece);
+          const uint32_t dst = sk + part * piece * 128;
 #pragma unroll
           for (int b = 0; b < C::KB; ++b) tma_load_2d(dst + b * kBox, &tmK, kv_full(stage), g * DIM + 64 * b, row, kEvictNormal);
 #pragma unroll
           for (int b = 0; b < C::VB; ++b) tma_load_2d(dst + (C::KB + b) * kBox, &tmV, kv_full(stage), g * VDIM + 64 * b, row, kEvictNormal);
         }
         if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
-        k0 = nx;
       }
     }
     __syncwarp();
   } else if (warp == 1) {
     // tile j: S in area j % NBUF, its P over it; S of tile j + NBUF behind P V of tile j, whose area it takes (one thread's products run in order)
-    int stage = 0, ahead = 0, ks = k_first, js = 0;  // stages of P V and of S; key and number of the next S
+    int stage = 0, ahead = 0, js = 0;  // stages of P V and of S; number of the next S
     uint32_t ahead_phase = 0;
     auto issue_s = [&]() {
       mbar_wait(kv_full(ahead), ahead_phase);
@@ -313,14 +314,13 @@ __global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __gri
       }
       __syncwarp();
       if (++ahead == C::STAGES) { ahead = 0; ahead_phase ^= 1; }
-      ks = next_tile(ks);
       ++js;
     };
     if (by_tma) mbar_wait(q_full, 0);
     for (int b = 0; b < C::NBUF; ++b)
-      if (ks <= kmax) issue_s();
-    int j = 0;
-    for (int k0 = k_first; k0 <= kmax; k0 = next_tile(k0), ++j) {
+      if (t0 + js < t1) issue_s();
+    for (int j = 0; t0 + j < t1; ++j) {
+      const int k0 = key_of(t0 + j);
       const uint32_t sv = kv0 + stage * C::KV_BYTES + C::KB * kBox, area = tmem + 96 * (j % C::NBUF);
       if (k0 + 63 > kmax) {  // the last tile: keys nobody sees weigh zero, whatever lies there
         for (int r = kmax + 1 - k0 + lane; r < 64; r += 32)
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __gri
         umma_commit(o_done(j & 1));
       }
       __syncwarp();
-      if (ks <= kmax) issue_s();
+      if (t0 + js < t1) issue_s();
       if (++stage == C::STAGES) stage = 0;
     }
   } else {
@@ -361,7 +361,8 @@ __global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __gri
     const float unit = plain ? scale * kLog2e : kLog2e, in = softcap > 0.f ? sc / softcap : 0.f;
     float m = -INFINITY, l = 0.f;
     int j = 0;
-    for (int k0 = k_first; k0 <= kmax; k0 = next_tile(k0), ++j) {
+    for (; t0 + j < t1; ++j) {
+      const int k0 = key_of(t0 + j);
       const uint32_t area = lanes + 96 * (j % C::NBUF);
       mbar_wait(s_full(j % C::NBUF), (j / C::NBUF) & 1);
       tc_fence_after();
@@ -452,67 +453,122 @@ __global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __gri
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full(j & 1));
     }
-    mbar_wait(o_done((j - 1) & 1), ((j - 1) >> 1) & 1);
-    tc_fence_after();
-    float osc = 1.f;
-    if (sx.sink != nullptr) {  // the sink joins the denominator once (m is in base-2 units)
-      const float sk = sx.sink[head] * kLog2e, mm = fmaxf(m, sk);
-      osc = exp2f(m - mm);
-      l = l * osc + exp2f(sk - mm);
+    if (!SPLIT || j > 0) {
+      mbar_wait(o_done((j - 1) & 1), ((j - 1) >> 1) & 1);
+      tc_fence_after();
     }
-    const float inv = osc / l * (sx.out_scale != 0.f ? sx.out_scale : 1.f);
-    const long long t = row0 + (there ? rr / gsz : 0), ldo = sx.out_ld > 0 ? sx.out_ld : static_cast<long long>(H) * VDIM;
-    bf16* o = out + t * ldo + static_cast<long long>(head) * VDIM;
-    const bf16* gt = gate == nullptr ? nullptr : gate + t * ldg + (gate_per_head ? static_cast<long long>(head) : static_cast<long long>(head) * VDIM);
-    bool odd = false;  // a sum of the row is not finite
-    const float gh = gate != nullptr && gate_per_head ? 1.0f / (1.0f + expf(-__bfloat162float(*gt))) : 1.f;
+    // SPLIT: the second CTA's maxima, sums and O of its 128 rows lie over its key tiles, [4 columns][row] and then [2][row]
+    float own = 1.f, other = 0.f;  // factors of this CTA's and the other's sums
+    uint32_t far = 0;
+    if constexpr (SPLIT) {
+      const uint32_t at = kv0 + r * 16, tail = kv0 + VDIM * 128 * 4 + r * 4;
+      if (rank == 1) {
 #pragma unroll 1
-    for (int c0 = 0; c0 < VDIM; c0 += 64) {
-      uint32_t all[4][16];
+        for (int c = 0; c < VDIM; c += 16) {
+          uint32_t v[16] = {};
+          if (j > 0) {
+            tmem_ld16(lanes + C::COL_O + c, v);
+            tmem_ld_wait();
+          }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) tmem_ld16(lanes + C::COL_O + c0 + 16 * i, all[i]);
-      tmem_ld_wait();
-#pragma unroll
-      for (int part = 0; part < 4; ++part) {
-        if (!there) break;
-        const int c = c0 + 16 * part;
-        const uint32_t(&v)[16] = all[part];
-        float x[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          odd = odd || (v[i] & 0x7f800000u) == 0x7f800000u;
-          x[i] = __uint_as_float(v[i]) * inv;
+          for (int i = 0; i < 4; ++i)
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at + (c / 4 + i) * 2048), "r"(v[4 * i]), "r"(v[4 * i + 1]), "r"(v[4 * i + 2]), "r"(v[4 * i + 3]) : "memory");
         }
-        if (gate != nullptr) {
-          if (gate_per_head) {
+        asm volatile("st.shared.f32 [%0], %1;" ::"r"(tail), "f"(m) : "memory");
+        asm volatile("st.shared.f32 [%0], %1;" ::"r"(tail + 512), "f"(l) : "memory");
+      }
+      cluster_sync_all();
+      if (rank == 0) {
+        uint32_t there_m;
+        float m2, l2;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, 1;" : "=r"(far) : "r"(at));
+        asm volatile("mapa.shared::cluster.u32 %0, %1, 1;" : "=r"(there_m) : "r"(tail));
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(m2) : "r"(there_m) : "memory");
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(l2) : "r"(there_m + 512) : "memory");
+        const float mm = fmaxf(m, m2);
+        own = ex2(m - mm);
+        other = ex2(m2 - mm);  // no key seen there: 0
+        l = l * own + l2 * other;
+        m = mm;
+      }
+    }
+    if (!SPLIT || rank == 0) {
+      float osc = 1.f;
+      if (sx.sink != nullptr) {  // the sink joins the denominator once (m is in base-2 units)
+        const float sk = sx.sink[head] * kLog2e, mm = fmaxf(m, sk);
+        osc = exp2f(m - mm);
+        l = l * osc + exp2f(sk - mm);
+      }
+      const float inv = osc / l * (sx.out_scale != 0.f ? sx.out_scale : 1.f);
+      const long long t = row0 + (there ? rr / gsz : 0), ldo = sx.out_ld > 0 ? sx.out_ld : static_cast<long long>(H) * VDIM;
+      bf16* o = out + t * ldo + static_cast<long long>(head) * VDIM;
+      const bf16* gt = gate == nullptr ? nullptr : gate + t * ldg + (gate_per_head ? static_cast<long long>(head) : static_cast<long long>(head) * VDIM);
+      bool odd = false;  // a sum of the row is not finite
+      const float gh = gate != nullptr && gate_per_head ? 1.0f / (1.0f + expf(-__bfloat162float(*gt))) : 1.f;
+#pragma unroll 1
+      for (int c0 = 0; c0 < VDIM; c0 += 64) {
+        uint32_t all[4][16];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) x[i] *= gh;
-          } else {
+        for (int i = 0; i < 4; ++i) tmem_ld16(lanes + C::COL_O + c0 + 16 * i, all[i]);
+        tmem_ld_wait();
+        if constexpr (SPLIT) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const float2 gg = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(gt + c)[i]);
-              x[2 * i] *= 1.0f / (1.0f + expf(-gg.x));
-              x[2 * i + 1] *= 1.0f / (1.0f + expf(-gg.y));
-            }
+          for (int i = 0; i < 16; ++i) {
+            float4 o2;
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(o2.x), "=f"(o2.y), "=f"(o2.z), "=f"(o2.w) : "r"(far + (c0 / 4 + i) * 2048) : "memory");
+            uint32_t* v = &all[i / 4][i % 4 * 4];
+            v[0] = __float_as_uint(fmaf(__uint_as_float(v[0]), own, o2.x * other));
+            v[1] = __float_as_uint(fmaf(__uint_as_float(v[1]), own, o2.y * other));
+            v[2] = __float_as_uint(fmaf(__uint_as_float(v[2]), own, o2.z * other));
+            v[3] = __float_as_uint(fmaf(__uint_as_float(v[3]), own, o2.w * other));
           }
         }
-        uint4* d = reinterpret_cast<uint4*>(o + c);
-        d[0] = make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
-        d[1] = make_uint4(pack_bf16(x[8], x[9]), pack_bf16(x[10], x[11]), pack_bf16(x[12], x[13]), pack_bf16(x[14], x[15]));
+#pragma unroll
+        for (int part = 0; part < 4; ++part) {
+          if (!there) break;
+          const int c = c0 + 16 * part;
+          const uint32_t(&v)[16] = all[part];
+          float x[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            odd = odd || (v[i] & 0x7f800000u) == 0x7f800000u;
+            x[i] = __uint_as_float(v[i]) * inv;
+          }
+          if (gate != nullptr) {
+            if (gate_per_head) {
+#pragma unroll
+              for (int i = 0; i < 16; ++i) x[i] *= gh;
+            } else {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const float2 gg = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(gt + c)[i]);
+                x[2 * i] *= 1.0f / (1.0f + expf(-gg.x));
+                x[2 * i + 1] *= 1.0f / (1.0f + expf(-gg.y));
+              }
+            }
+          }
+          uint4* d = reinterpret_cast<uint4*>(o + c);
+          d[0] = make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
+          d[1] = make_uint4(pack_bf16(x[8], x[9]), pack_bf16(x[10], x[11]), pack_bf16(x[12], x[13]), pack_bf16(x[14], x[15]));
+        }
+        __syncwarp();
       }
-      __syncwarp();
-    }
-    for (unsigned left = __ballot_sync(0xffffffffu, odd); left != 0; left &= left - 1) {
-      const int row = r0 + qd * 32 + __ffs(left) - 1, hd = g * gsz + row % gsz, last = ctx + row / gsz;
-      const long long tk = row0 + row / gsz;
-      row_from_visible_keys<DIM, VDIM>(q + (tk * H + hd) * DIM, k_pages + static_cast<long long>(g) * DIM, v_pages + static_cast<long long>(g) * VDIM,
-                                       page_table + static_cast<long long>(e) * max_pages, page, static_cast<long long>(G) * DIM, static_cast<long long>(G) * VDIM, last, last - window + 1, keep,
-                                       scale * (sx.head_scale != nullptr ? sx.head_scale[hd] : 1.f), softcap, sx.sink != nullptr ? sx.sink + hd : nullptr,
-                                       sx.out_scale != 0.f ? sx.out_scale : 1.f,
-                                       gate == nullptr ? nullptr : gate + tk * ldg + (gate_per_head ? static_cast<long long>(hd) : static_cast<long long>(hd) * VDIM), gate_per_head,
-                                       out + tk * ldo + static_cast<long long>(hd) * VDIM);
+      for (unsigned left = __ballot_sync(0xffffffffu, odd); left != 0; left &= left - 1) {
+        const int row = r0 + qd * 32 + __ffs(left) - 1, hd = g * gsz + row % gsz, last = ctx + row / gsz;
+        const long long tk = row0 + row / gsz;
+        row_from_visible_keys<DIM, VDIM>(q + (tk * H + hd) * DIM, k_pages + static_cast<long long>(g) * DIM, v_pages + static_cast<long long>(g) * VDIM,
+                                         page_table + static_cast<long long>(e) * max_pages, page, static_cast<long long>(G) * DIM, static_cast<long long>(G) * VDIM, last, last - window + 1, keep,
+                                         scale * (sx.head_scale != nullptr ? sx.head_scale[hd] : 1.f), softcap, sx.sink != nullptr ? sx.sink + hd : nullptr,
+                                         sx.out_scale != 0.f ? sx.out_scale : 1.f,
+                                         gate == nullptr ? nullptr : gate + tk * ldg + (gate_per_head ? static_cast<long long>(hd) : static_cast<long long>(hd) * VDIM), gate_per_head,
+                                         out + tk * ldo + static_cast<long long>(hd) * VDIM);
+      }
     }
     tc_fence_before();
+  }
+  if constexpr (SPLIT) {
+    if (warp < 2) cluster_sync_all();  // the second CTA's sums are there
+    cluster_sync_all();                // and have been read
   }
   __syncthreads();
   if (warp == 1) {
@@ -521,17 +577,17 @@ __global__ void __launch_bounds__(kThreads, 2) attn_ragged_tc_kernel(const __gri
   }
 }
 
-template <int DIM, int VDIM>
+template <int DIM, int VDIM, bool SPLIT>
 int launch(const void* q, const void* kp, const void* vp, const void* gate, long long ldg, void* out, const int* row0, const int* n, const int* ctx, const int* pt,
-           int max_pages, int page, int entries, int max_n, int H, int G, float scale, float softcap, int skip_single, int gate_per_head, const PgAttnScore& sx,
+           int max_pages, int page, int entries, int units, int max_n, int H, int G, float scale, float softcap, int skip_single, int gate_per_head, const PgAttnScore& sx,
            cudaStream_t st) {
   using C = Shape<DIM, VDIM>;
-  const long long ctas = (static_cast<long long>(max_n) * (H / G) + 127) / 128 * G * entries;
-  if (ctas > 0x7fffffff) return 1;
+  const long long ctas = (static_cast<long long>(max_n) * (H / G) + 127) / 128 * G * units;
+  if ((SPLIT ? 2 * ctas : ctas) > 0x7fffffff) return 1;
   static bool configured[kMaxDevices] = {};
   const int dev = current_device();
   if (!configured[dev]) {
-    if (cudaFuncSetAttribute(attn_ragged_tc_kernel<DIM, VDIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess) {
+    if (cudaFuncSetAttribute(attn_ragged_tc_kernel<DIM, VDIM, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess) {
       cudaGetLastError();
       return PG_ERR_CUDA;
     }
@@ -552,9 +608,19 @@ int launch(const void* q, const void* kp, const void* vp, const void* gate, long
   int rc;
   if ((rc = make_tmap_2d(&tk, kp, 1LL << 30, static_cast<long long>(G) * DIM, static_cast<long long>(G) * DIM, page < 64 ? page : 64)) != PG_OK) return rc;
   if ((rc = make_tmap_2d(&tv, vp, 1LL << 30, static_cast<long long>(G) * VDIM, static_cast<long long>(G) * VDIM, page < 64 ? page : 64)) != PG_OK) return rc;
-  launch_spread(attn_ragged_tc_kernel<DIM, VDIM>, dim3(static_cast<unsigned>(ctas)), dim3(kThreads), C::SMEM, st, tq, tk, tv, static_cast<const bf16*>(q),
-                static_cast<const bf16*>(kp), static_cast<const bf16*>(vp), static_cast<const bf16*>(gate), ldg, static_cast<bf16*>(out), row0, n, ctx, pt, max_pages, page, H, G,
-                scale, softcap, skip_single, gate_per_head, q_tma, entries, sx);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(SPLIT ? 2 * ctas : ctas));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = C::SMEM;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = SPLIT ? 1 : 0;  // (behind the whole of the kernel before, as launch_spread)
+  cudaLaunchKernelEx(&cfg, attn_ragged_tc_kernel<DIM, VDIM, SPLIT>, tq, tk, tv, static_cast<const bf16*>(q), static_cast<const bf16*>(kp), static_cast<const bf16*>(vp),
+                     static_cast<const bf16*>(gate), ldg, static_cast<bf16*>(out), row0, n, ctx, pt, max_pages, page, H, G, scale, softcap, skip_single, gate_per_head, q_tma, entries, units, sx);
   pg_count_launch(1);
   return cudaGetLastError() == cudaSuccess ? PG_OK : PG_ERR_CUDA;
 }
@@ -565,7 +631,7 @@ int launch(const void* q, const void* kp, const void* vp, const void* gate, long
 // Launches the call when it is one of this file's (PG_OK or an error), else returns 1.  Everything that pg_attn_ragged_mma checks has been checked.
 int pg_attn_ragged_tc(const void* q, const void* kp, const void* vp, const void* gate, long long ldg, void* out, const int* row0, const int* n, const int* ctx, const int* pt,
                       int max_pages, int page, int entries, int max_n, int H, int G, int dim, int vdim, float scale, float softcap, int skip_single, int gate_per_head,
-                      const PgAttnScore& sx, cudaStream_t st) {
+                      int portions, int longest, const PgAttnScore& sx, cudaStream_t st) {
   // pages that a tile of 64 keys divides, or that divide it in whole swizzle rows
   if (!(page > 0 && (page % 64 == 0 || (page % 8 == 0 && 64 % page == 0))) || sx.logistic || sx.dist_a != nullptr || sx.out_ld % 8 != 0) return 1;
   // Blocks of 128 rows do not pay for a handful of rows in more CTAs than SMs (the mma.sync kernel's warps without rows idle; us, mma.sync / here, 16 heads of 64: 16 x 8 tokens
@@ -573,14 +639,25 @@ int pg_attn_ragged_tc(const void* q, const void* kp, const void* vp, const void*
   // wave (16 heads: 400 tokens behind 2000 74 / 82, 200 tokens 12.7 / 15.4; 4 x 200 tokens, 256 CTAs, behind 500 41 / 29).
   const long long rows = static_cast<long long>(max_n) * (H / G), units = static_cast<long long>(G) * entries;
   if ((rows <= 16 && units > pg::num_sms()) || (dim == 64 && vdim == 128 && (rows + 63) / 64 * units <= pg::num_sms())) return 1;
-#define PG_TC(D, V) \
-  if (dim == D && vdim == V) \
-    return pg::launch<D, V>(q, kp, vp, gate, ldg, out, row0, n, ctx, pt, max_pages, page, entries, max_n, H, G, scale, softcap, skip_single, gate_per_head, sx, st)
+  // Two CTAs a block where the blocks are too few for the SMs and long enough to share out (portions and longest: entries with rows and the longest context with its new tokens, 0 where
+  // the caller does not know; us, one CTA / two: 80 blocks of 24 .. 28 tiles 38 / 31, 32 of 24 .. 26 28 / 21, 64 of 16 40 / 35, 96 of 26 of 96 / 64 37 / 33; but 160 blocks of 24 .. 28
+  // 40 / 41, 192 of 26 49 / 51, 128 of up to 8 15.6 / 16.5).
+  const long long blocks = (rows + 127) / 128 * G * portions;
+  const int reach = sx.window > 0 ? (longest < sx.window + (sx.keep_first > 0 ? sx.keep_first : 0) + 128 ? longest : sx.window + (sx.keep_first > 0 ? sx.keep_first : 0) + 128) : longest;
+  const bool split = vdim == 64 && portions > 0 && 4 * blocks <= 3LL * pg::num_sms() && reach >= 12 * 64;
+#define PG_TC1(D, V, S) return pg::launch<D, V, S>(q, kp, vp, gate, ldg, out, row0, n, ctx, pt, max_pages, page, entries, portions > 0 && portions < entries ? portions : entries, max_n, H, G, scale, softcap, \
+                                                   skip_single, gate_per_head, sx, st)
+#define PG_TC(D, V)                  \
+  if (dim == D && vdim == V) {       \
+    if (V == 64 && split) PG_TC1(D, V, (V == 64)); \
+    PG_TC1(D, V, false);             \
+  }
   PG_TC(64, 64);
   PG_TC(96, 64);
   PG_TC(128, 128);
   PG_TC(64, 128);
   PG_TC(128, 64);
+#undef PG_TC1
 #undef PG_TC
   return 1;
 }

@@ -442,9 +442,10 @@ def attn_ragged(q, k_pages, v_pages, gate, out, b: StepBatch, H, G, dim, vdim, s
         pass
     elif (singles < b.E and tensor_cores and not f32 and dense_rows and (dim, vdim) in MMA_HEAD_SIZES
             and (gate is None or gph or (ldg % 2 == 0 and gate.data_ptr() % 4 == 0))):
-        _lib.check(L.pg_attn_ragged_mma(q.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), _lib.ptr(gate), ldg, out.data_ptr(), b.row0.data_ptr(),
+        _lib.check(L.pg_attn_ragged_mma_sized(q.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), _lib.ptr(gate), ldg, out.data_ptr(), b.row0.data_ptr(),
                                         b.n.data_ptr(), b.ctx.data_ptr(), b.page_table.data_ptr(), b.max_pages, page, b.E, b.max_n, H, G, dim, vdim,
-                                        float(scale), float(softcap or 0.0), int(singles > 0), gph, sx, _lib.stream()), "pg_attn_ragged_mma")
+                                        float(scale), float(softcap or 0.0), int(singles > 0), gph, b.E - singles, b.dense_max_len, sx, _lib.stream()),
+                   "pg_attn_ragged_mma_sized")
     elif singles < b.E:
         _lib.check(L.pg_attn_ragged(q.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), _lib.ptr(gate), ldg, out.data_ptr(), b.row0.data_ptr(),
                                     b.n.data_ptr(), b.ctx.data_ptr(), b.page_table.data_ptr(), b.max_pages, page, b.E, b.max_n, H, G, dim, vdim,

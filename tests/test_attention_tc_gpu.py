@@ -59,6 +59,15 @@ def test_either_side_of_a_handful_of_rows(n):
     _run(64, 64, 40, 4, (n, 2, n, 1), (70, 0, 300, 5), 0, 0)  # 16 and 20 rows in 160 CTAs
 
 
+@pytest.mark.parametrize("dim,vdim,G,gsz", [(64, 64, 2, 4), (96, 64, 3, 1), (128, 64, 1, 5)])
+@pytest.mark.parametrize("ns,ctxs", [((130, 1, 3), (1000, 5, 0)), ((300,), (500,)), ((2, 65), (511, 800)), ((790,), (0,))])
+@pytest.mark.parametrize("window,keep", [(0, 0), (700, 5), (600, 130), (64, 1000)])
+@pytest.mark.parametrize("opts", [dict(), dict(softcap=3.0, hs=True, sink=True, gate="row", big=True)])
+def test_keys_shared_out_over_two_ctas(dim, vdim, G, gsz, ns, ctxs, window, keep, opts):
+    """Few blocks with many tiles: odd and even halves, blocks of a single tile whose second CTA has none, halves on both sides of the gap in front of a window."""
+    _run(dim, vdim, G, gsz, ns, ctxs, window, keep, **opts)
+
+
 @pytest.mark.parametrize("dim,vdim,G,gsz", [(64, 64, 2, 4), (96, 64, 3, 1), (128, 128, 1, 2)])
 @pytest.mark.parametrize("at", [0, 31, 32, 69])
 def test_portions_among_many_single_tokens(dim, vdim, G, gsz, at):
@@ -115,9 +124,10 @@ def _run(dim, vdim, G, gsz, ns, ctxs, window, keep, softcap=0.0, hs=False, sink=
 @pytest.mark.parametrize("dim,vdim,G,gsz,window,keep", [(64, 64, 2, 4, 0, 0), (64, 64, 1, 1, 0, 0), (128, 128, 1, 4, 0, 0), (96, 64, 2, 1, 70, 0), (64, 128, 16, 2, 33, 40),
                                                         (128, 64, 1, 129, 0, 0), (64, 64, 3, 2, 90, 5)])
 @pytest.mark.parametrize("opts", [dict(), dict(softcap=5.0, hs=True, sink=True, gate="head", ld=True), dict(gate="row")])
-def test_values_that_are_not_finite(dim, vdim, G, gsz, window, keep, opts, bad):
+@pytest.mark.parametrize("n", [300, 800])
+def test_values_that_are_not_finite(dim, vdim, G, gsz, window, keep, opts, bad, n):
     """A broken value reaches the rows that see it and no others: not those before it in their block, nor those whose window begins behind it."""
-    n, ctx, at = 300, 30, 207
+    ctx, at = 30, 207
     H, L, softcap = G * gsz, ctx + n, opts.get("softcap", 0.0)
     b = seq_ops.make_step_batch([dict(tokens=[1] * n, ctx=ctx, slot=0, pages=list(range((L + 63) // 64)))])
     kp, vp = (_t((L + 63) // 64, 64, G * d, seed=s) for d, s in ((dim, 2), (vdim, 3)))
