@@ -273,6 +273,12 @@ int pg_merge_scan(const long long* input_ids, const long long* attn_mask, int* p
                   int B, int S, int N, long long image_token, long long pad_token, void* stream);
 int pg_merge_text(const long long* input_ids, const int* src_scratch, const void* embed, float* h, int B, int S, int D, int N,
                   float text_scale, void* stream);
+/* The two halves with the input checks inside: pg_prompt_scan writes flags[b] (1: the row does not hold N image tokens, 2: an id outside [0, vocab)) and all of dst_row (B * S: no
+ * slot); pg_prompt_text fills rows of ids outside with zeros and, first_row != NULL, copies the merged row of every row's first image feature to first_row[b] (fp32 [B, D]). */
+int pg_prompt_scan(const long long* input_ids, const long long* attn_mask, int* pos, int* src_scratch, int* dst_row, int* flags, int B, int S, int N,
+                   long long vocab, long long image_token, long long pad_token, void* stream);
+int pg_prompt_text(const long long* input_ids, const int* src_scratch, const int* dst_row, const void* embed, float* h, float* first_row, int B, int S, int D, int N,
+                   long long vocab, float text_scale, void* stream);
 
 /* Decode-step embedding with the same merge rules at q_len = 1; tokens are int32 on the device; img may be NULL. */
 int pg_embed_tokens(const int* tokens, const void* embed, const float* img, float* h, int B, int D, int N,

@@ -61,6 +61,8 @@ SIGNATURES = {
     "pg_kv_gather": [p, p, p, i32, i32, i32, i32, i32, i32, p],
     "pg_merge_embeddings": [p, p, p, p, p, p, p, p, i32, i32, i32, i32, i64, i64, f32, f32, p],
     "pg_merge_scan": [p, p, p, p, p, p, i32, i32, i32, i64, i64, p],
+    "pg_prompt_scan": [p, p, p, p, p, p, i32, i32, i32, i64, i64, i64, p],
+    "pg_prompt_text": [p, p, p, p, p, p, i32, i32, i32, i32, i64, f32, p],
     "pg_merge_text": [p, p, p, p, i32, i32, i32, i32, f32, p],
     "pg_embed_tokens": [p, p, p, p, i32, i32, i32, f32, f32, i64, i64, p],
     "pg_argmax": [p, i64, p, i32, i32, p],

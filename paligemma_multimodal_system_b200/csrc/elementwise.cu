@@ -247,14 +247,19 @@ __global__ void pack_gate_up_kernel(const bf16* __restrict__ gate, const bf16* _
 // ---------------------------------------------------------------------------------------------------------
 // embedding merge (modeling_paligemma.py:93-128,195,288; modeling_gemma.py:510-511)
 // ---------------------------------------------------------------------------------------------------------
-// pass 1: one block per batch row; src[b,s] = j >= 0 (j-th image token) | -1 text | -2 pad; pos = cumsum(mask), 1 at mask==0
+// pass 1: one block per batch row; src[b,s] = j >= 0 (j-th image token) | -1 text | -2 pad; pos = cumsum(mask), 1 at mask==0.
+// vocab > 0: every row has a flag of its own, written and not raised (1: not N image tokens, 2: an id outside the vocabulary), and dst_row starts out as B * S everywhere -- nothing has
+// to be cleared in front, and the host can look at the flags while the tower still runs.
 __global__ void __launch_bounds__(1024) merge_scan_kernel(const long long* __restrict__ ids, const long long* __restrict__ mask,
                                                           int* __restrict__ src, int* __restrict__ pos, int* __restrict__ err,
                                                           int* __restrict__ dst_row, int S, int N, long long image_token,
-                                                          long long pad_token) {
+                                                          long long pad_token, long long vocab) {
   pg::griddep_begin();
   __shared__ int wsum_img[32], wsum_msk[32];
   __shared__ int carry_img, carry_msk;
+  int outside = 0;
+  if (vocab > 0)
+    for (int j = threadIdx.x; j < N; j += blockDim.x) dst_row[static_cast<long long>(blockIdx.x) * N + j] = gridDim.x * S;
   const int b = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) { carry_img = 0; carry_msk = 0; }
@@ -263,6 +268,7 @@ __global__ void __launch_bounds__(1024) merge_scan_kernel(const long long* __res
     const int s = base + threadIdx.x;
     long long id = 0, mk = 0;
     if (s < S) { id = ids[static_cast<long long>(b) * S + s]; mk = mask[static_cast<long long>(b) * S + s]; }
+    outside |= s < S && (id < 0 || id >= vocab);
     const int is_img = (s < S && id == image_token) ? 1 : 0;
     const int mv = (s < S) ? static_cast<int>(mk) : 0;
     int xi = is_img, xm = mv;  // inclusive warp scans
@@ -286,21 +292,34 @@ __global__ void __launch_bounds__(1024) merge_scan_kernel(const long long* __res
     if (threadIdx.x == blockDim.x - 1) { carry_img = oi + xi; carry_msk = om + xm; }
     __syncthreads();
   }
-  if (threadIdx.x == 0 && carry_img != N) atomicExch(err, 1);
+  if (vocab > 0) {
+    outside = __syncthreads_or(outside);
+    if (threadIdx.x == 0) err[b] = (carry_img != N ? 1 : 0) | (outside ? 2 : 0);
+  } else if (threadIdx.x == 0 && carry_img != N) {
+    atomicExch(err, 1);
+  }
 }
 
-// pass 2: one block per token
+// pass 2: one block per token; first_row != nullptr: and one per batch row, which copies the merged row of its first image feature there.  vocab > 0: ids outside are rows of zeros
+// (their flag is up), not rows outside the table
 __global__ void __launch_bounds__(256) merge_gather_kernel(const long long* __restrict__ ids, const int* __restrict__ src,
                                                            const bf16* __restrict__ embed, const float* __restrict__ img,
                                                            float* __restrict__ h, int S, int D, int N, float text_scale,
-                                                           float img_scale, int skip_image) {
+                                                           float img_scale, int skip_image, int B, const int* __restrict__ dst_row,
+                                                           float* __restrict__ first_row, long long vocab) {
   pg::griddep_begin();
   const long long tok = blockIdx.x;
+  if (tok >= static_cast<long long>(B) * S) {
+    const long long row = tok - static_cast<long long>(B) * S;
+    const float4* from = reinterpret_cast<const float4*>(h + static_cast<long long>(min(dst_row[row * N], B * S - 1)) * D);
+    for (int i = threadIdx.x; i < D / 4; i += blockDim.x) reinterpret_cast<float4*>(first_row + row * D)[i] = from[i];
+    return;
+  }
   const int b = static_cast<int>(tok / S);
   const int sidx = src[tok];
   float4* dst = reinterpret_cast<float4*>(h + tok * D);
   if (sidx >= 0 && skip_image) return;  // the projector GEMM has written this row (pg_gemm_bf16_fused out_row_map)
-  if (sidx == -2) {
+  if (sidx == -2 || (vocab > 0 && sidx == -1 && (ids[tok] < 0 || ids[tok] >= vocab))) {
     for (int i = threadIdx.x; i < D / 4; i += blockDim.x) dst[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   } else if (sidx >= 0) {
     const int j = sidx < N ? sidx : N - 1;  // (err flag already raised when counts mismatch)
@@ -552,18 +571,33 @@ extern "C" int pg_merge_embeddings(const long long* input_ids, const long long* 
                                    long long image_token, long long pad_token, float text_scale, float img_scale,
                                    void* stream) {
   if (B <= 0 || S <= 0 || D <= 0 || (D % 4)) return PG_ERR_ARG;
-  pg::launch_dependent(merge_scan_kernel, B, 1024, 0, PG_ST(stream), input_ids, attn_mask, src_scratch, pos, err_flag, nullptr, S, N, image_token, pad_token);
+  pg::launch_dependent(merge_scan_kernel, B, 1024, 0, PG_ST(stream), input_ids, attn_mask, src_scratch, pos, err_flag, nullptr, S, N, image_token, pad_token, 0LL);
   if (cudaGetLastError() != cudaSuccess) return PG_ERR_CUDA;
   pg_count_launch(1);
   pg::launch_dependent(merge_gather_kernel, B * S, 256, 0, PG_ST(stream), input_ids, src_scratch, static_cast<const bf16*>(embed), img, h, S, D, N,
-                                                        text_scale, img_scale, 0);
+                                                        text_scale, img_scale, 0, B, nullptr, nullptr, 0LL);
   PG_RET();
 }
 
 extern "C" int pg_merge_scan(const long long* input_ids, const long long* attn_mask, int* pos, int* src_scratch, int* dst_row,
                              int* err_flag, int B, int S, int N, long long image_token, long long pad_token, void* stream) {
   if (B <= 0 || S <= 0 || N < 0 || !input_ids || !attn_mask || !pos || !src_scratch || !err_flag) return PG_ERR_ARG;
-  pg::launch_dependent(merge_scan_kernel, B, 1024, 0, PG_ST(stream), input_ids, attn_mask, src_scratch, pos, err_flag, dst_row, S, N, image_token, pad_token);
+  pg::launch_dependent(merge_scan_kernel, B, 1024, 0, PG_ST(stream), input_ids, attn_mask, src_scratch, pos, err_flag, dst_row, S, N, image_token, pad_token, 0LL);
+  PG_RET();
+}
+
+extern "C" int pg_prompt_scan(const long long* input_ids, const long long* attn_mask, int* pos, int* src_scratch, int* dst_row, int* flags, int B, int S, int N,
+                              long long vocab, long long image_token, long long pad_token, void* stream) {
+  if (B <= 0 || S <= 0 || N < 0 || vocab <= 0 || !input_ids || !attn_mask || !pos || !src_scratch || !dst_row || !flags) return PG_ERR_ARG;
+  pg::launch_dependent(merge_scan_kernel, B, 1024, 0, PG_ST(stream), input_ids, attn_mask, src_scratch, pos, flags, dst_row, S, N, image_token, pad_token, vocab);
+  PG_RET();
+}
+
+extern "C" int pg_prompt_text(const long long* input_ids, const int* src_scratch, const int* dst_row, const void* embed, float* h, float* first_row, int B, int S, int D, int N,
+                              long long vocab, float text_scale, void* stream) {
+  if (B <= 0 || S <= 0 || D <= 0 || (D % 4) || vocab <= 0 || !input_ids || !src_scratch || !embed || !h || (first_row != nullptr && (N <= 0 || !dst_row))) return PG_ERR_ARG;
+  pg::launch_dependent(merge_gather_kernel, B * S + (first_row != nullptr ? B : 0), 256, 0, PG_ST(stream), input_ids, src_scratch, static_cast<const bf16*>(embed), nullptr, h, S, D, N,
+                       text_scale, 0.f, 1, B, dst_row, first_row, vocab);
   PG_RET();
 }
 
@@ -571,7 +605,7 @@ extern "C" int pg_merge_text(const long long* input_ids, const int* src_scratch,
                              int N, float text_scale, void* stream) {
   if (B <= 0 || S <= 0 || D <= 0 || (D % 4) || !input_ids || !src_scratch || !embed || !h) return PG_ERR_ARG;
   pg::launch_dependent(merge_gather_kernel, B * S, 256, 0, PG_ST(stream), input_ids, src_scratch, static_cast<const bf16*>(embed), nullptr, h, S, D, N,
-                                                        text_scale, 0.f, 1);
+                                                        text_scale, 0.f, 1, B, nullptr, nullptr, 0LL);
   PG_RET();
 }
 

@@ -35,6 +35,7 @@ class KVCache:
         self.v_pages = None
         self.page_table = None
         self.counters = None  # int32 [3, B]: pos, slot, kv_len  (device)
+        self._first_slot = None  # int32 [B] of zeros beside them
         self.image_feats = None  # projected image features of the request (decode-time <image> token parity): [B, n >= 1, D]
         self.image_feats_scaled = False  # True: the rows already carry hidden_size**-0.5 * sqrt(hidden) (written by _embed_prompt)
         self._len = 0
@@ -88,10 +89,10 @@ class KVCache:
     def allocate(self, B, layers, Hkv, dh, capacity_tokens):
         max_pages = (capacity_tokens + PAGE - 1) // PAGE
         self._geom = (B, layers, Hkv, dh)
-        self.k_pages = torch.zeros(layers, B * max_pages, PAGE, Hkv * dh, device="cuda", dtype=torch.bfloat16)
-        self.v_pages = torch.zeros_like(self.k_pages)
+        self.k_pages, self.v_pages = torch.zeros(2, layers, B * max_pages, PAGE, Hkv * dh, device="cuda", dtype=torch.bfloat16).unbind(0)
         self.page_table = torch.arange(B * max_pages, device="cuda", dtype=torch.int32).view(B, max_pages).contiguous()
-        self.counters = torch.zeros(3, B, device="cuda", dtype=torch.int32)
+        counters = torch.zeros(4, B, device="cuda", dtype=torch.int32)
+        self.counters, self._first_slot = counters[:3], counters[3]  # (the prompt's first slot of every row: 0)
         self._layer_len = []
         self._len = 0
 
@@ -297,7 +298,7 @@ class GemmaForCausalLM(nn.Module):
             if kv_cache._geom is None or kv_cache._geom != (B, c.num_hidden_layers, Hkv, dh):
                 kv_cache.allocate(B, c.num_hidden_layers, Hkv, dh, S + max(kv_cache.reserve_tokens, reserve_tokens))
             kv_cache.ensure_capacity(S + 1)
-            slot_base = torch.zeros(B, device=dev, dtype=torch.int32)
+            slot_base = kv_cache._first_slot if kv_cache._first_slot is not None else torch.zeros(B, device=dev, dtype=torch.int32)
             page_table = kv_cache.page_table
         W = (Hq + 2 * Hkv) * dh
         hn = torch.empty(T, D, device=dev, dtype=torch.bfloat16)

@@ -144,7 +144,7 @@ class PaliGemmaForConditionalGeneration(nn.Module):
         (modeling_paligemma.py:57-65) writes its rows, times hidden_size**-0.5 * sqrt(hidden) (:288 and modeling_gemma.py:510-511),
         straight to their `<image>` positions through its epilogue's row map, and a gather fills the text / pad rows.  No fp32
         [B, N, D] image-feature tensor exists.  Returns h fp32 [B*S, D], pos int32 [B*S] (+ the device error flag when
-        validate=False: CUDA-graph capture).  first_image_row [B, 1, D] receives every request's first projected, scaled feature row
+        validate=False: CUDA-graph capture: flags for _raise_flags).  first_image_row [B, 1, D] receives every request's first projected, scaled feature row
         (what a decode step needs when the sampled token is `<image>`, modeling_paligemma.py:116-121)."""
         L, lm = _lib.lib(), self.language_model
         pk = lm._packed or lm.pack()
@@ -155,30 +155,40 @@ class PaliGemmaForConditionalGeneration(nn.Module):
         dev = torch.device("cuda")
         ids = input_ids.to(device=dev, dtype=torch.int64).contiguous()
         mask = attention_mask.to(device=dev).to(torch.int64).contiguous()
-        if validate and bool(((ids < 0) | (ids >= V)).any()):
-            raise IndexError("input_ids out of range for the embedding table")
-        feats = self.vision_tower.forward_features(pixel_values, out_bf16=True)  # [B*N, Dv] bf16
-        N = feats.shape[0] // B
-        h = torch.empty(B * S + 1, D, device=dev, dtype=torch.float32)  # (+ one sink row for features without a slot)
+        # The scan and its flags come first: the host reads them while the tower runs, and nothing in front of the decoder waits for the GPU to be idle.
+        N = pixel_values.shape[0] * self.vision_tower.patches_per_image // B
         pos = torch.empty(B * S, device=dev, dtype=torch.int32)
         src = torch.empty(B * S, device=dev, dtype=torch.int32)
-        dst = torch.full((B * N,), B * S, device=dev, dtype=torch.int32)
-        err = torch.zeros(1, device=dev, dtype=torch.int32)
-        _lib.check(L.pg_merge_scan(ids.data_ptr(), mask.data_ptr(), pos.data_ptr(), src.data_ptr(), dst.data_ptr(), err.data_ptr(), B, S, N,
-                                   self.dummy_image_token_id, self.pad_token_id, _lib.stream()), "pg_merge_scan")
+        dst = torch.empty(B * N, device=dev, dtype=torch.int32)
+        flags = torch.empty(B, device=dev, dtype=torch.int32)
+        _lib.check(L.pg_prompt_scan(ids.data_ptr(), mask.data_ptr(), pos.data_ptr(), src.data_ptr(), dst.data_ptr(), flags.data_ptr(), B, S, N, V,
+                                    self.dummy_image_token_id, self.pad_token_id, _lib.stream()), "pg_prompt_scan")
+        if validate:
+            seen = torch.empty(B, dtype=torch.int32, pin_memory=True)
+            seen.copy_(flags, non_blocking=True)
+            there = torch.cuda.Event()
+            there.record()
+        feats = self.vision_tower.forward_features(pixel_values, out_bf16=True)  # [B*N, Dv] bf16
+        h = torch.empty(B * S + 1, D, device=dev, dtype=torch.float32)  # (+ one sink row for features without a slot)
         img_scale = (self.config.projection_dim ** -0.5) * (D ** 0.5)
         _lib.gemm(feats, self._proj_w, h, mode=_lib.EPI_F32, bias=self._proj_b, scale=img_scale, swap=0,
                   out_row_map=dst)
         h = h[: B * S]
-        _lib.check(L.pg_merge_text(ids.data_ptr(), src.data_ptr(), pk["embed"].data_ptr(), h.data_ptr(), B, S, D, N, D ** 0.5,
-                                   _lib.stream()), "pg_merge_text")
-        if first_image_row is not None:
-            first_image_row.view(B, D).copy_(h.index_select(0, dst.view(B, N)[:, 0].clamp(max=B * S - 1).long()))
+        _lib.check(L.pg_prompt_text(ids.data_ptr(), src.data_ptr(), dst.data_ptr(), pk["embed"].data_ptr(), h.data_ptr(), _lib.ptr(first_image_row), B, S, D, N, V, D ** 0.5,
+                                    _lib.stream()), "pg_prompt_text")
         if not validate:
-            return h, pos, err
-        if int(err.item()) != 0:
-            raise ValueError(f"every row of input_ids must hold exactly {N} image tokens (id {self.dummy_image_token_id})")
+            return h, pos, flags
+        there.synchronize()
+        self._raise_flags(seen, N)
         return h, pos
+
+    def _raise_flags(self, flags, N):
+        """flags: what pg_prompt_scan left for every row (on the host)."""
+        flags = flags.tolist()
+        if any(f & 2 for f in flags):
+            raise IndexError("input_ids out of range for the embedding table")
+        if any(flags):
+            raise ValueError(f"every row of input_ids must hold exactly {N} image tokens (id {self.dummy_image_token_id})")
 
     @torch.no_grad()
     def _decode_step(self, tokens_i32, kv_cache, bufs, B, inv_temperature=1.0):
@@ -260,12 +270,10 @@ class PaliGemmaForConditionalGeneration(nn.Module):
 
     def _prefill_graphed(self, stt, kv, input_ids, pixel_values, attention_mask, B, S, V):
         """Prefill of generate() through a CUDA graph (captured at the second call of a geometry; the first runs eagerly so
-        that lazy kernel attributes and the KV allocation exist).  Input validation keeps the eager path's errors: the id
-        range is checked before the launch, the image-token count flag right after the replay."""
+        that lazy kernel attributes and the KV allocation exist).  Input validation keeps the eager path's errors: the flags of the id
+        range and of the image-token count are read right after the replay."""
         lm, dev = self.language_model, torch.device("cuda")
         ids = input_ids.to(device=dev, dtype=torch.int64).contiguous()
-        if bool(((ids < 0) | (ids >= V)).any()):
-            raise IndexError("input_ids out of range for the embedding table")
         N = self.text_config.num_image_tokens
 
         def run(ids_t, mask_t, px_t):
@@ -293,8 +301,7 @@ class PaliGemmaForConditionalGeneration(nn.Module):
                 pf["graph"] = g
             pf["graph"].replay()
             logits, err = pf["logits"], pf["err"]
-        if int(err.item()) != 0:
-            raise ValueError(f"every row of input_ids must hold exactly {N} image tokens (id {self.dummy_image_token_id})")
+        self._raise_flags(err.cpu(), N)
         return logits
 
     @torch.no_grad()

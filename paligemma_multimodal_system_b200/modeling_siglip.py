@@ -143,6 +143,10 @@ class SiglipVisionModel(nn.Module):
         return pk
 
     # -- compute -------------------------------------------------------------------------------------------------
+    @property
+    def patches_per_image(self):
+        return (self.config.image_size // self.config.patch_size) ** 2
+
     @torch.no_grad()
     def forward_features(self, pixel_values, out_bf16=False):
         """Returns the post-LN features as a flat [B*N, hidden] tensor (fp32, or bf16 for the projector GEMM)."""
