@@ -24,3 +24,27 @@ def test_widths(D):
     _lib.rmsnorm(x, w, y, eps)
     want = xd / torch.sqrt((xd * xd).mean(-1, keepdim=True) + eps) * (1 + w.double())
     assert ((y.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -16).all()
+
+
+@pytest.mark.parametrize("rows", [1, 300])
+@pytest.mark.parametrize("D", [4, 100, 128, 1152, 2044, 2048, 2052, 4096, 5000, 8192])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_few_rows(rows, D, shift):
+    """A row in a block's registers, and weights off 16 bytes: in shared memory."""
+    from paligemma_multimodal_system_b200 import _lib
+    eps = 1e-6
+    g = torch.Generator(device="cuda").manual_seed(D)
+    x = torch.randn(rows, D, generator=g, device="cuda") * 3 + 0.5
+    w, b = (torch.randn(D + 1, generator=g, device="cuda")[shift:][:D] for _ in range(2))
+    y, f = torch.empty(rows, D, device="cuda", dtype=torch.bfloat16), torch.empty(rows, D, device="cuda")
+    xd = x.double()
+    m = xd.mean(-1, keepdim=True)
+    want = (xd - m) / torch.sqrt(((xd - m) ** 2).mean(-1, keepdim=True) + eps) * w.double() + b.double()
+    _lib.check(_lib.lib().pg_layernorm(x.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr(), f.data_ptr(), rows, D, eps, _lib.stream()), "pg_layernorm")
+    # as above; a row of four values may lie near its mean: its variance carries the error of the mean, 2^-22 of the row's values
+    tol = 2.0 ** -19 * 5 if D > 4 else 2.0 ** -12
+    assert ((f.double() - want).abs() <= tol * (1 + want.abs())).all()
+    assert ((y.double() - want).abs() <= 2.0 ** -8 * want.abs() + tol).all()
+    _lib.check(_lib.lib().pg_rmsnorm(x.data_ptr(), w.data_ptr(), y.data_ptr(), rows, D, eps, _lib.stream()), "pg_rmsnorm")
+    want = xd / torch.sqrt((xd * xd).mean(-1, keepdim=True) + eps) * (1 + w.double())
+    assert ((y.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -16).all()
