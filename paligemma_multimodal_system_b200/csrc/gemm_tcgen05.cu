@@ -1036,8 +1036,11 @@ __host__ __device__ constexpr int pair_stage_bytes(int BN) { return A_TILE_BYTES
 __host__ __device__ constexpr int pair_stages(int BN) { return (232448 - 256 - 8 * 4096) / pair_stage_bytes(BN); }        // 6 / 6
 __host__ __device__ constexpr int pair_smem(int BN) { return pair_stages(BN) * pair_stage_bytes(BN) + 8 * 4096 + 256; }
 
+// a second warp that issues loads, behind the epilogue's
+__host__ __device__ constexpr int pair_threads(bool epi8) { return (epi8 ? 320 : NUM_THREADS) + 32; }
+
 template <int BN, bool EPI8, bool ROPE>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(EPI8 ? 320 : NUM_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads(EPI8), 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB, const GemmArgs args) {
   constexpr int STAGES = pair_stages(BN), STAGE_BYTES = pair_stage_bytes(BN);
   constexpr int NEPI = EPI8 ? 8 : 4;
@@ -1085,8 +1088,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr_gen;
 
-  if (warp == 0) {
-    // =================================== TMA producer (both CTAs) ===================================
+  if (warp == 0 || warp == NEPI + 2) {
+    // =================================== TMA producers (both CTAs) ==================================
+    // Two warps, every other stage each (a stage keeps one producer: it has seen every earlier phase of the barrier that it waits on): one turns a stage around in about
+    // 290 ns, the pair's UMMAs read it in 270 at full clocks.  8192 tokens, 1152 x 1152 26.0 -> 25.7 us, 1152 x 4304 60.1 -> 59.2, 4304 x 1152 68.6 -> 67.3; products under the
+    // power cap (32768 x 2048) are as before, and so are the few-token kernels with two producers (48 x 16384 x 2048 15.4 / 15.1, 64 x 2048 x 8192 41.5 / 42.6)
+    const int mine = warp == 0 ? 0 : 1;
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
@@ -1096,15 +1103,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
       const uint64_t hintA = kEvictNormal;
       const uint64_t hintB = args.n_fast == 1 ? kEvictLast : kEvictNormal;
       griddep_wait();
-      griddep_launch_dependents();
+      if (mine == 0) griddep_launch_dependents();
       for (int tile = pair; tile < num_tiles; tile += num_pairs) {
         const TileInfo t = decode_tile(tile, m_blocks, n_blocks, total_kb, 1, args.n_fast);
         for (int kb = t.kb0; kb < t.kb1; ++kb) {
-          const uint32_t sa = smem_base + stage * STAGE_BYTES;
-          mbar_wait(empty_bar(stage), phase ^ 1);
-          if (leader) mbar_expect_tx(full_bar(stage), 2 * STAGE_BYTES);
-          tma_load_2d_pair(sa, &tmapA, full_bar(stage), kb * BK, (2 * t.m_blk + rank) * BM, hintA);
-          tma_load_2d_pair(sa + A_TILE_BYTES, &tmapB, full_bar(stage), kb * BK, t.n_blk * BN + rank * (BN / 2), hintB);
+          if (stage % 2 == mine) {
+            const uint32_t sa = smem_base + stage * STAGE_BYTES;
+            mbar_wait(empty_bar(stage), phase ^ 1);
+            if (leader) mbar_expect_tx(full_bar(stage), 2 * STAGE_BYTES);
+            tma_load_2d_pair(sa, &tmapA, full_bar(stage), kb * BK, (2 * t.m_blk + rank) * BM, hintA);
+            tma_load_2d_pair(sa + A_TILE_BYTES, &tmapB, full_bar(stage), kb * BK, t.n_blk * BN + rank * (BN / 2), hintB);
+          }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
@@ -1182,7 +1191,7 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmA
   }
   const int pairs = num_sms() / 2;
   const int grid = 2 * (num_tiles < pairs ? num_tiles : pairs);
-  return launch_kernel(gemm_pair_kernel<BN, EPI8, ROPE>, dim3(grid), dim3(EPI8 ? 320 : NUM_THREADS), pair_smem(BN), st, ta, tb, a) == cudaSuccess
+  return launch_kernel(gemm_pair_kernel<BN, EPI8, ROPE>, dim3(grid), dim3(pair_threads(EPI8)), pair_smem(BN), st, ta, tb, a) == cudaSuccess
              ? PG_OK : PG_ERR_CUDA;
 }
 
