@@ -366,8 +366,8 @@ __global__ void __launch_bounds__(256) rmsnorm_gate_reg_kernel(const float* __re
 
 // out[t, f] = gelu_tanh(gu[t, f]) * gu[t, F + f]    (unfused gate || up product: the exact-precision path)
 template <typename TA>
-__global__ void geglu_kernel(const TA* __restrict__ gu, long long ldgu, TA* __restrict__ out, long long ldo, int F, long long total) {
-  pg::griddep_begin();
+__global__ void geglu_kernel(const TA* __restrict__ gu, long long ldgu, TA* __restrict__ out, long long ldo, int F, long long total, int trigger) {
+  pg::griddep_begin_if(trigger);
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const long long t = i / F;
@@ -553,9 +553,9 @@ extern "C" int pg_geglu(const void* gu, long long ldgu, void* out, long long ldo
   const long long total = (long long)rows * F;
   const unsigned blocks = (unsigned)((total + 255) / 256);
   if (act_f32)
-    pg::launch_dependent(geglu_kernel<float>, blocks, 256, 0, PG_ST(stream), static_cast<const float*>(gu), ldgu, static_cast<float*>(out), ldo, F, total);
+    pg::launch_dependent(geglu_kernel<float>, blocks, 256, 0, PG_ST(stream), static_cast<const float*>(gu), ldgu, static_cast<float*>(out), ldo, F, total, pg::weights_follow());
   else
-    pg::launch_dependent(geglu_kernel<bf16>, blocks, 256, 0, PG_ST(stream), static_cast<const bf16*>(gu), ldgu, static_cast<bf16*>(out), ldo, F, total);
+    pg::launch_dependent(geglu_kernel<bf16>, blocks, 256, 0, PG_ST(stream), static_cast<const bf16*>(gu), ldgu, static_cast<bf16*>(out), ldo, F, total, pg::weights_follow());
   PG_RET();
 }
 

@@ -29,6 +29,7 @@ struct Fp32Args {
   int accumulate;
   float scale;
   const int* only_if;  // not NULL: a flag on the device that has to be set for anything to be computed (gemm_fp32_split.cu)
+  int early;  // rows kernel: nothing in front writes w (weights_follow), so that its first values may be requested ahead of the dependency wait
 };
 
 __device__ __forceinline__ void fma2(float2& d, float2 a, float2 b) {
@@ -182,6 +183,8 @@ __device__ __forceinline__ void scatter_sum(float (&v)[N]) {
 constexpr int kRowsK = 512, kRowsWarps = 8;  // k values of a staged run
 
 // TT token rows, RF features per warp, PF weight steps (RF float4 a lane each) in flight, CTAS per SM
+// The first PF steps are under way before the rows are (p.early): with the gate of the feed-forward letting its product come, five requests with 12 decode steps, four
+// layers of 2048, 8.79 -> 8.66 ms.
 template <int TT, int RF, int PF, int CTAS>
 __global__ void __launch_bounds__(kRowsWarps * 32, CTAS) gemm_fp32_rows_kernel(Fp32Args p) {
   extern __shared__ __align__(16) float sm[];  // two runs of TT token rows, [TT][kRowsK]
@@ -211,12 +214,16 @@ __global__ void __launch_bounds__(kRowsWarps * 32, CTAS) gemm_fp32_rows_kernel(F
   float2 acc[RF * TT];
 #pragma unroll
   for (int i = 0; i < RF * TT; ++i) acc[i] = make_float2(0.f, 0.f);
+  float4 b[PF][RF];
+  auto request = [&]() {
+#pragma unroll
+    for (int i = 0; i < PF; ++i) weights(b[i], k_lo + i * 128 + lane * 4);
+  };
+  if (p.early) request();
   pg::griddep_wait();
   pg::griddep_launch_dependents();
   if (p.only_if != nullptr && *p.only_if == 0) return;  // (the whole grid)
-  float4 b[PF][RF];
-#pragma unroll
-  for (int i = 0; i < PF; ++i) weights(b[i], k_lo + i * 128 + lane * 4);
+  if (!p.early) request();
   if (runs > 0) stage(0);
   pg::cp_async_commit();
   for (int run = 0; run < runs; ++run) {
@@ -359,7 +366,7 @@ double pg_gemm_fp32_estimate(int T, int F, int K, int accumulate) {
 int pg_gemm_fp32(const float* x, long long ldx, long long bsx, const float* w, long long ldw, long long bsw, float* out, long long ldo, long long bso,
                  const float* bias, int accumulate, float scale, int T, int F, int K, int batch, cudaStream_t st,
                  const int* only_if) {
-  Fp32Args p{x, w, bias, out, ldx, ldw, ldo, bsx, bsw, bso, T, F, K, 0, accumulate, scale, only_if};
+  Fp32Args p{x, w, bias, out, ldx, ldw, ldo, bsx, bsw, bso, T, F, K, 0, accumulate, scale, only_if, only_if == nullptr ? pg::weights_follow() : 0};
   const int sms = pg::num_sms();
   // 16-byte copies and loads want every row of every operand on a 16-byte boundary
   const bool wide = K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && bsx % 4 == 0 && bsw % 4 == 0 &&

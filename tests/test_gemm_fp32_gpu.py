@@ -72,3 +72,29 @@ def test_infinities_stay_in_their_rows():
 def test_no_rows_are_refused():
     w = torch.randn(8, 16, device="cuda")
     assert _lib.lib().pg_gemm_simt(w.data_ptr(), 16, w.data_ptr(), 16, w.data_ptr(), 8, 0, 8, 16, 1, 1, _lib.stream()) != 0
+
+
+@pytest.mark.parametrize("T", [1, 4, 6, 7, 16])
+@pytest.mark.parametrize("F,K", [(96, 64), (1000, 516), (2048, 8192), (4096, 2052)])
+def test_weights_requested_ahead_of_the_rows(T, F, K):
+    """In a step that says that weights follow, a few rows' product asks for its weights while the kernel in front writes the rows: the same sums bit for bit."""
+    g = torch.Generator(device="cuda").manual_seed(T + K)
+    gu, w = torch.randn(T, 2 * K, generator=g, device="cuda"), torch.randn(F, K, generator=g, device="cuda")
+    outs = []
+    for on in (False, True):
+        mid, out = torch.zeros(T, K, device="cuda"), torch.empty(T, F, device="cuda")
+        if on:
+            _lib.lib().pg_weights_follow(1)
+        try:
+            for _ in range(3):
+                seq_ops.geglu(gu, mid)
+                seq_ops.linear(mid, w, out)
+        finally:
+            if on:
+                _lib.lib().pg_weights_follow(0)
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1])
+    a = torch.nn.functional.gelu(gu[:, :K].double(), approximate="tanh") * gu[:, K:].double()
+    # the sums' bound, and 2^-20 of every value for gelu's and the product's roundings
+    want, mag = a @ w.double().T, a.abs() @ w.abs().double().T
+    assert ((outs[1].double() - want).abs() <= ((K / 2 + 48) * 2.0 ** -24 + 2.0 ** -20) * mag).all()
