@@ -687,6 +687,9 @@ int pg_moe_route(const float* logits, long long ld, const float* correction, int
 int pg_moe_tile_rows(void);
 int pg_moe_plan(const int* counts, const int* ids, int* offsets, int* fill, int* plan, int* sorted_pair, int* pair_row, int pairs,
                 int n_real, int max_tiles, void* stream);
+/* Both in two launches, for at most 4096 pairs and 1024 experts (else PG_ERR_ARG). */
+int pg_moe_route_plan(const float* logits, long long ld, const float* correction, int* ids, float* weights, int* offsets, int* plan, int* sorted_pair, int* pair_row, int tokens,
+                      int n_all, int n_real, int top, int group_count, int group_keep, float scale, const float* logit_bias, int flags, int max_tiles, void* stream);
 int pg_moe_gemm(const void* x, long long ldx, const int* sorted_pair, int src_div, const void* w, long long expert_stride, long long ldw,
                 void* out, long long ldo, const int* plan, int max_tiles, int F, int K, int act, int in_f32, int out_f32,
                 long long x_expert_off, long long out_expert_off, void* stream);

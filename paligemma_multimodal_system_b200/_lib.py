@@ -107,6 +107,7 @@ SIGNATURES = {
     "pg_moe_route": [p, i64, p, p, p, p, i32, i32, i32, i32, i32, i32, f32, p, i32, p],
     "pg_moe_combine_norm_add": [p, i64, p, p, p, p, p, i32, i32, i32, f32, i32, p],
     "pg_moe_tile_rows": [],
+    "pg_moe_route_plan": [p, i64, p, p, p, p, p, p, p, i32, i32, i32, i32, i32, i32, f32, p, i32, i32, p],
     "pg_moe_plan": [p, p, p, p, p, p, p, i32, i32, i32, p],
     "pg_moe_gemm": [p, i64, p, i32, p, i64, i64, p, i64, p, i32, i32, i32, i32, i32, i32, i64, i64, p],
     "pg_moe_gather_rows": [p, i64, p, p, i32, p, i64, i32, i32, i32, p],

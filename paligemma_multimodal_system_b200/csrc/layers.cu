@@ -178,7 +178,7 @@ extern "C" long long pg_routed_ff_scratch(const PgRoutedFf* a) {
 }
 
 // The launches of RoutedFeedForward for a step of few rows, issued by one call: eleven from Python cost 150 us of host time, more than the kernels of 300 tokens
-// take (109 -> 90 us for top 4 of 14 experts 2048 x 1024 with a shared one of 2048).  Same launches, same order.
+// take (109 -> 90 us for top 4 of 14 experts 2048 x 1024 with a shared one of 2048).  Same launches, same order, but for few pairs the plan in one.
 extern "C" int pg_routed_ff(const PgRoutedFf* args, const void* h, long long ldh, float* y, int accumulate, void* scratch, long long scratch_bytes, void* stream) {
   if (args == nullptr || h == nullptr || y == nullptr || scratch == nullptr || pg_routed_ff_scratch(args) == 0 || (reinterpret_cast<uintptr_t>(scratch) & 255) != 0) return PG_ERR_ARG;
   const PgRoutedFf& a = *args;
@@ -186,8 +186,13 @@ extern "C" int pg_routed_ff(const PgRoutedFf* args, const void* h, long long ldh
   if (scratch_bytes < s.bytes || s.max_tiles > 65535) return PG_ERR_ARG;
   const int T = a.tokens;
   PG_TRY(pg_linear_f32(h, ldh, a.router, a.D, s.z, a.n_pad, T, a.n_pad, a.D, stream));
-  PG_TRY(pg_moe_route(s.z, a.n_pad, a.correction, s.ids, s.wts, s.counts, T, a.n_all, a.n_real, a.top, a.group_count, a.group_keep, a.scale, a.router_b, a.flags, stream));
-  PG_TRY(pg_moe_plan(s.counts, s.ids, s.offsets, s.fill, s.plan, s.sorted_pair, s.pair_row, s.pairs, a.n_real, s.max_tiles, stream));
+  if (s.pairs <= 4096 && a.n_real <= 1024) {  // (what one CTA plans)
+    PG_TRY(pg_moe_route_plan(s.z, a.n_pad, a.correction, s.ids, s.wts, s.offsets, s.plan, s.sorted_pair, s.pair_row, T, a.n_all, a.n_real, a.top, a.group_count, a.group_keep, a.scale,
+                             a.router_b, a.flags, s.max_tiles, stream));
+  } else {
+    PG_TRY(pg_moe_route(s.z, a.n_pad, a.correction, s.ids, s.wts, s.counts, T, a.n_all, a.n_real, a.top, a.group_count, a.group_keep, a.scale, a.router_b, a.flags, stream));
+    PG_TRY(pg_moe_plan(s.counts, s.ids, s.offsets, s.fill, s.plan, s.sorted_pair, s.pair_row, s.pairs, a.n_real, s.max_tiles, stream));
+  }
   PG_TRY(pg_moe_products(h, ldh, s.sorted_pair, s.offsets + a.n_real, a.top, s.xg, a.w_up, a.w_down, s.mid, s.eo, s.plan, s.max_tiles, s.pairs, a.n_real, a.D, a.F, a.act,
                          stream));
   if (a.shared_up != nullptr) {

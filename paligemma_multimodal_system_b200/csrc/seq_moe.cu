@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict_
       if (my_id >= 0) {
         ids[(long long)t * top + base + lane] = my_id;
         weights[(long long)t * top + base + lane] = my_p;  // scaled below
-        if (my_id < n_real) atomicAdd(counts + my_id, 1);
+        if (counts != nullptr && my_id < n_real) atomicAdd(counts + my_id, 1);
       }
       my_id = -1;
     }
@@ -167,10 +167,7 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict_
 
 // counts -> offsets, tile list.  plan[0] = number of tiles; tiles: (expert, first sorted row, rows) triples from plan[4].
 // One warp: 32 experts at a time, prefix sums of their counts and tile numbers by shuffles.
-__global__ void moe_plan_kernel(const int* __restrict__ counts, int* __restrict__ offsets, int* __restrict__ fill, int* __restrict__ plan, int n_real,
-                                int max_tiles) {
-  pg::griddep_begin<true>();
-  const int lane = threadIdx.x;
+__device__ __forceinline__ void plan_of_counts(const int* counts, int* offsets, int* fill, int* plan, int* first_row, int n_real, int max_tiles, int lane) {
   int off = 0, nt = 0;
   for (int e0 = 0; e0 < n_real; e0 += 32) {
     const int e = e0 + lane, c = e < n_real ? counts[e] : 0, tiles = (c + MOE_TILE - 1) / MOE_TILE;
@@ -183,7 +180,8 @@ __global__ void moe_plan_kernel(const int* __restrict__ counts, int* __restrict_
     const int first = off + pc - c, tile0 = nt + ptl - tiles;
     if (e < n_real) {
       offsets[e] = first;
-      fill[e] = 0;
+      if (fill != nullptr) fill[e] = 0;
+      if (first_row != nullptr) first_row[e] = first;
     }
     for (int r = 0; r < tiles && tile0 + r < max_tiles; ++r) {
       int* p = plan + 4 + 3 * (tile0 + r);
@@ -197,6 +195,43 @@ __global__ void moe_plan_kernel(const int* __restrict__ counts, int* __restrict_
   if (lane == 0) {
     offsets[n_real] = off;
     plan[0] = nt < max_tiles ? nt : max_tiles;
+  }
+}
+
+__global__ void moe_plan_kernel(const int* __restrict__ counts, int* __restrict__ offsets, int* __restrict__ fill, int* __restrict__ plan, int n_real,
+                                int max_tiles) {
+  pg::griddep_begin<true>();
+  plan_of_counts(counts, offsets, fill, plan, nullptr, n_real, max_tiles, threadIdx.x);
+}
+
+// Few pairs: one CTA counts them in shared memory, which gives each its place among its expert's too, so that counters to clear, the plan and the scatter are one launch instead
+// of three (and the clearing no longer stands between the router's product and the routing).  What bounds it is its chain: ids, counters, one warp's scan, rows.  300 tokens,
+// top 4 of 14 experts 2048 x 1024: the routed feed-forward 91.5 -> 86.8 us.
+constexpr int kPlanThreads = 1024, kPlanPairs = 4 * kPlanThreads, kPlanExperts = 1024;
+__global__ void __launch_bounds__(kPlanThreads) moe_plan_pairs_kernel(const int* __restrict__ ids, int* __restrict__ offsets, int* __restrict__ plan, int* __restrict__ sorted_pair,
+                                                                      int* __restrict__ pair_row, int pairs, int n_real, int max_tiles) {
+  __shared__ int count[kPlanExperts], first_row[kPlanExperts];
+  for (int e = threadIdx.x; e < n_real; e += kPlanThreads) count[e] = 0;
+  pg::griddep_begin<true>();
+  int expert[4], place[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int p = j * kPlanThreads + threadIdx.x;
+    expert[j] = p < pairs ? ids[p] : n_real;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < 4; ++j) place[j] = expert[j] < n_real ? atomicAdd(count + expert[j], 1) : 0;
+  __syncthreads();
+  if (threadIdx.x < 32) plan_of_counts(count, offsets, nullptr, plan, first_row, n_real, max_tiles, threadIdx.x);
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int p = j * kPlanThreads + threadIdx.x;
+    if (p >= pairs) continue;
+    const int row = expert[j] < n_real ? first_row[expert[j]] + place[j] : -1;
+    if (row >= 0) sorted_pair[row] = p;
+    pair_row[p] = row;
   }
 }
 
@@ -542,17 +577,33 @@ extern "C" int pg_moe_combine_norm_add(const float* expert_out, long long ldy, c
   PG_RET();
 }
 
-extern "C" int pg_moe_route(const float* logits, long long ld, const float* correction, int* ids, float* weights, int* counts, int tokens, int n_all,
-                            int n_real, int top, int group_count, int group_keep, float scale, const float* logit_bias, int flags, void* stream) {
+static int route(const float* logits, long long ld, const float* correction, int* ids, float* weights, int* counts, int tokens, int n_all, int n_real, int top, int group_count,
+                 int group_keep, float scale, const float* logit_bias, int flags, bool counted, void* stream) {
   if (tokens <= 0 || n_all <= 0 || n_real < 0 || n_real > n_all || top <= 0 || top > n_all) return PG_ERR_ARG;
   if (group_count > 1 && (n_all % group_count != 0 || group_keep <= 0 || group_keep > group_count || group_count > 256)) return PG_ERR_ARG;
   if (group_count > 1 && top > (long long)group_keep * (n_all / group_count)) return PG_ERR_ARG;
   const size_t smem = (size_t)4 * 2 * n_all * sizeof(float);
   if (smem > 48 * 1024) return PG_ERR_ARG;
   cudaStream_t st = PG_ST(stream);
-  if (n_real > 0 && cudaMemsetAsync(counts, 0, (size_t)n_real * sizeof(int), st) != cudaSuccess) return PG_ERR_CUDA;
-  pg::launch_dependent(moe_route_kernel, (tokens + 3) / 4, 128, smem, st, logits, ld, correction, ids, weights, counts, tokens, n_all, n_real, top, group_count, group_keep,
-                                                        scale, logit_bias, flags);
+  if (counted && n_real > 0 && cudaMemsetAsync(counts, 0, (size_t)n_real * sizeof(int), st) != cudaSuccess) return PG_ERR_CUDA;
+  pg::launch_dependent(moe_route_kernel, (tokens + 3) / 4, 128, smem, st, logits, ld, correction, ids, weights, counted ? counts : nullptr, tokens, n_all, n_real, top,
+                       group_count, group_keep, scale, logit_bias, flags);
+  PG_RET();
+}
+
+extern "C" int pg_moe_route(const float* logits, long long ld, const float* correction, int* ids, float* weights, int* counts, int tokens, int n_all,
+                            int n_real, int top, int group_count, int group_keep, float scale, const float* logit_bias, int flags, void* stream) {
+  return route(logits, ld, correction, ids, weights, counts, tokens, n_all, n_real, top, group_count, group_keep, scale, logit_bias, flags, true, stream);
+}
+
+extern "C" int pg_moe_route_plan(const float* logits, long long ld, const float* correction, int* ids, float* weights, int* offsets, int* plan, int* sorted_pair, int* pair_row,
+                                 int tokens, int n_all, int n_real, int top, int group_count, int group_keep, float scale, const float* logit_bias, int flags, int max_tiles,
+                                 void* stream) {
+  const long long pairs = static_cast<long long>(tokens) * top;
+  if (n_real <= 0 || n_real > kPlanExperts || pairs <= 0 || pairs > kPlanPairs || max_tiles <= 0) return PG_ERR_ARG;
+  const int rc = route(logits, ld, correction, ids, weights, nullptr, tokens, n_all, n_real, top, group_count, group_keep, scale, logit_bias, flags, false, stream);
+  if (rc != PG_OK) return rc;
+  pg::launch_dependent(moe_plan_pairs_kernel, 1, kPlanThreads, 0, PG_ST(stream), ids, offsets, plan, sorted_pair, pair_row, static_cast<int>(pairs), n_real, max_tiles);
   PG_RET();
 }
 

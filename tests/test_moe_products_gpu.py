@@ -4,7 +4,7 @@ Bounds: the activations between the products are bf16 (2^-8 of the value that is
 import pytest
 import torch
 
-from paligemma_multimodal_system_b200 import seq_ops
+from paligemma_multimodal_system_b200 import _lib, seq_ops
 
 pytestmark = pytest.mark.gpu
 
@@ -142,3 +142,34 @@ def test_dense_runs(D, F, T, activation):
     mid = seq_ops.moe_gemm(h, plan, ff.w_up, prec.empty(plan.pairs, F), gather=True, act=ff.act)
     want = seq_ops.moe_gemm(mid, plan, ff.w_down, torch.empty(plan.pairs, D, device="cuda"), gather=False)
     assert (eo - want).abs().max() <= 2.0 ** -7 * mid.float().abs().max()
+
+
+@pytest.mark.parametrize("T,top,n_all,n_real,nan", [(1, 1, 1, 1, False), (1, 4, 14, 14, False), (300, 4, 16, 14, False), (1024, 4, 14, 14, False), (819, 5, 1100, 1024, False),
+                                                    (256, 4, 40, 33, True), (64, 8, 64, 1, False)])
+def test_plan_of_few_pairs(T, top, n_all, n_real, nan):
+    """Counters, plan and scatter in one launch against the three: the same choices, runs and tiles, and every pair on a row of its expert's run."""
+    logits = torch.randn(T, n_all, device="cuda")
+    if nan:
+        logits[::3] = float("nan")  # (a token that chooses expert 0 every time)
+    ids, wts, counts = seq_ops.moe_route(logits, None, n_real, top, 1, 1, 1.0)
+    ref = seq_ops.MoePlan(ids, counts, n_real)
+    ids2, wts2 = torch.empty_like(ids), torch.empty_like(wts)
+    offsets, plan, order, row = (torch.full_like(t, -7) for t in (ref.offsets, ref.plan, ref.sorted_pair, ref.pair_row))
+    _lib.check(_lib.lib().pg_moe_route_plan(logits.data_ptr(), n_all, 0, ids2.data_ptr(), wts2.data_ptr(), offsets.data_ptr(), plan.data_ptr(), order.data_ptr(), row.data_ptr(), T, n_all,
+                                            n_real, top, 1, 1, 1.0, 0, 0, ref.max_tiles, _lib.stream()), "plan")
+    assert torch.equal(ids, ids2) and torch.equal(wts.view(torch.int32), wts2.view(torch.int32)) and torch.equal(offsets, ref.offsets)
+    tiles = int(ref.plan[0])
+    assert torch.equal(plan[4:4 + 3 * tiles], ref.plan[4:4 + 3 * tiles]) and int(plan[0]) == tiles
+    flat, total = ids.flatten(), int(offsets[n_real])
+    real = flat < n_real
+    assert (row[~real] == -1).all() and torch.equal(row[real].sort().values, torch.arange(total, device="cuda", dtype=torch.int32))
+    assert torch.equal(order[row[real].long()], torch.nonzero(real).flatten().int())
+    e = flat[real].long()
+    assert (row[real] >= offsets[e]).all() and (row[real] < offsets[e + 1]).all()
+
+
+def test_plan_of_too_many_pairs_is_refused():
+    z, i = torch.zeros(1025, 4, device="cuda"), torch.zeros(4100, device="cuda", dtype=torch.int32)
+    for T, n in ((1025, 4), (4, 0), (4, 1025)):
+        assert _lib.lib().pg_moe_route_plan(z.data_ptr(), 4, 0, i.data_ptr(), z.data_ptr(), i.data_ptr(), i.data_ptr(), i.data_ptr(), i.data_ptr(), T, max(4, n), n, 4, 1, 1, 1.0, 0, 0, 99,
+                                            _lib.stream()) != 0
