@@ -31,8 +31,8 @@
 #include "paligemma_b200.h"
 #include "tmap.cuh"
 
-#ifndef PG_AP_POLY16
-#define PG_AP_POLY16 6
+#ifndef PG_AP_POLY8
+#define PG_AP_POLY8 3
 #endif
 
 namespace pg {
@@ -174,9 +174,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   // the row sums of the (bf16) probabilities on the tensor core and the softmax warps -- bound by instruction issue, ~4.5
   // instructions per score -- drop the FADD per score.  The lazy rescale of O carries the column along.
   constexpr bool TCSUM = DHP > DH;
-  // scores per 16 whose exponential runs on the FMA pipe (exp2_fma_pair): MUFU and FMA / issue time balance near 6 of 16 for dh <= 128;
+  // the last scores of every 8 whose exponential runs on the FMA pipe (exp2_fma_pair): MUFU and FMA / issue time balance near 3 of 8 for dh <= 128 (three pairs of sixteen take two
+  // moves less, 8 x 1024 keys 73.5 us for 74.9, but a score's form, and with it the last bit of its bf16 probability, would depend on how scores are paired);
   // dh = 256 has four times the tensor work per score and is not softmax-bound
-  constexpr int POLY16 = DH <= 128 ? PG_AP_POLY16 : 0;
+  constexpr int POLY8 = DH <= 128 ? PG_AP_POLY8 : 0;
   constexpr uint32_t IDESC_S = make_idesc_bf16(BM, BN);
   constexpr uint32_t IDESC_O = make_idesc_bf16(BM, DHP, 0, 1);  // B (= V) is MN-major
   extern __shared__ __align__(1024) uint8_t smem_ap[];
@@ -470,7 +471,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         const float m_new = need ? mx : m_used;
         const float alpha = need ? exp2f(m_used - m_new) : 1.0f;  // first tile: m_used = -inf -> 0 (O is overwritten)
         m_used = m_new;
-        uint64_t sum = 0;
+        float sum = 0.f;
         const uint32_t pdst = p_row + sb * C::P_BYTES;
         // Three separate passes over the thread's HB scores (exponent arguments, then the MUFU exponentials back to back, then
         // pack + store): interleaved chunk by chunk, each exp2 -> pack -> store chain exposed the ~40 clk MUFU latency with two
@@ -483,21 +484,30 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         // (an earlier variant with floorf / float->int range reduction was 40 % SLOWER: those conversions run on the XU pipe
         //  as well, so it added XU work instead of removing it)
 #pragma unroll
-        for (int i = 0; i < HB / 2; ++i) x[i] = (i & 7) >= 8 - POLY16 / 2 ? exp2_fma_pair(x[i]) : pair_of(exp2_mufu(lo_f32(x[i])), exp2_mufu(hi_f32(x[i])));
+        for (int i = 0; i < HB / 2; ++i) {
+          const bool both = POLY8 > 0 && (i & 3) >= 4 - POLY8 / 2;                            // scores 6 and 7 of eight
+          const bool one = POLY8 % 2 == 1 && (i & 3) == 3 - POLY8 / 2, first = (i & 4) == 0;  // score 5, with that of the next eight
+          if (both) x[i] = exp2_fma_pair(x[i]);
+          else if (one && first) {
+            const uint64_t y = exp2_fma_pair(pair_of(hi_f32(x[i]), hi_f32(x[i + 4])));
+            x[i] = pair_of(exp2_mufu(lo_f32(x[i])), lo_f32(y));
+            x[i + 4] = pair_of(exp2_mufu(lo_f32(x[i + 4])), hi_f32(y));
+          } else if (!one) x[i] = pair_of(exp2_mufu(lo_f32(x[i])), exp2_mufu(hi_f32(x[i])));
+        }
 #pragma unroll
         for (int cc = 0; cc < HB / 8; ++cc) {  // 16-byte chunks of 8 keys
           uint32_t pk[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const uint64_t pp = x[cc * 4 + e];
-            if constexpr (!TCSUM) sum = add_pair(sum, pp);
+            if constexpr (!TCSUM) sum += lo_f32(pp) + hi_f32(pp);  // (one sum: two side by side 72.6 us for 69.2 at 8 x 1024 keys, heads of 64)
             pk[e] = pack_bf16(lo_f32(pp), hi_f32(pp));
           }
           const int c = half * (HB / 8) + cc;  // chunk index inside the whole tile row
           const uint32_t addr = pdst + (c >> 3) * C::P_BOX + (((c & 7) ^ (r & 7)) << 4);
           asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
         }
-        l_run = l_run * alpha + (lo_f32(sum) + hi_f32(sum));  // (SW == 2: the sum over this thread's columns only; the halves are added at the end)
+        l_run = l_run * alpha + sum;  // (SW == 2: the sum over this thread's columns only; the halves are added at the end)
         if (trole < 3) stamp(trole, j, 4);
         if (j > first) {
           if (__any_sync(0xffffffffu, need)) {  // (both warps of a quadrant see the same maxima, hence the same decision)

@@ -41,3 +41,46 @@ def test_blocks_of_wide_heads():
         r = slice(b * S, (b + 1) * S)
         want = torch.softmax(q[r].double().view(S, Hq, dh).transpose(0, 1) @ k[r].double().T * dh ** -0.5, -1) @ v[r].double()
         assert (out[r].double().view(S, Hq, dh).transpose(0, 1) - want).abs().max() <= 2.0 ** -7 * max(1.0, want.abs().max().item())
+
+
+def _fma(a, b, c):  # one rounding (24-bit factors: the product is exact in 64 bits)
+    return (a.double() * b.double() + c.double()).float()
+
+
+@pytest.mark.parametrize("H,dh", [(4, 72), (8, 256)])
+def test_every_probability_keeps_its_form(H, dh):
+    """One-hot keys and values show the probabilities themselves.  Of every eight scores of a 72-wide head the last three take the polynomial, whatever they are paired with; the row sums
+    of a 256-wide head are added in the order of the keys, two at a time."""
+    from paligemma_multimodal_system_b200 import _lib
+    N, S, D = 256, 64, H * dh
+    g = torch.Generator(device="cuda").manual_seed(dh)
+    q = (torch.randn(N, H, dh, generator=g, device="cuda") * 12).to(torch.bfloat16)
+    eye = torch.eye(S, dh, device="cuda", dtype=torch.bfloat16)
+    out = torch.empty(N, H, dh, device="cuda", dtype=torch.bfloat16)
+    if dh == 72:
+        kv = eye.view(S, 1, dh).expand(S, H, dh).contiguous()
+        args = (1, H, N, S, dh, 1, N * D, D, 0, dh, S * D, D, dh, N * D, D, 0, dh)
+    else:
+        kv = eye
+        args = (1, 1, N * H, S, dh, H, N * D, D, dh, 0, S * dh, dh, 0, N * D, D, dh, 0)
+    scale = dh ** -0.5
+    _lib.check(_lib.lib().pg_attention_prefill(q.data_ptr(), kv.data_ptr(), kv.data_ptr(), out.data_ptr(), *args, scale, _lib.stream()), "prefill")
+    f32 = lambda v: torch.tensor(v, device="cuda", dtype=torch.float32)
+    unit = f32(scale) * f32(1.4426950408889634)
+    s = q[..., :S].float()
+    x = _fma(s, unit, -(s.amax(-1, keepdim=True) * unit))
+    p = torch.exp2(x)
+    if dh == 72:
+        c = x.clamp(min=-126.0)
+        t = c + 12582912.0
+        f = c - (t - 12582912.0)
+        y = _fma(_fma(_fma(f32(0.05518874), f, f32(0.24261212)), f, f32(0.69325641)), f, f32(0.99992746))
+        p = torch.where(torch.arange(S, device="cuda") % 8 >= 5, y * torch.exp2(t - 12582912.0), p)
+        total = p.to(torch.bfloat16).double().sum(-1).float()  # (on the tensor cores, which cut sums off: a last bit now and then)
+    else:
+        total = torch.zeros_like(p[..., 0])
+        for j in range(0, S, 2):
+            total = total + (p[..., j] + p[..., j + 1])
+    want = (p.to(torch.bfloat16).float() * (1.0 / total)[..., None]).to(torch.bfloat16)
+    # a score in the other form rounds elsewhere in one of a hundred cases, two sums side by side in one of a thousand rows; a last bit of the sum in one of 2^15
+    assert (out[..., :S] != want).float().mean() <= (1e-3 if dh == 72 else 0.0)
