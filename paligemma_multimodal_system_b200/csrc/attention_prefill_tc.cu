@@ -22,11 +22,12 @@
 //               column halves of one row exchanging their maxima through shared memory) remains for single-tile problems.
 // S_{j+1} is computed while the softmax of tile j runs, and P_j V_j runs while the softmax of tile j+1 runs.
 // A CTA takes blocks in turn, one CTA per SM: rings, S buffers and their barriers run on from block to block, so the next block's queries, keys and first scores are there
-// while the softmax warps still write the last one's rows (a CTA per block spent 7 us of each on its start and end: 64 x 256 keys 74 us, 57 now; 8 x 1024 83, 78 now; a single
-// round of 17 blocks of 256-wide heads 13.3, 13.9 now).
+// while the softmax warps still write the last one's rows (a CTA per block spent 7 us of each on its start and end: 64 x 256 keys 73 us, 52 now; 8 x 1024 88, 71 now).  ONE: a single
+// round of 256-wide heads has none of that and a kernel without the loop and its barriers (17 blocks, launch after launch: CTA per block 10.6 us, in the loop 11.2, ONE 10.6; 65 blocks of
+// 1031 keys 21.9, 22.2, 21.6).
 // Zero padding comes from TMA: columns beyond dh (72 -> 80) and key / query rows beyond the sequence are out-of-bounds
 // box elements and arrive as zeros; padded keys are masked to -inf before the softmax.
-// Timelines of one CTA: clock64 stamps through Params::trace.
+// Timelines of one CTA: clock64 stamps through Params::trace, in instances of their own (a test for them at each of the stamps: 8 x 1024 keys 74.9 us, 70.9 without).
 #include "common.cuh"
 #include "paligemma_b200.h"
 #include "tmap.cuh"
@@ -163,7 +164,8 @@ PG_DEVINL uint64_t exp2_fma_pair(uint64_t x) {
 // QT = query tiles (128 rows each) per CTA.  QT = 2 (dh <= 128): both tiles run against the SAME K / V tiles in shared
 // memory -- the kernel is bound by K/V delivery through the crossbar (profiles/r01d_prefill_attn72_ncu_full.csv), and two
 // query tiles halve the K/V bytes per FLOP; softmax warps 2-5 own tile 0, warps 6-9 tile 1 (no exchange between them).
-template <int DH, int SW, int QT>
+// ONE: a CTA has one block (DH > 128).
+template <int DH, int SW, int QT, bool ONE, bool TRACE>
 __global__ void __launch_bounds__(96 + 128 * SW * QT, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV, const Params p) {
@@ -175,7 +177,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   // instructions per score -- drop the FADD per score.  The lazy rescale of O carries the column along.
   constexpr bool TCSUM = DHP > DH;
   // the last scores of every 8 whose exponential runs on the FMA pipe (exp2_fma_pair): MUFU and FMA / issue time balance near 3 of 8 for dh <= 128 (three pairs of sixteen take two
-  // moves less, 8 x 1024 keys 73.5 us for 74.9, but a score's form, and with it the last bit of its bf16 probability, would depend on how scores are paired);
+  // moves less, 2 % of 8 x 1024 keys, but a score's form, and with it the last bit of its bf16 probability, would depend on how scores are paired);
   // dh = 256 has four times the tensor work per score and is not softmax-bound
   constexpr int POLY8 = DH <= 128 ? PG_AP_POLY8 : 0;
   constexpr uint32_t IDESC_S = make_idesc_bf16(BM, BN);
@@ -219,7 +221,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   // (The issuing warps and the softmax take them from lane 0: tile counts then stay uniform over the warp for the compiler, and with them descriptors and addresses.)
   auto keys = [&](const Item& it) { return p.key_lens ? max(1, min(p.keys, __ldg(p.key_lens + it.b))) : p.keys; };
   // profiling stamps (tiles 0..31 of CTA (0,0,0)): role 0 = MMA issuer, 1 = softmax warp 2, 2 = softmax warp 6; 8 events per tile
-  const bool tr_on = p.trace != nullptr && blockIdx.x == 0 && lane == 0;
+  const bool tr_on = TRACE && blockIdx.x == 0 && lane == 0;
   auto stamp = [&](int role, int j, int ev) {
     if (tr_on && j < 32) p.trace[(role * 32 + j) * 8 + ev] = clock64();
   };
@@ -256,11 +258,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     // ============================== TMA producer ==============================
     if (lane == 0) {
       int jt = 0, n = 0;  // key tiles and blocks so far
-      for (int idx = blockIdx.x; idx < p.items; idx += gridDim.x) {
+      for (int idx = blockIdx.x; idx < p.items; idx = ONE ? p.items : idx + static_cast<int>(gridDim.x)) {
         const Item it = idx == static_cast<int>(blockIdx.x) ? item0 : item(idx);
         if (it.nqt == 0) continue;
         const int n_keys = keys(it), n_tiles = (n_keys + BN - 1) / BN;
-        mbar_wait(q_empty, (n & 1) ^ 1);
+        if (!ONE) mbar_wait(q_empty, (n & 1) ^ 1);
         mbar_expect_tx(q_full, it.nqt * C::Q_BYTES);
 #pragma unroll
         for (int qt = 0; qt < QT; ++qt) {
@@ -311,7 +313,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
           }
           umma_commit(s_full(qt, sb));
           if (qt == nqt - 1) umma_commit(k_empty(ks));
-          if (qt == nqt - 1 && last) umma_commit(q_empty);
+          if (!ONE && qt == nqt - 1 && last) umma_commit(q_empty);
         }
         __syncwarp();
       }
@@ -320,7 +322,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     // issuing thread while the tensor pipe's queue is full, so one stream serialised S_{j+1}, its barrier round trips, the
     // ones column and P_j V_j into 2300 clk per 128-key tile -- longer than the softmax it was supposed to hide behind.
     int jt = 0, n = 0;
-    for (int idx = blockIdx.x; idx < p.items; idx += gridDim.x) {
+    for (int idx = blockIdx.x; idx < p.items; idx = ONE ? p.items : idx + static_cast<int>(gridDim.x)) {
       const Item it = idx == static_cast<int>(blockIdx.x) ? item0 : item(idx);
       if (it.nqt == 0) continue;
       const int n_keys = __shfl_sync(0xffffffffu, keys(it), 0), n_tiles = (n_keys + BN - 1) / BN;
@@ -335,7 +337,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   } else if (warp == 2 + 4 * SW * QT) {
     // ============================== P V issuer ================================
     int jt = 0, n = 0;
-    for (int idx = blockIdx.x; idx < p.items; idx += gridDim.x) {
+    for (int idx = blockIdx.x; idx < p.items; idx = ONE ? p.items : idx + static_cast<int>(gridDim.x)) {
       const Item it = idx == static_cast<int>(blockIdx.x) ? item0 : item(idx);
       if (it.nqt == 0) continue;
       const int n_keys = __shfl_sync(0xffffffffu, keys(it), 0), n_tiles = (n_keys + BN - 1) / BN;
@@ -360,7 +362,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 #pragma unroll
         for (int qt = 0; qt < QT; ++qt) {
           if (qt >= it.nqt) break;
-          if (j == first) mbar_wait(o_empty(qt), (n & 1) ^ 1);  // the softmax has read the accumulator of the block before
+          if (!ONE && j == first) mbar_wait(o_empty(qt), (n & 1) ^ 1);  // the softmax has read the accumulator of the block before
           mbar_wait(p_full(qt, pb), (j >> 1) & 1);
           if (qt == 0) stamp(0, j, 4);
           tc_fence_after();
@@ -396,7 +398,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory"); };  // the two warps of a quadrant
     const uint32_t p_row = sbase + C::OFF_P + qt * 2 * C::P_BYTES + r * 128;
     int jt = 0;
-    for (int idx = blockIdx.x; idx < p.items; idx += gridDim.x) {
+    for (int idx = blockIdx.x; idx < p.items; idx = ONE ? p.items : idx + static_cast<int>(gridDim.x)) {
       const Item it = idx == static_cast<int>(blockIdx.x) ? item0 : item(idx);
       if (it.nqt == 0) continue;
       const int n_keys = __shfl_sync(0xffffffffu, keys(it), 0), n_tiles = (n_keys + BN - 1) / BN;
@@ -559,7 +561,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         for (int i = 0; i < EB; ++i)
           if (c1 + 16 * SW * i < DHP) tmem_ld16(lane_addr + col_o + c1 + 16 * SW * i, all[i]);
         tmem_ld_wait();
-        if (c1 + 16 * SW * EB >= DHP) {  // O has been read: the next block's may be summed
+        if (!ONE && c1 + 16 * SW * EB >= DHP) {  // O has been read: the next block's may be summed
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(o_empty(qt));
@@ -612,20 +614,27 @@ static int make_tmap_nd(CUtensorMap* m, const void* ptr, int rank, const long lo
   return r == CUDA_SUCCESS ? PG_OK : PG_ERR_TMAP;
 }
 
-template <int DH, int SW, int QT>
-static int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const Params& p, int B, int H, cudaStream_t st) {
+template <int DH, int SW, int QT, bool ONE, bool TRACE>
+static int launch_as(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const Params& p, cudaStream_t st) {
   using C = Cfg<DH, QT>;
   static bool configured[kMaxDevices] = {};
   const int dev = current_device();
   if (!configured[dev]) {
-    if (cudaFuncSetAttribute(attn_prefill_tc_kernel<DH, SW, QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess) {
+    if (cudaFuncSetAttribute(attn_prefill_tc_kernel<DH, SW, QT, ONE, TRACE>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess) {
       cudaGetLastError();
       return PG_ERR_CUDA;
     }
     configured[dev] = true;
   }
+  const unsigned grid = static_cast<unsigned>(p.items < num_sms() ? p.items : num_sms());
+  return launch_kernel(attn_prefill_tc_kernel<DH, SW, QT, ONE, TRACE>, grid, dim3(96 + 128 * SW * QT), C::SMEM, st, tq, tk, tv, p) == cudaSuccess ? PG_OK : PG_ERR_CUDA;
+}
+
+template <int DH, int SW, int QT>
+static int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const Params& p, int B, int H, cudaStream_t st) {
+  using C = Cfg<DH, QT>;
   // One CTA per SM.  Where the last round has at most half as many blocks as SMs, the two query tiles of each go to two CTAs: a tile alone on an SM takes a little over half of what two
-  // together take (64 blocks of 1024 keys 25 -> 19 us, 192 47 -> 40, 512 of 4096 keys 295 -> 258, the packed exponentials of 3 % included).
+  // together take (64 blocks of 1024 keys 25 -> 19 us, 192 47 -> 40, 512 of 4096 keys 293 -> 248 with the exponentials in pairs).
   Params pp = p;
   pp.m_blks = (p.rows + C::BM * QT - 1) / (C::BM * QT);
   pp.heads = H;
@@ -635,8 +644,9 @@ static int launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
   const bool split = QT == 2 && 2 * rest <= num_sms();
   pp.whole = static_cast<int>(split ? blks - rest : blks);
   pp.items = static_cast<int>(split ? blks + rest : blks);
-  const unsigned grid = static_cast<unsigned>(pp.items < num_sms() ? pp.items : num_sms());
-  return launch_kernel(attn_prefill_tc_kernel<DH, SW, QT>, grid, dim3(96 + 128 * SW * QT), C::SMEM, st, tq, tk, tv, pp) == cudaSuccess ? PG_OK : PG_ERR_CUDA;
+  constexpr bool WIDE = DH > 128;
+  if (p.trace != nullptr) return WIDE && pp.items <= num_sms() ? launch_as<DH, SW, QT, WIDE, true>(tq, tk, tv, pp, st) : launch_as<DH, SW, QT, false, true>(tq, tk, tv, pp, st);
+  return WIDE && pp.items <= num_sms() ? launch_as<DH, SW, QT, WIDE, false>(tq, tk, tv, pp, st) : launch_as<DH, SW, QT, false, false>(tq, tk, tv, pp, st);
 }
 
 }  // namespace ap

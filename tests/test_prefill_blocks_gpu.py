@@ -84,3 +84,33 @@ def test_every_probability_keeps_its_form(H, dh):
     want = (p.to(torch.bfloat16).float() * (1.0 / total)[..., None]).to(torch.bfloat16)
     # a score in the other form rounds elsewhere in one of a hundred cases, two sums side by side in one of a thousand rows; a last bit of the sum in one of 2^15
     assert (out[..., :S] != want).float().mean() <= (1e-3 if dh == 72 else 0.0)
+
+
+@pytest.mark.parametrize("dh,S", [(256, 263), (256, 40), (72, 200)])
+def test_a_block_alone_is_as_among_others(dh, S):
+    """One round (256-wide heads: a kernel without the loop over blocks) and several give the same bits, with stamps and without."""
+    from paligemma_multimodal_system_b200 import _lib
+    L, B, H = _lib.lib(), 40, 8
+    g = torch.Generator(device="cuda").manual_seed(S)
+    kvh = 1 if dh == 256 else H
+    q, k, v = (torch.randn(B * S, n * dh, generator=g, device="cuda").to(torch.bfloat16) for n in (H, kvh, kvh))
+
+    def go(batch):
+        out = torch.full_like(q[: batch * S], float("nan"))
+        if dh == 256:
+            args = (batch, 1, S * H, S, dh, H, S * H * dh, H * dh, dh, 0, S * dh, dh, 0, S * H * dh, H * dh, dh, 0)
+        else:
+            args = (batch, H, S, S, dh, 1, S * H * dh, H * dh, 0, dh, S * H * dh, H * dh, dh, S * H * dh, H * dh, 0, dh)
+        _lib.check(L.pg_attention_prefill(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), *args, dh ** -0.5, _lib.stream()), "prefill")
+        return out
+
+    one, all_ = go(1), go(B)
+    assert one.isfinite().all() and torch.equal(one, all_[:S])
+    stamps = torch.zeros(3 * 32 * 8, device="cuda", dtype=torch.int64)
+    try:
+        L.pg_debug_set_attn_prefill_trace(stamps.data_ptr())
+        again = go(1), go(B)
+        torch.cuda.synchronize()
+    finally:
+        L.pg_debug_set_attn_prefill_trace(None)
+    assert torch.equal(again[0], one) and torch.equal(again[1], all_) and (stamps != 0).any()
