@@ -96,37 +96,35 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* __restrict__ 
 // ---------------------------------------------------------------------------------------------------------
 // Block-per-row variants for few rows (decode steps, prompts of an image or two): a thread keeps its NV float4 of the row, row and weights are requested together, and one barrier
 // separates a sum from its use.  What bounds them: one trip to memory and the barriers.  The forms above, with the row in shared memory, three barriers a sum and the weights requested
-// behind the last one, remain for addresses off 16 bytes (four encoder layers of one 224-pixel image, nine norms of 256 rows: 237 -> 229 us; 24 tokens of one request, 37 norms a step: 27.4 ->
-// 27.0 ms).
+// behind the last one, remain for addresses off 16 bytes (launch after launch, there / here: layer norm of 256 x
+// 1152 3.0 / 1.8 us; without a mean 263 x 2048 2.9 / 2.0, one row 2.0 / 1.4; four encoder layers of one 224-pixel image, nine norms, 237 -> 228; 24 tokens of one request, 37 norms a
+// step, 27.4 -> 27.0 ms).
+// Every sum has the threads, terms and order of the forms above, so a row's bits do not depend on where its weights lie.
 // ---------------------------------------------------------------------------------------------------------
-template <int WARPS>
-PG_DEVINL float row_sum(float v, float* red) {  // every thread gets the sum over the block's up to WARPS warps; `red` [WARPS] is used once
+// the sum over the block's eight warps, for every thread, in block_sum's order; `red` [8] is used once
+PG_DEVINL float row_sum(float v, float* red) {
   v = warp_sum(v);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
-  const int warps = blockDim.x >> 5;
-  float t = 0.f;
-#pragma unroll
-  for (int i = 0; i < WARPS; ++i)
-    if (i < warps) t += red[i];
-  return t;
+  const float4 a = *reinterpret_cast<const float4*>(red), b = *reinterpret_cast<const float4*>(red + 4);
+  return ((a.x + b.x) + (a.z + b.z)) + ((a.y + b.y) + (a.w + b.w));
 }
 
 template <int NV>
-__global__ void __launch_bounds__(512) layernorm_reg_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta, bf16* __restrict__ y_bf,
+__global__ void __launch_bounds__(256) layernorm_reg_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta, bf16* __restrict__ y_bf,
                                                             float* __restrict__ y_f, int D, float eps, int trigger) {
-  __shared__ float red[2][16];
+  __shared__ __align__(16) float red[2][8], row[1024 * NV];  // (the squares are summed over elements 256 apart)
   pg::griddep_begin_if(trigger);
   const long long r = blockIdx.x;
   float4 v[NV], g[NV], b[NV];
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
-    const int i = threadIdx.x + 512 * k;
+    const int i = threadIdx.x + 256 * k;
     v[k] = 4 * i < D ? reinterpret_cast<const float4*>(x + r * D)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
   }
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
-    const int i = threadIdx.x + 512 * k;
+    const int i = threadIdx.x + 256 * k;
     if (4 * i < D) {
       g[k] = reinterpret_cast<const float4*>(gamma)[i];
       b[k] = reinterpret_cast<const float4*>(beta)[i];
@@ -134,28 +132,32 @@ __global__ void __launch_bounds__(512) layernorm_reg_kernel(const float* __restr
   }
   float s = 0.f, ss = 0.f;
 #pragma unroll
-  for (int k = 0; k < NV; ++k) s += v[k].x + v[k].y + v[k].z + v[k].w;
-  const float mean = row_sum<16>(s, red[0]) / D;
-#pragma unroll
   for (int k = 0; k < NV; ++k) {
-    if (4 * (static_cast<int>(threadIdx.x) + 512 * k) >= D) continue;
-    v[k].x -= mean; v[k].y -= mean; v[k].z -= mean; v[k].w -= mean;
-    ss += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
+    s += v[k].x + v[k].y + v[k].z + v[k].w;
+    reinterpret_cast<float4*>(row)[threadIdx.x + 256 * k] = v[k];
   }
-  const float rstd = rsqrtf(row_sum<16>(ss, red[1]) / D + eps);
+  const float mean = row_sum(s, red[0]) / D;
+#pragma unroll
+  for (int k = 0; k < 4 * NV; ++k) {
+    const int i = threadIdx.x + 256 * k;
+    const float d = row[i] - mean;
+    if (i < D) ss += d * d;
+  }
+  const float rstd = rsqrtf(row_sum(ss, red[1]) / D + eps);
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
-    const int i = threadIdx.x + 512 * k;
+    const int i = threadIdx.x + 256 * k;
     if (4 * i >= D) continue;
-    const float4 o = make_float4(v[k].x * rstd * g[k].x + b[k].x, v[k].y * rstd * g[k].y + b[k].y, v[k].z * rstd * g[k].z + b[k].z, v[k].w * rstd * g[k].w + b[k].w);
+    const float4 o = make_float4((v[k].x - mean) * rstd * g[k].x + b[k].x, (v[k].y - mean) * rstd * g[k].y + b[k].y, (v[k].z - mean) * rstd * g[k].z + b[k].z,
+                                 (v[k].w - mean) * rstd * g[k].w + b[k].w);
     if (y_bf) reinterpret_cast<uint2*>(y_bf + r * D)[i] = make_uint2(pack_bf16(o.x, o.y), pack_bf16(o.z, o.w));
     if (y_f) reinterpret_cast<float4*>(y_f + r * D)[i] = o;
   }
 }
 
 template <int NV>
-__global__ void __launch_bounds__(512) rmsnorm_reg_kernel(const float* __restrict__ x, const float* __restrict__ w, bf16* __restrict__ y, int D, float eps, int early_trigger) {
-  __shared__ float red[16];
+__global__ void __launch_bounds__(256) rmsnorm_reg_kernel(const float* __restrict__ x, const float* __restrict__ w, bf16* __restrict__ y, int D, float eps, int early_trigger) {
+  __shared__ __align__(16) float red[8];
   const long long r = blockIdx.x;
   if (early_trigger && threadIdx.x == 0) griddep_launch_dependents();  // (as rmsnorm_kernel)
   griddep_wait();
@@ -163,29 +165,26 @@ __global__ void __launch_bounds__(512) rmsnorm_reg_kernel(const float* __restric
   float4 v[NV], g[NV];
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
-    const int i = threadIdx.x + 512 * k;
+    const int i = threadIdx.x + 256 * k;
     v[k] = 4 * i < D ? reinterpret_cast<const float4*>(x + r * D)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
   }
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
-    const int i = threadIdx.x + 512 * k;
+    const int i = threadIdx.x + 256 * k;
     if (4 * i < D) g[k] = reinterpret_cast<const float4*>(w)[i];
   }
   float ss = 0.f;
 #pragma unroll
   for (int k = 0; k < NV; ++k) ss += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
-  const float rstd = rsqrtf(row_sum<16>(ss, red) / D + eps);
+  const float rstd = rsqrtf(row_sum(ss, red) / D + eps);
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
-    const int i = threadIdx.x + 512 * k;
+    const int i = threadIdx.x + 256 * k;
     if (4 * i < D)
       reinterpret_cast<uint2*>(y + r * D)[i] = make_uint2(pack_bf16(v[k].x * rstd * (1.0f + g[k].x), v[k].y * rstd * (1.0f + g[k].y)),
                                                          pack_bf16(v[k].z * rstd * (1.0f + g[k].z), v[k].w * rstd * (1.0f + g[k].w)));
   }
 }
-
-// threads of a row: one float4 each where 512 hold it
-inline int row_threads(int D) { return D >= 2048 ? 512 : (D / 4 + 31) / 32 * 32; }
 
 // ---------------------------------------------------------------------------------------------------------
 // Warp-per-row variants for the prefill (tens of thousands of short rows): the row lives in registers (NV = D / 128 float4 per
@@ -610,9 +609,9 @@ extern "C" int pg_layernorm(const float* x, const float* gamma, const float* bet
   }
   if (al) {
     auto go = [&](auto kern) {
-      pg::launch_dependent(kern, rows, row_threads(D), 0, PG_ST(stream), x, gamma, beta, static_cast<bf16*>(y_bf16), y_f32, D, eps, pg::weights_follow());
+      pg::launch_dependent(kern, rows, 256, 0, PG_ST(stream), x, gamma, beta, static_cast<bf16*>(y_bf16), y_f32, D, eps, pg::weights_follow());
     };
-    if (D <= 2048) go(layernorm_reg_kernel<1>); else if (D <= 4096) go(layernorm_reg_kernel<2>); else go(layernorm_reg_kernel<4>);
+    if (D <= 1024) go(layernorm_reg_kernel<1>); else if (D <= 2048) go(layernorm_reg_kernel<2>); else if (D <= 4096) go(layernorm_reg_kernel<4>); else go(layernorm_reg_kernel<8>);
     PG_RET();
   }
   pg::launch_dependent(layernorm_kernel, rows, 256, (D + 33) * sizeof(float), PG_ST(stream), x, gamma, beta, static_cast<bf16*>(y_bf16), y_f32, D, eps, pg::weights_follow());
@@ -636,9 +635,9 @@ extern "C" int pg_rmsnorm(const float* x, const float* w, void* y_bf16, int rows
   }
   if (al) {
     auto go = [&](auto kern) {
-      return launch_kernel(kern, dim3(rows), dim3(row_threads(D)), 0, PG_ST(stream), x, w, static_cast<bf16*>(y_bf16), D, eps, g_rmsnorm_early_trigger) == cudaSuccess ? PG_OK : PG_ERR_CUDA;
+      return launch_kernel(kern, dim3(rows), dim3(256), 0, PG_ST(stream), x, w, static_cast<bf16*>(y_bf16), D, eps, g_rmsnorm_early_trigger) == cudaSuccess ? PG_OK : PG_ERR_CUDA;
     };
-    return D <= 2048 ? go(rmsnorm_reg_kernel<1>) : D <= 4096 ? go(rmsnorm_reg_kernel<2>) : go(rmsnorm_reg_kernel<4>);
+    return D <= 1024 ? go(rmsnorm_reg_kernel<1>) : D <= 2048 ? go(rmsnorm_reg_kernel<2>) : D <= 4096 ? go(rmsnorm_reg_kernel<4>) : go(rmsnorm_reg_kernel<8>);
   }
   return launch_kernel(rmsnorm_kernel, dim3(rows), dim3(256), (D + 33) * sizeof(float), PG_ST(stream), x, w,
                        static_cast<bf16*>(y_bf16), D, eps, g_rmsnorm_early_trigger) == cudaSuccess ? PG_OK : PG_ERR_CUDA;

@@ -48,3 +48,22 @@ def test_few_rows(rows, D, shift):
     _lib.check(_lib.lib().pg_rmsnorm(x.data_ptr(), w.data_ptr(), y.data_ptr(), rows, D, eps, _lib.stream()), "pg_rmsnorm")
     want = xd / torch.sqrt((xd * xd).mean(-1, keepdim=True) + eps) * (1 + w.double())
     assert ((y.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -16).all()
+
+
+@pytest.mark.parametrize("rows", [1, 300])
+@pytest.mark.parametrize("D", [4, 100, 1020, 1024, 1028, 1152, 2048, 2052, 4096, 4100, 8192])
+def test_bits_do_not_depend_on_where_weights_lie(rows, D):
+    """The form with the row in registers sums in the order of the one in shared memory, which weights off 16 bytes take."""
+    from paligemma_multimodal_system_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(D + rows)
+    x = torch.randn(rows, D, generator=g, device="cuda") * 3 + 0.5
+    w, b = (torch.randn(D, generator=g, device="cuda") for _ in range(2))
+    res = []
+    for shift in (0, 1):
+        ws, bs = (torch.cat([t.new_zeros(shift), t])[shift:] for t in (w, b))
+        f, y, z = torch.empty(rows, D, device="cuda"), *(torch.empty(rows, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+        _lib.check(_lib.lib().pg_layernorm(x.data_ptr(), ws.data_ptr(), bs.data_ptr(), y.data_ptr(), f.data_ptr(), rows, D, 1e-6, _lib.stream()), "pg_layernorm")
+        _lib.check(_lib.lib().pg_rmsnorm(x.data_ptr(), ws.data_ptr(), z.data_ptr(), rows, D, 1e-6, _lib.stream()), "pg_rmsnorm")
+        res.append((f, y, z))
+    for a, c in zip(*res):
+        assert torch.equal(a, c)
