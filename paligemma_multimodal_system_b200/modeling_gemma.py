@@ -29,13 +29,14 @@ class KVCache:
     `v_cache`.  Storage: k_pages / v_pages [layers, num_pages, 64, Hkv*dh] bf16 + page_table [B, max_pages] int32 + the
     per-row device counters the decode kernels read (position id, write slot, kv length)."""
 
+    _first_slot = None  # int32 [B] of zeros: the prompt's first slot of every row (a cache saved without them has none)
+
     def __init__(self, reserve_tokens: int = 256):
         self.reserve_tokens = reserve_tokens  # head-room (in tokens) allocated beyond the prefill length
         self.k_pages = None
         self.v_pages = None
         self.page_table = None
         self.counters = None  # int32 [3, B]: pos, slot, kv_len  (device)
-        self._first_slot = None  # int32 [B] of zeros beside them
         self.image_feats = None  # projected image features of the request (decode-time <image> token parity): [B, n >= 1, D]
         self.image_feats_scaled = False  # True: the rows already carry hidden_size**-0.5 * sqrt(hidden) (written by _embed_prompt)
         self._len = 0
@@ -89,10 +90,11 @@ class KVCache:
     def allocate(self, B, layers, Hkv, dh, capacity_tokens):
         max_pages = (capacity_tokens + PAGE - 1) // PAGE
         self._geom = (B, layers, Hkv, dh)
-        self.k_pages, self.v_pages = torch.zeros(2, layers, B * max_pages, PAGE, Hkv * dh, device="cuda", dtype=torch.bfloat16).unbind(0)
+        self.k_pages = torch.zeros(layers, B * max_pages, PAGE, Hkv * dh, device="cuda", dtype=torch.bfloat16)  # (memory of their own: each can be saved and freed without the other)
+        self.v_pages = torch.zeros_like(self.k_pages)
         self.page_table = torch.arange(B * max_pages, device="cuda", dtype=torch.int32).view(B, max_pages).contiguous()
-        counters = torch.zeros(4, B, device="cuda", dtype=torch.int32)
-        self.counters, self._first_slot = counters[:3], counters[3]  # (the prompt's first slot of every row: 0)
+        self.counters = torch.zeros(3, B, device="cuda", dtype=torch.int32)
+        self._first_slot = torch.zeros(B, device="cuda", dtype=torch.int32)
         self._layer_len = []
         self._len = 0
 

@@ -40,3 +40,21 @@ def test_a_cache_of_fewer_layers_is_refused(monkeypatch, layers, accepted):
         with pytest.raises(ValueError):
             run()
         assert not library.calls
+
+
+def test_keys_values_and_counters_are_blocks_of_their_own(monkeypatch):
+    """Each is as large as it says, so that saving or freeing one does not take or keep another's memory."""
+    zeros, arange = torch.zeros, torch.arange
+    monkeypatch.setattr(torch, "zeros", lambda *a, device=None, **k: zeros(*a, **k))
+    monkeypatch.setattr(torch, "arange", lambda *a, device=None, **k: arange(*a, **k))
+    kv = modeling_gemma.KVCache()
+    kv.allocate(2, 3, 1, 16, 100)
+    for t in (kv.k_pages, kv.v_pages, kv.counters, kv._first_slot):
+        assert t.untyped_storage().nbytes() == t.numel() * t.element_size() and not t.any()
+    assert kv.k_pages.shape == kv.v_pages.shape == (3, 4, 64, 16) and kv.counters.shape == (3, 2)
+
+
+def test_a_cache_saved_before_it_had_first_slots_is_read():
+    kv = modeling_gemma.KVCache.__new__(modeling_gemma.KVCache)
+    kv.__dict__.update(reserve_tokens=4, _geom=None)
+    assert kv._first_slot is None
