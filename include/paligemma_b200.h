@@ -108,7 +108,8 @@ int pg_gemm_residual(const void* x, long long ldx, const void* w, long long ldw,
                      int K, float scale, void* stream);
 
 /* Between pg_weights_follow(1) and pg_weights_follow(0) the calling thread promises that the second operand of every product it issues is a weight: nothing that kernels of the same
- * stream still write.  Norms, gates and attention then let the kernel behind them come early (it requests its weights while they run).  Calls nest. */
+ * stream still write.  Embeddings, norms, gates, attention and the rows of q without a cache (pg_attn_prepare, k_pages == NULL) then let the kernel behind them come early: it requests its
+ * weights while they run.  Kernels that write pages or positions never do, so nothing more is promised.  Calls nest; PG_ERR_ARG for a pg_weights_follow(0) without its (1). */
 int pg_weights_follow(int on);
 
 /* out[t,f] = sum_k x[t,k] w[f,k] in fp32 rows; few tokens and few output tiles: K is shared out over the GPU. */

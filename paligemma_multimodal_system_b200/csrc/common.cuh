@@ -175,7 +175,7 @@ PG_DEVINL void griddep_launch_dependents() { asm volatile("griddepcontrol.launch
 //     the weight operand of the product behind), pages or positions.
 //   * griddep_begin<true>(): waits, then triggers.  Kernels whose results are fp32 rows and integers that are read behind a wait only (routing, scans).
 //   * griddep_begin_if(weights_follow()): where a whole layer is issued by one call (layers.cu), or a model's step by an engine that says so (pg_weights_follow), it is known that the
-//     product behind a norm, a gate or an attention takes a weight (and the fp32 products of few rows may ask for it: they do not otherwise).
+//     product behind an embedding, a norm, a gate or an attention takes a weight (and the fp32 products of few rows may ask for it: they do not otherwise).  Not where pages are written.
 // What that costs against every kernel triggering ahead of its wait: 48 requests with 24 decode steps 16.5 -> 16.9 ms, one request through four narrow layers 5 %; a tower of
 // four layers, one image 252 -> 247 us, a routed feed-forward 91 us both.
 // (Products trigger behind their wait: their outputs are not weights.  rmsnorm_kernel of the Gemma decode chain triggers early: see there.)

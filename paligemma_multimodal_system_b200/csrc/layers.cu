@@ -9,6 +9,7 @@
 bool pg_gemm_sums_once(int tokens, int features, int K, const void* out, long long ldo, const float* bias, int swap);  // gemm_tcgen05.cu
 
 extern "C" int pg_weights_follow(int on) {
+  if (!on && pg::t_weights_follow <= 0) return PG_ERR_ARG;  // (not given: taken back, it would silence the next one)
   pg::t_weights_follow += on ? 1 : -1;
   return PG_OK;
 }

@@ -1228,7 +1228,7 @@ extern "C" int pg_attn_prepare(const void* qkv, long long ld, const int* pos, co
       pg::launch_dependent(kernel, (rows + tok - 1) / tok, 128, (size_t)(tok * rot_dims + 2) * sizeof(float), PG_ST(stream), 
           static_cast<const TA*>(qkv), ld, pos, row_entry, page_table, max_pages, page, freq, q_norm, k_norm, static_cast<TA*>(q_out), static_cast<TA*>(k_pages),
           static_cast<TA*>(v_pages), rows, H, G, dim, vdim, rot_dims, eps, norm_qk, norm_v, v_from_k, rot_gain, static_cast<const TA*>(v_other), ld_v_other, v_mix,
-          pg::weights_follow());
+          k_pages != nullptr ? 0 : pg::weights_follow());  // (pages may be read ahead of the wait of the kernel behind, whatever its products take)
     };
     // four tokens a CTA once that still fills the SMs
     const bool four = rows >= 4 * 4 * pg::num_sms(), rot8 = rot_dims % 8 == 0;

@@ -24,11 +24,11 @@ from .serving import StepScheduler, TokenRequest
 def _weights_follow():
     """The products of a model's step take weights as their second operand: the kernels in front of them may let them come early."""
     L = _lib.lib()
-    L.pg_weights_follow(1)
+    _lib.check(L.pg_weights_follow(1), "pg_weights_follow")
     try:
         yield
     finally:
-        L.pg_weights_follow(0)
+        _lib.check(L.pg_weights_follow(0), "pg_weights_follow")
 
 
 class SequenceEngine:

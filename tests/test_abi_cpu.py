@@ -61,3 +61,14 @@ def test_config_classes_match_reference_defaults():
     c = PaliGemmaConfig(**copy.deepcopy(TINY_CONFIG), some_unknown_key=1)  # unknown keys are swallowed (**kwargs)
     assert c.text_config.num_image_tokens == 256 and c.vision_config.projection_dim == 256
     assert c.vocab_size == 1281 and c.text_config.pad_token_id == 0 and c.ignore_index == -100
+
+
+def test_a_promise_is_taken_back_once():
+    """pg_weights_follow nests; taking back what was not given is an error and leaves the next promise standing."""
+    from paligemma_multimodal_system_b200 import _lib, build
+    build.build()
+    lib = ctypes.CDLL(_lib.LIB_PATH)
+    follow = lib.pg_weights_follow
+    assert follow(0) < 0
+    assert [follow(1), follow(1), follow(0), follow(0)] == [0] * 4
+    assert follow(0) < 0 and follow(1) == 0 and follow(0) == 0 and follow(0) < 0

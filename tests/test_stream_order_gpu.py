@@ -155,3 +155,42 @@ def test_fused_decode_attention_behind_the_append(B, Hq, dh, L):
         q = new.cpu()[:, :Hq * dh].bfloat16().float().view(B, Hq, dh)
         want = torch.softmax(q @ kv[:, :, 0].transpose(1, 2) / math.sqrt(dh), -1) @ kv[:, :, 1]
         assert (o.cpu().float().view(B, Hq, dh) - want).abs().max() <= 1.5e-2 * want.abs().max()
+
+
+@pytest.mark.parametrize("B,Hq,dh,L", [(4, 8, 256, 300), (64, 8, 256, 130), (2, 4, 64, 700)])
+def test_fused_decode_attention_behind_the_rows_of_a_prompt(B, Hq, dh, L):
+    """pg_attn_prepare writes pages, the fused decode attention reads pages ahead of its wait: in order also where the products are promised to take weights."""
+    page = 64
+    per = L // page + 1
+    table = torch.arange(B * per, device="cuda", dtype=torch.int32).view(B, per).flip(1).contiguous()
+    kp, vp = (torch.zeros(B * per, page, dh, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    entry, at = torch.arange(B, device="cuda", dtype=torch.int32).repeat_interleave(L), torch.arange(L, device="cuda", dtype=torch.int32).repeat(B)
+    freq, inv = torch.zeros(1, device="cuda", dtype=torch.float64), torch.zeros(dh // 2, device="cuda")
+    pos, kv_len = torch.zeros(B, device="cuda", dtype=torch.int32), torch.full((B,), L + 1, device="cuda", dtype=torch.int32)
+    rows = [_t(B * L, (Hq + 2) * dh, seed=s, scale=0.5, dtype=torch.bfloat16) for s in (8, 9)]
+    q = torch.empty(B * L, Hq * dh, device="cuda", dtype=torch.bfloat16)
+    new = _t(B, (Hq + 2) * dh, seed=10, scale=0.5)
+    outs = [torch.empty(B, Hq * dh, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+    lib = _lib.lib()
+
+    def prepare(r):
+        _lib.check(lib.pg_attn_prepare(r.data_ptr(), r.stride(0), at.data_ptr(), entry.data_ptr(), table.data_ptr(), per, page, freq.data_ptr(), 0, 0, q.data_ptr(), kp.data_ptr(),
+                                       vp.data_ptr(), B * L, Hq, 1, dh, dh, 0, 1e-6, 0, 0, 0, 1.0, 0, 0, 0.0, 0, _lib.stream()), "prepare")
+
+    def attend(out):
+        _lib.check(lib.pg_attention_decode_fused(new.data_ptr(), pos.data_ptr(), kv_len.data_ptr(), inv.data_ptr(), kp.data_ptr(), vp.data_ptr(), table.data_ptr(),
+                                                 out.data_ptr(), B, Hq, 1, dh, page, B * per, per, 1.0 / math.sqrt(dh), _lib.stream()), "attention")
+
+    _lib.check(lib.pg_weights_follow(1), "follow")
+    try:
+        _queued([c for r, o in zip(rows, outs) for c in (lambda r=r: prepare(r), lambda o=o: attend(o))])
+    finally:
+        _lib.check(lib.pg_weights_follow(0), "follow")
+    for r, o in zip(rows, outs):
+        prepare(r)
+        torch.cuda.synchronize()
+        again = torch.empty_like(o)
+        attend(again)
+        torch.cuda.synchronize()
+        assert torch.equal(o, again)
+    assert not torch.equal(outs[0], outs[1])
