@@ -521,6 +521,7 @@ __global__ void __launch_bounds__(128) attn_latent_decode_mma_kernel(const bf16*
   }
   l_l += __shfl_xor_sync(0xffffffffu, l_l, 1); l_l += __shfl_xor_sync(0xffffffffu, l_l, 2);
   l_h += __shfl_xor_sync(0xffffffffu, l_h, 1); l_h += __shfl_xor_sync(0xffffffffu, l_h, 2);
+  const bool pairs = (reinterpret_cast<uintptr_t>(partial) & 7) == 0;  // (widths are even; the scratch may start on any float)
 #pragma unroll
   for (int half = 0; half < 2; ++half) {
     const int head = h0 + (half ? rh : rl);
@@ -538,7 +539,13 @@ __global__ void __launch_bounds__(128) attn_latent_decode_mma_kernel(const bf16*
       if (tq == 0 && v0 == 0) { pp[0] = mrow * 0.6931471805599453f; pp[1] = lsum; }  // the merge kernel works with natural exponentials
 #pragma unroll
       for (int nv = 0; nv < NV; ++nv) {
-        *reinterpret_cast<float2*>(pp + 2 + v0 + nv * 8 + 2 * tq) = make_float2(oacc[nv][2 * half], oacc[nv][2 * half + 1]);  // (VDIM is even)
+        float* to = pp + 2 + v0 + nv * 8 + 2 * tq;
+        if (pairs) {
+          *reinterpret_cast<float2*>(to) = make_float2(oacc[nv][2 * half], oacc[nv][2 * half + 1]);
+        } else {
+          to[0] = oacc[nv][2 * half];
+          to[1] = oacc[nv][2 * half + 1];
+        }
       }
     }
   }
