@@ -494,7 +494,9 @@ int pg_attn_ragged_mma(const void* q, const void* k_pages, const void* v_pages, 
                        const int* entry_row0, const int* entry_n, const int* entry_ctx, const int* page_table, int max_pages, int page,
                        int entries, int max_n, int H, int G, int dim, int vdim, float scale, float softcap, int skip_single,
                        int gate_per_head, const PgAttnScore* score, void* stream);
-/* The same with what the host knows of the batch: how many entries have rows for this kernel, and the longest context with its new tokens among them. */
+/* The same with what the host knows of the batch: `portions` entries have rows for this kernel -- with skip_single exactly those whose entry_n is not 1, without it all of them (PG_ERR_ARG
+ * for fewer); 0 or less: not known -- and `longest` is the longest context with its new tokens among them (it only chooses the form).  The grid is made for `portions` entries: as with max_n, rows
+ * past what is promised are left out. */
 int pg_attn_ragged_mma_sized(const void* q, const void* k_pages, const void* v_pages, const void* gate, long long ldg, void* out,
                        const int* entry_row0, const int* entry_n, const int* entry_ctx, const int* page_table, int max_pages, int page,
                        int entries, int max_n, int H, int G, int dim, int vdim, float scale, float softcap, int skip_single,

@@ -634,6 +634,7 @@ extern "C" int pg_attn_ragged_mma_sized(const void* q, const void* k_pages, cons
                                   const int* entry_row0, const int* entry_n, const int* entry_ctx, const int* page_table, int max_pages, int page,
                                   int entries, int max_n, int H, int G, int dim, int vdim, float scale, float softcap, int skip_single, int gate_per_head,
                                   int portions, int longest, const PgAttnScore* score, void* stream) {
+  if (portions > 0 && portions < entries && !skip_single) return PG_ERR_ARG;  // (every entry has rows then)
   return attn_ragged_mma(q, k_pages, v_pages, gate, ldg, out, entry_row0, entry_n, entry_ctx, page_table, max_pages, page, entries, max_n, H, G, dim, vdim, scale, softcap, skip_single, gate_per_head, portions, longest, score, stream);
 }
 

@@ -72,3 +72,16 @@ def test_a_promise_is_taken_back_once():
     assert follow(0) < 0
     assert [follow(1), follow(1), follow(0), follow(0)] == [0] * 4
     assert follow(0) < 0 and follow(1) == 0 and follow(0) == 0 and follow(0) < 0
+
+
+def test_fewer_portions_than_entries_without_single_tokens_left_out_are_refused():
+    """Every entry has rows then, and a grid for fewer would leave some out.  (Refused before anything is looked at or launched.)"""
+    from paligemma_multimodal_system_b200 import _lib, build
+    build.build()
+    lib = _lib.lib()
+
+    def call(portions, skip):
+        return lib.pg_attn_ragged_mma_sized(16, 16, 16, 0, 0, 16, 16, 16, 16, 16, 1, 64, 3, 5, 4, 4, 64, 64, 1.0, 0.0, skip, 0, portions, 0, 0, 0)
+
+    arg = lib.pg_attn_ragged_mma_sized(16, 16, 16, 0, 0, 16, 16, 16, 16, 16, 1, 64, 0, 5, 4, 4, 64, 64, 1.0, 0.0, 0, 0, 0, 0, 0, 0)  # no entries
+    assert arg < 0 and [call(1, 0), call(2, 0)] == [arg] * 2

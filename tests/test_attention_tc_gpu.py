@@ -181,3 +181,24 @@ def test_page_sizes(page, dim, vdim):
         got = out[r:r + n].double().view(n, H, vdim)
         assert ((got - want).abs() <= want.abs() * 2.0 ** -8 + 5e-5).all(), (i, (got - want).abs().max().item())
         r += n
+
+
+@pytest.mark.parametrize("dim,vdim,G,gsz", [(64, 64, 2, 4), (96, 64, 3, 1), (128, 128, 1, 2), (192, 128, 1, 3), (32, 32, 2, 2)])
+@pytest.mark.parametrize("skip", [0, 1])
+def test_what_the_host_has_counted_changes_nothing(dim, vdim, G, gsz, skip):
+    """pg_attn_ragged_mma knows nothing of the batch; with the number of entries that have rows, the same bits (short contexts: the keys of a block stay with one CTA)."""
+    from paligemma_multimodal_system_b200 import _lib
+    ns, ctxs, H = [1, 200, 1, 1, 70, 1], [90, 40, 5, 300, 0, 64], G * gsz
+    b = seq_ops.make_step_batch([dict(tokens=[1] * n, ctx=c, slot=i, pages=[(7 * i + j) % 11 for j in range((n + c + 63) // 64)]) for i, (n, c) in enumerate(zip(ns, ctxs))])
+    q, kp, vp = _t(b.T, H * dim, seed=1), _t(11, 64, G * dim, seed=2), _t(11, 64, G * vdim, seed=3)
+    L, outs = _lib.lib(), []
+    for counted in (None, 0, 2 if skip else len(ns), len(ns)):
+        out = torch.full((b.T, H * vdim), 7.0, device="cuda", dtype=torch.bfloat16)
+        args = [q.data_ptr(), kp.data_ptr(), vp.data_ptr(), 0, 0, out.data_ptr(), b.row0.data_ptr(), b.n.data_ptr(), b.ctx.data_ptr(), b.page_table.data_ptr(), b.max_pages, 64, len(ns),
+                b.max_n, H, G, dim, vdim, dim ** -0.5, 0.0, skip, 0]
+        if counted is None:
+            _lib.check(L.pg_attn_ragged_mma(*args, 0, _lib.stream()), "pg_attn_ragged_mma")
+        else:
+            _lib.check(L.pg_attn_ragged_mma_sized(*args, counted, 240, 0, _lib.stream()), "pg_attn_ragged_mma_sized")
+        outs.append(out)
+    assert all(torch.equal(o, outs[0]) for o in outs) and (outs[0] == 7).all(1).sum() == (4 if skip else 0)
