@@ -28,11 +28,6 @@ namespace {
 constexpr int kFeat = 128, kKb = 64, kATile = kFeat * kKb * 2, kThreads = 320, kMaxSplit = 8;
 constexpr int kProducers = 4;  // warp 0 and warps 2 .. kProducers: every kProducers-th stage each
 constexpr int kSmemMax = 232448 - 256;  // barriers behind the stages
-// Shared memory of a CTA that waits for its cluster's peers: above half of an SM's 228 KB (a CTA takes 1 KB beside its own), so that two of them never share an
-// SM.  Such a CTA holds tensor memory while it waits; two clusters of two streams that met in opposite order on two SMs would wait for each other's
-// columns for ever.  (The CTA pairs of gemm_tcgen05.cu take all but a few KB.)
-constexpr int kSmemAlone = 114 * 1024;
-static_assert(2 * (kSmemAlone + 1024) > 228 * 1024, "two clustered CTAs would fit on one SM");
 
 PG_DEVINL float4 ld_cluster4(uint32_t addr, uint32_t rank) {
   uint32_t a;
@@ -358,7 +353,8 @@ int launch_cluster_gemm(const ClusterGemmPlan& plan, const void* x, long long ld
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((a.features + kFeat - 1) / kFeat * a.split, (a.tokens + a.tile_tokens - 1) / a.tile_tokens);
   cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = a.split > 1 && a.smem_tiles + 256 < kSmemAlone ? kSmemAlone : a.smem_tiles + 256;
+  if (a.tile_tokens > 256 && a.smem_tiles + 256 < kClusterSmemWide) return PG_ERR_ARG;  // (never: such tiles come in steps of 32 tokens)
+  cfg.dynamicSmemBytes = a.split > 1 && a.smem_tiles + 256 < kClusterSmemAlone ? kClusterSmemAlone : a.smem_tiles + 256;
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;

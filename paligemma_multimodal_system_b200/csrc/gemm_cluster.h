@@ -26,6 +26,16 @@ struct ClusterGemmPlan {
   float clocks;
 };
 
+// Shared memory of CTAs that hold tensor memory while they wait for their cluster's peers.  Two clusters of two streams that met in opposite order on two SMs would wait for each other's
+// columns for ever, so no two such CTAs whose columns are more than an SM's 512 may fit on one (228 KB; a CTA takes 1 KB beside its own):
+//   * split products (gemm_cluster.cu) take more than half, so that two of them never share an SM;
+//   * those of more than 256 tokens a tile hold all 512 columns and exchange kClusterWideTokens x 128 floats at least; shared prompt attention (seq_attention_tc.cu: 256 columns, two on
+//     an SM) takes so much that it does not fit beside them;
+//   * CTA pairs (gemm_tcgen05.cu) take all but a few KB.
+constexpr int kSmShared = 228 * 1024, kCtaShared = 1024;
+constexpr int kClusterSmemAlone = 114 * 1024, kClusterWideTokens = 288, kClusterSmemWide = kClusterWideTokens * 128 * 4 + 256;  // (barriers)
+static_assert(2 * (kClusterSmemAlone + kCtaShared) > kSmShared, "two clustered CTAs would fit on one SM");
+
 ClusterGemmPlan plan_cluster_gemm(int tokens, int features, int K);
 int launch_cluster_gemm(const ClusterGemmPlan& plan, const void* x, long long ldx, const void* w, long long ldw, ClusterGemmArgs a, cudaStream_t st);
 

@@ -25,6 +25,7 @@
 #include <string.h>
 
 #include "common.cuh"
+#include "gemm_cluster.h"
 #include "paligemma_b200.h"
 #include "tmap.cuh"
 
@@ -100,7 +101,10 @@ struct Shape {
   static constexpr int SMEM = Q_BYTES + STAGES * KV_BYTES + 256;
   static constexpr int NBUF = VDIM > 64 ? 1 : 2;                 // areas of 96 columns: S, then P over it
   static constexpr int COL_O = 96 * NBUF;
-  static_assert(COL_O + VDIM <= 256 && STAGES >= 2 && DIM % 16 == 0 && VDIM % 64 == 0, "two CTAs per SM");
+  // SPLIT holds its columns while it waits for its peer: it must not fit on an SM beside a split product that wants all 512 (gemm_cluster.h)
+  static constexpr int SMEM_SPLIT = SMEM > 83 * 1024 ? SMEM : 83 * 1024;
+  static_assert(COL_O + VDIM <= 256 && STAGES >= 2 && DIM % 16 == 0 && VDIM % 64 == 0 && 2 * (SMEM_SPLIT + kCtaShared) <= kSmShared, "two CTAs per SM");
+  static_assert(SMEM_SPLIT + kClusterSmemWide + 2 * kCtaShared > kSmShared, "a split product's CTA of 512 columns would fit beside a shared block's");
 };
 
 // One query row by a warp, from the keys that it sees and no others: for rows whose sums are not finite (see above).  Scores, probabilities and sums in fp32; a lane has a key of
@@ -582,12 +586,13 @@ int launch(const void* q, const void* kp, const void* vp, const void* gate, long
            int max_pages, int page, int entries, int units, int max_n, int H, int G, float scale, float softcap, int skip_single, int gate_per_head, const PgAttnScore& sx,
            cudaStream_t st) {
   using C = Shape<DIM, VDIM>;
+  constexpr int smem = SPLIT ? C::SMEM_SPLIT : C::SMEM;
   const long long ctas = (static_cast<long long>(max_n) * (H / G) + 127) / 128 * G * units;
   if ((SPLIT ? 2 * ctas : ctas) > 0x7fffffff) return 1;
   static bool configured[kMaxDevices] = {};
   const int dev = current_device();
   if (!configured[dev]) {
-    if (cudaFuncSetAttribute(attn_ragged_tc_kernel<DIM, VDIM, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess) {
+    if (cudaFuncSetAttribute(attn_ragged_tc_kernel<DIM, VDIM, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
       cudaGetLastError();
       return PG_ERR_CUDA;
     }
@@ -611,7 +616,7 @@ int launch(const void* q, const void* kp, const void* vp, const void* gate, long
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(SPLIT ? 2 * ctas : ctas));
   cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = C::SMEM;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
