@@ -528,13 +528,15 @@ int pg_attn_latent_decode_mma(const void* q, const void* pages, const void* gate
  * dim and vdim multiples of 8, 16-byte aligned rows; every fp32 operand as three bf16 terms).
  * options (NULL: silu on q, k and v, every entry): silu == 0 -- q and k are turned in pairs (2i, 2i + 1) by the table `rotate` (fp32
  * [rows, 2, pairs]: cosines, then sines, of the step's rows, made by pg_rotary_table; NULL: not turned), k is multiplied by kscale, and
- * v is taken as it is, all in fp32; entries with fewer than n_min or more than n_max new tokens are left alone. */
+ * v is taken as it is, all in fp32; entries with fewer than n_min or more than n_max new tokens are left alone.  portions: how many are not, where the host knows it (0: not known); it
+ * only chooses between forms of a block. */
 typedef struct PgLinearAttnOps {
   int silu;
   float kscale;
   const float* rotate;
   int pairs;
   int n_min, n_max;
+  int portions;
 } PgLinearAttnOps;
 /* out[t, 0, i] = gain * cos(pos[t] * freq[i]), out[t, 1, i] = gain * sin(pos[t] * freq[i]) for i < rot_dims / 2; 1 and 0 for the other pairs. */
 int pg_rotary_table(const int* pos, const double* freq, float* out, int rows, int rot_dims, int pairs, float gain, void* stream);

@@ -148,7 +148,7 @@ class RoutedFf(C.Structure):
 
 class LinearAttnOps(C.Structure):
     """Mirror of PgLinearAttnOps."""
-    _fields_ = [("silu", i32), ("kscale", f32), ("rotate", p), ("pairs", i32), ("n_min", i32), ("n_max", i32)]
+    _fields_ = [("silu", i32), ("kscale", f32), ("rotate", p), ("pairs", i32), ("n_min", i32), ("n_max", i32), ("portions", i32)]
 
 
 class ConvSections(C.Structure):

@@ -351,9 +351,10 @@ extern "C" int pg_linear_attn_blocks(const void* qkv, long long ld, float* state
   if (dim <= 0 || dim % 8 || dim > 128 || vdim <= 0 || vdim % 8 || ld % 8 || (reinterpret_cast<uintptr_t>(qkv) & 15)) return PG_ERR_ARG;
   if (!options->silu && options->rotate != nullptr && (2 * options->pairs < dim || options->pairs % 4 || (reinterpret_cast<uintptr_t>(options->rotate) & 15))) return PG_ERR_ARG;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  // heads up to 64 wide with silu: three CTAs per SM (and a few spills) once there are more than two for each, else two (us, 2 / 3: 1536 CTAs 327 / 283, 96 CTAs of 1500
-  // tokens 279 / 310; without silu 1536 CTAs 187 / 202)
-  const bool many = (long long)((vdim + 63) / 64) * H * entries > 2LL * pg::num_sms();
+  // heads up to 64 wide with silu: three CTAs per SM (and a few spills) once there are more than two with tokens for each, else two (us, 2 / 3: 1536 CTAs 327 / 283, 384 of 300 tokens
+  // 150 / 97, 288 84 / 102, 96 of 1500 tokens 279 / 310; without silu 1536 CTAs 187 / 202)
+  const int portions = options->portions > 0 && options->portions < entries ? options->portions : entries;
+  const bool many = (long long)((vdim + 63) / 64) * H * portions > 2LL * pg::num_sms();
 #define PG_LB1(D, C, SILU, CTAS) \
   return launch_blocks<D, C, SILU, CTAS>(static_cast<const bf16*>(qkv), ld, state, decay, out, entry_row0, entry_n, entry_ctx, entry_slot, entries, H, dim, vdim, *options, st)
 #define PG_LB(D, C, MANY)                            \

@@ -1368,8 +1368,12 @@ extern "C" int pg_linear_attn_chunked(const void* qkv, long long ld, float* stat
   if (!linear_attn_ops(options, dim, ops)) return PG_ERR_ARG;
   int VB = 64;
   while (VB > 8 && VB / 2 >= vdim) VB /= 2;
-  // narrower value blocks (the scores are recomputed per block) only while the grid does not even fill the SMs once
-  while (VB > 16 && (long long)((vdim + VB - 1) / VB) * H * entries < (long long)pg::num_sms()) VB /= 2;
+  // narrower value blocks (the scores are recomputed per block) only while the CTAs with tokens do not even fill the SMs once (2000 tokens beside 40 single ones, 16 heads x 64: with the
+  // blocks that 41 entries want 518 us, with those of one 327).  Where CTAs without tokens follow them, more than two thirds of the SMs' number are no longer placed one to an SM (28 heads:
+  // 56 / 112 CTAs 382 / 430 us, 329 where nothing follows the 112).
+  const int portions = ops.portions > 0 && ops.portions < entries ? ops.portions : entries;
+  auto ctas = [&](int vb) { return (long long)((vdim + vb - 1) / vb) * H * portions; };
+  while (VB > 16 && ctas(VB) < pg::num_sms() && (portions == entries || 3 * ctas(VB / 2) <= 2LL * pg::num_sms())) VB /= 2;
   const int dim4 = (dim + 3) & ~3;
   auto bytes = [&](int vb) { return ((size_t)2 * 32 * (dim4 + 4) + 32 * vb + 32 * 32 + (size_t)dim4 * vb + 36) * sizeof(float); };
   while (VB > 8 && bytes(VB) > 200 * 1024) VB /= 2;

@@ -704,29 +704,35 @@ LINEAR_ATTN_CHUNK_MIN = 8
 
 
 def linear_attn(qkv, state, decay, out, b: StepBatch, H, dim, vdim, chunked=None):
-    """S <- decay S + k v^T, out = S^T q per head (fp32 [T, H * vdim]) with q, k and v through silu.  Portions of some length go in blocks -- on the tensor cores for bf16
-    head sizes that fit, there an entry's own length decides -- the others token by token (chunked True / False: one form for every entry)."""
+    """S <- decay S + k v^T, out = S^T q per head (fp32 [T, H * vdim]) with q, k and v through silu.  Portions of some length go in blocks -- for bf16 head sizes that fit
+    an entry's own length decides, and on the tensor cores where there are enough of them -- the others token by token (chunked True / False: one form for every entry)."""
     import ctypes as C
     assert state.dtype == torch.float32 and out.dtype == torch.float32 and out.is_contiguous() and qkv.stride(1) == 1
     f32 = int(qkv.dtype == torch.float32)
     n_min = {None: LINEAR_ATTN_CHUNK_MIN, True: 1, False: FOREVER}[chunked]
     # not for a few heads of a few sequences: there the other block form has more CTAs (its value blocks get narrower), and a chain of blocks is what takes the time (us, FMA / tensor:
     # 32 CTAs of 64 columns, 2000 tokens 330 / 370, 2 x 1000 tokens 171 / 191; 64 CTAs of 2000 tokens 458 / 371, of 100 tokens 35 / 29)
-    tensor_cores = (not f32 and dim % 8 == 0 and dim <= 128 and vdim % 8 == 0 and qkv.stride(0) % 8 == 0 and _aligned(qkv)
-                    and b.E * H * ((vdim + 63) // 64) >= 64)
+    # Single tokens own no blocks (2000 tokens beside 40 of them, 16 heads, FMA / tensor with the form for few CTAs / with that for many 332 / 375 / 414); beside them the FMA form's narrow
+    # blocks pay for fewer heads (24 329 / 373, 28 382 / 373).
+    portions = b.E - (b.singles if n_min > 1 else 0)
+    fits = not f32 and dim % 8 == 0 and dim <= 128 and vdim % 8 == 0 and qkv.stride(0) % 8 == 0 and _aligned(qkv)
+    tensor_cores = portions * H * ((vdim + 63) // 64) >= (64 if portions == b.E else 25)
 
     def go(fn, lo, hi, *tail):
-        ops = _lib.LinearAttnOps(1, 1.0, 0, 0, lo, hi)
+        ops = _lib.LinearAttnOps(1, 1.0, 0, 0, lo, hi, portions if lo == n_min else 0)
         _lib.check(fn(qkv.data_ptr(), qkv.stride(0), state.data_ptr(), decay.data_ptr(), out.data_ptr(), b.row0.data_ptr(), b.n.data_ptr(), b.ctx.data_ptr(),
                       b.slot.data_ptr(), b.E, H, dim, vdim, C.addressof(ops), *tail, _lib.stream()), "pg_linear_attn")
 
     L = _lib.lib()
     if b.max_n < n_min:
         go(L.pg_linear_attn_scan, 1, FOREVER, f32)
-    elif not tensor_cores:
+    elif not fits:
         go(L.pg_linear_attn_chunked, 1, FOREVER, f32)
     else:
-        go(L.pg_linear_attn_blocks, n_min, FOREVER)
+        if tensor_cores:
+            go(L.pg_linear_attn_blocks, n_min, FOREVER)
+        else:
+            go(L.pg_linear_attn_chunked, n_min, FOREVER, f32)
         if b.min_n < n_min:
             go(L.pg_linear_attn_scan, 1, n_min - 1, f32)
 
@@ -752,7 +758,7 @@ def retention(qkv, state, decay, out, b: StepBatch, H, dim, vdim, kscale=1.0, ro
     n_min = {None: RECURRENCE_BLOCK_MIN if tensor_cores else LINEAR_ATTN_CHUNK_MIN, True: 1, False: FOREVER}[blocks]
 
     def go(fn, lo, hi, *tail):
-        ops = _lib.LinearAttnOps(0, float(kscale), _lib.ptr(rotate), 0 if rotate is None else rotate.shape[2], lo, hi)
+        ops = _lib.LinearAttnOps(0, float(kscale), _lib.ptr(rotate), 0 if rotate is None else rotate.shape[2], lo, hi, b.E - b.singles if lo == n_min > 1 else 0)
         _lib.check(fn(qkv.data_ptr(), qkv.stride(0), state.data_ptr(), decay.data_ptr(), out.data_ptr(), b.row0.data_ptr(), b.n.data_ptr(), b.ctx.data_ptr(),
                       b.slot.data_ptr(), b.E, H, dim, vdim, C.addressof(ops), *tail, _lib.stream()), "pg_linear_attn")
 

@@ -61,3 +61,19 @@ def test_a_value_that_is_not_finite_stays_with_its_column_and_the_tokens_of_its_
     other = torch.ones(64 * 64, dtype=torch.bool, device="cuda")
     other[5] = False
     assert torch.equal(out[:, other], clean[:, other]) and torch.equal(out[:48, 5], clean[:48, 5]) and not out[50:, 5].isfinite().any()
+
+
+@pytest.mark.parametrize("H,dim,vdim", [(16, 64, 64), (3, 32, 72), (5, 128, 128)])
+@pytest.mark.parametrize("ns", [(200,) + (1,) * 40, (1, 1, 70, 1, 7)])
+def test_one_portion_among_single_tokens(H, dim, vdim, ns):
+    """Single tokens own no blocks: a few heads of one portion take the FMA blocks in the widths of one entry, the others go token by token."""
+    ctxs = [(13 * i) % 40 for i in range(len(ns))]
+    b, qkv, state, decay = _case(ns, ctxs, H, dim, vdim)
+    st, out = state.clone(), torch.full((b.T, H * vdim), float("nan"), device="cuda")
+    seq_ops.linear_attn(qkv, st, decay, out, b, H, dim, vdim)
+    r = 0
+    for i, (n, c) in enumerate(zip(ns, ctxs)):
+        want, S = _want(qkv[r:r + n], state[i] * (c > 0), decay, H, dim, vdim)
+        # fp32 sums of up to 200 tokens and 128 products, silu to 2^-22: 2^-20
+        assert _far(out[r:r + n], want) <= 2.0 ** -20 and _far(st[i], S) <= 2.0 ** -20
+        r += n
