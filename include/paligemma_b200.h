@@ -566,6 +566,10 @@ typedef struct PgConvSections {
 int pg_short_conv(const void* x, long long ldx, const float* w, const float* bias, float* state, void* out, long long ldo, float* inv, int ldi,
                   const PgConvSections* sections, int taps, int C, const int* entry_row0, const int* entry_n, const int* entry_ctx,
                   const int* entry_slot, int entries, int max_n, int act_f32, void* stream);
+/* The same where the host knows how many entries have more than one new token (portions; 0: not known): it only chooses how rows are shared out. */
+int pg_short_conv_sized(const void* x, long long ldx, const float* w, const float* bias, float* state, void* out, long long ldo, float* inv, int ldi,
+                        const PgConvSections* sections, int taps, int C, const int* entry_row0, const int* entry_n, const int* entry_ctx,
+                        const int* entry_slot, int entries, int max_n, int portions, int act_f32, void* stream);
 
 /* Delta rule, one decay per head and key channel.  Row t, head h (hk = h / (H / G)): q = q[t * ldq + hk * dim ..] * inv[t * ldi + hk], k likewise
  * with inv[t * ldi + G + hk], v = v[t * ldv + h * vdim ..], b = sigmoid(beta[t * ldb + h]), g[d] = exp(-exp(A_log[h]) *

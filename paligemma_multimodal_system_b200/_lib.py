@@ -120,6 +120,7 @@ SIGNATURES = {
     "pg_sigmoid_gate_mul": [p, i64, p, i64, i32, i32, i32, p],
     "pg_layernorm_shift": [p, p, p, p, p, p, p, p, p, p, p, p, p, p, i32, i32, f32, i32, p],
     "pg_short_conv": [p, i64, p, p, p, p, i64, p, i32, p, i32, i32, p, p, p, p, i32, i32, i32, p],
+    "pg_short_conv_sized": [p, i64, p, p, p, p, i64, p, i32, p, i32, i32, p, p, p, p, i32, i32, i32, i32, p],
     "pg_recurrence_block": [i32],
     "pg_delta_scan": [p, i32, i32, i32, p],
     "pg_gated_scan": [p, i32, i32, i32, i32, p],

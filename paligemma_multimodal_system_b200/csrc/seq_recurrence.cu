@@ -782,15 +782,20 @@ inline int conv_vec_width(const void* x, long long ldx, const float* w, const fl
 template <int TAPS, int V>
 int launch_conv_vec(const void* x, long long ldx, const float* w, const float* bias, float* state, void* out, long long ldo, float* inv, int ldi,
                     const PgConvSections& sec, int taps, int C, const int* row0, const int* n, const int* ctx, const int* slot, int entries, int max_n,
-                    cudaStream_t st) {
+                    int portions, cudaStream_t st) {
   int warps = 0;
   for (int s = 0; s < sec.count; ++s) warps += (sec.total[s] + 32 * V - 1) / (32 * V);
-  // runs of 64 rows, shortened while an SM would have fewer than 24 warps; below 16 rows a warp's weights and section cost more than the rows, so runs of 8 only
-  // where even those leave an SM with fewer than 8 (3795 rows, 48 warps wide: runs of 16 / 32 42 / 28 us)
+  // runs of 64 rows, shortened while an SM would have fewer than 24 warps with rows; below 16 rows a warp's weights and section cost more than the rows, so runs of 8 only
+  // where even those leave an SM with fewer than 8 (3795 rows, 48 warps wide: runs of 16 / 32 42 / 28 us).  Single tokens have one run of one row and the grid's other runs as CTAs
+  // without rows, so those are kept below 96 for an SM (one portion beside 40 single tokens, runs of 16 / 32 / 64: 100 rows 6.6 / 9.5 / 15.1 us, 700 rows, the first past that line, 15.9 /
+  // 10.8 / 16.3; 2 x 2000 rows 58 / 38 / 29).
   int chunk = 64;
-  auto runs = [&](int c) { return (long long)warps * entries * ((max_n + c - 1) / c); };
-  while (chunk > 16 && runs(chunk) < 24LL * pg::num_sms()) chunk /= 2;
-  if (chunk == 16 && runs(16) < 8LL * pg::num_sms()) chunk = 8;
+  const bool mixed = portions > 0 && portions < entries;
+  auto per_entry = [&](int c) { return (long long)(max_n + c - 1) / c; };
+  auto runs = [&](int c) { return warps * (mixed ? portions * per_entry(c) + (entries - portions) : entries * per_entry(c)); };
+  auto room = [&](int c) { return !mixed || (warps + 3) / 4 * (entries - portions) * per_entry(c) <= 96LL * pg::num_sms(); };
+  while (chunk > 16 && runs(chunk) < 24LL * pg::num_sms() && room(chunk / 2)) chunk /= 2;
+  if (chunk == 16 && runs(16) < 8LL * pg::num_sms() && room(8)) chunk = 8;
   const dim3 grid((warps + 3) / 4, (max_n + chunk - 1) / chunk, entries);
   pg::launch_dependent(short_conv_vec_kernel<TAPS, V>, grid, 128, 0, st, static_cast<const bf16*>(x), ldx, w, bias, state, static_cast<bf16*>(out), ldo, inv, ldi, sec, taps, C, row0,
                                                         n, ctx, slot, chunk);
@@ -824,6 +829,12 @@ int conv_shape(const void* x, long long ldx, const float* w, const float* bias, 
 extern "C" int pg_short_conv(const void* x, long long ldx, const float* w, const float* bias, float* state, void* out, long long ldo, float* inv,
                              int ldi, const PgConvSections* sec, int taps, int C, const int* entry_row0, const int* entry_n, const int* entry_ctx,
                              const int* entry_slot, int entries, int max_n, int act_f32, void* stream) {
+  return pg_short_conv_sized(x, ldx, w, bias, state, out, ldo, inv, ldi, sec, taps, C, entry_row0, entry_n, entry_ctx, entry_slot, entries, max_n, 0, act_f32, stream);
+}
+
+extern "C" int pg_short_conv_sized(const void* x, long long ldx, const float* w, const float* bias, float* state, void* out, long long ldo, float* inv,
+                                   int ldi, const PgConvSections* sec, int taps, int C, const int* entry_row0, const int* entry_n, const int* entry_ctx,
+                                   const int* entry_slot, int entries, int max_n, int portions, int act_f32, void* stream) {
   if (sec == nullptr || sec->count <= 0 || sec->count > 3 || taps < 1 || taps > 8 || C <= 0 || entries <= 0 || entries > 65535 || max_n <= 0) return PG_ERR_ARG;
   if (taps > 1 && state == nullptr) return PG_ERR_ARG;
   for (int s = 0; s < sec->count; ++s) {
@@ -838,7 +849,7 @@ extern "C" int pg_short_conv(const void* x, long long ldx, const float* w, const
     PG_CV(float, 8);
   }
   const int vw = conv_vec_width(x, ldx, w, bias, state, out, ldo, C, *sec);
-#define PG_CVV(TAPS, V) return launch_conv_vec<TAPS, V>(x, ldx, w, bias, state, out, ldo, inv, ldi, *sec, taps, C, entry_row0, entry_n, entry_ctx, entry_slot, entries, max_n, s)
+#define PG_CVV(TAPS, V) return launch_conv_vec<TAPS, V>(x, ldx, w, bias, state, out, ldo, inv, ldi, *sec, taps, C, entry_row0, entry_n, entry_ctx, entry_slot, entries, max_n, portions, s)
   if (vw == 4 && taps <= 4) PG_CVV(4, 4);
   if (vw == 4) PG_CVV(8, 4);
   if (vw == 8 && taps <= 4) PG_CVV(4, 8);

@@ -806,9 +806,9 @@ def short_conv(x, w, state, out, sections: ConvSections, b: StepBatch, bias=None
     assert taps == 1 or (state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (taps - 1, chans))
     assert bias is None or (bias.dtype == torch.float32 and bias.numel() == chans)
     assert (inv is None) == (sections.unit_groups == 0) and (inv is None or (inv.dtype == torch.float32 and inv.is_contiguous() and inv.shape == (b.T, sections.unit_groups)))
-    _lib.check(_lib.lib().pg_short_conv(x.data_ptr(), x.stride(0), w.data_ptr(), _lib.ptr(bias), _lib.ptr(state), out.data_ptr(), out.stride(0), _lib.ptr(inv),
-                                        sections.unit_groups, C.addressof(sections.c), taps, chans, b.row0.data_ptr(), b.n.data_ptr(), b.ctx.data_ptr(),
-                                        b.slot.data_ptr(), b.E, b.max_n, int(x.dtype == torch.float32), _lib.stream()), "pg_short_conv")
+    _lib.check(_lib.lib().pg_short_conv_sized(x.data_ptr(), x.stride(0), w.data_ptr(), _lib.ptr(bias), _lib.ptr(state), out.data_ptr(), out.stride(0), _lib.ptr(inv),
+                                              sections.unit_groups, C.addressof(sections.c), taps, chans, b.row0.data_ptr(), b.n.data_ptr(), b.ctx.data_ptr(),
+                                              b.slot.data_ptr(), b.E, b.max_n, b.E - b.singles, int(x.dtype == torch.float32), _lib.stream()), "pg_short_conv")
     return out
 
 

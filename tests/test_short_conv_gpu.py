@@ -58,3 +58,27 @@ def test_rows(sections, taps, ns, ctxs, bias):
                 assert ((inv[r:r + n, u:u + s["groups"]].double() - want).abs() <= 2.0 ** -18 * want).all()
                 u += s["groups"]
         r += n
+
+
+@pytest.mark.parametrize("n,many", [(100, 40), (700, 40), (700, 3), (64, 300)])
+def test_how_rows_are_shared_out_changes_nothing(n, many):
+    """pg_short_conv knows nothing of the batch; told how many entries are more than single tokens it takes other runs of rows, and the same bits come out."""
+    import ctypes as C
+    from paligemma_multimodal_system_b200 import _lib
+    ns = [1] * (many // 2) + [n] + [1] * (many - many // 2)
+    b = seq_ops.make_step_batch([dict(tokens=[1] * k, ctx=i % 5, slot=i, pages=list(range(12))) for i, k in enumerate(ns)])
+    cs = seq_ops.ConvSections([dict(groups=8, size=64, xcol=0, ccol=0, unit=True), dict(groups=4, size=64, xcol=512, ccol=512)])
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x, w, state = torch.randn(b.T, 768, generator=g, device="cuda").to(torch.bfloat16), torch.randn(4, 768, generator=g, device="cuda"), torch.randn(len(ns), 3, 768, generator=g, device="cuda")
+    res, L = [], _lib.lib()
+    for portions in (None, 0, 1, len(ns)):
+        st, out, inv = state.clone(), torch.full_like(x, 7.0), torch.zeros(b.T, 8, device="cuda")
+        args = [x.data_ptr(), 768, w.data_ptr(), 0, st.data_ptr(), out.data_ptr(), 768, inv.data_ptr(), 8, C.addressof(cs.c), 4, 768, b.row0.data_ptr(), b.n.data_ptr(), b.ctx.data_ptr(),
+                b.slot.data_ptr(), len(ns), n]
+        if portions is None:
+            _lib.check(L.pg_short_conv(*args, 0, _lib.stream()), "pg_short_conv")
+        else:
+            _lib.check(L.pg_short_conv_sized(*args, portions, 0, _lib.stream()), "pg_short_conv_sized")
+        res.append((out, st, inv))
+    for r in res[1:]:
+        assert all(torch.equal(a, c) for a, c in zip(r, res[0]))

@@ -57,3 +57,12 @@ def test_linear_attention(library, monkeypatch, ns, H, dtype, want):
         setattr(library, name, note(name))
     seq_ops.linear_attn(qkv, state, torch.zeros(H), out, b, H, d, d)
     assert seen == want
+
+
+@pytest.mark.parametrize("ns,portions", [([700] + [1] * 40, 1), ([700, 2], 2), ([1] * 5, 0)])
+def test_short_convolution(library, ns, portions):
+    b = _batch(ns)
+    sec = seq_ops.ConvSections([dict(groups=1, size=8, xcol=0, ccol=0)])
+    seq_ops.short_conv(torch.zeros(b.T, 8), torch.zeros(4, 8), torch.zeros(1, 3, 8), torch.zeros(b.T, 8), sec, b)
+    (name, args), = library.calls
+    assert name == "pg_short_conv_sized" and args[16:19] == (len(ns), max(ns), portions)
