@@ -639,18 +639,20 @@ int pg_attn_ragged_tc(const void* q, const void* kp, const void* vp, const void*
                       int portions, int longest, const PgAttnScore& sx, cudaStream_t st) {
   // pages that a tile of 64 keys divides, or that divide it in whole swizzle rows
   if (!(page > 0 && (page % 64 == 0 || (page % 8 == 0 && 64 % page == 0))) || sx.logistic || sx.dist_a != nullptr || sx.out_ld % 8 != 0) return 1;
-  // Blocks of 128 rows do not pay for a handful of rows in more CTAs than SMs (the mma.sync kernel's warps without rows idle; us, mma.sync / here, 16 heads of 64: 16 x 8 tokens
-  // behind 2000 57 / 72, behind 500 19 / 25; 4 x 8 tokens behind 2000 50 / 49), nor, for 64 / 128, whose S waits for P V, while that kernel's twice as many CTAs are one
-  // wave (16 heads: 400 tokens behind 2000 74 / 82, 200 tokens 12.7 / 15.4; 4 x 200 tokens, 256 CTAs, behind 500 41 / 29).
-  const long long rows = static_cast<long long>(max_n) * (H / G), units = static_cast<long long>(G) * entries;
-  if ((rows <= 16 && units > pg::num_sms()) || (dim == 64 && vdim == 128 && (rows + 63) / 64 * units <= pg::num_sms())) return 1;
+  // Blocks of 128 rows do not pay for a handful of rows in more CTAs than SMs (the mma.sync kernel's warps without rows idle; us, mma.sync / here, rows of a block x CTAs behind contexts of 1000:
+  // 16 x 24 24.7 / 15.5, 16 x 96 24.9 / 21.5, 4 x 96 26.2 / 21.4, 4 x 192 28.8 / 33.4, 4 x 384 31.5 / 51.7; behind 500: 16 x 192 16.3 / 20.1, 8 x 320 17.8 / 29.6).  Entries without rows
+  // for this kernel are no CTAs (`portions`, where the caller knows): 4 tokens behind 1000 beside 40 single ones, 32 heads over 8: 24.7 / 16.0.  Values of 128 columns leave one area for S
+  // and P, so a few CTAs with short keys are as fast there (16 heads, mma.sync / here: 200 tokens 11.6 / 12.3, behind 500 25.6 / 22.4, 400 behind 2000 71 / 65).
+  const int counted = portions > 0 && portions < entries ? portions : entries;
+  const long long rows = static_cast<long long>(max_n) * (H / G), units = static_cast<long long>(G) * counted;
+  if ((rows <= 16 && units > pg::num_sms()) || (dim == 64 && vdim == 128 && longest <= 256 && (rows + 63) / 64 * units <= pg::num_sms())) return 1;  // (longest 0: not known)
   // Two CTAs a block where the blocks are too few for the SMs and long enough to share out (portions and longest: entries with rows and the longest context with its new tokens, 0 where
   // the caller does not know; us, one CTA / two: 80 blocks of 24 .. 28 tiles 38 / 31, 32 of 24 .. 26 28 / 21, 64 of 16 40 / 35, 96 of 26 of 96 / 64 37 / 33; but 160 blocks of 24 .. 28
   // 40 / 41, 192 of 26 49 / 51, 128 of up to 8 15.6 / 16.5).
   const long long blocks = (rows + 127) / 128 * G * portions;
   const int reach = sx.window > 0 ? (longest < sx.window + (sx.keep_first > 0 ? sx.keep_first : 0) + 128 ? longest : sx.window + (sx.keep_first > 0 ? sx.keep_first : 0) + 128) : longest;
   const bool split = vdim == 64 && portions > 0 && 4 * blocks <= 3LL * pg::num_sms() && reach >= 12 * 64;
-#define PG_TC1(D, V, S) return pg::launch<D, V, S>(q, kp, vp, gate, ldg, out, row0, n, ctx, pt, max_pages, page, entries, portions > 0 && portions < entries ? portions : entries, max_n, H, G, scale, softcap, \
+#define PG_TC1(D, V, S) return pg::launch<D, V, S>(q, kp, vp, gate, ldg, out, row0, n, ctx, pt, max_pages, page, entries, counted, max_n, H, G, scale, softcap, \
                                                    skip_single, gate_per_head, sx, st)
 #define PG_TC(D, V)                  \
   if (dim == D && vdim == V) {       \

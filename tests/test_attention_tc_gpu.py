@@ -202,3 +202,10 @@ def test_what_the_host_has_counted_changes_nothing(dim, vdim, G, gsz, skip):
             _lib.check(L.pg_attn_ragged_mma_sized(*args, counted, 240, 0, _lib.stream()), "pg_attn_ragged_mma_sized")
         outs.append(out)
     assert all(torch.equal(o, outs[0]) for o in outs) and (outs[0] == 7).all(1).sum() == (4 if skip else 0)
+
+
+@pytest.mark.parametrize("dim,vdim,G,gsz,n,ctx", [(64, 64, 8, 4, 4, 300), (64, 64, 16, 1, 2, 900), (64, 128, 16, 1, 200, 40), (64, 128, 16, 1, 200, 100), (64, 128, 4, 4, 70, 600)])
+@pytest.mark.parametrize("many", [0, 40])
+def test_a_few_rows_beside_single_tokens(dim, vdim, G, gsz, n, ctx, many):
+    """Single tokens left to another kernel are no CTAs of this one: the form is that of the portion alone, on either side of the lines between the two kernels."""
+    _run(dim, vdim, G, gsz, [1] * (many // 2) + [n] + [1] * (many // 2), [70] * (many // 2) + [ctx] + [0] * (many // 2), 0, 0, skip=True)
