@@ -12,7 +12,9 @@
 // rounded in fp32 (all products of a block on one accumulator: 1.3e-6 against 64 bits where it is 7.9e-8 now).  The raw rows of the next block and its cosines / sines are fetched into registers,
 // its values with cp.async (SILU: into registers as well; they are staged as three terms), while the current block is multiplied.
 //
-// What bounds it: the mma.sync pipe, six products for one of fp32 (about 650 instructions a warp and block of 64), and between them the cuts into terms; two CTAs per SM.
+// What bounds it: the mma.sync pipe, six products for one of fp32, and between them the cuts into terms; two CTAs per SM, or three (see the dispatch).  Blocks are 32 tokens: with 64 the
+// accumulators of their own do not fit the registers (without silu, 48 prompts of 193 .. 256 tokens, 16 heads, blocks of 64 / 32: 64 wide 126 / 97 us, 32 wide 72 / 62; 2 x 1000 tokens 118 /
+// 81; 64 with one accumulator, six times the error: 107, 69, 90).
 // SILU, 48 prompts of 193 .. 256 tokens, 32 heads of 64: FMA chains over blocks of 32 (linear_attn_chunked_kernel, bound by its shared-memory operands) 570 us, here 283; the error
 // against 64 bits 1.6e-7 there, 0.8e-7 here.
 #include "common.cuh"
@@ -188,7 +190,8 @@ __global__ void __launch_bounds__(128, CTAS) linear_attn_block_kernel(const bf16
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int away = ((i & 2) ? th : tl) - (j + (i & 1));
-          p[i] = away >= 0 ? ((s[0][nb][i] + s[1][nb][i]) + (sl[0][nb][i] + sl[1][nb][i])) * ap[away >= 0 ? away : 0] : 0.f;
+          const float sum = APART ? (s[0][nb][i] + s[1][nb][i]) + (sl[0][nb][i] + sl[1][nb][i]) : s[0][nb][i] + s[1][nb][i];
+          p[i] = away >= 0 ? sum * ap[away >= 0 ? away : 0] : 0.f;
         }
         uint32_t c[3][2];
         cut3(p[0], p[1], c[0][0], c[1][0], c[2][0]);
@@ -238,7 +241,10 @@ __global__ void __launch_bounds__(128, CTAS) linear_attn_block_kernel(const bf16
       for (int nb = 0; nb < C / 8; ++nb) {
         const float c0 = ap[nb * 8 + 2 * tq + 1], c1 = ap[nb * 8 + 2 * tq + 2];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) o[nb][i] = ((PAR == 2 ? oh[0][nb][i] + oh[PAR - 1][nb][i] : oh[0][nb][i]) + ol[nb][i]) * ((i & 1) ? c1 : c0);
+        for (int i = 0; i < 4; ++i) {
+          const float lead = PAR == 2 ? oh[0][nb][i] + oh[PAR - 1][nb][i] : oh[0][nb][i];
+          o[nb][i] = (APART ? lead + ol[nb][i] : lead) * ((i & 1) ? c1 : c0);
+        }
       }
     }
     const float carry = ap[cn];
