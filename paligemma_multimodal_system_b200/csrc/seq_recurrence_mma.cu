@@ -34,12 +34,6 @@ namespace {
 constexpr float LOG2E = 1.4426950408889634f;
 
 __device__ __forceinline__ float softplus(float z) { return fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))); }
-// 2^x by the hardware alone: exponents are differences <= 0, and what underflows weighs nothing
-__device__ __forceinline__ float ex2_ftz(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 __device__ __forceinline__ float lo_f(uint32_t u) { return __uint_as_float(u << 16); }
 __device__ __forceinline__ float hi_f(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
 
@@ -497,7 +491,7 @@ __global__ void __launch_bounds__(128) delta_blocks_kernel(PgDeltaArgs a, float*
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const float z = lg[it][i] + bias;
-      const float sp = fmaxf(z, 0.f) + log1pf(ex2_ftz(-fabsf(z) * LOG2E));
+      const float sp = fmaxf(z, 0.f) + log1pf(exp2f(-fabsf(z) * LOG2E));
       if (i < nt) run = fmaf(rate, sp, run);
       lg[it][i] = run;
     }
@@ -508,7 +502,7 @@ __global__ void __launch_bounds__(128) delta_blocks_kernel(PgDeltaArgs a, float*
       Lg[o + i * LD] = lg[it][i];
       Kn[o + i * LD] = kv;
       Qn[o + i * LD] = qv;
-      const float f = ex2_ftz(half == 0 ? run - lg[it][i] : lg[it][i]);
+      const float f = exp2f(half == 0 ? run - lg[it][i] : lg[it][i]);
       Kf[o + i * LD] = kv * f;
       if (half == 1) Qf[i * LD + d] = qv * f;
     }
@@ -537,7 +531,7 @@ __global__ void __launch_bounds__(128) delta_blocks_kernel(PgDeltaArgs a, float*
         const float4 lt = *reinterpret_cast<const float4*>(Lg + t * LD + d), lj = *reinterpret_cast<const float4*>(Lg + j * LD + d);
         const float4 kt = *reinterpret_cast<const float4*>(Kn + t * LD + d), kj = *reinterpret_cast<const float4*>(Kn + j * LD + d);
         const float4 qt = *reinterpret_cast<const float4*>(Qn + t * LD + d);
-        const float e0 = ex2_ftz(lt.x - lj.x) * kj.x, e1 = ex2_ftz(lt.y - lj.y) * kj.y, e2 = ex2_ftz(lt.z - lj.z) * kj.z, e3 = ex2_ftz(lt.w - lj.w) * kj.w;
+        const float e0 = exp2f(lt.x - lj.x) * kj.x, e1 = exp2f(lt.y - lj.y) * kj.y, e2 = exp2f(lt.z - lj.z) * kj.z, e3 = exp2f(lt.w - lj.w) * kj.w;
         sa = fmaf(kt.x, e0, fmaf(kt.y, e1, fmaf(kt.z, e2, fmaf(kt.w, e3, sa))));
         sb = fmaf(qt.x, e0, fmaf(qt.y, e1, fmaf(qt.z, e2, fmaf(qt.w, e3, sb))));
       }
@@ -678,18 +672,18 @@ __global__ void __launch_bounds__(DIM <= 64 ? 256 : 128, DIM <= 64 ? 2 : 1) delt
       uint32_t t[9][4];
 #pragma unroll
       for (int p = 0; p < 4; ++p) {
-        const float f0 = ex2_ftz(l[2 * p]), f1 = ex2_ftz(l[2 * p + 1]);
+        const float f0 = exp2f(l[2 * p]), f1 = exp2f(l[2 * p + 1]);
         const float k0 = lo_f(kw[p]) * ik, k1 = hi_f(kw[p]) * ik;
         cut3(k0 * f0, k1 * f1, t[0][p], t[1][p], t[2][p]);
         cut3(lo_f(qw[p]) * iq * f0, hi_f(qw[p]) * iq * f1, t[3][p], t[4][p], t[5][p]);
         // a row past the end has k = 0; its exponent must only not overflow
-        cut3(k0 * ex2_ftz(fminf(le[2 * p] - l[2 * p], 0.f)), k1 * ex2_ftz(fminf(le[2 * p + 1] - l[2 * p + 1], 0.f)), t[6][p], t[7][p], t[8][p]);
+        cut3(k0 * exp2f(fminf(le[2 * p] - l[2 * p], 0.f)), k1 * exp2f(fminf(le[2 * p + 1] - l[2 * p + 1], 0.f)), t[6][p], t[7][p], t[8][p]);
       }
 #pragma unroll
       for (int m = 0; m < 9; ++m) *reinterpret_cast<uint4*>(base + m * TILE + c) = make_uint4(t[m][0], t[m][1], t[m][2], t[m][3]);
       if (r == 0) {
 #pragma unroll
-        for (int x = 0; x < 8; ++x) Ge[buf * DIM + c + x] = ex2_ftz(le[x]);
+        for (int x = 0; x < 8; ++x) Ge[buf * DIM + c + x] = exp2f(le[x]);
       }
     }
   };
