@@ -269,12 +269,13 @@ int pg_merge_embeddings(const long long* input_ids, const long long* attn_mask, 
  *   pg_merge_scan  -> pos[b,s], src_scratch[b,s] (j >= 0: j-th image token | -1 text | -2 pad), err_flag, and (dst_row != NULL)
  *                     dst_row[b*N + j] = b*S + s: the merged row of image feature j, the out_row_map of the projector GEMM;
  *   pg_merge_text  -> fills the text / pad rows of h (embedding gather * text_scale, zeros) and leaves the image rows alone.
+ * For callers that check ids themselves and collect the count errors of several scans in one flag; the models of this package use the pair below.
  */
 int pg_merge_scan(const long long* input_ids, const long long* attn_mask, int* pos, int* src_scratch, int* dst_row, int* err_flag,
                   int B, int S, int N, long long image_token, long long pad_token, void* stream);
 int pg_merge_text(const long long* input_ids, const int* src_scratch, const void* embed, float* h, int B, int S, int D, int N,
                   float text_scale, void* stream);
-/* The two halves with the input checks inside: pg_prompt_scan writes flags[b] (1: the row does not hold N image tokens, 2: an id outside [0, vocab)) and all of dst_row (B * S: no
+/* The two halves with the input checks inside, one flag a row, which need nothing cleared in front: pg_prompt_scan writes flags[b] (1: the row does not hold N image tokens, 2: an id outside [0, vocab)) and all of dst_row (B * S: no
  * slot); pg_prompt_text fills rows of ids outside with zeros and, first_row != NULL, copies the merged row of every row's first image feature to first_row[b] (fp32 [B, D]). */
 int pg_prompt_scan(const long long* input_ids, const long long* attn_mask, int* pos, int* src_scratch, int* dst_row, int* flags, int B, int S, int N,
                    long long vocab, long long image_token, long long pad_token, void* stream);
@@ -494,7 +495,7 @@ int pg_attn_ragged_mma(const void* q, const void* k_pages, const void* v_pages, 
                        const int* entry_row0, const int* entry_n, const int* entry_ctx, const int* page_table, int max_pages, int page,
                        int entries, int max_n, int H, int G, int dim, int vdim, float scale, float softcap, int skip_single,
                        int gate_per_head, const PgAttnScore* score, void* stream);
-/* The same with what the host knows of the batch: `portions` entries have rows for this kernel -- with skip_single exactly those whose entry_n is not 1, without it all of them (PG_ERR_ARG
+/* The same with what the host knows of the batch (what this package's models call): `portions` entries have rows for this kernel -- with skip_single exactly those whose entry_n is not 1, without it all of them (PG_ERR_ARG
  * for fewer); 0 or less: not known -- and `longest` is the longest context with its new tokens among them (it only chooses the form).  The grid is made for `portions` entries: as with max_n, rows
  * past what is promised are left out. */
 int pg_attn_ragged_mma_sized(const void* q, const void* k_pages, const void* v_pages, const void* gate, long long ldg, void* out,

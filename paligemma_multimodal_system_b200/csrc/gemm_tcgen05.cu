@@ -1091,8 +1091,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constan
   if (warp == 0 || warp == NEPI + 2) {
     // =================================== TMA producers (both CTAs) ==================================
     // Two warps, every other stage each (a stage keeps one producer: it has seen every earlier phase of the barrier that it waits on): one turns a stage around in about
-    // 290 ns, the pair's UMMAs read it in 270 at full clocks.  8192 tokens, 1152 x 1152 26.0 -> 25.7 us, 1152 x 4304 60.1 -> 59.2, 4304 x 1152 68.6 -> 67.3; products under the
-    // power cap (32768 x 2048) are as before, and so are the few-token kernels with two producers (48 x 16384 x 2048 15.4 / 15.1, 64 x 2048 x 8192 41.5 / 42.6)
+    // 290 ns, the pair's UMMAs read it in 270 at full clocks.  8192 tokens, caches flushed before, K = 1152 to 4304 features 71.7 -> 69.7 us, K = 4304 to 1152 79.9 -> 77.8, 1152 to
+    // 1152 and 3456 as before (43.0, 61.4; launch after launch 1152 to 1152 29.6 -> 28.9); products under the power cap (32768 x 2048) are as before, and so are the few-token kernels
+    // with two producers (48 x 16384 x 2048 15.4 / 15.1, 64 x 2048 x 8192 41.5 / 42.6)
     const int mine = warp == 0 ? 0 : 1;
     if (lane == 0) {
       int stage = 0;

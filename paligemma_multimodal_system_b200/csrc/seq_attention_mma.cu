@@ -382,8 +382,8 @@ __global__ void __launch_bounds__(128, (DIM + VDIM <= 128) ? 4 : 2) attn_ragged_
 // so the values are neither stored nor fetched separately; probabilities stay fp32 and enter as three bf16 terms.
 // With several key splits the (max, sum, accumulator) triples go to `partial` in the layout of pg_attn_decode and its merge
 // kernel finishes the rows.  What bounds it: latencies -- a CTA of two warps and a few tiles -- and instructions, so the queries are requested together with the first keys, fragments come four
-// at a time and a tile of one page needs one table entry (us with the merge, 32 heads of 288 / 256, before / now: 40 tokens behind 550 .. 1100 46 / 28, 64 behind 3000 97 / 64, one 36 / 20;
-// columns of the values shared out over two warps each: 30, 72, 18).  VS > 1: the value columns are shared out over VS CTAs (each recomputes the scores; a thread's accumulators
+// at a time and a tile of one page needs one table entry (us with the merge, launch after launch, 32 heads of 288 / 256, before / now: 40 tokens behind 550 .. 1100 42 / 25, 64 behind 3000 97 / 60, one 35 / 19;
+// columns of the values shared out over two warps each were 7 % and 13 % slower for the many, 10 % faster for the one).  VS > 1: the value columns are shared out over VS CTAs (each recomputes the scores; a thread's accumulators
 // stay at 128 registers for value parts up to 512 wide).
 // ---------------------------------------------------------------------------------------------------------------------
 template <int DIM, int VDIM, int KT, int VS>
