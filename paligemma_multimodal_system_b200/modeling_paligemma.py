@@ -174,8 +174,13 @@ class PaliGemmaForConditionalGeneration(nn.Module):
         _lib.gemm(feats, self._proj_w, h, mode=_lib.EPI_F32, bias=self._proj_b, scale=img_scale, swap=0,
                   out_row_map=dst)
         h = h[: B * S]
-        _lib.check(L.pg_prompt_text(ids.data_ptr(), src.data_ptr(), dst.data_ptr(), pk["embed"].data_ptr(), h.data_ptr(), _lib.ptr(first_image_row), B, S, D, N, V, D ** 0.5,
+        first = first_image_row
+        if first is not None and not (first.is_cuda and first.dtype == torch.float32 and first.is_contiguous() and first.numel() == B * D and first.data_ptr() % 16 == 0):
+            first = torch.empty(B, D, device=dev, dtype=torch.float32)  # (what the kernel writes; then as any copy)
+        _lib.check(L.pg_prompt_text(ids.data_ptr(), src.data_ptr(), dst.data_ptr(), pk["embed"].data_ptr(), h.data_ptr(), _lib.ptr(first), B, S, D, N, V, D ** 0.5,
                                     _lib.stream()), "pg_prompt_text")
+        if first is not first_image_row:
+            first_image_row.view(B, D).copy_(first)
         if not validate:
             return h, pos, flags
         there.synchronize()

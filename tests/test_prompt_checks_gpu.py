@@ -63,3 +63,26 @@ def test_errors(replayed):
         with pytest.raises(error):
             call(bad)
     assert torch.equal(call(ids), good[-1])
+
+
+def _tiny():
+    from paligemma_multimodal_system_b200.modeling_paligemma import PaliGemmaConfig, PaliGemmaForConditionalGeneration
+    from paligemma_multimodal_system_b200.random_init import TINY_CONFIG, make_inputs, make_state_dict
+    model = PaliGemmaForConditionalGeneration(PaliGemmaConfig(**copy.deepcopy(TINY_CONFIG)), device="cuda", dtype=torch.bfloat16).eval()
+    model.load_state_dict(make_state_dict(TINY_CONFIG, "R1", seed=3), strict=True)
+    model.tie_weights()
+    inp = {k: v.cuda() for k, v in make_inputs(TINY_CONFIG, batch=2, prompt_len=4, seed=5).items() if torch.is_tensor(v)}
+    return model, inp["input_ids"], inp["pixel_values"], inp["attention_mask"]
+
+
+@pytest.mark.parametrize("dtype,pitch", [(torch.float32, 1), (torch.float32, 3), (torch.bfloat16, 1), (torch.float64, 2)])
+def test_the_first_image_row_goes_to_any_tensor(dtype, pitch):
+    model, ids, px, mask = _tiny()
+    D = model.text_config.hidden_size
+    first = torch.empty(2, 1, D, device="cuda")
+    h, _ = model._embed_prompt(ids, mask, px, first_image_row=first)
+    room = torch.full((2, pitch, D), 7.0, device="cuda", dtype=dtype)
+    model._embed_prompt(ids, mask, px, first_image_row=room[:, :1])
+    at = (ids == model.dummy_image_token_id).int().argmax(1)
+    assert torch.equal(first[:, 0], h.view(2, -1, D)[torch.arange(2, device="cuda"), at])
+    assert torch.equal(room[:, 0], first[:, 0].to(dtype)) and (room[:, 1:] == 7).all()
