@@ -276,7 +276,7 @@ int pg_merge_scan(const long long* input_ids, const long long* attn_mask, int* p
 int pg_merge_text(const long long* input_ids, const int* src_scratch, const void* embed, float* h, int B, int S, int D, int N,
                   float text_scale, void* stream);
 /* The two halves with the input checks inside, one flag a row, which need nothing cleared in front: pg_prompt_scan writes flags[b] (1: the row does not hold N image tokens, 2: an id outside [0, vocab)) and all of dst_row (B * S: no
- * slot); pg_prompt_text fills rows of ids outside with zeros and, first_row != NULL, copies the merged row of every row's first image feature to first_row[b] (fp32 [B, D]). */
+ * slot); pg_prompt_text fills rows of ids outside with zeros and, first_row != NULL, copies the merged row of every row's first image feature to first_row[b] (fp32 [B, D], on 16 bytes). */
 int pg_prompt_scan(const long long* input_ids, const long long* attn_mask, int* pos, int* src_scratch, int* dst_row, int* flags, int B, int S, int N,
                    long long vocab, long long image_token, long long pad_token, void* stream);
 int pg_prompt_text(const long long* input_ids, const int* src_scratch, const int* dst_row, const void* embed, float* h, float* first_row, int B, int S, int D, int N,

@@ -701,7 +701,7 @@ extern "C" int pg_prompt_scan(const long long* input_ids, const long long* attn_
 
 extern "C" int pg_prompt_text(const long long* input_ids, const int* src_scratch, const int* dst_row, const void* embed, float* h, float* first_row, int B, int S, int D, int N,
                               long long vocab, float text_scale, void* stream) {
-  if (B <= 0 || S <= 0 || D <= 0 || (D % 4) || vocab <= 0 || !input_ids || !src_scratch || !embed || !h || (first_row != nullptr && (N <= 0 || !dst_row))) return PG_ERR_ARG;
+  if (B <= 0 || S <= 0 || D <= 0 || (D % 4) || vocab <= 0 || !input_ids || !src_scratch || !embed || !h || (first_row != nullptr && (N <= 0 || !dst_row || (reinterpret_cast<uintptr_t>(first_row) & 15) != 0))) return PG_ERR_ARG;
   pg::launch_dependent(merge_gather_kernel, B * S + (first_row != nullptr ? B : 0), 256, 0, PG_ST(stream), input_ids, src_scratch, static_cast<const bf16*>(embed), nullptr, h, S, D, N,
                        text_scale, 0.f, 1, B, dst_row, first_row, vocab);
   PG_RET();

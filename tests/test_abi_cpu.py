@@ -85,3 +85,12 @@ def test_fewer_portions_than_entries_without_single_tokens_left_out_are_refused(
 
     arg = lib.pg_attn_ragged_mma_sized(16, 16, 16, 0, 0, 16, 16, 16, 16, 16, 1, 64, 0, 5, 4, 4, 64, 64, 1.0, 0.0, 0, 0, 0, 0, 0, 0)  # no entries
     assert arg < 0 and [call(1, 0), call(2, 0)] == [arg] * 2
+
+
+def test_a_first_image_row_off_sixteen_bytes_is_refused():
+    """It is written sixteen bytes at a time.  (Refused before anything is launched.)"""
+    from paligemma_multimodal_system_b200 import _lib, build
+    build.build()
+    lib = _lib.lib()
+    for off in (4, 8):
+        assert lib.pg_prompt_text(16, 16, 16, 16, 16, 16 + off, 1, 4, 64, 1, 100, 1.0, 0) == -1
