@@ -42,7 +42,6 @@ class StepBatch:
     max_pages: int
     singles: int = 0          # entries with one new token (decode rows)
     max_single_ctx: int = 0   # the longest context among them
-    min_n: int = 1            # the fewest new tokens of an entry (1 where that is not known)
     single_rows: Optional[tuple] = None  # (first, one past the last) row between which all of them lie; None: unknown
     # dense scratch layout of the entries with several new tokens (mixers that rebuild per-head keys / values from a compact
     # cache): entry e owns rows [dense_row0[e], + ctx + n) of a dense matrix, starting on a page boundary, so that
@@ -55,6 +54,7 @@ class StepBatch:
     # what one layer of the CURRENT step leaves for later ones (rotation tables, a layer's values); a model that uses it starts every step
     # with a fresh one (`step_scope`)
     shared: Optional[dict] = None
+    min_n: int = 1            # the fewest new tokens of an entry (1 where that is not known)
 
 
 def _single_rows(ns):

@@ -66,3 +66,11 @@ def test_short_convolution(library, ns, portions):
     seq_ops.short_conv(torch.zeros(b.T, 8), torch.zeros(4, 8), torch.zeros(1, 3, 8), torch.zeros(b.T, 8), sec, b)
     (name, args), = library.calls
     assert name == "pg_short_conv_sized" and args[16:19] == (len(ns), max(ns), portions)
+
+
+def test_a_step_is_described_in_the_order_that_it_was():
+    """Fields that came later stand behind those that a caller may give by position."""
+    import dataclasses
+    names = [f.name for f in dataclasses.fields(seq_ops.StepBatch)]
+    assert names == ["T", "E", "max_n", "tokens", "pos", "row_entry", "row0", "n", "ctx", "slot", "page_table", "max_pages", "singles", "max_single_ctx", "single_rows", "dense_row0", "dense_pages",
+                     "dense_max_pages", "dense_rows", "dense_max_len", "shared", "min_n"]
